@@ -306,3 +306,53 @@ inline cudaError_t b2w4_launch_chained(bool pdl, void (*kernel)(KArgs...), dim3 
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+// The same launch with clusters of `cluster` blocks along x.  More than eight blocks per
+// cluster need an opt-in, an attribute of a kernel per device like the shared-memory one.
+template <typename Kernel>
+inline cudaError_t b2w4_opt_in_cluster(b2w4_ctx* ctx, Kernel kern, b2w4_smem_optin& cache) {
+    if (cache.bytes[ctx->device])
+        return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+        cache.bytes[ctx->device] = 1;
+    return e;
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t b2w4_launch_chained_cluster(bool pdl, void (*kernel)(KArgs...), dim3 grid,
+                                               dim3 block, int cluster, size_t smem,
+                                               cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Two fp32 lanes per instruction (sm_100's packed single-precision arithmetic): each lane is
+// the IEEE round-to-nearest operation of its scalar counterpart.
+#ifdef __CUDACC__
+__device__ __forceinline__ uint64_t b2w4_pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void b2w4_unpack2(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t b2w4_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+#endif

@@ -10,6 +10,8 @@
 // All tensors are fp32, rows = tokens, features contiguous.
 #include "b200w4_internal.cuh"
 
+#include <cooperative_groups.h>
+
 namespace {
 
 constexpr int kNormThreads = 256;
@@ -390,6 +392,293 @@ attention_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
         out[((size_t)t * heads + h) * dim + threadIdx.x] = acc;
 }
 
+// The same attention for a few query tokens (a decode step): a cluster of kSplitCtas blocks
+// splits the visible keys of one (token, kv head, up to HR of its query heads), so a step
+// fills the chip instead of one block per head, and the query heads of a kv head read its
+// keys and values once.  What bounds it: bytes in flight -- a key and value row are read once
+// and used HR times -- until the cache is short, where it is the chain load, exchange, exp,
+// load, exchange.
+//   scores   eight lanes per key hold four features each of every 32, a warp has 4 (KI)
+//            x 4 keys' loads in flight; products in pairs (fma.rn.f32x2), then a butterfly
+//            over the eight lanes that halves the items held at each level
+//   softmax  over the block's own keys: max m, e_j = exp(s_j - m), l = sum e_j
+//   P*V      a warp per key, four features per lane, HR accumulator rows; the warps' sums are
+//            added through shared memory
+//   merge    block r adds its share of the features over the cluster (distributed shared
+//            memory): out = sum_c w_c o_c / sum_c w_c l_c, w_c = exp(m_c - max m)
+// Measured, a step of eight layers with 32 / 8 heads of 128: 6000 keys 3447 -> 522 us (one
+// block per head: 32 of 148 SMs, every key read four times), 300 keys 501 -> 384 us; clusters
+// of eight 619 and 376 us, so sixteen, which need the non-portable opt-in.
+// The split depends on the number of visible keys alone, so a position given by the host and
+// one read on the device leave the same bits.  A probability of zero contributes nothing
+// (whatever the value row holds), as in attention_kernel; a NaN score reaches every feature.
+constexpr int kSplitCtas = 16;
+template <int DIM, int HR>
+struct SplitSmem {  // floats of dynamic shared memory before the scores
+    static constexpr int kAcc = 0;                              // [kAttnWarps][HR][DIM]
+    static constexpr int kOut = kAcc + kAttnWarps * HR * DIM;   // [HR][DIM]
+    static constexpr int kMax = kOut + HR * DIM;                // [HR] m, read by the cluster
+    static constexpr int kSum = kMax + HR;                      // [HR] l
+    static constexpr int kPart = kSum + HR;                     // [kAttnWarps][HR]
+    static constexpr int kWeight = kPart + kAttnWarps * HR;     // [HR][kSplitCtas]
+    static constexpr int kTotal = kWeight + HR * kSplitCtas;    // [HR] 1 / sum follows
+    static constexpr int kScores = (kTotal + HR + 3) & ~3;      // [keys][HR]
+};
+template <int DIM, int HR>
+__global__ void __launch_bounds__(kAttnThreads)
+attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
+                       const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
+                       int heads, int kv_heads, int past0, const int* __restrict__ past_dev,
+                       int capacity, float scale) {
+    b2w4_pdl_chain_entry();
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int past = past_dev ? min(*past_dev, capacity - tokens) : past0;
+    using S = SplitSmem<DIM, HR>;
+    extern __shared__ __align__(16) float s_dyn[];
+    float* s_acc = s_dyn + S::kAcc;
+    float* s_out = s_dyn + S::kOut;
+    float* s_max = s_dyn + S::kMax;
+    float* s_sum = s_dyn + S::kSum;
+    float* s_part = s_dyn + S::kPart;
+    float* s_weight = s_dyn + S::kWeight;
+    float* s_total = s_dyn + S::kTotal;
+    float* s_sc = s_dyn + S::kScores;
+    const int rep = heads / kv_heads, sets = (rep + HR - 1) / HR;
+    const int kvh = blockIdx.y / sets, r0 = (blockIdx.y % sets) * HR;  // heads r0.. of the kv head
+    const int nh = min(HR, rep - r0), t = blockIdx.z, rank = blockIdx.x;
+    const int visible = past + t + 1;
+    const int per = (visible + kSplitCtas - 1) / kSplitCtas;
+    const int j0 = min(rank * per, visible), n = min(per, visible - j0);
+    const size_t row0 = ((size_t)t * heads + (size_t)kvh * rep + r0) * DIM;
+    const float* kc = k_cache + ((size_t)kvh * capacity + j0) * DIM;
+    const float* vc = v_cache + ((size_t)kvh * capacity + j0) * DIM;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // ---- scores ----
+    {
+        constexpr int kF4 = DIM / 32;             // float4 of a row per lane
+        constexpr int KI = DIM > 128 ? 2 : 4;     // keys per lane group in flight
+        constexpr int kItems = KI * HR;
+        const int part = lane & 7, sub = lane >> 3;
+        uint64_t qv[HR][2 * kF4];
+#pragma unroll
+        for (int h = 0; h < HR; ++h)
+#pragma unroll
+            for (int i = 0; i < kF4; ++i) {
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (h < nh)
+                    x = *reinterpret_cast<const float4*>(q + row0 + h * DIM + 32 * i + 4 * part);
+                qv[h][2 * i] = b2w4_pack2(x.x, x.y);
+                qv[h][2 * i + 1] = b2w4_pack2(x.z, x.w);
+            }
+        for (int j = warp * 4 * KI; j < n; j += kAttnWarps * 4 * KI) {
+            float4 kr[KI][kF4];
+#pragma unroll
+            for (int it = 0; it < KI; ++it)
+#pragma unroll
+                for (int i = 0; i < kF4; ++i) {
+                    const int key = min(j + it * 4 + sub, n - 1);  // past the end: dropped below
+                    kr[it][i] = *reinterpret_cast<const float4*>(kc + (size_t)key * DIM + 32 * i +
+                                                                 4 * part);
+                }
+            float v[kItems];  // item it * HR + h
+#pragma unroll
+            for (int it = 0; it < KI; ++it)
+#pragma unroll
+                for (int h = 0; h < HR; ++h) {
+                    uint64_t a = 0, b = 0;  // (0.f, 0.f)
+#pragma unroll
+                    for (int i = 0; i < kF4; ++i) {
+                        a = b2w4_fma2(qv[h][2 * i], b2w4_pack2(kr[it][i].x, kr[it][i].y), a);
+                        b = b2w4_fma2(qv[h][2 * i + 1], b2w4_pack2(kr[it][i].z, kr[it][i].w), b);
+                    }
+                    float a0, a1, b0, b1;
+                    b2w4_unpack2(a, a0, a1);
+                    b2w4_unpack2(b, b0, b1);
+                    v[it * HR + h] = __fadd_rn(__fadd_rn(a0, b0), __fadd_rn(a1, b1));
+                }
+            int first = 0;  // the lane's first item
+            constexpr int kLevel[3] = {4, 2, 1};
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                const int off = kLevel[l], have = kItems >> l;
+                if (have > 1) {
+                    const bool up = lane & off;
+#pragma unroll
+                    for (int i = 0; i < have / 2; ++i) {
+                        const float send = up ? v[i] : v[i + have / 2];
+                        const float keep = up ? v[i + have / 2] : v[i];
+                        v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, off));
+                    }
+                    first += up ? have / 2 : 0;
+                } else {
+                    v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < (kItems > 8 ? kItems / 8 : 1); ++i) {
+                const int item = first + i, key = j + (item / HR) * 4 + sub;
+                if (key < n)
+                    s_sc[key * HR + item % HR] = __fmul_rn(v[i], scale);
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- softmax over the block's keys; a thread's items all belong to head tid % HR ----
+    const int my_head = threadIdx.x % HR;
+    auto head_reduce = [&](float x, bool maximum) {
+#pragma unroll
+        for (int off = 16; off >= HR; off >>= 1) {
+            const float y = __shfl_xor_sync(0xffffffffu, x, off);
+            x = maximum ? fmaxf(x, y) : __fadd_rn(x, y);
+        }
+        if (lane < HR)
+            s_part[warp * HR + lane] = x;
+        __syncthreads();
+        x = s_part[my_head];
+#pragma unroll
+        for (int w = 1; w < kAttnWarps; ++w)
+            x = maximum ? fmaxf(x, s_part[w * HR + my_head])
+                        : __fadd_rn(x, s_part[w * HR + my_head]);
+        __syncthreads();
+        return x;
+    };
+    float m = -INFINITY;
+    for (int i = threadIdx.x; i < n * HR; i += kAttnThreads)
+        m = fmaxf(m, s_sc[i]);
+    m = head_reduce(m, true);
+    // scores of -inf only (or none): e_j = exp(-inf) = 0 here, and w_c = 0 unless every
+    // block's are, which gives the NaN that attention_kernel gives
+    const float base = m == -INFINITY ? 0.f : m;
+    float sum = 0.f;
+    for (int i = threadIdx.x; i < n * HR; i += kAttnThreads) {
+        const float e = (float)exp((double)__fsub_rn(s_sc[i], base));
+        s_sc[i] = e;
+        sum = __fadd_rn(sum, e);
+    }
+    sum = head_reduce(sum, false);
+    if (threadIdx.x < HR) {
+        s_max[threadIdx.x] = m;
+        s_sum[threadIdx.x] = sum;
+    }
+
+    // ---- P*V ----
+    {
+        constexpr int kLanes = DIM / 4 < 32 ? DIM / 4 : 32;  // lanes per value row
+        constexpr int kV4 = DIM / 4 / kLanes;                // float4 per lane
+        constexpr int kKeys = 32 / kLanes;                   // keys per warp and step
+        constexpr int U = 8 / kV4;                           // steps in flight
+        const int part = lane % kLanes, sub = lane / kLanes;
+        uint64_t acc[HR][2 * kV4];
+#pragma unroll
+        for (int h = 0; h < HR; ++h)
+#pragma unroll
+            for (int i = 0; i < 2 * kV4; ++i)
+                acc[h][i] = 0;
+        for (int j = warp * kKeys + sub; j < n; j += kAttnWarps * kKeys * U) {
+            float4 vr[U][kV4];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < kV4; ++i) {
+                    const int key = min(j + u * kAttnWarps * kKeys, n - 1);
+                    vr[u][i] = *reinterpret_cast<const float4*>(vc + (size_t)key * DIM +
+                                                                4 * (part + kLanes * i));
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int key = j + u * kAttnWarps * kKeys;
+                if (key < n) {
+#pragma unroll
+                    for (int h = 0; h < HR; ++h) {
+                        const float p = s_sc[key * HR + h];
+                        if (p != 0.f) {
+                            const uint64_t pp = b2w4_pack2(p, p);
+#pragma unroll
+                            for (int i = 0; i < kV4; ++i) {
+                                acc[h][2 * i] = b2w4_fma2(b2w4_pack2(vr[u][i].x, vr[u][i].y), pp,
+                                                          acc[h][2 * i]);
+                                acc[h][2 * i + 1] =
+                                    b2w4_fma2(b2w4_pack2(vr[u][i].z, vr[u][i].w), pp,
+                                              acc[h][2 * i + 1]);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < HR; ++h)
+#pragma unroll
+            for (int i = 0; i < kV4; ++i) {
+                float4 o;
+                b2w4_unpack2(acc[h][2 * i], o.x, o.y);
+                b2w4_unpack2(acc[h][2 * i + 1], o.z, o.w);
+                if (kKeys > 1) {  // two keys per step: the half-warps' sums
+                    o.x = __fadd_rn(o.x, __shfl_xor_sync(0xffffffffu, o.x, 16));
+                    o.y = __fadd_rn(o.y, __shfl_xor_sync(0xffffffffu, o.y, 16));
+                    o.z = __fadd_rn(o.z, __shfl_xor_sync(0xffffffffu, o.z, 16));
+                    o.w = __fadd_rn(o.w, __shfl_xor_sync(0xffffffffu, o.w, 16));
+                }
+                if (sub == 0)
+                    *reinterpret_cast<float4*>(s_acc + (warp * HR + h) * DIM +
+                                               4 * (part + kLanes * i)) = o;
+            }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < HR * DIM; i += kAttnThreads) {
+        float a = s_acc[i];
+#pragma unroll
+        for (int w = 1; w < kAttnWarps; ++w)
+            a = __fadd_rn(a, s_acc[w * HR * DIM + i]);
+        s_out[i] = a;
+    }
+    cluster.sync();
+
+    // ---- merge ----
+    if (warp < HR) {  // warp h: head h's weights, lane c: block c of the cluster
+        const float mc = lane < kSplitCtas ? cluster.map_shared_rank(s_max, lane % kSplitCtas)[warp]
+                                           : -INFINITY;
+        const float lc = lane < kSplitCtas ? cluster.map_shared_rank(s_sum, lane % kSplitCtas)[warp]
+                                           : 0.f;
+        float top = mc;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+        const float w = (float)exp((double)__fsub_rn(mc, top));
+        float l = lane < kSplitCtas ? __fmul_rn(w, lc) : 0.f;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, off));
+        if (lane < kSplitCtas)
+            s_weight[warp * kSplitCtas + lane] = w;
+        if (lane == 0)
+            s_total[warp] = l;
+    }
+    __syncthreads();
+    constexpr int kShare = HR * DIM / kSplitCtas;  // outputs per block
+    if (threadIdx.x < kShare) {
+        const int i = rank * kShare + threadIdx.x, h = i / DIM;
+        float o[kSplitCtas];
+#pragma unroll
+        for (int c = 0; c < kSplitCtas; ++c)
+            o[c] = cluster.map_shared_rank(s_out, c)[i];
+        float a = 0.f;
+#pragma unroll
+        for (int c = 0; c < kSplitCtas; ++c) {
+            const float w = s_weight[h * kSplitCtas + c];
+            if (w != 0.f)
+                a = __fmaf_rn(w, o[c], a);
+        }
+        const float l = s_total[h];  // NaN if any score was
+        if (h < nh)
+            out[row0 + i] = __fdiv_rn(a, l);
+    }
+    cluster.sync();  // nobody leaves while its sums may still be read
+}
+
 // The same attention for a run of new tokens (prefill): one block per (kv head, tile of query
 // tokens) serves every query head of that kv head -- up to kTileRows (token, head) rows --
 // so that a chunk of keys or values is fetched into shared memory once per tile instead of
@@ -736,7 +1025,44 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
     }
     const float* kc = k_cache_dev;
     const float* vc = v_cache_dev;
-    if (tiles) {
+    const bool aligned = !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev) & 15);
+    if (tokens < 8 && aligned && (dim == 64 || dim == 128 || dim == 256)) {
+        const int per = (keys + kSplitCtas - 1) / kSplitCtas;
+#define B2W4_SPLIT(D, HR)                                                                      \
+    do {                                                                                       \
+        static b2w4_smem_optin cfg;                                                            \
+        static b2w4_smem_optin wide;                                                           \
+        const size_t smem = sizeof(float) * (SplitSmem<D, HR>::kScores + (size_t)per * HR);    \
+        const dim3 grid(kSplitCtas, kv_heads * ((rep + HR - 1) / HR), tokens);                 \
+        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, attention_split_kernel<D, HR>, smem, cfg));       \
+        B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, attention_split_kernel<D, HR>, wide));         \
+        B2W4_CUDA(ctx, b2w4_launch_chained_cluster(                                            \
+                           ctx->pdl, attention_split_kernel<D, HR>, grid, dim3(kAttnThreads),  \
+                           kSplitCtas, smem, ctx->stream, q_dev, kc, vc, out_dev, tokens,      \
+                           heads, kv_heads, past, past_dev, capacity, scale));                 \
+    } while (0)
+        if (dim == 256) {
+            if (rep >= 2)
+                B2W4_SPLIT(256, 2);
+            else
+                B2W4_SPLIT(256, 1);
+        } else if (dim == 128) {
+            if (rep >= 3)
+                B2W4_SPLIT(128, 4);
+            else if (rep == 2)
+                B2W4_SPLIT(128, 2);
+            else
+                B2W4_SPLIT(128, 1);
+        } else {
+            if (rep >= 3)
+                B2W4_SPLIT(64, 4);
+            else if (rep == 2)
+                B2W4_SPLIT(64, 2);
+            else
+                B2W4_SPLIT(64, 1);
+        }
+#undef B2W4_SPLIT
+    } else if (tiles) {
         const int tq = kTileRows / rep;
         const dim3 grid((tokens + tq - 1) / tq, kv_heads);
 #define B2W4_TILE(D)                                                                          \

@@ -254,3 +254,57 @@ def test_tile_attention_equals_the_row_kernel(ctx, tokens, past, heads, kv_heads
     assert outs[2].tobytes() == outs[0].tobytes()
     want = ol.causal_attention(q, k_all, v_all, heads, kv_heads, past, scale)
     assert rel_l2(outs[1], want) < 1e-5
+
+
+def _attention_fp64(q, k_all, v_all, heads, kv_heads, past, scale):
+    """Causal attention in 64 bits, key rows with a vanishing probability left out."""
+    tokens, rep = q.shape[0], heads // kv_heads
+    out = np.zeros(q.shape)
+    for t in range(tokens):
+        for h in range(heads):
+            k = k_all[:past + t + 1, h // rep].astype(np.float64)
+            s = (k @ q[t, h].astype(np.float64)) * scale
+            p = np.exp(s - s.max())
+            seen = p > 0
+            v = v_all[:past + t + 1, h // rep][seen].astype(np.float64)
+            out[t, h] = (p[seen] / p.sum()) @ v
+    return out
+
+
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [
+    (1, 0, 4, 4, 64), (1, 14, 8, 8, 64), (1, 15, 12, 2, 64), (2, 16, 6, 2, 128),
+    (1, 127, 4, 1, 128), (7, 1000, 10, 2, 128), (1, 4100, 2, 2, 128), (3, 31, 2, 2, 256),
+    (1, 777, 6, 2, 256)])
+def test_split_attention_of_a_few_tokens(ctx, tokens, past, heads, kv_heads, dim):
+    """Up to seven query tokens: the keys are split over a cluster of blocks (ranges of zero,
+    one or many keys, head groups that do not fill a block's rows).  Tolerance: the fp32 dot
+    product of 256 terms, 2^-24 * (16 adds in sequence) * sum |q k| * scale <= 1e-5, is the
+    relative error of a probability.  Then with a key whose probability underflows to zero and
+    whose value row is NaN: nothing of it may reach the output."""
+    import torch
+    capacity, scale = past + tokens + 5, dim ** -0.5
+    rng = np.random.default_rng(past + dim)
+    q = rng.normal(0, 1, (tokens, heads, dim)).astype(np.float32)
+    k_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    v_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    for hole in (None, past // 2):
+        if hole is not None:
+            if past == 0 or tokens > 1 or heads != kv_heads:
+                continue
+            k_all[hole] = -1e30 * np.sign(q[0])
+            v_all[hole] = np.nan
+        kc = np.zeros((kv_heads, capacity, dim), dtype=np.float32)
+        vc = np.full((kv_heads, capacity, dim), np.nan, dtype=np.float32)  # past the position
+        kc[:, :past + tokens] = k_all.transpose(1, 0, 2)
+        vc[:, :past + tokens] = v_all.transpose(1, 0, 2)
+        kcd, vcd, qd = _dev(kc), _dev(vc), _dev(q)
+        outs = []
+        for past_dev in (None, torch.full((1,), past, dtype=torch.int32, device="cuda")):
+            out = torch.zeros((tokens, heads, dim), dtype=torch.float32, device="cuda")
+            ctx.attention(qd, None, None, kcd, vcd, out, tokens, heads, kv_heads, dim,
+                          past if past_dev is None else 0, capacity, scale, past_dev)
+            ctx.sync()
+            outs.append(out.cpu().numpy())
+        assert outs[1].tobytes() == outs[0].tobytes()
+        assert rel_l2(outs[0], _attention_fp64(q, k_all, v_all, heads, kv_heads, past,
+                                               scale)) < 1e-5
