@@ -286,18 +286,33 @@ __global__ void qkv_prepare_kernel(const float* __restrict__ qkv, int ld, int to
 }
 
 // Scaled-dot-product attention of one (query token, head) over the cache, the x86 reference's
-// arithmetic (kernels/attention_x86_avx512.cpp:47-109): scores = dot(q, k_j) * scale for the
-// visible keys (causal: keys 0 .. past + t), full-row softmax (max, exp, sum, times 1/sum),
-// then out = sum_j p_j * v_j accumulated key by key in ascending order with one fused
-// multiply-add per key and feature, as the reference's loop does.  One block per (token,
-// head).  Scores: a warp per key, four keys' loads in flight at a time.  P*V: thread d owns
-// output feature d and walks the keys in order; the value rows come through shared memory in
-// chunks that all threads fetch together, the next chunk's loads in flight while the current
-// one is consumed, so that the ordered sum does not wait on memory once per key.
+// operator (kernels/attention_x86_avx512.cpp:47-109): scores = dot(q, k_j) * scale for the
+// visible keys (causal: keys 0 .. past + t), softmax, then out = sum_j p_j * v_j in ascending
+// key order with one fused multiply-add per key and feature; a probability of zero
+// contributes nothing.  The softmax runs over blocks of kTileKeys keys in order (running
+// maximum m and sum l, earlier terms scaled by exp(m_old - m_new) when m moves), one division
+// at the end.  One block per (token, head), any head size: the form that serves what the two
+// kernels below do not take.  Its arithmetic is attention_tile_kernel's, operation for
+// operation: a dot product is summed per 32 features (even and odd ones apart), the parts in
+// order; a block's probabilities add up in an xor-tree.  Keys and values come through shared
+// memory in chunks that all threads fetch together, the next chunk's loads in flight while
+// the current one is consumed.
 constexpr int kAttnThreads = 256;
 constexpr int kAttnWarps = kAttnThreads / 32;
-constexpr int kAttnStage = 4096;                       // floats of V per chunk
+constexpr int kAttnStage = 4096;                       // floats of K or V per chunk
 constexpr int kAttnPerThread = kAttnStage / kAttnThreads;
+constexpr int kAttnStagePad = kAttnStage + kAttnStage / 32 + kAttnStage / 8;  // skewed keys
+constexpr int kTileKeys = 32;                          // keys per softmax block
+
+// running maximum over a further block of scores, and the factor for what is summed so far
+__device__ __forceinline__ float attn_rescale(float m_old, float m_new) {
+    return m_new == -INFINITY ? 1.f : (float)exp((double)__fsub_rn(m_old, m_new));
+}
+// exp(s - m); m = -inf: no score above -inf yet, every term is zero
+__device__ __forceinline__ float attn_prob(float s, float m) {
+    return (float)exp((double)__fsub_rn(s, m == -INFINITY ? 0.f : m));
+}
+
 __global__ void __launch_bounds__(kAttnThreads)
 attention_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                  const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
@@ -306,90 +321,138 @@ attention_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
     b2w4_pdl_chain_entry();
     const int past = past_dev ? min(*past_dev, capacity - tokens) : past0;
     extern __shared__ float s_dyn[];
-    float* s_scores = s_dyn;                // [score_slots] >= visible keys
-    float* s_stage = s_dyn + score_slots;   // [kAttnStage]
-    __shared__ float s_part[kAttnWarps];
+    float* s_scores = s_dyn;                            // [score_slots] >= visible keys
+    float* s_stage = s_scores + score_slots;            // [kAttnStagePad]
+    float* s_alpha = s_stage + kAttnStagePad;           // [blocks]: factor before block b
+    __shared__ float s_total;
     const int t = blockIdx.x / heads, h = blockIdx.x % heads;
     const int kvh = h / (heads / kv_heads);
-    const int visible = past + t + 1;
+    const int visible = past + t + 1, blocks = (visible + kTileKeys - 1) / kTileKeys;
     const float* qr = q + ((size_t)t * heads + h) * dim;
     const float* kc = k_cache + (size_t)kvh * capacity * dim;
     const float* vc = v_cache + (size_t)kvh * capacity * dim;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-    constexpr int kQ = kAttnMaxDim / 32, kKeys = 4;
-    float qv[kQ];
-#pragma unroll
-    for (int i = 0; i < kQ; ++i)
-        qv[i] = lane + 32 * i < dim ? qr[lane + 32 * i] : 0.f;
-    for (int j0 = warp * kKeys; j0 < visible; j0 += kAttnWarps * kKeys) {
-        float kv[kKeys][kQ];
-#pragma unroll
-        for (int u = 0; u < kKeys; ++u)
-#pragma unroll
-            for (int i = 0; i < kQ; ++i)
-                kv[u][i] = (j0 + u < visible && lane + 32 * i < dim)
-                               ? kc[(size_t)(j0 + u) * dim + lane + 32 * i] : 0.f;
-#pragma unroll
-        for (int u = 0; u < kKeys; ++u) {
-            float p = 0.f;
-#pragma unroll
-            for (int i = 0; i < kQ; ++i)
-                if (32 * i < dim)  // lanes past the last feature add +0 products
-                    p = __fmaf_rn(qv[i], kv[u][i], p);
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-                p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, off));
-            if (lane == 0 && j0 + u < visible)
-                s_scores[j0 + u] = __fmul_rn(p, scale);
-        }
-    }
-    __syncthreads();
-    float m = -INFINITY;
-    for (int j = threadIdx.x; j < visible; j += blockDim.x)
-        m = fmaxf(m, s_scores[j]);
-    m = block_max(m, s_part);
-    float sum = 0.f;
-    for (int j = threadIdx.x; j < visible; j += blockDim.x) {
-        const float e = (float)exp((double)__fsub_rn(s_scores[j], m));
-        s_scores[j] = e;
-        sum = __fadd_rn(sum, e);
-    }
-    sum = block_sum(sum, s_part);
-    const float inv = __fdiv_rn(1.f, sum);
-
     const int chunk = kAttnStage / dim;  // keys per chunk
     float r[kAttnPerThread];
-    auto fetch = [&](int j0) {
+    auto fetch = [&](const float* base, int j0) {
         const int n = min(chunk, visible - j0) * dim;
-        const float* src = vc + (size_t)j0 * dim;
+        const float* src = base + (size_t)j0 * dim;
 #pragma unroll
         for (int u = 0; u < kAttnPerThread; ++u) {
             const int i = threadIdx.x + kAttnThreads * u;
             r[u] = i < n ? src[i] : 0.f;
         }
     };
-    fetch(0);
+
+    // ---- scores: `parts` lanes per key, a lane per 32 features ----
+    const int parts = dim <= 32 ? 1 : dim <= 64 ? 2 : dim <= 128 ? 4 : 8;
+    const int part = lane % parts, sub = lane / parts, keys_warp = 32 / parts;
+    // a part starts 33 floats after the one before it, so that parts and keys spread over banks
+    const int pitch = dim <= 32 ? dim : dim + (dim + 31) / 32;
+    float qv[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+        qv[i] = part * 32 + i < dim ? qr[part * 32 + i] : 0.f;
+    fetch(kc, 0);
+    for (int j0 = 0; j0 < visible; j0 += chunk) {
+        __syncthreads();  // the previous chunk has been consumed
+#pragma unroll
+        for (int u = 0; u < kAttnPerThread; ++u) {
+            const int i = threadIdx.x + kAttnThreads * u, key = i / dim, d = i - key * dim;
+            if (key < chunk)
+                s_stage[key * pitch + d + (d >> 5)] = r[u];
+        }
+        __syncthreads();
+        if (j0 + chunk < visible)
+            fetch(kc, j0 + chunk);
+        const int nk = min(chunk, visible - j0);
+        for (int k0 = warp * keys_warp; k0 < nk; k0 += kAttnWarps * keys_warp) {
+            const int key = k0 + sub;
+            const float* kr = s_stage + min(key, nk - 1) * pitch + part * 33;
+            float even = 0.f, odd = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+                if (part * 32 + i < dim)
+                    even = __fmaf_rn(qv[i], kr[i], even);
+                if (part * 32 + i + 1 < dim)
+                    odd = __fmaf_rn(qv[i + 1], kr[i + 1], odd);
+            }
+            const float p = __fadd_rn(even, odd);
+            float s = 0.f;
+            for (int c = 0; c < parts; ++c)
+                s = __fadd_rn(s, __shfl_sync(0xffffffffu, p, sub * parts + c));
+            if (part == 0 && key < nk)
+                s_scores[j0 + key] = __fmul_rn(s, scale);
+        }
+    }
+    __syncthreads();
+    fetch(vc, 0);
+
+    // ---- softmax: block maxima, their running maximum, probabilities and block sums ----
+    float* s_max = s_stage;            // [blocks] running maximum (the stage is free here)
+    float* s_sum = s_alpha + blocks;   // [blocks]
+    for (int b = warp; b < blocks; b += kAttnWarps) {
+        const int j = b * kTileKeys + lane;
+        float m = j < visible ? s_scores[j] : -INFINITY;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+        if (lane == 0)
+            s_max[b] = fmaxf(m, -INFINITY);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float m = -INFINITY;
+        for (int b = 0; b < blocks; ++b)
+            s_max[b] = m = fmaxf(m, s_max[b]);
+    }
+    __syncthreads();
+    for (int b = warp; b < blocks; b += kAttnWarps) {
+        const int j = b * kTileKeys + lane;
+        const float m = s_max[b];
+        float e = 0.f;
+        if (j < visible)
+            s_scores[j] = e = attn_prob(s_scores[j], m);
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+            e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, off));
+        if (lane == 0) {
+            s_sum[b] = e;
+            s_alpha[b] = b ? attn_rescale(s_max[b - 1], m) : 1.f;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float l = 0.f;
+        for (int b = 0; b < blocks; ++b)
+            l = __fadd_rn(__fmul_rn(l, s_alpha[b]), s_sum[b]);
+        s_total = l;
+    }
+
     float acc = 0.f;
     for (int j0 = 0; j0 < visible; j0 += chunk) {
-        __syncthreads();  // the previous chunk has been consumed (and the scores are final)
+        __syncthreads();  // the previous chunk has been consumed (and the sums are final)
 #pragma unroll
         for (int u = 0; u < kAttnPerThread; ++u)
             s_stage[threadIdx.x + kAttnThreads * u] = r[u];
         __syncthreads();
         if (j0 + chunk < visible)
-            fetch(j0 + chunk);
+            fetch(vc, j0 + chunk);
         if (threadIdx.x < dim) {
             const int nk = min(chunk, visible - j0);
             for (int j = 0; j < nk; ++j) {
-                const float p = __fmul_rn(s_scores[j0 + j], inv);
+                if ((j0 + j) % kTileKeys == 0) {
+                    const float al = s_alpha[(j0 + j) / kTileKeys];
+                    acc = al == 0.f ? 0.f : __fmul_rn(acc, al);
+                }
+                const float p = s_scores[j0 + j];
                 if (p != 0.f)
                     acc = __fmaf_rn(s_stage[j * dim + threadIdx.x], p, acc);
             }
         }
     }
     if (threadIdx.x < dim)
-        out[((size_t)t * heads + h) * dim + threadIdx.x] = acc;
+        out[((size_t)t * heads + h) * dim + threadIdx.x] = __fdiv_rn(acc, s_total);
 }
 
 // The same attention for a few query tokens (a decode step): a cluster of kSplitCtas blocks
@@ -681,189 +744,289 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
 
 // The same attention for a run of new tokens (prefill): one block per (kv head, tile of query
 // tokens) serves every query head of that kv head -- up to kTileRows (token, head) rows --
-// so that a chunk of keys or values is fetched into shared memory once per tile instead of
-// once per row.  Every row's arithmetic is attention_kernel's, operation for operation (the
-// lanes' partial dot products and their xor-tree, the softmax sums per 256 strided partials,
-// the ordered P*V), so both kernels give the same bits.
-//   scores   warp w owns rows 4w .. 4w+3.  For eight keys at a time it forms the 32 partial
-//            products (4 rows x 8 keys) per lane, then a butterfly exchange that halves the
-//            items a lane holds at each of the xor-tree's five levels -- the same sums in the
-//            same order as five shuffles per item, for one shuffle per item
-//   softmax  per row by its warp; probabilities e_j / sum are stored back, zero past the
-//            row's last visible key
-//   P*V      thread (group, d): feature d of DIM/8 rows, keys in ascending order
-constexpr int kTileRows = 32;
+// against blocks of kTileKeys keys, with the running softmax of attention_kernel and its
+// arithmetic operation for operation, so both give the same bits.  Nothing grows with the
+// number of keys: any context length takes this form.
+// What bounds it: the fp32 multiply-adds of the two products (2 * keys * rows * DIM a tile),
+// issued two lanes at a time (fma.rn.f32x2); scores and probabilities stay in 32 bits, which
+// is why the products are not on the tensor cores.  Two blocks per SM, so that one block's
+// softmax (exp in 64 bits) and barriers run under the other's products.
+//   scores   thread = 4 rows x 2 keys, 16 bytes of features at a time: six shared loads, all
+//            free of bank conflicts (pitch DIM + 4), for sixteen paired multiply-adds
+//   softmax  four threads per row, eight keys each
+//   P*V      thread = 4 rows x DIM / 16 features, keys in ascending order
+// K of block b + 1 is copied (cp.async) under the softmax and P*V of block b, V of block b
+// under its scores.  A value row that is not finite must not reach a row that does not see it
+// (0 * inf): the copying threads look at what they fetched, and a block that holds such a
+// value runs P*V with the zero probabilities skipped.
+// Measured, eight layers of a prompt with 32 / 8 heads of 128 (all operators): 1500 tokens
+// 51.6 -> 18.8 ms (scores of that many keys did not fit the former tile kernel, and a block
+// per (token, head) read 37 GB of keys and values per layer); 256 tokens 3.47 -> 3.39 ms.
+constexpr int kTileRows = 64;
 template <int DIM>
-__global__ void __launch_bounds__(kAttnThreads)
+struct TileSmem {  // floats
+    static constexpr int kPitch = DIM + 4, kProbPitch = kTileKeys + 4;
+    static constexpr int kQ = 0;
+    static constexpr int kK = kQ + kTileRows * kPitch;
+    static constexpr int kV = kK + kTileKeys * kPitch;
+    static constexpr int kP = kV + kTileKeys * kPitch;
+    static constexpr int kAlpha = kP + kTileRows * kProbPitch;
+    static constexpr int kSum = kAlpha + kTileRows;
+    static constexpr int kBytes = (kSum + kTileRows) * 4;
+};
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kAttnThreads, DIM > 128 ? 1 : 2)
 attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                       const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
                       int heads, int kv_heads, int past0, const int* __restrict__ past_dev,
-                      int capacity, float scale, int slots, int tq) {
+                      int capacity, float scale, int tq) {
     b2w4_pdl_chain_entry();
     const int past = past_dev ? min(*past_dev, capacity - tokens) : past0;
-    extern __shared__ float s_dyn[];
-    float* s_sc = s_dyn;                           // [kTileRows][slots]
-    float* s_stage = s_dyn + kTileRows * slots;    // [kAttnStage]
-    constexpr int kQ = DIM / 32;                   // features per lane
-    constexpr int kChunk = kAttnStage / DIM;       // keys per staged chunk
+    using S = TileSmem<DIM>;
+    constexpr int P = S::kPitch, PP = S::kProbPitch;
+    extern __shared__ __align__(16) float s_dyn[];
+    float* s_q = s_dyn + S::kQ;
+    float* s_k = s_dyn + S::kK;
+    float* s_v = s_dyn + S::kV;
+    float* s_p = s_dyn + S::kP;
+    float* s_alpha = s_dyn + S::kAlpha;
+    float* s_sum = s_dyn + S::kSum;
     const int rep = heads / kv_heads;
     // the last tiles see the most keys: they go first
     const int kvh = blockIdx.y, t0 = (int)(gridDim.x - 1 - blockIdx.x) * tq;
-    const int t_end = min(t0 + tq, tokens);
-    const int vis_max = past + t_end;              // keys the tile's last token sees
+    const int vis_max = past + min(t0 + tq, tokens);  // keys the tile's last token sees
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float* kc = k_cache + (size_t)kvh * capacity * DIM;
     const float* vc = v_cache + (size_t)kvh * capacity * DIM;
     // row r of the tile: token t0 + r / rep, head kvh * rep + r % rep; rows past the tile's
     // tokens see no key
-    auto row_token = [&](int r) { return t0 + r / rep; };
     auto row_visible = [&](int r) {
-        return (r < tq * rep && row_token(r) < tokens) ? past + row_token(r) + 1 : 0;
+        return (r < tq * rep && t0 + r / rep < tokens) ? past + t0 + r / rep + 1 : 0;
     };
-
-    float r[kAttnPerThread];
-    auto fetch = [&](const float* base, int j0) {
-        const int n = min(kChunk, vis_max - j0) * DIM;
-        const float* src = base + (size_t)j0 * DIM;
+    auto row_offset = [&](int r) {
+        return ((size_t)(t0 + r / rep) * heads + kvh * rep + r % rep) * DIM;
+    };
+    constexpr int kRow4 = DIM / 4;                            // float4 per row
+    constexpr int kCopies = kTileKeys * kRow4 / kAttnThreads;  // per thread and block of keys
+    auto copy_keys = [&](float* dst, const float* base, int j0) {
 #pragma unroll
-        for (int u = 0; u < kAttnPerThread; ++u) {
-            const int i = threadIdx.x + kAttnThreads * u;
-            r[u] = i < n ? src[i] : 0.f;
+        for (int u = 0; u < kCopies; ++u) {
+            const int i = threadIdx.x + kAttnThreads * u, key = i / kRow4, c = i % kRow4;
+            const bool valid = j0 + key < vis_max;
+            cp_async16(dst + key * P + 4 * c, base + (size_t)(valid ? j0 + key : 0) * DIM + 4 * c,
+                       valid);
         }
+        cp_async_commit();
     };
-    auto stage = [&]() {
-        __syncthreads();  // the previous chunk has been consumed
-#pragma unroll
-        for (int u = 0; u < kAttnPerThread; ++u)
-            s_stage[threadIdx.x + kAttnThreads * u] = r[u];
-        __syncthreads();
-    };
-
-    // ---- scores ----
-    float qv[4][kQ];
-    int vis[4], vis_warp = 0;
-#pragma unroll
-    for (int rr = 0; rr < 4; ++rr) {
-        const int row = warp * 4 + rr;
-        vis[rr] = row_visible(row);
-        vis_warp = max(vis_warp, vis[rr]);
-        const float* qr = q + ((size_t)row_token(row) * heads + kvh * rep + row % rep) * DIM;
-#pragma unroll
-        for (int i = 0; i < kQ; ++i)
-            qv[rr][i] = vis[rr] ? qr[lane + 32 * i] : 0.f;
+    for (int i = threadIdx.x; i < kTileRows * kRow4; i += kAttnThreads) {
+        const int row = i / kRow4, c = i % kRow4;
+        const bool live = row_visible(row) > 0;
+        cp_async16(s_q + row * P + 4 * c, q + (live ? row_offset(row) : 0) + 4 * c, live);
     }
-    fetch(kc, 0);
-    for (int j0 = 0; j0 < vis_max; j0 += kChunk) {
-        stage();
-        if (j0 + kChunk < vis_max)
-            fetch(kc, j0 + kChunk);
-        for (int sub = 0; sub < kChunk / 8 && j0 + sub * 8 < vis_warp; ++sub) {
-            float v[32];  // item rr * 8 + kk: row rr of the warp, key kk of the eight
+    copy_keys(s_k, kc, 0);  // Q and the first keys: one group
+
+    // products: rows r_of(i) = ra + 16 i, keys kb + 16 j, features 4 kb + 64 i .. + 3
+    const int ra = (warp >> 1) * 4 + (lane >> 3), kb = (warp & 1) * 8 + (lane & 7);
+    // softmax: row sr, keys 8 sq .. 8 sq + 7 of a block
+    const int sr = threadIdx.x >> 2, sq = threadIdx.x & 3;
+    const int s_vis = row_visible(sr);
+    float m = -INFINITY, l = 0.f;
+    constexpr int NV = DIM / 64;
+    uint64_t acc[4][2 * NV];
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                float kr[kQ];
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int i = 0; i < kQ; ++i)
-                    kr[i] = s_stage[(sub * 8 + kk) * DIM + lane + 32 * i];
+        for (int c = 0; c < 2 * NV; ++c)
+            acc[i][c] = 0;
+
+    for (int j0 = 0; j0 < vis_max; j0 += kTileKeys) {
+        copy_keys(s_v, vc, j0);
+        cp_async_wait<1>();
+        __syncthreads();  // K of this block is in place
+        {
+            float sc[4][2];
 #pragma unroll
-                for (int rr = 0; rr < 4; ++rr) {
-                    float p = 0.f;
+            for (int i = 0; i < 4; ++i)
+                sc[i][0] = sc[i][1] = 0.f;
+#pragma unroll 1
+            for (int c = 0; c < DIM; c += 32) {
+                uint64_t a[4][2];
 #pragma unroll
-                    for (int i = 0; i < kQ; ++i)
-                        p = __fmaf_rn(qv[rr][i], kr[i], p);
-                    v[rr * 8 + kk] = p;
+                for (int i = 0; i < 4; ++i)
+                    a[i][0] = a[i][1] = 0;
+#pragma unroll
+                for (int d = 0; d < 32; d += 4) {
+                    ulonglong2 qv[4], kv[2];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        qv[i] = *reinterpret_cast<const ulonglong2*>(s_q + (ra + 16 * i) * P + c + d);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        kv[j] = *reinterpret_cast<const ulonglong2*>(s_k + (kb + 16 * j) * P + c + d);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j)
+                            a[i][j] = b2w4_fma2(qv[i].x, kv[j].x, a[i][j]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j)
+                            a[i][j] = b2w4_fma2(qv[i].y, kv[j].y, a[i][j]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        float lo, hi;
+                        b2w4_unpack2(a[i][j], lo, hi);
+                        sc[i][j] = __fadd_rn(sc[i][j], __fadd_rn(lo, hi));
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    s_p[(ra + 16 * i) * PP + kb + 16 * j] = __fmul_rn(sc[i][j], scale);
+        }
+        __syncthreads();  // scores in place, K consumed
+        if (j0 + kTileKeys < vis_max)
+            copy_keys(s_k, kc, j0 + kTileKeys);
+        else
+            cp_async_commit();  // an empty group keeps the count
+        {
+            float* row = s_p + sr * PP + 8 * sq;
+            float e[8];
+            *reinterpret_cast<float4*>(e) = *reinterpret_cast<const float4*>(row);
+            *reinterpret_cast<float4*>(e + 4) = *reinterpret_cast<const float4*>(row + 4);
+            float mb = m;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (j0 + 8 * sq + i < s_vis)
+                    mb = fmaxf(mb, e[i]);
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
+            const float alpha = j0 ? attn_rescale(m, mb) : 1.f;
+            m = mb;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                e[i] = j0 + 8 * sq + i < s_vis ? attn_prob(e[i], m) : 0.f;
+            *reinterpret_cast<float4*>(row) = *reinterpret_cast<const float4*>(e);
+            *reinterpret_cast<float4*>(row + 4) = *reinterpret_cast<const float4*>(e + 4);
+            float sum = __fadd_rn(__fadd_rn(__fadd_rn(e[0], e[1]), __fadd_rn(e[2], e[3])),
+                                  __fadd_rn(__fadd_rn(e[4], e[5]), __fadd_rn(e[6], e[7])));
+            sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 1));
+            sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 2));
+            l = __fadd_rn(__fmul_rn(l, alpha), sum);
+            if (sq == 0)
+                s_alpha[sr] = alpha;
+        }
+        cp_async_wait<1>();  // V of this block
+        bool odd_value = false;
+#pragma unroll
+        for (int u = 0; u < kCopies; ++u) {
+            const int i = threadIdx.x + kAttnThreads * u, key = i / kRow4, c = i % kRow4;
+            const float4 x = *reinterpret_cast<const float4*>(s_v + key * P + 4 * c);
+            // inf and NaN, times zero, are NaN
+            const float z = __fadd_rn(__fadd_rn(__fmul_rn(x.x, 0.f), __fmul_rn(x.y, 0.f)),
+                                      __fadd_rn(__fmul_rn(x.z, 0.f), __fmul_rn(x.w, 0.f)));
+            odd_value |= z != 0.f;
+        }
+        const bool careful = __syncthreads_or(odd_value);  // V, probabilities, factors in place
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float al = s_alpha[ra + 16 * i];
+            if (al != 1.f) {
+                const uint64_t al2 = b2w4_pack2(al, al);
+#pragma unroll
+                for (int c = 0; c < 2 * NV; ++c)
+                    acc[i][c] = al == 0.f ? 0 : b2w4_mul2(acc[i][c], al2);
+            }
+        }
+        if (!careful) {
+#pragma unroll 2
+            for (int j = 0; j < kTileKeys; j += 4) {
+                float4 p4[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    p4[i] = *reinterpret_cast<const float4*>(s_p + (ra + 16 * i) * PP + j);
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) {
+                    ulonglong2 v[NV];
+#pragma unroll
+                    for (int c = 0; c < NV; ++c)
+                        v[c] = *reinterpret_cast<const ulonglong2*>(s_v + (j + jj) * P + 4 * kb +
+                                                                    64 * c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float p = jj == 0 ? p4[i].x : jj == 1 ? p4[i].y
+                                      : jj == 2 ? p4[i].z : p4[i].w;
+                        const uint64_t pp = b2w4_pack2(p, p);
+#pragma unroll
+                        for (int c = 0; c < NV; ++c) {
+                            acc[i][2 * c] = b2w4_fma2(v[c].x, pp, acc[i][2 * c]);
+                            acc[i][2 * c + 1] = b2w4_fma2(v[c].y, pp, acc[i][2 * c + 1]);
+                        }
+                    }
                 }
             }
-            // xor-tree levels 16, 8, 4, 2, 1; after level `off` a lane keeps the half of its
-            // items selected by that bit of its index, so it ends with item `lane`
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < kTileKeys; ++j) {
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const bool up = lane & off;
+                for (int i = 0; i < 4; ++i) {
+                    const float p = s_p[(ra + 16 * i) * PP + j];
+                    if (p != 0.f) {
+                        const uint64_t pp = b2w4_pack2(p, p);
 #pragma unroll
-                for (int i = 0; i < off; ++i) {
-                    const float send = up ? v[i] : v[i + off];
-                    const float keep = up ? v[i + off] : v[i];
-                    v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, off));
+                        for (int c = 0; c < NV; ++c) {
+                            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(
+                                s_v + j * P + 4 * kb + 64 * c);
+                            acc[i][2 * c] = b2w4_fma2(v.x, pp, acc[i][2 * c]);
+                            acc[i][2 * c + 1] = b2w4_fma2(v.y, pp, acc[i][2 * c + 1]);
+                        }
+                    }
                 }
             }
-            const int rr = lane >> 3, key = j0 + sub * 8 + (lane & 7);
-            int my_vis = vis[0];
-            my_vis = rr == 1 ? vis[1] : my_vis;
-            my_vis = rr == 2 ? vis[2] : my_vis;
-            my_vis = rr == 3 ? vis[3] : my_vis;
-            if (key < my_vis)
-                s_sc[(warp * 4 + rr) * slots + key] = __fmul_rn(v[0], scale);
         }
+        __syncthreads();  // V and the probabilities are consumed
     }
-    __syncwarp();
-
-    // ---- softmax, a row at a time by the warp that owns it ----
-#pragma unroll 1
-    for (int rr = 0; rr < 4; ++rr) {
-        float* sc = s_sc + (warp * 4 + rr) * slots;
-        const int n = vis[rr];
-        float m = -INFINITY;
-        for (int j = lane; j < n; j += 32)
-            m = fmaxf(m, sc[j]);
+    if (sq == 0)
+        s_sum[sr] = l;
+    __syncthreads();
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-        // the sum of attention_kernel: 256 partials of stride 256, a tree per 32 of them,
-        // the eight results added in order
-        float sum = 0.f;
-#pragma unroll 1
-        for (int w = 0; w < kAttnWarps; ++w) {
-            float part = 0.f;
-            for (int j = w * 32 + lane; j < n; j += kAttnThreads) {
-                const float e = (float)exp((double)__fsub_rn(sc[j], m));
-                sc[j] = e;
-                part = __fadd_rn(part, e);
-            }
+    for (int i = 0; i < 4; ++i) {
+        const int row = ra + 16 * i;
+        if (row_visible(row)) {
+            const float total = s_sum[row];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-                part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, off));
-            sum = __fadd_rn(sum, part);
-        }
-        const float inv = __fdiv_rn(1.f, sum);
-        for (int j = lane; j < ((vis_max + 3) & ~3); j += 32)  // P*V reads four at a time
-            sc[j] = j < n ? __fmul_rn(sc[j], inv) : 0.f;
-    }
-
-    // ---- P*V ----
-    constexpr int kGroups = kAttnThreads / DIM, kRG = kTileRows / kGroups;
-    const int grp = threadIdx.x / DIM, d = threadIdx.x % DIM;
-    float acc[kRG];
-#pragma unroll
-    for (int i = 0; i < kRG; ++i)
-        acc[i] = 0.f;
-    fetch(vc, 0);
-    for (int j0 = 0; j0 < vis_max; j0 += kChunk) {
-        stage();  // its first barrier also orders the probabilities before their use
-        if (j0 + kChunk < vis_max)
-            fetch(vc, j0 + kChunk);
-        const int nk = min(kChunk, vis_max - j0);
-        const float* pr = s_sc + grp * kRG * slots + j0;
-        // four keys at a time; a zero probability leaves the sum as it is (values are
-        // finite), which is what attention_kernel's skip does
-        for (int j = 0; j < nk; j += 4) {
-            const float v0 = s_stage[j * DIM + d], v1 = s_stage[(j + 1) * DIM + d];
-            const float v2 = s_stage[(j + 2) * DIM + d], v3 = s_stage[(j + 3) * DIM + d];
-#pragma unroll
-            for (int i = 0; i < kRG; ++i) {
-                const float4 p = *reinterpret_cast<const float4*>(pr + i * slots + j);
-                acc[i] = __fmaf_rn(v0, p.x, acc[i]);
-                acc[i] = __fmaf_rn(v1, p.y, acc[i]);
-                acc[i] = __fmaf_rn(v2, p.z, acc[i]);
-                acc[i] = __fmaf_rn(v3, p.w, acc[i]);
+            for (int c = 0; c < NV; ++c) {
+                float4 o;
+                b2w4_unpack2(acc[i][2 * c], o.x, o.y);
+                b2w4_unpack2(acc[i][2 * c + 1], o.z, o.w);
+                o.x = __fdiv_rn(o.x, total);
+                o.y = __fdiv_rn(o.y, total);
+                o.z = __fdiv_rn(o.z, total);
+                o.w = __fdiv_rn(o.w, total);
+                *reinterpret_cast<float4*>(out + row_offset(row) + 4 * kb + 64 * c) = o;
             }
         }
     }
-#pragma unroll
-    for (int i = 0; i < kRG; ++i) {
-        const int row = grp * kRG + i;
-        if (row_visible(row))
-            out[((size_t)row_token(row) * heads + kvh * rep + row % rep) * DIM + d] = acc[i];
-    }
+    cp_async_wait<0>();
 }
 
 // A position counter on the device: *counter += by (after a decode step of a replayed graph),
@@ -1006,14 +1169,17 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
     const int keys = past_dev ? capacity : past + tokens;  // position on the device: sized
                                                            // for a full cache
     const int rep = heads / kv_heads;
-    // a run of tokens takes the tile kernel while a tile's scores fit in shared memory
-    const int tile_slots = ((keys + 31) & ~31) + 8;  // rows 8 banks apart
-    const size_t tile_smem = sizeof(float) * ((size_t)kTileRows * tile_slots + kAttnStage);
-    const bool tiles = tokens >= 8 && ctx->attn_tiles && rep <= kTileRows &&
-                       (dim == 64 || dim == 128 || dim == 256) && tile_smem <= 200 * 1024;
+    // Head sizes of 64, 128 and 256 with 16-byte aligned rows: up to seven query tokens go to
+    // the cluster kernel (it splits the keys, so few rows still fill the chip), a run of eight
+    // or more to the tile kernel (it shares keys and values among 64 rows).  The rest: one
+    // block per (token, head).
+    const bool wide = (dim == 64 || dim == 128 || dim == 256) &&
+                      !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev |
+                         (uintptr_t)out_dev) & 15);
+    const bool split = wide && tokens < 8;
+    const bool tiles = wide && !split && ctx->attn_tiles && rep <= kTileRows;
     const int score_slots = (keys + 3) & ~3;
-    const size_t row_smem = sizeof(float) * ((size_t)score_slots + kAttnStage);
-    if (!tiles && row_smem > 200 * 1024)
+    if (sizeof(float) * ((size_t)score_slots + kAttnStage) > 200 * 1024)
         return b2w4_fail(ctx, B2W4_E_INVALID, "attention: %d keys exceed the score buffer", keys);
     if (append) {
         const size_t n = (size_t)tokens * kv_heads * dim;
@@ -1025,8 +1191,7 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
     }
     const float* kc = k_cache_dev;
     const float* vc = v_cache_dev;
-    const bool aligned = !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev) & 15);
-    if (tokens < 8 && aligned && (dim == 64 || dim == 128 || dim == 256)) {
+    if (split) {
         const int per = (keys + kSplitCtas - 1) / kSplitCtas;
 #define B2W4_SPLIT(D, HR)                                                                      \
     do {                                                                                       \
@@ -1068,11 +1233,12 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
 #define B2W4_TILE(D)                                                                          \
     do {                                                                                      \
         static b2w4_smem_optin cfg;                                                           \
-        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, attention_tile_kernel<D>, tile_smem, cfg));      \
+        const size_t smem = TileSmem<D>::kBytes;                                              \
+        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, attention_tile_kernel<D>, smem, cfg));           \
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, attention_tile_kernel<D>, grid,          \
-                                           dim3(kAttnThreads), tile_smem, ctx->stream, q_dev, \
-                                           kc, vc, out_dev, tokens, heads, kv_heads, past,    \
-                                           past_dev, capacity, scale, tile_slots, tq));       \
+                                           dim3(kAttnThreads), smem, ctx->stream, q_dev, kc,  \
+                                           vc, out_dev, tokens, heads, kv_heads, past,        \
+                                           past_dev, capacity, scale, tq));                   \
     } while (0)
         if (dim == 64)
             B2W4_TILE(64);
@@ -1083,6 +1249,8 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
 #undef B2W4_TILE
     } else {
         static b2w4_smem_optin configured;
+        const size_t row_smem = sizeof(float) * ((size_t)score_slots + kAttnStagePad +
+                                                 2 * ((keys + kTileKeys - 1) / kTileKeys));
         B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, attention_kernel, row_smem, configured));
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, attention_kernel, dim3(tokens * heads),
                                            dim3(kAttnThreads), row_smem, ctx->stream, q_dev, kc,

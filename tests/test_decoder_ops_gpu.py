@@ -308,3 +308,34 @@ def test_split_attention_of_a_few_tokens(ctx, tokens, past, heads, kv_heads, dim
         assert outs[1].tobytes() == outs[0].tobytes()
         assert rel_l2(outs[0], _attention_fp64(q, k_all, v_all, heads, kv_heads, past,
                                                scale)) < 1e-5
+
+
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [
+    (8, 0, 64, 1, 64), (9, 1600, 8, 2, 128), (31, 33, 3, 1, 128), (70, 0, 5, 5, 256),
+    (2, 70, 4, 2, 80), (1, 300, 3, 3, 20), (12, 40, 2, 1, 96), (9, 3, 65, 1, 64)])
+def test_tile_and_row_attention(ctx, tokens, past, heads, kv_heads, dim):
+    """Runs of eight or more tokens (tile kernel: several softmax blocks, head groups that do
+    not fill a tile, more keys than a block's scores would hold) and the shapes that only the
+    one-row kernel takes (other head sizes, more heads per kv head than a tile has rows),
+    against 64 bits; tolerance as for the split kernel.  Value rows past the last position are
+    NaN, and so is the last token's: the earlier tokens do not see them."""
+    import torch
+    capacity, scale = past + tokens + 40, dim ** -0.5
+    rng = np.random.default_rng(past + dim)
+    q = rng.normal(0, 1, (tokens, heads, dim)).astype(np.float32)
+    k_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    v_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    v_all[-1] = np.nan
+    kc = np.zeros((kv_heads, capacity, dim), dtype=np.float32)
+    vc = np.full((kv_heads, capacity, dim), np.nan, dtype=np.float32)
+    kc[:, :past + tokens] = k_all.transpose(1, 0, 2)
+    vc[:, :past + tokens] = v_all.transpose(1, 0, 2)
+    out = torch.zeros((tokens, heads, dim), dtype=torch.float32, device="cuda")
+    ctx.attention(_dev(q), None, None, _dev(kc), _dev(vc), out, tokens, heads, kv_heads, dim,
+                  past, capacity, scale)
+    ctx.sync()
+    got = out.cpu().numpy()
+    assert np.isnan(got[-1]).all()
+    if tokens > 1:
+        want = _attention_fp64(q, k_all, v_all, heads, kv_heads, past, scale)
+        assert rel_l2(got[:-1], want[:-1]) < 1e-5
