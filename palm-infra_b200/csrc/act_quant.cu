@@ -65,6 +65,7 @@ template <bool A32>
 __global__ void quantize_rows_umma_kernel(const float* __restrict__ x, int lda, int m, int k,
                                           int m_pad, int8_t* __restrict__ q,
                                           float* __restrict__ scales) {
+    b2w4_pdl_chain_entry();
     const int groups = k >> 7;
     long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -72,7 +73,19 @@ __global__ void quantize_rows_umma_kernel(const float* __restrict__ x, int lda, 
         return;
     const int row = (int)(wid / groups), g = (int)(wid % groups);
     const float* src = x + (size_t)row * lda + (size_t)g * 128 + lane * 4;
-    float v0 = src[0], v1 = src[1], v2 = src[2], v3 = src[3];
+    float v0, v1, v2, v3;
+    if (((reinterpret_cast<uintptr_t>(x) & 15) | (lda & 3)) == 0) {
+        const float4 v = *reinterpret_cast<const float4*>(src);
+        v0 = v.x;
+        v1 = v.y;
+        v2 = v.z;
+        v3 = v.w;
+    } else {
+        v0 = src[0];
+        v1 = src[1];
+        v2 = src[2];
+        v3 = src[3];
+    }
     float amax = fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3)));
     // per 128 values: all 32 lanes; per 32 values: the 8 lanes of a 32-block
 #pragma unroll
@@ -107,7 +120,7 @@ __global__ void quantize_rows_mma_kernel(const float* __restrict__ x, int lda, i
                                          int m_pad, int8_t* __restrict__ q,
                                          float* __restrict__ scales_t,
                                          int32_t* __restrict__ es_t) {
-    b2w4_pdl_launch_dependents();  // the GEMM behind may start fetching its weights
+    b2w4_pdl_chain_entry();  // the GEMM behind may start fetching its weights
     const int groups = k >> 7;
     long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -155,13 +168,14 @@ int b2w4_launch_quantize_mma(b2w4_ctx* ctx, const float* x, int lda, int m, int 
     long long warps = (long long)m * (k / 128);
     int grid = (int)((warps * 32 + 255) / 256);
     if (act_rule == B2W4_ACT_G32)
-        quantize_rows_mma_kernel<true><<<grid, 256, 0, ctx->stream>>>(x, lda, m, k, m_pad, q,
-                                                                      scales_t, es_t);
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, quantize_rows_mma_kernel<true>, dim3(grid),
+                                           dim3(256), 0, ctx->stream, x, lda, m, k, m_pad, q,
+                                           scales_t, es_t));
     else
-        quantize_rows_mma_kernel<false><<<grid, 256, 0, ctx->stream>>>(x, lda, m, k, m_pad, q,
-                                                                       scales_t, es_t);
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, quantize_rows_mma_kernel<false>, dim3(grid),
+                                           dim3(256), 0, ctx->stream, x, lda, m, k, m_pad, q,
+                                           scales_t, es_t));
     ctx->launches++;
-    B2W4_CUDA(ctx, cudaGetLastError());
     return B2W4_OK;
 }
 
@@ -170,13 +184,14 @@ int b2w4_launch_quantize_umma(b2w4_ctx* ctx, const float* x, int lda, int m, int
     long long warps = (long long)m * (k / 128);
     int grid = (int)((warps * 32 + 255) / 256);
     if (act_rule == B2W4_ACT_G32)
-        quantize_rows_umma_kernel<true><<<grid, 256, 0, ctx->stream>>>(x, lda, m, k, m_pad, q,
-                                                                       scales);
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, quantize_rows_umma_kernel<true>, dim3(grid),
+                                           dim3(256), 0, ctx->stream, x, lda, m, k, m_pad, q,
+                                           scales));
     else
-        quantize_rows_umma_kernel<false><<<grid, 256, 0, ctx->stream>>>(x, lda, m, k, m_pad, q,
-                                                                        scales);
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, quantize_rows_umma_kernel<false>, dim3(grid),
+                                           dim3(256), 0, ctx->stream, x, lda, m, k, m_pad, q,
+                                           scales));
     ctx->launches++;
-    B2W4_CUDA(ctx, cudaGetLastError());
     return B2W4_OK;
 }
 

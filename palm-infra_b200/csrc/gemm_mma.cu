@@ -34,7 +34,7 @@ namespace {
 
 constexpr int kGemmWarps = 16;
 constexpr int kGemmThreads = kGemmWarps * 32;
-constexpr int kRowBytes = 144;  // a token's 128 bytes of a stage + 16: conflict-free 16-byte reads
+constexpr int kRowBytes = 144;  // ring: a token's 128 bytes of a stage + 16: conflict-free reads
 constexpr int kMaxRows = 256;   // tokens per launch
 
 struct GemmMmaArgs {
@@ -56,10 +56,6 @@ __device__ __forceinline__ uint32_t gm_smem_u32(const void* p) {
 }
 __device__ __forceinline__ void gm_cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(gm_smem_u32(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void gm_cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(gm_smem_u32(dst)), "l"(src)
                  : "memory");
 }
 // lane (gid = lane/4, tid = lane%4): a0 row gid, k 4*tid..+3; a1 row gid+8; a2/a3 k+16;
@@ -89,23 +85,49 @@ __device__ __forceinline__ void gm_wait_groups(int n) {
     }
 }
 
-// one stage = one 128-k group of every token: codes, scales, accumulator biases
+// one stage = one 128-k group of every token: codes, scales, accumulator biases.  A group's
+// scales of all tokens are one contiguous run (m_pad tokens per scale), and so are its biases,
+// so all three are 16-byte copies dealt out by one index: with few tokens a thread issues at
+// most one.
 template <int SPG>
 __device__ __forceinline__ void load_stage(const GemmMmaArgs& a, int g, uint8_t* s_b, float* s_as,
                                            int* s_es) {
-    const int chunks = a.m * 8;  // 16-byte chunks
-    for (int i = threadIdx.x; i < chunks; i += kGemmThreads) {
-        const int t = i >> 3, c = i & 7;
-        gm_cp_async16(s_b + t * kRowBytes + c * 16,
-                      a.qa + (size_t)t * a.k + (size_t)g * 128 + c * 16);
-    }
-    const int m8 = (a.m + 7) & ~7;
-#pragma unroll
-    for (int sb = 0; sb < SPG; ++sb)
-        for (int t = threadIdx.x; t < a.m; t += kGemmThreads) {
-            gm_cp_async4(s_as + sb * m8 + t, a.as_t + (size_t)(g * SPG + sb) * a.m_pad + t);
-            gm_cp_async4(s_es + sb * m8 + t, a.es_t + (size_t)(g * SPG + sb) * a.m_pad + t);
+    const int codes = a.m * 8, run = SPG * a.m_pad / 4;
+    for (int i = threadIdx.x; i < codes + 2 * run; i += kGemmThreads) {
+        if (i < codes) {
+            const int t = i >> 3, c = i & 7;
+            gm_cp_async16(s_b + t * kRowBytes + c * 16,
+                          a.qa + (size_t)t * a.k + (size_t)g * 128 + c * 16);
+        } else if (i < codes + run) {
+            const int c = (i - codes) * 4;
+            gm_cp_async16(s_as + c, a.as_t + (size_t)g * SPG * a.m_pad + c);
+        } else {
+            const int c = (i - codes - run) * 4;
+            gm_cp_async16(s_es + c, a.es_t + (size_t)g * SPG * a.m_pad + c);
         }
+    }
+}
+
+// All groups at once (resident mode): a warp copies whole token rows, and the scales and
+// biases of all groups are one contiguous run each.  Group by group, with 4-byte copies of
+// the scales, issuing the copies was 4.7 of the kernel's 7.1 million warp instructions and 12
+// of its 21 us (16 rows per 32 values, [9728, 2560]; 16 such matmuls 361 -> 195 us).
+template <int SPG>
+__device__ __forceinline__ void load_all(const GemmMmaArgs& a, int row_bytes, uint8_t* s_b,
+                                         float* s_as, int* s_es) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int t = warp; t < a.m; t += kGemmWarps) {
+        const int8_t* src = a.qa + (size_t)t * a.k;
+        uint8_t* dst = s_b + (size_t)t * row_bytes;
+#pragma unroll 4
+        for (int c = lane * 16; c < a.k; c += 32 * 16)
+            gm_cp_async16(dst + c, src + c);
+    }
+    const int n = a.groups * SPG * a.m_pad;
+    for (int c = threadIdx.x * 4; c < n; c += kGemmThreads * 4) {
+        gm_cp_async16(s_as + c, a.as_t + c);
+        gm_cp_async16(s_es + c, a.es_t + c);
+    }
 }
 
 template <int CB, bool SCL16, bool A32>
@@ -119,7 +141,7 @@ gemm_w4a8_mma_kernel(const GemmMmaArgs a) {
     uint8_t* s_w = smem;                                      // [cap][G][512]
     uint8_t* s_scl = s_w + (size_t)a.tile_cap * tile_bytes;   // [cap][G][8]
     const int S = a.stages;
-    uint8_t* s_b = s_scl + (size_t)a.tile_cap * scl_tile_bytes;  // [S][m8][kRowBytes]
+    uint8_t* s_b = s_scl + (size_t)a.tile_cap * scl_tile_bytes;  // codes, see below
     constexpr int SPG = A32 ? 4 : 1;  // scales / biases per group
     float* s_as = reinterpret_cast<float*>(s_b + S * (size_t)m8 * kRowBytes);  // [S][SPG][m8]
     int* s_es = reinterpret_cast<int*>(s_as + S * SPG * m8);                    // [S][SPG][m8]
@@ -147,17 +169,21 @@ gemm_w4a8_mma_kernel(const GemmMmaArgs a) {
     // Ring mode: stages 0 .. S-2 in flight, one barrier per group.  Resident mode (S >= G,
     // few tokens): every group is loaded up front, one barrier in all, and the warps run
     // their K loops without meeting again.  The first copies also carry the weights.
+    // Codes in shared memory: ring mode [stage][token][128 + 16], resident mode
+    // [token][K + 16], which is smaller and as free of bank conflicts.
     const bool resident = S >= G;
-    const int pre = resident ? G : S - 1;
-    for (int g = 0; g < pre; ++g) {
-        if (g < G)
-            load_stage<SPG>(a, g, s_b + (size_t)g * m8 * kRowBytes, s_as + g * SPG * m8,
-                       s_es + g * SPG * m8);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
+    const int row_bytes = resident ? a.k + 16 : kRowBytes;
+    const int stage_bytes = resident ? 128 : m8 * kRowBytes;  // from a group to the next
     if (resident) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        load_all<SPG>(a, row_bytes, s_b, s_as, s_es);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
         __syncthreads();
+    } else {
+        for (int g = 0; g < S - 1; ++g) {
+            load_stage<SPG>(a, g, s_b + (size_t)g * stage_bytes, s_as + g * SPG * m8,
+                            s_es + g * SPG * m8);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
     }
 
     // this warp's pair of tiles and its range of 8-token column blocks
@@ -184,14 +210,14 @@ gemm_w4a8_mma_kernel(const GemmMmaArgs a) {
             __syncthreads();  // stage g visible to all; everyone is done with stage g-1
             if (g + S - 1 < G) {
                 const int sn = (g + S - 1) % S;  // the slot stage g-1 used
-                load_stage<SPG>(a, g + S - 1, s_b + (size_t)sn * m8 * kRowBytes, s_as + sn * SPG * m8,
-                           s_es + sn * SPG * m8);
+                load_stage<SPG>(a, g + S - 1, s_b + (size_t)sn * stage_bytes, s_as + sn * SPG * m8,
+                                s_es + sn * SPG * m8);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         const int st = resident ? g : g % S;
         if (cb0 < cb1) {
-            const uint8_t* b = s_b + (size_t)st * m8 * kRowBytes;
+            const uint8_t* b = s_b + (size_t)st * stage_bytes;
             const float* as = s_as + st * SPG * m8;
             const int* es = s_es + st * SPG * m8;
             // word `lane` of the 128 bytes of (tile, group, 32-block s): row gid, k 8*tid..+7
@@ -213,12 +239,12 @@ gemm_w4a8_mma_kernel(const GemmMmaArgs a) {
                 !two ? 0.f
                      : (SCL16 ? __half2float(reinterpret_cast<const __half*>(s_scl)[si + G * 8])
                               : reinterpret_cast<const float*>(s_scl)[si + G * 8]);
-            const uint8_t* bl = b + gid * kRowBytes + tid * 32;
+            const uint8_t* bl = b + gid * row_bytes + tid * 32;
 #pragma unroll
             for (int j = 0; j < CB; ++j) {
                 const int cb = cb0 + j;
                 if (cb < cb1) {  // warp-uniform
-                    const uint4* bp = reinterpret_cast<const uint4*>(bl + cb * (8 * kRowBytes));
+                    const uint4* bp = reinterpret_cast<const uint4*>(bl + (size_t)cb * 8 * row_bytes);
                     const uint4 be = bp[0], bo = bp[1];
                     const int tk = cb * 8 + tid * 2;  // tokens of this lane's accumulators
                     if (A32) {
