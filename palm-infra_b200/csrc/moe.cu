@@ -1052,6 +1052,14 @@ struct GroupedArgs {
     int k, groups, n_e, tiles_e, tpc;
 };
 
+template <int BYTES>
+__device__ __forceinline__ void moe_cp_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(BYTES)
+                 : "memory");
+}
+
 __device__ __forceinline__ void moe_mma_16x8x32(int (&d)[4], uint32_t a0, uint32_t a1,
                                                 uint32_t a2, uint32_t a3, uint32_t b0,
                                                 uint32_t b1) {
@@ -1129,18 +1137,20 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
 
     for (int base = r0; base < r1; base += kGR) {
         const int mc = min(kGR, r1 - base);
-        // quantised activations of this pass's routes
-        for (int i = threadIdx.x; i < mc * (K / 16); i += kGT) {
-            const int mi = i / (K / 16), c = i - mi * (K / 16);
+        // quantised activations of this pass's routes, a warp per row, all copies in flight at
+        // once (through registers a thread's eight loads were eight memory latencies;
+        // 256 tokens on 128 experts of 768, the whole operator: 330 -> 315 us)
+        for (int mi = warp; mi < mc; mi += kGW) {
             const int src_row = a.row_map ? a.row_map[base + mi] : base + mi;
-            *reinterpret_cast<uint4*>(s_qa + (size_t)mi * row_bytes + c * 16) =
-                reinterpret_cast<const uint4*>(qa_src + (size_t)src_row * K)[c];
+            const int8_t* src = qa_src + (size_t)src_row * K;
+            const float* as = as_src + (size_t)src_row * as_stride;
+#pragma unroll 4
+            for (int c = lane * 16; c < K; c += 32 * 16)
+                moe_cp_async<16>(s_qa + (size_t)mi * row_bytes + c, src + c);
+            for (int gs = lane; gs < G * SPG; gs += 32)
+                moe_cp_async<4>(s_as + gs * kGR + mi, as + gs);
         }
-        for (int i = threadIdx.x; i < mc * G * SPG; i += kGT) {
-            const int mi = i / (G * SPG), gs = i - mi * (G * SPG);
-            const int src_row = a.row_map ? a.row_map[base + mi] : base + mi;
-            s_as[gs * kGR + mi] = as_src[(size_t)src_row * as_stride + gs];
-        }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         // accumulator bias per (route, group): 0x4B400000 - 8 * (sum of the group's codes);
         // per-32 rule: per (route, 32-block).  In tensor-operand order the codes of 32-block
