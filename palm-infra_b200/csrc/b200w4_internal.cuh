@@ -192,9 +192,13 @@ int b2w4_launch_gemv_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, in
 
 int b2w4_launch_quantize_umma(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
                               int act_rule, int8_t* q, float* scales);
+// more rows than the kernels above take, on tcgen05: per-128 rule (gemm_tcgen05.cu) and
+// per-32 rule (gemm_tcgen05_a32.cu)
 int b2w4_launch_gemm_tc(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
-                        float* y, int ldc, int m, int act_rule, int activation, int act_n_begin,
+                        float* y, int ldc, int m, int activation, int act_n_begin,
                         int act_n_len);
+int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
+                          int ldc, int m, int activation, int act_n_begin, int act_n_len);
 
 // activation-quantiser output layouts
 enum {
@@ -358,6 +362,11 @@ __device__ __forceinline__ uint64_t b2w4_fma2(uint64_t a, uint64_t b, uint64_t c
 __device__ __forceinline__ uint64_t b2w4_mul2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t b2w4_sub2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 #endif

@@ -326,8 +326,11 @@ static int matmul_dispatch(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, 
         return b2w4_launch_gemm_mma(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
                                     act_n_len);
     if (tc)
-        return b2w4_launch_gemm_tc(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
-                                   act_n_len);
+        return act_rule == B2W4_ACT_G32
+                   ? b2w4_launch_gemm_tc32(ctx, w, x, lda, y, ldc, m, activation, act_n_begin,
+                                           act_n_len)
+                   : b2w4_launch_gemm_tc(ctx, w, x, lda, y, ldc, m, activation, act_n_begin,
+                                         act_n_len);
     return b2w4_launch_gemv(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
                             act_n_len, nullptr);
 }

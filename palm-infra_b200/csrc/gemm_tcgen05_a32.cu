@@ -1,0 +1,565 @@
+// W4G128 x int8 GEMM on tcgen05.mma kind::i8 under the reference's rule for several rows: one
+// activation scale per 32 values (kernels/matmul_w4.cpp:785-901 with the per-32 quantiser,
+// kernels/matmul_quant.cpp:280-329).  Per 32-k block b of a group
+//   D_b = sum q4*q8 over the block;  y = fma(float(D_b), fp32(ws*as[g][b]), y)
+// blocks ascending inside groups ascending.  A block is exactly one K = 32 MMA step, so every
+// step has an accumulator of its own and the fp32 chain takes four steps per group.
+//
+// What bounds it: the issue slots and the fp32 pipe of that chain (M*N*K/32 sums); the MMAs
+// keep the tensor pipe under a tenth busy.  So everything around the chain is kept out of it:
+//   epilogue   sixteen warps, thread = one token x a quarter of the tile's columns.  Four
+//              warps per scheduler hide each other's latencies (tensor-memory loads, shared
+//              loads).  A unit is handed back as soon as it is in registers.
+//   unpack     a nibble becomes a signed byte of 16 q with one AND (high nibble) or a shift
+//              and an AND (low nibble): three instructions per eight weights, so the sums
+//              are 16 D, |16 D| < 2^19.
+//   to float   the hardware conversion, which has a pipe of its own (a warp instruction in two
+//              cycles per scheduler, measured), so that the fp32 pipe sees only the scale
+//              product and the multiply-add, both paired (fma.rn.f32x2).  It also moves the
+//              sums from the registers that the fetch filled to register pairs.  The scales
+//              are staged as w / 16: a power of two, exact while w * as / 16 is a normal number.
+//   MMA        one thread; two accumulator units (a group each) or more in tensor
+//              memory, and one barrier frees an activation and a weight stage together.
+// Measured against the form this replaces (the accumulator switch of the per-128 kernel, two
+// integer adds and a subtraction per pair of sums, four hand-overs per two groups): 1000 rows,
+// [4100, 9728], three matmuls 1173 -> 882 us; eight layers of a 256-token prompt, all
+// operators, 3.39 -> 2.79 ms.
+// Tokens sit on the MMA's M side (128 per CTA), weight rows on its N side.  The next launch
+// is released at the start (programmatic dependent launch): weights and scales are fetched
+// while the quantiser in front still runs.  Every wait is bounded; on a timeout the kernel
+// flags the status word and drains.
+#include "tcgen05_ops.cuh"
+
+namespace {
+
+constexpr int kProducerWarp = 0;
+constexpr int kMmaWarp = 1;
+constexpr int kUnpackWarp0 = 2, kUnpackWarps = 2;
+// four epilogue warpgroups, one per column quarter; a warp's TMEM lane quarter is its index
+// mod 4
+constexpr int kEpiWarp0 = 4, kEpiWarps = 16;
+constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;  // 640
+constexpr int kStages = 4;    // activation and unpacked-weight stages (one group each)
+constexpr int kRawSlots = 3;  // nibble chunks of kGC groups in flight
+constexpr int kMaxG = 80;     // K <= 10240
+
+template <int RP>
+struct Smem {
+    static constexpr int kActStage = 128 * 128;            // 128 tokens x 128 B, swizzled
+    static constexpr int kBStage = RP * 128;               // int8 weights, swizzled
+    static constexpr int kRawSlot = (RP / 8) * kGC * 512;  // nibbles: [tile][kGC][512]
+    static constexpr int kActOff = 0;
+    static constexpr int kBOff = kActOff + kStages * kActStage;
+    static constexpr int kRawOff = kBOff + kStages * kBStage;
+    static constexpr int kWsOff = kRawOff + kRawSlots * kRawSlot;  // fp32 [G][RP]
+    static constexpr int kBarOff = kWsOff + kMaxG * RP * 4;
+    static constexpr int kTotal = kBarOff + 512 + 1024;  // barriers, + slack to align the base
+    static constexpr int kStagePitch = RP / 4 + 4;       // output staging, floats per token
+    static_assert(kEpiWarps * 32 * kStagePitch * 4 <= kStages * kActStage, "output staging");
+    static_assert(kTotal <= 227 * 1024, "shared memory");
+};
+
+// N columns of two blocks, complete when the statement is: loads and wait are one statement.
+template <int N>
+__device__ __forceinline__ void tmem_fetch2(uint32_t t0, uint32_t t1, uint32_t (&r)[2][N]);
+template <>
+__device__ __forceinline__ void tmem_fetch2<8>(uint32_t t0, uint32_t t1, uint32_t (&r)[2][8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
+        "%0, %1, %2, %3, %4, %5, %6, %7"
+        "}, [%16];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
+        "%8, %9, %10, %11, %12, %13, %14, %15"
+        "}, [%17];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]),
+          "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
+          "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]),
+          "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]), "=&r"(r[1][7])
+        : "r"(t0), "r"(t1)
+        : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_fetch2<12>(uint32_t t0, uint32_t t1, uint32_t (&r)[2][12]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
+        "%0, %1, %2, %3, %4, %5, %6, %7"
+        "}, [%24];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {"
+        "%8, %9, %10, %11"
+        "}, [%24+8];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
+        "%12, %13, %14, %15, %16, %17, %18, %19"
+        "}, [%25];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {"
+        "%20, %21, %22, %23"
+        "}, [%25+8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]),
+          "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
+          "=&r"(r[0][8]), "=&r"(r[0][9]), "=&r"(r[0][10]), "=&r"(r[0][11]),
+          "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]),
+          "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]), "=&r"(r[1][7]),
+          "=&r"(r[1][8]), "=&r"(r[1][9]), "=&r"(r[1][10]), "=&r"(r[1][11])
+        : "r"(t0), "r"(t1)
+        : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_fetch2<16>(uint32_t t0, uint32_t t1, uint32_t (&r)[2][16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {"
+        "%0, %1, %2, %3, %4, %5, %6, %7, "
+        "%8, %9, %10, %11, %12, %13, %14, %15"
+        "}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {"
+        "%16, %17, %18, %19, %20, %21, %22, %23, "
+        "%24, %25, %26, %27, %28, %29, %30, %31"
+        "}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]),
+          "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
+          "=&r"(r[0][8]), "=&r"(r[0][9]), "=&r"(r[0][10]), "=&r"(r[0][11]),
+          "=&r"(r[0][12]), "=&r"(r[0][13]), "=&r"(r[0][14]), "=&r"(r[0][15]),
+          "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]),
+          "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]), "=&r"(r[1][7]),
+          "=&r"(r[1][8]), "=&r"(r[1][9]), "=&r"(r[1][10]), "=&r"(r[1][11]),
+          "=&r"(r[1][12]), "=&r"(r[1][13]), "=&r"(r[1][14]), "=&r"(r[1][15])
+        : "r"(t0), "r"(t1)
+        : "memory");
+}
+
+template <int RP, bool SCL16>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_w4a8_tc32_kernel(const GemmArgs a) {
+    constexpr int CH = RP / 4;  // columns per epilogue thread
+    // A unit is what the MMA warp hands to the epilogue: a group's accumulators, four blocks
+    // of RP columns each.
+    constexpr int kAccCols = 4 * RP;
+    constexpr int kAcc = 512 / kAccCols;
+    static_assert(kAcc >= 2, "no accumulator to run ahead into");
+    extern __shared__ uint8_t smem_raw[];
+    // swizzle atoms need a 1024-byte aligned base
+    uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    using S = Smem<RP>;
+    const int G = a.groups;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int R = min(a.rows_per_cta, a.n - (int)blockIdx.x * a.rows_per_cta);  // may be ragged
+    const int r_tiles = (R + 7) / 8;
+    const int tile0 = blockIdx.x * (a.rows_per_cta / 8);
+    const int tok0 = blockIdx.y * 128;
+    const int m_here = min(128, a.m - tok0);
+
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kBarOff);
+    uint64_t* act_full = bars;                  // [kStages] activations of a group landed
+    uint64_t* b_full = act_full + kStages;      // [kStages] unpack done
+    uint64_t* ab_free = b_full + kStages;       // [kStages] MMAs that read both retired
+    uint64_t* raw_full = ab_free + kStages;     // [kRawSlots] nibble chunk landed
+    uint64_t* raw_free = raw_full + kRawSlots;  // [kRawSlots] unpack warps are done with it
+    uint64_t* acc_full = raw_free + kRawSlots;  // [kAcc] unit complete
+    uint64_t* acc_free = acc_full + kAcc;       // [kAcc] epilogue has fetched it
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + kAcc);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    b2w4_pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(&act_full[s], 1);
+            mbar_init(&b_full[s], kUnpackWarps);
+            mbar_init(&ab_free[s], 1);
+        }
+        for (int b = 0; b < kRawSlots; ++b) {
+            mbar_init(&raw_full[b], 1);
+            mbar_init(&raw_free[b], kUnpackWarps);
+        }
+        for (int b = 0; b < kAcc; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_free[b], kEpiWarps);
+        }
+        *s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {  // one warp owns the TMEM allocation: 512 columns
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(tmem_slot)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    auto fail = [&]() {
+        *s_abort = 1;
+        b2w4_report_timeout(a.status);
+    };
+    // a wait that looks at the abort word only when the phase is not there yet
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+        return mbar_try_wait(bar, parity) || (!*s_abort && mbar_wait(bar, parity));
+    };
+
+    if (warp == kProducerWarp) {
+        // =============================== producer ===================================
+        // lane t copies row tile t's share of a nibble chunk, lane 31 a group's activations
+        const int chunks = (G + kGC - 1) / kGC;
+        auto load_chunk = [&](int chunk) {
+            const int slot = chunk % kRawSlots, g = chunk * kGC, gc = min(kGC, G - g);
+            if (lane == 0)
+                mbar_expect_tx(&raw_full[slot], (uint32_t)r_tiles * gc * 512);
+            __syncwarp();
+            if (lane < r_tiles)
+                bulk_g2s(smem + S::kRawOff + slot * S::kRawSlot + lane * (kGC * 512),
+                         a.nib + ((size_t)(tile0 + lane) * G + g) * 512, (uint32_t)gc * 512,
+                         &raw_full[slot]);
+        };
+        // the weights do not depend on the quantiser in front of this kernel
+        for (int c = 0; c < min(kRawSlots, chunks); ++c)
+            load_chunk(c);
+        b2w4_pdl_wait();
+        // only the 8-token atoms that hold real tokens are copied; the MMA reads whatever the
+        // rest of the 128-token block holds and the epilogue ignores those accumulator rows
+        const uint32_t act_bytes = (uint32_t)((m_here + 7) / 8) * 1024;
+        bool ok = true;
+        for (int g = 0; g < G; ++g) {
+            if (g % kGC == 0 && g / kGC >= kRawSlots) {
+                const int chunk = g / kGC, slot = chunk % kRawSlots, use = chunk / kRawSlots;
+                ok = __all_sync(0xffffffffu, wait(&raw_free[slot], (use - 1) & 1));
+                if (!ok)
+                    break;
+                load_chunk(chunk);
+            }
+            const int s = g % kStages, round = g / kStages;
+            if (round > 0)
+                ok = __all_sync(0xffffffffu, wait(&ab_free[s], (round - 1) & 1));
+            if (!ok)
+                break;
+            if (lane == 31) {
+                mbar_expect_tx(&act_full[s], act_bytes);
+                bulk_g2s(smem + S::kActOff + s * S::kActStage,
+                         a.qa + ((size_t)g * a.m_pad + tok0) * 128, act_bytes, &act_full[s]);
+            }
+        }
+        if (!ok && lane == 0)
+            fail();
+    } else if (warp == kMmaWarp) {
+        // =============================== MMA issue ===================================
+        if (lane == 0) {
+            const uint32_t idesc = umma_idesc_i8(RP);
+            const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kActOff));
+            const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kBOff));
+            int u = 0, use = 0;  // unit buffer and how often it has been filled
+            for (int g = 0; g < G; ++g) {
+                const int s = g % kStages, round = g / kStages;
+                if (!wait(&act_full[s], round & 1) || !wait(&b_full[s], round & 1) ||
+                    (use > 0 && !wait(&acc_free[u], (use - 1) & 1))) {
+                    fail();
+                    break;
+                }
+                // descriptor addresses count 16-byte units
+                const uint64_t a_desc = a_desc0 + (uint64_t)(s * (S::kActStage >> 4));
+                const uint64_t b_desc = b_desc0 + (uint64_t)(s * (S::kBStage >> 4));
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 4; ++j)  // a K = 32 step (32 bytes) = a 32-k block
+                    umma_i8(tmem_base + (uint32_t)(u * kAccCols + j * RP),
+                            a_desc + (uint64_t)(j * 2), b_desc + (uint64_t)(j * 2), idesc, 0u);
+                umma_commit(&acc_full[u]);  // the group's sums are complete
+                if (++u == kAcc) {
+                    u = 0;
+                    ++use;
+                }
+                umma_commit(&ab_free[s]);  // both stages may be refilled
+            }
+        }
+    } else if (warp < kEpiWarp0) {
+        // =============================== unpack ======================================
+        const int ut = (warp - kUnpackWarp0) * 32 + lane;
+        for (int g = 0; g < G; ++g) {
+            const int chunk = g / kGC, slot = chunk % kRawSlots, cuse = chunk / kRawSlots;
+            const int gi = g % kGC;
+            const int s = g % kStages, round = g / kStages;
+            bool ok = true;
+            if (gi == 0)  // the chunk's nibbles landed
+                ok = __all_sync(0xffffffffu, wait(&raw_full[slot], cuse & 1));
+            if (ok && round > 0)  // MMAs left this stage
+                ok = __all_sync(0xffffffffu, wait(&ab_free[s], (round - 1) & 1));
+            if (!ok) {
+                fail();
+                break;
+            }
+            // raw slot: [tile][kGC groups][32 chunks of 16 B]
+            const uint4* raw =
+                reinterpret_cast<const uint4*>(smem + S::kRawOff + slot * S::kRawSlot) + gi * 32;
+            uint8_t* bst = smem + S::kBOff + s * S::kBStage;
+            // chunk c of tile t: sub = c/8, row = c%8 -> 32 k of weight row t*8+row
+#pragma unroll 4
+            for (int c = ut; c < r_tiles * 32; c += kUnpackWarps * 32) {
+                const int t = c >> 5, sub = (c >> 3) & 3, row = c & 7;
+                const uint4 w = raw[t * (kGC * 32) + (c & 31)];
+                // low nibbles = even k, high nibbles = odd k, in two's complement: a nibble in
+                // the upper half of a byte is the signed byte 16 q
+                constexpr uint32_t kHigh = 0xF0F0F0F0u;
+                const uint4 ev = make_uint4((w.x << 4) & kHigh, (w.y << 4) & kHigh,
+                                            (w.z << 4) & kHigh, (w.w << 4) & kHigh);
+                const uint4 od = make_uint4(w.x & kHigh, w.y & kHigh, w.z & kHigh, w.w & kHigh);
+                // weight row r = t*8+row: atom t (1024 B), row `row` (128 B), 16-byte
+                // chunks 2*sub (even k) and 2*sub+1 (odd k), XOR-swizzled with the row
+                uint8_t* rowp = bst + t * 1024 + row * 128;
+                *reinterpret_cast<uint4*>(rowp + (((2 * sub) ^ row) << 4)) = ev;
+                *reinterpret_cast<uint4*>(rowp + (((2 * sub + 1) ^ row) << 4)) = od;
+            }
+            // make the generic-proxy writes visible to the tensor core's async proxy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&b_full[s]);
+                if (gi == kGC - 1 || g == G - 1)
+                    mbar_arrive(&raw_free[slot]);  // this warp is done with the chunk
+            }
+        }
+    } else {
+        // =============================== epilogue ====================================
+        const int ew = warp - kEpiWarp0;       // 0..15
+        const int ch = ew >> 2;                // column quarter
+        const int lq = warp & 3;               // TMEM lane quarter this warp may read
+        const int tok = tok0 + lq * 32 + lane;
+        // a warp whose 32 tokens all lie past the last row has no chain to run
+        const bool active = lq * 32 < m_here;
+        // weight scales / 16 -> fp32 [G][RP] (column = row of the CTA), shared by all tokens
+        {
+            float* wsf = reinterpret_cast<float*>(smem + S::kWsOff);
+            // eight scales of one (tile, group) are contiguous
+            for (int i = ew * 32 + lane; i < G * (RP / 8); i += kEpiWarps * 32) {
+                const int t = i / G, g = i - t * G;
+                float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+                if (t < r_tiles) {
+                    const size_t idx = ((size_t)(tile0 + t) * G + g) * 8;
+                    if (SCL16) {
+                        const uint4 raw = *reinterpret_cast<const uint4*>(
+                            reinterpret_cast<const __half*>(a.scl) + idx);
+                        const __half2* h = reinterpret_cast<const __half2*>(&raw);
+                        const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]);
+                        const float2 f2 = __half22float2(h[2]), f3 = __half22float2(h[3]);
+                        lo = make_float4(f0.x, f0.y, f1.x, f1.y);
+                        hi = make_float4(f2.x, f2.y, f3.x, f3.y);
+                    } else {
+                        const float4* f = reinterpret_cast<const float4*>(
+                            reinterpret_cast<const float*>(a.scl) + idx);
+                        lo = f[0];
+                        hi = f[1];
+                    }
+                }
+                auto scaled = [](float4 v) {
+                    return make_float4(__fmul_rn(v.x, 0.0625f), __fmul_rn(v.y, 0.0625f),
+                                       __fmul_rn(v.z, 0.0625f), __fmul_rn(v.w, 0.0625f));
+                };
+                *reinterpret_cast<float4*>(wsf + g * RP + t * 8) = scaled(lo);
+                *reinterpret_cast<float4*>(wsf + g * RP + t * 8 + 4) = scaled(hi);
+            }
+        }
+        // named barrier among the epilogue warps only
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+        b2w4_pdl_wait();  // the quantiser's scales; and y may still be in use before this
+        const float* wsf = reinterpret_cast<const float*>(smem + S::kWsOff) + ch * CH;
+        const bool has_tok = tok < a.m;
+        // the token's four block scales of a group are one 16-byte load, fetched two groups
+        // ahead (a group's chain is long enough to cover the load)
+        const float4* as4 = reinterpret_cast<const float4*>(a.as) + tok;
+        auto load_as = [&](int g) {
+            return (has_tok && g < G) ? as4[(size_t)g * a.m_pad]
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        float4 a0 = load_as(0), a1 = load_as(1);
+        uint64_t acc2[CH / 2];  // the chain values, columns (2i, 2i + 1) side by side
+#pragma unroll
+        for (int i = 0; i < CH / 2; ++i)
+            acc2[i] = 0ull;
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(ch * CH);
+        int u = 0, use = 0;  // unit buffer and how often it has been filled before
+        bool live = true;
+        for (int g = 0; g < G; ++g) {
+            const float asv[4] = {a0.x, a0.y, a0.z, a0.w};
+            a0 = a1;
+            a1 = load_as(g + 2);
+            const bool ready = mbar_try_wait(&acc_full[u], use & 1);
+            if (!__all_sync(0xffffffffu, ready)) {
+                live = __all_sync(0xffffffffu, ready || wait(&acc_full[u], use & 1));
+                if (!live)
+                    break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t r[2][CH];
+            const uint32_t t = lane_addr + (uint32_t)(u * kAccCols);
+            const float* ws = wsf + g * RP;
+            auto chain = [&](float b0, float b1) {  // two blocks, in ascending order
+                const uint64_t s0 = b2w4_pack2(b0, b0), s1 = b2w4_pack2(b1, b1);
+#pragma unroll
+                for (int c = 0; c < CH; c += 4) {
+                    const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(ws + c);
+                    auto sums = [&](int j, int i) {
+                        return b2w4_pack2(__int2float_rn((int)r[j][i]),
+                                          __int2float_rn((int)r[j][i + 1]));
+                    };
+                    uint64_t& lo = acc2[c / 2];
+                    uint64_t& hi = acc2[c / 2 + 1];
+                    lo = b2w4_fma2(sums(0, c), b2w4_mul2(w2.x, s0), lo);
+                    hi = b2w4_fma2(sums(0, c + 2), b2w4_mul2(w2.y, s0), hi);
+                    lo = b2w4_fma2(sums(1, c), b2w4_mul2(w2.x, s1), lo);
+                    hi = b2w4_fma2(sums(1, c + 2), b2w4_mul2(w2.y, s1), hi);
+                }
+            };
+            if (active) {
+                tmem_fetch2<CH>(t, t + RP, r);
+                chain(asv[0], asv[1]);
+                tmem_fetch2<CH>(t + 2 * RP, t + 3 * RP, r);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&acc_free[u]);
+            if (++u == kAcc) {
+                u = 0;
+                ++use;
+            }
+            if (active)
+                chain(asv[2], asv[3]);
+        }
+        if (!live)
+            fail();
+        // Output: a thread holds one token's CH columns, which lie CH*4 bytes apart from the
+        // next token's in y.  Stage the warp's 32 x CH block in shared memory (the operand
+        // ring is idle: the last accumulator was complete, so every MMA and copy has
+        // retired) and store token rows with the lanes running along the columns.
+        if (active && live && !*s_abort) {
+            constexpr int SP = S::kStagePitch;  // 16-byte aligned rows
+            float* stage = reinterpret_cast<float*>(smem + S::kActOff) + ew * (32 * SP);
+            const int n0 = blockIdx.x * a.rows_per_cta + ch * CH;
+#pragma unroll
+            for (int c = 0; c < CH; c += 4) {
+                float4 v;
+                b2w4_unpack2(acc2[c / 2], v.x, v.y);
+                b2w4_unpack2(acc2[c / 2 + 1], v.z, v.w);
+                if (a.activation != B2W4_NONE) {
+                    float* e = &v.x;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (b2w4_act_applies(n0 + c + i, a.activation, a.act_n_begin,
+                                             a.act_n_len, a.n))
+                            e[i] = gemm_activation(e[i], a.activation);
+                }
+                *reinterpret_cast<float4*>(stage + lane * SP + c) = v;
+            }
+            __syncwarp();
+            const int tok_w = tok0 + lq * 32;  // first token of this warp
+            const int rows_w = min(32, a.m - tok_w);
+            const bool vec_ok = (a.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
+            constexpr int V = CH / 4;  // float4s per token row
+#pragma unroll 4
+            for (int i = lane; i < rows_w * V; i += 32) {
+                const int rr = i / V, c = (i - rr * V) * 4;
+                const float4 v = *reinterpret_cast<const float4*>(stage + rr * SP + c);
+                float* dst = a.y + (size_t)(tok_w + rr) * a.ldc + n0 + c;
+                const int left = R - (ch * CH + c);  // valid columns from here on
+                if (left >= 4 && vec_ok) {
+                    *reinterpret_cast<float4*>(dst) = v;
+                } else {
+                    if (left > 0) dst[0] = v.x;
+                    if (left > 1) dst[1] = v.y;
+                    if (left > 2) dst[2] = v.z;
+                    if (left > 3) dst[3] = v.w;
+                }
+            }
+        }
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                     ::"r"(tmem_base), "r"(512)
+                     : "memory");
+    }
+}
+
+template <int RP>
+int launch_rp(b2w4_ctx* ctx, const GemmArgs& a, bool scl16, dim3 grid) {
+    using S = Smem<RP>;
+    auto kern = scl16 ? gemm_w4a8_tc32_kernel<RP, true> : gemm_w4a8_tc32_kernel<RP, false>;
+    static b2w4_smem_optin configured[2];  // per instantiation and device
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, S::kTotal, configured[scl16]));
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kThreads), S::kTotal,
+                                       ctx->stream, a));
+    ctx->launches++;
+    return B2W4_OK;
+}
+
+// What a group costs beside its columns, in columns (measured: 1000 rows, [4100, 9728]: five
+// rounds of 48 columns take 314 us, four of 64 286 us).
+constexpr int kFixedColumns = 64;
+// accumulator columns of the instantiation that takes r row tiles
+int columns_for(int r) { return r <= 4 ? 32 : r <= 6 ? 48 : 64; }
+
+// Rows per CTA.  The fp32 chain paces a CTA, so its time grows with the accumulator columns
+// of its instantiation (plus a fixed part per group); the launch takes as many rounds as the
+// CTAs need on the SMs.  Pick the tile count with the least product.
+int row_tiles(int tiles, int token_blocks, int sm_count) {
+    int best = 1;
+    long best_cost = -1;
+    for (int r = 1; r <= 8; ++r) {
+        const long ctas = (long)((tiles + r - 1) / r) * token_blocks;
+        const long rounds = (ctas + sm_count - 1) / sm_count;
+        const long cost = rounds * (columns_for(r) + kFixedColumns);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = r;
+        }
+    }
+    return best;
+}
+
+}  // namespace
+
+// Quantises the activations per 32 values (separate launch), then runs the kernel above.
+int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
+                          int ldc, int m, int activation, int act_n_begin, int act_n_len) {
+    const int G = w->groups;
+    if (G > kMaxG)
+        return b2w4_fail(ctx, B2W4_E_INVALID, "gemm: K=%d exceeds the scale staging (K<=10240)",
+                         w->k);
+    const int m_pad = (m + 127) / 128 * 128;
+    void *qa = nullptr, *as = nullptr;
+    int rc;
+    if ((rc = b2w4_reserve(ctx, SCR_QA, (size_t)G * m_pad * 128, &qa)) != B2W4_OK ||
+        (rc = b2w4_reserve(ctx, SCR_AS, sizeof(float) * (size_t)G * m_pad * 4, &as)) != B2W4_OK)
+        return rc;
+    if ((rc = b2w4_launch_quantize_umma(ctx, x, lda, m, w->k, m_pad, B2W4_ACT_G32,
+                                        static_cast<int8_t*>(qa), static_cast<float*>(as))) !=
+        B2W4_OK)
+        return rc;
+    const int token_blocks = m_pad / 128;
+    const int r_tiles = row_tiles(w->tiles, token_blocks, ctx->sm_count);
+    GemmArgs a;
+    a.nib = reinterpret_cast<const uint8_t*>(w->nib);
+    a.scl = w->scl;
+    a.qa = static_cast<const int8_t*>(qa);
+    a.as = static_cast<const float*>(as);
+    a.y = y;
+    a.status = ctx->status_dev;
+    a.ldc = ldc;
+    a.m = m;
+    a.m_pad = m_pad;
+    a.n = w->n;
+    a.groups = G;
+    a.tiles = w->tiles;
+    a.rows_per_cta = r_tiles * 8;
+    a.activation = activation;
+    a.act_n_begin = act_n_begin;
+    a.act_n_len = act_n_len;
+    const dim3 grid((w->tiles + r_tiles - 1) / r_tiles, token_blocks);
+    const bool scl16 = w->scales_fp16 != 0;
+    switch (columns_for(r_tiles)) {
+    case 32: return launch_rp<32>(ctx, a, scl16, grid);
+    case 48: return launch_rp<48>(ctx, a, scl16, grid);
+    default: return launch_rp<64>(ctx, a, scl16, grid);
+    }
+}

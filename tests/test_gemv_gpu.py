@@ -289,6 +289,20 @@ def test_per32_rule_many_rows_bit_exact(ctx_mma, ctx_tc, kind, m, n, k):
     assert y.tobytes() == y_ref.tobytes()
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 8, 128), (128, 11832, 256), (300, 4100, 384),
+                                   (130, 9472, 512), (1000, 4100, 640), (97, 7104, 1664),
+                                   (160, 1184, 10240)])
+def test_per32_tensor_core_tiles_bit_exact(ctx_tc, m, n, k):
+    """The per-32 tcgen05 kernel in each of its tile widths (32, 48 and 64 columns), one and
+    several rounds of CTAs, ragged tokens and weight rows, fewer groups than pipeline stages
+    and the largest K, with codes at both ends of the range: its sums arrive as 16 D."""
+    blocks = pkg.synth.bg128_weight(20261125, n + k + m + 2, n, k)
+    x = pkg.synth.activations(7, m + 11, m, k)
+    x[m // 2] = np.sign(x[m // 2])  # every code +-127: the largest sums
+    y, _ = run_gpu(ctx_tc, blocks, n, k, x, rule=ol.ACT_G32, sums=False, pad=4 if n % 16 else 0)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).tobytes()
+
+
 def test_config2_prefill_m256_reference_rule(ctx):
     """M=256, K=2560, N=9728 (benchmark configuration 2, prefill) under the reference's rule
     for several rows (per 32 values), the kernel the library picks by itself: bit-exact
