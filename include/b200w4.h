@@ -362,13 +362,13 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      kernels/attention_x86_avx512.cpp:47-109 for the arithmetic):
  *                      appends the new tokens' k, v [tokens][kv_heads][dim] at
  *                      positions past.., then causal attention of q
- *                      [tokens][heads][dim] over keys 0 .. past + t, full-row softmax,
- *                      P*V accumulated in ascending key order (dim <= 256; the scores
- *                      of all visible keys are held in shared memory, which bounds
- *                      them near 45,000; runs of eight or more tokens take a tiled
- *                      form -- one block per kv head and tile of query tokens, keys
- *                      and values staged once per tile, the same bits -- while a
- *                      tile's scores fit, about 1,400 keys); past_dev (optional)
+ *                      [tokens][heads][dim] over keys 0 .. past + t, softmax and
+ *                      P*V in 32 bits (exp in 64; dim <= 256, about 47,000 keys at
+ *                      most).  Heads of 64, 128 or 256 features on 16-byte aligned
+ *                      rows: up to seven tokens split the keys over a cluster of
+ *                      blocks, longer runs take a tiled form with a running softmax;
+ *                      other sizes one block per (token, head);
+ *                      past_dev (optional)
  *                      gives `past` from device memory instead
  *                      k_dev and v_dev both NULL: nothing is appended, the cache rows
  *                      past .. past + tokens - 1 are in place already (b2w4_qkv_prepare)

@@ -4,9 +4,9 @@
 // attention over the cache, embedding-row lookup.  Semantics follow the reference's CPU
 // operators (the x86 build: its scalar and AVX-512 paths), cited per kernel.  Sums over a row
 // are tree reductions here where the reference's scalar loops are sequential, so these ops
-// agree with the reference to fp32 rounding of a reassociated sum, not bit for bit; everything
-// that is element-wise (rotary embedding, add, multiply, the P*V accumulation in key order)
-// uses the reference's operation order with no contraction.
+// agree with the reference to fp32 rounding of a reassociated sum, not bit for bit (attention:
+// dot products, and a softmax that runs over blocks of keys); everything that is element-wise
+// (rotary embedding, add, multiply) uses the reference's operation order with no contraction.
 // All tensors are fp32, rows = tokens, features contiguous.
 #include "b200w4_internal.cuh"
 
