@@ -5,7 +5,7 @@
 // operators (the x86 build: its scalar and AVX-512 paths), cited per kernel.  Sums over a row
 // are tree reductions here where the reference's scalar loops are sequential, so these ops
 // agree with the reference to fp32 rounding of a reassociated sum, not bit for bit (attention:
-// dot products, and a softmax that runs over blocks of keys); everything that is element-wise
+// dot products, and in some forms a softmax over parts of the keys); everything element-wise
 // (rotary embedding, add, multiply) uses the reference's operation order with no contraction.
 // All tensors are fp32, rows = tokens, features contiguous.
 #include "b200w4_internal.cuh"
@@ -286,33 +286,24 @@ __global__ void qkv_prepare_kernel(const float* __restrict__ qkv, int ld, int to
 }
 
 // Scaled-dot-product attention of one (query token, head) over the cache, the x86 reference's
-// operator (kernels/attention_x86_avx512.cpp:47-109): scores = dot(q, k_j) * scale for the
-// visible keys (causal: keys 0 .. past + t), softmax, then out = sum_j p_j * v_j in ascending
-// key order with one fused multiply-add per key and feature; a probability of zero
-// contributes nothing.  The softmax runs over blocks of kTileKeys keys in order (running
-// maximum m and sum l, earlier terms scaled by exp(m_old - m_new) when m moves), one division
-// at the end.  One block per (token, head), any head size: the form that serves what the two
-// kernels below do not take.  Its arithmetic is attention_tile_kernel's, operation for
-// operation: a dot product is summed per 32 features (even and odd ones apart), the parts in
-// order; a block's probabilities add up in an xor-tree.  Keys and values come through shared
-// memory in chunks that all threads fetch together, the next chunk's loads in flight while
-// the current one is consumed.
+// arithmetic (kernels/attention_x86_avx512.cpp:47-109): scores = dot(q, k_j) * scale for the
+// visible keys (causal: keys 0 .. past + t), full-row softmax (max, exp, sum, times 1/sum),
+// then out = sum_j p_j * v_j accumulated key by key in ascending order with one fused
+// multiply-add per key and feature, as the reference's loop does; a probability of zero
+// contributes nothing.  One block per (token, head): the form that takes any head size and
+// any alignment.  Scores: a warp per key, four keys' loads in flight at a time.  P*V: thread d
+// owns output feature d and walks the keys in order; the value rows come through shared memory
+// in chunks that all threads fetch together, the next chunk's loads in flight while the current
+// one is consumed, so that the ordered sum does not wait on memory once per key.
+// What bounds it: the latency of those loads (16 KB in flight per block).  Keys staged through
+// shared memory with a lane per 32 features and a running softmax, so that the sums follow
+// attention_tile_kernel's order, was slower on every shape that takes this form: 32 / 8 heads
+// of 80, one token behind 1000 keys 71 us against 42, 32 tokens 318 against 140; of 96 tokens
+// behind 6000 keys 2028 against 830.
 constexpr int kAttnThreads = 256;
 constexpr int kAttnWarps = kAttnThreads / 32;
-constexpr int kAttnStage = 4096;                       // floats of K or V per chunk
+constexpr int kAttnStage = 4096;                       // floats of V per chunk
 constexpr int kAttnPerThread = kAttnStage / kAttnThreads;
-constexpr int kAttnStagePad = kAttnStage + kAttnStage / 32 + kAttnStage / 8;  // skewed keys
-constexpr int kTileKeys = 32;                          // keys per softmax block
-
-// running maximum over a further block of scores, and the factor for what is summed so far
-__device__ __forceinline__ float attn_rescale(float m_old, float m_new) {
-    return m_new == -INFINITY ? 1.f : (float)exp((double)__fsub_rn(m_old, m_new));
-}
-// exp(s - m); m = -inf: no score above -inf yet, every term is zero
-__device__ __forceinline__ float attn_prob(float s, float m) {
-    return (float)exp((double)__fsub_rn(s, m == -INFINITY ? 0.f : m));
-}
-
 __global__ void __launch_bounds__(kAttnThreads)
 attention_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                  const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
@@ -321,9 +312,120 @@ attention_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
     b2w4_pdl_chain_entry();
     const int past = past_dev ? min(*past_dev, capacity - tokens) : past0;
     extern __shared__ float s_dyn[];
-    float* s_scores = s_dyn;                            // [score_slots] >= visible keys
-    float* s_stage = s_scores + score_slots;            // [kAttnStagePad]
-    float* s_alpha = s_stage + kAttnStagePad;           // [blocks]: factor before block b
+    float* s_scores = s_dyn;                // [score_slots] >= visible keys
+    float* s_stage = s_dyn + score_slots;   // [kAttnStage]
+    __shared__ float s_part[kAttnWarps];
+    const int t = blockIdx.x / heads, h = blockIdx.x % heads;
+    const int kvh = h / (heads / kv_heads);
+    const int visible = past + t + 1;
+    const float* qr = q + ((size_t)t * heads + h) * dim;
+    const float* kc = k_cache + (size_t)kvh * capacity * dim;
+    const float* vc = v_cache + (size_t)kvh * capacity * dim;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    constexpr int kQ = kAttnMaxDim / 32, kKeys = 4;
+    float qv[kQ];
+#pragma unroll
+    for (int i = 0; i < kQ; ++i)
+        qv[i] = lane + 32 * i < dim ? qr[lane + 32 * i] : 0.f;
+    for (int j0 = warp * kKeys; j0 < visible; j0 += kAttnWarps * kKeys) {
+        float kv[kKeys][kQ];
+#pragma unroll
+        for (int u = 0; u < kKeys; ++u)
+#pragma unroll
+            for (int i = 0; i < kQ; ++i)
+                kv[u][i] = (j0 + u < visible && lane + 32 * i < dim)
+                               ? kc[(size_t)(j0 + u) * dim + lane + 32 * i] : 0.f;
+#pragma unroll
+        for (int u = 0; u < kKeys; ++u) {
+            float p = 0.f;
+#pragma unroll
+            for (int i = 0; i < kQ; ++i)
+                if (32 * i < dim)  // lanes past the last feature add +0 products
+                    p = __fmaf_rn(qv[i], kv[u][i], p);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+                p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, off));
+            if (lane == 0 && j0 + u < visible)
+                s_scores[j0 + u] = __fmul_rn(p, scale);
+        }
+    }
+    __syncthreads();
+    float m = -INFINITY;
+    for (int j = threadIdx.x; j < visible; j += blockDim.x)
+        m = fmaxf(m, s_scores[j]);
+    m = block_max(m, s_part);
+    float sum = 0.f;
+    for (int j = threadIdx.x; j < visible; j += blockDim.x) {
+        const float e = (float)exp((double)__fsub_rn(s_scores[j], m));
+        s_scores[j] = e;
+        sum = __fadd_rn(sum, e);
+    }
+    sum = block_sum(sum, s_part);
+    const float inv = __fdiv_rn(1.f, sum);
+
+    const int chunk = kAttnStage / dim;  // keys per chunk
+    float r[kAttnPerThread];
+    auto fetch = [&](int j0) {
+        const int n = min(chunk, visible - j0) * dim;
+        const float* src = vc + (size_t)j0 * dim;
+#pragma unroll
+        for (int u = 0; u < kAttnPerThread; ++u) {
+            const int i = threadIdx.x + kAttnThreads * u;
+            r[u] = i < n ? src[i] : 0.f;
+        }
+    };
+    fetch(0);
+    float acc = 0.f;
+    for (int j0 = 0; j0 < visible; j0 += chunk) {
+        __syncthreads();  // the previous chunk has been consumed (and the scores are final)
+#pragma unroll
+        for (int u = 0; u < kAttnPerThread; ++u)
+            s_stage[threadIdx.x + kAttnThreads * u] = r[u];
+        __syncthreads();
+        if (j0 + chunk < visible)
+            fetch(j0 + chunk);
+        if (threadIdx.x < dim) {
+            const int nk = min(chunk, visible - j0);
+            for (int j = 0; j < nk; ++j) {
+                const float p = __fmul_rn(s_scores[j0 + j], inv);
+                if (p != 0.f)
+                    acc = __fmaf_rn(s_stage[j * dim + threadIdx.x], p, acc);
+            }
+        }
+    }
+    if (threadIdx.x < dim)
+        out[((size_t)t * heads + h) * dim + threadIdx.x] = acc;
+}
+
+// Softmax over blocks of kTileKeys keys in order: the running maximum m moves, and what is
+// summed so far is scaled by exp(m_old - m_new).
+constexpr int kTileKeys = 32;
+__device__ __forceinline__ float attn_rescale(float m_old, float m_new) {
+    return m_new == -INFINITY ? 1.f : (float)exp((double)__fsub_rn(m_old, m_new));
+}
+// exp(s - m); m = -inf: no score above -inf yet, every term is zero
+__device__ __forceinline__ float attn_prob(float s, float m) {
+    return (float)exp((double)__fsub_rn(s, m == -INFINITY ? 0.f : m));
+}
+
+// attention_tile_kernel's arithmetic, operation for operation, one block per (token, head): a
+// dot product is summed per 32 features (even and odd ones apart), the parts in order; the
+// softmax runs over blocks of keys; a block's probabilities add up in an xor-tree; one division
+// at the end.  Written plainly (a thread per key, one warp for the softmax, a thread per
+// feature): B2W4_ATTN=row runs it on the head sizes of the tile and cluster kernels, to compare
+// them with.
+__global__ void __launch_bounds__(kAttnThreads)
+attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
+                       const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
+                       int heads, int kv_heads, int dim, int past0,
+                       const int* __restrict__ past_dev, int capacity, float scale,
+                       int score_slots) {
+    b2w4_pdl_chain_entry();
+    const int past = past_dev ? min(*past_dev, capacity - tokens) : past0;
+    extern __shared__ float s_dyn[];
+    float* s_scores = s_dyn;               // [score_slots] >= visible keys
+    float* s_alpha = s_dyn + score_slots;  // [blocks]: factor before block b
     __shared__ float s_total;
     const int t = blockIdx.x / heads, h = blockIdx.x % heads;
     const int kvh = h / (heads / kv_heads);
@@ -331,128 +433,58 @@ attention_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
     const float* qr = q + ((size_t)t * heads + h) * dim;
     const float* kc = k_cache + (size_t)kvh * capacity * dim;
     const float* vc = v_cache + (size_t)kvh * capacity * dim;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int chunk = kAttnStage / dim;  // keys per chunk
-    float r[kAttnPerThread];
-    auto fetch = [&](const float* base, int j0) {
-        const int n = min(chunk, visible - j0) * dim;
-        const float* src = base + (size_t)j0 * dim;
-#pragma unroll
-        for (int u = 0; u < kAttnPerThread; ++u) {
-            const int i = threadIdx.x + kAttnThreads * u;
-            r[u] = i < n ? src[i] : 0.f;
-        }
-    };
-
-    // ---- scores: `parts` lanes per key, a lane per 32 features ----
-    const int parts = dim <= 32 ? 1 : dim <= 64 ? 2 : dim <= 128 ? 4 : 8;
-    const int part = lane % parts, sub = lane / parts, keys_warp = 32 / parts;
-    // a part starts 33 floats after the one before it, so that parts and keys spread over banks
-    const int pitch = dim <= 32 ? dim : dim + (dim + 31) / 32;
-    float qv[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-        qv[i] = part * 32 + i < dim ? qr[part * 32 + i] : 0.f;
-    fetch(kc, 0);
-    for (int j0 = 0; j0 < visible; j0 += chunk) {
-        __syncthreads();  // the previous chunk has been consumed
-#pragma unroll
-        for (int u = 0; u < kAttnPerThread; ++u) {
-            const int i = threadIdx.x + kAttnThreads * u, key = i / dim, d = i - key * dim;
-            if (key < chunk)
-                s_stage[key * pitch + d + (d >> 5)] = r[u];
-        }
-        __syncthreads();
-        if (j0 + chunk < visible)
-            fetch(kc, j0 + chunk);
-        const int nk = min(chunk, visible - j0);
-        for (int k0 = warp * keys_warp; k0 < nk; k0 += kAttnWarps * keys_warp) {
-            const int key = k0 + sub;
-            const float* kr = s_stage + min(key, nk - 1) * pitch + part * 33;
+    const int lane = threadIdx.x & 31;
+    for (int j = threadIdx.x; j < visible; j += kAttnThreads) {
+        const float* kr = kc + (size_t)j * dim;
+        float s = 0.f;
+        for (int c = 0; c < dim; c += 32) {
             float even = 0.f, odd = 0.f;
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-                if (part * 32 + i < dim)
-                    even = __fmaf_rn(qv[i], kr[i], even);
-                if (part * 32 + i + 1 < dim)
-                    odd = __fmaf_rn(qv[i + 1], kr[i + 1], odd);
+            for (int i = c; i < c + 32; i += 2) {
+                even = __fmaf_rn(qr[i], kr[i], even);
+                odd = __fmaf_rn(qr[i + 1], kr[i + 1], odd);
             }
-            const float p = __fadd_rn(even, odd);
-            float s = 0.f;
-            for (int c = 0; c < parts; ++c)
-                s = __fadd_rn(s, __shfl_sync(0xffffffffu, p, sub * parts + c));
-            if (part == 0 && key < nk)
-                s_scores[j0 + key] = __fmul_rn(s, scale);
+            s = __fadd_rn(s, __fadd_rn(even, odd));
         }
+        s_scores[j] = __fmul_rn(s, scale);
     }
     __syncthreads();
-    fetch(vc, 0);
-
-    // ---- softmax: block maxima, their running maximum, probabilities and block sums ----
-    float* s_max = s_stage;            // [blocks] running maximum (the stage is free here)
-    float* s_sum = s_alpha + blocks;   // [blocks]
-    for (int b = warp; b < blocks; b += kAttnWarps) {
-        const int j = b * kTileKeys + lane;
-        float m = j < visible ? s_scores[j] : -INFINITY;
+    if (threadIdx.x < 32) {
+        float m = -INFINITY, l = 0.f;
+        for (int b = 0; b < blocks; ++b) {
+            const int j = b * kTileKeys + lane;
+            float mb = j < visible ? fmaxf(m, s_scores[j]) : m;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+            for (int off = 16; off > 0; off >>= 1)
+                mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, off));
+            const float alpha = b ? attn_rescale(m, mb) : 1.f;
+            m = mb;
+            float e = 0.f;
+            if (j < visible)
+                s_scores[j] = e = attn_prob(s_scores[j], m);
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1)
+                e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, off));
+            l = __fadd_rn(__fmul_rn(l, alpha), e);
+            if (lane == 0)
+                s_alpha[b] = alpha;
+        }
         if (lane == 0)
-            s_max[b] = fmaxf(m, -INFINITY);
+            s_total = l;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float m = -INFINITY;
-        for (int b = 0; b < blocks; ++b)
-            s_max[b] = m = fmaxf(m, s_max[b]);
-    }
-    __syncthreads();
-    for (int b = warp; b < blocks; b += kAttnWarps) {
-        const int j = b * kTileKeys + lane;
-        const float m = s_max[b];
-        float e = 0.f;
-        if (j < visible)
-            s_scores[j] = e = attn_prob(s_scores[j], m);
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1)
-            e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, off));
-        if (lane == 0) {
-            s_sum[b] = e;
-            s_alpha[b] = b ? attn_rescale(s_max[b - 1], m) : 1.f;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float l = 0.f;
-        for (int b = 0; b < blocks; ++b)
-            l = __fadd_rn(__fmul_rn(l, s_alpha[b]), s_sum[b]);
-        s_total = l;
-    }
-
+    if (threadIdx.x >= dim)
+        return;
     float acc = 0.f;
-    for (int j0 = 0; j0 < visible; j0 += chunk) {
-        __syncthreads();  // the previous chunk has been consumed (and the sums are final)
-#pragma unroll
-        for (int u = 0; u < kAttnPerThread; ++u)
-            s_stage[threadIdx.x + kAttnThreads * u] = r[u];
-        __syncthreads();
-        if (j0 + chunk < visible)
-            fetch(vc, j0 + chunk);
-        if (threadIdx.x < dim) {
-            const int nk = min(chunk, visible - j0);
-            for (int j = 0; j < nk; ++j) {
-                if ((j0 + j) % kTileKeys == 0) {
-                    const float al = s_alpha[(j0 + j) / kTileKeys];
-                    acc = al == 0.f ? 0.f : __fmul_rn(acc, al);
-                }
-                const float p = s_scores[j0 + j];
-                if (p != 0.f)
-                    acc = __fmaf_rn(s_stage[j * dim + threadIdx.x], p, acc);
-            }
+    for (int j = 0; j < visible; ++j) {
+        if (j % kTileKeys == 0) {
+            const float al = s_alpha[j / kTileKeys];
+            acc = al == 0.f ? 0.f : __fmul_rn(acc, al);
         }
+        const float p = s_scores[j];
+        if (p != 0.f)
+            acc = __fmaf_rn(vc[(size_t)j * dim + threadIdx.x], p, acc);
     }
-    if (threadIdx.x < dim)
-        out[((size_t)t * heads + h) * dim + threadIdx.x] = __fdiv_rn(acc, s_total);
+    out[((size_t)t * heads + h) * dim + threadIdx.x] = __fdiv_rn(acc, s_total);
 }
 
 // The same attention for a few query tokens (a decode step): a cluster of kSplitCtas blocks
@@ -744,8 +776,8 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
 
 // The same attention for a run of new tokens (prefill): one block per (kv head, tile of query
 // tokens) serves every query head of that kv head -- up to kTileRows (token, head) rows --
-// against blocks of kTileKeys keys, with the running softmax of attention_kernel and its
-// arithmetic operation for operation, so both give the same bits.  Nothing grows with the
+// against blocks of kTileKeys keys, with a running softmax (attention_plain_kernel's arithmetic,
+// operation for operation: the same bits).  Nothing grows with the
 // number of keys: any context length takes this form.
 // What bounds it: the fp32 multiply-adds of the two products (2 * keys * rows * DIM a tile),
 // issued two lanes at a time (fma.rn.f32x2); scores and probabilities stay in 32 bits, which
@@ -1177,7 +1209,8 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
                       !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev |
                          (uintptr_t)out_dev) & 15);
     const bool split = wide && tokens < 8;
-    const bool tiles = wide && !split && ctx->attn_tiles && rep <= kTileRows;
+    const bool tiles = wide && ctx->attn_tiles && !split && rep <= kTileRows;
+    const bool plain = !ctx->attn_tiles && (dim == 64 || dim == 128 || dim == 256);
     const int score_slots = (keys + 3) & ~3;
     if (sizeof(float) * ((size_t)score_slots + kAttnStage) > 200 * 1024)
         return b2w4_fail(ctx, B2W4_E_INVALID, "attention: %d keys exceed the score buffer", keys);
@@ -1248,11 +1281,13 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
             B2W4_TILE(256);
 #undef B2W4_TILE
     } else {
-        static b2w4_smem_optin configured;
-        const size_t row_smem = sizeof(float) * ((size_t)score_slots + kAttnStagePad +
-                                                 2 * ((keys + kTileKeys - 1) / kTileKeys));
-        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, attention_kernel, row_smem, configured));
-        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, attention_kernel, dim3(tokens * heads),
+        static b2w4_smem_optin configured[2];
+        auto kern = plain ? attention_plain_kernel : attention_kernel;
+        const size_t row_smem =
+            sizeof(float) * ((size_t)score_slots +
+                             (plain ? (keys + kTileKeys - 1) / kTileKeys : kAttnStage));
+        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, row_smem, configured[plain]));
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(tokens * heads),
                                            dim3(kAttnThreads), row_smem, ctx->stream, q_dev, kc,
                                            vc, out_dev, tokens, heads, kv_heads, dim, past,
                                            past_dev, capacity, scale, score_slots));

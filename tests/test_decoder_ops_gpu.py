@@ -339,3 +339,75 @@ def test_tile_and_row_attention(ctx, tokens, past, heads, kv_heads, dim):
     if tokens > 1:
         want = _attention_fp64(q, k_all, v_all, heads, kv_heads, past, scale)
         assert rel_l2(got[:-1], want[:-1]) < 1e-5
+
+
+def _row_context():
+    """A context whose attention keeps one block per (token, head)."""
+    import os
+    os.environ["B2W4_ATTN"] = "row"
+    try:
+        return pkg.capi.Context(0)
+    finally:
+        del os.environ["B2W4_ATTN"]
+
+
+def _staged(rng, heads, kv_heads, dim, keys, levels):
+    """q of one token and a cache whose scores (scale 1) are levels[i] in the i-th part of the
+    keys, the same for every head: feature 0 carries the score, the others are zero."""
+    q = np.zeros((1, heads, dim), dtype=np.float32)
+    q[:, :, 0] = 1.0
+    k = np.zeros((keys, kv_heads, dim), dtype=np.float32)
+    for i, part in enumerate(np.array_split(np.arange(keys), len(levels))):
+        k[part, :, 0] = levels[i]
+    v = rng.normal(0, 1, (keys, kv_heads, dim)).astype(np.float32)
+    return q, k, v
+
+
+@pytest.mark.parametrize("row", [False, True])
+@pytest.mark.parametrize("tokens,heads,kv_heads,dim", [(1, 4, 2, 80), (10, 4, 2, 80)])
+def test_attention_ignores_value_rows_of_zero_probability(ctx, tokens, heads, kv_heads, dim, row):
+    """Scores of 0, 80 and 160 in the three parts of the cache: a key of the first part has
+    the probability e^-160 = 0, but e^-80 > 0 against the middle part, and 1 against its own
+    neighbours.  Its value row is NaN (then infinite): nothing of it may reach the output, in
+    whatever order or split the keys are taken.  Then value rows near the largest number under
+    equal scores: a sum before the division would overflow, the result does not.  Tolerance:
+    300 terms summed in fp32 at most one after the other, 300 * 2^-24 = 2e-5 of their
+    magnitudes; the mean of 1e38 rows keeps 1e-5 since all terms have one sign."""
+    import torch
+    rng = np.random.default_rng(dim + tokens)
+    keys = 300 + tokens
+    q1, k, v = _staged(rng, heads, kv_heads, dim, keys, [0.0, 80.0, 160.0])
+    q = np.repeat(q1, tokens, axis=0)
+    c = _row_context() if row else ctx
+    capacity = keys + 3
+
+    def run():
+        kc = np.zeros((kv_heads, capacity, dim), dtype=np.float32)
+        vc = np.zeros((kv_heads, capacity, dim), dtype=np.float32)
+        kc[:, :keys], vc[:, :keys] = k.transpose(1, 0, 2), v.transpose(1, 0, 2)
+        out = torch.zeros((tokens, heads, dim), dtype=torch.float32, device="cuda")
+        c.attention(_dev(q), None, None, _dev(kc), _dev(vc), out, tokens, heads, kv_heads, dim,
+                    keys - tokens, capacity, 1.0)
+        c.sync()
+        return out.cpu().numpy()
+
+    clean = _attention_fp64(q, k, np.where(np.arange(keys)[:, None, None] < 100, 0, v), heads,
+                            kv_heads, keys - tokens, 1.0)
+    for bad in (np.nan, np.inf, -np.inf):
+        v[3] = bad
+        v[50, :, dim // 2] = bad
+        got = run()
+        assert np.isfinite(got).all()
+        assert rel_l2(got, clean) < 2e-5
+    k[:] = 0.0
+    v[:] = 3e38 * rng.uniform(0.5, 1.0, v.shape)
+    got = run()
+    want = _attention_fp64(q, k, v, heads, kv_heads, keys - tokens, 1.0)
+    assert np.isfinite(got).all()
+    assert rel_l2(got / 3e38, want / 3e38) < 1e-5
+    k[:] = 0.0
+    v[:] = rng.normal(0, 1, v.shape)
+    v[7] = np.nan  # seen: every feature is NaN, as the sum has it
+    assert np.isnan(run()).all()
+    if row:
+        c.close()
