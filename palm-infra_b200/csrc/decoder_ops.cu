@@ -1208,7 +1208,7 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
     const bool wide = (dim == 64 || dim == 128 || dim == 256) &&
                       !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev |
                          (uintptr_t)out_dev) & 15);
-    const bool split = wide && tokens < 8;
+    const bool split = wide && ctx->attn_tiles && tokens < 8;
     const bool tiles = wide && ctx->attn_tiles && !split && rep <= kTileRows;
     const bool plain = !ctx->attn_tiles && (dim == 64 || dim == 128 || dim == 256);
     const int score_slots = (keys + 3) & ~3;

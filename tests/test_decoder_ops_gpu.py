@@ -351,6 +351,36 @@ def _row_context():
         del os.environ["B2W4_ATTN"]
 
 
+@pytest.mark.parametrize("past,heads,kv_heads,dim", [(0, 4, 2, 128), (31, 2, 2, 64),
+                                                     (300, 8, 2, 128), (97, 6, 2, 256)])
+def test_row_switch_holds_for_a_single_token(ctx, past, heads, kv_heads, dim):
+    """B2W4_ATTN=row keeps the one-row kernel for single tokens too: the last token of a run
+    through the tile kernel and that token alone through the row switch leave the same bits
+    (one arithmetic), and the default form of the single token agrees with both (tolerance as
+    for the split kernel)."""
+    import torch
+    tokens, scale = 9, dim ** -0.5
+    capacity = past + tokens + 2
+    rng = np.random.default_rng(past + dim)
+    q = _dev(rng.normal(0, 1, (tokens, heads, dim)).astype(np.float32))
+    kc, vc = (_dev(rng.normal(0, 1, (kv_heads, capacity, dim)).astype(np.float32))
+              for _ in range(2))
+    run, row, one = (torch.zeros((n, heads, dim), dtype=torch.float32, device="cuda")
+                     for n in (tokens, 1, 1))
+    ctx_row = _row_context()
+    last = q[-1:].contiguous()
+    ctx.attention(q, None, None, kc, vc, run, tokens, heads, kv_heads, dim, past, capacity, scale)
+    ctx_row.attention(last, None, None, kc, vc, row, 1, heads, kv_heads, dim,
+                      past + tokens - 1, capacity, scale)
+    ctx.attention(last, None, None, kc, vc, one, 1, heads, kv_heads, dim, past + tokens - 1,
+                  capacity, scale)
+    ctx.sync()
+    ctx_row.sync()
+    ctx_row.close()
+    assert row.cpu().numpy().tobytes() == run[-1:].contiguous().cpu().numpy().tobytes()
+    assert rel_l2(one.cpu().numpy(), row.cpu().numpy()) < 1e-5
+
+
 def _staged(rng, heads, kv_heads, dim, keys, levels):
     """q of one token and a cache whose scores (scale 1) are levels[i] in the i-th part of the
     keys, the same for every head: feature 0 carries the score, the others are zero."""
