@@ -10,6 +10,8 @@
 // All tensors are fp32, rows = tokens, features contiguous.
 #include "b200w4_internal.cuh"
 
+#include <cfloat>
+
 #include <cooperative_groups.h>
 
 namespace {
@@ -426,7 +428,7 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
     extern __shared__ float s_dyn[];
     float* s_scores = s_dyn;               // [score_slots] >= visible keys
     float* s_alpha = s_dyn + score_slots;  // [blocks]: factor before block b
-    __shared__ float s_total;
+    __shared__ float s_max, s_total;
     const int t = blockIdx.x / heads, h = blockIdx.x % heads;
     const int kvh = h / (heads / kv_heads);
     const int visible = past + t + 1, blocks = (visible + kTileKeys - 1) / kTileKeys;
@@ -434,20 +436,23 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
     const float* kc = k_cache + (size_t)kvh * capacity * dim;
     const float* vc = v_cache + (size_t)kvh * capacity * dim;
     const int lane = threadIdx.x & 31;
-    for (int j = threadIdx.x; j < visible; j += kAttnThreads) {
-        const float* kr = kc + (size_t)j * dim;
-        float s = 0.f;
-        for (int c = 0; c < dim; c += 32) {
-            float even = 0.f, odd = 0.f;
-            for (int i = c; i < c + 32; i += 2) {
-                even = __fmaf_rn(qr[i], kr[i], even);
-                odd = __fmaf_rn(qr[i + 1], kr[i + 1], odd);
+    auto scores = [&]() {
+        for (int j = threadIdx.x; j < visible; j += kAttnThreads) {
+            const float* kr = kc + (size_t)j * dim;
+            float s = 0.f;
+            for (int c = 0; c < dim; c += 32) {
+                float even = 0.f, odd = 0.f;
+                for (int i = c; i < c + 32; i += 2) {
+                    even = __fmaf_rn(qr[i], kr[i], even);
+                    odd = __fmaf_rn(qr[i + 1], kr[i + 1], odd);
+                }
+                s = __fadd_rn(s, __fadd_rn(even, odd));
             }
-            s = __fadd_rn(s, __fadd_rn(even, odd));
+            s_scores[j] = __fmul_rn(s, scale);
         }
-        s_scores[j] = __fmul_rn(s, scale);
-    }
-    __syncthreads();
+        __syncthreads();
+    };
+    scores();
     if (threadIdx.x < 32) {
         float m = -INFINITY, l = 0.f;
         for (int b = 0; b < blocks; ++b) {
@@ -468,23 +473,36 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
             if (lane == 0)
                 s_alpha[b] = alpha;
         }
-        if (lane == 0)
+        if (lane == 0) {
+            s_max = m;
             s_total = l;
+        }
     }
     __syncthreads();
-    if (threadIdx.x >= dim)
-        return;
-    float acc = 0.f;
-    for (int j = 0; j < visible; ++j) {
-        if (j % kTileKeys == 0) {
-            const float al = s_alpha[j / kTileKeys];
-            acc = al == 0.f ? 0.f : __fmul_rn(acc, al);
+    auto weigh = [&](bool final_pass) {  // thread d: feature d
+        float acc = 0.f;
+        for (int j = 0; threadIdx.x < dim && j < visible; ++j) {
+            if (j % kTileKeys == 0 && !final_pass) {
+                const float al = s_alpha[j / kTileKeys];
+                acc = al == 0.f ? 0.f : __fmul_rn(acc, al);
+            }
+            const float p = s_scores[j];
+            if (p != 0.f)
+                acc = __fmaf_rn(vc[(size_t)j * dim + threadIdx.x], p, acc);
         }
-        const float p = s_scores[j];
-        if (p != 0.f)
-            acc = __fmaf_rn(vc[(size_t)j * dim + threadIdx.x], p, acc);
+        return final_pass ? acc : __fdiv_rn(acc, s_total);
+    };
+    float o = weigh(false);
+    if (__syncthreads_or(threadIdx.x < dim && !(fabsf(o) <= FLT_MAX))) {
+        scores();
+        const float inv = __fdiv_rn(1.f, s_total);
+        for (int j = threadIdx.x; j < visible; j += kAttnThreads)
+            s_scores[j] = __fmul_rn(attn_prob(s_scores[j], s_max), inv);
+        __syncthreads();
+        o = weigh(true);
     }
-    out[((size_t)t * heads + h) * dim + threadIdx.x] = __fdiv_rn(acc, s_total);
+    if (threadIdx.x < dim)
+        out[((size_t)t * heads + h) * dim + threadIdx.x] = o;
 }
 
 // The same attention for a few query tokens (a decode step): a cluster of kSplitCtas blocks
@@ -506,7 +524,9 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
 // of eight 619 and 376 us, so sixteen, which need the non-portable opt-in.
 // The split depends on the number of visible keys alone, so a position given by the host and
 // one read on the device leave the same bits.  A probability of zero contributes nothing
-// (whatever the value row holds), as in attention_kernel; a NaN score reaches every feature.
+// (whatever the value row holds), as in attention_kernel: where a block's sums are not finite
+// -- a value row that is not, or values near the largest number added up before the division
+// -- every block runs P*V again on the final probabilities.  A NaN score reaches every feature.
 constexpr int kSplitCtas = 16;
 template <int DIM, int HR>
 struct SplitSmem {  // floats of dynamic shared memory before the scores
@@ -516,8 +536,9 @@ struct SplitSmem {  // floats of dynamic shared memory before the scores
     static constexpr int kSum = kMax + HR;                      // [HR] l
     static constexpr int kPart = kSum + HR;                     // [kAttnWarps][HR]
     static constexpr int kWeight = kPart + kAttnWarps * HR;     // [HR][kSplitCtas]
-    static constexpr int kTotal = kWeight + HR * kSplitCtas;    // [HR] 1 / sum follows
-    static constexpr int kScores = (kTotal + HR + 3) & ~3;      // [keys][HR]
+    static constexpr int kTotal = kWeight + HR * kSplitCtas;    // [HR] sum over the cluster
+    static constexpr int kOdd = kTotal + HR;                    // 1: not finite; [1]: any block's
+    static constexpr int kScores = (kOdd + 2 + 3) & ~3;         // [keys][HR]
 };
 template <int DIM, int HR>
 __global__ void __launch_bounds__(kAttnThreads)
@@ -538,6 +559,7 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
     float* s_part = s_dyn + S::kPart;
     float* s_weight = s_dyn + S::kWeight;
     float* s_total = s_dyn + S::kTotal;
+    float* s_odd = s_dyn + S::kOdd;
     float* s_sc = s_dyn + S::kScores;
     const int rep = heads / kv_heads, sets = (rep + HR - 1) / HR;
     const int kvh = blockIdx.y / sets, r0 = (blockIdx.y % sets) * HR;  // heads r0.. of the kv head
@@ -658,9 +680,11 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
         s_max[threadIdx.x] = m;
         s_sum[threadIdx.x] = sum;
     }
+    if (threadIdx.x == 0)
+        s_odd[0] = 0.f;
 
-    // ---- P*V ----
-    {
+    // ---- P*V; a second time, on final probabilities, if a sum is not finite ----
+    for (int pass = 0;; ++pass) {
         constexpr int kLanes = DIM / 4 < 32 ? DIM / 4 : 32;  // lanes per value row
         constexpr int kV4 = DIM / 4 / kLanes;                // float4 per lane
         constexpr int kKeys = 32 / kLanes;                   // keys per warp and step
@@ -721,38 +745,59 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
                     *reinterpret_cast<float4*>(s_acc + (warp * HR + h) * DIM +
                                                4 * (part + kLanes * i)) = o;
             }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < HR * DIM; i += kAttnThreads) {
-        float a = s_acc[i];
+        __syncthreads();
+        for (int i = threadIdx.x; i < HR * DIM; i += kAttnThreads) {
+            float a = s_acc[i];
 #pragma unroll
-        for (int w = 1; w < kAttnWarps; ++w)
-            a = __fadd_rn(a, s_acc[w * HR * DIM + i]);
-        s_out[i] = a;
+            for (int w = 1; w < kAttnWarps; ++w)
+                a = __fadd_rn(a, s_acc[w * HR * DIM + i]);
+            if (!(fabsf(a) <= FLT_MAX))
+                s_odd[0] = 1.f;
+            s_out[i] = a;
+        }
+        cluster.sync();
+        if (pass)
+            break;
+
+        // weights of the merge; warp h: head h's, lane c: block c of the cluster
+        if (warp < HR) {
+            const int c = lane % kSplitCtas;
+            const bool in = lane < kSplitCtas;
+            const float mc = in ? cluster.map_shared_rank(s_max, c)[warp] : -INFINITY;
+            const float lc = in ? cluster.map_shared_rank(s_sum, c)[warp] : 0.f;
+            const float odd = in ? cluster.map_shared_rank(s_odd, c)[0] : 0.f;
+            float top = mc;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+            const float w = (float)exp((double)__fsub_rn(mc, top));
+            float l = in ? __fmul_rn(w, lc) : 0.f;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+                l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, off));
+            if (in)
+                s_weight[warp * kSplitCtas + lane] = w;
+            if (lane == 0)
+                s_total[warp] = l;
+            const bool any = __any_sync(0xffffffffu, odd != 0.f);
+            if (threadIdx.x == 0)
+                s_odd[1] = any ? 1.f : 0.f;
+        }
+        __syncthreads();
+        if (s_odd[1] == 0.f)  // the same in every block of the cluster
+            break;
+        const float w = s_weight[my_head * kSplitCtas + rank];
+        const float inv = __fdiv_rn(1.f, s_total[my_head]);
+        for (int i = threadIdx.x; i < n * HR; i += kAttnThreads)
+            s_sc[i] = __fmul_rn(__fmul_rn(s_sc[i], w), inv);
+        __syncthreads();  // scores final, weights read
+        for (int i = threadIdx.x; i < HR * kSplitCtas; i += kAttnThreads)
+            s_weight[i] = 1.f;
+        if (threadIdx.x < HR)
+            s_total[threadIdx.x] = 1.f;
     }
-    cluster.sync();
 
     // ---- merge ----
-    if (warp < HR) {  // warp h: head h's weights, lane c: block c of the cluster
-        const float mc = lane < kSplitCtas ? cluster.map_shared_rank(s_max, lane % kSplitCtas)[warp]
-                                           : -INFINITY;
-        const float lc = lane < kSplitCtas ? cluster.map_shared_rank(s_sum, lane % kSplitCtas)[warp]
-                                           : 0.f;
-        float top = mc;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-        const float w = (float)exp((double)__fsub_rn(mc, top));
-        float l = lane < kSplitCtas ? __fmul_rn(w, lc) : 0.f;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, off));
-        if (lane < kSplitCtas)
-            s_weight[warp * kSplitCtas + lane] = w;
-        if (lane == 0)
-            s_total[warp] = l;
-    }
-    __syncthreads();
     constexpr int kShare = HR * DIM / kSplitCtas;  // outputs per block
     if (threadIdx.x < kShare) {
         const int i = rank * kShare + threadIdx.x, h = i / DIM;
@@ -767,7 +812,17 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
             if (w != 0.f)
                 a = __fmaf_rn(w, o[c], a);
         }
-        const float l = s_total[h];  // NaN if any score was
+        float l = s_total[h];  // NaN if any score was
+        if (!(fabsf(a) <= FLT_MAX)) {  // finite sums that overflow together
+            a = 0.f;
+#pragma unroll
+            for (int c = 0; c < kSplitCtas; ++c) {
+                const float w = __fdiv_rn(s_weight[h * kSplitCtas + c], l);
+                if (w != 0.f)
+                    a = __fmaf_rn(w, o[c], a);
+            }
+            l = 1.f;
+        }
         if (h < nh)
             out[row0 + i] = __fdiv_rn(a, l);
     }
@@ -788,9 +843,10 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
 //   softmax  four threads per row, eight keys each
 //   P*V      thread = 4 rows x DIM / 16 features, keys in ascending order
 // K of block b + 1 is copied (cp.async) under the softmax and P*V of block b, V of block b
-// under its scores.  A value row that is not finite must not reach a row that does not see it
-// (0 * inf): the copying threads look at what they fetched, and a block that holds such a
-// value runs P*V with the zero probabilities skipped.
+// under its scores.  A probability of zero contributes nothing (whatever the value row holds):
+// where an output is not finite -- a value row that is not, or values near the largest number
+// added up before the division -- the tile runs again with the rows' final maxima and sums,
+// probabilities of zero skipped, as attention_kernel has it.
 // Measured, eight layers of a prompt with 32 / 8 heads of 128 (all operators): 1500 tokens
 // 51.6 -> 18.8 ms (scores of that many keys did not fit the former tile kernel, and a block
 // per (token, head) read 37 GB of keys and values per layer); 256 tokens 3.47 -> 3.39 ms.
@@ -869,7 +925,6 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         const bool live = row_visible(row) > 0;
         cp_async16(s_q + row * P + 4 * c, q + (live ? row_offset(row) : 0) + 4 * c, live);
     }
-    copy_keys(s_k, kc, 0);  // Q and the first keys: one group
 
     // products: rows r_of(i) = ra + 16 i, keys kb + 16 j, features 4 kb + 64 i .. + 3
     const int ra = (warp >> 1) * 4 + (lane >> 3), kb = (warp & 1) * 8 + (lane & 7);
@@ -877,7 +932,10 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
     const int sr = threadIdx.x >> 2, sq = threadIdx.x & 3;
     const int s_vis = row_visible(sr);
     float m = -INFINITY, l = 0.f;
+    bool final_pass = false;  // m and 1 / l are the row's final ones, in m and l
     constexpr int NV = DIM / 64;
+    for (;;) {
+    copy_keys(s_k, kc, 0);  // the first time with Q: one group
     uint64_t acc[4][2 * NV];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -952,33 +1010,29 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                     mb = fmaxf(mb, e[i]);
             mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
             mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
-            const float alpha = j0 ? attn_rescale(m, mb) : 1.f;
-            m = mb;
+            const float alpha = j0 && !final_pass ? attn_rescale(m, mb) : 1.f;
+            m = mb;  // final_pass: as it was
 #pragma unroll
             for (int i = 0; i < 8; ++i)
                 e[i] = j0 + 8 * sq + i < s_vis ? attn_prob(e[i], m) : 0.f;
+            if (final_pass) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    e[i] = __fmul_rn(e[i], l);
+            }
             *reinterpret_cast<float4*>(row) = *reinterpret_cast<const float4*>(e);
             *reinterpret_cast<float4*>(row + 4) = *reinterpret_cast<const float4*>(e + 4);
             float sum = __fadd_rn(__fadd_rn(__fadd_rn(e[0], e[1]), __fadd_rn(e[2], e[3])),
                                   __fadd_rn(__fadd_rn(e[4], e[5]), __fadd_rn(e[6], e[7])));
             sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 1));
             sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 2));
-            l = __fadd_rn(__fmul_rn(l, alpha), sum);
+            if (!final_pass)
+                l = __fadd_rn(__fmul_rn(l, alpha), sum);
             if (sq == 0)
                 s_alpha[sr] = alpha;
         }
         cp_async_wait<1>();  // V of this block
-        bool odd_value = false;
-#pragma unroll
-        for (int u = 0; u < kCopies; ++u) {
-            const int i = threadIdx.x + kAttnThreads * u, key = i / kRow4, c = i % kRow4;
-            const float4 x = *reinterpret_cast<const float4*>(s_v + key * P + 4 * c);
-            // inf and NaN, times zero, are NaN
-            const float z = __fadd_rn(__fadd_rn(__fmul_rn(x.x, 0.f), __fmul_rn(x.y, 0.f)),
-                                      __fadd_rn(__fmul_rn(x.z, 0.f), __fmul_rn(x.w, 0.f)));
-            odd_value |= z != 0.f;
-        }
-        const bool careful = __syncthreads_or(odd_value);  // V, probabilities, factors in place
+        __syncthreads();  // V, probabilities, factors in place
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float al = s_alpha[ra + 16 * i];
@@ -989,7 +1043,7 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                     acc[i][c] = al == 0.f ? 0 : b2w4_mul2(acc[i][c], al2);
             }
         }
-        if (!careful) {
+        if (!final_pass) {
 #pragma unroll 2
             for (int j = 0; j < kTileKeys; j += 4) {
                 float4 p4[4];
@@ -1038,8 +1092,9 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         __syncthreads();  // V and the probabilities are consumed
     }
     if (sq == 0)
-        s_sum[sr] = l;
+        s_sum[sr] = final_pass ? 1.f : l;
     __syncthreads();
+    bool odd = false;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = ra + 16 * i;
@@ -1054,11 +1109,20 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                 o.y = __fdiv_rn(o.y, total);
                 o.z = __fdiv_rn(o.z, total);
                 o.w = __fdiv_rn(o.w, total);
+                // inf and NaN, times zero, are NaN
+                const float z = __fadd_rn(__fadd_rn(__fmul_rn(o.x, 0.f), __fmul_rn(o.y, 0.f)),
+                                          __fadd_rn(__fmul_rn(o.z, 0.f), __fmul_rn(o.w, 0.f)));
+                odd |= z != 0.f;
                 *reinterpret_cast<float4*>(out + row_offset(row) + 4 * kb + 64 * c) = o;
             }
         }
     }
     cp_async_wait<0>();
+    if (final_pass || !__syncthreads_or(odd))
+        return;
+    final_pass = true;
+    l = __fdiv_rn(1.f, l);
+    }
 }
 
 // A position counter on the device: *counter += by (after a decode step of a replayed graph),

@@ -394,7 +394,9 @@ def _staged(rng, heads, kv_heads, dim, keys, levels):
 
 
 @pytest.mark.parametrize("row", [False, True])
-@pytest.mark.parametrize("tokens,heads,kv_heads,dim", [(1, 4, 2, 80), (10, 4, 2, 80)])
+@pytest.mark.parametrize("tokens,heads,kv_heads,dim", [
+    (1, 2, 2, 64), (1, 4, 2, 64), (1, 8, 2, 128), (1, 2, 1, 256), (3, 3, 1, 128),
+    (12, 8, 2, 128), (12, 2, 2, 64), (9, 2, 1, 256), (1, 4, 2, 80), (10, 4, 2, 80)])
 def test_attention_ignores_value_rows_of_zero_probability(ctx, tokens, heads, kv_heads, dim, row):
     """Scores of 0, 80 and 160 in the three parts of the cache: a key of the first part has
     the probability e^-160 = 0, but e^-80 > 0 against the middle part, and 1 against its own
