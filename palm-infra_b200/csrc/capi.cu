@@ -99,6 +99,9 @@ int b2w4_ctx_create(int device, b2w4_ctx** out) {
     const char* at = getenv("B2W4_ATTN");  // debug: "row" keeps the one-row attention kernel
     if (at && at[0] == 'r')
         ctx->attn_tiles = false;
+    const char* ac = getenv("B2W4_ATTN_CLUSTER");  // tuning: blocks that share a query's keys
+    if (ac && atoi(ac) >= 0)
+        ctx->attn_cluster = std::min(atoi(ac), 16);
     const char* gmr = getenv("B2W4_GEMV_MAX_ROWS");  // tuning/debug: rows kept on the GEMV
     if (gmr && atoi(gmr) > 0)
         ctx->gemv_max_rows = atoi(gmr);

@@ -11,6 +11,7 @@
 #include "b200w4_internal.cuh"
 
 #include <cfloat>
+#include <type_traits>
 
 #include <cooperative_groups.h>
 
@@ -505,12 +506,11 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
         out[((size_t)t * heads + h) * dim + threadIdx.x] = o;
 }
 
-// The same attention for a few query tokens (a decode step): a cluster of kSplitCtas blocks
-// splits the visible keys of one (token, kv head, up to HR of its query heads), so a step
-// fills the chip instead of one block per head, and the query heads of a kv head read its
-// keys and values once.  What bounds it: bytes in flight -- a key and value row are read once
-// and used HR times -- until the cache is short, where it is the chain load, exchange, exp,
-// load, exchange.
+// The same attention for few query tokens (a decode step, a short run): one block per (token,
+// kv head, up to HR of its query heads), or a cluster of `ctas` blocks that splits the visible
+// keys, so that a step fills the chip.  The query heads of a kv head read its keys and values
+// once.  What bounds it: bytes in flight -- a key and value row are read once and used HR times
+// -- until the cache is short, where it is the chain load, exchange, exp, load, exchange.
 //   scores   eight lanes per key hold four features each of every 32, a warp has 4 (KI)
 //            x 4 keys' loads in flight; products in pairs (fma.rn.f32x2), then a butterfly
 //            over the eight lanes that halves the items held at each level
@@ -519,33 +519,36 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
 //            added through shared memory
 //   merge    block r adds its share of the features over the cluster (distributed shared
 //            memory): out = sum_c w_c o_c / sum_c w_c l_c, w_c = exp(m_c - max m)
-// Measured, a step of eight layers with 32 / 8 heads of 128: 6000 keys 3447 -> 522 us (one
-// block per head: 32 of 148 SMs, every key read four times), 300 keys 501 -> 384 us; clusters
-// of eight 619 and 376 us, so sixteen, which need the non-portable opt-in.
-// The split depends on the number of visible keys alone, so a position given by the host and
-// one read on the device leave the same bits.  A probability of zero contributes nothing
-// (whatever the value row holds), as in attention_kernel: where a block's sums are not finite
-// -- a value row that is not, or values near the largest number added up before the division
-// -- every block runs P*V again on the final probabilities.  A NaN score reaches every feature.
-constexpr int kSplitCtas = 16;
+// Up to `one_range` visible keys the first block takes them all and the others leave: a cluster
+// costs more than it gives there (a step at position 0, 32 / 8 heads of 128: 3.1 us with one
+// block per head, 6.2 split over sixteen, 3.3 as it is; seven tokens 3.8, 23.4, 3.5).
+// Measured, a step with 32 / 8 heads of 128 behind 6000 keys: 313 us with one block per head
+// (32 of 148 SMs, every key read four times), 22.6 us over sixteen blocks, 34 over eight.
+// The split depends on the number of visible keys and the call's sizes, so a position given by
+// the host and one read on the device leave the same bits.  A probability of zero contributes
+// nothing (whatever the value row holds), as in attention_kernel: where a block's sums are not
+// finite -- a value row that is not, or values near the largest number added up before the
+// division -- every block runs P*V again on the final probabilities.  A NaN score reaches every
+// feature.
+constexpr int kMaxRanges = 16;
 template <int DIM, int HR>
 struct SplitSmem {  // floats of dynamic shared memory before the scores
     static constexpr int kAcc = 0;                              // [kAttnWarps][HR][DIM]
     static constexpr int kOut = kAcc + kAttnWarps * HR * DIM;   // [HR][DIM]
     static constexpr int kMax = kOut + HR * DIM;                // [HR] m, read by the cluster
     static constexpr int kSum = kMax + HR;                      // [HR] l
-    static constexpr int kPart = kSum + HR;                     // [kAttnWarps][HR]
-    static constexpr int kWeight = kPart + kAttnWarps * HR;     // [HR][kSplitCtas]
-    static constexpr int kTotal = kWeight + HR * kSplitCtas;    // [HR] sum over the cluster
+    static constexpr int kPart = kSum + HR;                     // [2][kAttnWarps][HR]
+    static constexpr int kWeight = kPart + 2 * kAttnWarps * HR;  // [HR][kMaxRanges]
+    static constexpr int kTotal = kWeight + HR * kMaxRanges;    // [HR] sum over the cluster
     static constexpr int kOdd = kTotal + HR;                    // 1: not finite; [1]: any block's
     static constexpr int kScores = (kOdd + 2 + 3) & ~3;         // [keys][HR]
 };
 template <int DIM, int HR>
-__global__ void __launch_bounds__(kAttnThreads)
+__global__ void __launch_bounds__(kAttnThreads, 2)
 attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                        const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
                        int heads, int kv_heads, int past0, const int* __restrict__ past_dev,
-                       int capacity, float scale) {
+                       int capacity, float scale, int ctas, int one_range) {
     b2w4_pdl_chain_entry();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -565,7 +568,10 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
     const int kvh = blockIdx.y / sets, r0 = (blockIdx.y % sets) * HR;  // heads r0.. of the kv head
     const int nh = min(HR, rep - r0), t = blockIdx.z, rank = blockIdx.x;
     const int visible = past + t + 1;
-    const int per = (visible + kSplitCtas - 1) / kSplitCtas;
+    const int ranges = visible <= one_range ? 1 : ctas;
+    if (rank >= ranges)  // a barrier of the cluster waits for the blocks that are still there
+        return;
+    const int per = (visible + ranges - 1) / ranges;
     const int j0 = min(rank * per, visible), n = min(per, visible - j0);
     const size_t row0 = ((size_t)t * heads + (size_t)kvh * rep + r0) * DIM;
     const float* kc = k_cache + ((size_t)kvh * capacity + j0) * DIM;
@@ -575,8 +581,6 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
     // ---- scores ----
     {
         constexpr int kF4 = DIM / 32;             // float4 of a row per lane
-        constexpr int KI = DIM > 128 ? 2 : 4;     // keys per lane group in flight
-        constexpr int kItems = KI * HR;
         const int part = lane & 7, sub = lane >> 3;
         uint64_t qv[HR][2 * kF4];
 #pragma unroll
@@ -589,57 +593,66 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
                 qv[h][2 * i] = b2w4_pack2(x.x, x.y);
                 qv[h][2 * i + 1] = b2w4_pack2(x.z, x.w);
             }
-        for (int j = warp * 4 * KI; j < n; j += kAttnWarps * 4 * KI) {
-            float4 kr[KI][kF4];
+        // keys per lane group in flight; few keys: one, so that all warps take part
+        auto score = [&](auto in_flight) {
+            constexpr int KI = decltype(in_flight)::value;
+            constexpr int kItems = KI * HR;
+            for (int j = warp * 4 * KI; j < n; j += kAttnWarps * 4 * KI) {
+                float4 kr[KI][kF4];
 #pragma unroll
-            for (int it = 0; it < KI; ++it)
-#pragma unroll
-                for (int i = 0; i < kF4; ++i) {
-                    const int key = min(j + it * 4 + sub, n - 1);  // past the end: dropped below
-                    kr[it][i] = *reinterpret_cast<const float4*>(kc + (size_t)key * DIM + 32 * i +
-                                                                 4 * part);
-                }
-            float v[kItems];  // item it * HR + h
-#pragma unroll
-            for (int it = 0; it < KI; ++it)
-#pragma unroll
-                for (int h = 0; h < HR; ++h) {
-                    uint64_t a = 0, b = 0;  // (0.f, 0.f)
+                for (int it = 0; it < KI; ++it)
 #pragma unroll
                     for (int i = 0; i < kF4; ++i) {
-                        a = b2w4_fma2(qv[h][2 * i], b2w4_pack2(kr[it][i].x, kr[it][i].y), a);
-                        b = b2w4_fma2(qv[h][2 * i + 1], b2w4_pack2(kr[it][i].z, kr[it][i].w), b);
+                        const int key = min(j + it * 4 + sub, n - 1);  // past the end: dropped below
+                        kr[it][i] = *reinterpret_cast<const float4*>(kc + (size_t)key * DIM + 32 * i +
+                                                                     4 * part);
                     }
-                    float a0, a1, b0, b1;
-                    b2w4_unpack2(a, a0, a1);
-                    b2w4_unpack2(b, b0, b1);
-                    v[it * HR + h] = __fadd_rn(__fadd_rn(a0, b0), __fadd_rn(a1, b1));
+                float v[kItems];  // item it * HR + h
+#pragma unroll
+                for (int it = 0; it < KI; ++it)
+#pragma unroll
+                    for (int h = 0; h < HR; ++h) {
+                        uint64_t a = 0, b = 0;  // (0.f, 0.f)
+#pragma unroll
+                        for (int i = 0; i < kF4; ++i) {
+                            a = b2w4_fma2(qv[h][2 * i], b2w4_pack2(kr[it][i].x, kr[it][i].y), a);
+                            b = b2w4_fma2(qv[h][2 * i + 1], b2w4_pack2(kr[it][i].z, kr[it][i].w), b);
+                        }
+                        float a0, a1, b0, b1;
+                        b2w4_unpack2(a, a0, a1);
+                        b2w4_unpack2(b, b0, b1);
+                        v[it * HR + h] = __fadd_rn(__fadd_rn(a0, b0), __fadd_rn(a1, b1));
+                    }
+                int first = 0;  // the lane's first item
+                constexpr int kLevel[3] = {4, 2, 1};
+#pragma unroll
+                for (int l = 0; l < 3; ++l) {
+                    const int off = kLevel[l], have = kItems >> l;
+                    if (have > 1) {
+                        const bool up = lane & off;
+#pragma unroll
+                        for (int i = 0; i < have / 2; ++i) {
+                            const float send = up ? v[i] : v[i + have / 2];
+                            const float keep = up ? v[i + have / 2] : v[i];
+                            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, off));
+                        }
+                        first += up ? have / 2 : 0;
+                    } else {
+                        v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
+                    }
                 }
-            int first = 0;  // the lane's first item
-            constexpr int kLevel[3] = {4, 2, 1};
 #pragma unroll
-            for (int l = 0; l < 3; ++l) {
-                const int off = kLevel[l], have = kItems >> l;
-                if (have > 1) {
-                    const bool up = lane & off;
-#pragma unroll
-                    for (int i = 0; i < have / 2; ++i) {
-                        const float send = up ? v[i] : v[i + have / 2];
-                        const float keep = up ? v[i + have / 2] : v[i];
-                        v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, off));
-                    }
-                    first += up ? have / 2 : 0;
-                } else {
-                    v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
+                for (int i = 0; i < (kItems > 8 ? kItems / 8 : 1); ++i) {
+                    const int item = first + i, key = j + (item / HR) * 4 + sub;
+                    if (key < n)
+                        s_sc[key * HR + item % HR] = __fmul_rn(v[i], scale);
                 }
             }
-#pragma unroll
-            for (int i = 0; i < (kItems > 8 ? kItems / 8 : 1); ++i) {
-                const int item = first + i, key = j + (item / HR) * 4 + sub;
-                if (key < n)
-                    s_sc[key * HR + item % HR] = __fmul_rn(v[i], scale);
-            }
-        }
+        };
+        if (n <= 4 * kAttnWarps)
+            score(std::integral_constant<int, 1>());
+        else
+            score(std::integral_constant<int, (DIM > 128 ? 2 : 4)>());
     }
     __syncthreads();
 
@@ -651,15 +664,15 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
             const float y = __shfl_xor_sync(0xffffffffu, x, off);
             x = maximum ? fmaxf(x, y) : __fadd_rn(x, y);
         }
+        float* parts = s_part + (maximum ? 0 : kAttnWarps * HR);
         if (lane < HR)
-            s_part[warp * HR + lane] = x;
+            parts[warp * HR + lane] = x;
         __syncthreads();
-        x = s_part[my_head];
+        x = parts[my_head];
 #pragma unroll
         for (int w = 1; w < kAttnWarps; ++w)
-            x = maximum ? fmaxf(x, s_part[w * HR + my_head])
-                        : __fadd_rn(x, s_part[w * HR + my_head]);
-        __syncthreads();
+            x = maximum ? fmaxf(x, parts[w * HR + my_head])
+                        : __fadd_rn(x, parts[w * HR + my_head]);
         return x;
     };
     float m = -INFINITY;
@@ -746,23 +759,42 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
                                                4 * (part + kLanes * i)) = o;
             }
         __syncthreads();
+        bool odd = false;
         for (int i = threadIdx.x; i < HR * DIM; i += kAttnThreads) {
             float a = s_acc[i];
 #pragma unroll
             for (int w = 1; w < kAttnWarps; ++w)
                 a = __fadd_rn(a, s_acc[w * HR * DIM + i]);
-            if (!(fabsf(a) <= FLT_MAX))
-                s_odd[0] = 1.f;
-            s_out[i] = a;
+            const int h = i / DIM;
+            if (ranges == 1) {
+                if (!pass)
+                    a = __fdiv_rn(a, s_sum[h]);
+                if (h < nh)
+                    out[row0 + i] = a;
+            } else {
+                s_out[i] = a;
+            }
+            odd |= !(fabsf(a) <= FLT_MAX);
         }
+        if (ranges == 1) {
+            if (pass || !__syncthreads_or(odd))
+                return;
+            const float inv = __fdiv_rn(1.f, s_sum[my_head]);
+            for (int i = threadIdx.x; i < n * HR; i += kAttnThreads)
+                s_sc[i] = __fmul_rn(s_sc[i], inv);
+            __syncthreads();
+            continue;
+        }
+        if (odd)
+            s_odd[0] = 1.f;
         cluster.sync();
         if (pass)
             break;
 
         // weights of the merge; warp h: head h's, lane c: block c of the cluster
         if (warp < HR) {
-            const int c = lane % kSplitCtas;
-            const bool in = lane < kSplitCtas;
+            const int c = min(lane, ctas - 1);
+            const bool in = lane < ctas;
             const float mc = in ? cluster.map_shared_rank(s_max, c)[warp] : -INFINITY;
             const float lc = in ? cluster.map_shared_rank(s_sum, c)[warp] : 0.f;
             const float odd = in ? cluster.map_shared_rank(s_odd, c)[0] : 0.f;
@@ -776,7 +808,7 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
             for (int off = 16; off > 0; off >>= 1)
                 l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, off));
             if (in)
-                s_weight[warp * kSplitCtas + lane] = w;
+                s_weight[warp * kMaxRanges + lane] = w;
             if (lane == 0)
                 s_total[warp] = l;
             const bool any = __any_sync(0xffffffffu, odd != 0.f);
@@ -786,41 +818,44 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
         __syncthreads();
         if (s_odd[1] == 0.f)  // the same in every block of the cluster
             break;
-        const float w = s_weight[my_head * kSplitCtas + rank];
+        const float w = s_weight[my_head * kMaxRanges + rank];
         const float inv = __fdiv_rn(1.f, s_total[my_head]);
         for (int i = threadIdx.x; i < n * HR; i += kAttnThreads)
             s_sc[i] = __fmul_rn(__fmul_rn(s_sc[i], w), inv);
         __syncthreads();  // scores final, weights read
-        for (int i = threadIdx.x; i < HR * kSplitCtas; i += kAttnThreads)
+        for (int i = threadIdx.x; i < HR * kMaxRanges; i += kAttnThreads)
             s_weight[i] = 1.f;
         if (threadIdx.x < HR)
             s_total[threadIdx.x] = 1.f;
     }
 
     // ---- merge ----
-    constexpr int kShare = HR * DIM / kSplitCtas;  // outputs per block
-    if (threadIdx.x < kShare) {
-        const int i = rank * kShare + threadIdx.x, h = i / DIM;
-        float o[kSplitCtas];
+    const int share = HR * DIM / ctas;  // outputs per block, a power of two
+    for (int i = rank * share + threadIdx.x; i < (rank + 1) * share; i += kAttnThreads) {
+        const int h = i / DIM;
+        float o[kMaxRanges];
 #pragma unroll
-        for (int c = 0; c < kSplitCtas; ++c)
-            o[c] = cluster.map_shared_rank(s_out, c)[i];
+        for (int c = 0; c < kMaxRanges; ++c)
+            if (c < ctas)
+                o[c] = cluster.map_shared_rank(s_out, c)[i];
         float a = 0.f;
 #pragma unroll
-        for (int c = 0; c < kSplitCtas; ++c) {
-            const float w = s_weight[h * kSplitCtas + c];
-            if (w != 0.f)
-                a = __fmaf_rn(w, o[c], a);
-        }
+        for (int c = 0; c < kMaxRanges; ++c)
+            if (c < ctas) {
+                const float w = s_weight[h * kMaxRanges + c];
+                if (w != 0.f)
+                    a = __fmaf_rn(w, o[c], a);
+            }
         float l = s_total[h];  // NaN if any score was
         if (!(fabsf(a) <= FLT_MAX)) {  // finite sums that overflow together
             a = 0.f;
 #pragma unroll
-            for (int c = 0; c < kSplitCtas; ++c) {
-                const float w = __fdiv_rn(s_weight[h * kSplitCtas + c], l);
-                if (w != 0.f)
-                    a = __fmaf_rn(w, o[c], a);
-            }
+            for (int c = 0; c < kMaxRanges; ++c)
+                if (c < ctas) {
+                    const float w = __fdiv_rn(s_weight[h * kMaxRanges + c], l);
+                    if (w != 0.f)
+                        a = __fmaf_rn(w, o[c], a);
+                }
             l = 1.f;
         }
         if (h < nh)
@@ -1162,6 +1197,162 @@ __global__ void embed_rows_kernel(const __half* __restrict__ table, const int32_
     out[(size_t)r * ldo + d] = __half2float(table[(size_t)ids[r] * dim + d]);
 }
 
+// ---- which kernel a call takes, and its launch ----
+enum AttnForm { ATTN_ROW, ATTN_PLAIN, ATTN_SPLIT, ATTN_TILE };
+struct AttnPlan {
+    int form;
+    int rows;       // ATTN_TILE: rows per tile
+    int ctas;       // ATTN_SPLIT: blocks per cluster
+    int one_range;  // ATTN_SPLIT: visible keys up to which one block takes them all
+};
+struct AttnArgs {
+    const float *q, *k_cache, *v_cache;
+    float* out;
+    int tokens, heads, kv_heads, past;
+    const int* past_dev;
+    int capacity;
+    float scale;
+};
+
+// query heads of a kv head that a block of the split kernel serves
+int split_heads(int dim, int rep) { return dim == 256 ? min(rep, 2) : rep >= 3 ? 4 : rep; }
+
+// A call's form depends on its sizes and the cache's capacity, not on the position, so that a
+// position given by the host and one read on the device leave the same bits.  The lines,
+// times on a B200:
+//   few rows   `groups` blocks with all keys (one_range), or clusters that split them.  A
+//              cluster costs 2 to 3 us, more where there are many; 32 / 8 heads of 128, one
+//              block against clusters: one token, 64 keys 5.1 / 5.6 us, 160 keys 7.1 / 5.8; 16
+//              tokens, 300 keys 12.6 / 15.7, 1000 keys 36 / 26.  The cluster sizes keep all of
+//              them resident at once: sixteen against eight, one token, 6000 keys 22.6 / 34.1,
+//              seven tokens 73 / 62, with four 59.
+AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int capacity,
+                   bool aligned, bool row_only, int max_cluster, int sm_count) {
+    const int rep = heads / kv_heads;
+    AttnPlan p = {ATTN_ROW, 0, 0, 0};
+    if (dim != 64 && dim != 128 && dim != 256)
+        return p;
+    if (row_only) {
+        p.form = ATTN_PLAIN;
+        return p;
+    }
+    const int hr = split_heads(dim, rep);
+    const long groups = (long)tokens * kv_heads * ((rep + hr - 1) / hr);
+    if (aligned && tokens < 8 && groups / tokens <= 65535) {
+        p.form = ATTN_SPLIT;
+        p.ctas = capacity > 1024 && groups * 32 <= 3l * sm_count ? 16
+                 : groups * 8 <= 2l * sm_count                   ? 8
+                                                                 : 4;
+        p.one_range = (int)min(4096l, max(p.ctas == 16 ? 96l : 128l, groups * groups / 32));
+        while (p.ctas > max_cluster)
+            p.ctas /= 2;
+        return p;
+    }
+    if (rep > kTileRows || tokens < 8 || !aligned)
+        return p;
+    p.form = ATTN_TILE;
+    p.rows = kTileRows;
+    return p;
+}
+
+// The largest cluster of the kernel, up to `want` blocks, that the device can hold (a slice of
+// it may not have sixteen or eight multiprocessors side by side); 0: none.
+template <typename Kernel>
+int placeable_cluster(b2w4_ctx* ctx, Kernel kern, int want, size_t smem) {
+    for (int c = want; c > 1; c /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(kAttnThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = c;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
+            return c;
+        (void)cudaGetLastError();
+    }
+    return 0;
+}
+
+template <int DIM, int HR>
+int launch_split_hr(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
+                    bool* placed) {
+    static b2w4_smem_optin cfg, wide, most;  // most: largest cluster + 1, per device
+    auto kern = attention_split_kernel<DIM, HR>;
+    const int rep = a.heads / a.kv_heads;
+    const bool one = keys <= plan.one_range;
+    B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, kern, wide));
+    size_t& largest = most.bytes[ctx->device];
+    auto bytes = [&](int ctas) {
+        const int range = max((keys + ctas - 1) / ctas, min(keys, plan.one_range));
+        return sizeof(float) * (SplitSmem<DIM, HR>::kScores + (size_t)range * HR);
+    };
+    if (!one && !largest) {
+        const size_t smem = sizeof(float) * SplitSmem<DIM, HR>::kScores + 64 * 1024;
+        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, cfg));
+        largest = 1 + placeable_cluster(ctx, kern, kMaxRanges, smem);
+    }
+    const int ctas = one ? 1 : min(plan.ctas, (int)largest - 1);
+    if (ctas < (one ? 1 : 2) || bytes(ctas) > 220 * 1024)
+        return B2W4_OK;  // not placed
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, bytes(ctas), cfg));
+    const dim3 grid(ctas, a.kv_heads * ((rep + HR - 1) / HR), a.tokens);
+    if (one)
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), bytes(1),
+                                           ctx->stream, a.q, a.k_cache, a.v_cache, a.out,
+                                           a.tokens, a.heads, a.kv_heads, a.past, a.past_dev,
+                                           a.capacity, a.scale, 1, plan.one_range));
+    else
+        B2W4_CUDA(ctx, b2w4_launch_chained_cluster(
+                           ctx->pdl, kern, grid, dim3(kAttnThreads), ctas, bytes(ctas),
+                           ctx->stream, a.q, a.k_cache, a.v_cache, a.out, a.tokens, a.heads,
+                           a.kv_heads, a.past, a.past_dev, a.capacity, a.scale, ctas,
+                           plan.one_range));
+    ctx->launches++;
+    *placed = true;
+    return B2W4_OK;
+}
+
+int launch_split(b2w4_ctx* ctx, const AttnArgs& a, int dim, int keys, const AttnPlan& plan,
+                 bool* placed) {
+    const int hr = split_heads(dim, a.heads / a.kv_heads);
+    switch (dim * 8 + hr) {
+    case 64 * 8 + 1: return launch_split_hr<64, 1>(ctx, a, keys, plan, placed);
+    case 64 * 8 + 2: return launch_split_hr<64, 2>(ctx, a, keys, plan, placed);
+    case 64 * 8 + 4: return launch_split_hr<64, 4>(ctx, a, keys, plan, placed);
+    case 128 * 8 + 1: return launch_split_hr<128, 1>(ctx, a, keys, plan, placed);
+    case 128 * 8 + 2: return launch_split_hr<128, 2>(ctx, a, keys, plan, placed);
+    case 128 * 8 + 4: return launch_split_hr<128, 4>(ctx, a, keys, plan, placed);
+    case 256 * 8 + 1: return launch_split_hr<256, 1>(ctx, a, keys, plan, placed);
+    default: return launch_split_hr<256, 2>(ctx, a, keys, plan, placed);
+    }
+}
+
+template <int DIM>
+int launch_tile_dim(b2w4_ctx* ctx, const AttnArgs& a) {
+    static b2w4_smem_optin cfg;
+    const size_t smem = TileSmem<DIM>::kBytes;
+    auto kern = attention_tile_kernel<DIM>;
+    const int tq = kTileRows / (a.heads / a.kv_heads);
+    const dim3 grid((a.tokens + tq - 1) / tq, a.kv_heads);
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, cfg));
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), smem,
+                                       ctx->stream, a.q, a.k_cache, a.v_cache, a.out, a.tokens,
+                                       a.heads, a.kv_heads, a.past, a.past_dev, a.capacity,
+                                       a.scale, tq));
+    ctx->launches++;
+    return B2W4_OK;
+}
+int launch_tile(b2w4_ctx* ctx, const AttnArgs& a, int dim) {
+    return dim == 64    ? launch_tile_dim<64>(ctx, a)
+           : dim == 128 ? launch_tile_dim<128>(ctx, a)
+                        : launch_tile_dim<256>(ctx, a);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1264,17 +1455,11 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
                          tokens, past, capacity, heads, kv_heads);
     const int keys = past_dev ? capacity : past + tokens;  // position on the device: sized
                                                            // for a full cache
-    const int rep = heads / kv_heads;
-    // Head sizes of 64, 128 and 256 with 16-byte aligned rows: up to seven query tokens go to
-    // the cluster kernel (it splits the keys, so few rows still fill the chip), a run of eight
-    // or more to the tile kernel (it shares keys and values among 64 rows).  The rest: one
-    // block per (token, head).
-    const bool wide = (dim == 64 || dim == 128 || dim == 256) &&
-                      !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev |
-                         (uintptr_t)out_dev) & 15);
-    const bool split = wide && ctx->attn_tiles && tokens < 8;
-    const bool tiles = wide && ctx->attn_tiles && !split && rep <= kTileRows;
-    const bool plain = !ctx->attn_tiles && (dim == 64 || dim == 128 || dim == 256);
+    const bool aligned = !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev |
+                            (uintptr_t)out_dev) & 15);
+    const AttnPlan plan = attn_plan(tokens, heads, kv_heads, dim,
+                                    past_dev ? capacity - tokens : past, capacity, aligned,
+                                    !ctx->attn_tiles, ctx->attn_cluster, ctx->sm_count);
     const int score_slots = (keys + 3) & ~3;
     if (sizeof(float) * ((size_t)score_slots + kAttnStage) > 200 * 1024)
         return b2w4_fail(ctx, B2W4_E_INVALID, "attention: %d keys exceed the score buffer", keys);
@@ -1286,78 +1471,40 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
                                            tokens, kv_heads, dim, past, past_dev, capacity));
         ctx->launches++;
     }
-    const float* kc = k_cache_dev;
-    const float* vc = v_cache_dev;
-    if (split) {
-        const int per = (keys + kSplitCtas - 1) / kSplitCtas;
-#define B2W4_SPLIT(D, HR)                                                                      \
-    do {                                                                                       \
-        static b2w4_smem_optin cfg;                                                            \
-        static b2w4_smem_optin wide;                                                           \
-        const size_t smem = sizeof(float) * (SplitSmem<D, HR>::kScores + (size_t)per * HR);    \
-        const dim3 grid(kSplitCtas, kv_heads * ((rep + HR - 1) / HR), tokens);                 \
-        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, attention_split_kernel<D, HR>, smem, cfg));       \
-        B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, attention_split_kernel<D, HR>, wide));         \
-        B2W4_CUDA(ctx, b2w4_launch_chained_cluster(                                            \
-                           ctx->pdl, attention_split_kernel<D, HR>, grid, dim3(kAttnThreads),  \
-                           kSplitCtas, smem, ctx->stream, q_dev, kc, vc, out_dev, tokens,      \
-                           heads, kv_heads, past, past_dev, capacity, scale));                 \
-    } while (0)
-        if (dim == 256) {
-            if (rep >= 2)
-                B2W4_SPLIT(256, 2);
-            else
-                B2W4_SPLIT(256, 1);
-        } else if (dim == 128) {
-            if (rep >= 3)
-                B2W4_SPLIT(128, 4);
-            else if (rep == 2)
-                B2W4_SPLIT(128, 2);
-            else
-                B2W4_SPLIT(128, 1);
-        } else {
-            if (rep >= 3)
-                B2W4_SPLIT(64, 4);
-            else if (rep == 2)
-                B2W4_SPLIT(64, 2);
-            else
-                B2W4_SPLIT(64, 1);
-        }
-#undef B2W4_SPLIT
-    } else if (tiles) {
-        const int tq = kTileRows / rep;
-        const dim3 grid((tokens + tq - 1) / tq, kv_heads);
-#define B2W4_TILE(D)                                                                          \
-    do {                                                                                      \
-        static b2w4_smem_optin cfg;                                                           \
-        const size_t smem = TileSmem<D>::kBytes;                                              \
-        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, attention_tile_kernel<D>, smem, cfg));           \
-        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, attention_tile_kernel<D>, grid,          \
-                                           dim3(kAttnThreads), smem, ctx->stream, q_dev, kc,  \
-                                           vc, out_dev, tokens, heads, kv_heads, past,        \
-                                           past_dev, capacity, scale, tq));                   \
-    } while (0)
-        if (dim == 64)
-            B2W4_TILE(64);
-        else if (dim == 128)
-            B2W4_TILE(128);
-        else
-            B2W4_TILE(256);
-#undef B2W4_TILE
-    } else {
-        static b2w4_smem_optin configured[2];
-        auto kern = plain ? attention_plain_kernel : attention_kernel;
-        const size_t row_smem =
-            sizeof(float) * ((size_t)score_slots +
-                             (plain ? (keys + kTileKeys - 1) / kTileKeys : kAttnStage));
-        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, row_smem, configured[plain]));
-        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(tokens * heads),
-                                           dim3(kAttnThreads), row_smem, ctx->stream, q_dev, kc,
-                                           vc, out_dev, tokens, heads, kv_heads, dim, past,
-                                           past_dev, capacity, scale, score_slots));
+    const AttnArgs a = {q_dev, k_cache_dev, v_cache_dev, out_dev, tokens, heads, kv_heads, past,
+                        past_dev, capacity, scale};
+    if (plan.form == ATTN_SPLIT) {
+        bool placed = false;
+        const int rc = launch_split(ctx, a, dim, keys, plan, &placed);
+        if (rc != B2W4_OK || placed)
+            return rc;
     }
+    if (plan.form == ATTN_TILE)
+        return launch_tile(ctx, a, dim);
+    static b2w4_smem_optin configured[2];
+    const bool plain = plan.form == ATTN_PLAIN;
+    auto kern = plain ? attention_plain_kernel : attention_kernel;
+    const size_t row_smem =
+        sizeof(float) *
+        ((size_t)score_slots + (plain ? (keys + kTileKeys - 1) / kTileKeys : kAttnStage));
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, row_smem, configured[plain]));
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(tokens * heads), dim3(kAttnThreads),
+                                       row_smem, ctx->stream, q_dev, k_cache_dev, v_cache_dev,
+                                       out_dev, tokens, heads, kv_heads, dim, past, past_dev,
+                                       capacity, scale, score_slots));
     ctx->launches++;
     return B2W4_OK;
+}
+
+// What attn_plan says, for checks without a device: the form; out: rows, ctas, one_range.
+int b2w4_attention_plan(int tokens, int heads, int kv_heads, int dim, int past, int capacity,
+                        int aligned, int row_only, int max_cluster, int sm_count, int* out) {
+    const AttnPlan p = attn_plan(tokens, heads, kv_heads, dim, past, capacity, aligned, row_only,
+                                 max_cluster, sm_count);
+    out[0] = p.rows;
+    out[1] = p.ctas;
+    out[2] = p.one_range;
+    return p.form;
 }
 
 int b2w4_qkv_prepare(b2w4_ctx* ctx, const float* qkv_dev, int ld, int tokens, int heads,

@@ -443,3 +443,46 @@ def test_attention_ignores_value_rows_of_zero_probability(ctx, tokens, heads, kv
     assert np.isnan(run()).all()
     if row:
         c.close()
+
+
+@pytest.mark.parametrize("cluster", [0, 1, 3, 4, 8, 16])
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [
+    (1, 94, 8, 2, 64), (3, 94, 4, 2, 128), (2, 126, 3, 3, 128), (7, 126, 6, 1, 256),
+    (1, 1500, 8, 2, 128), (5, 700, 5, 5, 64)])
+def test_split_attention_on_either_side_of_one_range(ctx, tokens, past, heads, kv_heads, dim,
+                                                     cluster):
+    """Runs whose tokens see 95 .. 133 keys, the last counts that one block takes alone and the
+    first that a cluster splits, and longer ones; clusters of every size that a device may
+    allow, and none (one block per (token, head)).  Position on the host or on the device: the
+    same bits.  Tolerance as for the split kernel."""
+    import os
+    import torch
+    capacity, scale = 1600, dim ** -0.5
+    rng = np.random.default_rng(past + dim + cluster)
+    q = rng.normal(0, 1, (tokens, heads, dim)).astype(np.float32)
+    k_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    v_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    kc = np.zeros((kv_heads, capacity, dim), dtype=np.float32)
+    vc = np.full((kv_heads, capacity, dim), np.nan, dtype=np.float32)
+    kc[:, :past + tokens] = k_all.transpose(1, 0, 2)
+    vc[:, :past + tokens] = v_all.transpose(1, 0, 2)
+    kcd, vcd, qd = _dev(kc), _dev(vc), _dev(q)
+    os.environ["B2W4_ATTN_CLUSTER"] = str(cluster)
+    try:
+        c = pkg.capi.Context(0)
+    finally:
+        del os.environ["B2W4_ATTN_CLUSTER"]
+    outs = []
+    for past_dev in (None, torch.full((1,), past, dtype=torch.int32, device="cuda")):
+        out = torch.zeros((tokens, heads, dim), dtype=torch.float32, device="cuda")
+        c.attention(qd, None, None, kcd, vcd, out, tokens, heads, kv_heads, dim,
+                    past if past_dev is None else 0, capacity, scale, past_dev)
+        c.sync()
+        outs.append(out.cpu().numpy())
+    c.close()
+    want = _attention_fp64(q, k_all, v_all, heads, kv_heads, past, scale)
+    assert rel_l2(outs[0], want) < 1e-5
+    if cluster >= 2:
+        assert outs[1].tobytes() == outs[0].tobytes()
+    else:  # few keys known to the host need no cluster; the device's position does
+        assert rel_l2(outs[1], want) < 1e-5
