@@ -865,37 +865,37 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
 }
 
 // The same attention for a run of new tokens (prefill): one block per (kv head, tile of query
-// tokens) serves every query head of that kv head -- up to kTileRows (token, head) rows --
-// against blocks of kTileKeys keys, with a running softmax (attention_plain_kernel's arithmetic,
-// operation for operation: the same bits).  Nothing grows with the
-// number of keys: any context length takes this form.
+// tokens) serves every query head of that kv head -- up to ROWS (token, head) rows -- against
+// blocks of kTileKeys keys, with a running softmax (attention_plain_kernel's arithmetic,
+// operation for operation: the same bits).  Nothing in the kernel grows with the number of keys.
 // What bounds it: the fp32 multiply-adds of the two products (2 * keys * rows * DIM a tile),
 // issued two lanes at a time (fma.rn.f32x2); scores and probabilities stay in 32 bits, which
-// is why the products are not on the tensor cores.  Two blocks per SM, so that one block's
-// softmax (exp in 64 bits) and barriers run under the other's products.
-//   scores   thread = 4 rows x 2 keys, 16 bytes of features at a time: six shared loads, all
-//            free of bank conflicts (pitch DIM + 4), for sixteen paired multiply-adds
-//   softmax  four threads per row, eight keys each
-//   P*V      thread = 4 rows x DIM / 16 features, keys in ascending order
+// is why the products are not on the tensor cores.  With 64 rows and two blocks per SM one
+// block's softmax (exp in 64 bits) and barriers run under the other's products; where there are
+// fewer tiles than that, a tile is a serial chain over the keys, which 32 rows shorten.
+//   scores   thread = ROWS / 16 rows x 2 keys, 16 bytes of features at a time; shared loads
+//            free of bank conflicts (pitch DIM + 4)
+//   softmax  256 / ROWS threads per row
+//   P*V      thread = ROWS / 16 rows x DIM / 16 features, keys in ascending order
 // K of block b + 1 is copied (cp.async) under the softmax and P*V of block b, V of block b
-// under its scores.  A probability of zero contributes nothing (whatever the value row holds):
-// where an output is not finite -- a value row that is not, or values near the largest number
-// added up before the division -- the tile runs again with the rows' final maxima and sums,
-// probabilities of zero skipped, as attention_kernel has it.
-// Measured, eight layers of a prompt with 32 / 8 heads of 128 (all operators): 1500 tokens
-// 51.6 -> 18.8 ms (scores of that many keys did not fit the former tile kernel, and a block
-// per (token, head) read 37 GB of keys and values per layer); 256 tokens 3.47 -> 3.39 ms.
-constexpr int kTileRows = 64;
-template <int DIM>
+// under its scores.
+// A probability of zero contributes nothing (whatever the value row holds): where an output is
+// not finite -- a value row that is not, or values near the largest number added up before the
+// division -- the tile runs again with the rows' final maxima and sums, probabilities of zero
+// skipped, as attention_kernel has it.
+// Measured, 32 / 8 heads of 128, against the former tile kernel (all scores in shared memory,
+// one block per (token, head) beyond 1400 keys): 256 tokens 80 -> 39 us, behind 300 keys 131 ->
+// 108; 1200 tokens 753 -> 387; 600 tokens behind 1000 keys 3339 -> 512.
+template <int DIM, int ROWS>
 struct TileSmem {  // floats
     static constexpr int kPitch = DIM + 4, kProbPitch = kTileKeys + 4;
     static constexpr int kQ = 0;
-    static constexpr int kK = kQ + kTileRows * kPitch;
+    static constexpr int kK = kQ + ROWS * kPitch;
     static constexpr int kV = kK + kTileKeys * kPitch;
     static constexpr int kP = kV + kTileKeys * kPitch;
-    static constexpr int kAlpha = kP + kTileRows * kProbPitch;
-    static constexpr int kSum = kAlpha + kTileRows;
-    static constexpr int kBytes = (kSum + kTileRows) * 4;
+    static constexpr int kAlpha = kP + ROWS * kProbPitch;
+    static constexpr int kSum = kAlpha + ROWS;
+    static constexpr int kBytes = (kSum + ROWS) * 4;
 };
 __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
@@ -911,7 +911,7 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int DIM>
+template <int DIM, int ROWS>
 __global__ void __launch_bounds__(kAttnThreads, DIM > 128 ? 1 : 2)
 attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                       const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
@@ -919,7 +919,9 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                       int capacity, float scale, int tq) {
     b2w4_pdl_chain_entry();
     const int past = past_dev ? min(*past_dev, capacity - tokens) : past0;
-    using S = TileSmem<DIM>;
+    using S = TileSmem<DIM, ROWS>;
+    constexpr int RS = kAttnThreads / 16, RT = ROWS / RS;           // rows of a thread, RS apart
+    constexpr int ST = kAttnThreads / ROWS, SK = kTileKeys / ST;    // softmax: threads and keys a row
     constexpr int P = S::kPitch, PP = S::kProbPitch;
     extern __shared__ __align__(16) float s_dyn[];
     float* s_q = s_dyn + S::kQ;
@@ -929,8 +931,8 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
     float* s_alpha = s_dyn + S::kAlpha;
     float* s_sum = s_dyn + S::kSum;
     const int rep = heads / kv_heads;
-    // the last tiles see the most keys: they go first
-    const int kvh = blockIdx.y, t0 = (int)(gridDim.x - 1 - blockIdx.x) * tq;
+    // the last tiles see the most keys: they go first, of all kv heads
+    const int kvh = blockIdx.x, t0 = (int)(gridDim.y - 1 - blockIdx.y) * tq;
     const int vis_max = past + min(t0 + tq, tokens);  // keys the tile's last token sees
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float* kc = k_cache + (size_t)kvh * capacity * DIM;
@@ -950,30 +952,29 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         for (int u = 0; u < kCopies; ++u) {
             const int i = threadIdx.x + kAttnThreads * u, key = i / kRow4, c = i % kRow4;
             const bool valid = j0 + key < vis_max;
-            cp_async16(dst + key * P + 4 * c, base + (size_t)(valid ? j0 + key : 0) * DIM + 4 * c,
-                       valid);
+            cp_async16(dst + key * P + 4 * c, base + (size_t)(valid ? j0 + key : 0) * DIM + 4 * c, valid);
         }
         cp_async_commit();
     };
-    for (int i = threadIdx.x; i < kTileRows * kRow4; i += kAttnThreads) {
+    for (int i = threadIdx.x; i < ROWS * kRow4; i += kAttnThreads) {
         const int row = i / kRow4, c = i % kRow4;
         const bool live = row_visible(row) > 0;
         cp_async16(s_q + row * P + 4 * c, q + (live ? row_offset(row) : 0) + 4 * c, live);
     }
 
-    // products: rows r_of(i) = ra + 16 i, keys kb + 16 j, features 4 kb + 64 i .. + 3
+    // products: rows ra + RS i, keys kb + 16 j, features 4 kb + 64 i .. + 3
     const int ra = (warp >> 1) * 4 + (lane >> 3), kb = (warp & 1) * 8 + (lane & 7);
-    // softmax: row sr, keys 8 sq .. 8 sq + 7 of a block
-    const int sr = threadIdx.x >> 2, sq = threadIdx.x & 3;
+    // softmax: row sr, keys SK sq .. SK sq + SK - 1 of a block
+    const int sr = threadIdx.x / ST, sq = threadIdx.x % ST;
     const int s_vis = row_visible(sr);
     float m = -INFINITY, l = 0.f;
     bool final_pass = false;  // m and 1 / l are the row's final ones, in m and l
     constexpr int NV = DIM / 64;
     for (;;) {
     copy_keys(s_k, kc, 0);  // the first time with Q: one group
-    uint64_t acc[4][2 * NV];
+    uint64_t acc[RT][2 * NV];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
         for (int c = 0; c < 2 * NV; ++c)
             acc[i][c] = 0;
@@ -983,38 +984,38 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         cp_async_wait<1>();
         __syncthreads();  // K of this block is in place
         {
-            float sc[4][2];
+            float sc[RT][2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RT; ++i)
                 sc[i][0] = sc[i][1] = 0.f;
 #pragma unroll 1
             for (int c = 0; c < DIM; c += 32) {
-                uint64_t a[4][2];
+                uint64_t a[RT][2];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < RT; ++i)
                     a[i][0] = a[i][1] = 0;
 #pragma unroll
                 for (int d = 0; d < 32; d += 4) {
-                    ulonglong2 qv[4], kv[2];
+                    ulonglong2 qv[RT], kv[2];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        qv[i] = *reinterpret_cast<const ulonglong2*>(s_q + (ra + 16 * i) * P + c + d);
+                    for (int i = 0; i < RT; ++i)
+                        qv[i] = *reinterpret_cast<const ulonglong2*>(s_q + (ra + RS * i) * P + c + d);
 #pragma unroll
                     for (int j = 0; j < 2; ++j)
                         kv[j] = *reinterpret_cast<const ulonglong2*>(s_k + (kb + 16 * j) * P + c + d);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < RT; ++i)
 #pragma unroll
                         for (int j = 0; j < 2; ++j)
                             a[i][j] = b2w4_fma2(qv[i].x, kv[j].x, a[i][j]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < RT; ++i)
 #pragma unroll
                         for (int j = 0; j < 2; ++j)
                             a[i][j] = b2w4_fma2(qv[i].y, kv[j].y, a[i][j]);
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < RT; ++i)
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         float lo, hi;
@@ -1023,10 +1024,10 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                     }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RT; ++i)
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
-                    s_p[(ra + 16 * i) * PP + kb + 16 * j] = __fmul_rn(sc[i][j], scale);
+                    s_p[(ra + RS * i) * PP + kb + 16 * j] = __fmul_rn(sc[i][j], scale);
         }
         __syncthreads();  // scores in place, K consumed
         if (j0 + kTileKeys < vis_max)
@@ -1034,33 +1035,41 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         else
             cp_async_commit();  // an empty group keeps the count
         {
-            float* row = s_p + sr * PP + 8 * sq;
-            float e[8];
-            *reinterpret_cast<float4*>(e) = *reinterpret_cast<const float4*>(row);
-            *reinterpret_cast<float4*>(e + 4) = *reinterpret_cast<const float4*>(row + 4);
+            float* row = s_p + sr * PP + SK * sq;
+            float e[SK];
+#pragma unroll
+            for (int i = 0; i < SK; i += 4)
+                *reinterpret_cast<float4*>(e + i) = *reinterpret_cast<const float4*>(row + i);
             float mb = m;
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (j0 + 8 * sq + i < s_vis)
+            for (int i = 0; i < SK; ++i)
+                if (j0 + SK * sq + i < s_vis)
                     mb = fmaxf(mb, e[i]);
-            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
-            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
+#pragma unroll
+            for (int off = 1; off < ST; off <<= 1)
+                mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, off));
             const float alpha = j0 && !final_pass ? attn_rescale(m, mb) : 1.f;
             m = mb;  // final_pass: as it was
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                e[i] = j0 + 8 * sq + i < s_vis ? attn_prob(e[i], m) : 0.f;
+            for (int i = 0; i < SK; ++i)
+                e[i] = j0 + SK * sq + i < s_vis ? attn_prob(e[i], m) : 0.f;
             if (final_pass) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < SK; ++i)
                     e[i] = __fmul_rn(e[i], l);
             }
-            *reinterpret_cast<float4*>(row) = *reinterpret_cast<const float4*>(e);
-            *reinterpret_cast<float4*>(row + 4) = *reinterpret_cast<const float4*>(e + 4);
-            float sum = __fadd_rn(__fadd_rn(__fadd_rn(e[0], e[1]), __fadd_rn(e[2], e[3])),
-                                  __fadd_rn(__fadd_rn(e[4], e[5]), __fadd_rn(e[6], e[7])));
-            sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 1));
-            sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 2));
+#pragma unroll
+            for (int i = 0; i < SK; i += 4)
+                *reinterpret_cast<float4*>(row + i) = *reinterpret_cast<const float4*>(e + i);
+#pragma unroll
+            for (int n = 1; n < SK; n <<= 1)
+#pragma unroll
+                for (int i = 0; i < SK; i += 2 * n)
+                    e[i] = __fadd_rn(e[i], e[i + n]);
+            float sum = e[0];
+#pragma unroll
+            for (int off = 1; off < ST; off <<= 1)
+                sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off));
             if (!final_pass)
                 l = __fadd_rn(__fmul_rn(l, alpha), sum);
             if (sq == 0)
@@ -1069,7 +1078,7 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         cp_async_wait<1>();  // V of this block
         __syncthreads();  // V, probabilities, factors in place
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < RT; ++i) {
             const float al = s_alpha[ra + 16 * i];
             if (al != 1.f) {
                 const uint64_t al2 = b2w4_pack2(al, al);
@@ -1081,10 +1090,10 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         if (!final_pass) {
 #pragma unroll 2
             for (int j = 0; j < kTileKeys; j += 4) {
-                float4 p4[4];
+                float4 p4[RT];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    p4[i] = *reinterpret_cast<const float4*>(s_p + (ra + 16 * i) * PP + j);
+                for (int i = 0; i < RT; ++i)
+                    p4[i] = *reinterpret_cast<const float4*>(s_p + (ra + RS * i) * PP + j);
 #pragma unroll
                 for (int jj = 0; jj < 4; ++jj) {
                     ulonglong2 v[NV];
@@ -1093,7 +1102,7 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                         v[c] = *reinterpret_cast<const ulonglong2*>(s_v + (j + jj) * P + 4 * kb +
                                                                     64 * c);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < RT; ++i) {
                         const float p = jj == 0 ? p4[i].x : jj == 1 ? p4[i].y
                                       : jj == 2 ? p4[i].z : p4[i].w;
                         const uint64_t pp = b2w4_pack2(p, p);
@@ -1109,8 +1118,8 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
 #pragma unroll 1
             for (int j = 0; j < kTileKeys; ++j) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float p = s_p[(ra + 16 * i) * PP + j];
+                for (int i = 0; i < RT; ++i) {
+                    const float p = s_p[(ra + RS * i) * PP + j];
                     if (p != 0.f) {
                         const uint64_t pp = b2w4_pack2(p, p);
 #pragma unroll
@@ -1131,8 +1140,8 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
     __syncthreads();
     bool odd = false;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = ra + 16 * i;
+    for (int i = 0; i < RT; ++i) {
+        const int row = ra + RS * i;
         if (row_visible(row)) {
             const float total = s_sum[row];
 #pragma unroll
@@ -1204,6 +1213,7 @@ struct AttnPlan {
     int rows;       // ATTN_TILE: rows per tile
     int ctas;       // ATTN_SPLIT: blocks per cluster
     int one_range;  // ATTN_SPLIT: visible keys up to which one block takes them all
+    bool alone;     // ATTN_TILE: one block per multiprocessor
 };
 struct AttnArgs {
     const float *q, *k_cache, *v_cache;
@@ -1217,19 +1227,46 @@ struct AttnArgs {
 // query heads of a kv head that a block of the split kernel serves
 int split_heads(int dim, int rep) { return dim == 256 ? min(rep, 2) : rep >= 3 ? 4 : rep; }
 
+// Time of the tile kernel with one block per multiprocessor, in the time of the largest tile
+// (its last token sees past + tokens keys, the first tile's about past): one wave is as long as
+// its largest tile; in a second one the largest tiles that are left go where the smallest of
+// the first wave were, and all such pairs are equally long; beyond that the load counts.
+double tile_blocks(int tokens, int rep, int rows, int kv_heads) {
+    return rep > rows ? 1e9 : (double)((tokens + rows / rep - 1) / (rows / rep)) * kv_heads;
+}
+double tile_load(int tokens, int rep, int rows, int kv_heads, int past, int sms) {
+    return tile_blocks(tokens, rep, rows, kv_heads) / sms * (past + 0.5 * tokens) / (past + tokens);
+}
+double tile_time(int tokens, int rep, int rows, int kv_heads, int past, int sms) {
+    const double n = tile_blocks(tokens, rep, rows, kv_heads);
+    if (n <= sms)
+        return 1.0;
+    if (n <= 2.0 * sms)
+        return max(1.0, 2.0 * (1.0 - (double)tokens / (past + tokens) * sms / n));
+    return tile_load(tokens, rep, rows, kv_heads, past, sms) + 0.3;
+}
+
 // A call's form depends on its sizes and the cache's capacity, not on the position, so that a
-// position given by the host and one read on the device leave the same bits.  The lines,
-// times on a B200:
+// position given by the host and one read on the device leave the same bits (the tile kernel's
+// variants do, too, so those are chosen by `past`).  The lines, times on a B200:
 //   few rows   `groups` blocks with all keys (one_range), or clusters that split them.  A
 //              cluster costs 2 to 3 us, more where there are many; 32 / 8 heads of 128, one
 //              block against clusters: one token, 64 keys 5.1 / 5.6 us, 160 keys 7.1 / 5.8; 16
 //              tokens, 300 keys 12.6 / 15.7, 1000 keys 36 / 26.  The cluster sizes keep all of
 //              them resident at once: sixteen against eight, one token, 6000 keys 22.6 / 34.1,
 //              seven tokens 73 / 62, with four 59.
+//   up to      10 groups per multiprocessor; against the tile kernel: 32 / 8 heads of 128, 100
+//              tokens behind 300 keys 41 / 57 us, 256 tokens 108 / 108; 16 / 8 heads of 64, 160
+//              tokens 36 / 42, 256 tokens 56 / 49.
+//   from       a capacity of 384 for runs of eight or more: below that the tile kernel is at
+//              most some tens of us long, and keeps the bits of the one-row arithmetic.
+//   tiles      of 32 rows alone on a multiprocessor, of 64 alone (1.41 times as long), or two of
+//              64 (1.6 times that, 0.82 of it per tile), by tile_time: 600 tokens of 32 / 8
+//              heads 178 / 134 / 174 us, 1200 tokens 661 / 473 / 387, 256 tokens 39 / 52 / 62.
 AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int capacity,
                    bool aligned, bool row_only, int max_cluster, int sm_count) {
     const int rep = heads / kv_heads;
-    AttnPlan p = {ATTN_ROW, 0, 0, 0};
+    AttnPlan p = {ATTN_ROW, 0, 0, 0, false};
     if (dim != 64 && dim != 128 && dim != 256)
         return p;
     if (row_only) {
@@ -1238,7 +1275,8 @@ AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int c
     }
     const int hr = split_heads(dim, rep);
     const long groups = (long)tokens * kv_heads * ((rep + hr - 1) / hr);
-    if (aligned && tokens < 8 && groups / tokens <= 65535) {
+    if (aligned && groups / tokens <= 65535 &&
+        (tokens < 8 || (capacity >= 384 && groups <= 10l * sm_count))) {
         p.form = ATTN_SPLIT;
         p.ctas = capacity > 1024 && groups * 32 <= 3l * sm_count ? 16
                  : groups * 8 <= 2l * sm_count                   ? 8
@@ -1248,10 +1286,15 @@ AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int c
             p.ctas /= 2;
         return p;
     }
-    if (rep > kTileRows || tokens < 8 || !aligned)
+    if (rep > 64 || tokens < 8 || !aligned)
         return p;
     p.form = ATTN_TILE;
-    p.rows = kTileRows;
+    const double whole32 = tile_time(tokens, rep, 32, kv_heads, past, sm_count);
+    const double whole64 = 1.41 * tile_time(tokens, rep, 64, kv_heads, past, sm_count);
+    const double shared64 =
+        1.41 * max(1.6, 0.82 * tile_load(tokens, rep, 64, kv_heads, past, sm_count));
+    p.rows = whole32 <= min(whole64, shared64) ? 32 : 64;
+    p.alone = p.rows == 32 || whole64 <= shared64;
     return p;
 }
 
@@ -1332,13 +1375,15 @@ int launch_split(b2w4_ctx* ctx, const AttnArgs& a, int dim, int keys, const Attn
     }
 }
 
-template <int DIM>
-int launch_tile_dim(b2w4_ctx* ctx, const AttnArgs& a) {
+// more dynamic shared memory than this, and a multiprocessor holds one block
+constexpr size_t kHalfSmem = 114 * 1024;
+template <int DIM, int ROWS>
+int launch_tile_as(b2w4_ctx* ctx, const AttnArgs& a, bool alone) {
     static b2w4_smem_optin cfg;
-    const size_t smem = TileSmem<DIM>::kBytes;
-    auto kern = attention_tile_kernel<DIM>;
-    const int tq = kTileRows / (a.heads / a.kv_heads);
-    const dim3 grid((a.tokens + tq - 1) / tq, a.kv_heads);
+    auto kern = attention_tile_kernel<DIM, ROWS>;
+    const int tq = ROWS / (a.heads / a.kv_heads);
+    const dim3 grid(a.kv_heads, (a.tokens + tq - 1) / tq);
+    const size_t smem = max((size_t)TileSmem<DIM, ROWS>::kBytes, alone ? kHalfSmem + 1 : 0);
     B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, cfg));
     B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), smem,
                                        ctx->stream, a.q, a.k_cache, a.v_cache, a.out, a.tokens,
@@ -1347,10 +1392,15 @@ int launch_tile_dim(b2w4_ctx* ctx, const AttnArgs& a) {
     ctx->launches++;
     return B2W4_OK;
 }
-int launch_tile(b2w4_ctx* ctx, const AttnArgs& a, int dim) {
-    return dim == 64    ? launch_tile_dim<64>(ctx, a)
-           : dim == 128 ? launch_tile_dim<128>(ctx, a)
-                        : launch_tile_dim<256>(ctx, a);
+template <int DIM>
+int launch_tile_dim(b2w4_ctx* ctx, const AttnArgs& a, const AttnPlan& plan) {
+    return plan.rows == 32 ? launch_tile_as<DIM, 32>(ctx, a, plan.alone)
+                           : launch_tile_as<DIM, 64>(ctx, a, plan.alone);
+}
+int launch_tile(b2w4_ctx* ctx, const AttnArgs& a, int dim, const AttnPlan& plan) {
+    return dim == 64    ? launch_tile_dim<64>(ctx, a, plan)
+           : dim == 128 ? launch_tile_dim<128>(ctx, a, plan)
+                        : launch_tile_dim<256>(ctx, a, plan);
 }
 
 }  // namespace
@@ -1480,7 +1530,7 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
             return rc;
     }
     if (plan.form == ATTN_TILE)
-        return launch_tile(ctx, a, dim);
+        return launch_tile(ctx, a, dim, plan);
     static b2w4_smem_optin configured[2];
     const bool plain = plan.form == ATTN_PLAIN;
     auto kern = plain ? attention_plain_kernel : attention_kernel;
@@ -1496,7 +1546,7 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
     return B2W4_OK;
 }
 
-// What attn_plan says, for checks without a device: the form; out: rows, ctas, one_range.
+// What attn_plan says, for checks without a device: the form; out: rows, ctas, one_range, alone.
 int b2w4_attention_plan(int tokens, int heads, int kv_heads, int dim, int past, int capacity,
                         int aligned, int row_only, int max_cluster, int sm_count, int* out) {
     const AttnPlan p = attn_plan(tokens, heads, kv_heads, dim, past, capacity, aligned, row_only,
@@ -1504,6 +1554,7 @@ int b2w4_attention_plan(int tokens, int heads, int kv_heads, int dim, int past, 
     out[0] = p.rows;
     out[1] = p.ctas;
     out[2] = p.one_range;
+    out[3] = p.alone;
     return p.form;
 }
 

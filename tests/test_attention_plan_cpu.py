@@ -57,3 +57,29 @@ def test_smaller_clusters():
         assert form == SPLIT and p["ctas"] <= cluster
         assert p["ctas"] & (p["ctas"] - 1) == 0  # divides a block's share of the features
         assert p["one_range"] == 96
+
+
+@pytest.mark.parametrize("heads,kv_heads", HEADS[:5] + HEADS[6:7] + HEADS[8:])
+def test_runs_behind_a_context(heads, kv_heads):
+    """Eight or more tokens on a cache of 384 rows or more: never tiles that leave most of the
+    chip idle while they walk the keys one block after the other."""
+    for tokens, dim, past in itertools.product((8, 9, 16, 33, 64, 100, 256, 600, 1400),
+                                               (64, 128, 256), (0, 100, 1000, 6000, 40000)):
+        capacity = max(384, past + tokens)
+        form, p = plan(tokens, heads, kv_heads, dim, past, capacity)
+        hr = (min(2, heads // kv_heads) if dim == 256 else
+              4 if heads // kv_heads >= 3 else heads // kv_heads)
+        groups = tokens * kv_heads * -(-(heads // kv_heads) // hr)
+        assert form == (SPLIT if groups <= 10 * SMS else TILE)
+        if form == TILE:
+            rep = heads // kv_heads
+            tiles = -(-tokens // (p["rows"] // rep)) * kv_heads
+            assert p["rows"] in (32, 64) and rep <= p["rows"]
+            assert tiles >= SMS // 4
+            assert p["alone"] or tiles > SMS
+        # a cache of 384 rows: the same form wherever the position is
+        assert plan(tokens, heads, kv_heads, dim, 0, capacity)[0] == form
+        if tokens < 300:
+            assert plan(tokens, heads, kv_heads, dim, 0, 383)[0] == TILE
+    assert plan(40, 71, 1, 128)[0] == ROW  # more query heads per kv head than a tile has rows
+    assert plan(40, 64, 1, 128) == (TILE, dict(rows=64, ctas=0, one_range=0, alone=1))

@@ -486,3 +486,58 @@ def test_split_attention_on_either_side_of_one_range(ctx, tokens, past, heads, k
         assert outs[1].tobytes() == outs[0].tobytes()
     else:  # few keys known to the host need no cluster; the device's position does
         assert rel_l2(outs[1], want) < 1e-5
+
+
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [
+    (8, 376, 8, 2, 128), (9, 1600, 3, 1, 64), (16, 3000, 2, 2, 256), (33, 4090, 4, 2, 128),
+    (64, 500, 32, 8, 64), (200, 300, 6, 2, 128)])
+def test_short_runs_behind_a_context(ctx, tokens, past, heads, kv_heads, dim):
+    """Runs of eight or more tokens on a cache of at least 384 rows whose tiles would leave
+    most of the chip idle go to the split kernel: some tokens within one block's range of keys
+    and some beyond.  The position on the device leaves the same bits.  Tolerance as for the
+    split kernel."""
+    import torch
+    capacity, scale = past + tokens, dim ** -0.5
+    rng = np.random.default_rng(past + dim)
+    q = rng.normal(0, 1, (tokens, heads, dim)).astype(np.float32)
+    k_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    v_all = rng.normal(0, 1, (past + tokens, kv_heads, dim)).astype(np.float32)
+    kcd, vcd = (_dev(np.ascontiguousarray(x.transpose(1, 0, 2))) for x in (k_all, v_all))
+    qd = _dev(q)
+    outs = []
+    for past_dev in (None, torch.full((1,), past, dtype=torch.int32, device="cuda")):
+        out = torch.zeros((tokens, heads, dim), dtype=torch.float32, device="cuda")
+        ctx.attention(qd, None, None, kcd, vcd, out, tokens, heads, kv_heads, dim,
+                      past if past_dev is None else 0, capacity, scale, past_dev)
+        ctx.sync()
+        outs.append(out.cpu().numpy())
+    assert outs[1].tobytes() == outs[0].tobytes()
+    some = [0, 1, tokens // 2, tokens - 1]
+    for t in some:
+        want = _attention_fp64(q[t:t + 1], k_all, v_all, heads, kv_heads, past + t, scale)
+        assert rel_l2(outs[0][t:t + 1], want) < 1e-5
+
+
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [
+    (31, 0, 8, 8, 64), (260, 90, 20, 20, 64), (600, 100, 8, 8, 128), (700, 0, 33, 1, 64),
+    (640, 0, 32, 8, 64), (1300, 0, 16, 8, 64), (500, 3, 16, 4, 256)])
+def test_tile_variants_equal_the_row_arithmetic(ctx, tokens, past, heads, kv_heads, dim):
+    """Tiles of 32 and 64 rows, one or two per multiprocessor, grids of one wave and of several,
+    ragged last tiles: the bits of the one-row form, row by row."""
+    import torch
+    capacity, scale = past + tokens, dim ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(tokens + dim)
+    q = torch.randn((tokens, heads, dim), device="cuda", generator=g)
+    kc, vc = (torch.randn((kv_heads, capacity, dim), device="cuda", generator=g)
+              for _ in range(2))
+    ctx_row = _row_context()
+    outs = []
+    for c in (ctx, ctx_row):
+        out = torch.zeros_like(q)
+        c.attention(q, None, None, kc, vc, out, tokens, heads, kv_heads, dim, past, capacity,
+                    scale)
+        c.sync()
+        outs.append(out.cpu().numpy())
+    ctx_row.close()
+    assert np.isfinite(outs[0]).all()
+    assert outs[0].tobytes() == outs[1].tobytes()
