@@ -878,7 +878,8 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
 //   softmax  256 / ROWS threads per row
 //   P*V      thread = ROWS / 16 rows x DIM / 16 features, keys in ascending order
 // K of block b + 1 is copied (cp.async) under the softmax and P*V of block b, V of block b
-// under its scores.
+// under its scores; in 4-byte copies where a row is not 16-byte aligned (!ALIGNED; 32 / 8 heads
+// of 128, 160 tokens behind 300 keys 93 -> 103 us, one block per (token, head): 730).
 // A probability of zero contributes nothing (whatever the value row holds): where an output is
 // not finite -- a value row that is not, or values near the largest number added up before the
 // division -- the tile runs again with the rows' final maxima and sums, probabilities of zero
@@ -903,6 +904,12 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool va
                  "l"(src), "r"(valid ? 16 : 0)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(valid ? 4 : 0)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -911,7 +918,7 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int DIM, int ROWS>
+template <int DIM, int ROWS, bool ALIGNED>
 __global__ void __launch_bounds__(kAttnThreads, DIM > 128 ? 1 : 2)
 attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                       const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
@@ -947,19 +954,28 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
     };
     constexpr int kRow4 = DIM / 4;                            // float4 per row
     constexpr int kCopies = kTileKeys * kRow4 / kAttnThreads;  // per thread and block of keys
+    auto copy4 = [&](float* dst, const float* src, bool valid) {
+        if constexpr (ALIGNED) {
+            cp_async16(dst, src, valid);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                cp_async4(dst + i, src + i, valid);
+        }
+    };
     auto copy_keys = [&](float* dst, const float* base, int j0) {
 #pragma unroll
         for (int u = 0; u < kCopies; ++u) {
             const int i = threadIdx.x + kAttnThreads * u, key = i / kRow4, c = i % kRow4;
             const bool valid = j0 + key < vis_max;
-            cp_async16(dst + key * P + 4 * c, base + (size_t)(valid ? j0 + key : 0) * DIM + 4 * c, valid);
+            copy4(dst + key * P + 4 * c, base + (size_t)(valid ? j0 + key : 0) * DIM + 4 * c, valid);
         }
         cp_async_commit();
     };
     for (int i = threadIdx.x; i < ROWS * kRow4; i += kAttnThreads) {
         const int row = i / kRow4, c = i % kRow4;
         const bool live = row_visible(row) > 0;
-        cp_async16(s_q + row * P + 4 * c, q + (live ? row_offset(row) : 0) + 4 * c, live);
+        copy4(s_q + row * P + 4 * c, q + (live ? row_offset(row) : 0) + 4 * c, live);
     }
 
     // products: rows ra + RS i, keys kb + 16 j, features 4 kb + 64 i .. + 3
@@ -1157,7 +1173,15 @@ attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                 const float z = __fadd_rn(__fadd_rn(__fmul_rn(o.x, 0.f), __fmul_rn(o.y, 0.f)),
                                           __fadd_rn(__fmul_rn(o.z, 0.f), __fmul_rn(o.w, 0.f)));
                 odd |= z != 0.f;
-                *reinterpret_cast<float4*>(out + row_offset(row) + 4 * kb + 64 * c) = o;
+                float* dst = out + row_offset(row) + 4 * kb + 64 * c;
+                if constexpr (ALIGNED) {
+                    *reinterpret_cast<float4*>(dst) = o;
+                } else {
+                    dst[0] = o.x;
+                    dst[1] = o.y;
+                    dst[2] = o.z;
+                    dst[3] = o.w;
+                }
             }
         }
     }
@@ -1260,6 +1284,8 @@ double tile_time(int tokens, int rep, int rows, int kv_heads, int past, int sms)
 //              tokens 36 / 42, 256 tokens 56 / 49.
 //   from       a capacity of 384 for runs of eight or more: below that the tile kernel is at
 //              most some tens of us long, and keeps the bits of the one-row arithmetic.
+//   unaligned  one block per (token, head) up to five per multiprocessor, then tiles: 32 / 8
+//              heads of 128, 8 tokens behind 6000 keys 430 / 830 us, 32 tokens 910 / 840.
 //   tiles      of 32 rows alone on a multiprocessor, of 64 alone (1.41 times as long), or two of
 //              64 (1.6 times that, 0.82 of it per tile), by tile_time: 600 tokens of 32 / 8
 //              heads 178 / 134 / 174 us, 1200 tokens 661 / 473 / 387, 256 tokens 39 / 52 / 62.
@@ -1286,7 +1312,7 @@ AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int c
             p.ctas /= 2;
         return p;
     }
-    if (rep > 64 || tokens < 8 || !aligned)
+    if (rep > 64 || tokens < 8 || (!aligned && (long)tokens * heads <= 5l * sm_count))
         return p;
     p.form = ATTN_TILE;
     const double whole32 = tile_time(tokens, rep, 32, kv_heads, past, sm_count);
@@ -1377,10 +1403,10 @@ int launch_split(b2w4_ctx* ctx, const AttnArgs& a, int dim, int keys, const Attn
 
 // more dynamic shared memory than this, and a multiprocessor holds one block
 constexpr size_t kHalfSmem = 114 * 1024;
-template <int DIM, int ROWS>
+template <int DIM, int ROWS, bool ALIGNED>
 int launch_tile_as(b2w4_ctx* ctx, const AttnArgs& a, bool alone) {
     static b2w4_smem_optin cfg;
-    auto kern = attention_tile_kernel<DIM, ROWS>;
+    auto kern = attention_tile_kernel<DIM, ROWS, ALIGNED>;
     const int tq = ROWS / (a.heads / a.kv_heads);
     const dim3 grid(a.kv_heads, (a.tokens + tq - 1) / tq);
     const size_t smem = max((size_t)TileSmem<DIM, ROWS>::kBytes, alone ? kHalfSmem + 1 : 0);
@@ -1393,14 +1419,17 @@ int launch_tile_as(b2w4_ctx* ctx, const AttnArgs& a, bool alone) {
     return B2W4_OK;
 }
 template <int DIM>
-int launch_tile_dim(b2w4_ctx* ctx, const AttnArgs& a, const AttnPlan& plan) {
-    return plan.rows == 32 ? launch_tile_as<DIM, 32>(ctx, a, plan.alone)
-                           : launch_tile_as<DIM, 64>(ctx, a, plan.alone);
+int launch_tile_dim(b2w4_ctx* ctx, const AttnArgs& a, const AttnPlan& plan, bool aligned) {
+    if (plan.rows == 32)
+        return aligned ? launch_tile_as<DIM, 32, true>(ctx, a, plan.alone)
+                       : launch_tile_as<DIM, 32, false>(ctx, a, plan.alone);
+    return aligned ? launch_tile_as<DIM, 64, true>(ctx, a, plan.alone)
+                   : launch_tile_as<DIM, 64, false>(ctx, a, plan.alone);
 }
-int launch_tile(b2w4_ctx* ctx, const AttnArgs& a, int dim, const AttnPlan& plan) {
-    return dim == 64    ? launch_tile_dim<64>(ctx, a, plan)
-           : dim == 128 ? launch_tile_dim<128>(ctx, a, plan)
-                        : launch_tile_dim<256>(ctx, a, plan);
+int launch_tile(b2w4_ctx* ctx, const AttnArgs& a, int dim, const AttnPlan& plan, bool aligned) {
+    return dim == 64    ? launch_tile_dim<64>(ctx, a, plan, aligned)
+           : dim == 128 ? launch_tile_dim<128>(ctx, a, plan, aligned)
+                        : launch_tile_dim<256>(ctx, a, plan, aligned);
 }
 
 }  // namespace
@@ -1530,7 +1559,7 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
             return rc;
     }
     if (plan.form == ATTN_TILE)
-        return launch_tile(ctx, a, dim, plan);
+        return launch_tile(ctx, a, dim, plan, aligned);
     static b2w4_smem_optin configured[2];
     const bool plain = plan.form == ATTN_PLAIN;
     auto kern = plain ? attention_plain_kernel : attention_kernel;

@@ -83,3 +83,12 @@ def test_runs_behind_a_context(heads, kv_heads):
             assert plan(tokens, heads, kv_heads, dim, 0, 383)[0] == TILE
     assert plan(40, 71, 1, 128)[0] == ROW  # more query heads per kv head than a tile has rows
     assert plan(40, 64, 1, 128) == (TILE, dict(rows=64, ctas=0, one_range=0, alone=1))
+
+
+def test_unaligned_runs():
+    """Rows that are not 16-byte aligned: tiles too, unless one block per (token, head) is few
+    blocks."""
+    for tokens, (heads, kv_heads) in itertools.product((8, 23, 24, 100, 600), HEADS):
+        for capacity in (tokens, 5000):
+            form = plan(tokens, heads, kv_heads, 128, 0, capacity, aligned=0)[0]
+            assert form == (ROW if heads // kv_heads > 64 or tokens * heads <= 5 * SMS else TILE)

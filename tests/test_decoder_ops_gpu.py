@@ -541,3 +541,35 @@ def test_tile_variants_equal_the_row_arithmetic(ctx, tokens, past, heads, kv_hea
     ctx_row.close()
     assert np.isfinite(outs[0]).all()
     assert outs[0].tobytes() == outs[1].tobytes()
+
+
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [
+    (1, 40, 8, 2, 128), (25, 50, 32, 8, 128), (70, 300, 16, 8, 64), (600, 0, 16, 4, 128),
+    (300, 7, 16, 4, 256)])
+def test_attention_on_unaligned_rows(ctx, tokens, past, heads, kv_heads, dim):
+    """q, the caches and the output one float past a 16-byte boundary: runs take the tile
+    kernel with narrow copies (the bits of the one-row form), few rows one block per (token,
+    head) (tolerance as for the split kernel)."""
+    import torch
+    capacity, scale = past + tokens + 1, dim ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(tokens + dim)
+
+    def odd(*shape):
+        n = int(np.prod(shape))
+        return torch.randn(n + 1, device="cuda", generator=g)[1:].view(*shape)
+
+    q, out = odd(tokens, heads, dim), odd(tokens, heads, dim)
+    kc, vc = odd(kv_heads, capacity, dim), odd(kv_heads, capacity, dim)
+    row = torch.zeros((tokens, heads, dim), device="cuda")
+    assert q.data_ptr() % 16 and out.data_ptr() % 16 and kc.data_ptr() % 16
+    ctx_row = _row_context()
+    ctx.attention(q, None, None, kc, vc, out, tokens, heads, kv_heads, dim, past, capacity, scale)
+    ctx_row.attention(q, None, None, kc, vc, row, tokens, heads, kv_heads, dim, past, capacity,
+                      scale)
+    ctx.sync()
+    ctx_row.sync()
+    ctx_row.close()
+    got, want = out.cpu().numpy(), row.cpu().numpy()
+    if tokens >= 8:
+        assert got.tobytes() == want.tobytes()
+    assert rel_l2(got, want) < 1e-5
