@@ -516,21 +516,24 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
 //            over the eight lanes that halves the items held at each level
 //   softmax  over the block's own keys: max m, e_j = exp(s_j - m), l = sum e_j
 //   P*V      a warp per key, four features per lane, HR accumulator rows; the warps' sums are
-//            added through shared memory
+//            added through shared memory; the first value rows are fetched before the softmax
+//            (6000 keys 22.7 -> 21.4 us)
 //   merge    block r adds its share of the features over the cluster (distributed shared
 //            memory): out = sum_c w_c o_c / sum_c w_c l_c, w_c = exp(m_c - max m)
 // Up to `one_range` visible keys the first block takes them all and the others leave: a cluster
 // costs more than it gives there (a step at position 0, 32 / 8 heads of 128: 3.1 us with one
-// block per head, 6.2 split over sixteen, 3.3 as it is; seven tokens 3.8, 23.4, 3.5).
+// block per head, 6.2 split over sixteen, 3.0 as it is; seven tokens 3.8, 23.4, 3.3).
 // Measured, a step with 32 / 8 heads of 128 behind 6000 keys: 313 us with one block per head
-// (32 of 148 SMs, every key read four times), 22.6 us over sixteen blocks, 34 over eight.
+// (32 of 148 SMs, every key read four times), 21.4 us over sixteen blocks, 32 over eight.
 // The split depends on the number of visible keys and the call's sizes, so a position given by
 // the host and one read on the device leave the same bits.  A probability of zero contributes
 // nothing (whatever the value row holds), as in attention_kernel: where a block's sums are not
 // finite -- a value row that is not, or values near the largest number added up before the
-// division -- every block runs P*V again on the final probabilities.  A NaN score reaches every
+// division -- every block forms them again from the final probabilities.  A NaN score reaches every
 // feature.
 constexpr int kMaxRanges = 16;
+// blocks per multiprocessor that the registers allow
+constexpr int split_blocks(int dim, int hr) { return dim * hr <= 128 ? 4 : dim * hr <= 256 ? 3 : 2; }
 template <int DIM, int HR>
 struct SplitSmem {  // floats of dynamic shared memory before the scores
     static constexpr int kAcc = 0;                              // [kAttnWarps][HR][DIM]
@@ -543,12 +546,12 @@ struct SplitSmem {  // floats of dynamic shared memory before the scores
     static constexpr int kOdd = kTotal + HR;                    // 1: not finite; [1]: any block's
     static constexpr int kScores = (kOdd + 2 + 3) & ~3;         // [keys][HR]
 };
-template <int DIM, int HR>
-__global__ void __launch_bounds__(kAttnThreads, 2)
+template <int DIM, int HR, int CTAS>
+__global__ void __launch_bounds__(kAttnThreads, split_blocks(DIM, HR))
 attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                        const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
                        int heads, int kv_heads, int past0, const int* __restrict__ past_dev,
-                       int capacity, float scale, int ctas, int one_range) {
+                       int capacity, float scale, int one_range) {
     b2w4_pdl_chain_entry();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -568,10 +571,10 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
     const int kvh = blockIdx.y / sets, r0 = (blockIdx.y % sets) * HR;  // heads r0.. of the kv head
     const int nh = min(HR, rep - r0), t = blockIdx.z, rank = blockIdx.x;
     const int visible = past + t + 1;
-    const int ranges = visible <= one_range ? 1 : ctas;
-    if (rank >= ranges)  // a barrier of the cluster waits for the blocks that are still there
+    const int ranges = CTAS == 1 || visible <= one_range ? 1 : CTAS;
+    if (CTAS > 1 && rank >= ranges)  // nobody waits for a block that has left
         return;
-    const int per = (visible + ranges - 1) / ranges;
+    const int per = ranges == 1 ? visible : (visible + CTAS - 1) / CTAS;
     const int j0 = min(rank * per, visible), n = min(per, visible - j0);
     const size_t row0 = ((size_t)t * heads + (size_t)kvh * rep + r0) * DIM;
     const float* kc = k_cache + ((size_t)kvh * capacity + j0) * DIM;
@@ -656,6 +659,27 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
     }
     __syncthreads();
 
+    // value rows: a warp per key (two for 64 features), U steps of keys in flight; the first
+    // ones are on their way during the softmax
+    constexpr int kLanes = DIM / 4 < 32 ? DIM / 4 : 32;  // lanes per value row
+    constexpr int kV4 = DIM / 4 / kLanes;                // float4 per lane
+    constexpr int kKeys = 32 / kLanes;                   // keys per warp and step
+    constexpr int U = 8 / kV4;                           // steps in flight
+    const int v_part = lane % kLanes, v_sub = lane / kLanes, v_first = warp * kKeys + v_sub;
+    float4 vr[U][kV4];
+    auto fetch_values = [&](int j) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < kV4; ++i) {
+                const int key = min(j + u * kAttnWarps * kKeys, n - 1);
+                vr[u][i] = *reinterpret_cast<const float4*>(vc + (size_t)key * DIM +
+                                                            4 * (v_part + kLanes * i));
+            }
+    };
+    if (v_first < n)
+        fetch_values(v_first);
+
     // ---- softmax over the block's keys; a thread's items all belong to head tid % HR ----
     const int my_head = threadIdx.x % HR;
     auto head_reduce = [&](float x, bool maximum) {
@@ -696,29 +720,17 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
     if (threadIdx.x == 0)
         s_odd[0] = 0.f;
 
-    // ---- P*V; a second time, on final probabilities, if a sum is not finite ----
-    for (int pass = 0;; ++pass) {
-        constexpr int kLanes = DIM / 4 < 32 ? DIM / 4 : 32;  // lanes per value row
-        constexpr int kV4 = DIM / 4 / kLanes;                // float4 per lane
-        constexpr int kKeys = 32 / kLanes;                   // keys per warp and step
-        constexpr int U = 8 / kV4;                           // steps in flight
-        const int part = lane % kLanes, sub = lane / kLanes;
+    // ---- P*V ----
+    {
         uint64_t acc[HR][2 * kV4];
 #pragma unroll
         for (int h = 0; h < HR; ++h)
 #pragma unroll
             for (int i = 0; i < 2 * kV4; ++i)
                 acc[h][i] = 0;
-        for (int j = warp * kKeys + sub; j < n; j += kAttnWarps * kKeys * U) {
-            float4 vr[U][kV4];
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int i = 0; i < kV4; ++i) {
-                    const int key = min(j + u * kAttnWarps * kKeys, n - 1);
-                    vr[u][i] = *reinterpret_cast<const float4*>(vc + (size_t)key * DIM +
-                                                                4 * (part + kLanes * i));
-                }
+        for (int j = v_first; j < n; j += kAttnWarps * kKeys * U) {
+            if (j != v_first)
+                fetch_values(j);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int key = j + u * kAttnWarps * kKeys;
@@ -754,108 +766,120 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
                     o.z = __fadd_rn(o.z, __shfl_xor_sync(0xffffffffu, o.z, 16));
                     o.w = __fadd_rn(o.w, __shfl_xor_sync(0xffffffffu, o.w, 16));
                 }
-                if (sub == 0)
+                if (v_sub == 0)
                     *reinterpret_cast<float4*>(s_acc + (warp * HR + h) * DIM +
-                                               4 * (part + kLanes * i)) = o;
+                                               4 * (v_part + kLanes * i)) = o;
             }
-        __syncthreads();
-        bool odd = false;
+    }
+    __syncthreads();
+    // where sums are not finite: once more on final probabilities, zero ones skipped
+    auto weigh_again = [&](float* sums) {
+#pragma unroll 1
         for (int i = threadIdx.x; i < HR * DIM; i += kAttnThreads) {
-            float a = s_acc[i];
-#pragma unroll
-            for (int w = 1; w < kAttnWarps; ++w)
-                a = __fadd_rn(a, s_acc[w * HR * DIM + i]);
-            const int h = i / DIM;
-            if (ranges == 1) {
-                if (!pass)
-                    a = __fdiv_rn(a, s_sum[h]);
-                if (h < nh)
-                    out[row0 + i] = a;
-            } else {
-                s_out[i] = a;
+            const int h = i / DIM, d = i % DIM;
+            float a = 0.f;
+#pragma unroll 1
+            for (int j = 0; j < n; ++j) {
+                const float p = s_sc[j * HR + h];
+                if (p != 0.f)
+                    a = __fmaf_rn(vc[(size_t)j * DIM + d], p, a);
             }
-            odd |= !(fabsf(a) <= FLT_MAX);
+            sums[i] = a;
         }
+    };
+    bool odd = false;
+    for (int i = threadIdx.x; i < HR * DIM; i += kAttnThreads) {
+        float a = s_acc[i];
+#pragma unroll
+        for (int w = 1; w < kAttnWarps; ++w)
+            a = __fadd_rn(a, s_acc[w * HR * DIM + i]);
         if (ranges == 1) {
-            if (pass || !__syncthreads_or(odd))
-                return;
+            a = __fdiv_rn(a, s_sum[i / DIM]);
+            if (i / DIM < nh)
+                out[row0 + i] = a;
+        } else {
+            s_out[i] = a;
+        }
+        odd |= !(fabsf(a) <= FLT_MAX);
+    }
+    if (ranges == 1) {
+        if (__syncthreads_or(odd)) {
             const float inv = __fdiv_rn(1.f, s_sum[my_head]);
             for (int i = threadIdx.x; i < n * HR; i += kAttnThreads)
                 s_sc[i] = __fmul_rn(s_sc[i], inv);
             __syncthreads();
-            continue;
+            weigh_again(s_out);  // a thread's own sums
+            for (int i = threadIdx.x; i < nh * DIM; i += kAttnThreads)
+                out[row0 + i] = s_out[i];
         }
-        if (odd)
-            s_odd[0] = 1.f;
-        cluster.sync();
-        if (pass)
-            break;
+        return;
+    }
+    if (odd)
+        s_odd[0] = 1.f;
+    cluster.sync();
 
-        // weights of the merge; warp h: head h's, lane c: block c of the cluster
-        if (warp < HR) {
-            const int c = min(lane, ctas - 1);
-            const bool in = lane < ctas;
-            const float mc = in ? cluster.map_shared_rank(s_max, c)[warp] : -INFINITY;
-            const float lc = in ? cluster.map_shared_rank(s_sum, c)[warp] : 0.f;
-            const float odd = in ? cluster.map_shared_rank(s_odd, c)[0] : 0.f;
-            float top = mc;
+    // ---- merge ----
+    // weights: warp h, head h's; lane c, block c of the cluster
+    if (warp < HR) {
+        const int c = lane % CTAS;
+        const bool in = lane < CTAS;
+        const float mc = in ? cluster.map_shared_rank(s_max, c)[warp] : -INFINITY;
+        const float lc = in ? cluster.map_shared_rank(s_sum, c)[warp] : 0.f;
+        const float any = in ? cluster.map_shared_rank(s_odd, c)[0] : 0.f;
+        float top = mc;
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-            const float w = (float)exp((double)__fsub_rn(mc, top));
-            float l = in ? __fmul_rn(w, lc) : 0.f;
+        for (int off = 16; off > 0; off >>= 1)
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+        const float w = (float)exp((double)__fsub_rn(mc, top));
+        float l = in ? __fmul_rn(w, lc) : 0.f;
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-                l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, off));
-            if (in)
-                s_weight[warp * kMaxRanges + lane] = w;
-            if (lane == 0)
-                s_total[warp] = l;
-            const bool any = __any_sync(0xffffffffu, odd != 0.f);
-            if (threadIdx.x == 0)
-                s_odd[1] = any ? 1.f : 0.f;
-        }
-        __syncthreads();
-        if (s_odd[1] == 0.f)  // the same in every block of the cluster
-            break;
+        for (int off = 16; off > 0; off >>= 1)
+            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, off));
+        if (in)
+            s_weight[warp * kMaxRanges + lane] = w;
+        if (lane == 0)
+            s_total[warp] = l;
+        const bool again = __any_sync(0xffffffffu, any != 0.f);
+        if (threadIdx.x == 0)
+            s_odd[1] = again ? 1.f : 0.f;
+    }
+    __syncthreads();
+    if (s_odd[1] != 0.f) {  // the same in every block of the cluster
         const float w = s_weight[my_head * kMaxRanges + rank];
         const float inv = __fdiv_rn(1.f, s_total[my_head]);
         for (int i = threadIdx.x; i < n * HR; i += kAttnThreads)
             s_sc[i] = __fmul_rn(__fmul_rn(s_sc[i], w), inv);
         __syncthreads();  // scores final, weights read
+        weigh_again(s_out);
         for (int i = threadIdx.x; i < HR * kMaxRanges; i += kAttnThreads)
             s_weight[i] = 1.f;
         if (threadIdx.x < HR)
             s_total[threadIdx.x] = 1.f;
+        cluster.sync();
     }
-
-    // ---- merge ----
-    const int share = HR * DIM / ctas;  // outputs per block, a power of two
-    for (int i = rank * share + threadIdx.x; i < (rank + 1) * share; i += kAttnThreads) {
-        const int h = i / DIM;
-        float o[kMaxRanges];
+    constexpr int kShare = HR * DIM / CTAS;  // outputs per block
+    for (int u = threadIdx.x; u < kShare; u += kAttnThreads) {
+        const int i = rank * kShare + u, h = i / DIM;
+        float o[CTAS];
 #pragma unroll
-        for (int c = 0; c < kMaxRanges; ++c)
-            if (c < ctas)
-                o[c] = cluster.map_shared_rank(s_out, c)[i];
+        for (int c = 0; c < CTAS; ++c)
+            o[c] = cluster.map_shared_rank(s_out, c)[i];
         float a = 0.f;
 #pragma unroll
-        for (int c = 0; c < kMaxRanges; ++c)
-            if (c < ctas) {
-                const float w = s_weight[h * kMaxRanges + c];
-                if (w != 0.f)
-                    a = __fmaf_rn(w, o[c], a);
-            }
+        for (int c = 0; c < CTAS; ++c) {
+            const float w = s_weight[h * kMaxRanges + c];
+            if (w != 0.f)
+                a = __fmaf_rn(w, o[c], a);
+        }
         float l = s_total[h];  // NaN if any score was
         if (!(fabsf(a) <= FLT_MAX)) {  // finite sums that overflow together
             a = 0.f;
-#pragma unroll
-            for (int c = 0; c < kMaxRanges; ++c)
-                if (c < ctas) {
-                    const float w = __fdiv_rn(s_weight[h * kMaxRanges + c], l);
-                    if (w != 0.f)
-                        a = __fmaf_rn(w, o[c], a);
-                }
+#pragma unroll 1
+            for (int c = 0; c < CTAS; ++c) {
+                const float w = __fdiv_rn(s_weight[h * kMaxRanges + c], l);
+                if (w != 0.f)
+                    a = __fmaf_rn(w, cluster.map_shared_rank(s_out, c)[i], a);
+            }
             l = 1.f;
         }
         if (h < nh)
@@ -1277,8 +1301,9 @@ double tile_time(int tokens, int rep, int rows, int kv_heads, int past, int sms)
 //              cluster costs 2 to 3 us, more where there are many; 32 / 8 heads of 128, one
 //              block against clusters: one token, 64 keys 5.1 / 5.6 us, 160 keys 7.1 / 5.8; 16
 //              tokens, 300 keys 12.6 / 15.7, 1000 keys 36 / 26.  The cluster sizes keep all of
-//              them resident at once: sixteen against eight, one token, 6000 keys 22.6 / 34.1,
-//              seven tokens 73 / 62, with four 59.
+//              them resident at once (`places`, short of the last): sixteen against eight, one
+//              token, 6000 keys 21.4 / 32.2, seven tokens 71 / 60, with four 59; and behind 300
+//              keys eight are enough, one token 6.9 / 5.9.
 //   up to      10 groups per multiprocessor; against the tile kernel: 32 / 8 heads of 128, 100
 //              tokens behind 300 keys 41 / 57 us, 256 tokens 108 / 108; 16 / 8 heads of 64, 160
 //              tokens 36 / 42, 256 tokens 56 / 49.
@@ -1304,9 +1329,10 @@ AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int c
     if (aligned && groups / tokens <= 65535 &&
         (tokens < 8 || (capacity >= 384 && groups <= 10l * sm_count))) {
         p.form = ATTN_SPLIT;
-        p.ctas = capacity > 1024 && groups * 32 <= 3l * sm_count ? 16
-                 : groups * 8 <= 2l * sm_count                   ? 8
-                                                                 : 4;
+        const long places = (long)split_blocks(dim, hr) * sm_count;
+        p.ctas = capacity >= 768 && groups * 16 * 5 <= places * 4 ? 16
+                 : groups * 8 * 10 <= places * 9                  ? 8
+                                                                  : 4;
         p.one_range = (int)min(4096l, max(p.ctas == 16 ? 96l : 128l, groups * groups / 32));
         while (p.ctas > max_cluster)
             p.ctas /= 2;
@@ -1324,66 +1350,74 @@ AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int c
     return p;
 }
 
-// The largest cluster of the kernel, up to `want` blocks, that the device can hold (a slice of
-// it may not have sixteen or eight multiprocessors side by side); 0: none.
+// Whether the device can hold a cluster of the kernel (a slice of it may not have sixteen, or
+// eight, multiprocessors side by side).
+constexpr size_t kMaxBlockSmem = 220 * 1024;
 template <typename Kernel>
-int placeable_cluster(b2w4_ctx* ctx, Kernel kern, int want, size_t smem) {
-    for (int c = want; c > 1; c /= 2) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(c);
-        cfg.blockDim = dim3(kAttnThreads);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = c;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
-            return c;
-        (void)cudaGetLastError();
-    }
-    return 0;
+bool cluster_fits(Kernel kern, int ctas) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kAttnThreads);
+    cfg.dynamicSmemBytes = 32 * 1024;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
+        return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
-template <int DIM, int HR>
-int launch_split_hr(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
-                    bool* placed) {
-    static b2w4_smem_optin cfg, wide, most;  // most: largest cluster + 1, per device
-    auto kern = attention_split_kernel<DIM, HR>;
-    const int rep = a.heads / a.kv_heads;
-    const bool one = keys <= plan.one_range;
-    B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, kern, wide));
-    size_t& largest = most.bytes[ctx->device];
-    auto bytes = [&](int ctas) {
-        const int range = max((keys + ctas - 1) / ctas, min(keys, plan.one_range));
-        return sizeof(float) * (SplitSmem<DIM, HR>::kScores + (size_t)range * HR);
-    };
-    if (!one && !largest) {
-        const size_t smem = sizeof(float) * SplitSmem<DIM, HR>::kScores + 64 * 1024;
-        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, cfg));
-        largest = 1 + placeable_cluster(ctx, kern, kMaxRanges, smem);
-    }
-    const int ctas = one ? 1 : min(plan.ctas, (int)largest - 1);
-    if (ctas < (one ? 1 : 2) || bytes(ctas) > 220 * 1024)
+template <int DIM, int HR, int CTAS>
+int launch_split_ctas(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
+                      bool* placed) {
+    static b2w4_smem_optin cfg, wide, fits;  // fits: 1 yes, 2 no, per device
+    auto kern = attention_split_kernel<DIM, HR, CTAS>;
+    const int range = max((keys + CTAS - 1) / CTAS, min(keys, plan.one_range));
+    const size_t smem = sizeof(float) * (SplitSmem<DIM, HR>::kScores + (size_t)range * HR);
+    const dim3 grid(CTAS, a.kv_heads * ((a.heads / a.kv_heads + HR - 1) / HR), a.tokens);
+    if (smem > kMaxBlockSmem)
         return B2W4_OK;  // not placed
-    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, bytes(ctas), cfg));
-    const dim3 grid(ctas, a.kv_heads * ((rep + HR - 1) / HR), a.tokens);
-    if (one)
-        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), bytes(1),
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, cfg));
+    if constexpr (CTAS == 1) {
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), smem,
                                            ctx->stream, a.q, a.k_cache, a.v_cache, a.out,
                                            a.tokens, a.heads, a.kv_heads, a.past, a.past_dev,
-                                           a.capacity, a.scale, 1, plan.one_range));
-    else
+                                           a.capacity, a.scale, plan.one_range));
+    } else {
+        B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, kern, wide));
+        size_t& fit = fits.bytes[ctx->device];
+        if (!fit)
+            fit = cluster_fits(kern, CTAS) ? 1 : 2;
+        if (fit == 2)
+            return B2W4_OK;
         B2W4_CUDA(ctx, b2w4_launch_chained_cluster(
-                           ctx->pdl, kern, grid, dim3(kAttnThreads), ctas, bytes(ctas),
-                           ctx->stream, a.q, a.k_cache, a.v_cache, a.out, a.tokens, a.heads,
-                           a.kv_heads, a.past, a.past_dev, a.capacity, a.scale, ctas,
-                           plan.one_range));
+                           ctx->pdl, kern, grid, dim3(kAttnThreads), CTAS, smem, ctx->stream,
+                           a.q, a.k_cache, a.v_cache, a.out, a.tokens, a.heads, a.kv_heads,
+                           a.past, a.past_dev, a.capacity, a.scale, plan.one_range));
+    }
     ctx->launches++;
     *placed = true;
     return B2W4_OK;
+}
+// The planned cluster, or the next smaller one that the device can place.
+template <int DIM, int HR>
+int launch_split_hr(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
+                    bool* placed) {
+    if (keys <= plan.one_range)
+        return launch_split_ctas<DIM, HR, 1>(ctx, a, keys, plan, placed);
+    int rc = B2W4_OK;
+    if (plan.ctas >= 16)
+        rc = launch_split_ctas<DIM, HR, 16>(ctx, a, keys, plan, placed);
+    if (rc == B2W4_OK && !*placed && plan.ctas >= 8)
+        rc = launch_split_ctas<DIM, HR, 8>(ctx, a, keys, plan, placed);
+    if (rc == B2W4_OK && !*placed && plan.ctas >= 4)
+        rc = launch_split_ctas<DIM, HR, 4>(ctx, a, keys, plan, placed);
+    return rc;
 }
 
 int launch_split(b2w4_ctx* ctx, const AttnArgs& a, int dim, int keys, const AttnPlan& plan,

@@ -482,7 +482,7 @@ def test_split_attention_on_either_side_of_one_range(ctx, tokens, past, heads, k
     c.close()
     want = _attention_fp64(q, k_all, v_all, heads, kv_heads, past, scale)
     assert rel_l2(outs[0], want) < 1e-5
-    if cluster >= 2:
+    if cluster >= 4:
         assert outs[1].tobytes() == outs[0].tobytes()
     else:  # few keys known to the host need no cluster; the device's position does
         assert rel_l2(outs[1], want) < 1e-5
