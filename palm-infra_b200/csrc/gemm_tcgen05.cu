@@ -146,7 +146,7 @@ gemm_w4a8_tc_kernel(const GemmArgs a) {
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    // accumulator b, token block mb: columns [b*256 + mb*RP, +RP)
+    // accumulator b, token block mb: columns [b*kAccCols + mb*RP, +RP)
     auto fail = [&]() {
         *s_abort = 1;
         b2w4_report_timeout(a.status);
@@ -356,15 +356,14 @@ gemm_w4a8_tc_kernel(const GemmArgs a) {
                 constexpr int kBatch = 24;
 #pragma unroll
                 for (int b0 = 0; b0 < CH; b0 += kBatch) {
-                    constexpr int kMaxB = kBatch;
-                    uint32_t r[kMaxB];
+                    uint32_t r[kBatch];
 #pragma unroll
-                    for (int c0 = 0; c0 < kMaxB; c0 += 8)
+                    for (int c0 = 0; c0 < kBatch; c0 += 8)
                         if (b0 + c0 < CH)
                             tmem_ld8(taddr + b0 + c0, *reinterpret_cast<uint32_t(*)[8]>(&r[c0]));
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int c = 0; c < kMaxB; c += 4) {
+                    for (int c = 0; c < kBatch; c += 4) {
                         if (b0 + c < CH) {
                             const float4 w4 =
                                 *reinterpret_cast<const float4*>(wsf + g * RP + b0 + c);
