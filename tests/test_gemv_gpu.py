@@ -303,6 +303,34 @@ def test_per32_tensor_core_tiles_bit_exact(ctx_tc, m, n, k):
     assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).tobytes()
 
 
+def _tiny_products(exponent, m=70, n=40, k=512):
+    """fp32 weight scales and activations whose scale products lie in 2^exponent times [1, 4)."""
+    rng = np.random.default_rng(-exponent)
+    q = rng.integers(-8, 8, (n, k)).astype(np.int8)
+    ws = (rng.uniform(1, 2, (n, k // 128)) * 2.0 ** -60).astype(np.float32)
+    x = rng.uniform(-1, 1, (m, k // 32, 32))
+    x /= np.abs(x).max(axis=2, keepdims=True)
+    x *= 127 * rng.uniform(1, 2, (m, k // 32, 1)) * 2.0 ** (exponent + 60)
+    return ol.bg128_encode(q, ws), np.ascontiguousarray(x.reshape(m, k).astype(np.float32)), n, k
+
+
+def test_per32_tensor_core_scales_near_the_smallest_normal(ctx_tc):
+    """The per-32 tcgen05 kernel stages weight scales as w / 16 and sums as 16 D: the oracle's
+    bits while every w * a / 16 is a normal number (2^-126 and up).  Below, the product loses
+    bits, at most 2^-150 each: with |16 D| <= 16 * 32 * 8 * 127 that is 2^19 * 2^-150 per
+    32-block, beside 2^15 * 2^-150 for the oracle's own product and fp32 rounding of the sum."""
+    blocks, x, n, k = _tiny_products(-122)
+    y, _ = run_gpu(ctx_tc, blocks, n, k, x, rule=ol.ACT_G32, sums=False)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).tobytes()
+    blocks, x, n, k = _tiny_products(-126)
+    y, _ = run_gpu(ctx_tc, blocks, n, k, x, rule=ol.ACT_G32, sums=False)
+    want = ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).astype(np.float64)
+    bound = (k // 32) * (2.0 ** 19 + 2.0 ** 15) * 2.0 ** -150 + \
+        2 * (k // 32) * 2.0 ** -24 * (k // 32) * 2.0 ** 15 * 2.0 ** -124
+    assert np.max(np.abs(y - want)) <= bound
+    assert np.max(np.abs(want)) > 50 * bound  # the results are far above it
+
+
 def test_config2_prefill_m256_reference_rule(ctx):
     """M=256, K=2560, N=9728 (benchmark configuration 2, prefill) under the reference's rule
     for several rows (per 32 values), the kernel the library picks by itself: bit-exact
