@@ -364,12 +364,18 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      positions past.., then causal attention of q
  *                      [tokens][heads][dim] over keys 0 .. past + t, softmax and
  *                      P*V in 32 bits (exp in 64; dim <= 256, about 47,000 keys at
- *                      most).  Heads of 64, 128 or 256 features on 16-byte aligned
- *                      rows: up to seven tokens split the keys over a cluster of
- *                      blocks, longer runs take a tiled form with a running softmax;
- *                      other sizes one block per (token, head);
+ *                      most in every form).  A key whose probability is zero in 32
+ *                      bits contributes nothing, whatever its value row holds.
+ *                      Forms, by sizes, capacity and alignment, not by position:
+ *                      heads of 64, 128 or 256 features on 16-byte aligned rows take
+ *                      the keys in one block or over a cluster of blocks (up to seven
+ *                      tokens, and runs that would leave most of the chip idle), or
+ *                      in tiles with a running softmax; any other size or alignment
+ *                      one block per (token, head), runs of the three head sizes
+ *                      tiles too.  The forms sum in different orders, so a token's
+ *                      row agrees between them to fp32 rounding, not bit for bit;
  *                      past_dev (optional)
- *                      gives `past` from device memory instead
+ *                      gives `past` from device memory instead (the same bits)
  *                      k_dev and v_dev both NULL: nothing is appended, the cache rows
  *                      past .. past + tokens - 1 are in place already (b2w4_qkv_prepare)
  *   b2w4_qkv_prepare   what sits between the fused qkv matmul and attention, in one

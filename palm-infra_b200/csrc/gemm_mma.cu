@@ -88,7 +88,7 @@ __device__ __forceinline__ void gm_wait_groups(int n) {
 // one stage = one 128-k group of every token: codes, scales, accumulator biases.  A group's
 // scales of all tokens are one contiguous run (m_pad tokens per scale), and so are its biases,
 // so all three are 16-byte copies dealt out by one index: with few tokens a thread issues at
-// most one.
+// most one (ring form, 16 rows, [4100, 9728]: 72 -> 65 us per 32 values, 44.3 -> 43.6 per 128).
 template <int SPG>
 __device__ __forceinline__ void load_stage(const GemmMmaArgs& a, int g, uint8_t* s_b, float* s_as,
                                            int* s_es) {
