@@ -1570,9 +1570,11 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
                                                            // for a full cache
     const bool aligned = !(((uintptr_t)q_dev | (uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev |
                             (uintptr_t)out_dev) & 15);
-    const AttnPlan plan = attn_plan(tokens, heads, kv_heads, dim,
-                                    past_dev ? capacity - tokens : past, capacity, aligned,
-                                    !ctx->attn_tiles, ctx->attn_cluster, ctx->sm_count);
+    auto plan_for = [&](int cap) {
+        return attn_plan(tokens, heads, kv_heads, dim, past_dev ? capacity - tokens : past, cap,
+                         aligned, !ctx->attn_tiles, ctx->attn_cluster, ctx->sm_count);
+    };
+    AttnPlan plan = plan_for(capacity);
     const int score_slots = (keys + 3) & ~3;
     if (sizeof(float) * ((size_t)score_slots + kAttnStage) > 200 * 1024)
         return b2w4_fail(ctx, B2W4_E_INVALID, "attention: %d keys exceed the score buffer", keys);
@@ -1591,6 +1593,7 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
         const int rc = launch_split(ctx, a, dim, keys, plan, &placed);
         if (rc != B2W4_OK || placed)
             return rc;
+        plan = plan_for(0);  // no cluster fits: runs as on a small cache, few tokens by row
     }
     if (plan.form == ATTN_TILE)
         return launch_tile(ctx, a, dim, plan, aligned);

@@ -449,12 +449,12 @@ def test_attention_ignores_value_rows_of_zero_probability(ctx, tokens, heads, kv
 @pytest.mark.parametrize("cluster", [0, 1, 3, 4, 8, 16])
 @pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [
     (1, 94, 8, 2, 64), (3, 94, 4, 2, 128), (2, 126, 3, 3, 128), (7, 126, 6, 1, 256),
-    (1, 1500, 8, 2, 128), (5, 700, 5, 5, 64)])
+    (1, 1500, 8, 2, 128), (5, 700, 5, 5, 64), (12, 1200, 4, 2, 64)])
 def test_split_attention_on_either_side_of_one_range(ctx, tokens, past, heads, kv_heads, dim,
                                                      cluster):
     """Runs whose tokens see 95 .. 133 keys, the last counts that one block takes alone and the
     first that a cluster splits, and longer ones; clusters of every size that a device may
-    allow, and none (one block per (token, head)).  Position on the host or on the device: the
+    allow, and none (one block per (token, head), or tiles).  Position on the host or on the device: the
     same bits.  Tolerance as for the split kernel."""
     import os
     import torch
