@@ -14,6 +14,8 @@
 // sums, fp32 chain in group order), so a route's result equals a one-row GEMV of that
 // expert's weight slice.  Nothing is atomically accumulated: every output is written by one
 // thread in a fixed order.
+#include <type_traits>
+
 #include "b200w4_internal.cuh"
 
 namespace {
@@ -500,6 +502,67 @@ moe_route_fused_kernel(const float* __restrict__ hidden, int ldx, int tokens, in
 // ---- 6. SwiGLU + quantiser: one warp per (route, 128-wide group of I) ------------------
 // inter = (g * 1/(1+exp(-g))) * u with gate = columns [0,I), up = [I,2I)
 // (kernels/moe.cpp:160-183), then the per-128 quantiser; codes in tensor-operand order.
+// The grouped matmul multiplies unsigned nibbles q+8: its int32 accumulator starts at
+// 0x4B400000 - 8 * (sum of the codes), per group or per 32-block (dst[0..3], the lane's block is
+// lane / 8).  `sum`: of the lane's four codes.
+__device__ __forceinline__ void store_code_bias(int sum, int lane, bool a32, int32_t* dst) {
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1)  // integer: order-free
+        sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (a32) {
+        if ((lane & 7) == 0)
+            dst[lane >> 3] = 0x4B400000 - 8 * sum;
+        return;
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+    if (lane == 0)
+        *dst = 0x4B400000 - 8 * sum;
+}
+
+// Hidden rows for the grouped matmul, one warp per (token, 128-group): codes in tensor-operand
+// order, scales and accumulator biases per 128 values, and (q32 != null) per 32 values as well.
+__global__ void moe_quantize_hidden_kernel(const float* __restrict__ hidden, int ldx, int tokens,
+                                           int hidden_size, int8_t* __restrict__ q,
+                                           float* __restrict__ scales, int32_t* __restrict__ es,
+                                           int8_t* __restrict__ q32, float* __restrict__ scales32,
+                                           int32_t* __restrict__ es32) {
+    b2w4_pdl_chain_entry();
+    const int G = hidden_size >> 7;
+    const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (wid >= (long long)tokens * G)
+        return;
+    const int row = (int)(wid / G), g = (int)(wid % G);
+    const float* src = hidden + (size_t)row * ldx + (size_t)g * 128 + lane * 4;
+    const float v[4] = {src[0], src[1], src[2], src[3]};
+    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1)  // the lane's 32-block: eight lanes
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    const size_t at = (size_t)row * hidden_size + (size_t)g * 128 + ((lane & 7) >> 1) * 32 +
+                      (lane >> 3) * 4 + (lane & 1) * 2;
+    auto store = [&](float max, bool a32, int8_t* dst, float* scale_dst, int32_t* bias_dst) {
+        float scale, inv;
+        b2w4_quant_params(max, scale, inv);
+        const int c0 = b2w4_quant_code(v[0], inv), c1 = b2w4_quant_code(v[1], inv);
+        const int c2 = b2w4_quant_code(v[2], inv), c3 = b2w4_quant_code(v[3], inv);
+        if (a32 ? (lane & 7) == 0 : lane == 0)
+            scale_dst[a32 ? lane >> 3 : 0] = scale;
+        store_code_bias(c0 + c1 + c2 + c3, lane, a32, bias_dst);
+        *reinterpret_cast<char2*>(dst) = make_char2((signed char)c0, (signed char)c2);
+        *reinterpret_cast<char2*>(dst + 16) = make_char2((signed char)c1, (signed char)c3);
+    };
+    if (q32) {
+        const size_t s = ((size_t)row * G + g) * 4;
+        store(amax, true, q32 + at, scales32 + s, es32 + s);
+    }
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 8));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 16));
+    const size_t s = (size_t)row * G + g;
+    store(amax, false, q + at, scales + s, es + s);
+}
+
 // one warp: 128 values of one route, written to `group_dst` (the 128 code bytes of the group)
 // and `scale_dst`
 // a32: one scale per 32 values (scale_dst[0..3], the lane's block is lane / 8) instead of one
@@ -507,7 +570,7 @@ moe_route_fused_kernel(const float* __restrict__ hidden, int ldx, int tokens, in
 __device__ __forceinline__ void swiglu_quant_warp(const float* __restrict__ gate_row,
                                                   const float* __restrict__ up_row, int lane,
                                                   int8_t* group_dst, float* scale_dst,
-                                                  bool a32 = false) {
+                                                  bool a32 = false, int32_t* bias_dst = nullptr) {
     const float* gp = gate_row + lane * 4;
     const float* up = up_row + lane * 4;
     float v[4];
@@ -536,6 +599,8 @@ __device__ __forceinline__ void swiglu_quant_warp(const float* __restrict__ gate
     } else if (lane == 0) {
         *scale_dst = scale;
     }
+    if (bias_dst)
+        store_code_bias(c0 + c1 + c2 + c3, lane, a32, bias_dst);
     // tensor-operand order inside the group: [word position][even words of the four
     // 32-blocks, then the odd words]; the lane holds k = 4*lane..+3: 32-block lane/8, even
     // codes at even index 2*(lane%8), 2*(lane%8)+1
@@ -544,13 +609,13 @@ __device__ __forceinline__ void swiglu_quant_warp(const float* __restrict__ gate
     *reinterpret_cast<char2*>(blk + 16) = make_char2((signed char)c1, (signed char)c3);
 }
 
-// scales: [routes][scale_stride].  offsets (null = per-128 everywhere): first compact route of
+// scales, es (accumulator biases): [routes][scale_stride].  offsets (null = per-128 everywhere): first compact route of
 // every expert, [num_experts + 1]; a route whose expert holds several routes is quantised per
 // 32 values (scales[r][4*g + block]), a lone route per 128 (scales[r][g]).
 __global__ void moe_swiglu_quant_kernel(const float* __restrict__ gu, int routes,
                                         int intermediate, int8_t* __restrict__ q,
-                                        float* __restrict__ scales, int scale_stride,
-                                        const int32_t* __restrict__ offsets, int num_experts,
+                                        float* __restrict__ scales, int32_t* __restrict__ es,
+                                        int scale_stride, const int32_t* __restrict__ offsets, int num_experts,
                                         const int32_t* __restrict__ route_lo,
                                         const int32_t* __restrict__ route_hi) {
     b2w4_pdl_chain_entry();
@@ -578,7 +643,8 @@ __global__ void moe_swiglu_quant_kernel(const float* __restrict__ gu, int routes
     const float* gp = gu + (size_t)r * 2 * intermediate + (size_t)g * 128;
     swiglu_quant_warp(gp, gp + intermediate, lane,
                       q + (size_t)r * intermediate + (size_t)g * 128,
-                      scales + (size_t)r * scale_stride + (a32 ? g * 4 : g), a32);
+                      scales + (size_t)r * scale_stride + (a32 ? g * 4 : g), a32,
+                      es + (size_t)r * scale_stride + (a32 ? g * 4 : g));
 }
 
 // ---- 8. combine: one block per (token, 512 hidden columns) -------------------------------
@@ -1012,44 +1078,55 @@ size_t grouped_small_smem(int k, int groups, int tpc, bool scl16) {
 }
 
 // ---- 5 / 7. grouped expert matmul over ragged route lists ------------------------------
-// grid = (CTAs per expert, experts that have routes).  CTA (c, y) owns `tpc` 8-row tiles of
-// one expert's slice of the aggregate weight and every route of that expert.  The slice's
-// nibble stream is bulk-copied into shared memory once and reused for all of the expert's
-// routes, sixteen at a time.  The integer sums come from the warp-level int8 tensor
-// instruction (mma.sync m16n8k32): 16 weight rows of a tile pair are its rows, eight routes
-// its columns.  A warp owns one tile pair and one or two column blocks and runs the whole K
-// loop on its own: per 128-k group it splits its weight words into unsigned bytes q+8
-// (lo = (w ^ 0x08080808) & 0x0F0F0F0F for even k, hi = ((w >> 4) ^ 0x08080808) & 0x0F0F0F0F
-// for odd k), accumulates four instructions into an int32 that starts at
-// 0x4B400000 - 8*sum(codes) and therefore ends as the bit pattern of the float 12582912 + D,
-// and folds D into fp32 chain values  y = fma(float(D), fp32(ws*as), y)  that stay in its
-// registers until the last group: no shared-memory hand-off, no barrier inside the K loop.
-// The math is the dense kernels', route by route.
+// Work: an expert's routes, sixteen at a time (a pass), against its tile pairs (16 weight rows
+// each).  A unit is one pass against eight pairs, a pair per warp; the units of all experts lie
+// in one line (expert, pass, pairs) of which every CTA takes an equal, contiguous share, two
+// CTAs per SM, so that one computes while the other changes to another pass.  A pass's int8
+// rows, scales and accumulator biases are staged in shared memory once and serve all units of
+// the share that belong to it.
+//
+// The integer sums come from the warp-level int8 tensor instruction (mma.sync m16n8k32): the
+// pair's weight rows are its rows, eight routes its columns.  A warp runs the whole K loop of its
+// pair on its own, with the weights straight from global memory: a 32-k block of a tile is 128
+// contiguous bytes, a word per lane, fetched kAhead groups before use (16 warps x 32 lanes x 10
+// words x 3 groups: 60 KB in flight per SM).  A word is split into unsigned bytes q+8
+// (lo = (w ^ 0x08080808) & 0x0F0F0F0F for even k, hi = ((w >> 4) ^ 0x08080808) & 0x0F0F0F0F for
+// odd k); the accumulator starts at 0x4B400000 - 8*sum(codes), read from shared memory as the
+// four words the instruction takes, and ends as the bit pattern of the float 12582912 + D.  D is
+// folded into fp32 chain values  y = fma(float(D), fp32(ws*as), y)  that stay in the warp's
+// registers until the last group, two columns per instruction.  The math is the dense kernels',
+// route by route.
+// What bounds it: issue slots (about 120 instructions per group and pair with sixteen routes,
+// most of them the chain and the split of the words), close to the time the weights take from
+// HBM at sixteen routes per expert.
 constexpr int kGW = 8;          // warps
 constexpr int kGT = kGW * 32;
 constexpr int kGR = 16;         // routes per pass: two column blocks
 constexpr int kRowPad = 16;     // bytes added to a staged activation row: conflict-free reads
+constexpr int kAhead = 3;       // groups whose weights are in flight per warp
 
 struct GroupedArgs {
     const uint8_t* nib;
     const void* scl;
     const int8_t* qa;         // [rows][K] int8, tensor-operand order inside each group
     const float* as;          // [rows][as_stride]: one scale per 128 values at [g]
+    const int32_t* es;        // same shape: 0x4B400000 - 8 * (sum of the group's codes)
     // The reference's rule for an expert that holds SEVERAL rows (kernels/moe.cpp:1055-1058
-    // -> kernels/matmul_w4.cpp:1125-1154): one activation scale per 32 values.  qa32 / as32
-    // are those rows quantised that way (as32[r][4*g + block]); null = per-128 for every
+    // -> kernels/matmul_w4.cpp:1125-1154): one activation scale per 32 values.  qa32 / as32 /
+    // es32 are those rows quantised that way (as32[r][4*g + block]); null = per-128 for every
     // expert.  An expert with a single row keeps the per-128 rule (:1058-1075).
     const int8_t* qa32;
     const float* as32;
+    const int32_t* es32;
     int as_stride, as32_stride;
     const int4* slots;        // y-th expert with routes: (expert, first route, end), else empty
+    int slot_count;           // entries of slots that can hold an expert
     int num_experts_all;      // experts routed over
     int expert_begin;         // first expert whose weights this aggregate holds
     int expert_count;         // experts held
     const int32_t* row_map;   // route -> activation row, or null for identity
     float* out;               // [routes][n_e]
-    int* status;
-    int k, groups, n_e, tiles_e, tpc;
+    int k, groups, n_e, tiles_e;
 };
 
 template <int BYTES>
@@ -1062,14 +1139,96 @@ __device__ __forceinline__ void moe_cp_async(void* dst, const void* src) {
 
 __device__ __forceinline__ void moe_mma_16x8x32(int (&d)[4], uint32_t a0, uint32_t a1,
                                                 uint32_t a2, uint32_t a3, uint32_t b0,
-                                                uint32_t b1) {
+                                                uint32_t b1, int4 c) {
     // lane (gid = lane/4, tid = lane%4): a0 row gid, k 4*tid..+3; a1 row gid+8; a2/a3 k+16;
     // b0 k 4*tid..+3 of column gid, b1 k+16; d0/d1 row gid, columns 2*tid, 2*tid+1; d2/d3 row
     // gid+8.  A unsigned bytes, B signed bytes.
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-        "{%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+        "{%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c.x), "r"(c.y), "r"(c.z),
+          "r"(c.w));
+}
+
+// one group's weights of a lane: a word of each 32-k block of both tiles' row gid, both scales
+template <bool SCL16>
+struct PairWords {
+    uint32_t w[2][4];
+    float ws[2];
+    __device__ __forceinline__ void load(const uint8_t* nib, size_t tile_bytes, const uint8_t* scl,
+                                         size_t scl_tile_bytes, int g) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const uint8_t* p = nib + t * tile_bytes + g * 512;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                w[t][b] = __ldg(reinterpret_cast<const uint32_t*>(p + b * 128));
+            const uint8_t* q = scl + t * scl_tile_bytes + g * (SCL16 ? 16 : 32);
+            ws[t] = SCL16 ? __half2float(*reinterpret_cast<const __half*>(q))
+                          : *reinterpret_cast<const float*>(q);
+        }
+    }
+};
+
+// Folds one group of sixteen weight rows into the chain values of `ncb` blocks of eight routes.
+// acc[j][0]: row gid, routes 2*tid and 2*tid+1 of block j; acc[j][1]: row gid+8.
+template <bool A32, bool SCL16>
+__device__ __forceinline__ void pair_group(const PairWords<SCL16>& pw, const uint8_t* rows,
+                                           int row_bytes, const float* s_as, const int4* s_bias,
+                                           int g, int ncb, int tid, uint64_t (&acc)[2][2]) {
+    uint32_t lo[2][4], hi[2][4];
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            lo[t][b] = (pw.w[t][b] ^ 0x08080808u) & 0x0F0F0F0Fu;
+            hi[t][b] = ((pw.w[t][b] >> 4) ^ 0x08080808u) & 0x0F0F0F0Fu;
+        }
+    const uint64_t magic = b2w4_pack2(12582912.f, 12582912.f);
+    const uint64_t w0 = b2w4_pack2(pw.ws[0], pw.ws[0]), w1 = b2w4_pack2(pw.ws[1], pw.ws[1]);
+    auto fold = [&](const int (&c)[4], uint64_t as2, uint64_t (&y)[2]) {
+        // c = 0x4B400000 + D: as a float 12582912 + D, exactly
+        const uint64_t d0 = b2w4_sub2(b2w4_pack2(__int_as_float(c[0]), __int_as_float(c[1])), magic);
+        const uint64_t d1 = b2w4_sub2(b2w4_pack2(__int_as_float(c[2]), __int_as_float(c[3])), magic);
+        y[0] = b2w4_fma2(d0, b2w4_mul2(w0, as2), y[0]);
+        y[1] = b2w4_fma2(d1, b2w4_mul2(w1, as2), y[1]);
+    };
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        if (j < ncb) {  // warp-uniform; unused columns of the last block are never stored
+            const uint4* bp = reinterpret_cast<const uint4*>(rows + j * 8 * row_bytes + g * 128);
+            const uint4 be = bp[0], bo = bp[1];
+            const uint32_t bev[4] = {be.x, be.y, be.z, be.w}, bov[4] = {bo.x, bo.y, bo.z, bo.w};
+            if (A32) {
+                // one instruction = one 32-block: its own accumulator, bias and activation
+                // scale, folded in ascending block order (kernels/matmul_w4.cpp:785-901)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const int at = (g * 4 + b) * (kGR / 2) + j * 4 + tid;
+                    int c[4];
+                    moe_mma_16x8x32(c, lo[0][b], lo[1][b], hi[0][b], hi[1][b], bev[b], bov[b],
+                                    s_bias[at]);
+                    fold(c, reinterpret_cast<const uint64_t*>(s_as)[at], acc[j]);
+                }
+            } else {
+                // two chains of two instructions (latency), joined by one add
+                const int at = g * (kGR / 2) + j * 4 + tid;
+                int c[4], c2[4];
+                moe_mma_16x8x32(c, lo[0][0], lo[1][0], hi[0][0], hi[1][0], bev[0], bov[0],
+                                s_bias[at]);
+                moe_mma_16x8x32(c2, lo[0][1], lo[1][1], hi[0][1], hi[1][1], bev[1], bov[1],
+                                make_int4(0, 0, 0, 0));
+                moe_mma_16x8x32(c, lo[0][2], lo[1][2], hi[0][2], hi[1][2], bev[2], bov[2],
+                                make_int4(c[0], c[1], c[2], c[3]));
+                moe_mma_16x8x32(c2, lo[0][3], lo[1][3], hi[0][3], hi[1][3], bev[3], bov[3],
+                                make_int4(c2[0], c2[1], c2[2], c2[3]));
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    c[i] += c2[i];
+                fold(c, reinterpret_cast<const uint64_t*>(s_as)[at], acc[j]);
+            }
+        }
+    }
 }
 
 template <bool SCL16>
@@ -1077,223 +1236,147 @@ __global__ void __launch_bounds__(kGT, 2)
 moe_grouped_gemv_kernel(const GroupedArgs a) {
     b2w4_pdl_chain_entry();
     extern __shared__ __align__(128) uint8_t smem[];
-    // blockIdx.y walks the experts that have routes, not all experts: a decode token
-    // touches top_k of them
-    const int4 slot = a.slots[blockIdx.y];
-    const int e_all = slot.x, r0 = slot.y, r1 = slot.z;
-    const int e = e_all - a.expert_begin;  // index inside the aggregate held here
-    if (e < 0 || e >= a.expert_count)
-        return;
-    const int tl0 = blockIdx.x * a.tpc;
-    const int ntile = min(a.tpc, a.tiles_e - tl0);
-    if (r0 >= r1 || ntile <= 0)
-        return;
     const int G = a.groups, K = a.k;
-    const int tile_bytes = G * 512;
-    const int scl_tile_bytes = G * 8 * (SCL16 ? 2 : 4);
     const int row_bytes = K + kRowPad;
-    uint8_t* s_w = smem;
-    uint8_t* s_scl = s_w + (size_t)a.tpc * tile_bytes;
-    uint8_t* s_qa = s_scl + (size_t)a.tpc * scl_tile_bytes;                         // [kGR][K+pad]
-    // per (group or 32-block, route): activation scale and accumulator bias; sized for the
-    // per-32 rule (four entries per group)
-    float* s_as = reinterpret_cast<float*>(s_qa + (size_t)kGR * row_bytes);         // [4G][kGR]
-    int* s_bias = reinterpret_cast<int*>(s_as + kGR * G * 4);                       // [4G][kGR]
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(
-        (reinterpret_cast<uintptr_t>(s_bias + kGR * G * 4) + 7) & ~uintptr_t(7));
-    // the expert's rule: per 32 values when it holds several rows
-    const bool a32 = a.qa32 != nullptr && (r1 - r0) >= 2;
-    const int8_t* const qa_src = a32 ? a.qa32 : a.qa;
-    const float* const as_src = a32 ? a.as32 : a.as;
-    const int as_stride = a32 ? a.as32_stride : a.as_stride;
-    const int SPG = a32 ? 4 : 1;  // scales per group
-
+    // per (group or 32-block, route): accumulator bias and activation scale; sized for the
+    // per-32 rule (four entries per group).  A bias is stored as the instruction takes it:
+    // (b[2p], b[2p+1], b[2p], b[2p+1]) for the route pair p.
+    int4* s_bias = reinterpret_cast<int4*>(smem);                                 // [4G][kGR / 2]
+    float* s_as = reinterpret_cast<float*>(s_bias + (size_t)4 * G * (kGR / 2));   // [4G][kGR]
+    uint8_t* s_qa = reinterpret_cast<uint8_t*>(s_as + (size_t)4 * G * kGR);       // [kGR][K+pad]
+    int* s_pre = reinterpret_cast<int*>(s_qa + (size_t)kGR * row_bytes);          // [slots + 1]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tid = lane & 3;
-    const size_t gtile0 = (size_t)e * a.tiles_e + tl0;  // tile index in the aggregate
 
+    // passes before slot y (experts held elsewhere have none)
     if (warp == 0) {
-        if (lane == 0)
-            mbar_init(&s_bar[0], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-            const uint32_t wb = (uint32_t)ntile * tile_bytes, sb = (uint32_t)ntile * scl_tile_bytes;
-            mbar_expect_tx(&s_bar[0], wb + sb);
-            bulk_g2s(s_w, a.nib + gtile0 * tile_bytes, wb, &s_bar[0]);
-            bulk_g2s(s_scl, reinterpret_cast<const uint8_t*>(a.scl) + gtile0 * scl_tile_bytes, sb,
-                     &s_bar[0]);
+        int carry = 0;
+        for (int y0 = 0; y0 < a.slot_count; y0 += 32) {
+            int passes = 0;
+            if (y0 + lane < a.slot_count) {
+                const int4 slot = a.slots[y0 + lane];
+                const int e = slot.x - a.expert_begin;
+                if (e >= 0 && e < a.expert_count && slot.z > slot.y)
+                    passes = (slot.z - slot.y + kGR - 1) / kGR;
+            }
+            int run = passes;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int other = __shfl_up_sync(0xffffffffu, run, off);
+                if (lane >= off)
+                    run += other;
+            }
+            if (y0 + lane < a.slot_count)
+                s_pre[y0 + lane] = carry + run - passes;
+            carry += __shfl_sync(0xffffffffu, run, 31);
         }
+        if (lane == 0)
+            s_pre[a.slot_count] = carry;
     }
-    // this warp's tile pair and column blocks: with fewer pairs than warps the two column
-    // blocks of a pass go to different warps, otherwise a warp takes both (one split of the
-    // weight words serves both)
-    const int npair = (ntile + 1) >> 1;
-    const int npair_cap = (a.tpc + 1) >> 1;
-    const int wpp = npair_cap < kGW ? (kGW / npair_cap >= 2 ? 2 : 1) : 1;  // warps per pair
-    const uint32_t* s_w32 = reinterpret_cast<const uint32_t*>(s_w);
-    const int tile_words = tile_bytes >> 2;
-    bool weights_ready = false;
+    __syncthreads();
+    // tiles_e is a multiple of 16 (n_e is one of 128): whole rounds of kGW pairs
+    const int rounds = a.tiles_e / (2 * kGW);
+    const long long total = (long long)s_pre[a.slot_count] * rounds;
+    long long u = total * blockIdx.x / gridDim.x;
+    const long long u_end = total * (blockIdx.x + 1) / gridDim.x;
+    const size_t tile_bytes = (size_t)G * 512, scl_tile_bytes = (size_t)G * (SCL16 ? 16 : 32);
 
-    for (int base = r0; base < r1; base += kGR) {
-        const int mc = min(kGR, r1 - base);
-        // quantised activations of this pass's routes, a warp per row, all copies in flight at
-        // once (through registers a thread's eight loads were eight memory latencies;
-        // 256 tokens on 128 experts of 768, the whole operator: 330 -> 315 us)
+    while (u < u_end) {
+        const int pass_all = (int)(u / rounds);
+        const int round0 = (int)(u - (long long)pass_all * rounds);
+        const int round1 = (int)min((long long)rounds, round0 + (u_end - u));
+        u += round1 - round0;
+        int y = 0, y_hi = a.slot_count;  // the slot of this pass: s_pre[y] <= pass < s_pre[y+1]
+        while (y_hi - y > 1) {
+            const int mid = (y + y_hi) >> 1;
+            if (s_pre[mid] <= pass_all)
+                y = mid;
+            else
+                y_hi = mid;
+        }
+        const int4 slot = a.slots[y];
+        const int base = slot.y + (pass_all - s_pre[y]) * kGR;
+        const int mc = min(kGR, slot.z - base);
+        // the expert's rule: per 32 values when it holds several rows
+        const bool a32 = a.qa32 != nullptr && slot.z - slot.y >= 2;
+        const int spg = a32 ? 4 : 1;  // scales per group
+
+        // this lane's words of a pair: row gid of the tile, bytes 4*tid..+3 of every block
+        const size_t tile0 = (size_t)(slot.x - a.expert_begin) * a.tiles_e;
+        const uint8_t* nib = a.nib + (tile0 + 2 * (round0 * kGW + warp)) * tile_bytes + lane * 4;
+        const uint8_t* scl = reinterpret_cast<const uint8_t*>(a.scl) +
+                             (tile0 + 2 * (round0 * kGW + warp)) * scl_tile_bytes +
+                             gid * (SCL16 ? 2 : 4);
+        PairWords<SCL16> pw[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+            if (i < G)
+                pw[i].load(nib, tile_bytes, scl, scl_tile_bytes, i);
+
+        // the pass's rows, a warp per row, all copies in flight at once
         for (int mi = warp; mi < mc; mi += kGW) {
-            const int src_row = a.row_map ? a.row_map[base + mi] : base + mi;
-            const int8_t* src = qa_src + (size_t)src_row * K;
-            const float* as = as_src + (size_t)src_row * as_stride;
+            const int row = a.row_map ? a.row_map[base + mi] : base + mi;
+            const int8_t* src = (a32 ? a.qa32 : a.qa) + (size_t)row * K;
+            const size_t at = (size_t)row * (a32 ? a.as32_stride : a.as_stride);
+            const float* as = (a32 ? a.as32 : a.as) + at;
+            const int32_t* es = (a32 ? a.es32 : a.es) + at;
 #pragma unroll 4
             for (int c = lane * 16; c < K; c += 32 * 16)
                 moe_cp_async<16>(s_qa + (size_t)mi * row_bytes + c, src + c);
-            for (int gs = lane; gs < G * SPG; gs += 32)
+            for (int gs = lane; gs < G * spg; gs += 32) {
                 moe_cp_async<4>(s_as + gs * kGR + mi, as + gs);
+                int* bias = reinterpret_cast<int*>(s_bias + gs * (kGR / 2) + (mi >> 1)) + (mi & 1);
+                moe_cp_async<4>(bias, es + gs);
+                moe_cp_async<4>(bias + 2, es + gs);
+            }
         }
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        // accumulator bias per (route, group): 0x4B400000 - 8 * (sum of the group's codes);
-        // per-32 rule: per (route, 32-block).  In tensor-operand order the codes of 32-block
-        // b are word b of each of the eight 16-byte chunks of the group.
-        for (int i = threadIdx.x; i < mc * G; i += kGT) {
-            const int mi = i / G, g = i - mi * G;
-            const uint4* q = reinterpret_cast<const uint4*>(s_qa + (size_t)mi * row_bytes + g * 128);
-            int sum[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint4 v = q[c];
-                sum[0] = __dp4a(0x01010101, (int)v.x, sum[0]);
-                sum[1] = __dp4a(0x01010101, (int)v.y, sum[1]);
-                sum[2] = __dp4a(0x01010101, (int)v.z, sum[2]);
-                sum[3] = __dp4a(0x01010101, (int)v.w, sum[3]);
-            }
-            if (a32) {
-#pragma unroll
-                for (int b = 0; b < 4; ++b)
-                    s_bias[(g * 4 + b) * kGR + mi] = 0x4B400000 - 8 * sum[b];
-            } else {
-                s_bias[g * kGR + mi] = 0x4B400000 - 8 * (sum[0] + sum[1] + sum[2] + sum[3]);
-            }
-        }
-        if (!weights_ready) {
-            if (!mbar_wait_bounded(&s_bar[0])) {
-                if (lane == 0)
-                    b2w4_report_timeout(a.status);
-                return;  // every thread sees the same barrier: the exit is CTA-uniform
-            }
-            weights_ready = true;
-        }
-        __syncthreads();
+
         const int ncb = (mc + 7) >> 3;  // column blocks in this pass: 1 or 2
+        const uint8_t* rows = s_qa + gid * row_bytes + tid * 32;
 #pragma unroll 1
-        for (int pair = warp / wpp; pair < npair; pair += kGW / wpp) {
-            const int wj = warp % wpp;
-            // column blocks of this warp: both, or the one matching its position in the pair;
-            // with a single column block (decode) the pair's two warps take one tile each
-            // instead (half of the instruction's rows idle, no warp idle)
-            const bool split_tiles = wpp == 2 && ncb == 1;
-            const int cb_lo = split_tiles ? 0 : (wpp == 2 ? wj : 0);
-            const int cb_hi = split_tiles ? 1 : (wpp == 2 ? wj + 1 : 2);
-            const int t0 = split_tiles ? pair * 2 + wj : pair * 2;
-            if (cb_lo >= ncb || t0 >= ntile)
-                continue;
-            const bool two = !split_tiles && t0 + 1 < ntile;
-            float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll 4
-            for (int g = 0; g < G; ++g) {
-                // word `lane` of the 128 bytes of (tile, group, 32-block s): row gid, k 8*tid..+7
-                const int wbase = t0 * tile_words + g * 128 + lane;
-                uint32_t lo0[4], hi0[4], lo1[4], hi1[4];
+        for (int round = round0; round < round1; ++round) {
+            uint64_t acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+            auto run = [&](auto rule) {
+#pragma unroll 3
+                for (int g = 0; g < G; ++g) {
+                    const PairWords<SCL16> now = pw[0];
 #pragma unroll
-                for (int sb = 0; sb < 4; ++sb) {
-                    const uint32_t u = s_w32[wbase + sb * 32];
-                    const uint32_t v = two ? s_w32[wbase + tile_words + sb * 32] : 0u;  // q = 0
-                    lo0[sb] = (u ^ 0x08080808u) & 0x0F0F0F0Fu;
-                    hi0[sb] = ((u >> 4) ^ 0x08080808u) & 0x0F0F0F0Fu;
-                    lo1[sb] = (v ^ 0x08080808u) & 0x0F0F0F0Fu;
-                    hi1[sb] = ((v >> 4) ^ 0x08080808u) & 0x0F0F0F0Fu;
+                    for (int i = 0; i + 1 < kAhead; ++i)
+                        pw[i] = pw[i + 1];
+                    if (g + kAhead < G)
+                        pw[kAhead - 1].load(nib, tile_bytes, scl, scl_tile_bytes, g + kAhead);
+                    pair_group<decltype(rule)::value, SCL16>(now, rows, row_bytes, s_as, s_bias, g,
+                                                             ncb, tid, acc);
                 }
-                const int si = (t0 * G + g) * 8 + gid;
-                const float ws0 = SCL16 ? __half2float(reinterpret_cast<const __half*>(s_scl)[si])
-                                        : reinterpret_cast<const float*>(s_scl)[si];
-                const float ws1 =
-                    !two ? 0.f
-                         : (SCL16 ? __half2float(
-                                        reinterpret_cast<const __half*>(s_scl)[si + G * 8])
-                                  : reinterpret_cast<const float*>(s_scl)[si + G * 8]);
+            };
+            if (a32)
+                run(std::true_type{});
+            else
+                run(std::false_type{});
+            nib += 2 * kGW * tile_bytes;
+            scl += 2 * kGW * scl_tile_bytes;
+            if (round + 1 < round1) {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int cb = cb_lo + j;
-                    if (cb < cb_hi && cb < ncb) {  // warp-uniform
-                        // unused columns of the last block read stale rows: never stored
-                        const uint4* bp = reinterpret_cast<const uint4*>(
-                            s_qa + (size_t)(cb * 8 + gid) * row_bytes + g * 128 + tid * 32);
-                        const uint4 be = bp[0], bo = bp[1];
-                        if (a32) {
-                            // one instruction = one 32-block: its own accumulator, bias and
-                            // activation scale, folded into the chain in ascending block order
-                            // (kernels/matmul_w4.cpp:785-901)
-                            const uint32_t bev[4] = {be.x, be.y, be.z, be.w};
-                            const uint32_t bov[4] = {bo.x, bo.y, bo.z, bo.w};
-#pragma unroll
-                            for (int b = 0; b < 4; ++b) {
-                                const int tk = (g * 4 + b) * kGR + cb * 8 + tid * 2;
-                                const int2 bias = *reinterpret_cast<const int2*>(s_bias + tk);
-                                const float2 asv = *reinterpret_cast<const float2*>(s_as + tk);
-                                int c[4] = {bias.x, bias.y, bias.x, bias.y};
-                                moe_mma_16x8x32(c, lo0[b], lo1[b], hi0[b], hi1[b], bev[b], bov[b]);
-                                acc[j][0] = __fmaf_rn(__fsub_rn(__int_as_float(c[0]), 12582912.f),
-                                                      __fmul_rn(ws0, asv.x), acc[j][0]);
-                                acc[j][1] = __fmaf_rn(__fsub_rn(__int_as_float(c[1]), 12582912.f),
-                                                      __fmul_rn(ws0, asv.y), acc[j][1]);
-                                acc[j][2] = __fmaf_rn(__fsub_rn(__int_as_float(c[2]), 12582912.f),
-                                                      __fmul_rn(ws1, asv.x), acc[j][2]);
-                                acc[j][3] = __fmaf_rn(__fsub_rn(__int_as_float(c[3]), 12582912.f),
-                                                      __fmul_rn(ws1, asv.y), acc[j][3]);
-                            }
-                            continue;
-                        }
-                        const int tk = g * kGR + cb * 8 + tid * 2;  // routes of this lane's columns
-                        const int2 bias = *reinterpret_cast<const int2*>(s_bias + tk);
-                        const float2 asv = *reinterpret_cast<const float2*>(s_as + tk);
-                        // two chains of two instructions (latency), joined by one add
-                        int c[4] = {bias.x, bias.y, bias.x, bias.y}, c2[4] = {0, 0, 0, 0};
-                        moe_mma_16x8x32(c, lo0[0], lo1[0], hi0[0], hi1[0], be.x, bo.x);
-                        moe_mma_16x8x32(c2, lo0[1], lo1[1], hi0[1], hi1[1], be.y, bo.y);
-                        moe_mma_16x8x32(c, lo0[2], lo1[2], hi0[2], hi1[2], be.z, bo.z);
-                        moe_mma_16x8x32(c2, lo0[3], lo1[3], hi0[3], hi1[3], be.w, bo.w);
-                        // c + c2 = 0x4B400000 + D: as a float 12582912 + D, exactly
-                        acc[j][0] = __fmaf_rn(
-                            __fsub_rn(__int_as_float(c[0] + c2[0]), 12582912.f),
-                            __fmul_rn(ws0, asv.x), acc[j][0]);
-                        acc[j][1] = __fmaf_rn(
-                            __fsub_rn(__int_as_float(c[1] + c2[1]), 12582912.f),
-                            __fmul_rn(ws0, asv.y), acc[j][1]);
-                        acc[j][2] = __fmaf_rn(
-                            __fsub_rn(__int_as_float(c[2] + c2[2]), 12582912.f),
-                            __fmul_rn(ws1, asv.x), acc[j][2]);
-                        acc[j][3] = __fmaf_rn(
-                            __fsub_rn(__int_as_float(c[3] + c2[3]), 12582912.f),
-                            __fmul_rn(ws1, asv.y), acc[j][3]);
-                    }
-                }
+                for (int i = 0; i < kAhead; ++i)
+                    if (i < G)
+                        pw[i].load(nib, tile_bytes, scl, scl_tile_bytes, i);
             }
             // out[route][n]: the eight lanes of a quarter-warp hold eight consecutive n
-            const int n0 = (tl0 + t0) * 8 + gid, n1 = n0 + 8;
+            const int n0 = (round * kGW + warp) * 16 + gid;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const int cb = cb_lo + j;
-                if (cb < cb_hi && cb < ncb) {
+                float v[2][2];
+                b2w4_unpack2(acc[j][0], v[0][0], v[0][1]);
+                b2w4_unpack2(acc[j][1], v[1][0], v[1][1]);
 #pragma unroll
-                    for (int cc = 0; cc < 2; ++cc) {
-                        const int mi = cb * 8 + tid * 2 + cc;
-                        if (mi < mc) {
-                            float* o = a.out + (size_t)(base + mi) * a.n_e;
-                            if (n0 < a.n_e)
-                                o[n0] = acc[j][cc];
-                            if (two && n1 < a.n_e)
-                                o[n1] = acc[j][2 + cc];
-                        }
+                for (int cc = 0; cc < 2; ++cc) {
+                    const int mi = j * 8 + tid * 2 + cc;
+                    if (mi < mc) {
+                        float* o = a.out + (size_t)(base + mi) * a.n_e + n0;
+                        o[0] = v[0][cc];
+                        o[8] = v[1][cc];
                     }
                 }
             }
@@ -1302,19 +1385,20 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
     }
 }
 
-size_t grouped_smem(int k, int groups, int tpc, bool scl16) {
-    return (size_t)tpc * groups * 512 + (size_t)tpc * groups * 8 * (scl16 ? 2 : 4) +
-           (size_t)kGR * (k + kRowPad) + 2 * sizeof(float) * kGR * groups * 4 + 8 + 16;
+size_t grouped_smem(int k, int groups, int slots) {
+    return (size_t)4 * groups * (kGR / 2) * sizeof(int4) + sizeof(float) * kGR * groups * 4 +
+           (size_t)kGR * (k + kRowPad) + sizeof(int) * (slots + 1);
 }
 
 // `decode` (few tokens): the shared-memory variant, optionally with SwiGLU + quantiser fused
 // into its prologue (fused_gate_up = the gate_up matmul's fp32 output).
 // qa32 / as32: the same rows quantised per 32 values, for experts that hold several routes
-// (null: per-128 for all); as_stride / as32_stride: floats per row of as / as32.
+// (null: per-128 for all); es / es32: accumulator biases, one per scale (not read by the decode
+// variant); as_stride / as32_stride: scales per row of as / as32.
 int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int expert_begin,
                    int expert_count, int routes, const int8_t* qa, const float* as,
-                   int as_stride, const int8_t* qa32, const float* as32, int as32_stride,
-                   const int4* slots, const int32_t* row_map, float* out, bool decode,
+                   const int32_t* es, int as_stride, const int8_t* qa32, const float* as32,
+                   const int32_t* es32, int as32_stride, const int4* slots, const int32_t* row_map, float* out, bool decode,
                    const float* fused_gate_up = nullptr, const b2w4_tp_args* peers = nullptr,
                    int stage_rows = 0) {
     const int n_e = w->n / expert_count;
@@ -1364,33 +1448,36 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
     a.scl = w->scl;
     a.qa = qa;
     a.as = as;
+    a.es = es;
     a.as_stride = as_stride;
     a.qa32 = qa32;
     a.as32 = as32;
+    a.es32 = es32;
     a.as32_stride = as32_stride;
     a.slots = slots;
+    a.slot_count = slots_y;
     a.num_experts_all = num_experts_all;
     a.expert_begin = expert_begin;
     a.expert_count = expert_count;
     a.row_map = row_map;
     a.out = out;
-    a.status = ctx->status_dev;
     a.k = w->k;
     a.groups = w->groups;
     a.n_e = n_e;
     a.tiles_e = n_e / 8;
-    int tpc = 16;
-    while (tpc > 2 && grouped_smem(w->k, w->groups, tpc, scl16) > 113 * 1024)
-        tpc -= 2;  // even: tiles are taken in pairs
-    a.tpc = tpc;
-    const size_t smem = grouped_smem(w->k, w->groups, tpc, scl16);
-    if (smem > 220 * 1024)
+    const size_t smem = grouped_smem(w->k, w->groups, slots_y);
+    // the longest rows: those that fit with a pair of tiles beside them (7936, or 7808 with fp32
+    // scales), the limit of the operator
+    const size_t pair = (size_t)2 * w->groups * (512 + 8 * (scl16 ? 2 : 4));
+    if (smem > 220 * 1024 || grouped_smem(w->k, w->groups, 0) + pair > 235 * 1024)
         return b2w4_fail(ctx, B2W4_E_INVALID, "moe: K=%d needs %zu B shared memory", w->k, smem);
     auto kern = scl16 ? moe_grouped_gemv_kernel<true> : moe_grouped_gemv_kernel<false>;
     static b2w4_smem_optin configured[2];  // per instantiation and device
     B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[scl16]));
-    dim3 grid((a.tiles_e + tpc - 1) / tpc, slots_y);
-    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kGT), smem, ctx->stream, a));
+    // no more CTAs than there can be units (a pass holds at least one route)
+    const long long units = (long long)routes * (a.tiles_e / (2 * kGW));
+    const int ctas = (int)(units < 2 * ctx->sm_count ? units : 2 * ctx->sm_count);
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(ctas), dim3(kGT), smem, ctx->stream, a));
     ctx->launches++;
     return B2W4_OK;
 }
@@ -1473,8 +1560,11 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     const size_t o_asi = align_up(o_qi + (size_t)routes * intermediate, 256);
     const size_t o_qh32 = align_up(o_asi + sizeof(float) * routes * gi * 4, 256);
     const size_t o_ash32 = align_up(o_qh32 + (rule32 ? (size_t)tokens * hidden_size : 0), 256);
-    const size_t quant_bytes =
-        align_up(o_ash32 + (rule32 ? sizeof(float) * tokens * gh * 4 : 0), 256);
+    const size_t o_es = align_up(o_ash32 + (rule32 ? sizeof(float) * tokens * gh * 4 : 0), 256);
+    const size_t o_es32 = align_up(o_es + sizeof(int32_t) * tokens * gh, 256);
+    const size_t o_esi =
+        align_up(o_es32 + (rule32 ? sizeof(int32_t) * tokens * gh * 4 : 0), 256);
+    const size_t quant_bytes = align_up(o_esi + sizeof(int32_t) * routes * gi * 4, 256);
     void *sm = nullptr, *qb = nullptr, *gu = nullptr, *dn = nullptr;
     int rc;
     if ((rc = b2w4_reserve(ctx, SCR_MOE_A, small_bytes, &sm)) != B2W4_OK ||
@@ -1499,6 +1589,9 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     float* as_inter = reinterpret_cast<float*>(qbb + o_asi);  // [routes][4 * gi]
     int8_t* q_hidden32 = rule32 ? reinterpret_cast<int8_t*>(qbb + o_qh32) : nullptr;
     float* as_hidden32 = rule32 ? reinterpret_cast<float*>(qbb + o_ash32) : nullptr;
+    int32_t* es_hidden = reinterpret_cast<int32_t*>(qbb + o_es);
+    int32_t* es_hidden32 = rule32 ? reinterpret_cast<int32_t*>(qbb + o_es32) : nullptr;
+    int32_t* es_inter = reinterpret_cast<int32_t*>(qbb + o_esi);  // [routes][4 * gi]
     cudaStream_t st = ctx->stream;
 
     const __half* router = static_cast<const __half*>(router_fp16_dev);
@@ -1546,23 +1639,25 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
                                            tokens, top_k, num_experts, offsets, route_token, pos,
                                            slots));
         ctx->launches++;
-        B2W4_CUDA(ctx, cudaGetLastError());
-        if ((rc = b2w4_launch_quantize(ctx, hidden_dev, ldx, tokens, hidden_size, B2W4_ACT_G128,
-                                       q_hidden, as_hidden, QLAYOUT_MMA)) != B2W4_OK)
-            return rc;
     }
-    if (rule32 && (rc = b2w4_launch_quantize(ctx, hidden_dev, ldx, tokens, hidden_size,
-                                             B2W4_ACT_G32, q_hidden32, as_hidden32,
-                                             QLAYOUT_MMA)) != B2W4_OK)
-        return rc;
     // which grouped-matmul variant: the few-token one implements the per-128 rule only
     const bool decode = rule32 ? false : tokens <= kFusedSwigluTokens;
+    // (the decode variant takes the rows that the fused routing kernel quantised)
+    if (!decode || !fused) {
+        const long long threads = (long long)tokens * gh * 32;
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, moe_quantize_hidden_kernel,
+                                           dim3((int)((threads + 255) / 256)), dim3(256), 0, st,
+                                           hidden_dev, ldx, tokens, hidden_size, q_hidden,
+                                           as_hidden, es_hidden, q_hidden32, as_hidden32,
+                                           es_hidden32));
+        ctx->launches++;
+    }
     // compact positions stay global; the grouped kernels skip experts held elsewhere
     const int32_t* local_offsets = offsets + expert_begin;
     const bool partial = expert_count != num_experts;
     if ((rc = launch_grouped(ctx, gate_up, num_experts, expert_begin, expert_count, routes,
-                             q_hidden, as_hidden, gh, q_hidden32, as_hidden32, gh * 4, slots,
-                             route_token, static_cast<float*>(gu), decode)) != B2W4_OK)
+                             q_hidden, as_hidden, es_hidden, gh, q_hidden32, as_hidden32,
+                             es_hidden32, gh * 4, slots, route_token, static_cast<float*>(gu), decode)) != B2W4_OK)
         return rc;
     // few routes: SwiGLU and its quantiser run inside the down-projection's CTAs
     const bool fuse_swiglu = decode;
@@ -1571,7 +1666,7 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
         B2W4_CUDA(ctx, b2w4_launch_chained(
                            ctx->pdl, moe_swiglu_quant_kernel, dim3((int)((threads + 255) / 256)),
                            dim3(256), 0, st, static_cast<const float*>(gu), routes, intermediate,
-                           q_inter, as_inter, gi * 4,
+                           q_inter, as_inter, es_inter, gi * 4,
                            rule32 ? static_cast<const int32_t*>(offsets) : nullptr, num_experts,
                            partial ? local_offsets : nullptr,
                            partial ? local_offsets + expert_count : nullptr));
@@ -1581,8 +1676,8 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     const bool fused_handover = peers != nullptr && decode;
     // a route's SwiGLU row was quantised by its own expert's rule: one code buffer serves both
     if ((rc = launch_grouped(ctx, down, num_experts, expert_begin, expert_count, routes, q_inter,
-                             as_inter, gi * 4, rule32 ? q_inter : nullptr,
-                             rule32 ? as_inter : nullptr, gi * 4, slots, nullptr,
+                             as_inter, es_inter, gi * 4, rule32 ? q_inter : nullptr,
+                             rule32 ? as_inter : nullptr, es_inter, gi * 4, slots, nullptr,
                              static_cast<float*>(dn), decode,
                              fuse_swiglu ? static_cast<const float*>(gu) : nullptr,
                              fused_handover ? peers : nullptr, stage_rows)) != B2W4_OK)

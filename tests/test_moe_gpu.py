@@ -363,3 +363,21 @@ def test_hand_over_with_a_silent_peer_times_out(ctx):
     wd.free()
     want = run_moe(ctx, hidden, router, top_k, inter, gu, dn)  # the context still works
     assert np.isfinite(want[0]).all()
+
+
+@pytest.mark.parametrize("rule", [REF, ol.ACT_G128])
+@pytest.mark.parametrize("t,h,inter", [(8, 128, 128), (9, 384, 256), (16, 512, 384),
+                                       (17, 640, 128), (33, 896, 640)])
+def test_grouped_matmul_pass_edges(ctx, t, h, inter, rule):
+    """Prefill matmul of the experts at the edges of its passes (sixteen routes, two column
+    blocks) and of its look-ahead over the groups (1, 3, 4, 5 and 7 groups, fewer and more than
+    it keeps in flight): two experts that take every token, one that takes none."""
+    hidden = np.abs(pkg.synth.activations(11, t, t, h)) + 0.1
+    router = pkg.synth.router_weight(20261125, 3, 3, h, std=0.01)
+    router[2] = -1.0  # positive rows: never among the two largest
+    gu = pkg.synth.bg128_weight(20261125, 300 + t, 3 * 2 * inter, h)
+    dn = pkg.synth.bg128_weight(20261125, 400 + t, 3 * h, inter)
+    got = run_moe(ctx, hidden, router, 2, inter, gu, dn, rule=rule)
+    want = ol.moe_forward(hidden, router, 2, inter, gu, dn, rule=rule)
+    assert not (want[2] == 2).any()
+    check_against_oracle(got, want)
