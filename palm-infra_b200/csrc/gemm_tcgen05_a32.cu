@@ -7,23 +7,23 @@
 //
 // What bounds it: the issue slots and the fp32 pipe of that chain (M*N*K/32 sums); the MMAs
 // keep the tensor pipe under a tenth busy.  So everything around the chain is kept out of it:
-//   epilogue   sixteen warps, thread = one token x a quarter of the tile's columns.  Four
-//              warps per scheduler hide each other's latencies (tensor-memory loads, shared
-//              loads).  A unit is handed back as soon as it is in registers.
+//   epilogue   eight warps, thread = one token x half of the tile's columns.  Eight columns of
+//              two blocks are fetched from tensor memory while the eight before them are folded,
+//              across hand-overs too, so a warp waits for no fetch; a tile of up to 128 columns
+//              (row_tiles) spreads what a group costs beside its columns.
 //   unpack     a nibble becomes a signed byte of 16 q with one AND (high nibble) or a shift
 //              and an AND (low nibble): three instructions per eight weights, so the sums
 //              are 16 D, |16 D| < 2^19.
-//   to float   the hardware conversion, which has a pipe of its own (a warp instruction in two
-//              cycles per scheduler, measured), so that the fp32 pipe sees only the scale
-//              product and the multiply-add, both paired (fma.rn.f32x2).  It also moves the
-//              sums from the registers that the fetch filled to register pairs.  The scales
-//              are staged as w / 16: a power of two, exact while w * as / 16 is a normal number.
-//   MMA        one thread; two accumulator units (a group each) or more in tensor
-//              memory, and one barrier frees an activation and a weight stage together.
-// Measured against the form this replaces (the accumulator switch of the per-128 kernel, two
-// integer adds and a subtraction per pair of sums, four hand-overs per two groups): 1000 rows,
-// [4100, 9728], three matmuls 1173 -> 882 us; eight layers of a 256-token prompt, all
-// operators, 3.39 -> 2.79 ms.
+//   to float   the hardware conversion, so that the fp32 pipe sees only the scale product and
+//              the multiply-add, both paired (fma.rn.f32x2).  It also moves the sums from the
+//              registers that the fetch filled to register pairs.  The scales are staged as
+//              w / 16: a power of two, exact while w * as / 16 is a normal number.
+//   MMA        one thread; two accumulator units (a group each, or half a group where tiles are
+//              wide) or more in tensor memory, and one barrier frees an activation and a weight
+//              stage together.
+// Measured against sixteen epilogue warps with a quarter of at most 64 columns each, fetch and
+// chain in turn: 1000 rows, [4100, 9728], three matmuls 882 -> 715 us; eight layers of a
+// 256-token prompt, all operators, 2.47 -> 2.20 ms.
 // Tokens sit on the MMA's M side (128 per CTA), weight rows on its N side.  The next launch
 // is released at the start (programmatic dependent launch): weights and scales are fetched
 // while the quantiser in front still runs.  Every wait is bounded; on a timeout the kernel
@@ -32,109 +32,64 @@
 
 namespace {
 
+// Roles: producer, MMA issue, two unpack warps, then eight epilogue warps (two column halves x
+// four TMEM lane quarters; a warp's lane quarter is its index mod 4).
 constexpr int kProducerWarp = 0;
 constexpr int kMmaWarp = 1;
 constexpr int kUnpackWarp0 = 2, kUnpackWarps = 2;
-// four epilogue warpgroups, one per column quarter; a warp's TMEM lane quarter is its index
-// mod 4
-constexpr int kEpiWarp0 = 4, kEpiWarps = 16;
-constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;  // 640
+constexpr int kEpiWarp0 = 4, kEpiWarps = 8;
+constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;  // 384: up to 168 registers each
 constexpr int kStages = 4;    // activation and unpacked-weight stages (one group each)
-constexpr int kRawSlots = 3;  // nibble chunks of kGC groups in flight
+constexpr int kRawGroups = 2; // groups per nibble copy
+constexpr int kRawSlots = 3;  // nibble copies in flight
 constexpr int kMaxG = 80;     // K <= 10240
 
 template <int RP>
 struct Smem {
-    static constexpr int kActStage = 128 * 128;            // 128 tokens x 128 B, swizzled
-    static constexpr int kBStage = RP * 128;               // int8 weights, swizzled
-    static constexpr int kRawSlot = (RP / 8) * kGC * 512;  // nibbles: [tile][kGC][512]
+    static constexpr int kActStage = 128 * 128;  // 128 tokens x 128 B, swizzled
+    static constexpr int kBStage = RP * 128;     // int8 weights, swizzled
+    static constexpr int kRawSlot = (RP / 8) * kRawGroups * 512;  // nibbles: [tile][groups][512]
     static constexpr int kActOff = 0;
     static constexpr int kBOff = kActOff + kStages * kActStage;
     static constexpr int kRawOff = kBOff + kStages * kBStage;
     static constexpr int kWsOff = kRawOff + kRawSlots * kRawSlot;  // fp32 [G][RP]
     static constexpr int kBarOff = kWsOff + kMaxG * RP * 4;
     static constexpr int kTotal = kBarOff + 512 + 1024;  // barriers, + slack to align the base
-    static constexpr int kStagePitch = RP / 4 + 4;       // output staging, floats per token
-    static_assert(kEpiWarps * 32 * kStagePitch * 4 <= kStages * kActStage, "output staging");
+    static constexpr int kStagePitch = RP / 2 + 4;       // output staging, floats per token
+    static_assert(kEpiWarps * 32 * kStagePitch * 4 <= kRawOff, "output staging");
     static_assert(kTotal <= 227 * 1024, "shared memory");
 };
 
-// N columns of two blocks, complete when the statement is: loads and wait are one statement.
-template <int N>
-__device__ __forceinline__ void tmem_fetch2(uint32_t t0, uint32_t t1, uint32_t (&r)[2][N]);
-template <>
-__device__ __forceinline__ void tmem_fetch2<8>(uint32_t t0, uint32_t t1, uint32_t (&r)[2][8]) {
+// eight columns of two blocks: issue, and the wait that makes the registers readable
+__device__ __forceinline__ void tmem_issue(uint32_t t0, uint32_t t1, uint32_t (&r)[2][8]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
-        "%0, %1, %2, %3, %4, %5, %6, %7"
-        "}, [%16];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
-        "%8, %9, %10, %11, %12, %13, %14, %15"
-        "}, [%17];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]),
-          "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
-          "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]),
-          "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]), "=&r"(r[1][7])
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];"
+        : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[0][4]),
+          "=r"(r[0][5]), "=r"(r[0][6]), "=r"(r[0][7]), "=r"(r[1][0]), "=r"(r[1][1]),
+          "=r"(r[1][2]), "=r"(r[1][3]), "=r"(r[1][4]), "=r"(r[1][5]), "=r"(r[1][6]),
+          "=r"(r[1][7])
         : "r"(t0), "r"(t1)
         : "memory");
 }
-template <>
-__device__ __forceinline__ void tmem_fetch2<12>(uint32_t t0, uint32_t t1, uint32_t (&r)[2][12]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
-        "%0, %1, %2, %3, %4, %5, %6, %7"
-        "}, [%24];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {"
-        "%8, %9, %10, %11"
-        "}, [%24+8];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
-        "%12, %13, %14, %15, %16, %17, %18, %19"
-        "}, [%25];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {"
-        "%20, %21, %22, %23"
-        "}, [%25+8];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]),
-          "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
-          "=&r"(r[0][8]), "=&r"(r[0][9]), "=&r"(r[0][10]), "=&r"(r[0][11]),
-          "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]),
-          "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]), "=&r"(r[1][7]),
-          "=&r"(r[1][8]), "=&r"(r[1][9]), "=&r"(r[1][10]), "=&r"(r[1][11])
-        : "r"(t0), "r"(t1)
-        : "memory");
-}
-template <>
-__device__ __forceinline__ void tmem_fetch2<16>(uint32_t t0, uint32_t t1, uint32_t (&r)[2][16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {"
-        "%0, %1, %2, %3, %4, %5, %6, %7, "
-        "%8, %9, %10, %11, %12, %13, %14, %15"
-        "}, [%32];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {"
-        "%16, %17, %18, %19, %20, %21, %22, %23, "
-        "%24, %25, %26, %27, %28, %29, %30, %31"
-        "}, [%33];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]),
-          "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
-          "=&r"(r[0][8]), "=&r"(r[0][9]), "=&r"(r[0][10]), "=&r"(r[0][11]),
-          "=&r"(r[0][12]), "=&r"(r[0][13]), "=&r"(r[0][14]), "=&r"(r[0][15]),
-          "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]),
-          "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]), "=&r"(r[1][7]),
-          "=&r"(r[1][8]), "=&r"(r[1][9]), "=&r"(r[1][10]), "=&r"(r[1][11]),
-          "=&r"(r[1][12]), "=&r"(r[1][13]), "=&r"(r[1][14]), "=&r"(r[1][15])
-        : "r"(t0), "r"(t1)
-        : "memory");
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[2][8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[0][4]),
+                   "+r"(r[0][5]), "+r"(r[0][6]), "+r"(r[0][7]), "+r"(r[1][0]), "+r"(r[1][1]),
+                   "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[1][4]), "+r"(r[1][5]), "+r"(r[1][6]),
+                   "+r"(r[1][7])
+                 :
+                 : "memory");
 }
 
 template <int RP, bool SCL16>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a8_tc32_kernel(const GemmArgs a) {
-    constexpr int CH = RP / 4;  // columns per epilogue thread
-    // A unit is what the MMA warp hands to the epilogue: a group's accumulators, four blocks
-    // of RP columns each.
-    constexpr int kAccCols = 4 * RP;
+    constexpr int CH = RP / 2;  // columns per epilogue thread
+    // A unit is what the MMA warp hands to the epilogue: the accumulators of a group, four
+    // blocks of RP columns each, or of half a group where four blocks leave no second buffer.
+    constexpr int kUnitBlocks = RP <= 64 ? 4 : 2;
+    constexpr int kAccCols = kUnitBlocks * RP;
     constexpr int kAcc = 512 / kAccCols;
     static_assert(kAcc >= 2, "no accumulator to run ahead into");
     extern __shared__ uint8_t smem_raw[];
@@ -173,7 +128,7 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         }
         for (int b = 0; b < kAcc; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_free[b], kEpiWarps);
+            mbar_init(&acc_free[b], 2 * ((m_here + 31) / 32));  // the warps that have tokens
         }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -200,14 +155,14 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
     if (warp == kProducerWarp) {
         // =============================== producer ===================================
         // lane t copies row tile t's share of a nibble chunk, lane 31 a group's activations
-        const int chunks = (G + kGC - 1) / kGC;
+        const int chunks = (G + kRawGroups - 1) / kRawGroups;
         auto load_chunk = [&](int chunk) {
-            const int slot = chunk % kRawSlots, g = chunk * kGC, gc = min(kGC, G - g);
+            const int slot = chunk % kRawSlots, g = chunk * kRawGroups, gc = min(kRawGroups, G - g);
             if (lane == 0)
                 mbar_expect_tx(&raw_full[slot], (uint32_t)r_tiles * gc * 512);
             __syncwarp();
             if (lane < r_tiles)
-                bulk_g2s(smem + S::kRawOff + slot * S::kRawSlot + lane * (kGC * 512),
+                bulk_g2s(smem + S::kRawOff + slot * S::kRawSlot + lane * (kRawGroups * 512),
                          a.nib + ((size_t)(tile0 + lane) * G + g) * 512, (uint32_t)gc * 512,
                          &raw_full[slot]);
         };
@@ -220,8 +175,8 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         const uint32_t act_bytes = (uint32_t)((m_here + 7) / 8) * 1024;
         bool ok = true;
         for (int g = 0; g < G; ++g) {
-            if (g % kGC == 0 && g / kGC >= kRawSlots) {
-                const int chunk = g / kGC, slot = chunk % kRawSlots, use = chunk / kRawSlots;
+            if (g % kRawGroups == 0 && g / kRawGroups >= kRawSlots) {
+                const int chunk = g / kRawGroups, slot = chunk % kRawSlots, use = chunk / kRawSlots;
                 ok = __all_sync(0xffffffffu, wait(&raw_free[slot], (use - 1) & 1));
                 if (!ok)
                     break;
@@ -249,8 +204,7 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
             int u = 0, use = 0;  // unit buffer and how often it has been filled
             for (int g = 0; g < G; ++g) {
                 const int s = g % kStages, round = g / kStages;
-                if (!wait(&act_full[s], round & 1) || !wait(&b_full[s], round & 1) ||
-                    (use > 0 && !wait(&acc_free[u], (use - 1) & 1))) {
+                if (!wait(&act_full[s], round & 1) || !wait(&b_full[s], round & 1)) {
                     fail();
                     break;
                 }
@@ -258,14 +212,28 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
                 const uint64_t a_desc = a_desc0 + (uint64_t)(s * (S::kActStage >> 4));
                 const uint64_t b_desc = b_desc0 + (uint64_t)(s * (S::kBStage >> 4));
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                bool ok = true;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)  // a K = 32 step (32 bytes) = a 32-k block
-                    umma_i8(tmem_base + (uint32_t)(u * kAccCols + j * RP),
-                            a_desc + (uint64_t)(j * 2), b_desc + (uint64_t)(j * 2), idesc, 0u);
-                umma_commit(&acc_full[u]);  // the group's sums are complete
-                if (++u == kAcc) {
-                    u = 0;
-                    ++use;
+                for (int j0 = 0; j0 < 4; j0 += kUnitBlocks) {
+                    if (use > 0 && !wait(&acc_free[u], (use - 1) & 1)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < kUnitBlocks; ++j)  // a K = 32 step = a 32-k block
+                        umma_i8(tmem_base + (uint32_t)(u * kAccCols + j * RP),
+                                a_desc + (uint64_t)((j0 + j) * 2),
+                                b_desc + (uint64_t)((j0 + j) * 2), idesc, 0u);
+                    umma_commit(&acc_full[u]);  // the unit's sums are complete
+                    if (++u == kAcc) {
+                        u = 0;
+                        ++use;
+                    }
+                }
+                if (!ok) {
+                    fail();
+                    break;
                 }
                 umma_commit(&ab_free[s]);  // both stages may be refilled
             }
@@ -274,8 +242,8 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         // =============================== unpack ======================================
         const int ut = (warp - kUnpackWarp0) * 32 + lane;
         for (int g = 0; g < G; ++g) {
-            const int chunk = g / kGC, slot = chunk % kRawSlots, cuse = chunk / kRawSlots;
-            const int gi = g % kGC;
+            const int chunk = g / kRawGroups, slot = chunk % kRawSlots, cuse = chunk / kRawSlots;
+            const int gi = g % kRawGroups;
             const int s = g % kStages, round = g / kStages;
             bool ok = true;
             if (gi == 0)  // the chunk's nibbles landed
@@ -286,7 +254,7 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
                 fail();
                 break;
             }
-            // raw slot: [tile][kGC groups][32 chunks of 16 B]
+            // raw slot: [tile][kRawGroups groups][32 chunks of 16 B]
             const uint4* raw =
                 reinterpret_cast<const uint4*>(smem + S::kRawOff + slot * S::kRawSlot) + gi * 32;
             uint8_t* bst = smem + S::kBOff + s * S::kBStage;
@@ -294,7 +262,7 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
 #pragma unroll 4
             for (int c = ut; c < r_tiles * 32; c += kUnpackWarps * 32) {
                 const int t = c >> 5, sub = (c >> 3) & 3, row = c & 7;
-                const uint4 w = raw[t * (kGC * 32) + (c & 31)];
+                const uint4 w = raw[t * (kRawGroups * 32) + (c & 31)];
                 // low nibbles = even k, high nibbles = odd k, in two's complement: a nibble in
                 // the upper half of a byte is the signed byte 16 q
                 constexpr uint32_t kHigh = 0xF0F0F0F0u;
@@ -312,14 +280,14 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&b_full[s]);
-                if (gi == kGC - 1 || g == G - 1)
+                if (gi == kRawGroups - 1 || g == G - 1)
                     mbar_arrive(&raw_free[slot]);  // this warp is done with the chunk
             }
         }
     } else {
         // =============================== epilogue ====================================
-        const int ew = warp - kEpiWarp0;       // 0..15
-        const int ch = ew >> 2;                // column quarter
+        const int ew = warp - kEpiWarp0;       // 0..7
+        const int ch = ew >> 2;                // column half
         const int lq = warp & 3;               // TMEM lane quarter this warp may read
         const int tok = tok0 + lq * 32 + lane;
         // a warp whose 32 tokens all lie past the last row has no chain to run
@@ -374,54 +342,74 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         for (int i = 0; i < CH / 2; ++i)
             acc2[i] = 0ull;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(ch * CH);
-        int u = 0, use = 0;  // unit buffer and how often it has been filled before
         bool live = true;
-        for (int g = 0; g < G; ++g) {
-            const float asv[4] = {a0.x, a0.y, a0.z, a0.w};
-            a0 = a1;
-            a1 = load_as(g + 2);
-            const bool ready = mbar_try_wait(&acc_full[u], use & 1);
-            if (!__all_sync(0xffffffffu, ready)) {
-                live = __all_sync(0xffffffffu, ready || wait(&acc_full[u], use & 1));
-                if (!live)
-                    break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t r[2][CH];
-            const uint32_t t = lane_addr + (uint32_t)(u * kAccCols);
-            const float* ws = wsf + g * RP;
-            auto chain = [&](float b0, float b1) {  // two blocks, in ascending order
-                const uint64_t s0 = b2w4_pack2(b0, b0), s1 = b2w4_pack2(b1, b1);
-#pragma unroll
-                for (int c = 0; c < CH; c += 4) {
-                    const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(ws + c);
-                    auto sums = [&](int j, int i) {
-                        return b2w4_pack2(__int2float_rn((int)r[j][i]),
-                                          __int2float_rn((int)r[j][i + 1]));
-                    };
-                    uint64_t& lo = acc2[c / 2];
-                    uint64_t& hi = acc2[c / 2 + 1];
-                    lo = b2w4_fma2(sums(0, c), b2w4_mul2(w2.x, s0), lo);
-                    hi = b2w4_fma2(sums(0, c + 2), b2w4_mul2(w2.y, s0), hi);
-                    lo = b2w4_fma2(sums(1, c), b2w4_mul2(w2.x, s1), lo);
-                    hi = b2w4_fma2(sums(1, c + 2), b2w4_mul2(w2.y, s1), hi);
+        if (active) {
+            int u = 0, use = 0;  // unit buffer and how often it has been filled before
+            auto unit_wait = [&]() {
+                const bool ready = mbar_try_wait(&acc_full[u], use & 1);
+                if (!__all_sync(0xffffffffu, ready))
+                    live &= __all_sync(0xffffffffu, ready || wait(&acc_full[u], use & 1)) != 0;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            };
+            auto unit_done = [&]() {  // every fetch of the unit is in registers
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(&acc_free[u]);
+                if (++u == kAcc) {
+                    u = 0;
+                    ++use;
                 }
             };
-            if (active) {
-                tmem_fetch2<CH>(t, t + RP, r);
-                chain(asv[0], asv[1]);
-                tmem_fetch2<CH>(t + 2 * RP, t + 3 * RP, r);
+            // A chunk is eight columns of two blocks; the next chunk's fetch is in flight while
+            // one is folded into the chain, across units and groups too.
+            constexpr int kChunks = CH / 4, kHalf = kChunks / 2;  // per group, per block pair
+            static_assert(kChunks % 2 == 0 && CH % 8 == 0, "chunk buffers alternate");
+            uint32_t r[2][2][8];
+            auto issue = [&](int i) {
+                const int j = i / kHalf * 2 % kUnitBlocks, c = i % kHalf * 8;
+                const uint32_t t = lane_addr + (uint32_t)(u * kAccCols + j * RP + c);
+                tmem_issue(t, t + RP, r[i & 1]);
+            };
+            unit_wait();
+            issue(0);
+            for (int g = 0; g < G; ++g) {
+                const float asv[4] = {a0.x, a0.y, a0.z, a0.w};
+                a0 = a1;
+                a1 = load_as(g + 2);
+                const float* ws = wsf + g * RP;
+#pragma unroll
+                for (int i = 0; i < kChunks; ++i) {
+                    tmem_wait(r[i & 1]);
+                    if (i + 1 == kChunks || (kUnitBlocks == 2 && i + 1 == kHalf)) {
+                        unit_done();
+                        if (i + 1 < kChunks || g + 1 < G) {
+                            unit_wait();
+                            issue((i + 1) % kChunks);
+                        }
+                    } else {
+                        issue(i + 1);
+                    }
+                    // two blocks, in ascending order
+                    const int j = i / kHalf * 2, c = i % kHalf * 8;
+                    const uint64_t s0 = b2w4_pack2(asv[j], asv[j]);
+                    const uint64_t s1 = b2w4_pack2(asv[j + 1], asv[j + 1]);
+#pragma unroll
+                    for (int h = 0; h < 8; h += 4) {
+                        const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(ws + c + h);
+                        auto sums = [&](int b, int e) {
+                            return b2w4_pack2(__int2float_rn((int)r[i & 1][b][e]),
+                                              __int2float_rn((int)r[i & 1][b][e + 1]));
+                        };
+                        uint64_t& lo = acc2[(c + h) / 2];
+                        uint64_t& hi = acc2[(c + h) / 2 + 1];
+                        lo = b2w4_fma2(sums(0, h), b2w4_mul2(w2.x, s0), lo);
+                        hi = b2w4_fma2(sums(0, h + 2), b2w4_mul2(w2.y, s0), hi);
+                        lo = b2w4_fma2(sums(1, h), b2w4_mul2(w2.x, s1), lo);
+                        hi = b2w4_fma2(sums(1, h + 2), b2w4_mul2(w2.y, s1), hi);
+                    }
+                }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(&acc_free[u]);
-            if (++u == kAcc) {
-                u = 0;
-                ++use;
-            }
-            if (active)
-                chain(asv[2], asv[3]);
         }
         if (!live)
             fail();
@@ -493,13 +481,10 @@ int launch_rp(b2w4_ctx* ctx, const GemmArgs& a, bool scl16, dim3 grid) {
     return B2W4_OK;
 }
 
-// What a group costs beside its columns, in columns (measured: 1000 rows, [4100, 9728]: five
-// rounds of 48 columns take 314 us, four of 64 286 us).  The choice it makes was timed against
-// the kernel before on six shapes from [500, 512] to [20000, 1024] and 33 to 1000 rows: 17 to
-// 33 % below it on each ([9728, 2560], 33 rows 45 -> 33 us, 256 rows 67 -> 56).
-constexpr int kFixedColumns = 64;
+// What a group costs beside its columns, in columns.
+constexpr int kFixedColumns = 24;
 // accumulator columns of the instantiation that takes r row tiles
-int columns_for(int r) { return r <= 4 ? 32 : r <= 6 ? 48 : 64; }
+int columns_for(int r) { return r <= 4 ? 32 : (r + 1) / 2 * 16; }
 
 // Rows per CTA.  The fp32 chain paces a CTA, so its time grows with the accumulator columns
 // of its instantiation (plus a fixed part per group); the launch takes as many rounds as the
@@ -507,7 +492,7 @@ int columns_for(int r) { return r <= 4 ? 32 : r <= 6 ? 48 : 64; }
 int row_tiles(int tiles, int token_blocks, int sm_count) {
     int best = 1;
     long best_cost = -1;
-    for (int r = 1; r <= 8; ++r) {
+    for (int r = 1; r <= 16; ++r) {
         const long ctas = (long)((tiles + r - 1) / r) * token_blocks;
         const long rounds = (ctas + sm_count - 1) / sm_count;
         const long cost = rounds * (columns_for(r) + kFixedColumns);
@@ -562,6 +547,10 @@ int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
     switch (columns_for(r_tiles)) {
     case 32: return launch_rp<32>(ctx, a, scl16, grid);
     case 48: return launch_rp<48>(ctx, a, scl16, grid);
-    default: return launch_rp<64>(ctx, a, scl16, grid);
+    case 64: return launch_rp<64>(ctx, a, scl16, grid);
+    case 80: return launch_rp<80>(ctx, a, scl16, grid);
+    case 96: return launch_rp<96>(ctx, a, scl16, grid);
+    case 112: return launch_rp<112>(ctx, a, scl16, grid);
+    default: return launch_rp<128>(ctx, a, scl16, grid);
     }
 }

@@ -331,6 +331,18 @@ def test_per32_tensor_core_scales_near_the_smallest_normal(ctx_tc):
     assert np.max(np.abs(want)) > 50 * bound  # the results are far above it
 
 
+@pytest.mark.parametrize("tiles", [3, 5, 7, 9, 12, 14, 15, 16])
+def test_per32_tensor_core_wide_tiles_bit_exact(ctx_tc, tiles):
+    """One round of CTAs whose tiles are 32 to 128 columns wide (multiples of 16, whole and with
+    a last one that is not full), 33 tokens: all warps of one lane quarter and one lane of the
+    next have a token."""
+    n, k, m = 148 * 8 * tiles - 8, 384, 33
+    blocks = pkg.synth.bg128_weight(20261125, n + k + 3, n, k)
+    x = pkg.synth.activations(7, tiles, m, k)
+    y, _ = run_gpu(ctx_tc, blocks, n, k, x, rule=ol.ACT_G32, sums=False)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).tobytes()
+
+
 def test_config2_prefill_m256_reference_rule(ctx):
     """M=256, K=2560, N=9728 (benchmark configuration 2, prefill) under the reference's rule
     for several rows (per 32 values), the kernel the library picks by itself: bit-exact
