@@ -271,99 +271,82 @@ __global__ void moe_select_routes_kernel(const float* __restrict__ logits, int t
     select_routes_any(logits, t, num_experts, top_k, idx, weights, lane);
 }
 
-// ---- 3. compaction: one block ------------------------------------------------------------
+// ---- 3. compaction: a block per expert -----------------------------------------------------
 // counts, exclusive offsets, and per expert its routes in ascending token order
 // (kernels/moe.cpp:759-776).  pos[t][j] = the compact position of token t's j-th route;
 // slots[y] = (expert, first route, one past its last route) of the y-th expert that has routes,
 // ascending; empty (0, 0, 0) from the number of such experts on: what a grouped-matmul CTA
 // needs to start, in one 16-byte load.
-// Stable placement, a chunk of routes at a time (one route per thread): lanes of a warp that
-// hold the same expert find each other with match.any, the lowest of them records the warp's
-// count for that expert, a scan over the warps turns the counts into first slots, and every
-// route lands at its warp's first slot plus its rank among the matching lanes.
-constexpr int kCompactThreads = 1024;
-constexpr int kCompactTableInts = 8192;  // warps x experts count table
+// A block reads all routes: its expert's first position is the number of routes of lower experts,
+// its slot the number of lower experts that have any, so no block waits for another.  Thread t
+// owns a run of consecutive routes, a scan over the threads places its routes.  (In one block,
+// with the counts of all experts, the same took 12 us for 2048 routes over 128 experts.)
+constexpr int kCompactThreads = 256;
 __global__ void __launch_bounds__(kCompactThreads)
 moe_compact_kernel(const int32_t* __restrict__ idx, int tokens, int top_k, int num_experts,
                    int32_t* __restrict__ offsets, int32_t* __restrict__ route_token,
                    int32_t* __restrict__ pos, int4* __restrict__ slots) {
     b2w4_pdl_chain_entry();
-    extern __shared__ int s_int[];
-    const int E = num_experts;
-    const int nw = min(kCompactThreads / 32, max(1, kCompactTableInts / E));  // warps placing
-    int* s_cnt = s_int;             // [E+1] counts
-    int* s_cursor = s_cnt + E + 1;  // [E] next free slot per expert
-    int* s_wc = s_cursor + E;       // [nw][E]
-    const int routes = tokens * top_k;
+    __shared__ unsigned s_has[kSelectMaxExperts / 32];  // experts with routes
+    __shared__ int s_warp[kCompactThreads / 32][2];
+    const int e = blockIdx.x, routes = tokens * top_k;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    for (int e = threadIdx.x; e <= E; e += blockDim.x)
-        s_cnt[e] = 0;
-    for (int y = threadIdx.x; y < E; y += blockDim.x)
-        slots[y] = make_int4(0, 0, 0, 0);  // experts with routes overwrite theirs below
+    for (int w = threadIdx.x; w < (num_experts + 31) / 32; w += kCompactThreads)
+        s_has[w] = 0;
     __syncthreads();
-    for (int i0 = 0; i0 < routes; i0 += blockDim.x) {
-        const int i = i0 + threadIdx.x;
-        const int e = i < routes ? idx[i] : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, e);
-        if (e >= 0 && (peers & lt) == 0)
-            atomicAdd(&s_cnt[e], __popc(peers));  // integer counts: order-free
-    }
-    __syncthreads();
-    // exclusive offsets and the list of experts with routes: entry e sums the counts below it
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) {
-        int run = 0, rank = 0;
-        for (int q = 0; q < e; ++q) {
-            const int c = s_cnt[q];
-            run += c;
-            rank += c > 0;
-        }
-        offsets[e] = run;
-        if (e < E) {
-            s_cursor[e] = run;
-            if (s_cnt[e] > 0)
-                slots[rank] = make_int4(e, run, run + s_cnt[e], 0);
+    const int per = (routes + kCompactThreads - 1) / kCompactThreads;
+    const int i0 = min(routes, (int)threadIdx.x * per), i1 = min(routes, i0 + per);
+    int lower = 0, mine = 0;
+    for (int i = i0; i < i1; ++i) {
+        const int x = idx[i];
+        if (x >= 0) {
+            lower += x < e;
+            mine += x == e;
+            if (!(s_has[x >> 5] >> (x & 31) & 1))  // most are there already
+                atomicOr(&s_has[x >> 5], 1u << (x & 31));
         }
     }
-    __syncthreads();
-    const int chunk = nw * 32;
-    for (int c0 = 0; c0 < routes; c0 += chunk) {
-        for (int w = threadIdx.x; w < nw * E; w += blockDim.x)
-            s_wc[w] = 0;
-        __syncthreads();
-        const int i = c0 + threadIdx.x;
-        int e = -1;
-        unsigned peers = 0;
-        if (warp < nw) {  // warp-uniform
-            e = i < routes ? idx[i] : -1;
-            peers = __match_any_sync(0xffffffffu, e);
-            if (e >= 0 && (peers & lt) == 0)
-                s_wc[warp * E + e] = __popc(peers);
-        }
-        __syncthreads();
-        for (int x = threadIdx.x; x < E; x += blockDim.x) {
-            int run = s_cursor[x];
-            for (int w = 0; w < nw; ++w) {
-                const int c = s_wc[w * E + x];
-                s_wc[w * E + x] = run;
-                run += c;
-            }
-            s_cursor[x] = run;
-        }
-        __syncthreads();
-        if (e >= 0) {
-            const int slot = s_wc[warp * E + e] + __popc(peers & lt);
-            route_token[slot] = i / top_k;
-            pos[i] = slot;
-        }
-        __syncthreads();
+    int first = mine;  // inclusive scan of `mine`, sum of `lower`
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int f = __shfl_up_sync(0xffffffffu, first, off);
+        if (lane >= off)
+            first += f;
+        lower += __shfl_xor_sync(0xffffffffu, lower, off);
     }
-}
-
-size_t compact_smem(int num_experts) {
-    int nw = kCompactTableInts / num_experts;
-    nw = nw < 1 ? 1 : (nw > kCompactThreads / 32 ? kCompactThreads / 32 : nw);
-    return sizeof(int) * ((size_t)2 * num_experts + 1 + (size_t)nw * num_experts);
+    if (lane == 31) {
+        s_warp[warp][0] = first;
+        s_warp[warp][1] = lower;
+    }
+    __syncthreads();
+    int before = 0, count = 0, start = 0;
+#pragma unroll
+    for (int w = 0; w < kCompactThreads / 32; ++w) {
+        before += w < warp ? s_warp[w][0] : 0;
+        count += s_warp[w][0];
+        start += s_warp[w][1];
+    }
+    int at = start + before + first - mine;
+    for (int i = i0; i < i1 && mine > 0; ++i)
+        if (idx[i] == e) {
+            route_token[at] = i / top_k;
+            pos[i] = at++;
+        }
+    if (threadIdx.x == 0) {
+        int rank = 0, active = 0;  // experts with routes below this one, and in all
+        for (int w = 0; w < (num_experts + 31) / 32; ++w) {
+            const int n = __popc(s_has[w]);
+            active += n;
+            rank += w < (e >> 5) ? n : w == (e >> 5) ? __popc(s_has[w] & ((1u << (e & 31)) - 1)) : 0;
+        }
+        offsets[e] = start;
+        if (e == num_experts - 1)
+            offsets[num_experts] = start + count;
+        if (count > 0)
+            slots[rank] = make_int4(e, start, start + count, 0);
+        else
+            slots[active + e - rank] = make_int4(0, 0, 0, 0);
+    }
 }
 
 // ---- 1-4 fused for a few tokens (decode) ---------------------------------------------------
@@ -1634,10 +1617,9 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
                                            dim3(128), 0, st, logits, tokens, num_experts, top_k, idx,
                                            wts));
         ctx->launches++;
-        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, moe_compact_kernel, dim3(1),
-                                           dim3(kCompactThreads), compact_smem(num_experts), st, idx,
-                                           tokens, top_k, num_experts, offsets, route_token, pos,
-                                           slots));
+        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, moe_compact_kernel, dim3(num_experts),
+                                           dim3(kCompactThreads), 0, st, idx, tokens, top_k,
+                                           num_experts, offsets, route_token, pos, slots));
         ctx->launches++;
     }
     // which grouped-matmul variant: the few-token one implements the per-128 rule only
