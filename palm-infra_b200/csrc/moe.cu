@@ -1062,17 +1062,20 @@ size_t grouped_small_smem(int k, int groups, int tpc, bool scl16) {
 
 // ---- 5 / 7. grouped expert matmul over ragged route lists ------------------------------
 // Work: an expert's routes, sixteen at a time (a pass), against its tile pairs (16 weight rows
-// each).  A unit is one pass against eight pairs, a pair per warp; the units of all experts lie
-// in one line (expert, pass, pairs) of which every CTA takes an equal, contiguous share, two
-// CTAs per SM, so that one computes while the other changes to another pass.  A pass's int8
-// rows, scales and accumulator biases are staged in shared memory once and serve all units of
-// the share that belong to it.
+// each).  A unit is one pass against a pair per warp of a CTA; the units of all experts lie in
+// one line (expert, pass, pairs) of which every CTA takes an equal, contiguous share, two CTAs
+// of eight warps per SM, so that one computes while the other changes to another pass, or one
+// CTA of sixteen warps where a pass's rows leave no room for two.  A pass's int8 rows, scales
+// and accumulator biases are staged in shared memory once and serve all units of the share that
+// belong to it.
 //
 // The integer sums come from the warp-level int8 tensor instruction (mma.sync m16n8k32): the
 // pair's weight rows are its rows, eight routes its columns.  A warp runs the whole K loop of its
-// pair on its own, with the weights straight from global memory: a 32-k block of a tile is 128
-// contiguous bytes, a word per lane, fetched kAhead groups before use (16 warps x 32 lanes x 10
-// words x 3 groups: 60 KB in flight per SM).  A word is split into unsigned bytes q+8
+// pair on its own: the pair's weights stream through a ring in shared memory that only this warp
+// reads and fills (cp.async), kDepth - 1 groups ahead, on into the next pair, with no barrier in
+// the K loop.  (Straight into registers, three groups ahead, they came later: a warp's
+// outstanding loads share six scoreboards, so a wait for an old group waited for the newest
+// too.)  A word is split into unsigned bytes q+8
 // (lo = (w ^ 0x08080808) & 0x0F0F0F0F for even k, hi = ((w >> 4) ^ 0x08080808) & 0x0F0F0F0F for
 // odd k); the accumulator starts at 0x4B400000 - 8*sum(codes), read from shared memory as the
 // four words the instruction takes, and ends as the bit pattern of the float 12582912 + D.  D is
@@ -1082,11 +1085,8 @@ size_t grouped_small_smem(int k, int groups, int tpc, bool scl16) {
 // What bounds it: issue slots (about 120 instructions per group and pair with sixteen routes,
 // most of them the chain and the split of the words), close to the time the weights take from
 // HBM at sixteen routes per expert.
-constexpr int kGW = 8;          // warps
-constexpr int kGT = kGW * 32;
 constexpr int kGR = 16;         // routes per pass: two column blocks
 constexpr int kRowPad = 16;     // bytes added to a staged activation row: conflict-free reads
-constexpr int kAhead = 3;       // groups whose weights are in flight per warp
 
 struct GroupedArgs {
     const uint8_t* nib;
@@ -1134,29 +1134,18 @@ __device__ __forceinline__ void moe_mma_16x8x32(int (&d)[4], uint32_t a0, uint32
 }
 
 // one group's weights of a lane: a word of each 32-k block of both tiles' row gid, both scales
-template <bool SCL16>
 struct PairWords {
     uint32_t w[2][4];
     float ws[2];
-    __device__ __forceinline__ void load(const uint8_t* nib, size_t tile_bytes, const uint8_t* scl,
-                                         size_t scl_tile_bytes, int g) {
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const uint8_t* p = nib + t * tile_bytes + g * 512;
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-                w[t][b] = __ldg(reinterpret_cast<const uint32_t*>(p + b * 128));
-            const uint8_t* q = scl + t * scl_tile_bytes + g * (SCL16 ? 16 : 32);
-            ws[t] = SCL16 ? __half2float(*reinterpret_cast<const __half*>(q))
-                          : *reinterpret_cast<const float*>(q);
-        }
-    }
 };
+// a warp's ring slot: [2 tiles][512 B], then [2 tiles][8 scales]
+template <bool SCL16>
+constexpr int kPairSlot = 1024 + (SCL16 ? 32 : 64);
 
 // Folds one group of sixteen weight rows into the chain values of `ncb` blocks of eight routes.
 // acc[j][0]: row gid, routes 2*tid and 2*tid+1 of block j; acc[j][1]: row gid+8.
-template <bool A32, bool SCL16>
-__device__ __forceinline__ void pair_group(const PairWords<SCL16>& pw, const uint8_t* rows,
+template <bool A32>
+__device__ __forceinline__ void pair_group(const PairWords& pw, const uint8_t* rows,
                                            int row_bytes, const float* s_as, const int4* s_bias,
                                            int g, int ncb, int tid, uint64_t (&acc)[2][2]) {
     uint32_t lo[2][4], hi[2][4];
@@ -1214,11 +1203,12 @@ __device__ __forceinline__ void pair_group(const PairWords<SCL16>& pw, const uin
     }
 }
 
-template <bool SCL16>
-__global__ void __launch_bounds__(kGT, 2)
+template <bool SCL16, int kGW, int kDepth>
+__global__ void __launch_bounds__(kGW * 32, 16 / kGW)
 moe_grouped_gemv_kernel(const GroupedArgs a) {
     b2w4_pdl_chain_entry();
     extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int kSlot = kPairSlot<SCL16>;
     const int G = a.groups, K = a.k;
     const int row_bytes = K + kRowPad;
     // per (group or 32-block, route): accumulator bias and activation scale; sized for the
@@ -1227,7 +1217,8 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
     int4* s_bias = reinterpret_cast<int4*>(smem);                                 // [4G][kGR / 2]
     float* s_as = reinterpret_cast<float*>(s_bias + (size_t)4 * G * (kGR / 2));   // [4G][kGR]
     uint8_t* s_qa = reinterpret_cast<uint8_t*>(s_as + (size_t)4 * G * kGR);       // [kGR][K+pad]
-    int* s_pre = reinterpret_cast<int*>(s_qa + (size_t)kGR * row_bytes);          // [slots + 1]
+    uint8_t* s_ring = s_qa + (size_t)kGR * row_bytes;                             // [kGW][kDepth]
+    int* s_pre = reinterpret_cast<int*>(s_ring + kGW * kDepth * kSlot);           // [slots + 1]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tid = lane & 3;
 
@@ -1257,8 +1248,8 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
             s_pre[a.slot_count] = carry;
     }
     __syncthreads();
-    // tiles_e is a multiple of 16 (n_e is one of 128): whole rounds of kGW pairs
-    const int rounds = a.tiles_e / (2 * kGW);
+    const int pairs = a.tiles_e / 2;  // n_e is a multiple of 128
+    const int rounds = (pairs + kGW - 1) / kGW;
     const long long total = (long long)s_pre[a.slot_count] * rounds;
     long long u = total * blockIdx.x / gridDim.x;
     const long long u_end = total * (blockIdx.x + 1) / gridDim.x;
@@ -1284,17 +1275,37 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
         const bool a32 = a.qa32 != nullptr && slot.z - slot.y >= 2;
         const int spg = a32 ? 4 : 1;  // scales per group
 
-        // this lane's words of a pair: row gid of the tile, bytes 4*tid..+3 of every block
+        // this warp's pairs in the share, group by group: the next one to fetch
         const size_t tile0 = (size_t)(slot.x - a.expert_begin) * a.tiles_e;
-        const uint8_t* nib = a.nib + (tile0 + 2 * (round0 * kGW + warp)) * tile_bytes + lane * 4;
-        const uint8_t* scl = reinterpret_cast<const uint8_t*>(a.scl) +
-                             (tile0 + 2 * (round0 * kGW + warp)) * scl_tile_bytes +
-                             gid * (SCL16 ? 2 : 4);
-        PairWords<SCL16> pw[kAhead];
+        int f_pair = round0 * kGW + warp, f_g = 0, f_slot = 0;
+        const int pair_end = min(pairs, round1 * kGW);
+        uint8_t* const ring = s_ring + warp * (kDepth * kSlot);
+        auto fetch = [&]() {
+            if (f_pair < pair_end) {
+                const size_t at = (tile0 + 2 * f_pair) * G + f_g;
+                uint8_t* dst = ring + f_slot * kSlot;
 #pragma unroll
-        for (int i = 0; i < kAhead; ++i)
-            if (i < G)
-                pw[i].load(nib, tile_bytes, scl, scl_tile_bytes, i);
+                for (int t = 0; t < 2; ++t)
+                    moe_cp_async<16>(dst + t * 512 + lane * 16,
+                                     a.nib + (at + (size_t)t * G) * 512 + lane * 16);
+                constexpr int kScl = SCL16 ? 16 : 32;  // bytes of a tile's eight scales
+                if (lane < kScl / 8) {
+                    const int t = lane / (kScl / 16), c = lane % (kScl / 16);
+                    moe_cp_async<16>(dst + 1024 + lane * 16,
+                                     reinterpret_cast<const uint8_t*>(a.scl) +
+                                         (at + (size_t)t * G) * kScl + c * 16);
+                }
+                f_slot = f_slot + 1 == kDepth ? 0 : f_slot + 1;
+                if (++f_g == G) {
+                    f_g = 0;
+                    f_pair += kGW;
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll
+        for (int i = 0; i < kDepth - 1; ++i)
+            fetch();
 
         // the pass's rows, a warp per row, all copies in flight at once
         for (int mi = warp; mi < mc; mi += kGW) {
@@ -1318,34 +1329,41 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
 
         const int ncb = (mc + 7) >> 3;  // column blocks in this pass: 1 or 2
         const uint8_t* rows = s_qa + gid * row_bytes + tid * 32;
+        int slot_at = 0;
 #pragma unroll 1
         for (int round = round0; round < round1; ++round) {
+            if (round * kGW + warp >= pairs)
+                break;
             uint64_t acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
             auto run = [&](auto rule) {
-#pragma unroll 3
+#pragma unroll 2
                 for (int g = 0; g < G; ++g) {
-                    const PairWords<SCL16> now = pw[0];
+                    __syncwarp();  // every lane has read the slot that is filled now
+                    fetch();
+                    asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+                    __syncwarp();
+                    const uint8_t* src = ring + slot_at * kSlot;
+                    slot_at = slot_at + 1 == kDepth ? 0 : slot_at + 1;
+                    PairWords now;
 #pragma unroll
-                    for (int i = 0; i + 1 < kAhead; ++i)
-                        pw[i] = pw[i + 1];
-                    if (g + kAhead < G)
-                        pw[kAhead - 1].load(nib, tile_bytes, scl, scl_tile_bytes, g + kAhead);
-                    pair_group<decltype(rule)::value, SCL16>(now, rows, row_bytes, s_as, s_bias, g,
-                                                             ncb, tid, acc);
+                    for (int t = 0; t < 2; ++t) {
+#pragma unroll
+                        for (int b = 0; b < 4; ++b)
+                            now.w[t][b] = *reinterpret_cast<const uint32_t*>(src + t * 512 +
+                                                                             b * 128 + lane * 4);
+                        now.ws[t] =
+                            SCL16 ? __half2float(reinterpret_cast<const __half*>(src + 1024)[t * 8 +
+                                                                                             gid])
+                                  : reinterpret_cast<const float*>(src + 1024)[t * 8 + gid];
+                    }
+                    pair_group<decltype(rule)::value>(now, rows, row_bytes, s_as, s_bias, g, ncb,
+                                                      tid, acc);
                 }
             };
             if (a32)
                 run(std::true_type{});
             else
                 run(std::false_type{});
-            nib += 2 * kGW * tile_bytes;
-            scl += 2 * kGW * scl_tile_bytes;
-            if (round + 1 < round1) {
-#pragma unroll
-                for (int i = 0; i < kAhead; ++i)
-                    if (i < G)
-                        pw[i].load(nib, tile_bytes, scl, scl_tile_bytes, i);
-            }
             // out[route][n]: the eight lanes of a quarter-warp hold eight consecutive n
             const int n0 = (round * kGW + warp) * 16 + gid;
 #pragma unroll
@@ -1368,9 +1386,24 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
     }
 }
 
-size_t grouped_smem(int k, int groups, int slots) {
+size_t grouped_smem(int k, int groups, int slots, bool scl16, int warps, int depth) {
     return (size_t)4 * groups * (kGR / 2) * sizeof(int4) + sizeof(float) * kGR * groups * 4 +
-           (size_t)kGR * (k + kRowPad) + sizeof(int) * (slots + 1);
+           (size_t)kGR * (k + kRowPad) + sizeof(int) * (slots + 1) +
+           (size_t)warps * depth * (scl16 ? kPairSlot<true> : kPairSlot<false>);
+}
+
+template <int W, int D>
+int launch_grouped_as(b2w4_ctx* ctx, const GroupedArgs& a, bool scl16, size_t smem, int routes) {
+    auto kern = scl16 ? moe_grouped_gemv_kernel<true, W, D> : moe_grouped_gemv_kernel<false, W, D>;
+    static b2w4_smem_optin configured[2];  // per instantiation and device
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[scl16]));
+    // no more CTAs than there can be units (a pass holds at least one route)
+    const long long units = (long long)routes * ((a.tiles_e / 2 + W - 1) / W);
+    const long long room = 16 / W * ctx->sm_count;
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3((int)(units < room ? units : room)),
+                                       dim3(W * 32), smem, ctx->stream, a));
+    ctx->launches++;
+    return B2W4_OK;
 }
 
 // `decode` (few tokens): the shared-memory variant, optionally with SwiGLU + quantiser fused
@@ -1448,21 +1481,20 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
     a.groups = w->groups;
     a.n_e = n_e;
     a.tiles_e = n_e / 8;
-    const size_t smem = grouped_smem(w->k, w->groups, slots_y);
     // the longest rows: those that fit with a pair of tiles beside them (7936, or 7808 with fp32
     // scales), the limit of the operator
     const size_t pair = (size_t)2 * w->groups * (512 + 8 * (scl16 ? 2 : 4));
-    if (smem > 220 * 1024 || grouped_smem(w->k, w->groups, 0) + pair > 235 * 1024)
-        return b2w4_fail(ctx, B2W4_E_INVALID, "moe: K=%d needs %zu B shared memory", w->k, smem);
-    auto kern = scl16 ? moe_grouped_gemv_kernel<true> : moe_grouped_gemv_kernel<false>;
-    static b2w4_smem_optin configured[2];  // per instantiation and device
-    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[scl16]));
-    // no more CTAs than there can be units (a pass holds at least one route)
-    const long long units = (long long)routes * (a.tiles_e / (2 * kGW));
-    const int ctas = (int)(units < 2 * ctx->sm_count ? units : 2 * ctx->sm_count);
-    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(ctas), dim3(kGT), smem, ctx->stream, a));
-    ctx->launches++;
-    return B2W4_OK;
+    if (grouped_smem(w->k, w->groups, 0, scl16, 0, 0) + pair > 235 * 1024)
+        return b2w4_fail(ctx, B2W4_E_INVALID, "moe: K=%d needs too much shared memory", w->k);
+    auto bytes = [&](int warps, int depth) {
+        return grouped_smem(w->k, w->groups, slots_y, scl16, warps, depth);
+    };
+    // two CTAs per SM, else sixteen warps in one, else what the rows leave room for
+    if (bytes(8, 6) <= 112 * 1024)
+        return launch_grouped_as<8, 6>(ctx, a, scl16, bytes(8, 6), routes);
+    if (bytes(16, 6) <= 226 * 1024)
+        return launch_grouped_as<16, 6>(ctx, a, scl16, bytes(16, 6), routes);
+    return launch_grouped_as<8, 4>(ctx, a, scl16, bytes(8, 4), routes);
 }
 
 }  // namespace
