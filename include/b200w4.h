@@ -386,6 +386,26 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      in q_out [tokens][heads][dim], K and V in their cache rows
  *                      past + t.  Bit-identical to b2w4_rms_norm + b2w4_rope +
  *                      the append of b2w4_attention.  dim a multiple of 64, <= 256
+ *   b2w4_attention_step  b2w4_qkv_prepare and b2w4_attention of one token, in one launch
+ *                      where the keys are taken in one block or over a cluster: every
+ *                      block makes the query rows it needs, the one with the last key
+ *                      writes the new cache rows.  The same bits as the two calls;
+ *                      q_work_dev [heads * dim] is used where they are made after all
+ *   b2w4_matmul_norm   b2w4_add_rms_norm (update NULL: b2w4_rms_norm) and b2w4_matmul of
+ *                      its result, which is quantised as it is made and not written;
+ *                      the residual is updated in place.  The same bits as the two
+ *                      calls
+ *   b2w4_matmul_swiglu b2w4_swiglu of merged rows [2k] and b2w4_matmul of its result,
+ *                      likewise
+ *   b2w4_step_matmul   the matmul of a decode step with its neighbours in it (one row,
+ *                      per-128 rule): v = residual (+ update, may be NULL), written to
+ *                      residual_out (another buffer than either; may be NULL without
+ *                      an update); h = rms_norm(v) * norm_weight, written to hidden_out
+ *                      unless NULL; y = w h.  swiglu: w's rows are gate | up and y
+ *                      [n / 2] = SwiGLU of them (n a multiple of 16).  token_dev
+ *                      instead of y: the greedy token.  All rows 16-byte aligned.  The
+ *                      same bits as b2w4_add_rms_norm, b2w4_matmul / b2w4_matmul_argmax
+ *                      and b2w4_swiglu in turn
  *   b2w4_advance       *counter_dev += by, after history_dev[*counter_dev] = *token_dev
  *                      (both optional).  With the position on the device a decode
  *                      step is the same sequence of launches for every token and can
@@ -416,6 +436,20 @@ int b2w4_qkv_prepare(b2w4_ctx* ctx, const float* qkv_dev, int ld, int tokens, in
                      float eps, const float* cos_dev, const float* sin_dev, int past,
                      const int* past_dev, float* q_out_dev, float* k_cache_dev, float* v_cache_dev,
                      int capacity);
+int b2w4_attention_step(b2w4_ctx* ctx, const float* qkv_dev, int heads, int kv_heads, int dim,
+                        const float* q_weight_dev, const float* k_weight_dev, float eps,
+                        const float* cos_dev, const float* sin_dev, int past, const int* past_dev,
+                        float* q_work_dev, float* k_cache_dev, float* v_cache_dev, float* out_dev,
+                        int capacity, float scale);
+int b2w4_matmul_norm(b2w4_ctx* ctx, const b2w4_weight* w, float* residual_dev, int ldr,
+                     const float* update_dev, int ldu, const float* norm_weight_dev, float eps,
+                     float* y_dev, int ldc, int m, int act_rule);
+int b2w4_matmul_swiglu(b2w4_ctx* ctx, const b2w4_weight* w, const float* merged_dev, int ldm,
+                       float* y_dev, int ldc, int m, int act_rule);
+int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_dev,
+                     const float* update_dev, const float* norm_weight_dev, float eps,
+                     float* residual_out_dev, float* hidden_out_dev, int swiglu, float* y_dev,
+                     int32_t* token_dev);
 int b2w4_advance(b2w4_ctx* ctx, int* counter_dev, int by, const int32_t* token_dev,
                  int32_t* history_dev, int history_len);
 int b2w4_copy_rows(b2w4_ctx* ctx, const float* src_dev, int ld_src, float* dst_dev, int ld_dst,

@@ -14,7 +14,7 @@ LIB = os.path.join(HERE, "libb200w4.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 FLAGS = [
-    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
+    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++20",
     "-Xcompiler", "-fPIC",
     # no fast-math anywhere: every rounding point of the W4A8 arithmetic is explicit
     "--fmad=false", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC,

@@ -29,7 +29,8 @@ SYMBOLS = [
     "b2w4_chain_input", "b2w4_chain_output", "b2w4_chain_weight_bytes", "b2w4_chain_set_trace",
     "b2w4_rms_norm", "b2w4_add_rms_norm", "b2w4_swiglu", "b2w4_elementwise", "b2w4_rope",
     "b2w4_attention", "b2w4_embed_rows", "b2w4_copy_rows", "b2w4_advance",
-    "b2w4_qkv_prepare", "b2w4_rope_tables",
+    "b2w4_qkv_prepare", "b2w4_rope_tables", "b2w4_step_matmul", "b2w4_attention_step",
+    "b2w4_matmul_norm", "b2w4_matmul_swiglu",
     "b2w4_kernel_launches",
 ]
 
@@ -131,6 +132,11 @@ def lib():
         L.b2w4_rope_tables.argtypes = [vp, vp, i, i, i, fl]
         L.b2w4_qkv_prepare.argtypes = [vp, f_p, i, i, i, i, i, f_p, f_p, fl, f_p, f_p, i, vp,
                                        f_p, f_p, f_p, i]
+        L.b2w4_matmul_norm.argtypes = [vp, vp, f_p, i, f_p, i, f_p, fl, f_p, i, i, i]
+        L.b2w4_matmul_swiglu.argtypes = [vp, vp, f_p, i, f_p, i, i, i]
+        L.b2w4_step_matmul.argtypes = [vp, vp, f_p, f_p, f_p, fl, f_p, f_p, i, f_p, vp]
+        L.b2w4_attention_step.argtypes = [vp, f_p, i, i, i, f_p, f_p, fl, f_p, f_p, i, vp, f_p,
+                                          f_p, f_p, f_p, i, fl]
         L.b2w4_embed_rows.argtypes = [vp, vp, vp, i, i, f_p, i]
         L.b2w4_copy_rows.argtypes = [vp, f_p, i, f_p, i, i, i]
         L.b2w4_kernel_launches.argtypes = [vp]
@@ -448,6 +454,35 @@ class Context:
             self.handle, _dptr(qkv), qkv.stride(0), tokens, heads, kv_heads, dim,
             _dptr(q_weight), _dptr(k_weight), eps, _dptr(cos), _dptr(sin), past, _dptr(past_dev),
             _dptr(q_out), _dptr(k_cache), _dptr(v_cache), capacity))
+
+    def matmul_norm(self, w, residual, update, norm_weight, eps, y, rule=ACT_G128):
+        """residual += update (if given); y = w rms_norm(residual)."""
+        self._check(lib().b2w4_matmul_norm(
+            self.handle, w.handle, _dptr(residual), residual.stride(0), _dptr(update),
+            update.stride(0) if update is not None else 0, _dptr(norm_weight), eps, _dptr(y),
+            y.stride(0), residual.shape[0], rule))
+
+    def matmul_swiglu(self, w, merged, y, rule=ACT_G128):
+        """y = w swiglu(merged), merged rows gate | up."""
+        self._check(lib().b2w4_matmul_swiglu(self.handle, w.handle, _dptr(merged),
+                                             merged.stride(0), _dptr(y), y.stride(0),
+                                             merged.shape[0], rule))
+
+    def step_matmul(self, w, residual, update, norm_weight, eps, residual_out, y=None,
+                    tokens=None, hidden_out=None, swiglu=False):
+        """One row: the matmul of rms_norm(residual + update); residual_out = residual + update.
+        y: the output row, or its SwiGLU; tokens: the greedy token instead."""
+        self._check(lib().b2w4_step_matmul(
+            self.handle, w.handle, _dptr(residual), _dptr(update), _dptr(norm_weight), eps,
+            _dptr(residual_out), _dptr(hidden_out), int(swiglu), _dptr(y), _dptr(tokens)))
+
+    def attention_step(self, qkv, heads, kv_heads, dim, q_weight, k_weight, eps, cos, sin, past,
+                       q_work, k_cache, v_cache, out, capacity, scale, past_dev=None):
+        """qkv_prepare and attention of one token."""
+        self._check(lib().b2w4_attention_step(
+            self.handle, _dptr(qkv), heads, kv_heads, dim, _dptr(q_weight), _dptr(k_weight), eps,
+            _dptr(cos), _dptr(sin), past, _dptr(past_dev), _dptr(q_work), _dptr(k_cache),
+            _dptr(v_cache), _dptr(out), capacity, scale))
 
     def advance(self, counter_dev, by=1, token_dev=None, history_dev=None):
         """counter_dev[0] += by after history_dev[counter_dev[0]] = token_dev[0]."""

@@ -97,6 +97,20 @@ inline cudaError_t b2w4_opt_in_smem(b2w4_ctx* ctx, Kernel kern, size_t smem,
     return e;
 }
 
+// Rows that a many-row matmul's quantiser makes itself (instead of reading x): residual add (in
+// place) and RMSNorm, or SwiGLU of merged rows [2k].
+struct b2w4_rows {
+    enum { NORM, SWIGLU };
+    int kind, ld;
+    float* residual;
+    const float *update, *weight;
+    int ldu;
+    float eps;
+    const float* merged;
+};
+// NORM: the longest row that fits the shared memory a kernel has without opting in for more
+constexpr int kRowsNormMaxK = 12160;
+
 // kernels' host launchers (defined in the .cu files)
 int b2w4_launch_repack(b2w4_ctx* ctx, const void* dev_blocks, b2w4_weight* w);
 int b2w4_launch_quantize(b2w4_ctx* ctx, const float* x, int lda, int m, int k,
@@ -107,8 +121,14 @@ bool b2w4_gemm_mma_resident(const b2w4_weight* w, int m, int act_rule, int sm_co
 int b2w4_launch_gemm_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                          float* y, int ldc, int m, int act_rule, int activation,
                          int act_n_begin, int act_n_len);
+// 9..32 rows (gemm_rows.cu)
+int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
+                          int ldc, int m, int act_rule, int activation, int act_n_begin,
+                          int act_n_len, const b2w4_rows* from = nullptr);
+// quads: es_t holds every bias twice, (b[2p], b[2p+1], b[2p], b[2p+1]) for the row pair p
 int b2w4_launch_quantize_mma(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
-                             int act_rule, int8_t* q, float* scales_t, int32_t* es_t);
+                             int act_rule, int8_t* q, float* scales_t, int32_t* es_t,
+                             bool quads = false, const b2w4_rows* from = nullptr);
 // Tensor-parallel epilogue of the one-row GEMV: the kernel stores its rows into every rank's
 // copy of the output and the launch's last CTA bumps this rank's arrival counter on every
 // rank.  world == 0: off.
@@ -174,10 +194,22 @@ __device__ __forceinline__ void b2w4_top1_finish(const b2w4_top1_args& t, unsign
 #endif
 
 
+// The row of a decode step's matmul made in its prologue: v = residual (+ update), written to
+// residual_out if given; x = (v * 1/sqrt(mean(v^2) + eps)) * weight, written to hidden_out if
+// given.  16-byte aligned; residual_out is neither residual nor update.
+struct b2w4_norm_args {
+    const float *residual, *update, *weight;
+    float eps;
+    float *residual_out, *hidden_out;
+};
+
+// one row of the GEMV kernel; norm / swiglu (one row, per-128 rule): x made in the prologue, y
+// [n / 2] = silu(first half) * second half (n a multiple of 16)
 int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                      float* y, int ldc, int m, int act_rule, int activation,
                      int act_n_begin, int act_n_len, int32_t* sums,
-                     const b2w4_tp_args* tp = nullptr, const b2w4_top1_args* top1 = nullptr);
+                     const b2w4_tp_args* tp = nullptr, const b2w4_top1_args* top1 = nullptr,
+                     const b2w4_norm_args* norm = nullptr, bool swiglu = false);
 int b2w4_launch_tp_gather(b2w4_ctx* ctx, unsigned long long* stage_local, float* y, int m,
                           int ldc);
 int b2w4_launch_top1_token(b2w4_ctx* ctx, unsigned long long* cells, int32_t* token, int m);
@@ -192,14 +224,16 @@ int b2w4_launch_gemv_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, in
                      const b2w4_tp_args* tp = nullptr, const b2w4_top1_args* top1 = nullptr);
 
 int b2w4_launch_quantize_umma(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
-                              int act_rule, int8_t* q, float* scales);
+                              int act_rule, int8_t* q, float* scales,
+                              const b2w4_rows* from = nullptr);
 // more rows than the kernels above take, on tcgen05: per-128 rule (gemm_tcgen05.cu) and
 // per-32 rule (gemm_tcgen05_a32.cu)
 int b2w4_launch_gemm_tc(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                         float* y, int ldc, int m, int activation, int act_n_begin,
-                        int act_n_len);
+                        int act_n_len, const b2w4_rows* from = nullptr);
 int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
-                          int ldc, int m, int activation, int act_n_begin, int act_n_len);
+                          int ldc, int m, int activation, int act_n_begin, int act_n_len,
+                          const b2w4_rows* from = nullptr);
 
 // activation-quantiser output layouts
 enum {
@@ -249,6 +283,13 @@ __device__ __forceinline__ bool b2w4_act_applies(int n, int act, int begin, int 
     if (len < 0 || (begin == 0 && len >= n_total))
         return true;
     return n >= begin && n < begin + len;
+}
+
+// SWIGLU of kernel_elementwise (kernels/elementwise.cpp:529-570): a division, unlike the MoE
+// op's and the matmul epilogue's g * (1 / (1 + exp(-g))); exp in double, rounded once
+__device__ __forceinline__ float b2w4_swiglu_value(float g, float u) {
+    const float e = (float)exp(-(double)g);
+    return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.f, e)), u);
 }
 
 // One activation group: amax -> scale / inverse -> round-to-nearest-even codes.

@@ -306,25 +306,25 @@ static int check_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const void* x, int 
 }
 
 // Up to eight activation rows stream the weight once through the GEMV kernels (one row:
-// dp4a; two to eight: the warp-level int8 tensor instruction); more rows go to the tcgen05
-// kernel (K <= 10240).  All produce the same bits for the same activation rule.
+// dp4a; two to eight: the warp-level int8 tensor instruction), up to 32 through the kernel of
+// gemm_rows.cu; more rows go to the tcgen05 kernels (K <= 10240).  All produce the same bits for
+// the same activation rule.
 static int matmul_dispatch(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                            float* y, int ldc, int m, int act_rule, int activation,
                            int act_n_begin, int act_n_len) {
     const bool rows = m > ctx->gemv_max_rows;
-    // unaligned activation rows: the tcgen05 path's quantiser reads scalars
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (lda & 3) == 0;
     const bool tc = rows && w->groups <= 80;
-    // mma.sync with register accumulators: when asked for, or when the tensor-core kernel
-    // cannot take the call; of itself under the per-128 rule for weights whose CTAs are all
-    // resident at once, and under the per-32 rule for up to 32 rows (measured: a quarter of
-    // a token block does not pay for the tensor-memory pipeline)
+    if (rows && m <= 32 && ctx->gemm_kind == 0)
+        return b2w4_launch_gemm_rows(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
+                                     act_n_len);
+    // mma.sync with the weights in shared memory (its quantiser needs aligned rows): when asked
+    // for, when the tensor-core kernel cannot take the call, or, under the per-128 rule, for
+    // weights whose CTAs are all resident at once
     const bool mma = rows && vec && b2w4_gemm_mma_fits(w, m, act_rule) &&
                      (ctx->gemm_kind == 2 || !tc ||
-                      (ctx->gemm_kind == 0 &&
-                       (act_rule == B2W4_ACT_G128
-                            ? b2w4_gemm_mma_resident(w, m, act_rule, ctx->sm_count)
-                            : m <= 32)));
+                      (ctx->gemm_kind == 0 && act_rule == B2W4_ACT_G128 &&
+                       b2w4_gemm_mma_resident(w, m, act_rule, ctx->sm_count)));
     if (mma)
         return b2w4_launch_gemm_mma(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
                                     act_n_len);
@@ -346,6 +346,63 @@ int b2w4_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* x_dev, int lda
         return rc;
     return matmul_dispatch(ctx, w, x_dev, lda, y_dev, ldc, m, act_rule, activation,
                            act_n_begin, act_n_len);
+}
+
+// A matmul whose rows the quantiser makes.  Calls that go to a kernel with a quantiser of its own
+// inside (few rows, weights resident in shared memory) get them made in scratch.
+static int matmul_rows(b2w4_ctx* ctx, const b2w4_weight* w, const b2w4_rows& from, float* y,
+                       int ldc, int m, int act_rule) {
+    // (the norm's quantiser keeps a row in shared memory, and adds as the operator's block does)
+    const bool made = from.kind == b2w4_rows::SWIGLU || (w->k <= kRowsNormMaxK && w->k > 256);
+    if (made && m > ctx->gemv_max_rows && ctx->gemm_kind == 0) {
+        if (m <= 32)
+            return b2w4_launch_gemm_rows(ctx, w, nullptr, 0, y, ldc, m, act_rule, B2W4_NONE, 0, -1,
+                                         &from);
+        if (w->groups <= 80 && act_rule == B2W4_ACT_G32)
+            return b2w4_launch_gemm_tc32(ctx, w, nullptr, 0, y, ldc, m, B2W4_NONE, 0, -1, &from);
+        if (w->groups <= 80 && !b2w4_gemm_mma_resident(w, m, act_rule, ctx->sm_count))
+            return b2w4_launch_gemm_tc(ctx, w, nullptr, 0, y, ldc, m, B2W4_NONE, 0, -1, &from);
+    }
+    void* x = nullptr;
+    int rc = b2w4_reserve(ctx, SCR_STAGE_X, sizeof(float) * (size_t)m * w->k, &x);
+    if (rc != B2W4_OK)
+        return rc;
+    float* rows = static_cast<float*>(x);
+    if (from.kind == b2w4_rows::SWIGLU)
+        rc = b2w4_swiglu(ctx, from.merged, from.ld, m, w->k, rows, w->k);
+    else if (from.update)
+        rc = b2w4_add_rms_norm(ctx, from.residual, from.ld, from.update, from.ldu, m, w->k,
+                               from.weight, from.eps, rows, w->k);
+    else
+        rc = b2w4_rms_norm(ctx, from.residual, from.ld, m, w->k, from.weight, from.eps, rows,
+                           w->k);
+    if (rc != B2W4_OK)
+        return rc;
+    return matmul_dispatch(ctx, w, rows, w->k, y, ldc, m, act_rule, B2W4_NONE, 0, -1);
+}
+
+int b2w4_matmul_norm(b2w4_ctx* ctx, const b2w4_weight* w, float* residual_dev, int ldr,
+                     const float* update_dev, int ldu, const float* norm_weight_dev, float eps,
+                     float* y_dev, int ldc, int m, int act_rule) {
+    int rc = check_matmul(ctx, w, residual_dev, ldr, y_dev, ldc, m, act_rule, B2W4_NONE);
+    if (rc != B2W4_OK)
+        return rc;
+    if (!norm_weight_dev || (update_dev && ldu < w->k))
+        return b2w4_fail(ctx, B2W4_E_INVALID, "matmul_norm: bad argument");
+    const b2w4_rows from = {b2w4_rows::NORM, ldr, residual_dev, update_dev, norm_weight_dev, ldu,
+                            eps, nullptr};
+    return matmul_rows(ctx, w, from, y_dev, ldc, m, act_rule);
+}
+
+int b2w4_matmul_swiglu(b2w4_ctx* ctx, const b2w4_weight* w, const float* merged_dev, int ldm,
+                       float* y_dev, int ldc, int m, int act_rule) {
+    int rc = check_matmul(ctx, w, merged_dev, ldm, y_dev, ldc, m, act_rule, B2W4_NONE);
+    if (rc != B2W4_OK)
+        return rc;
+    if (ldm < 2 * w->k)
+        return b2w4_fail(ctx, B2W4_E_INVALID, "matmul_swiglu: merged rows hold 2 * %d values", w->k);
+    const b2w4_rows from = {b2w4_rows::SWIGLU, ldm, nullptr, nullptr, nullptr, 0, 0.f, merged_dev};
+    return matmul_rows(ctx, w, from, y_dev, ldc, m, act_rule);
 }
 
 int b2w4_matmul_host(b2w4_ctx* ctx, const b2w4_weight* w, const float* x_host, int lda,
@@ -440,6 +497,34 @@ int b2w4_matmul_argmax(b2w4_ctx* ctx, const b2w4_weight* w, const float* x_dev, 
     if (rc != B2W4_OK)
         return rc;
     return b2w4_launch_top1_token(ctx, top1.cells, token_dev, m);
+}
+
+int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_dev,
+                     const float* update_dev, const float* norm_weight_dev, float eps,
+                     float* residual_out_dev, float* hidden_out_dev, int swiglu, float* y_dev,
+                     int32_t* token_dev) {
+    if (!ctx)
+        return B2W4_E_INVALID;
+    if (!w || !residual_dev || !norm_weight_dev || (update_dev && !residual_out_dev) ||
+        (swiglu ? token_dev || !y_dev || w->n % 16 : !token_dev == !y_dev))
+        return b2w4_fail(ctx, B2W4_E_INVALID, "step_matmul: bad argument");
+    const uintptr_t all = (uintptr_t)residual_dev | (uintptr_t)update_dev |
+                          (uintptr_t)norm_weight_dev | (uintptr_t)residual_out_dev |
+                          (uintptr_t)hidden_out_dev;
+    if ((all & 15) || residual_out_dev == residual_dev ||
+        (update_dev && residual_out_dev == update_dev))
+        return b2w4_fail(ctx, B2W4_E_INVALID,
+                         "step_matmul: rows must be 16-byte aligned, the new residual apart");
+    const b2w4_norm_args norm = {residual_dev, update_dev, norm_weight_dev, eps, residual_out_dev,
+                                 hidden_out_dev};
+    b2w4_top1_args top1;
+    top1.cells = top1_cells(ctx);
+    int rc = b2w4_launch_gemv(ctx, w, nullptr, w->k, y_dev, w->n, 1, B2W4_ACT_G128, B2W4_NONE, 0,
+                              -1, nullptr, nullptr, token_dev ? &top1 : nullptr, &norm,
+                              swiglu != 0);
+    if (rc != B2W4_OK || !token_dev)
+        return rc;
+    return b2w4_launch_top1_token(ctx, top1.cells, token_dev, 1);
 }
 
 static int tp_args_from_group(b2w4_ctx* ctx, const b2w4_tp_group* group, int n_offset,

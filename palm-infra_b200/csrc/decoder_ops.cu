@@ -148,8 +148,7 @@ __global__ void swiglu_kernel(const float* __restrict__ merged, int ldm, int row
     const int r = (int)(i / inter), c = (int)(i - (size_t)r * inter);
     const float g = merged[(size_t)r * ldm + c];
     const float u = merged[(size_t)r * ldm + inter + c];
-    const float e = (float)exp(-(double)g);  // in double, rounded once
-    out[(size_t)r * ldo + c] = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.f, e)), u);
+    out[(size_t)r * ldo + c] = b2w4_swiglu_value(g, u);
 }
 
 __global__ void binary_kernel(const float* __restrict__ a, const float* __restrict__ b,
@@ -218,74 +217,71 @@ __global__ void kv_append_kernel(const float* __restrict__ k, const float* __res
 // per-head RMSNorm (weights optional) and the rotary embedding, with exactly the operations of
 // rms_norm_warp_kernel and rope_kernel in their order, Q goes to q_out [tokens][heads][dim],
 // K and V go straight to their cache rows.  Needs rope over the whole head and dim / 2 a
-// multiple of 32, so that both halves of a rotary pair sit in one lane.
-__global__ void qkv_prepare_kernel(const float* __restrict__ qkv, int ld, int tokens, int heads,
-                                   int kv_heads, int dim, const float* __restrict__ q_weight,
-                                   const float* __restrict__ k_weight, float eps,
-                                   const float* __restrict__ cosv, const float* __restrict__ sinv,
-                                   int pos0, const int* __restrict__ pos_dev,
-                                   float* __restrict__ q_out, float* __restrict__ k_cache,
-                                   float* __restrict__ v_cache, int capacity) {
-    b2w4_pdl_chain_entry();
-    const int slots = heads + 2 * kv_heads;
-    const size_t row = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (row >= (size_t)tokens * slots)
-        return;
-    const int pos = pos_dev ? min(*pos_dev, capacity - tokens) : pos0;
-    const int t = (int)(row / slots), slot = (int)(row % slots);
-    const float* xr = qkv + (size_t)t * ld + (size_t)slot * dim;
-    constexpr int kPer = kAttnMaxDim / 32;
+// multiple of 32, so that both halves of a rotary pair sit in one lane.  The head size is a
+// constant of the kernel and indices have 32 bits: 1500 tokens of 32 / 8 heads of 128 took 28 us
+// with a size read at run time and 64-bit divisions.
+// One query or key row, by one warp; stored to dst.
+template <int DIM>
+__device__ __forceinline__ void prepare_row(const float* __restrict__ x,
+                                            const float* __restrict__ w, float eps,
+                                            const float* __restrict__ cosv,
+                                            const float* __restrict__ sinv, int lane,
+                                            float* __restrict__ dst) {
+    constexpr int kPer = DIM / 32, kHi = kPer / 2;  // v[i] pairs with v[i + kHi]
     float v[kPer];
 #pragma unroll
     for (int i = 0; i < kPer; ++i)
-        v[i] = lane + 32 * i < dim ? xr[lane + 32 * i] : 0.f;
-    if (slot >= heads + kv_heads) {  // a value row: copied to its cache row
-        float* dst = v_cache + ((size_t)(slot - heads - kv_heads) * capacity + pos + t) * dim;
-#pragma unroll
-        for (int i = 0; i < kPer; ++i)
-            if (lane + 32 * i < dim)
-                dst[lane + 32 * i] = v[i];
-        return;
-    }
-    const bool is_q = slot < heads;
-    const float* w = is_q ? q_weight : k_weight;
+        v[i] = x[lane + 32 * i];
     if (w) {
         float ss = 0.f;
 #pragma unroll
         for (int i = 0; i < kPer; ++i)
-            if (lane + 32 * i < dim)
-                ss = __fadd_rn(ss, __fmul_rn(v[i], v[i]));
+            ss = __fadd_rn(ss, __fmul_rn(v[i], v[i]));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1)
             ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, off));
-        const float r = __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)dim), eps)));
+        const float r = __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)DIM), eps)));
 #pragma unroll
         for (int i = 0; i < kPer; ++i)
-            if (lane + 32 * i < dim)
-                v[i] = __fmul_rn(__fmul_rn(v[i], r), w[lane + 32 * i]);
+            v[i] = __fmul_rn(__fmul_rn(v[i], r), w[lane + 32 * i]);
     }
-    const int half = dim >> 1, hi = half >> 5;  // v[i] pairs with v[i + hi]
-    float* dst = is_q ? q_out + ((size_t)t * heads + slot) * dim
-                      : k_cache + ((size_t)(slot - heads) * capacity + pos + t) * dim;
 #pragma unroll
-    for (int i = 0; i < kPer / 2; ++i) {
-        if (i < hi) {
-            const int j = lane + 32 * i;
-            const float c = cosv[(size_t)(pos + t) * half + j];
-            const float sn = sinv[(size_t)(pos + t) * half + j];
-            float x0 = 0.f, x1 = 0.f;
-#pragma unroll
-            for (int u = 0; u < kPer; ++u) {  // register picks with compile-time indices
-                if (u == i)
-                    x0 = v[u];
-                if (u == i + hi)
-                    x1 = v[u];
-            }
-            dst[j] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn));
-            dst[j + half] = __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, c));
-        }
+    for (int i = 0; i < kHi; ++i) {
+        const int j = lane + 32 * i;
+        const float c = cosv[j], sn = sinv[j];
+        dst[j] = __fsub_rn(__fmul_rn(v[i], c), __fmul_rn(v[i + kHi], sn));
+        dst[j + DIM / 2] = __fadd_rn(__fmul_rn(v[i], sn), __fmul_rn(v[i + kHi], c));
     }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(256)
+qkv_prepare_kernel(const float* __restrict__ qkv, int ld, unsigned tokens, int heads, int kv_heads,
+                   const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+                   float eps, const float* __restrict__ cosv, const float* __restrict__ sinv,
+                   int pos0, const int* __restrict__ pos_dev, float* __restrict__ q_out,
+                   float* __restrict__ k_cache, float* __restrict__ v_cache, int capacity) {
+    b2w4_pdl_chain_entry();
+    const unsigned slots = heads + 2 * kv_heads;
+    const unsigned row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (row >= tokens * slots)
+        return;
+    const int pos = pos_dev ? min(*pos_dev, capacity - (int)tokens) : pos0;
+    const int t = (int)(row / slots), slot = (int)(row - t * slots);
+    const float* x = qkv + (size_t)t * ld + (size_t)slot * DIM;
+    if (slot >= heads + kv_heads) {  // a value row: copied to its cache row
+        float* dst = v_cache + ((size_t)(slot - heads - kv_heads) * capacity + pos + t) * DIM;
+#pragma unroll
+        for (int i = 0; i < DIM; i += 32)
+            dst[lane + i] = x[lane + i];
+        return;
+    }
+    const bool is_q = slot < heads;
+    prepare_row<DIM>(x, is_q ? q_weight : k_weight, eps, cosv + (size_t)(pos + t) * (DIM / 2),
+                     sinv + (size_t)(pos + t) * (DIM / 2), lane,
+                     is_q ? q_out + ((size_t)t * heads + slot) * DIM
+                          : k_cache + ((size_t)(slot - heads) * capacity + pos + t) * DIM);
 }
 
 // Scaled-dot-product attention of one (query token, head) over the cache, the x86 reference's
@@ -531,6 +527,15 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
 // finite -- a value row that is not, or values near the largest number added up before the
 // division -- every block forms them again from the final probabilities.  A NaN score reaches every
 // feature.
+// PREP (one token): the rows come straight from the fused qkv matmul.  Every block makes the
+// query rows it needs (qkv_prepare_kernel's norm and rotary embedding, a warp per row); the
+// block whose keys end with the new one makes that key and value row too and writes them to the
+// cache before it reads its keys.  A launch of its own for that costs 2.5 to 3 us a layer.
+struct PrepArgs {
+    const float *qkv, *q_weight, *k_weight, *cosv, *sinv;
+    float eps;
+    float *k_cache, *v_cache;
+};
 constexpr int kMaxRanges = 16;
 // blocks per multiprocessor that the registers allow
 constexpr int split_blocks(int dim, int hr) { return dim * hr <= 128 ? 4 : dim * hr <= 256 ? 3 : 2; }
@@ -546,12 +551,13 @@ struct SplitSmem {  // floats of dynamic shared memory before the scores
     static constexpr int kOdd = kTotal + HR;                    // 1: not finite; [1]: any block's
     static constexpr int kScores = (kOdd + 2 + 3) & ~3;         // [keys][HR]
 };
-template <int DIM, int HR, int CTAS>
+// k_cache, v_cache: no __restrict__, with PREP the block reads a row that it wrote
+template <int DIM, int HR, int CTAS, bool PREP>
 __global__ void __launch_bounds__(kAttnThreads, split_blocks(DIM, HR))
-attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
-                       const float* __restrict__ v_cache, float* __restrict__ out, int tokens,
-                       int heads, int kv_heads, int past0, const int* __restrict__ past_dev,
-                       int capacity, float scale, int one_range) {
+attention_split_kernel(const float* __restrict__ q, const float* k_cache, const float* v_cache,
+                       float* __restrict__ out, int tokens, int heads, int kv_heads, int past0,
+                       const int* __restrict__ past_dev, int capacity, float scale, int one_range,
+                       const PrepArgs prep) {
     b2w4_pdl_chain_entry();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -580,6 +586,25 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
     const float* kc = k_cache + ((size_t)kvh * capacity + j0) * DIM;
     const float* vc = v_cache + ((size_t)kvh * capacity + j0) * DIM;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (PREP) {  // query rows to the head of s_acc, which is free until P*V
+        const float* cosv = prep.cosv + (size_t)past * (DIM / 2);
+        const float* sinv = prep.sinv + (size_t)past * (DIM / 2);
+        const size_t row = ((size_t)kvh * capacity + past) * DIM;
+        const bool owner = n > 0 && j0 + n == visible;  // of the new key, the last one
+        if (warp < nh) {
+            prepare_row<DIM>(prep.qkv + row0 + warp * DIM, prep.q_weight, prep.eps, cosv, sinv,
+                             lane, s_acc + warp * DIM);
+        } else if (warp == HR && owner) {
+            prepare_row<DIM>(prep.qkv + (size_t)(heads + kvh) * DIM, prep.k_weight, prep.eps,
+                             cosv, sinv, lane, prep.k_cache + row);
+        } else if (warp == HR + 1 && owner) {
+            const float* x = prep.qkv + (size_t)(heads + kv_heads + kvh) * DIM;
+#pragma unroll
+            for (int i = lane; i < DIM; i += 32)
+                prep.v_cache[row + i] = x[i];
+        }
+        __syncthreads();
+    }
 
     // ---- scores ----
     {
@@ -592,7 +617,8 @@ attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_
             for (int i = 0; i < kF4; ++i) {
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (h < nh)
-                    x = *reinterpret_cast<const float4*>(q + row0 + h * DIM + 32 * i + 4 * part);
+                    x = *reinterpret_cast<const float4*>((PREP ? s_acc : q + row0) + h * DIM +
+                                                         32 * i + 4 * part);
                 qv[h][2 * i] = b2w4_pack2(x.x, x.y);
                 qv[h][2 * i + 1] = b2w4_pack2(x.z, x.w);
             }
@@ -1244,14 +1270,25 @@ __global__ void copy_rows_kernel(const float* __restrict__ src, int ld_src,
 
 // Embedding lookup: rows of an fp16 table widened to fp32 (the reference's EMBEDDING input
 // path widens fp16 rows the same way, engine/engine.cpp:637-672 uploads "hidden").
-__global__ void embed_rows_kernel(const __half* __restrict__ table, const int32_t* __restrict__ ids,
-                                  int rows, int dim, float* __restrict__ out, int ldo) {
+// One block per 1024 features of a row, four per thread (8-byte loads, 16-byte stores where the
+// rows allow it); a thread per feature with 64-bit divisions took 18.5 us for 1500 rows of 2560.
+constexpr int kEmbedThreads = 256;
+__global__ void __launch_bounds__(kEmbedThreads)
+embed_rows_kernel(const __half* __restrict__ table, const int32_t* __restrict__ ids, int dim,
+                  float* __restrict__ out, int ldo, bool aligned) {
     b2w4_pdl_chain_entry();
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * dim)
-        return;
-    const int r = (int)(i / dim), d = (int)(i - (size_t)r * dim);
-    out[(size_t)r * ldo + d] = __half2float(table[(size_t)ids[r] * dim + d]);
+    const int d = (blockIdx.y * kEmbedThreads + threadIdx.x) * 4;
+    const __half* src = table + (size_t)ids[blockIdx.x] * dim + d;
+    float* dst = out + (size_t)blockIdx.x * ldo + d;
+    if (aligned && d < dim) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(src);
+        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+        const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+        *reinterpret_cast<float4*>(dst) = make_float4(lo.x, lo.y, hi.x, hi.y);
+    } else {
+        for (int i = 0; i < 4 && d + i < dim; ++i)
+            dst[i] = __half2float(src[i]);
+    }
 }
 
 // ---- which kernel a call takes, and its launch ----
@@ -1270,6 +1307,7 @@ struct AttnArgs {
     const int* past_dev;
     int capacity;
     float scale;
+    const PrepArgs* prep;  // the split kernel with one token: rows from the qkv matmul
 };
 
 // query heads of a kv head that a block of the split kernel serves
@@ -1372,11 +1410,12 @@ bool cluster_fits(Kernel kern, int ctas) {
     return false;
 }
 
-template <int DIM, int HR, int CTAS>
-int launch_split_ctas(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
-                      bool* placed) {
+template <int DIM, int HR, int CTAS, bool PREP>
+int launch_split_as(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
+                    bool* placed) {
     static b2w4_smem_optin cfg, wide, fits;  // fits: 1 yes, 2 no, per device
-    auto kern = attention_split_kernel<DIM, HR, CTAS>;
+    auto kern = attention_split_kernel<DIM, HR, CTAS, PREP>;
+    const PrepArgs prep = PREP ? *a.prep : PrepArgs();
     const int range = max((keys + CTAS - 1) / CTAS, min(keys, plan.one_range));
     const size_t smem = sizeof(float) * (SplitSmem<DIM, HR>::kScores + (size_t)range * HR);
     const dim3 grid(CTAS, a.kv_heads * ((a.heads / a.kv_heads + HR - 1) / HR), a.tokens);
@@ -1387,7 +1426,7 @@ int launch_split_ctas(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), smem,
                                            ctx->stream, a.q, a.k_cache, a.v_cache, a.out,
                                            a.tokens, a.heads, a.kv_heads, a.past, a.past_dev,
-                                           a.capacity, a.scale, plan.one_range));
+                                           a.capacity, a.scale, plan.one_range, prep));
     } else {
         B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, kern, wide));
         size_t& fit = fits.bytes[ctx->device];
@@ -1398,11 +1437,17 @@ int launch_split_ctas(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan
         B2W4_CUDA(ctx, b2w4_launch_chained_cluster(
                            ctx->pdl, kern, grid, dim3(kAttnThreads), CTAS, smem, ctx->stream,
                            a.q, a.k_cache, a.v_cache, a.out, a.tokens, a.heads, a.kv_heads,
-                           a.past, a.past_dev, a.capacity, a.scale, plan.one_range));
+                           a.past, a.past_dev, a.capacity, a.scale, plan.one_range, prep));
     }
     ctx->launches++;
     *placed = true;
     return B2W4_OK;
+}
+template <int DIM, int HR, int CTAS>
+int launch_split_ctas(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
+                      bool* placed) {
+    return a.prep ? launch_split_as<DIM, HR, CTAS, true>(ctx, a, keys, plan, placed)
+                  : launch_split_as<DIM, HR, CTAS, false>(ctx, a, keys, plan, placed);
 }
 // The planned cluster, or the next smaller one that the device can place.
 template <int DIM, int HR>
@@ -1587,7 +1632,7 @@ int b2w4_attention(b2w4_ctx* ctx, const float* q_dev, const float* k_dev, const 
         ctx->launches++;
     }
     const AttnArgs a = {q_dev, k_cache_dev, v_cache_dev, out_dev, tokens, heads, kv_heads, past,
-                        past_dev, capacity, scale};
+                        past_dev, capacity, scale, nullptr};
     if (plan.form == ATTN_SPLIT) {
         bool placed = false;
         const int rc = launch_split(ctx, a, dim, keys, plan, &placed);
@@ -1637,14 +1682,58 @@ int b2w4_qkv_prepare(b2w4_ctx* ctx, const float* qkv_dev, int ld, int tokens, in
         return b2w4_fail(ctx, B2W4_E_INVALID,
                          "qkv_prepare: bad argument (tokens=%d past=%d capacity=%d dim=%d)", tokens,
                          past, capacity, dim);
-    const size_t threads = (size_t)tokens * (heads + 2 * kv_heads) * 32;
-    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, qkv_prepare_kernel,
-                                       dim3((unsigned)((threads + 255) / 256)), dim3(256), 0,
-                                       ctx->stream, qkv_dev, ld, tokens, heads, kv_heads, dim,
-                                       q_weight_dev, k_weight_dev, eps, cos_dev, sin_dev, past,
-                                       past_dev, q_out_dev, k_cache_dev, v_cache_dev, capacity));
+    auto kern = dim == 64    ? qkv_prepare_kernel<64>
+                : dim == 128 ? qkv_prepare_kernel<128>
+                : dim == 192 ? qkv_prepare_kernel<192>
+                             : qkv_prepare_kernel<256>;
+    const size_t warps = (size_t)tokens * (heads + 2 * kv_heads);
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3((unsigned)((warps + 7) / 8)),
+                                       dim3(256), 0, ctx->stream, qkv_dev, ld, (unsigned)tokens,
+                                       heads, kv_heads, q_weight_dev, k_weight_dev, eps, cos_dev,
+                                       sin_dev, past, past_dev, q_out_dev, k_cache_dev,
+                                       v_cache_dev, capacity));
     ctx->launches++;
     return B2W4_OK;
+}
+
+int b2w4_attention_step(b2w4_ctx* ctx, const float* qkv_dev, int heads, int kv_heads, int dim,
+                        const float* q_weight_dev, const float* k_weight_dev, float eps,
+                        const float* cos_dev, const float* sin_dev, int past, const int* past_dev,
+                        float* q_work_dev, float* k_cache_dev, float* v_cache_dev, float* out_dev,
+                        int capacity, float scale) {
+    if (!ctx)
+        return B2W4_E_INVALID;
+    if (!qkv_dev || !cos_dev || !sin_dev || !q_work_dev || !k_cache_dev || !v_cache_dev ||
+        !out_dev || heads <= 0 || kv_heads <= 0 || heads % kv_heads || dim <= 0 ||
+        dim > kAttnMaxDim || dim % 64 || past < 0 || past + 1 > capacity)
+        return b2w4_fail(ctx, B2W4_E_INVALID,
+                         "attention_step: bad argument (past=%d capacity=%d heads=%d/%d dim=%d)",
+                         past, capacity, heads, kv_heads, dim);
+    const int keys = past_dev ? capacity : past + 1;
+    const bool aligned = !(((uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev |
+                            (uintptr_t)out_dev) & 15);
+    const AttnPlan plan = attn_plan(1, heads, kv_heads, dim, past_dev ? capacity - 1 : past,
+                                    capacity, aligned, !ctx->attn_tiles, ctx->attn_cluster,
+                                    ctx->sm_count);
+    // the refusal of long caches is b2w4_attention's, in every form
+    if (plan.form == ATTN_SPLIT && sizeof(float) * (((keys + 3) & ~3) + kAttnStage) <= 200 * 1024) {
+        const PrepArgs prep = {qkv_dev, q_weight_dev, k_weight_dev, cos_dev, sin_dev,
+                               eps,     k_cache_dev,  v_cache_dev};
+        const AttnArgs a = {nullptr, k_cache_dev, v_cache_dev, out_dev,  1,     heads,
+                            kv_heads, past,       past_dev,    capacity, scale, &prep};
+        bool placed = false;
+        const int rc = launch_split(ctx, a, dim, keys, plan, &placed);
+        if (rc != B2W4_OK || placed)
+            return rc;
+    }
+    const int rc = b2w4_qkv_prepare(ctx, qkv_dev, (heads + 2 * kv_heads) * dim, 1, heads,
+                                    kv_heads, dim, q_weight_dev, k_weight_dev, eps, cos_dev,
+                                    sin_dev, past, past_dev, q_work_dev, k_cache_dev, v_cache_dev,
+                                    capacity);
+    if (rc != B2W4_OK)
+        return rc;
+    return b2w4_attention(ctx, q_work_dev, nullptr, nullptr, k_cache_dev, v_cache_dev, out_dev, 1,
+                          heads, kv_heads, dim, past, past_dev, capacity, scale);
 }
 
 int b2w4_advance(b2w4_ctx* ctx, int* counter_dev, int by, const int32_t* token_dev,
@@ -1679,11 +1768,14 @@ int b2w4_embed_rows(b2w4_ctx* ctx, const void* table_fp16_dev, const int32_t* id
         return B2W4_E_INVALID;
     if (!table_fp16_dev || !ids_dev || !out_dev || rows <= 0 || dim <= 0 || ldo < dim)
         return b2w4_fail(ctx, B2W4_E_INVALID, "embed_rows: bad argument");
-    const size_t n = (size_t)rows * dim;
+    const bool aligned = !(((uintptr_t)table_fp16_dev & 7) | ((uintptr_t)out_dev & 15) |
+                           (dim & 3) | (ldo & 3));
+    const int per_block = 4 * kEmbedThreads;
     B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, embed_rows_kernel,
-                                       dim3((unsigned)((n + 255) / 256)), dim3(256), 0,
-                                       ctx->stream, static_cast<const __half*>(table_fp16_dev),
-                                       ids_dev, rows, dim, out_dev, ldo));
+                                       dim3(rows, (dim + per_block - 1) / per_block),
+                                       dim3(kEmbedThreads), 0, ctx->stream,
+                                       static_cast<const __half*>(table_fp16_dev), ids_dev, dim,
+                                       out_dev, ldo, aligned));
     ctx->launches++;
     return B2W4_OK;
 }

@@ -1,0 +1,330 @@
+// W4G128 x int8 matmul for a few activation rows (9..32: batched decode, short prompts) on the
+// warp-level int8 tensor instruction (mma.sync m16n8k32).
+//
+// Arithmetic = the reference's, row by row, under either rule (kernels/matmul_w4.cpp:211-295 with
+// one activation scale per 128 values, :785-901 with one per 32): per group or 32-k block
+//   D = sum q4*q8 (int32);  y = fma(float(D), fp32(ws*as), y)
+// in ascending order.  The chain value of every (row, weight row) stays in one register of one
+// thread for the whole K loop.
+//
+// Work split.  A warp owns a pair of 8-row weight tiles (the sixteen rows of the instruction) and
+// one or two blocks of eight activation rows (its columns); with more than eight rows two warps
+// share a pair; a CTA holds up to ten warps, so that one or two CTAs per SM take the whole weight
+// in one round.  Weights,
+// codes, scales and accumulator biases stream through a ring of shared-memory stages of four
+// groups, one barrier per stage; the weights of the first stages are on their way before the
+// kernel waits for the quantiser in front (programmatic dependent launch).  (Fetched into
+// registers four groups ahead instead, the weights came no sooner: a warp's outstanding loads
+// share six scoreboards, so a wait for an old group waited for the newest too; 16 rows,
+// [9728, 2560], 23.5 us.)
+// A weight word is split into unsigned bytes q+8 (lo = (w ^ 0x08080808) & 0x0F0F0F0F: even k;
+// hi = ((w >> 4) ^ 0x08080808) & 0x0F0F0F0F: odd k).  The accumulator starts at
+// 0x4B400000 - 8*sum(codes), stored by the quantiser as the four words that the instruction takes,
+// and ends as the bit pattern of the float 12582912 + D (|D| < 2^22): D costs one subtraction,
+// for two columns at once.
+#include "b200w4_internal.cuh"
+
+namespace {
+
+constexpr int kRowsWarps = 10;        // warps per CTA at most
+constexpr int kRowsThreads = kRowsWarps * 32;
+constexpr int kChunk = 4;             // groups per stage
+constexpr int kPitch = kChunk * 128 + 16;  // bytes between a stage's rows: conflict-free reads
+
+struct GemmRowsArgs {
+    const uint8_t* nib;
+    const void* scl;
+    const int8_t* qa;    // [m][K] int8, tensor-operand order inside each group
+    const float* as_t;   // [G * spg][m8] activation scales
+    const int4* es_t;    // [G * spg][m8 / 2] accumulator biases of a row pair, twice
+    float* y;
+    int ldc, m, m8, n, k, groups, tiles, pairs;
+    int activation, act_n_begin, act_n_len;
+};
+
+__device__ __forceinline__ void rows_cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src)
+                 : "memory");
+}
+// lane (gid = lane/4, tid = lane%4): a0 row gid, k 4*tid..+3; a1 row gid+8; a2/a3 k+16;
+// b0 k 4*tid..+3 of column gid, b1 k+16; d0/d1 row gid, columns 2*tid, 2*tid+1; d2/d3 row gid+8
+__device__ __forceinline__ void rows_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                         uint32_t a3, uint32_t b0, uint32_t b1, int4 c) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+        "{%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c.x), "r"(c.y), "r"(c.z),
+          "r"(c.w));
+}
+
+__device__ __noinline__ float rows_activation(float v, int act) { return b2w4_activation(v, act); }
+
+__host__ __device__ constexpr size_t rows_stage_bytes(int m8, int spg, int pairs, bool scl16) {
+    return (size_t)m8 * (kPitch + kChunk * spg * 12) +
+           (size_t)pairs * 2 * kChunk * (512 + (scl16 ? 16 : 32));
+}
+
+// PW warps per pair of weight tiles, CB blocks of eight activation rows per warp, S stages.
+template <int PW, int CB, bool SCL16, bool A32, int S>
+__global__ void __launch_bounds__(kRowsThreads, 2)
+gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
+    constexpr int SPG = A32 ? 4 : 1;  // scales / biases per group
+    constexpr int kScl = SCL16 ? 16 : 32;  // bytes of a tile's scales of a group
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int G = a.groups, m8 = a.m8;
+    const int warps = blockDim.x / 32, pairs = warps / PW;
+    const int bias_bytes = kChunk * SPG * m8 * 8, as_bytes = kChunk * SPG * m8 * 4;
+    const int nib_off = bias_bytes + as_bytes + m8 * kPitch;
+    const int scl_off = nib_off + pairs * 2 * kChunk * 512;
+    const int stage_bytes = (int)rows_stage_bytes(m8, SPG, pairs, SCL16);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gid = lane >> 2, tid = lane & 3;
+    const int pair0 = blockIdx.x * pairs, pair = pair0 + warp / PW;
+    const int cb0 = (warp % PW) * CB;  // first column block
+    const int ncb = min(CB, m8 / 8 - cb0);     // may be none
+    const bool busy = pair < a.pairs && ncb > 0;
+    const int t0 = 2 * pair;
+    const bool two = t0 + 1 < a.tiles;
+    const int tiles_here = min(2 * pairs, a.tiles - 2 * pair0);
+    const int chunks = (G + kChunk - 1) / kChunk;
+
+    b2w4_pdl_launch_dependents();
+    // stage: [tile][group of the chunk][512], then [tile][group][8 scales]
+    auto load_weights = [&](int c) {
+        if (c < chunks) {
+            uint8_t* s = smem + (c % S) * stage_bytes;
+            const int g0 = c * kChunk, gc = min(kChunk, G - g0);
+            const int n16 = gc * 32, s16 = gc * (kScl / 16);
+            for (int t = warp; t < tiles_here; t += warps) {  // a tile per warp
+                const size_t at = (size_t)(2 * pair0 + t) * G + g0;
+                for (int i = lane; i < n16; i += 32)
+                    rows_cp_async16(s + nib_off + t * (kChunk * 512) + i * 16,
+                                    a.nib + at * 512 + i * 16);
+                if (lane < s16)
+                    rows_cp_async16(s + scl_off + t * (kChunk * kScl) + lane * 16,
+                                    reinterpret_cast<const uint8_t*>(a.scl) + at * kScl + lane * 16);
+            }
+        }
+    };
+#pragma unroll
+    for (int c = 0; c < S - 1; ++c)
+        load_weights(c);
+
+    b2w4_pdl_wait();  // quantised activations come from the previous kernel
+    auto load_rows = [&](int c) {
+        if (c < chunks) {
+            uint8_t* s = smem + (c % S) * stage_bytes;
+            const int g0 = c * kChunk, gc = min(kChunk, G - g0);
+            const int n_bias = gc * SPG * m8 / 2, n_as = gc * SPG * m8 / 4, n_row = gc * 8;
+            const int4* es = a.es_t + (size_t)g0 * SPG * (m8 / 2);
+            const float* as = a.as_t + (size_t)g0 * SPG * m8;
+            for (int i = threadIdx.x; i < n_bias; i += blockDim.x)
+                rows_cp_async16(s + i * 16, es + i);
+            for (int i = threadIdx.x; i < n_as; i += blockDim.x)
+                rows_cp_async16(s + bias_bytes + i * 16, as + i * 4);
+            uint8_t* rows = s + bias_bytes + as_bytes;
+            for (int t = warp; t < a.m; t += warps)
+                if (lane < n_row)
+                    rows_cp_async16(rows + t * kPitch + lane * 16,
+                                    a.qa + (size_t)t * a.k + (size_t)g0 * 128 + lane * 16);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int c = 0; c < S - 1; ++c)
+        load_rows(c);
+
+    uint64_t acc[CB][2];  // [0]: row gid, columns 2*tid and 2*tid+1; [1]: row gid+8
+#pragma unroll
+    for (int j = 0; j < CB; ++j)
+        acc[j][0] = acc[j][1] = 0ull;
+    const uint64_t magic = b2w4_pack2(12582912.f, 12582912.f);
+
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+        __syncthreads();  // stage c visible to all; everyone is done with stage c-1
+        load_weights(c + S - 1);
+        load_rows(c + S - 1);
+        const uint8_t* s = smem + (c % S) * stage_bytes;
+        const int4* s_bias = reinterpret_cast<const int4*>(s) + cb0 * 4 + tid;
+        const uint64_t* s_as = reinterpret_cast<const uint64_t*>(s + bias_bytes) + cb0 * 4 + tid;
+        const uint8_t* rows = s + bias_bytes + as_bytes + (cb0 * 8 + gid) * kPitch + tid * 32;
+        // this lane's words: row gid of each tile, bytes 4*tid..+3 of every 32-k block
+        const int tl = t0 - 2 * pair0;
+        const uint32_t* s_w = reinterpret_cast<const uint32_t*>(s + nib_off) + tl * (kChunk * 128) + lane;
+        const uint8_t* s_scl = s + scl_off + tl * (kChunk * kScl) + gid * (kScl / 8);
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i) {
+            if (c * kChunk + i < G && busy) {  // warp-uniform
+                uint32_t lo[2][4], hi[2][4];
+                uint64_t ws2[2];
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const bool have = t == 0 || two;  // a missing tile: zeros
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const uint32_t w = have ? s_w[t * (kChunk * 128) + i * 128 + b * 32] : 0u;
+                        lo[t][b] = (w ^ 0x08080808u) & 0x0F0F0F0Fu;
+                        hi[t][b] = ((w >> 4) ^ 0x08080808u) & 0x0F0F0F0Fu;
+                    }
+                    const uint8_t* q = s_scl + t * (kChunk * kScl) + i * kScl;
+                    const float ws = !have  ? 0.f
+                                     : SCL16 ? __half2float(*reinterpret_cast<const __half*>(q))
+                                             : *reinterpret_cast<const float*>(q);
+                    ws2[t] = b2w4_pack2(ws, ws);
+                }
+                const uint64_t w0 = ws2[0], w1 = ws2[1];
+#pragma unroll
+                for (int j = 0; j < CB; ++j) {
+                    if (j < ncb) {
+                        const uint4* bp =
+                            reinterpret_cast<const uint4*>(rows + j * 8 * kPitch + i * 128);
+                        const uint4 be = bp[0], bo = bp[1];
+                        const uint32_t bev[4] = {be.x, be.y, be.z, be.w};
+                        const uint32_t bov[4] = {bo.x, bo.y, bo.z, bo.w};
+                        auto fold = [&](const int (&d)[4], uint64_t as2) {
+                            // d = 0x4B400000 + D: as a float 12582912 + D, exactly
+                            const uint64_t d0 = b2w4_sub2(
+                                b2w4_pack2(__int_as_float(d[0]), __int_as_float(d[1])), magic);
+                            const uint64_t d1 = b2w4_sub2(
+                                b2w4_pack2(__int_as_float(d[2]), __int_as_float(d[3])), magic);
+                            acc[j][0] = b2w4_fma2(d0, b2w4_mul2(w0, as2), acc[j][0]);
+                            acc[j][1] = b2w4_fma2(d1, b2w4_mul2(w1, as2), acc[j][1]);
+                        };
+                        if (A32) {
+                            // one instruction = one 32-block, folded in ascending order
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) {
+                                const int at = (i * 4 + b) * (m8 / 2) + j * 4;
+                                int d[4];
+                                rows_mma(d, lo[0][b], lo[1][b], hi[0][b], hi[1][b], bev[b], bov[b],
+                                         s_bias[at]);
+                                fold(d, s_as[at]);
+                            }
+                        } else {
+                            // two chains of two instructions (latency), joined by one add
+                            const int at = i * (m8 / 2) + j * 4;
+                            int d[4], e[4];
+                            rows_mma(d, lo[0][0], lo[1][0], hi[0][0], hi[1][0], bev[0], bov[0],
+                                     s_bias[at]);
+                            rows_mma(e, lo[0][1], lo[1][1], hi[0][1], hi[1][1], bev[1], bov[1],
+                                     make_int4(0, 0, 0, 0));
+                            rows_mma(d, lo[0][2], lo[1][2], hi[0][2], hi[1][2], bev[2], bov[2],
+                                     make_int4(d[0], d[1], d[2], d[3]));
+                            rows_mma(e, lo[0][3], lo[1][3], hi[0][3], hi[1][3], bev[3], bov[3],
+                                     make_int4(e[0], e[1], e[2], e[3]));
+#pragma unroll
+                            for (int x = 0; x < 4; ++x)
+                                d[x] += e[x];
+                            fold(d, s_as[at]);
+                        }
+                    }
+                }
+            }
+        }
+    }
+
+    // y[row][n]: for one row, the eight lanes of a quarter-warp hold eight consecutive n
+    if (busy) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int n = (t0 + t) * 8 + gid;
+            const bool act = b2w4_act_applies(n, a.activation, a.act_n_begin, a.act_n_len, a.n);
+#pragma unroll
+            for (int j = 0; j < CB; ++j) {
+                float v[2];
+                b2w4_unpack2(acc[j][t], v[0], v[1]);
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int r = (cb0 + j) * 8 + tid * 2 + x;
+                    if (r < a.m && n < a.n)
+                        a.y[(size_t)r * a.ldc + n] = act ? rows_activation(v[x], a.activation) : v[x];
+                }
+            }
+        }
+    }
+}
+
+template <int PW, int CB, bool SCL16, bool A32>
+int rows_launch(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
+    const int ctas = (a.pairs + pairs_per_cta - 1) / pairs_per_cta;
+    const size_t stage = rows_stage_bytes(a.m8, A32 ? 4 : 1, pairs_per_cta, SCL16);
+    // one CTA per SM: a deeper ring
+    const bool deep = ctas <= ctx->sm_count && 6 * stage <= 220 * 1024;
+    auto kern = deep ? gemm_w4a8_rows_kernel<PW, CB, SCL16, A32, 6>
+                     : gemm_w4a8_rows_kernel<PW, CB, SCL16, A32, 3>;
+    const size_t smem = (deep ? 6 : 3) * stage;
+    static b2w4_smem_optin configured[2];  // per instantiation and device
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[deep]));
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(ctas),
+                                       dim3(pairs_per_cta * PW * 32), smem, ctx->stream,
+                                       a));
+    ctx->launches++;
+    return B2W4_OK;
+}
+
+}  // namespace
+
+int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
+                          int ldc, int m, int act_rule, int activation, int act_n_begin,
+                          int act_n_len, const b2w4_rows* from) {
+    const bool a32 = act_rule == B2W4_ACT_G32;
+    const int G = w->groups, spg = a32 ? 4 : 1, m8 = (m + 7) & ~7;
+    void *qa = nullptr, *sc = nullptr;
+    int rc;
+    // biases (two words per row and scale) in front: sixteen-byte aligned
+    const size_t scales = (size_t)G * spg * m8;
+    if ((rc = b2w4_reserve(ctx, SCR_QA, (size_t)m * w->k, &qa)) != B2W4_OK ||
+        (rc = b2w4_reserve(ctx, SCR_AS, 3 * sizeof(float) * scales, &sc)) != B2W4_OK)
+        return rc;
+    int32_t* es_t = static_cast<int32_t*>(sc);
+    float* as_t = reinterpret_cast<float*>(es_t + 2 * scales);
+    if ((rc = b2w4_launch_quantize_mma(ctx, x, lda, m, w->k, m8, act_rule,
+                                       static_cast<int8_t*>(qa), as_t, es_t, true,
+                                       from)) != B2W4_OK)
+        return rc;
+    GemmRowsArgs a;
+    a.nib = reinterpret_cast<const uint8_t*>(w->nib);
+    a.scl = w->scl;
+    a.qa = static_cast<const int8_t*>(qa);
+    a.as_t = as_t;
+    a.es_t = reinterpret_cast<const int4*>(es_t);
+    a.y = y;
+    a.ldc = ldc;
+    a.m = m;
+    a.m8 = m8;
+    a.n = w->n;
+    a.k = w->k;
+    a.groups = G;
+    a.tiles = w->tiles;
+    a.pairs = (w->tiles + 1) / 2;
+    a.activation = activation;
+    a.act_n_begin = act_n_begin;
+    a.act_n_len = act_n_len;
+    // Up to eight rows a warp per pair, else two.  Pairs per CTA: the fullest SM decides, so the
+    // least (CTAs on it) x (pairs of each); a CTA's own share of the activations counts as half
+    // a pair.
+    const int pw = m8 > 8 ? 2 : 1;
+    int best = 1;
+    long best_cost = -1;
+    for (int p = 1; p <= kRowsWarps / pw; ++p) {
+        const long ctas = (a.pairs + p - 1) / p;
+        const long cost = (ctas + ctx->sm_count - 1) / ctx->sm_count * (2 * p + 1);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = p;
+        }
+    }
+    const bool scl16 = w->scales_fp16 != 0;
+#define B2W4_ROWS(PW, CB)                                                                \
+    (scl16 ? (a32 ? rows_launch<PW, CB, true, true>(ctx, a, best)                        \
+                  : rows_launch<PW, CB, true, false>(ctx, a, best))                      \
+           : (a32 ? rows_launch<PW, CB, false, true>(ctx, a, best)                       \
+                  : rows_launch<PW, CB, false, false>(ctx, a, best)))
+    return m8 > 16 ? B2W4_ROWS(2, 2) : m8 > 8 ? B2W4_ROWS(2, 1) : B2W4_ROWS(1, 1);
+#undef B2W4_ROWS
+}

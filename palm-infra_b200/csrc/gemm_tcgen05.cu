@@ -193,25 +193,28 @@ gemm_w4a8_tc_kernel(const GemmArgs a) {
             fail();
     } else if (warp == kMmaWarp) {
         // =============================== MMA issue ===================================
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_i8(RP);
-            // made once: formed anew for every instruction, the descriptors of a group took
-            // longer than its instructions (1000 rows, [4100, 9728]: 248 -> 189 us)
-            const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kActOff));
-            const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kBOff));
-            for (int g = 0; g < G; ++g) {
-                const int sa = g % kAStages, ra = g / kAStages;
-                const int sb = g % kBStages, rb = g / kBStages;
-                const int b = g % kAcc, use = g / kAcc;
-                if (!mbar_wait(&b_full[sb], rb & 1) || !mbar_wait(&act_full[sa], ra & 1) ||
-                    (use > 0 && !mbar_wait(&acc_free[b], (use - 1) & 1))) {
+        // The whole warp walks the loop and one lane issues; descriptors are made once.  With one
+        // lane walking it and descriptors formed for every instruction, a group's issue took
+        // longer than its instructions (1000 rows, [4100, 9728]: 248 -> 189 us).
+        const uint32_t idesc = umma_idesc_i8(RP);
+        const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kActOff));
+        const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kBOff));
+        for (int g = 0; g < G; ++g) {
+            const int sa = g % kAStages, ra = g / kAStages;
+            const int sb = g % kBStages, rb = g / kBStages;
+            const int b = g % kAcc, use = g / kAcc;
+            const bool ok = mbar_wait(&b_full[sb], rb & 1) && mbar_wait(&act_full[sa], ra & 1) &&
+                            (use == 0 || mbar_wait(&acc_free[b], (use - 1) & 1));
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0)
                     fail();
-                    break;
-                }
-                // descriptor addresses count 16-byte units
-                const uint64_t a_desc = a_desc0 + (uint64_t)(sa * (S::kActStage >> 4));
-                const uint64_t b_desc = b_desc0 + (uint64_t)(sb * (S::kBStage >> 4));
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                break;
+            }
+            // descriptor addresses count 16-byte units
+            const uint64_t a_desc = a_desc0 + (uint64_t)(sa * (S::kActStage >> 4));
+            const uint64_t b_desc = b_desc0 + (uint64_t)(sb * (S::kBStage >> 4));
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
                 for (int mb = 0; mb < n_blocks; ++mb) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j)  // four K = 32 steps inside the swizzle row,
@@ -225,6 +228,7 @@ gemm_w4a8_tc_kernel(const GemmArgs a) {
                 umma_commit(&act_free[sa]);  // the activation stage may be refilled
                 umma_commit(&b_free[sb]);    // the unpacked weights may be overwritten
             }
+            __syncwarp();
         }
     } else if (warp < kEpiWarp0 || warp >= kEpiWarp0 + kEpiActive) {
         // =============================== unpack ======================================
@@ -477,7 +481,7 @@ int launch_nb(b2w4_ctx* ctx, const GemmArgs& a, bool scl16, dim3 grid, int rows)
 // Quantises the activations (separate launch), then runs the tensor-core kernel.
 int b2w4_launch_gemm_tc(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                         float* y, int ldc, int m, int activation, int act_n_begin,
-                        int act_n_len) {
+                        int act_n_len, const b2w4_rows* from) {
     const int G = w->groups;
     if (G > 80)
         return b2w4_fail(ctx, B2W4_E_INVALID, "gemm: K=%d exceeds the scale staging (K<=10240)",
@@ -490,8 +494,8 @@ int b2w4_launch_gemm_tc(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int
             B2W4_OK)
         return rc;
     if ((rc = b2w4_launch_quantize_umma(ctx, x, lda, m, w->k, m_pad, B2W4_ACT_G128,
-                                        static_cast<int8_t*>(qa), static_cast<float*>(as))) !=
-        B2W4_OK)
+                                        static_cast<int8_t*>(qa), static_cast<float*>(as),
+                                        from)) != B2W4_OK)
         return rc;
     // rows per CTA: one wave of CTAs over the SMs when the token extent is one block
     const int nb = m > 128 ? 2 : 1;  // token blocks of 128 per CTA

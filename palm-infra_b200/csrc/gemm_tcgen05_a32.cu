@@ -28,68 +28,91 @@
 // is released at the start (programmatic dependent launch): weights and scales are fetched
 // while the quantiser in front still runs.  Every wait is bounded; on a timeout the kernel
 // flags the status word and drains.
+#include <utility>
+
 #include "tcgen05_ops.cuh"
 
 namespace {
 
-// Roles: producer, MMA issue, two unpack warps, then eight epilogue warps (two column halves x
-// four TMEM lane quarters; a warp's lane quarter is its index mod 4).
-constexpr int kProducerWarp = 0;
-constexpr int kMmaWarp = 1;
-constexpr int kUnpackWarp0 = 2, kUnpackWarps = 2;
-constexpr int kEpiWarp0 = 4, kEpiWarps = 8;
-constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;  // 384: up to 168 registers each
-constexpr int kStages = 4;    // activation and unpacked-weight stages (one group each)
-constexpr int kRawGroups = 2; // groups per nibble copy
-constexpr int kRawSlots = 3;  // nibble copies in flight
-constexpr int kMaxG = 80;     // K <= 10240
+// Roles: one warp that issues MMAs, three that bring operands in, a group in turn, then sixteen
+// epilogue warps (four column quarters x four TMEM lane quarters; a warp's lane quarter is its
+// index mod 4).  640 threads start with 96 registers each; the epilogue's four warpgroups take
+// what the first one gives up.
+constexpr int kMmaWarp = 0;
+constexpr int kUnpackWarp0 = 1, kUnpackWarps = 3;
+constexpr int kEpiWarp0 = 4, kEpiWarps = 16;
+constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;
+constexpr int kRegsStart = 96, kRegsEpi = 104, kRegsOther = 64;
+static_assert(kRegsOther + 4 * kRegsEpi <= 5 * kRegsStart, "registers of the block");
+constexpr int kMaxG = 80;  // K <= 10240
 
 template <int RP>
 struct Smem {
+    // activation and unpacked-weight stages (one group each), groups of nibbles in flight
+    static constexpr int kStages = RP <= 64 ? 6 : 4, kRawSlots = RP <= 64 ? 12 : 6;
     static constexpr int kActStage = 128 * 128;  // 128 tokens x 128 B, swizzled
     static constexpr int kBStage = RP * 128;     // int8 weights, swizzled
-    static constexpr int kRawSlot = (RP / 8) * kRawGroups * 512;  // nibbles: [tile][groups][512]
+    static constexpr int kRawSlot = (RP / 8) * 512;  // nibbles of a group: [tile][512]
     static constexpr int kActOff = 0;
     static constexpr int kBOff = kActOff + kStages * kActStage;
     static constexpr int kRawOff = kBOff + kStages * kBStage;
     static constexpr int kWsOff = kRawOff + kRawSlots * kRawSlot;  // fp32 [G][RP]
     static constexpr int kBarOff = kWsOff + kMaxG * RP * 4;
     static constexpr int kTotal = kBarOff + 512 + 1024;  // barriers, + slack to align the base
-    static constexpr int kStagePitch = RP / 2 + 4;       // output staging, floats per token
+    static constexpr int kStagePitch = RP / 4 + 4;       // output staging, floats per token
     static_assert(kEpiWarps * 32 * kStagePitch * 4 <= kRawOff, "output staging");
     static_assert(kTotal <= 227 * 1024, "shared memory");
 };
 
-// eight columns of two blocks: issue, and the wait that makes the registers readable
+// W (eight or four) columns of two blocks: issue, and the wait that makes the registers readable
+template <int W>
 __device__ __forceinline__ void tmem_issue(uint32_t t0, uint32_t t1, uint32_t (&r)[2][8]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];"
-        : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[0][4]),
-          "=r"(r[0][5]), "=r"(r[0][6]), "=r"(r[0][7]), "=r"(r[1][0]), "=r"(r[1][1]),
-          "=r"(r[1][2]), "=r"(r[1][3]), "=r"(r[1][4]), "=r"(r[1][5]), "=r"(r[1][6]),
-          "=r"(r[1][7])
-        : "r"(t0), "r"(t1)
-        : "memory");
+    if constexpr (W == 8)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];"
+            : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[0][4]),
+              "=r"(r[0][5]), "=r"(r[0][6]), "=r"(r[0][7]), "=r"(r[1][0]), "=r"(r[1][1]),
+              "=r"(r[1][2]), "=r"(r[1][3]), "=r"(r[1][4]), "=r"(r[1][5]), "=r"(r[1][6]),
+              "=r"(r[1][7])
+            : "r"(t0), "r"(t1)
+            : "memory");
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%8];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4, %5, %6, %7}, [%9];"
+            : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[1][0]),
+              "=r"(r[1][1]), "=r"(r[1][2]), "=r"(r[1][3])
+            : "r"(t0), "r"(t1)
+            : "memory");
 }
+template <int W>
 __device__ __forceinline__ void tmem_wait(uint32_t (&r)[2][8]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[0][4]),
-                   "+r"(r[0][5]), "+r"(r[0][6]), "+r"(r[0][7]), "+r"(r[1][0]), "+r"(r[1][1]),
-                   "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[1][4]), "+r"(r[1][5]), "+r"(r[1][6]),
-                   "+r"(r[1][7])
-                 :
-                 : "memory");
+    if constexpr (W == 8)
+        asm volatile("tcgen05.wait::ld.sync.aligned;"
+                     : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[0][4]),
+                       "+r"(r[0][5]), "+r"(r[0][6]), "+r"(r[0][7]), "+r"(r[1][0]), "+r"(r[1][1]),
+                       "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[1][4]), "+r"(r[1][5]), "+r"(r[1][6]),
+                       "+r"(r[1][7])
+                     :
+                     : "memory");
+    else
+        asm volatile("tcgen05.wait::ld.sync.aligned;"
+                     : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[1][0]),
+                       "+r"(r[1][1]), "+r"(r[1][2]), "+r"(r[1][3])
+                     :
+                     : "memory");
 }
 
 template <int RP, bool SCL16>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a8_tc32_kernel(const GemmArgs a) {
-    constexpr int CH = RP / 2;  // columns per epilogue thread
+    constexpr int CH = RP / 4;  // columns per epilogue thread
     // A unit is what the MMA warp hands to the epilogue: the accumulators of a group, four
     // blocks of RP columns each, or of half a group where four blocks leave no second buffer.
     constexpr int kUnitBlocks = RP <= 64 ? 4 : 2;
     constexpr int kAccCols = kUnitBlocks * RP;
+    constexpr int kStages = Smem<RP>::kStages, kRawSlots = Smem<RP>::kRawSlots;
     constexpr int kAcc = 512 / kAccCols;
     static_assert(kAcc >= 2, "no accumulator to run ahead into");
     extern __shared__ uint8_t smem_raw[];
@@ -108,9 +131,7 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
     uint64_t* act_full = bars;                  // [kStages] activations of a group landed
     uint64_t* b_full = act_full + kStages;      // [kStages] unpack done
     uint64_t* ab_free = b_full + kStages;       // [kStages] MMAs that read both retired
-    uint64_t* raw_full = ab_free + kStages;     // [kRawSlots] nibble chunk landed
-    uint64_t* raw_free = raw_full + kRawSlots;  // [kRawSlots] unpack warps are done with it
-    uint64_t* acc_full = raw_free + kRawSlots;  // [kAcc] unit complete
+    uint64_t* acc_full = ab_free + kStages;     // [kAcc] unit complete
     uint64_t* acc_free = acc_full + kAcc;       // [kAcc] epilogue has fetched it
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + kAcc);
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -119,16 +140,12 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(&act_full[s], 1);
-            mbar_init(&b_full[s], kUnpackWarps);
+            mbar_init(&b_full[s], 1);
             mbar_init(&ab_free[s], 1);
-        }
-        for (int b = 0; b < kRawSlots; ++b) {
-            mbar_init(&raw_full[b], 1);
-            mbar_init(&raw_free[b], kUnpackWarps);
         }
         for (int b = 0; b < kAcc; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_free[b], 2 * ((m_here + 31) / 32));  // the warps that have tokens
+            mbar_init(&acc_free[b], 4 * ((m_here + 31) / 32));  // the warps that have tokens
         }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -152,73 +169,30 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         return mbar_try_wait(bar, parity) || (!*s_abort && mbar_wait(bar, parity));
     };
 
-    if (warp == kProducerWarp) {
-        // =============================== producer ===================================
-        // lane t copies row tile t's share of a nibble chunk, lane 31 a group's activations
-        const int chunks = (G + kRawGroups - 1) / kRawGroups;
-        auto load_chunk = [&](int chunk) {
-            const int slot = chunk % kRawSlots, g = chunk * kRawGroups, gc = min(kRawGroups, G - g);
-            if (lane == 0)
-                mbar_expect_tx(&raw_full[slot], (uint32_t)r_tiles * gc * 512);
-            __syncwarp();
-            if (lane < r_tiles)
-                bulk_g2s(smem + S::kRawOff + slot * S::kRawSlot + lane * (kRawGroups * 512),
-                         a.nib + ((size_t)(tile0 + lane) * G + g) * 512, (uint32_t)gc * 512,
-                         &raw_full[slot]);
-        };
-        // the weights do not depend on the quantiser in front of this kernel
-        for (int c = 0; c < min(kRawSlots, chunks); ++c)
-            load_chunk(c);
-        b2w4_pdl_wait();
-        // only the 8-token atoms that hold real tokens are copied; the MMA reads whatever the
-        // rest of the 128-token block holds and the epilogue ignores those accumulator rows
-        const uint32_t act_bytes = (uint32_t)((m_here + 7) / 8) * 1024;
-        bool ok = true;
-        for (int g = 0; g < G; ++g) {
-            if (g % kRawGroups == 0 && g / kRawGroups >= kRawSlots) {
-                const int chunk = g / kRawGroups, slot = chunk % kRawSlots, use = chunk / kRawSlots;
-                ok = __all_sync(0xffffffffu, wait(&raw_free[slot], (use - 1) & 1));
-                if (!ok)
-                    break;
-                load_chunk(chunk);
-            }
-            const int s = g % kStages, round = g / kStages;
-            if (round > 0)
-                ok = __all_sync(0xffffffffu, wait(&ab_free[s], (round - 1) & 1));
-            if (!ok)
-                break;
-            if (lane == 31) {
-                mbar_expect_tx(&act_full[s], act_bytes);
-                bulk_g2s(smem + S::kActOff + s * S::kActStage,
-                         a.qa + ((size_t)g * a.m_pad + tok0) * 128, act_bytes, &act_full[s]);
-            }
-        }
-        if (!ok && lane == 0)
-            fail();
-    } else if (warp == kMmaWarp) {
+    if (warp < kEpiWarp0)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
+    else
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsEpi));
+
+    if (warp == kMmaWarp) {
         // =============================== MMA issue ===================================
         if (lane == 0) {
             const uint32_t idesc = umma_idesc_i8(RP);
             const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kActOff));
             const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kBOff));
             int u = 0, use = 0;  // unit buffer and how often it has been filled
-            for (int g = 0; g < G; ++g) {
+            bool ok = true;
+            for (int g = 0; g < G && ok; ++g) {
                 const int s = g % kStages, round = g / kStages;
-                if (!wait(&act_full[s], round & 1) || !wait(&b_full[s], round & 1)) {
-                    fail();
-                    break;
-                }
+                ok = wait(&act_full[s], round & 1) && wait(&b_full[s], round & 1);
                 // descriptor addresses count 16-byte units
                 const uint64_t a_desc = a_desc0 + (uint64_t)(s * (S::kActStage >> 4));
                 const uint64_t b_desc = b_desc0 + (uint64_t)(s * (S::kBStage >> 4));
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                bool ok = true;
 #pragma unroll
                 for (int j0 = 0; j0 < 4; j0 += kUnitBlocks) {
-                    if (use > 0 && !wait(&acc_free[u], (use - 1) & 1)) {
-                        ok = false;
+                    ok = ok && (use == 0 || wait(&acc_free[u], (use - 1) & 1));
+                    if (!ok)
                         break;
-                    }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                     for (int j = 0; j < kUnitBlocks; ++j)  // a K = 32 step = a 32-k block
@@ -231,63 +205,89 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
                         ++use;
                     }
                 }
-                if (!ok) {
-                    fail();
+                if (!ok)
                     break;
-                }
                 umma_commit(&ab_free[s]);  // both stages may be refilled
             }
+            if (!ok)
+                fail();
         }
     } else if (warp < kEpiWarp0) {
-        // =============================== unpack ======================================
-        const int ut = (warp - kUnpackWarp0) * 32 + lane;
-        for (int g = 0; g < G; ++g) {
-            const int chunk = g / kRawGroups, slot = chunk % kRawSlots, cuse = chunk / kRawSlots;
-            const int gi = g % kRawGroups;
+        // ============================ operands of a group ============================
+        // Warp w takes every third group: when the stage is free it starts the bulk copy of the
+        // group's activations and unpacks its nibbles, which it has copied itself, some groups
+        // ahead and before the quantiser in front has finished: no barrier between that copy and
+        // its use.  (All unpack warps on one group at a time, a group took their whole latency;
+        // nibbles by one bulk copy per row tile, issuing those took a warp 1700 of a group's
+        // 2500 cycles.)
+        const int w0 = warp - kUnpackWarp0;
+        const uint8_t* nib = a.nib + (size_t)tile0 * G * 512 + lane * 16;
+        auto fetch = [&](int g) {
+            if (g < G) {
+                const uint32_t dst =
+                    smem_u32(smem + S::kRawOff + (g % kRawSlots) * S::kRawSlot) + lane * 16;
+                const uint8_t* src = nib + (size_t)g * 512;
+                for (int t = 0; t < r_tiles; ++t)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + t * 512),
+                                 "l"(src + (size_t)t * G * 512)
+                                 : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        constexpr int kOwn = kRawSlots / kUnpackWarps;  // groups a warp has in flight
+        static_assert(kRawSlots % kUnpackWarps == 0, "slots");
+        for (int i = 0; i < kOwn - 1; ++i)
+            fetch(w0 + i * kUnpackWarps);
+        // only the 8-token atoms that hold real tokens are copied; the MMA reads whatever the
+        // rest of the 128-token block holds and the epilogue ignores those rows
+        const uint32_t act_bytes = (uint32_t)((m_here + 7) / 8) * 1024;
+        b2w4_pdl_wait();  // quantised activations come from the previous kernel
+        // chunk `lane` of a tile: 32 k (sub) of weight row `row`; in the operand: atom t (1024 B),
+        // row (128 B), 16-byte chunks 2*sub (even k) and 2*sub+1 (odd k), XOR-swizzled with the row
+        const int sub = lane >> 3, row = lane & 7;
+        const uint32_t even = row * 128 + (((2 * sub) ^ row) << 4);
+        const uint32_t odd = row * 128 + (((2 * sub + 1) ^ row) << 4);
+        for (int g = w0; g < G; g += kUnpackWarps) {
             const int s = g % kStages, round = g / kStages;
-            bool ok = true;
-            if (gi == 0)  // the chunk's nibbles landed
-                ok = __all_sync(0xffffffffu, wait(&raw_full[slot], cuse & 1));
-            if (ok && round > 0)  // MMAs left this stage
-                ok = __all_sync(0xffffffffu, wait(&ab_free[s], (round - 1) & 1));
-            if (!ok) {
+            fetch(g + (kOwn - 1) * kUnpackWarps);  // into the slot of the group before
+            // MMAs left this stage
+            if (round > 0 && !__all_sync(0xffffffffu, wait(&ab_free[s], (round - 1) & 1))) {
                 fail();
                 break;
             }
-            // raw slot: [tile][kRawGroups groups][32 chunks of 16 B]
-            const uint4* raw =
-                reinterpret_cast<const uint4*>(smem + S::kRawOff + slot * S::kRawSlot) + gi * 32;
+            if (lane == 0) {
+                mbar_expect_tx(&act_full[s], act_bytes);
+                bulk_g2s(smem + S::kActOff + s * S::kActStage,
+                         a.qa + ((size_t)g * a.m_pad + tok0) * 128, act_bytes, &act_full[s]);
+            }
+            asm volatile("cp.async.wait_group %0;" ::"n"(kOwn - 1) : "memory");
+            __syncwarp();
+            const uint8_t* raw =
+                smem + S::kRawOff + (g % kRawSlots) * S::kRawSlot + lane * 16;
             uint8_t* bst = smem + S::kBOff + s * S::kBStage;
-            // chunk c of tile t: sub = c/8, row = c%8 -> 32 k of weight row t*8+row
 #pragma unroll 4
-            for (int c = ut; c < r_tiles * 32; c += kUnpackWarps * 32) {
-                const int t = c >> 5, sub = (c >> 3) & 3, row = c & 7;
-                const uint4 w = raw[t * (kRawGroups * 32) + (c & 31)];
+            for (int t = 0; t < r_tiles; ++t) {
+                const uint4 w = *reinterpret_cast<const uint4*>(raw + t * 512);
                 // low nibbles = even k, high nibbles = odd k, in two's complement: a nibble in
                 // the upper half of a byte is the signed byte 16 q
                 constexpr uint32_t kHigh = 0xF0F0F0F0u;
-                const uint4 ev = make_uint4((w.x << 4) & kHigh, (w.y << 4) & kHigh,
-                                            (w.z << 4) & kHigh, (w.w << 4) & kHigh);
-                const uint4 od = make_uint4(w.x & kHigh, w.y & kHigh, w.z & kHigh, w.w & kHigh);
-                // weight row r = t*8+row: atom t (1024 B), row `row` (128 B), 16-byte
-                // chunks 2*sub (even k) and 2*sub+1 (odd k), XOR-swizzled with the row
-                uint8_t* rowp = bst + t * 1024 + row * 128;
-                *reinterpret_cast<uint4*>(rowp + (((2 * sub) ^ row) << 4)) = ev;
-                *reinterpret_cast<uint4*>(rowp + (((2 * sub + 1) ^ row) << 4)) = od;
+                *reinterpret_cast<uint4*>(bst + t * 1024 + even) =
+                    make_uint4((w.x << 4) & kHigh, (w.y << 4) & kHigh, (w.z << 4) & kHigh,
+                               (w.w << 4) & kHigh);
+                *reinterpret_cast<uint4*>(bst + t * 1024 + odd) =
+                    make_uint4(w.x & kHigh, w.y & kHigh, w.z & kHigh, w.w & kHigh);
             }
             // make the generic-proxy writes visible to the tensor core's async proxy
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
+            if (lane == 0)
                 mbar_arrive(&b_full[s]);
-                if (gi == kRawGroups - 1 || g == G - 1)
-                    mbar_arrive(&raw_free[slot]);  // this warp is done with the chunk
-            }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else {
         // =============================== epilogue ====================================
-        const int ew = warp - kEpiWarp0;       // 0..7
-        const int ch = ew >> 2;                // column half
+        const int ew = warp - kEpiWarp0;       // 0..15
+        const int ch = ew >> 2;                // column quarter
         const int lq = warp & 3;               // TMEM lane quarter this warp may read
         const int tok = tok0 + lq * 32 + lane;
         // a warp whose 32 tokens all lie past the last row has no chain to run
@@ -361,45 +361,35 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
                     ++use;
                 }
             };
-            // A chunk is eight columns of two blocks; the next chunk's fetch is in flight while
-            // one is folded into the chain, across units and groups too.
-            constexpr int kChunks = CH / 4, kHalf = kChunks / 2;  // per group, per block pair
-            static_assert(kChunks % 2 == 0 && CH % 8 == 0, "chunk buffers alternate");
-            uint32_t r[2][2][8];
-            auto issue = [&](int i) {
-                const int j = i / kHalf * 2 % kUnitBlocks, c = i % kHalf * 8;
-                const uint32_t t = lane_addr + (uint32_t)(u * kAccCols + j * RP + c);
-                tmem_issue(t, t + RP, r[i & 1]);
-            };
-            unit_wait();
-            issue(0);
+            // A chunk is eight columns (the last one of a thread may be four) of two blocks.
+            constexpr int kHalf = (CH + 7) / 8, kChunks = 2 * kHalf;  // per block pair, per group
+            static_assert(CH % 4 == 0, "columns");
             for (int g = 0; g < G; ++g) {
                 const float asv[4] = {a0.x, a0.y, a0.z, a0.w};
                 a0 = a1;
                 a1 = load_as(g + 2);
                 const float* ws = wsf + g * RP;
-#pragma unroll
-                for (int i = 0; i < kChunks; ++i) {
-                    tmem_wait(r[i & 1]);
-                    if (i + 1 == kChunks || (kUnitBlocks == 2 && i + 1 == kHalf)) {
+                auto step = [&](auto chunk) {
+                    constexpr int i = decltype(chunk)::value;
+                    constexpr int j = i / kHalf * 2, c = i % kHalf * 8, W = c + 8 <= CH ? 8 : 4;
+                    constexpr int ju = j % kUnitBlocks;
+                    if constexpr (ju == 0 && c == 0)
+                        unit_wait();
+                    uint32_t r[2][8];
+                    const uint32_t t = lane_addr + (uint32_t)(u * kAccCols + ju * RP + c);
+                    tmem_issue<W>(t, t + RP, r);
+                    tmem_wait<W>(r);
+                    if constexpr (i + 1 == kChunks || (kUnitBlocks == 2 && i + 1 == kHalf))
                         unit_done();
-                        if (i + 1 < kChunks || g + 1 < G) {
-                            unit_wait();
-                            issue((i + 1) % kChunks);
-                        }
-                    } else {
-                        issue(i + 1);
-                    }
                     // two blocks, in ascending order
-                    const int j = i / kHalf * 2, c = i % kHalf * 8;
                     const uint64_t s0 = b2w4_pack2(asv[j], asv[j]);
                     const uint64_t s1 = b2w4_pack2(asv[j + 1], asv[j + 1]);
 #pragma unroll
-                    for (int h = 0; h < 8; h += 4) {
+                    for (int h = 0; h < W; h += 4) {
                         const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(ws + c + h);
                         auto sums = [&](int b, int e) {
-                            return b2w4_pack2(__int2float_rn((int)r[i & 1][b][e]),
-                                              __int2float_rn((int)r[i & 1][b][e + 1]));
+                            return b2w4_pack2(__int2float_rn((int)r[b][e]),
+                                              __int2float_rn((int)r[b][e + 1]));
                         };
                         uint64_t& lo = acc2[(c + h) / 2];
                         uint64_t& hi = acc2[(c + h) / 2 + 1];
@@ -408,7 +398,10 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
                         lo = b2w4_fma2(sums(1, h), b2w4_mul2(w2.x, s1), lo);
                         hi = b2w4_fma2(sums(1, h + 2), b2w4_mul2(w2.y, s1), hi);
                     }
-                }
+                };
+                [&]<int... I>(std::integer_sequence<int, I...>) {
+                    (step(std::integral_constant<int, I>()), ...);
+                }(std::make_integer_sequence<int, kChunks>());
             }
         }
         if (!live)
@@ -508,7 +501,8 @@ int row_tiles(int tiles, int token_blocks, int sm_count) {
 
 // Quantises the activations per 32 values (separate launch), then runs the kernel above.
 int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
-                          int ldc, int m, int activation, int act_n_begin, int act_n_len) {
+                          int ldc, int m, int activation, int act_n_begin, int act_n_len,
+                          const b2w4_rows* from) {
     const int G = w->groups;
     if (G > kMaxG)
         return b2w4_fail(ctx, B2W4_E_INVALID, "gemm: K=%d exceeds the scale staging (K<=10240)",
@@ -520,7 +514,8 @@ int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
         (rc = b2w4_reserve(ctx, SCR_AS, sizeof(float) * (size_t)G * m_pad * 4, &as)) != B2W4_OK)
         return rc;
     if ((rc = b2w4_launch_quantize_umma(ctx, x, lda, m, w->k, m_pad, B2W4_ACT_G32,
-                                        static_cast<int8_t*>(qa), static_cast<float*>(as))) !=
+                                        static_cast<int8_t*>(qa), static_cast<float*>(as),
+                                        from)) !=
         B2W4_OK)
         return rc;
     const int token_blocks = m_pad / 128;

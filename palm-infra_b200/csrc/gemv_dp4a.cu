@@ -35,6 +35,14 @@
 // integer sum (as a float: exact) and the scale product fp32(ws*as) go to shared memory.
 // Phase 2, after one barrier: one thread per (tile, weight row, activation row) runs the
 // order-sensitive chain of fused multiply-adds over the groups in ascending order.
+//
+// A decode step's neighbours of the matmul run inside it (b2w4_step_matmul), because as launches
+// of their own they cost 2 to 3 us each, all of it latency:
+//   NORM          the row is made here, x = rms_norm(residual + update): every CTA sums the
+//                 squares of the whole row (10 KB from L2) and the first one writes the new
+//                 residual, to another buffer than the one that the others still read
+//   kModeSwiglu   a CTA takes as many tiles of the up rows as of the gate rows, the same ones,
+//                 and stores silu(gate) * up
 #include "b200w4_internal.cuh"
 
 namespace {
@@ -61,9 +69,12 @@ struct GemvArgs {
     int activation, act_n_begin, act_n_len;
     b2w4_tp_args tp;  // tensor-parallel epilogue (world == 0: off)
     b2w4_top1_args top1;  // greedy-token epilogue (MODE 2)
+    b2w4_norm_args norm;  // NORM: how the row is made
+    bool swiglu;          // kModeSwiglu asked for
 };
-// Kernel modes: plain, with the int32 group sums written out, with the greedy-token epilogue.
-constexpr int kModePlain = 0, kModeSums = 1, kModeTop1 = 2;
+// Kernel modes: plain, with the int32 group sums written out, with the greedy-token epilogue,
+// with SwiGLU over the two halves of the weight's rows.
+constexpr int kModePlain = 0, kModeSums = 1, kModeTop1 = 2, kModeSwiglu = 3;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -128,7 +139,7 @@ __device__ __noinline__ float gemv_activation(float v, int act) {
     return b2w4_activation(v, act);
 }
 
-template <int MT, bool SCL16, bool A32, int MODE>
+template <int MT, bool SCL16, bool A32, int MODE, bool NORM = false>
 __global__ void __launch_bounds__(gemv_warps(MT) * 32, 2)
 gemv_w4a8_kernel(const GemvArgs a) {
     constexpr int kWarps = gemv_warps(MT);
@@ -158,8 +169,11 @@ gemv_w4a8_kernel(const GemvArgs a) {
     unsigned long long top1_best = 0ull;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gl = lane >> 3, row = lane & 7;
-    const int tile0 = blockIdx.x * a.tpc;
-    const int ntile = min(a.tpc, a.tiles - tile0);
+    // SwiGLU: half the CTA's tiles are gate tiles, the other half the up tiles of the same rows
+    constexpr bool SWIGLU = MODE == kModeSwiglu;
+    const int tile0 = blockIdx.x * (SWIGLU ? a.tpc / 2 : a.tpc);
+    const int run = SWIGLU ? min(a.tpc / 2, a.tiles / 2 - tile0) : min(a.tpc, a.tiles - tile0);
+    const int ntile = SWIGLU ? 2 * run : run;
 
     // Let the next kernel in the stream become resident and start its own weight copies.
     b2w4_pdl_launch_dependents();
@@ -172,16 +186,19 @@ gemv_w4a8_kernel(const GemvArgs a) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         __syncwarp();
         if (lane < ntile) {
+            const int tile = lane < run ? tile0 + lane : a.tiles / 2 + tile0 + lane - run;
             mbar_expect_tx(&s_bar[lane], (uint32_t)tile_bytes);
             bulk_g2s(s_w + (size_t)lane * tile_bytes,
-                     reinterpret_cast<const uint8_t*>(a.nib) +
-                         (size_t)(tile0 + lane) * tile_bytes,
+                     reinterpret_cast<const uint8_t*>(a.nib) + (size_t)tile * tile_bytes,
                      (uint32_t)tile_bytes, &s_bar[lane]);
         } else if (lane == ntile) {
-            mbar_expect_tx(&s_bar[ntile], (uint32_t)(ntile * scl_tile_bytes));
-            bulk_g2s(s_scl,
-                     reinterpret_cast<const uint8_t*>(a.scl) + (size_t)tile0 * scl_tile_bytes,
-                     (uint32_t)(ntile * scl_tile_bytes), &s_bar[ntile]);
+            const uint8_t* scl = reinterpret_cast<const uint8_t*>(a.scl);
+            const uint32_t run_bytes = (uint32_t)(run * scl_tile_bytes);
+            mbar_expect_tx(&s_bar[ntile], SWIGLU ? 2 * run_bytes : run_bytes);
+            bulk_g2s(s_scl, scl + (size_t)tile0 * scl_tile_bytes, run_bytes, &s_bar[ntile]);
+            if (SWIGLU)
+                bulk_g2s(s_scl + run_bytes, scl + (size_t)(a.tiles / 2 + tile0) * scl_tile_bytes,
+                         run_bytes, &s_bar[ntile]);
         }
     }
 
@@ -199,6 +216,71 @@ gemv_w4a8_kernel(const GemvArgs a) {
     {
         const int half = lane >> 4, h = lane & 15;
         const int n_q = a.m * G;
+        // NORM: residual + update, the row's sum of squares, then (v * r) * weight: the bits of
+        // b2w4_add_rms_norm, whose 256 threads each add every 256th square.  The half-warp's
+        // first group stays in registers; rows of more than 4096 values read the others again.
+        const float* const nr = a.norm.residual;
+        const float* const nu = a.norm.update;
+        auto load8 = [](const float* p, float (&v)[8]) {
+            const float4 lo = *reinterpret_cast<const float4*>(p);
+            const float4 hi = *reinterpret_cast<const float4*>(p + 4);
+            v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+            v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+        };
+        auto store8 = [](float* p, const float (&v)[8]) {
+            *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        };
+        auto residual8 = [&](int at, float (&v)[8]) {
+            load8(nr + at, v);
+            if (nu) {
+                float u[8];
+                load8(nu + at, u);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    v[i] = __fadd_rn(v[i], u[i]);
+            }
+        };
+        float kept[8], kept_w[8], rms = 0.f;
+        if (NORM) {
+            __shared__ float s_ss[8];
+            float ss = 0.f;
+            if (threadIdx.x < 256) {
+#pragma unroll 5
+                for (int d = threadIdx.x; d < K; d += 256) {
+                    const float v = nu ? __fadd_rn(nr[d], nu[d]) : nr[d];
+                    ss = __fadd_rn(ss, __fmul_rn(v, v));
+                }
+            }
+#pragma unroll 1
+            for (int g = warp * 2 + half; g < G; g += kWarps * 2) {
+                const int at = g * 128 + h * 8;
+                const bool keep = g < kWarps * 2;
+                if (!keep && (blockIdx.x != 0 || !a.norm.residual_out))
+                    break;
+                float v[8];
+                residual8(at, v);
+                if (keep) {
+                    load8(a.norm.weight + at, kept_w);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        kept[i] = v[i];
+                }
+                if (blockIdx.x == 0 && a.norm.residual_out)
+                    store8(a.norm.residual_out + at, v);
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+                ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, off));
+            if (lane == 0 && warp < 8)
+                s_ss[warp] = ss;
+            __syncthreads();
+            ss = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
+                ss = __fadd_rn(ss, s_ss[w]);
+            rms = __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)K), a.norm.eps)));
+        }
         const bool vec_x = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (a.lda & 3) == 0;
         // the trip count is the same for both halves of the warp (the shuffles below name
         // all 32 lanes); a half without an item works on zeros and stores nothing
@@ -209,11 +291,19 @@ gemv_w4a8_kernel(const GemvArgs a) {
             const int mi = live ? item / G : 0, g = live ? item % G : 0;
             const float* src = a.x + (size_t)mi * a.lda + (size_t)g * 128 + h * 8;
             float v[8];
-            if (live && vec_x) {  // two 16-byte loads instead of eight scalar ones
-                const float4 lo = *reinterpret_cast<const float4*>(src);
-                const float4 hi = *reinterpret_cast<const float4*>(src + 4);
-                v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
-                v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+            if (NORM) {
+                const int at = g * 128 + h * 8;
+                if (base >= kWarps * 2 && live) {
+                    residual8(at, kept);
+                    load8(a.norm.weight + at, kept_w);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    v[i] = live ? __fmul_rn(__fmul_rn(kept[i], rms), kept_w[i]) : 0.f;
+                if (blockIdx.x == 0 && a.norm.hidden_out && live)
+                    store8(a.norm.hidden_out + at, v);
+            } else if (live && vec_x) {  // two 16-byte loads instead of eight scalar ones
+                load8(src, v);
             } else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -336,6 +426,7 @@ gemv_w4a8_kernel(const GemvArgs a) {
         b2w4_report_timeout(a.status);
     __syncthreads();
 
+    __shared__ float s_gu[SWIGLU ? kMaxTpc * 8 : 1];  // gate rows, then up rows
     // ---- phase 2: fp32 chain, one thread per (tile, activation row, weight row) ---------
 #pragma unroll 1
     for (int t = threadIdx.x; t < ntile * MT * 8; t += kThreads) {
@@ -354,7 +445,9 @@ gemv_w4a8_kernel(const GemvArgs a) {
             if (SUMS && n < a.n)
                 a.sums[((size_t)mi * a.n + n) * (G * SPG) + j] = (int)dv;
         }
-        if (n < a.n) {
+        if (SWIGLU) {
+            s_gu[t] = acc;
+        } else if (n < a.n) {
             if (b2w4_act_applies(n, a.activation, a.act_n_begin, a.act_n_len, a.n))
                 acc = gemv_activation(acc, a.activation);
             if (MODE == kModeTop1) {
@@ -384,6 +477,11 @@ gemv_w4a8_kernel(const GemvArgs a) {
     }
     if (MODE == kModeTop1)
         b2w4_top1_finish(a.top1, top1_best, (threadIdx.x >> 3) % MT, a.m, s_top1);
+    if (SWIGLU) {  // the operations of b2w4_swiglu
+        __syncthreads();
+        for (int t = threadIdx.x; t < run * 8; t += kThreads)
+            a.y[tile0 * 8 + t] = b2w4_swiglu_value(s_gu[t], s_gu[run * 8 + t]);
+    }
 }
 
 // Second half of the tensor-parallel exchange: waits (bounded) until every entry of the
@@ -515,13 +613,15 @@ size_t gemv_smem_bytes(int mt, int k, int groups, int tpc, bool scl16, bool a32)
            sizeof(uint64_t) * (tpc + 1);
 }
 
-template <int MT, bool SCL16, bool A32, int MODE>
+template <int MT, bool SCL16, bool A32, int MODE, bool NORM = false>
 int launch_one(b2w4_ctx* ctx, const GemvArgs& a, size_t smem) {
-    auto kern = gemv_w4a8_kernel<MT, SCL16, A32, MODE>;
+    auto kern = gemv_w4a8_kernel<MT, SCL16, A32, MODE, NORM>;
     static b2w4_smem_optin configured;  // per instantiation and device
     B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((a.tiles + a.tpc - 1) / a.tpc);
+    const int per_cta = MODE == kModeSwiglu ? a.tpc / 2 : a.tpc;
+    const int tiles = MODE == kModeSwiglu ? a.tiles / 2 : a.tiles;
+    cfg.gridDim = dim3((tiles + per_cta - 1) / per_cta);
     cfg.blockDim = dim3(gemv_warps(MT) * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
@@ -538,6 +638,16 @@ int launch_one(b2w4_ctx* ctx, const GemvArgs& a, size_t smem) {
 template <int MT>
 int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, size_t smem) {
     const int mode = a.sums ? kModeSums : (a.top1.cells ? kModeTop1 : kModePlain);
+    if (a.swiglu || a.norm.weight) {  // a decode step: one row, per-128 rule
+        if (a.swiglu)
+            return scl16 ? launch_one<MT, true, false, kModeSwiglu, true>(ctx, a, smem)
+                         : launch_one<MT, false, false, kModeSwiglu, true>(ctx, a, smem);
+        if (a.top1.cells)
+            return scl16 ? launch_one<MT, true, false, kModeTop1, true>(ctx, a, smem)
+                         : launch_one<MT, false, false, kModeTop1, true>(ctx, a, smem);
+        return scl16 ? launch_one<MT, true, false, kModePlain, true>(ctx, a, smem)
+                     : launch_one<MT, false, false, kModePlain, true>(ctx, a, smem);
+    }
 #define B2W4_GEMV_MODES(S, A)                                              \
     (mode == kModeSums   ? launch_one<MT, S, A, kModeSums>(ctx, a, smem)   \
      : mode == kModeTop1 ? launch_one<MT, S, A, kModeTop1>(ctx, a, smem)   \
@@ -554,7 +664,7 @@ int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, size_t sme
 int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                      float* y, int ldc, int m, int act_rule, int activation,
                      int act_n_begin, int act_n_len, int32_t* sums, const b2w4_tp_args* tp,
-                     const b2w4_top1_args* top1) {
+                     const b2w4_top1_args* top1, const b2w4_norm_args* norm, bool swiglu) {
     if (tp && m > kTpMaxRows)
         return b2w4_fail(ctx, B2W4_E_INVALID, "tensor-parallel epilogue: at most %d rows",
                          kTpMaxRows);
@@ -592,6 +702,10 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
         a.top1 = b2w4_top1_args();
         if (top1)
             a.top1 = *top1;
+        a.norm = b2w4_norm_args();
+        if (norm)
+            a.norm = *norm;
+        a.swiglu = swiglu;
         // Tiles per CTA: a CTA's shared memory stays under half an SM's so that two CTAs share
         // an SM, and the launch is one wave of at most 1.75 CTAs per SM.  Measured on the
         // decode shapes of a 4B dense model (148 SMs): N=9728 K=2560 (1216 tiles) 244 CTAs
@@ -607,6 +721,10 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
         tpc = min(tpc, max(1, one_wave));
         if (ctx->gemv_tpc_override > 0)
             tpc = min(tpc, ctx->gemv_tpc_override);
+        if (swiglu) {  // gate and up tiles in pairs
+            const int pairs = w->tiles / 2, ctas = (w->tiles + tpc - 1) / tpc;
+            tpc = min(max(2, budget / per_tile / 2 * 2), 2 * ((pairs + ctas - 1) / ctas));
+        }
         a.tpc = tpc;
         {
             const int ipt = (w->groups + 3) / 4;

@@ -40,16 +40,17 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// The hint lets the hardware park the thread until the phase completes (or about 20 us pass)
-// instead of having it spin through the issue slots the fp32 chain needs.
+// Without a suspend-time hint: with one, waiting threads stay out of the working warps' issue
+// slots but wake late (per-32 matmul, [4100, 9728]: 33 rows 43.9 us with a hint of 20 us, 41.1
+// without; 1000 rows 209 / 206).
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
+        : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     return ok != 0;
 }
@@ -86,6 +87,16 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
     d |= (uint64_t)1 << 46;
     d |= (uint64_t)2 << 61;
     return d;
+}
+// True in one lane (the same one every time) of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(one));
+    return one != 0;
 }
 // kind::i8, int32 accumulate, signed 8-bit A and B, both K-major, M = 128, N = n.
 __device__ __forceinline__ uint32_t umma_idesc_i8(int n) {

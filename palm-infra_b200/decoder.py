@@ -121,6 +121,9 @@ class DenseDecoder:
         self.multi_row_rule = multi_row_rule
         can_fuse = cfg.head_dim % 64 == 0 and cfg.head_dim <= 256
         self.fused_qkv = can_fuse if fused_qkv is None else (fused_qkv and can_fuse)
+        # norms and SwiGLU made by the matmuls' quantisers (contexts without these entries run
+        # operator by operator)
+        self.fused_rows = self.fused_qkv and hasattr(ctx, "matmul_norm")
         sh = weights["shapes"]
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
         self.layers = []
@@ -170,10 +173,15 @@ class DenseDecoder:
         if not cfg.experts:
             gu, act = self._b("gu", T, 2 * cfg.intermediate), self._b("act", T, cfg.intermediate)
         dn = self._b("dn", T, H)
+        fused = T > 1 and self.fused_rows
         c.embed_rows(self.embed, ids_dev, x)
-        c.rms_norm(x, self.layers[0]["ln1"], cfg.eps, h)
+        if not fused:
+            c.rms_norm(x, self.layers[0]["ln1"], cfg.eps, h)
         for li, L in enumerate(self.layers):
-            c.matmul(L["qkv"], h, qkv, rule=rule)
+            if fused:  # x += dn of the layer before
+                c.matmul_norm(L["qkv"], x, dn if li else None, L["ln1"], cfg.eps, qkv, rule=rule)
+            else:
+                c.matmul(L["qkv"], h, qkv, rule=rule)
             if self.fused_qkv:  # norm + rotary embedding + cache append in one launch
                 c.qkv_prepare(qkv, T, cfg.heads, cfg.kv_heads, D, L["q_norm"], L["k_norm"],
                               cfg.eps, self.cos, self.sin, self.past, q, L["k_cache"],
@@ -192,14 +200,20 @@ class DenseDecoder:
                 c.attention(qh, kh, v, L["k_cache"], L["v_cache"], attn, T, cfg.heads,
                             cfg.kv_heads, D, self.past, self.capacity, D ** -0.5, pos_dev)
             c.matmul(L["o"], attn, o, rule=rule)
-            c.add_rms_norm(x, o, L["ln2"], cfg.eps, h)       # x += o; h = norm(x)
+            if not fused or cfg.experts:
+                c.add_rms_norm(x, o, L["ln2"], cfg.eps, h)   # x += o; h = norm(x)
             if cfg.experts:  # router, selection, expert matmuls and combine: one operator
                 c.moe_forward(h, L["router"], cfg.top_k, cfg.intermediate, L["gate_up"],
                               L["down"], dn)
+            elif fused:
+                c.matmul_norm(L["gate_up"], x, o, L["ln2"], cfg.eps, gu, rule=rule)
+                c.matmul_swiglu(L["down"], gu, dn, rule=rule)
             else:
                 c.matmul(L["gate_up"], h, gu, rule=rule)
                 c.swiglu(gu, act)
                 c.matmul(L["down"], act, dn, rule=rule)
+            if fused and li + 1 < len(self.layers):
+                continue
             nxt = self.layers[li + 1]["ln1"] if li + 1 < len(self.layers) else self.final_norm
             c.add_rms_norm(x, dn, nxt, cfg.eps, h)           # x += dn; h = next norm(x)
         if on_device_position:  # history[past] = the token that went in; past += 1

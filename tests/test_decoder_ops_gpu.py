@@ -574,3 +574,125 @@ def test_attention_on_unaligned_rows(ctx, tokens, past, heads, kv_heads, dim):
     if tokens >= 8:
         assert got.tobytes() == want.tobytes()
     assert rel_l2(got, want) < 1e-5
+
+
+@pytest.mark.parametrize("past,heads,kv_heads,dim", [(0, 4, 2, 128), (31, 16, 2, 128),
+                                                     (300, 32, 8, 128), (127, 8, 2, 64),
+                                                     (500, 6, 6, 64), (1000, 4, 2, 256),
+                                                     (40, 6, 2, 192)])
+@pytest.mark.parametrize("on_device", [False, True])
+def test_attention_step_equals_prepare_and_attention(ctx, past, heads, kv_heads, dim, on_device):
+    """One token's norm, rotary embedding, cache append and attention in one launch (or, for a
+    head size that is not split, in the two launches): the bits of the separate operators."""
+    import torch
+    rng = np.random.default_rng(past + dim)
+    cap = past + 70
+    qkv = _dev(rng.normal(0, 1, (1, (heads + 2 * kv_heads) * dim)).astype(np.float32))
+    qw, kw = (_dev(rng.normal(1, 0.1, dim).astype(np.float32)) for _ in range(2))
+    cos, sin = (_dev(t) for t in pkg.decoder.rope_tables(range(cap), dim, 1e6))
+    cache = [_dev(rng.normal(0, 1, (kv_heads, cap, dim)).astype(np.float32)) for _ in range(2)]
+    pos = torch.tensor([past], dtype=torch.int32, device="cuda") if on_device else None
+    host_past = 0 if on_device else past
+    want_kv = [c.clone() for c in cache]
+    q, want, got = (torch.zeros((1, heads * dim), device="cuda") for _ in range(3))
+    ctx.qkv_prepare(qkv, 1, heads, kv_heads, dim, qw, kw, 1e-6, cos, sin, host_past, q,
+                    *want_kv, cap, pos)
+    ctx.attention(q, None, None, *want_kv, want, 1, heads, kv_heads, dim, host_past, cap,
+                  dim ** -0.5, pos)
+    ctx.attention_step(qkv, heads, kv_heads, dim, qw, kw, 1e-6, cos, sin, host_past,
+                       torch.zeros_like(q), *cache, got, cap, dim ** -0.5, pos)
+    ctx.sync()
+    for a, b in zip(cache, want_kv):
+        assert torch.equal(a, b) and torch.equal(got, want)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n,k", [(16, 128), (272, 2560), (4864, 4096), (2560, 9728),
+                                 (19456, 2560)])
+@pytest.mark.parametrize("with_update", [False, True])
+def test_step_matmul_equals_its_operators(ctx, n, k, with_update):
+    """The matmul with the residual add and norm in front and SwiGLU or the greedy token behind:
+    the bits of the operators in turn (rows up to and beyond the 4096 values that stay in
+    registers)."""
+    import torch
+    rng = np.random.default_rng(n + k)
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, n + k, n, k), n, k)
+    x, u, g = (_dev(rng.normal(m, s, (1, k)).astype(np.float32))
+               for m, s in ((0, 2), (0, 1), (1, 0.2)))
+    upd = u if with_update else None
+    res, hid = (torch.zeros((1, k), device="cuda") for _ in range(2))
+    y, want = (torch.zeros((1, n), device="cuda") for _ in range(2))
+    act, want_act = (torch.zeros((1, n // 2), device="cuda") for _ in range(2))
+    tok, want_tok = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+    ctx.step_matmul(w, x, upd, g, 1e-6, res, y=y, hidden_out=hid)
+    ctx.step_matmul(w, x, upd, g, 1e-6, res, y=act, swiglu=True)
+    ctx.step_matmul(w, x, upd, g, 1e-6, res, tokens=tok)
+    want_res, want_hid = x.clone(), torch.zeros((1, k), device="cuda")
+    ctx.add_rms_norm(want_res, u if with_update else torch.zeros_like(x), g, 1e-6, want_hid)
+    ctx.matmul(w, want_hid, want, rule=ol.ACT_G128)
+    ctx.swiglu(want, want_act)
+    ctx.matmul_argmax(w, want_hid, want_tok)
+    ctx.sync()
+    assert torch.equal(res, want_res) and torch.equal(hid, want_hid)
+    assert torch.equal(y, want) and torch.equal(act, want_act) and torch.equal(tok, want_tok)
+    w.free()
+
+
+def test_step_matmul_refuses_what_it_cannot_take(ctx):
+    """The new residual in the old one's place, both or no outputs, rows off 16 bytes."""
+    import torch
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, 1, 24, 128), 24, 128)
+    x, u, g, r = (torch.ones((1, 128), device="cuda") for _ in range(4))
+    y = torch.zeros((1, 24), device="cuda")
+    tok = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for kw in (dict(residual_out=x, y=y), dict(residual_out=u, y=y), dict(residual_out=None, y=y),
+               dict(residual_out=r), dict(residual_out=r, y=y, tokens=tok),
+               dict(residual_out=r, y=y, swiglu=True),
+               dict(residual_out=torch.ones(129, device="cuda")[1:], y=y)):
+        with pytest.raises(pkg.capi.B200W4Error):
+            ctx.step_matmul(w, x, u, g, 1e-6, **kw)
+    w.free()
+
+
+@pytest.mark.parametrize("rows,dim,off", [(1, 2560, 0), (3, 1026, 0), (2, 1024, 1), (70000, 8, 0)])
+def test_embedding_rows_of_any_size(ctx, rows, dim, off):
+    """Rows that four features divide and that they do not, off the store's alignment, and more
+    rows than a grid's second dimension holds."""
+    import torch
+    table = torch.randn((50, dim), device="cuda").half()
+    ids = torch.randint(0, 50, (rows,), dtype=torch.int32, device="cuda")
+    out = torch.zeros(rows * dim + off, device="cuda")[off:].view(rows, dim)
+    ctx.embed_rows(table, ids, out)
+    ctx.sync()
+    assert torch.equal(out, table.float()[ids.long()])
+
+
+@pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
+@pytest.mark.parametrize("m,n,k", [(1, 72, 384), (6, 72, 640), (9, 264, 2560), (33, 136, 5120),
+                                   (150, 264, 5376), (40, 48, 256), (12, 40, 12416)])
+def test_matmuls_that_make_their_rows(ctx, m, n, k, rule):
+    """Residual add + norm, or SwiGLU, in the matmul's quantiser (and, for row counts, weights and
+    row lengths that it does not take, in scratch): the bits of the two calls."""
+    import torch
+    rng = np.random.default_rng(m + k)
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, n + k, n, k), n, k)
+    dev = lambda *shape: _dev(rng.normal(0, 1, shape).astype(np.float32))
+    x, u, g, merged = dev(m, k), dev(m, k), _dev(rng.normal(1, 0.2, k).astype(np.float32)), \
+        dev(m, 2 * k)
+    got, want, h, act = (torch.zeros((m, c), device="cuda") for c in (n, n, k, k))
+    ctx.matmul_swiglu(w, merged, got, rule=rule)
+    ctx.swiglu(merged, act)
+    ctx.matmul(w, act, want, rule=rule)
+    ctx.sync()
+    assert torch.equal(got, want)
+    for update in (None, u):
+        a, b = x.clone(), x.clone()
+        ctx.matmul_norm(w, a, update, g, 1e-6, got, rule=rule)
+        if update is None:
+            ctx.rms_norm(b, g, 1e-6, h)
+        else:
+            ctx.add_rms_norm(b, update, g, 1e-6, h)
+        ctx.matmul(w, h, want, rule=rule)
+        ctx.sync()
+        assert torch.equal(a, b) and torch.equal(got, want)
+    w.free()

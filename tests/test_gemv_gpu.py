@@ -343,6 +343,20 @@ def test_per32_tensor_core_wide_tiles_bit_exact(ctx_tc, tiles):
     assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).tobytes()
 
 
+@pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
+@pytest.mark.parametrize("m,n,k", [(9, 8, 128), (16, 24, 384), (17, 4100, 512), (24, 1000, 640),
+                                   (25, 11848, 256), (32, 9728, 2560), (12, 72, 10368)])
+def test_few_rows_bit_exact(ctx, m, n, k, rule):
+    """9 to 32 rows: one and two column blocks per warp, a last block that is not full, a missing
+    second tile of a pair, fewer groups than are in flight, one to five pairs per CTA, K beyond
+    the tcgen05 kernels'."""
+    blocks = pkg.synth.bg128_weight(20261125, n + k + m + 4, n, k)
+    x = pkg.synth.activations(7, m + 13, m, k)
+    x[m // 3, 32:64] = 0.0  # an all-zero 32-block
+    y, _ = run_gpu(ctx, blocks, n, k, x, rule=rule, sums=False, pad=4 if n % 16 else 0)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=rule).tobytes()
+
+
 def test_config2_prefill_m256_reference_rule(ctx):
     """M=256, K=2560, N=9728 (benchmark configuration 2, prefill) under the reference's rule
     for several rows (per 32 values), the kernel the library picks by itself: bit-exact
