@@ -202,6 +202,9 @@ struct b2w4_norm_args {
     float eps;
     float *residual_out, *hidden_out;
 };
+constexpr int kStepNormMaxK = 4096;  // longest row that the GEMV kernel makes itself
+// the same as a launch of its own (decoder_ops.cu); hidden instead of hidden_out
+int b2w4_launch_step_norm(b2w4_ctx* ctx, const b2w4_norm_args& norm, int k, float* hidden);
 
 // one row of the GEMV kernel; norm / swiglu (one row, per-128 rule): x made in the prologue, y
 // [n / 2] = silu(first half) * second half (n a multiple of 16)

@@ -305,9 +305,27 @@ static int check_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const void* x, int 
     return B2W4_OK;
 }
 
+// Two to eight rows: whether the kernel of gemm_rows.cu (a quantiser's launch, then two latencies
+// of a group per group) is faster than the GEMV kernel on the tensor instruction (one launch; its
+// per-group work grows with the rows, four times as fast per 32 values, and with long rows its CTAs
+// are few).  us, old / new: [9728, 2560] per 32 values 2 rows 8.0 / 9.2, 4 13.5 / 9.2, 8 24.8 / 9.7,
+// per 128 4 6.9 / 8.9, 8 9.7 / 9.2; [2560, 9728] per 32 2 23.5 / 23.0, 8 66.5 / 26.6, per 128 2
+// 10.7 / 22.9, 4 25.3 / 24.0, 8 62.7 / 26.3; [2560, 4096] per 32 4 9.2 / 10.8, 8 21.0 / 11.7, per
+// 128 8 9.6 / 11.7; [19456, 2560] per 32 2 15.0 / 12.0, per 128 2 8.7 / 10.8, 4 13.0 / 10.9;
+// [20000, 1024] per 32 2 6.7 / 5.8, per 128 4 5.1 / 5.5, 8 6.6 / 5.7; [500, 512] never.
+static bool few_rows_streamed(const b2w4_weight* w, int m, int act_rule) {
+    if (m < 2 || w->tiles < 200)
+        return false;
+    if (act_rule == B2W4_ACT_G32)
+        return w->groups >= 48 || w->tiles >= 2048 || m >= (w->tiles >= 512 ? 3 : 5);
+    if (w->groups >= 48)
+        return m >= 4;
+    return w->tiles >= 768 && (m == 8 || (m >= 4 && w->tiles >= 2048 && w->groups >= 16));
+}
+
 // Up to eight activation rows stream the weight once through the GEMV kernels (one row:
-// dp4a; two to eight: the warp-level int8 tensor instruction), up to 32 through the kernel of
-// gemm_rows.cu; more rows go to the tcgen05 kernels (K <= 10240).  All produce the same bits for
+// dp4a; two to eight: the warp-level int8 tensor instruction) or, as up to 32 rows do, through
+// the kernel of gemm_rows.cu; more rows go to the tcgen05 kernels (K <= 10240).  All produce the same bits for
 // the same activation rule.
 static int matmul_dispatch(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                            float* y, int ldc, int m, int act_rule, int activation,
@@ -315,7 +333,8 @@ static int matmul_dispatch(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, 
     const bool rows = m > ctx->gemv_max_rows;
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (lda & 3) == 0;
     const bool tc = rows && w->groups <= 80;
-    if (rows && m <= 32 && ctx->gemm_kind == 0)
+    if (m <= 32 && ctx->gemm_kind == 0 &&
+        (rows || (ctx->gemv_max_rows == 8 && few_rows_streamed(w, m, act_rule))))
         return b2w4_launch_gemm_rows(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
                                      act_n_len);
     // mma.sync with the weights in shared memory (its quantiser needs aligned rows): when asked
@@ -515,16 +534,23 @@ int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_
         (update_dev && residual_out_dev == update_dev))
         return b2w4_fail(ctx, B2W4_E_INVALID,
                          "step_matmul: rows must be 16-byte aligned, the new residual apart");
-    const b2w4_norm_args norm = {residual_dev, update_dev, norm_weight_dev, eps, residual_out_dev,
-                                 hidden_out_dev};
-    b2w4_top1_args top1;
-    top1.cells = top1_cells(ctx);
-    int rc = b2w4_launch_gemv(ctx, w, nullptr, w->k, y_dev, w->n, 1, B2W4_ACT_G128, B2W4_NONE, 0,
-                              -1, nullptr, nullptr, token_dev ? &top1 : nullptr, &norm,
-                              swiglu != 0);
-    if (rc != B2W4_OK || !token_dev)
+    b2w4_norm_args norm = {residual_dev, update_dev, norm_weight_dev, eps, residual_out_dev,
+                           hidden_out_dev};
+    if (!token_dev && w->k <= kStepNormMaxK)
+        return b2w4_launch_gemv(ctx, w, nullptr, w->k, y_dev, w->n, 1, B2W4_ACT_G128, B2W4_NONE, 0,
+                                -1, nullptr, nullptr, nullptr, &norm, swiglu != 0);
+    // the row made first: many CTAs per SM, or more values than a CTA takes up
+    int rc = B2W4_OK;
+    void* hidden = hidden_out_dev;
+    if (!hidden && (rc = b2w4_reserve(ctx, SCR_STAGE_X, sizeof(float) * w->k, &hidden)) != B2W4_OK)
         return rc;
-    return b2w4_launch_top1_token(ctx, top1.cells, token_dev, 1);
+    if ((rc = b2w4_launch_step_norm(ctx, norm, w->k, static_cast<float*>(hidden))) != B2W4_OK)
+        return rc;
+    const float* x = static_cast<const float*>(hidden);
+    if (token_dev)
+        return b2w4_matmul_argmax(ctx, w, x, w->k, 1, nullptr, 0, token_dev);
+    return b2w4_launch_gemv(ctx, w, x, w->k, y_dev, w->n, 1, B2W4_ACT_G128, B2W4_NONE, 0, -1,
+                            nullptr, nullptr, nullptr, nullptr, swiglu != 0);
 }
 
 static int tp_args_from_group(b2w4_ctx* ctx, const b2w4_tp_group* group, int n_offset,

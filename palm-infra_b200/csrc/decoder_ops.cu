@@ -54,14 +54,15 @@ __device__ __forceinline__ float block_max(float v, float* s_part) {
 
 // kernel_rms_norm (kernels/norm.cpp:13-31, :95-121): r = 1/sqrt(sum(x^2)/D + eps),
 // out = (x * r) * w.  With `update`: kernel_add_rms_norm (:123-190): the sum x + update is
-// written back into x (the residual stream) first.  One block per row.
+// written to `sum` (x itself: the residual stream in place) first.  One block per row.
 __global__ void __launch_bounds__(kNormThreads)
-rms_norm_kernel(float* __restrict__ x, int ldx, const float* __restrict__ update, int ldu,
+rms_norm_kernel(const float* x, int ldx, const float* __restrict__ update, int ldu, float* sum,
                 int dim, const float* __restrict__ weight, float eps, float* __restrict__ out,
                 int ldo) {
     b2w4_pdl_chain_entry();
     __shared__ float s_part[kNormThreads / 32];
-    float* xr = x + (size_t)blockIdx.x * ldx;
+    const float* xr = x + (size_t)blockIdx.x * ldx;
+    float* sr = sum + (size_t)blockIdx.x * ldx;
     const float* ur = update ? update + (size_t)blockIdx.x * ldu : nullptr;
     float* orow = out + (size_t)blockIdx.x * ldo;
     // up to kNormHeld values per thread stay in registers between the two passes, all their
@@ -82,7 +83,7 @@ rms_norm_kernel(float* __restrict__ x, int ldx, const float* __restrict__ update
                 const int d = threadIdx.x + kNormThreads * u;
                 if (d < dim) {
                     v[u] = __fadd_rn(v[u], ur[d]);
-                    xr[d] = v[u];
+                    sr[d] = v[u];
                 }
             }
         }
@@ -104,14 +105,14 @@ rms_norm_kernel(float* __restrict__ x, int ldx, const float* __restrict__ update
         float v = xr[d];
         if (ur) {
             v = __fadd_rn(v, ur[d]);
-            xr[d] = v;
+            sr[d] = v;
         }
         ss = __fadd_rn(ss, __fmul_rn(v, v));
     }
     ss = block_sum(ss, s_part);
     const float r = __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)dim), eps)));
     for (int d = threadIdx.x; d < dim; d += blockDim.x)
-        orow[d] = __fmul_rn(__fmul_rn(xr[d], r), weight[d]);
+        orow[d] = __fmul_rn(__fmul_rn(ur ? sr[d] : xr[d], r), weight[d]);
 }
 
 // Small rows (the per-head Q/K norm: 128 values): one warp per row.
@@ -1513,6 +1514,17 @@ int launch_tile(b2w4_ctx* ctx, const AttnArgs& a, int dim, const AttnPlan& plan,
 
 }  // namespace
 
+int b2w4_launch_step_norm(b2w4_ctx* ctx, const b2w4_norm_args& n, int k, float* hidden) {
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, rms_norm_kernel, dim3(1), dim3(kNormThreads), 0,
+                                       ctx->stream, n.residual, k, n.update, k, n.residual_out, k,
+                                       n.weight, n.eps, hidden, k));
+    ctx->launches++;
+    if (!n.update && n.residual_out)
+        B2W4_CUDA(ctx, cudaMemcpyAsync(n.residual_out, n.residual, sizeof(float) * k,
+                                       cudaMemcpyDeviceToDevice, ctx->stream));
+    return B2W4_OK;
+}
+
 extern "C" {
 
 int b2w4_rms_norm(b2w4_ctx* ctx, const float* x_dev, int ldx, int rows, int dim,
@@ -1530,9 +1542,9 @@ int b2w4_rms_norm(b2w4_ctx* ctx, const float* x_dev, int ldx, int rows, int dim,
     } else {
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, rms_norm_kernel, dim3(rows),
                                            dim3(kNormThreads), 0, ctx->stream,
-                                           const_cast<float*>(x_dev), ldx,
-                                           static_cast<const float*>(nullptr), 0, dim, weight_dev,
-                                           eps, out_dev, ldo));
+                                           x_dev, ldx, static_cast<const float*>(nullptr), 0,
+                                           static_cast<float*>(nullptr), dim, weight_dev, eps,
+                                           out_dev, ldo));
     }
     ctx->launches++;
     return B2W4_OK;
@@ -1547,8 +1559,8 @@ int b2w4_add_rms_norm(b2w4_ctx* ctx, float* residual_dev, int ldr, const float* 
         ldr < dim || ldu < dim || ldo < dim)
         return b2w4_fail(ctx, B2W4_E_INVALID, "add_rms_norm: bad argument");
     B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, rms_norm_kernel, dim3(rows), dim3(kNormThreads), 0,
-                                       ctx->stream, residual_dev, ldr, update_dev, ldu, dim,
-                                       weight_dev, eps, out_dev, ldo));
+                                       ctx->stream, residual_dev, ldr, update_dev, ldu,
+                                       residual_dev, dim, weight_dev, eps, out_dev, ldo));
     ctx->launches++;
     return B2W4_OK;
 }

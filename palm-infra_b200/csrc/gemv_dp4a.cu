@@ -38,11 +38,15 @@
 //
 // A decode step's neighbours of the matmul run inside it (b2w4_step_matmul), because as launches
 // of their own they cost 2 to 3 us each, all of it latency:
-//   NORM          the row is made here, x = rms_norm(residual + update): every CTA sums the
-//                 squares of the whole row (10 KB from L2) and the first one writes the new
-//                 residual, to another buffer than the one that the others still read
+//   NORM          the row (up to 4096 values) is made here, x = rms_norm(residual + update):
+//                 every CTA sums the squares of the whole row (10 KB from L2) and the first one
+//                 writes the new residual, to another buffer than the one that the others still
+//                 read.  For a launch of one wave; where CTAs follow one another on an SM the
+//                 repeated sum costs more than a launch (an lm_head of 2111 CTAs: 46 -> 65 us)
 //   kModeSwiglu   a CTA takes as many tiles of the up rows as of the gate rows, the same ones,
 //                 and stores silu(gate) * up
+#include <cooperative_groups.h>
+
 #include "b200w4_internal.cuh"
 
 namespace {
@@ -134,6 +138,27 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
     return d;
 }
 
+// Integer sum of one weight row and group: wt = the row's four 16-byte chunks (one every eight
+// uint4), qa = the group's even / odd de-interleaved codes, es = -8 * sum of the even-k codes.
+__device__ __forceinline__ int group_sum(const uint4* wt, const uint4* qa, int es) {
+    int pt = es, qt = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const uint4 w = wt[s * 8], ae = qa[s * 2], ao = qa[s * 2 + 1];
+        int p = dp4a_us((w.x ^ 0x08080808u) & 0x0F0F0F0Fu, ae.x, 0);
+        int q = __dp4a((int)(w.x & 0xF0F0F0F0u), (int)ao.x, 0);
+        p = dp4a_us((w.y ^ 0x08080808u) & 0x0F0F0F0Fu, ae.y, p);
+        q = __dp4a((int)(w.y & 0xF0F0F0F0u), (int)ao.y, q);
+        p = dp4a_us((w.z ^ 0x08080808u) & 0x0F0F0F0Fu, ae.z, p);
+        q = __dp4a((int)(w.z & 0xF0F0F0F0u), (int)ao.z, q);
+        p = dp4a_us((w.w ^ 0x08080808u) & 0x0F0F0F0Fu, ae.w, p);
+        q = __dp4a((int)(w.w & 0xF0F0F0F0u), (int)ao.w, q);
+        pt += p;
+        qt += q;
+    }
+    return pt + (qt >> 4);  // qt sums 16*q4*a: an exact multiple of 16
+}
+
 // the fused activations carry fp64 exp / tanh code: keep one out-of-line copy
 __device__ __noinline__ float gemv_activation(float v, int act) {
     return b2w4_activation(v, act);
@@ -202,6 +227,13 @@ gemv_w4a8_kernel(const GemvArgs a) {
         }
     }
 
+    float kept_w[8];  // NORM: the half-warp's weights, which do not depend on the predecessor
+    if (NORM && warp * 2 + (lane >> 4) < G) {
+        const float4* w = reinterpret_cast<const float4*>(
+            a.norm.weight + (warp * 2 + (lane >> 4)) * 128 + (lane & 15) * 8);
+        *reinterpret_cast<float4*>(kept_w) = w[0];
+        *reinterpret_cast<float4*>(kept_w + 4) = w[1];
+    }
     b2w4_pdl_wait();  // activations come from the previous kernel
 
     // Tensor-parallel exchange number: one more than the count of completed gathers, kept in
@@ -216,11 +248,6 @@ gemv_w4a8_kernel(const GemvArgs a) {
     {
         const int half = lane >> 4, h = lane & 15;
         const int n_q = a.m * G;
-        // NORM: residual + update, the row's sum of squares, then (v * r) * weight: the bits of
-        // b2w4_add_rms_norm, whose 256 threads each add every 256th square.  The half-warp's
-        // first group stays in registers; rows of more than 4096 values read the others again.
-        const float* const nr = a.norm.residual;
-        const float* const nu = a.norm.update;
         auto load8 = [](const float* p, float (&v)[8]) {
             const float4 lo = *reinterpret_cast<const float4*>(p);
             const float4 hi = *reinterpret_cast<const float4*>(p + 4);
@@ -231,51 +258,44 @@ gemv_w4a8_kernel(const GemvArgs a) {
             *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
             *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
         };
-        auto residual8 = [&](int at, float (&v)[8]) {
-            load8(nr + at, v);
-            if (nu) {
-                float u[8];
-                load8(nu + at, u);
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    v[i] = __fadd_rn(v[i], u[i]);
-            }
-        };
-        float kept[8], kept_w[8], rms = 0.f;
+        // NORM: residual + update, the row's sum of squares, then (v * r) * weight: the bits of
+        // b2w4_add_rms_norm, whose 256 threads each add every 256th square.  A half-warp's one
+        // group stays in registers; the squares are taken from a copy in shared memory.
+        float kept[8], rms = 0.f;
         if (NORM) {
             __shared__ float s_ss[8];
-            float ss = 0.f;
-            if (threadIdx.x < 256) {
-#pragma unroll 5
-                for (int d = threadIdx.x; d < K; d += 256) {
-                    const float v = nu ? __fadd_rn(nr[d], nu[d]) : nr[d];
-                    ss = __fadd_rn(ss, __fmul_rn(v, v));
-                }
-            }
-#pragma unroll 1
-            for (int g = warp * 2 + half; g < G; g += kWarps * 2) {
-                const int at = g * 128 + h * 8;
-                const bool keep = g < kWarps * 2;
-                if (!keep && (blockIdx.x != 0 || !a.norm.residual_out))
-                    break;
-                float v[8];
-                residual8(at, v);
-                if (keep) {
-                    load8(a.norm.weight + at, kept_w);
+            float* s_row = reinterpret_cast<float*>(
+                (reinterpret_cast<uintptr_t>(s_bar + a.tpc + 1) + 15) & ~uintptr_t(15));
+            const int g = warp * 2 + half, at = g * 128 + h * 8;
+            if (g < G) {
+                load8(a.norm.residual + at, kept);
+                if (a.norm.update) {
+                    float u[8];
+                    load8(a.norm.update + at, u);
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        kept[i] = v[i];
+                        kept[i] = __fadd_rn(kept[i], u[i]);
                 }
+                store8(s_row + at, kept);
                 if (blockIdx.x == 0 && a.norm.residual_out)
-                    store8(a.norm.residual_out + at, v);
+                    store8(a.norm.residual_out + at, kept);
             }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-                ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, off));
-            if (lane == 0 && warp < 8)
-                s_ss[warp] = ss;
             __syncthreads();
-            ss = 0.f;
+            if (warp < 8) {
+                float ss = 0.f;
+#pragma unroll 10
+                for (int d = threadIdx.x; d < K; d += 256) {
+                    const float v = s_row[d];
+                    ss = __fadd_rn(ss, __fmul_rn(v, v));
+                }
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1)
+                    ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, off));
+                if (lane == 0)
+                    s_ss[warp] = ss;
+            }
+            __syncthreads();
+            float ss = 0.f;
 #pragma unroll
             for (int w = 0; w < 8; ++w)
                 ss = __fadd_rn(ss, s_ss[w]);
@@ -291,17 +311,12 @@ gemv_w4a8_kernel(const GemvArgs a) {
             const int mi = live ? item / G : 0, g = live ? item % G : 0;
             const float* src = a.x + (size_t)mi * a.lda + (size_t)g * 128 + h * 8;
             float v[8];
-            if (NORM) {
-                const int at = g * 128 + h * 8;
-                if (base >= kWarps * 2 && live) {
-                    residual8(at, kept);
-                    load8(a.norm.weight + at, kept_w);
-                }
+            if (NORM) {  // one pass: this half-warp's group
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     v[i] = live ? __fmul_rn(__fmul_rn(kept[i], rms), kept_w[i]) : 0.f;
                 if (blockIdx.x == 0 && a.norm.hidden_out && live)
-                    store8(a.norm.hidden_out + at, v);
+                    store8(a.norm.hidden_out + g * 128 + h * 8, v);
             } else if (live && vec_x) {  // two 16-byte loads instead of eight scalar ones
                 load8(src, v);
             } else {
@@ -484,6 +499,153 @@ gemv_w4a8_kernel(const GemvArgs a) {
     }
 }
 
+// ---- long rows: the groups split over a cluster ----------------------------------------------
+// A cluster of kSplit CTAs takes `tpc` tiles; CTA r quantises and multiplies groups [r * per,
+// (r + 1) * per) of all of them and stores each (integer sum, scale product) into the shared
+// memory of the CTA that owns the tile (tile % kSplit), which after one cluster barrier runs the
+// tiles' chains over all groups in ascending order: the kernel above, its bits, with a quarter
+// of the row per CTA.  What that mends where rows are long: a CTA of the kernel above holds whole
+// tiles, so a weight of few long rows leaves SMs with one or two of them (an [2560, 9728] weight:
+// 160 CTAs of two tiles, 12 SMs with two such CTAs), and every CTA quantises the whole row.
+constexpr int kSplit = 4;
+constexpr int kSplitMaxTiles = 16;
+template <bool SCL16>
+__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(512, 2)
+gemv_w4a8_split_kernel(const GemvArgs a) {
+    constexpr int kWarps = 16, kScl = SCL16 ? 16 : 32;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int G = a.groups, per = (G + kSplit - 1) / kSplit;
+    const int rank = blockIdx.x % kSplit, tile0 = blockIdx.x / kSplit * a.tpc;
+    const int ntile = min(a.tpc, a.tiles - tile0);
+    const int g0 = min(G, rank * per), n_g = min(per, G - g0);
+    const int owned = (a.tpc + kSplit - 1) / kSplit;
+    uint8_t* s_w = smem;                                                 // [tpc][per][512]
+    uint8_t* s_scl = s_w + (size_t)a.tpc * per * 512;                    // [tpc][per][8]
+    uint4* s_qa = reinterpret_cast<uint4*>(s_scl + (size_t)a.tpc * per * kScl);  // [per][128]
+    float* s_as = reinterpret_cast<float*>(s_qa + per * 8);              // [per]
+    int* s_es = reinterpret_cast<int*>(s_as + per);                      // [per]
+    float* s_d = reinterpret_cast<float*>(s_es + per);                   // [owned][d_stride]
+    float* s_sc = s_d + (size_t)owned * a.d_stride;
+    __shared__ uint64_t s_bar[kSplitMaxTiles];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    b2w4_pdl_launch_dependents();
+    if (warp == 0) {  // lane t: tile t's share
+        if (lane < ntile)
+            mbar_init(&s_bar[lane], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncwarp();
+        if (lane < ntile && n_g > 0) {
+            const size_t at = (size_t)(tile0 + lane) * G + g0;
+            mbar_expect_tx(&s_bar[lane], (uint32_t)n_g * (512 + kScl));
+            bulk_g2s(s_w + (size_t)lane * per * 512,
+                     reinterpret_cast<const uint8_t*>(a.nib) + at * 512, (uint32_t)n_g * 512,
+                     &s_bar[lane]);
+            bulk_g2s(s_scl + (size_t)lane * per * kScl,
+                     reinterpret_cast<const uint8_t*>(a.scl) + at * kScl, (uint32_t)n_g * kScl,
+                     &s_bar[lane]);
+        }
+    }
+    b2w4_pdl_wait();  // activations come from the previous kernel
+    // quantiser, as above: a half-warp per group
+    {
+        const int half = lane >> 4, h = lane & 15;
+        const bool vec_x = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0;
+#pragma unroll 1
+        for (int base = warp * 2; base < n_g; base += kWarps * 2) {
+            const int g = base + half;
+            const bool live = g < n_g;
+            const float* src = a.x + (size_t)(g0 + (live ? g : 0)) * 128 + h * 8;
+            float v[8];
+            if (live && vec_x) {
+                const float4 lo = *reinterpret_cast<const float4*>(src);
+                const float4 hi = *reinterpret_cast<const float4*>(src + 4);
+                v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+                v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    v[i] = live ? src[i] : 0.f;
+            }
+            float amax = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1)
+                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+            float scale, inv;
+            b2w4_quant_params(amax, scale, inv);
+            int c[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                c[i] = b2w4_quant_code(v[i], inv);
+            int esum = c[0] + c[2] + c[4] + c[6];
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1)
+                esum += __shfl_xor_sync(0xffffffffu, esum, off);
+            if (!live)
+                continue;
+            if (h == 0) {
+                s_as[g] = scale;
+                s_es[g] = -8 * esum;
+            }
+            uint8_t* blk = reinterpret_cast<uint8_t*>(s_qa) + (size_t)g * 128 + (h >> 2) * 32;
+            const int j = (h & 3) * 4;
+            *reinterpret_cast<char4*>(blk + j) = make_char4(
+                (signed char)c[0], (signed char)c[2], (signed char)c[4], (signed char)c[6]);
+            *reinterpret_cast<char4*>(blk + 16 + j) = make_char4(
+                (signed char)c[1], (signed char)c[3], (signed char)c[5], (signed char)c[7]);
+        }
+    }
+    // every CTA of the cluster runs before its shared memory is written from another one
+    cluster.sync();
+
+    // integer sums: an item is four consecutive groups of one tile
+    const int gl = lane >> 3, row = lane & 7, ipt = (n_g + 3) >> 2;
+    bool timed_out = false;
+#pragma unroll 1
+    for (int it = warp; it < ntile * ipt && !timed_out; it += kWarps) {
+        const int tl = it / ipt, g = (it - tl * ipt) * 4 + gl;
+        if (!mbar_wait_bounded(&s_bar[tl])) {
+            timed_out = true;
+            break;
+        }
+        if (g < n_g) {
+            const int at = tl * per + g;
+            const int d = group_sum(reinterpret_cast<const uint4*>(s_w) + at * 32 + row,
+                                    s_qa + g * 8, s_es[g]);
+            const float ws = SCL16 ? __half2float(reinterpret_cast<const __half*>(s_scl)[at * 8 + row])
+                                   : reinterpret_cast<const float*>(s_scl)[at * 8 + row];
+            const int slot = (tl / kSplit) * a.d_stride + (g0 + g) * 8 + row, owner = tl % kSplit;
+            cluster.map_shared_rank(s_d, owner)[slot] = (float)d;
+            cluster.map_shared_rank(s_sc, owner)[slot] = __fmul_rn(ws, s_as[g]);
+        }
+    }
+    if (timed_out && lane == 0)
+        b2w4_report_timeout(a.status);
+    cluster.sync();
+
+    // the owned tiles' chains: tiles rank, rank + kSplit, ...
+    for (int t = threadIdx.x; t < owned * 8; t += kWarps * 32) {
+        const int rr = t & 7, to = t >> 3, tl = to * kSplit + rank;
+        const int n = (tile0 + tl) * 8 + rr;
+        if (tl >= ntile || n >= a.n)
+            continue;
+        const float* dsrc = s_d + (size_t)to * a.d_stride + rr;
+        const float* csrc = s_sc + (size_t)to * a.d_stride + rr;
+        float acc = 0.f;
+#pragma unroll 10
+        for (int j = 0; j < G; ++j)
+            acc = __fmaf_rn(dsrc[j * 8], csrc[j * 8], acc);
+        if (b2w4_act_applies(n, a.activation, a.act_n_begin, a.act_n_len, a.n))
+            acc = gemv_activation(acc, a.activation);
+        a.y[n] = acc;
+    }
+}
+
 // Second half of the tensor-parallel exchange: waits (bounded) until every entry of the
 // current exchange's half of the staging buffer carries the exchange number -- written by this
 // GPU's own matmul (complete: this kernel is ordered after it) and by the peers' -- and unpacks
@@ -635,16 +797,31 @@ int launch_one(b2w4_ctx* ctx, const GemvArgs& a, size_t smem) {
     return B2W4_OK;
 }
 
+size_t gemv_split_bytes(int per, int tpc, int d_stride, bool scl16) {
+    return (size_t)tpc * per * (512 + (scl16 ? 16 : 32)) + (size_t)per * (128 + 8) +
+           2 * sizeof(float) * ((tpc + kSplit - 1) / kSplit) * d_stride;
+}
+int launch_split(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, size_t smem) {
+    auto kern = scl16 ? gemv_w4a8_split_kernel<true> : gemv_w4a8_split_kernel<false>;
+    static b2w4_smem_optin configured[2];  // per instantiation and device
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[scl16]));
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern,
+                                       dim3((a.tiles + a.tpc - 1) / a.tpc * kSplit), dim3(512),
+                                       smem, ctx->stream, a));
+    ctx->launches++;
+    return B2W4_OK;
+}
+
 template <int MT>
 int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, size_t smem) {
     const int mode = a.sums ? kModeSums : (a.top1.cells ? kModeTop1 : kModePlain);
     if (a.swiglu || a.norm.weight) {  // a decode step: one row, per-128 rule
-        if (a.swiglu)
+        if (a.swiglu && a.norm.weight)
             return scl16 ? launch_one<MT, true, false, kModeSwiglu, true>(ctx, a, smem)
                          : launch_one<MT, false, false, kModeSwiglu, true>(ctx, a, smem);
-        if (a.top1.cells)
-            return scl16 ? launch_one<MT, true, false, kModeTop1, true>(ctx, a, smem)
-                         : launch_one<MT, false, false, kModeTop1, true>(ctx, a, smem);
+        if (a.swiglu)
+            return scl16 ? launch_one<MT, true, false, kModeSwiglu>(ctx, a, smem)
+                         : launch_one<MT, false, false, kModeSwiglu>(ctx, a, smem);
         return scl16 ? launch_one<MT, true, false, kModePlain, true>(ctx, a, smem)
                      : launch_one<MT, false, false, kModePlain, true>(ctx, a, smem);
     }
@@ -714,7 +891,8 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
         // CTAs 8.65.
         const int per_tile = w->groups * (512 + (scl16 ? 16 : 32)) +
                              8 * gemv_d_stride(mt, w->groups, a32);
-        const int budget = 113 * 1024 - mt * w->k - 8 * mt * w->groups * spg - 1024;
+        const int budget = 113 * 1024 - mt * w->k - 8 * mt * w->groups * spg - 1024 -
+                           (norm ? 4 * w->k + 16 : 0);
         int tpc = max(1, min(budget / per_tile, kMaxTpc));
         const int wave_ctas = ctx->sm_count * 7 / 4;
         const int one_wave = (w->tiles + wave_ctas - 1) / wave_ctas;
@@ -734,7 +912,21 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
                     a.ipt_magic = 0;
         }
         a.d_stride = gemv_d_stride(mt, w->groups, a32);
-        const size_t smem = gemv_smem_bytes(mt, w->k, w->groups, tpc, scl16, a32);
+        // long rows, split over clusters
+        if (!a32 && !sums && !tp && !top1 && !norm && !swiglu && ctx->gemv_tpc_override == 0 &&
+            w->groups >= 48 && tpc <= 4) {
+            const int per = (w->groups + kSplit - 1) / kSplit;
+            // clusters in one wave of at most 1.75 CTAs per SM, two CTAs' memory per SM
+            const int clusters = wave_ctas / kSplit;
+            a.tpc = min(kSplitMaxTiles, (w->tiles + clusters - 1) / clusters);
+            const size_t bytes = gemv_split_bytes(per, a.tpc, a.d_stride, scl16);
+            if (bytes <= 113 * 1024)
+                return launch_split(ctx, a, scl16, bytes);
+            a.tpc = tpc;
+        }
+        size_t smem = gemv_smem_bytes(mt, w->k, w->groups, tpc, scl16, a32);
+        if (norm)  // the row's copy, 16-byte aligned behind the barriers
+            smem += sizeof(float) * w->k + 16;
         if (smem > 220 * 1024)
             return b2w4_fail(ctx, B2W4_E_INVALID, "gemv: K=%d needs %zu B shared memory",
                              w->k, smem);

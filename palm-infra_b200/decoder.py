@@ -121,9 +121,9 @@ class DenseDecoder:
         self.multi_row_rule = multi_row_rule
         can_fuse = cfg.head_dim % 64 == 0 and cfg.head_dim <= 256
         self.fused_qkv = can_fuse if fused_qkv is None else (fused_qkv and can_fuse)
-        # norms and SwiGLU made by the matmuls' quantisers (contexts without these entries run
-        # operator by operator)
-        self.fused_rows = self.fused_qkv and hasattr(ctx, "matmul_norm")
+        # norms, SwiGLU and a step's cache append inside the matmuls and attention (contexts
+        # without these entries run operator by operator)
+        self.fused_step = self.fused_qkv and hasattr(ctx, "step_matmul")
         sh = weights["shapes"]
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
         self.layers = []
@@ -162,6 +162,8 @@ class DenseDecoder:
         comes from self.past_dev inside the kernels (the form a CUDA graph can replay)."""
         c, cfg, ctx = self.ctx, self.cfg, self.ctx
         T, H, D = tokens, cfg.hidden, cfg.head_dim
+        if T == 1 and self.fused_step:
+            return self._forward_step(ids_dev, on_device_position)
         rule = capi.ACT_G128 if T == 1 else self.multi_row_rule
         pos_dev = self.past_dev if on_device_position else None
         x = self._b("x", T, H)
@@ -173,7 +175,7 @@ class DenseDecoder:
         if not cfg.experts:
             gu, act = self._b("gu", T, 2 * cfg.intermediate), self._b("act", T, cfg.intermediate)
         dn = self._b("dn", T, H)
-        fused = T > 1 and self.fused_rows
+        fused = self.fused_step  # norms and SwiGLU made by the matmuls' quantisers
         c.embed_rows(self.embed, ids_dev, x)
         if not fused:
             c.rms_norm(x, self.layers[0]["ln1"], cfg.eps, h)
@@ -221,6 +223,44 @@ class DenseDecoder:
         c.matmul_argmax(self.lm_head, h[T - 1:T], self.token)
         if not on_device_position:
             self.past += T
+
+    def _forward_step(self, ids_dev, on_device_position):
+        """forward() of one token, five launches per layer."""
+        c, cfg = self.ctx, self.cfg
+        H, D, inter = cfg.hidden, cfg.head_dim, cfg.intermediate
+        pos_dev = self.past_dev if on_device_position else None
+        # the residual stream moves between two buffers: a matmul's blocks read the old one
+        # while the first of them writes the new one
+        x, x_new = self._b("x", 1, H), self._b("x_new", 1, H)
+        h, o, dn = self._b("h", 1, H), self._b("o", 1, H), self._b("dn", 1, H)
+        qkv = self._b("qkv", 1, cfg.q_dim + 2 * cfg.kv_dim)
+        q, attn = self._b("q", 1, cfg.q_dim), self._b("attn", 1, cfg.q_dim)
+        act = None if cfg.experts else self._b("act", 1, inter)
+        c.embed_rows(self.embed, ids_dev, x)
+        update = None
+        for L in self.layers:
+            c.step_matmul(L["qkv"], x, update, L["ln1"], cfg.eps,
+                          None if update is None else x_new, y=qkv)
+            if update is not None:
+                x, x_new = x_new, x
+            c.attention_step(qkv, cfg.heads, cfg.kv_heads, D, L["q_norm"], L["k_norm"], cfg.eps,
+                             self.cos, self.sin, self.past, q, L["k_cache"], L["v_cache"], attn,
+                             self.capacity, D ** -0.5, pos_dev)
+            c.matmul(L["o"], attn, o, rule=capi.ACT_G128)
+            if cfg.experts:
+                c.add_rms_norm(x, o, L["ln2"], cfg.eps, h)
+                c.moe_forward(h, L["router"], cfg.top_k, inter, L["gate_up"], L["down"], dn)
+            else:
+                c.step_matmul(L["gate_up"], x, o, L["ln2"], cfg.eps, x_new, y=act, swiglu=True)
+                x, x_new = x_new, x
+                c.matmul(L["down"], act, dn, rule=capi.ACT_G128)
+            update = dn
+        if on_device_position:
+            c.advance(self.past_dev, 1, ids_dev, self.history)
+        c.step_matmul(self.lm_head, x, update, self.final_norm, cfg.eps, x_new,
+                      tokens=self.token, hidden_out=h)
+        if not on_device_position:
+            self.past += 1
 
     def prefill(self, ids):
         ids_dev = self.torch.from_numpy(np.asarray(ids, dtype=np.int32)).to(self.device)

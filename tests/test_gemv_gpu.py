@@ -465,3 +465,33 @@ def test_matmul_argmax_bad_arguments(ctx):
         ctx.matmul_argmax(w, torch.zeros((1, 128), device="cuda"), tok,
                           torch.zeros((1, 32), device="cuda"))           # logits row too short
     w.free()
+
+
+@pytest.mark.parametrize("n,k,f32", [(8, 6144, False), (2560, 9728, False), (1003, 6272, True),
+                                     (40, 12160, False), (2072, 6144, True)])
+def test_long_rows_split_over_a_cluster(ctx, n, k, f32):
+    """One row against long weight rows, whose groups a cluster shares: group counts that four
+    divides and does not, ragged last tiles and clusters, fp32 scales, a fused activation; the
+    oracle's bits."""
+    blocks = pkg.synth.bg128_weight(20261125, n + k, n, k)
+    if f32:  # scales that fp16 cannot hold
+        blocks = np.array(blocks, copy=True)
+        s = blocks.reshape(-1, 544)[:, :32].copy().view(np.float32)
+        blocks.reshape(-1, 544)[:, :32] = (s * np.float32(1.0000001) + np.float32(1e-9) *
+                                           (s != 0)).astype(np.float32).view(np.uint8)
+    x = pkg.synth.activations(7, n, 1, k)
+    x[0, 128:256] = 0.0  # a group of zeros
+    y, _ = run_gpu(ctx, blocks, n, k, x, sums=False)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x).tobytes()
+
+
+@pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
+@pytest.mark.parametrize("m,n,k", [(2, 16392, 256), (3, 4104, 512), (8, 6152, 640), (5, 1608, 384),
+                                   (2, 1608, 6272), (7, 1603, 6144)])
+def test_two_to_eight_rows_on_the_streamed_kernel(ctx, m, n, k, rule):
+    """Row counts and weights on which few rows take the kernel of 9 to 32 rows: a warp per pair,
+    up to ten pairs per CTA."""
+    blocks = pkg.synth.bg128_weight(20261125, n + k + m + 5, n, k)
+    x = pkg.synth.activations(7, m + 17, m, k)
+    y, _ = run_gpu(ctx, blocks, n, k, x, rule=rule, sums=False, pad=4 if n % 16 else 0)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=rule).tobytes()
