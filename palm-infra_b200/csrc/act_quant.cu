@@ -40,11 +40,6 @@ __global__ void quantize_rows_kernel(const float* __restrict__ x, int lda, int m
         char4 packed = make_char4((signed char)c0, (signed char)c1, (signed char)c2,
                                   (signed char)c3);
         *reinterpret_cast<char4*>(dst + lane * 4) = packed;
-    } else if (LAYOUT == QLAYOUT_MMA) {
-        // the lane holds k = 4*lane..+3: 32-block lane/8, even-k indices 2*(lane%8) and +1
-        int8_t* blk = dst + ((lane & 7) >> 1) * 32 + (lane >> 3) * 4 + (lane & 1) * 2;
-        *reinterpret_cast<char2*>(blk) = make_char2((signed char)c0, (signed char)c2);
-        *reinterpret_cast<char2*>(blk + 16) = make_char2((signed char)c1, (signed char)c3);
     } else {
         // 32-block `sub` = lane/8 stored as 16 even-k codes then 16 odd-k codes
         int8_t* blk = dst + (lane >> 3) * 32;
@@ -63,19 +58,21 @@ __global__ void quantize_rows_kernel(const float* __restrict__ x, int lda, int m
 //          MMA's shared-memory descriptor expects, so the plane can be bulk-copied into shared
 //          memory as is.  Scales: fp32 [groups][m_pad]; with one scale per 32 values (A32)
 //          [groups][m_pad][4], a row's four block scales side by side
-//   MMA    the mma.sync GEMM: codes int8 [m][K] in tensor-operand order (QLAYOUT_MMA), scales and
+//   MMA    the mma.sync GEMM: codes int8 [m][K] in tensor-operand order (inside a 128-group
+//          [word position p 0..3][32 bytes]: the even-k codes 4p..4p+3 of the four 32-blocks, then
+//          the odd ones, so that the B words of a lane of m16n8k32 are contiguous), scales and
 //          the accumulator bias 0x4B400000 - 8 * (sum of the group's codes) transposed to
 //          [groups][m_pad] (A32: [groups*4][m_pad], one entry per 32-block) so that one group of
 //          all rows is contiguous.  (The kernel multiplies unsigned nibbles q+8; starting its
 //          int32 accumulator at the bias makes it end as 0x4B400000 + D, the bit pattern of the
 //          float 12582912 + D.)
-//   QUADS  the same with a row pair's biases as the four words of the accumulator, (b[2p],
-//          b[2p+1]) twice
-enum { OUT_UMMA, OUT_MMA, OUT_QUADS };
+//   ROWS   the kernel for a few rows: codes as MMA, scales [groups][m_pad] (A32: [groups]
+//          [m_pad / 2][4][2], a row pair's block scales side by side), no biases
+enum { OUT_UMMA, OUT_MMA, OUT_ROWS };
 struct QuantOut {
     int8_t* q;
     float* scales;
-    int32_t* es;  // MMA, QUADS
+    int32_t* es;  // MMA
     int k, m_pad;
 };
 
@@ -106,20 +103,19 @@ __device__ __forceinline__ void quantize_group(const QuantOut& o, int row, int g
         *reinterpret_cast<char2*>(rowp + (((2 * sub + 1) ^ sw) << 4) + j) = odd;
         return;
     }
-    int esum = c0 + c1 + c2 + c3;  // integer: order-free
+    if (OUT == OUT_MMA) {
+        int esum = c0 + c1 + c2 + c3;  // integer: order-free
 #pragma unroll
-    for (int off = A32 ? 4 : 16; off > 0; off >>= 1)
-        esum += __shfl_xor_sync(0xffffffffu, esum, off);
-    if (first) {
-        const size_t run = (size_t)(A32 ? g * 4 + sub : g) * o.m_pad;
-        const int bias = 0x4B400000 - 8 * esum;
-        o.scales[run + row] = scale;
-        if (OUT == OUT_QUADS) {
-            int32_t* quad = o.es + 2 * run + (row >> 1) * 4 + (row & 1);
-            quad[0] = quad[2] = bias;
-        } else {
-            o.es[run + row] = bias;
+        for (int off = A32 ? 4 : 16; off > 0; off >>= 1)
+            esum += __shfl_xor_sync(0xffffffffu, esum, off);
+        if (first) {
+            const size_t at = (size_t)(A32 ? g * 4 + sub : g) * o.m_pad + row;
+            o.scales[at] = scale;
+            o.es[at] = 0x4B400000 - 8 * esum;
         }
+    } else if (first) {
+        o.scales[A32 ? (size_t)g * 4 * o.m_pad + (row >> 1) * 8 + sub * 2 + (row & 1)
+                     : (size_t)g * o.m_pad + row] = scale;
     }
     // the lane's codes: even-k indices 2*(lane%8) and +1 of its 32-block, and the odd ones
     int8_t* blk = o.q + (size_t)row * o.k + (size_t)g * 128 + ((lane & 7) >> 1) * 32 + sub * 4 +
@@ -240,17 +236,24 @@ cudaError_t launch_quantize_many(b2w4_ctx* ctx, const float* x, int lda, int m, 
 }  // namespace
 
 int b2w4_launch_quantize_mma(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
-                             int act_rule, int8_t* q, float* scales_t, int32_t* es_t, bool quads,
-                             const b2w4_rows* from) {
-    if (!quads && ((reinterpret_cast<uintptr_t>(x) & 15) || (lda & 3)))
+                             int act_rule, int8_t* q, float* scales_t, int32_t* es_t) {
+    if ((reinterpret_cast<uintptr_t>(x) & 15) || (lda & 3))
         return b2w4_fail(ctx, B2W4_E_INVALID, "quantize: rows must be 16-byte aligned");
     const QuantOut o = {q, scales_t, es_t, k, m_pad};
-    const bool a32 = act_rule == B2W4_ACT_G32;
-    const cudaError_t e =
-        quads ? (a32 ? launch_quantize_many<OUT_QUADS, true>(ctx, x, lda, m, o, from)
-                     : launch_quantize_many<OUT_QUADS, false>(ctx, x, lda, m, o, from))
-              : (a32 ? launch_quantize_many<OUT_MMA, true>(ctx, x, lda, m, o, from)
-                     : launch_quantize_many<OUT_MMA, false>(ctx, x, lda, m, o, from));
+    const cudaError_t e = act_rule == B2W4_ACT_G32
+                              ? launch_quantize_many<OUT_MMA, true>(ctx, x, lda, m, o, nullptr)
+                              : launch_quantize_many<OUT_MMA, false>(ctx, x, lda, m, o, nullptr);
+    B2W4_CUDA(ctx, e);
+    ctx->launches++;
+    return B2W4_OK;
+}
+
+int b2w4_launch_quantize_rows(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
+                              int act_rule, int8_t* q, float* scales, const b2w4_rows* from) {
+    const QuantOut o = {q, scales, nullptr, k, m_pad};
+    const cudaError_t e = act_rule == B2W4_ACT_G32
+                              ? launch_quantize_many<OUT_ROWS, true>(ctx, x, lda, m, o, from)
+                              : launch_quantize_many<OUT_ROWS, false>(ctx, x, lda, m, o, from);
     B2W4_CUDA(ctx, e);
     ctx->launches++;
     return B2W4_OK;
@@ -281,14 +284,10 @@ int b2w4_launch_quantize(b2w4_ctx* ctx, const float* x, int lda, int m, int k,
                                        dim3(256), 0, ctx->stream, x, lda, m, k, q, scales))
     if (act_rule == 128 && layout == QLAYOUT_NATURAL)
         LAUNCH(128, QLAYOUT_NATURAL);
-    else if (act_rule == 128 && layout == QLAYOUT_MMA)
-        LAUNCH(128, QLAYOUT_MMA);
     else if (act_rule == 128)
         LAUNCH(128, QLAYOUT_EVEN_ODD);
     else if (layout == QLAYOUT_NATURAL)
         LAUNCH(32, QLAYOUT_NATURAL);
-    else if (layout == QLAYOUT_MMA)
-        LAUNCH(32, QLAYOUT_MMA);
     else
         LAUNCH(32, QLAYOUT_EVEN_ODD);
 #undef LAUNCH

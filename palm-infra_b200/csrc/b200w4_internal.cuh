@@ -125,10 +125,10 @@ int b2w4_launch_gemm_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, in
 int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
                           int ldc, int m, int act_rule, int activation, int act_n_begin,
                           int act_n_len, const b2w4_rows* from = nullptr);
-// quads: es_t holds every bias twice, (b[2p], b[2p+1], b[2p], b[2p+1]) for the row pair p
 int b2w4_launch_quantize_mma(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
-                             int act_rule, int8_t* q, float* scales_t, int32_t* es_t,
-                             bool quads = false, const b2w4_rows* from = nullptr);
+                             int act_rule, int8_t* q, float* scales_t, int32_t* es_t);
+int b2w4_launch_quantize_rows(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
+                              int act_rule, int8_t* q, float* scales, const b2w4_rows* from);
 // Tensor-parallel epilogue of the one-row GEMV: the kernel stores its rows into every rank's
 // copy of the output and the launch's last CTA bumps this rank's arrival counter on every
 // rank.  world == 0: off.
@@ -242,10 +242,6 @@ int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
 enum {
     QLAYOUT_NATURAL = 0,  // int8 [M][K], k ascending
     QLAYOUT_EVEN_ODD = 1, // int8 [M][K], each 32-block stored as even16|odd16
-    // int8 [M][K]; inside each 128-group: [word position p 0..3][32 bytes], the 32 bytes
-    // being the even-k codes 4p..4p+3 of the four 32-blocks (16 bytes) then the odd-k ones:
-    // the B-operand words of one lane of the m16n8k32 tensor instruction, contiguous
-    QLAYOUT_MMA = 2,
 };
 
 // ---------------------------------------------------------------------------

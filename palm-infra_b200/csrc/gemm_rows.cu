@@ -8,20 +8,20 @@
 // thread for the whole K loop.
 //
 // Work split.  A warp owns a pair of 8-row weight tiles (the sixteen rows of the instruction) and
-// one or two blocks of eight activation rows (its columns); with more than eight rows two warps
+// all blocks of eight activation rows (its columns), or, where there are few pairs, several warps
 // share a pair; a CTA holds up to ten warps, so that one or two CTAs per SM take the whole weight
-// in one round.  Weights,
-// codes, scales and accumulator biases stream through a ring of shared-memory stages of four
+// in one round.  Weights, codes and scales stream through a ring of shared-memory stages of four
 // groups, one barrier per stage; the weights of the first stages are on their way before the
 // kernel waits for the quantiser in front (programmatic dependent launch).  (Fetched into
 // registers four groups ahead instead, the weights came no sooner: a warp's outstanding loads
 // share six scoreboards, so a wait for an old group waited for the newest too; 16 rows,
 // [9728, 2560], 23.5 us.)
-// A weight word is split into unsigned bytes q+8 (lo = (w ^ 0x08080808) & 0x0F0F0F0F: even k;
-// hi = ((w >> 4) ^ 0x08080808) & 0x0F0F0F0F: odd k).  The accumulator starts at
-// 0x4B400000 - 8*sum(codes), stored by the quantiser as the four words that the instruction takes,
-// and ends as the bit pattern of the float 12582912 + D (|D| < 2^22): D costs one subtraction,
-// for two columns at once.
+// A weight word is split into signed bytes 16 q (lo = (w << 4) & 0xF0F0F0F0: even k; hi = w &
+// 0xF0F0F0F0: odd k).  Every accumulator starts at 0x49400000, the bits of the float 786432 whose
+// last place is worth 1/16, and ends as the bits of 786432 + D, exactly, since
+// |16 D| <= 128 * 127 * 128 < 2^22: D costs one subtraction, for two columns at once.  (Unsigned
+// bytes q + 8 need a start that depends on the sum of the codes, four more words per instruction
+// to make, copy and read: 16 rows, [9728, 2560], per 32 values, 11.1 -> 9.6 us.)
 #include "b200w4_internal.cuh"
 
 namespace {
@@ -35,8 +35,7 @@ struct GemmRowsArgs {
     const uint8_t* nib;
     const void* scl;
     const int8_t* qa;    // [m][K] int8, tensor-operand order inside each group
-    const float* as_t;   // [G * spg][m8] activation scales
-    const int4* es_t;    // [G * spg][m8 / 2] accumulator biases of a row pair, twice
+    const float* as_t;   // activation scales [G][m8], per 32 values [G][m8 / 2][4 blocks][2 rows]
     float* y;
     int ldc, m, m8, n, k, groups, tiles, pairs;
     int activation, act_n_begin, act_n_len;
@@ -52,7 +51,7 @@ __device__ __forceinline__ void rows_cp_async16(void* dst, const void* src) {
 // b0 k 4*tid..+3 of column gid, b1 k+16; d0/d1 row gid, columns 2*tid, 2*tid+1; d2/d3 row gid+8
 __device__ __forceinline__ void rows_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                          uint32_t a3, uint32_t b0, uint32_t b1, int4 c) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
         "{%8,%9}, {%10,%11,%12,%13};"
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c.x), "r"(c.y), "r"(c.z),
@@ -62,7 +61,7 @@ __device__ __forceinline__ void rows_mma(int (&d)[4], uint32_t a0, uint32_t a1, 
 __device__ __noinline__ float rows_activation(float v, int act) { return b2w4_activation(v, act); }
 
 __host__ __device__ constexpr size_t rows_stage_bytes(int m8, int spg, int pairs, bool scl16) {
-    return (size_t)m8 * (kPitch + kChunk * spg * 12) +
+    return (size_t)m8 * (kPitch + kChunk * spg * 4) +
            (size_t)pairs * 2 * kChunk * (512 + (scl16 ? 16 : 32));
 }
 
@@ -70,13 +69,13 @@ __host__ __device__ constexpr size_t rows_stage_bytes(int m8, int spg, int pairs
 template <int PW, int CB, bool SCL16, bool A32, int S>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
-    constexpr int SPG = A32 ? 4 : 1;  // scales / biases per group
+    constexpr int SPG = A32 ? 4 : 1;  // scales per group
     constexpr int kScl = SCL16 ? 16 : 32;  // bytes of a tile's scales of a group
     extern __shared__ __align__(128) uint8_t smem[];
     const int G = a.groups, m8 = a.m8;
     const int warps = blockDim.x / 32, pairs = warps / PW;
-    const int bias_bytes = kChunk * SPG * m8 * 8, as_bytes = kChunk * SPG * m8 * 4;
-    const int nib_off = bias_bytes + as_bytes + m8 * kPitch;
+    const int as_bytes = kChunk * SPG * m8 * 4;
+    const int nib_off = as_bytes + m8 * kPitch;
     const int scl_off = nib_off + pairs * 2 * kChunk * 512;
     const int stage_bytes = (int)rows_stage_bytes(m8, SPG, pairs, SCL16);
 
@@ -84,7 +83,7 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
     const int gid = lane >> 2, tid = lane & 3;
     const int pair0 = blockIdx.x * pairs, pair = pair0 + warp / PW;
     const int cb0 = (warp % PW) * CB;  // first column block
-    const int ncb = min(CB, m8 / 8 - cb0);     // may be none
+    const int ncb = PW == 1 ? CB : min(CB, m8 / 8 - cb0);  // may be none
     const bool busy = pair < a.pairs && ncb > 0;
     const int t0 = 2 * pair;
     const bool two = t0 + 1 < a.tiles;
@@ -118,14 +117,11 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
         if (c < chunks) {
             uint8_t* s = smem + (c % S) * stage_bytes;
             const int g0 = c * kChunk, gc = min(kChunk, G - g0);
-            const int n_bias = gc * SPG * m8 / 2, n_as = gc * SPG * m8 / 4, n_row = gc * 8;
-            const int4* es = a.es_t + (size_t)g0 * SPG * (m8 / 2);
+            const int n_as = gc * SPG * m8 / 4, n_row = gc * 8;
             const float* as = a.as_t + (size_t)g0 * SPG * m8;
-            for (int i = threadIdx.x; i < n_bias; i += blockDim.x)
-                rows_cp_async16(s + i * 16, es + i);
             for (int i = threadIdx.x; i < n_as; i += blockDim.x)
-                rows_cp_async16(s + bias_bytes + i * 16, as + i * 4);
-            uint8_t* rows = s + bias_bytes + as_bytes;
+                rows_cp_async16(s + i * 16, as + i * 4);
+            uint8_t* rows = s + as_bytes;
             for (int t = warp; t < a.m; t += warps)
                 if (lane < n_row)
                     rows_cp_async16(rows + t * kPitch + lane * 16,
@@ -141,7 +137,8 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
 #pragma unroll
     for (int j = 0; j < CB; ++j)
         acc[j][0] = acc[j][1] = 0ull;
-    const uint64_t magic = b2w4_pack2(12582912.f, 12582912.f);
+    const uint64_t magic = b2w4_pack2(786432.f, 786432.f);
+    const int4 start = make_int4(0x49400000, 0x49400000, 0x49400000, 0x49400000);
 
 #pragma unroll 1
     for (int c = 0; c < chunks; ++c) {
@@ -150,9 +147,9 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
         load_weights(c + S - 1);
         load_rows(c + S - 1);
         const uint8_t* s = smem + (c % S) * stage_bytes;
-        const int4* s_bias = reinterpret_cast<const int4*>(s) + cb0 * 4 + tid;
-        const uint64_t* s_as = reinterpret_cast<const uint64_t*>(s + bias_bytes) + cb0 * 4 + tid;
-        const uint8_t* rows = s + bias_bytes + as_bytes + (cb0 * 8 + gid) * kPitch + tid * 32;
+        // the scales of row pair 4 * cb0 + tid of the first group
+        const uint64_t* s_as = reinterpret_cast<const uint64_t*>(s) + (cb0 * 4 + tid) * SPG;
+        const uint8_t* rows = s + as_bytes + (cb0 * 8 + gid) * kPitch + tid * 32;
         // this lane's words: row gid of each tile, bytes 4*tid..+3 of every 32-k block
         const int tl = t0 - 2 * pair0;
         const uint32_t* s_w = reinterpret_cast<const uint32_t*>(s + nib_off) + tl * (kChunk * 128) + lane;
@@ -168,8 +165,8 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
                         const uint32_t w = have ? s_w[t * (kChunk * 128) + i * 128 + b * 32] : 0u;
-                        lo[t][b] = (w ^ 0x08080808u) & 0x0F0F0F0Fu;
-                        hi[t][b] = ((w >> 4) ^ 0x08080808u) & 0x0F0F0F0Fu;
+                        lo[t][b] = (w << 4) & 0xF0F0F0F0u;
+                        hi[t][b] = w & 0xF0F0F0F0u;
                     }
                     const uint8_t* q = s_scl + t * (kChunk * kScl) + i * kScl;
                     const float ws = !have  ? 0.f
@@ -187,7 +184,7 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
                         const uint32_t bev[4] = {be.x, be.y, be.z, be.w};
                         const uint32_t bov[4] = {bo.x, bo.y, bo.z, bo.w};
                         auto fold = [&](const int (&d)[4], uint64_t as2) {
-                            // d = 0x4B400000 + D: as a float 12582912 + D, exactly
+                            // d = 0x49400000 + 16 D: as a float 786432 + D, exactly
                             const uint64_t d0 = b2w4_sub2(
                                 b2w4_pack2(__int_as_float(d[0]), __int_as_float(d[1])), magic);
                             const uint64_t d1 = b2w4_sub2(
@@ -195,22 +192,24 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
                             acc[j][0] = b2w4_fma2(d0, b2w4_mul2(w0, as2), acc[j][0]);
                             acc[j][1] = b2w4_fma2(d1, b2w4_mul2(w1, as2), acc[j][1]);
                         };
+                        const int at = (i * (m8 / 2) + j * 4) * SPG;
                         if (A32) {
                             // one instruction = one 32-block, folded in ascending order
+                            const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(s_as + at);
+                            const ulonglong2 a01 = ap[0], a23 = ap[1];
+                            const uint64_t as2[4] = {a01.x, a01.y, a23.x, a23.y};
 #pragma unroll
                             for (int b = 0; b < 4; ++b) {
-                                const int at = (i * 4 + b) * (m8 / 2) + j * 4;
                                 int d[4];
                                 rows_mma(d, lo[0][b], lo[1][b], hi[0][b], hi[1][b], bev[b], bov[b],
-                                         s_bias[at]);
-                                fold(d, s_as[at]);
+                                         start);
+                                fold(d, as2[b]);
                             }
                         } else {
                             // two chains of two instructions (latency), joined by one add
-                            const int at = i * (m8 / 2) + j * 4;
                             int d[4], e[4];
                             rows_mma(d, lo[0][0], lo[1][0], hi[0][0], hi[1][0], bev[0], bov[0],
-                                     s_bias[at]);
+                                     start);
                             rows_mma(e, lo[0][1], lo[1][1], hi[0][1], hi[1][1], bev[1], bov[1],
                                      make_int4(0, 0, 0, 0));
                             rows_mma(d, lo[0][2], lo[1][2], hi[0][2], hi[1][2], bev[2], bov[2],
@@ -276,23 +275,18 @@ int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
     const int G = w->groups, spg = a32 ? 4 : 1, m8 = (m + 7) & ~7;
     void *qa = nullptr, *sc = nullptr;
     int rc;
-    // biases (two words per row and scale) in front: sixteen-byte aligned
-    const size_t scales = (size_t)G * spg * m8;
     if ((rc = b2w4_reserve(ctx, SCR_QA, (size_t)m * w->k, &qa)) != B2W4_OK ||
-        (rc = b2w4_reserve(ctx, SCR_AS, 3 * sizeof(float) * scales, &sc)) != B2W4_OK)
+        (rc = b2w4_reserve(ctx, SCR_AS, sizeof(float) * G * spg * m8, &sc)) != B2W4_OK)
         return rc;
-    int32_t* es_t = static_cast<int32_t*>(sc);
-    float* as_t = reinterpret_cast<float*>(es_t + 2 * scales);
-    if ((rc = b2w4_launch_quantize_mma(ctx, x, lda, m, w->k, m8, act_rule,
-                                       static_cast<int8_t*>(qa), as_t, es_t, true,
-                                       from)) != B2W4_OK)
+    float* as_t = static_cast<float*>(sc);
+    if ((rc = b2w4_launch_quantize_rows(ctx, x, lda, m, w->k, m8, act_rule,
+                                        static_cast<int8_t*>(qa), as_t, from)) != B2W4_OK)
         return rc;
     GemmRowsArgs a;
     a.nib = reinterpret_cast<const uint8_t*>(w->nib);
     a.scl = w->scl;
     a.qa = static_cast<const int8_t*>(qa);
     a.as_t = as_t;
-    a.es_t = reinterpret_cast<const int4*>(es_t);
     a.y = y;
     a.ldc = ldc;
     a.m = m;
@@ -305,10 +299,16 @@ int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
     a.activation = activation;
     a.act_n_begin = act_n_begin;
     a.act_n_len = act_n_len;
-    // Up to eight rows a warp per pair, else two.  Pairs per CTA: the fullest SM decides, so the
-    // least (CTAs on it) x (pairs of each); a CTA's own share of the activations counts as half
-    // a pair.
-    const int pw = m8 > 8 ? 2 : 1;
+    // Warps per pair: one, which splits a weight word once for all column blocks, while that
+    // gives every scheduler a warp; with fewer pairs the column blocks go to several.
+    const int ncb = m8 / 8, room = 10 * ctx->sm_count;
+    int pw = 1;
+    if (ncb == 2 || ncb == 4)
+        pw = a.pairs * 2 <= room ? 2 : 1;
+    else if (ncb == 3)
+        pw = a.pairs * 3 <= room ? 3 : 1;
+    // Pairs per CTA: the fullest SM decides, so the least (CTAs on it) x (pairs of each); a CTA's
+    // own share of the activations counts as half a pair.
     int best = 1;
     long best_cost = -1;
     for (int p = 1; p <= kRowsWarps / pw; ++p) {
@@ -325,6 +325,14 @@ int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
                   : rows_launch<PW, CB, true, false>(ctx, a, best))                      \
            : (a32 ? rows_launch<PW, CB, false, true>(ctx, a, best)                       \
                   : rows_launch<PW, CB, false, false>(ctx, a, best)))
-    return m8 > 16 ? B2W4_ROWS(2, 2) : m8 > 8 ? B2W4_ROWS(2, 1) : B2W4_ROWS(1, 1);
+    switch (ncb * 8 + pw) {
+    case 1 * 8 + 1: return B2W4_ROWS(1, 1);
+    case 2 * 8 + 1: return B2W4_ROWS(1, 2);
+    case 2 * 8 + 2: return B2W4_ROWS(2, 1);
+    case 3 * 8 + 1: return B2W4_ROWS(1, 3);
+    case 3 * 8 + 3: return B2W4_ROWS(3, 1);
+    case 4 * 8 + 1: return B2W4_ROWS(1, 4);
+    default: return B2W4_ROWS(2, 2);
+    }
 #undef B2W4_ROWS
 }

@@ -485,31 +485,13 @@ moe_route_fused_kernel(const float* __restrict__ hidden, int ldx, int tokens, in
 // ---- 6. SwiGLU + quantiser: one warp per (route, 128-wide group of I) ------------------
 // inter = (g * 1/(1+exp(-g))) * u with gate = columns [0,I), up = [I,2I)
 // (kernels/moe.cpp:160-183), then the per-128 quantiser; codes in tensor-operand order.
-// The grouped matmul multiplies unsigned nibbles q+8: its int32 accumulator starts at
-// 0x4B400000 - 8 * (sum of the codes), per group or per 32-block (dst[0..3], the lane's block is
-// lane / 8).  `sum`: of the lane's four codes.
-__device__ __forceinline__ void store_code_bias(int sum, int lane, bool a32, int32_t* dst) {
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1)  // integer: order-free
-        sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    if (a32) {
-        if ((lane & 7) == 0)
-            dst[lane >> 3] = 0x4B400000 - 8 * sum;
-        return;
-    }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    if (lane == 0)
-        *dst = 0x4B400000 - 8 * sum;
-}
-
 // Hidden rows for the grouped matmul, one warp per (token, 128-group): codes in tensor-operand
-// order, scales and accumulator biases per 128 values, and (q32 != null) per 32 values as well.
+// order and scales per 128 values, and (q32 != null) per 32 values as well.
 __global__ void moe_quantize_hidden_kernel(const float* __restrict__ hidden, int ldx, int tokens,
                                            int hidden_size, int8_t* __restrict__ q,
-                                           float* __restrict__ scales, int32_t* __restrict__ es,
-                                           int8_t* __restrict__ q32, float* __restrict__ scales32,
-                                           int32_t* __restrict__ es32) {
+                                           float* __restrict__ scales,
+                                           int8_t* __restrict__ q32,
+                                           float* __restrict__ scales32) {
     b2w4_pdl_chain_entry();
     const int G = hidden_size >> 7;
     const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -525,25 +507,21 @@ __global__ void moe_quantize_hidden_kernel(const float* __restrict__ hidden, int
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
     const size_t at = (size_t)row * hidden_size + (size_t)g * 128 + ((lane & 7) >> 1) * 32 +
                       (lane >> 3) * 4 + (lane & 1) * 2;
-    auto store = [&](float max, bool a32, int8_t* dst, float* scale_dst, int32_t* bias_dst) {
+    auto store = [&](float max, bool a32, int8_t* dst, float* scale_dst) {
         float scale, inv;
         b2w4_quant_params(max, scale, inv);
         const int c0 = b2w4_quant_code(v[0], inv), c1 = b2w4_quant_code(v[1], inv);
         const int c2 = b2w4_quant_code(v[2], inv), c3 = b2w4_quant_code(v[3], inv);
         if (a32 ? (lane & 7) == 0 : lane == 0)
             scale_dst[a32 ? lane >> 3 : 0] = scale;
-        store_code_bias(c0 + c1 + c2 + c3, lane, a32, bias_dst);
         *reinterpret_cast<char2*>(dst) = make_char2((signed char)c0, (signed char)c2);
         *reinterpret_cast<char2*>(dst + 16) = make_char2((signed char)c1, (signed char)c3);
     };
-    if (q32) {
-        const size_t s = ((size_t)row * G + g) * 4;
-        store(amax, true, q32 + at, scales32 + s, es32 + s);
-    }
+    if (q32)
+        store(amax, true, q32 + at, scales32 + ((size_t)row * G + g) * 4);
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 8));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 16));
-    const size_t s = (size_t)row * G + g;
-    store(amax, false, q + at, scales + s, es + s);
+    store(amax, false, q + at, scales + (size_t)row * G + g);
 }
 
 // one warp: 128 values of one route, written to `group_dst` (the 128 code bytes of the group)
@@ -553,7 +531,7 @@ __global__ void moe_quantize_hidden_kernel(const float* __restrict__ hidden, int
 __device__ __forceinline__ void swiglu_quant_warp(const float* __restrict__ gate_row,
                                                   const float* __restrict__ up_row, int lane,
                                                   int8_t* group_dst, float* scale_dst,
-                                                  bool a32 = false, int32_t* bias_dst = nullptr) {
+                                                  bool a32 = false) {
     const float* gp = gate_row + lane * 4;
     const float* up = up_row + lane * 4;
     float v[4];
@@ -582,8 +560,6 @@ __device__ __forceinline__ void swiglu_quant_warp(const float* __restrict__ gate
     } else if (lane == 0) {
         *scale_dst = scale;
     }
-    if (bias_dst)
-        store_code_bias(c0 + c1 + c2 + c3, lane, a32, bias_dst);
     // tensor-operand order inside the group: [word position][even words of the four
     // 32-blocks, then the odd words]; the lane holds k = 4*lane..+3: 32-block lane/8, even
     // codes at even index 2*(lane%8), 2*(lane%8)+1
@@ -592,13 +568,13 @@ __device__ __forceinline__ void swiglu_quant_warp(const float* __restrict__ gate
     *reinterpret_cast<char2*>(blk + 16) = make_char2((signed char)c1, (signed char)c3);
 }
 
-// scales, es (accumulator biases): [routes][scale_stride].  offsets (null = per-128 everywhere): first compact route of
+// scales: [routes][scale_stride].  offsets (null = per-128 everywhere): first compact route of
 // every expert, [num_experts + 1]; a route whose expert holds several routes is quantised per
 // 32 values (scales[r][4*g + block]), a lone route per 128 (scales[r][g]).
 __global__ void moe_swiglu_quant_kernel(const float* __restrict__ gu, int routes,
                                         int intermediate, int8_t* __restrict__ q,
-                                        float* __restrict__ scales, int32_t* __restrict__ es,
-                                        int scale_stride, const int32_t* __restrict__ offsets, int num_experts,
+                                        float* __restrict__ scales, int scale_stride,
+                                        const int32_t* __restrict__ offsets, int num_experts,
                                         const int32_t* __restrict__ route_lo,
                                         const int32_t* __restrict__ route_hi) {
     b2w4_pdl_chain_entry();
@@ -626,8 +602,7 @@ __global__ void moe_swiglu_quant_kernel(const float* __restrict__ gu, int routes
     const float* gp = gu + (size_t)r * 2 * intermediate + (size_t)g * 128;
     swiglu_quant_warp(gp, gp + intermediate, lane,
                       q + (size_t)r * intermediate + (size_t)g * 128,
-                      scales + (size_t)r * scale_stride + (a32 ? g * 4 : g), a32,
-                      es + (size_t)r * scale_stride + (a32 ? g * 4 : g));
+                      scales + (size_t)r * scale_stride + (a32 ? g * 4 : g), a32);
 }
 
 // ---- 8. combine: one block per (token, 512 hidden columns) -------------------------------
@@ -834,7 +809,6 @@ struct GroupedSmallArgs {
     const float* gate_up;     // if set (few routes): the activations are silu(gate)*up of these
                               // fp32 [routes][2K] rows, quantised here instead of read from qa
     const int4* slots;        // y-th expert with routes: (expert, first route, end), else empty
-    int num_experts_all;      // experts routed over
     int expert_begin;         // first expert whose weights this aggregate holds
     int expert_count;         // experts held
     const int32_t* row_map;   // route -> activation row, or null for identity
@@ -1075,14 +1049,19 @@ size_t grouped_small_smem(int k, int groups, int tpc, bool scl16) {
 // reads and fills (cp.async), kDepth - 1 groups ahead, on into the next pair, with no barrier in
 // the K loop.  (Straight into registers, three groups ahead, they came later: a warp's
 // outstanding loads share six scoreboards, so a wait for an old group waited for the newest
-// too.)  A word is split into unsigned bytes q+8
-// (lo = (w ^ 0x08080808) & 0x0F0F0F0F for even k, hi = ((w >> 4) ^ 0x08080808) & 0x0F0F0F0F for
-// odd k); the accumulator starts at 0x4B400000 - 8*sum(codes), read from shared memory as the
-// four words the instruction takes, and ends as the bit pattern of the float 12582912 + D.  D is
-// folded into fp32 chain values  y = fma(float(D), fp32(ws*as), y)  that stay in the warp's
-// registers until the last group, two columns per instruction.  The math is the dense kernels',
-// route by route.
-// What bounds it: issue slots (about 120 instructions per group and pair with sixteen routes,
+// too.)
+//
+// A word is split into signed bytes 16 q (lo = (w << 4) & 0xF0F0F0F0 for even k, hi = w &
+// 0xF0F0F0F0 for odd k: a nibble in the upper half of a byte is its two's complement value times
+// sixteen).  Every accumulator starts at 0x49400000, the bits of the float 786432 whose last place
+// is worth 1/16, and ends as 0x49400000 + 16 D: the bits of 786432 + D, exactly, since
+// |16 D| <= 128 * 127 * 128 < 2^22.  So D costs one subtraction, for two columns at once, and no
+// correction by the sum of the codes has to be made, staged and read (with unsigned q + 8 bytes it
+// had: 128-bit reads of four words per instruction were most of the shared-memory traffic, whose
+// pipe was 68 % busy; 256 tokens, 128 experts of 768: 231 -> 191 us).  D is folded into fp32 chain values
+// y = fma(float(D), fp32(ws*as), y)  that stay in the warp's registers until the last group, two
+// columns per instruction.  The math is the dense kernels', route by route.
+// What bounds it: issue slots (about 110 instructions per group and pair with sixteen routes,
 // most of them the chain and the split of the words), close to the time the weights take from
 // HBM at sixteen routes per expert.
 constexpr int kGR = 16;         // routes per pass: two column blocks
@@ -1093,18 +1072,15 @@ struct GroupedArgs {
     const void* scl;
     const int8_t* qa;         // [rows][K] int8, tensor-operand order inside each group
     const float* as;          // [rows][as_stride]: one scale per 128 values at [g]
-    const int32_t* es;        // same shape: 0x4B400000 - 8 * (sum of the group's codes)
     // The reference's rule for an expert that holds SEVERAL rows (kernels/moe.cpp:1055-1058
-    // -> kernels/matmul_w4.cpp:1125-1154): one activation scale per 32 values.  qa32 / as32 /
-    // es32 are those rows quantised that way (as32[r][4*g + block]); null = per-128 for every
-    // expert.  An expert with a single row keeps the per-128 rule (:1058-1075).
+    // -> kernels/matmul_w4.cpp:1125-1154): one activation scale per 32 values.  qa32 / as32 are
+    // those rows quantised that way (as32[r][4*g + block]); null = per-128 for every expert.
+    //  An expert with a single row keeps the per-128 rule (:1058-1075).
     const int8_t* qa32;
     const float* as32;
-    const int32_t* es32;
     int as_stride, as32_stride;
     const int4* slots;        // y-th expert with routes: (expert, first route, end), else empty
     int slot_count;           // entries of slots that can hold an expert
-    int num_experts_all;      // experts routed over
     int expert_begin;         // first expert whose weights this aggregate holds
     int expert_count;         // experts held
     const int32_t* row_map;   // route -> activation row, or null for identity
@@ -1125,8 +1101,8 @@ __device__ __forceinline__ void moe_mma_16x8x32(int (&d)[4], uint32_t a0, uint32
                                                 uint32_t b1, int4 c) {
     // lane (gid = lane/4, tid = lane%4): a0 row gid, k 4*tid..+3; a1 row gid+8; a2/a3 k+16;
     // b0 k 4*tid..+3 of column gid, b1 k+16; d0/d1 row gid, columns 2*tid, 2*tid+1; d2/d3 row
-    // gid+8.  A unsigned bytes, B signed bytes.
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+    // gid+8.
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
         "{%8,%9}, {%10,%11,%12,%13};"
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c.x), "r"(c.y), "r"(c.z),
@@ -1146,20 +1122,21 @@ constexpr int kPairSlot = 1024 + (SCL16 ? 32 : 64);
 // acc[j][0]: row gid, routes 2*tid and 2*tid+1 of block j; acc[j][1]: row gid+8.
 template <bool A32>
 __device__ __forceinline__ void pair_group(const PairWords& pw, const uint8_t* rows,
-                                           int row_bytes, const float* s_as, const int4* s_bias,
-                                           int g, int ncb, int tid, uint64_t (&acc)[2][2]) {
+                                           int row_bytes, const float* s_as, int g, int ncb,
+                                           int tid, uint64_t (&acc)[2][2]) {
     uint32_t lo[2][4], hi[2][4];
 #pragma unroll
     for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            lo[t][b] = (pw.w[t][b] ^ 0x08080808u) & 0x0F0F0F0Fu;
-            hi[t][b] = ((pw.w[t][b] >> 4) ^ 0x08080808u) & 0x0F0F0F0Fu;
+            lo[t][b] = (pw.w[t][b] << 4) & 0xF0F0F0F0u;
+            hi[t][b] = pw.w[t][b] & 0xF0F0F0F0u;
         }
-    const uint64_t magic = b2w4_pack2(12582912.f, 12582912.f);
+    const uint64_t magic = b2w4_pack2(786432.f, 786432.f);
+    const int4 start = make_int4(0x49400000, 0x49400000, 0x49400000, 0x49400000);
     const uint64_t w0 = b2w4_pack2(pw.ws[0], pw.ws[0]), w1 = b2w4_pack2(pw.ws[1], pw.ws[1]);
     auto fold = [&](const int (&c)[4], uint64_t as2, uint64_t (&y)[2]) {
-        // c = 0x4B400000 + D: as a float 12582912 + D, exactly
+        // c = 0x49400000 + 16 D: as a float 786432 + D, exactly
         const uint64_t d0 = b2w4_sub2(b2w4_pack2(__int_as_float(c[0]), __int_as_float(c[1])), magic);
         const uint64_t d1 = b2w4_sub2(b2w4_pack2(__int_as_float(c[2]), __int_as_float(c[3])), magic);
         y[0] = b2w4_fma2(d0, b2w4_mul2(w0, as2), y[0]);
@@ -1172,22 +1149,25 @@ __device__ __forceinline__ void pair_group(const PairWords& pw, const uint8_t* r
             const uint4 be = bp[0], bo = bp[1];
             const uint32_t bev[4] = {be.x, be.y, be.z, be.w}, bov[4] = {bo.x, bo.y, bo.z, bo.w};
             if (A32) {
-                // one instruction = one 32-block: its own accumulator, bias and activation
-                // scale, folded in ascending block order (kernels/matmul_w4.cpp:785-901)
+                // one instruction = one 32-block: its own accumulator and activation scale,
+                // folded in ascending block order (kernels/matmul_w4.cpp:785-901)
+                const ulonglong2* ap =
+                    reinterpret_cast<const ulonglong2*>(s_as) + (g * (kGR / 2) + j * 4 + tid) * 2;
+                const ulonglong2 a01 = ap[0], a23 = ap[1];
+                const uint64_t as2[4] = {a01.x, a01.y, a23.x, a23.y};
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    const int at = (g * 4 + b) * (kGR / 2) + j * 4 + tid;
                     int c[4];
                     moe_mma_16x8x32(c, lo[0][b], lo[1][b], hi[0][b], hi[1][b], bev[b], bov[b],
-                                    s_bias[at]);
-                    fold(c, reinterpret_cast<const uint64_t*>(s_as)[at], acc[j]);
+                                    start);
+                    fold(c, as2[b], acc[j]);
                 }
             } else {
                 // two chains of two instructions (latency), joined by one add
                 const int at = g * (kGR / 2) + j * 4 + tid;
                 int c[4], c2[4];
                 moe_mma_16x8x32(c, lo[0][0], lo[1][0], hi[0][0], hi[1][0], bev[0], bov[0],
-                                s_bias[at]);
+                                start);
                 moe_mma_16x8x32(c2, lo[0][1], lo[1][1], hi[0][1], hi[1][1], bev[1], bov[1],
                                 make_int4(0, 0, 0, 0));
                 moe_mma_16x8x32(c, lo[0][2], lo[1][2], hi[0][2], hi[1][2], bev[2], bov[2],
@@ -1211,46 +1191,60 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
     constexpr int kSlot = kPairSlot<SCL16>;
     const int G = a.groups, K = a.k;
     const int row_bytes = K + kRowPad;
-    // per (group or 32-block, route): accumulator bias and activation scale; sized for the
-    // per-32 rule (four entries per group).  A bias is stored as the instruction takes it:
-    // (b[2p], b[2p+1], b[2p], b[2p+1]) for the route pair p.
-    int4* s_bias = reinterpret_cast<int4*>(smem);                                 // [4G][kGR / 2]
-    float* s_as = reinterpret_cast<float*>(s_bias + (size_t)4 * G * (kGR / 2));   // [4G][kGR]
+    // activation scales [G][kGR], per 32 values [G][kGR / 2][4 blocks][2 routes]
+    float* s_as = reinterpret_cast<float*>(smem);
     uint8_t* s_qa = reinterpret_cast<uint8_t*>(s_as + (size_t)4 * G * kGR);       // [kGR][K+pad]
     uint8_t* s_ring = s_qa + (size_t)kGR * row_bytes;                             // [kGW][kDepth]
-    int* s_pre = reinterpret_cast<int*>(s_ring + kGW * kDepth * kSlot);           // [slots + 1]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tid = lane & 3;
 
-    // passes before slot y (experts held elsewhere have none)
-    if (warp == 0) {
-        int carry = 0;
-        for (int y0 = 0; y0 < a.slot_count; y0 += 32) {
-            int passes = 0;
-            if (y0 + lane < a.slot_count) {
-                const int4 slot = a.slots[y0 + lane];
-                const int e = slot.x - a.expert_begin;
-                if (e >= 0 && e < a.expert_count && slot.z > slot.y)
-                    passes = (slot.z - slot.y + kGR - 1) / kGR;
-            }
-            int run = passes;
+    // Passes before a slot (experts held elsewhere have none), by every warp for itself: a lane
+    // sums `per` slots in a row, the warp the lanes.  One trip to L2 and no barrier before the
+    // first weights are asked for, which is what a few routes wait for.
+    const int per = (a.slot_count + 31) / 32;
+    auto passes_of = [&](int4 slot) {
+        const int e = slot.x - a.expert_begin;
+        return e >= 0 && e < a.expert_count && slot.z > slot.y
+                   ? (slot.z - slot.y + kGR - 1) / kGR
+                   : 0;
+    };
+    auto scan = [&](int v) {  // inclusive, over the lanes
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int other = __shfl_up_sync(0xffffffffu, run, off);
-                if (lane >= off)
-                    run += other;
-            }
-            if (y0 + lane < a.slot_count)
-                s_pre[y0 + lane] = carry + run - passes;
-            carry += __shfl_sync(0xffffffffu, run, 31);
+        for (int off = 1; off < 32; off <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, v, off);
+            if (lane >= off)
+                v += other;
         }
-        if (lane == 0)
-            s_pre[a.slot_count] = carry;
-    }
-    __syncthreads();
+        return v;
+    };
+    int4 own = make_int4(0, 0, 0, 0);
+    int mine = 0;
+    for (int i = 0; i < per; ++i)
+        if (lane * per + i < a.slot_count) {
+            own = a.slots[lane * per + i];
+            mine += passes_of(own);
+        }
+    const int run = scan(mine), before = run - mine;
+    // the slot that pass p belongs to, and p's number within it
+    auto find = [&](int p, int4& slot) {
+        int at = __popc(__ballot_sync(0xffffffffu, run <= p));  // the lane
+        int pre = __shfl_sync(0xffffffffu, before, at);
+        int4 mem = own;
+        if (per > 1) {
+            const int y = at * per + lane;
+            mem = lane < per && y < a.slot_count ? a.slots[y] : make_int4(0, 0, 0, 0);
+            const int n = passes_of(mem), upto = scan(n);
+            at = __popc(__ballot_sync(0xffffffffu, pre + upto <= p));
+            pre += __shfl_sync(0xffffffffu, upto - n, at);
+        }
+        slot.x = __shfl_sync(0xffffffffu, mem.x, at);
+        slot.y = __shfl_sync(0xffffffffu, mem.y, at);
+        slot.z = __shfl_sync(0xffffffffu, mem.z, at);
+        return p - pre;
+    };
     const int pairs = a.tiles_e / 2;  // n_e is a multiple of 128
     const int rounds = (pairs + kGW - 1) / kGW;
-    const long long total = (long long)s_pre[a.slot_count] * rounds;
+    const long long total = (long long)__shfl_sync(0xffffffffu, run, 31) * rounds;
     long long u = total * blockIdx.x / gridDim.x;
     const long long u_end = total * (blockIdx.x + 1) / gridDim.x;
     const size_t tile_bytes = (size_t)G * 512, scl_tile_bytes = (size_t)G * (SCL16 ? 16 : 32);
@@ -1260,16 +1254,9 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
         const int round0 = (int)(u - (long long)pass_all * rounds);
         const int round1 = (int)min((long long)rounds, round0 + (u_end - u));
         u += round1 - round0;
-        int y = 0, y_hi = a.slot_count;  // the slot of this pass: s_pre[y] <= pass < s_pre[y+1]
-        while (y_hi - y > 1) {
-            const int mid = (y + y_hi) >> 1;
-            if (s_pre[mid] <= pass_all)
-                y = mid;
-            else
-                y_hi = mid;
-        }
-        const int4 slot = a.slots[y];
-        const int base = slot.y + (pass_all - s_pre[y]) * kGR;
+        int4 slot;
+        const int pass = find(pass_all, slot);
+        const int base = slot.y + pass * kGR;
         const int mc = min(kGR, slot.z - base);
         // the expert's rule: per 32 values when it holds several rows
         const bool a32 = a.qa32 != nullptr && slot.z - slot.y >= 2;
@@ -1313,15 +1300,13 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
             const int8_t* src = (a32 ? a.qa32 : a.qa) + (size_t)row * K;
             const size_t at = (size_t)row * (a32 ? a.as32_stride : a.as_stride);
             const float* as = (a32 ? a.as32 : a.as) + at;
-            const int32_t* es = (a32 ? a.es32 : a.es) + at;
 #pragma unroll 4
             for (int c = lane * 16; c < K; c += 32 * 16)
                 moe_cp_async<16>(s_qa + (size_t)mi * row_bytes + c, src + c);
             for (int gs = lane; gs < G * spg; gs += 32) {
-                moe_cp_async<4>(s_as + gs * kGR + mi, as + gs);
-                int* bias = reinterpret_cast<int*>(s_bias + gs * (kGR / 2) + (mi >> 1)) + (mi & 1);
-                moe_cp_async<4>(bias, es + gs);
-                moe_cp_async<4>(bias + 2, es + gs);
+                const int to = a32 ? (gs >> 2) * (4 * kGR) + (mi >> 1) * 8 + (gs & 3) * 2 + (mi & 1)
+                                   : gs * kGR + mi;
+                moe_cp_async<4>(s_as + to, as + gs);
             }
         }
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
@@ -1356,8 +1341,8 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
                                                                                              gid])
                                   : reinterpret_cast<const float*>(src + 1024)[t * 8 + gid];
                     }
-                    pair_group<decltype(rule)::value>(now, rows, row_bytes, s_as, s_bias, g, ncb,
-                                                      tid, acc);
+                    pair_group<decltype(rule)::value>(now, rows, row_bytes, s_as, g, ncb, tid,
+                                                      acc);
                 }
             };
             if (a32)
@@ -1386,9 +1371,8 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
     }
 }
 
-size_t grouped_smem(int k, int groups, int slots, bool scl16, int warps, int depth) {
-    return (size_t)4 * groups * (kGR / 2) * sizeof(int4) + sizeof(float) * kGR * groups * 4 +
-           (size_t)kGR * (k + kRowPad) + sizeof(int) * (slots + 1) +
+size_t grouped_smem(int k, int groups, bool scl16, int warps, int depth) {
+    return sizeof(float) * kGR * groups * 4 + (size_t)kGR * (k + kRowPad) +
            (size_t)warps * depth * (scl16 ? kPairSlot<true> : kPairSlot<false>);
 }
 
@@ -1409,12 +1393,11 @@ int launch_grouped_as(b2w4_ctx* ctx, const GroupedArgs& a, bool scl16, size_t sm
 // `decode` (few tokens): the shared-memory variant, optionally with SwiGLU + quantiser fused
 // into its prologue (fused_gate_up = the gate_up matmul's fp32 output).
 // qa32 / as32: the same rows quantised per 32 values, for experts that hold several routes
-// (null: per-128 for all); es / es32: accumulator biases, one per scale (not read by the decode
-// variant); as_stride / as32_stride: scales per row of as / as32.
+// (null: per-128 for all); as_stride / as32_stride: scales per row of as / as32.
 int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int expert_begin,
                    int expert_count, int routes, const int8_t* qa, const float* as,
-                   const int32_t* es, int as_stride, const int8_t* qa32, const float* as32,
-                   const int32_t* es32, int as32_stride, const int4* slots, const int32_t* row_map, float* out, bool decode,
+                   int as_stride, const int8_t* qa32, const float* as32, int as32_stride,
+                   const int4* slots, const int32_t* row_map, float* out, bool decode,
                    const float* fused_gate_up = nullptr, const b2w4_tp_args* peers = nullptr,
                    int stage_rows = 0) {
     const int n_e = w->n / expert_count;
@@ -1428,7 +1411,6 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
         a.as = as;
         a.slots = slots;
         a.gate_up = fused_gate_up;
-        a.num_experts_all = num_experts_all;
         a.expert_begin = expert_begin;
         a.expert_count = expert_count;
         a.row_map = row_map;
@@ -1464,15 +1446,12 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
     a.scl = w->scl;
     a.qa = qa;
     a.as = as;
-    a.es = es;
     a.as_stride = as_stride;
     a.qa32 = qa32;
     a.as32 = as32;
-    a.es32 = es32;
     a.as32_stride = as32_stride;
     a.slots = slots;
     a.slot_count = slots_y;
-    a.num_experts_all = num_experts_all;
     a.expert_begin = expert_begin;
     a.expert_count = expert_count;
     a.row_map = row_map;
@@ -1481,13 +1460,10 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
     a.groups = w->groups;
     a.n_e = n_e;
     a.tiles_e = n_e / 8;
-    // the longest rows: those that fit with a pair of tiles beside them (7936, or 7808 with fp32
-    // scales), the limit of the operator
-    const size_t pair = (size_t)2 * w->groups * (512 + 8 * (scl16 ? 2 : 4));
-    if (grouped_smem(w->k, w->groups, 0, scl16, 0, 0) + pair > 235 * 1024)
+    if (w->k > (scl16 ? 7936 : 7808))  // the limit of the operator
         return b2w4_fail(ctx, B2W4_E_INVALID, "moe: K=%d needs too much shared memory", w->k);
     auto bytes = [&](int warps, int depth) {
-        return grouped_smem(w->k, w->groups, slots_y, scl16, warps, depth);
+        return grouped_smem(w->k, w->groups, scl16, warps, depth);
     };
     // two CTAs per SM, else sixteen warps in one, else what the rows leave room for
     if (bytes(8, 6) <= 112 * 1024)
@@ -1575,11 +1551,8 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     const size_t o_asi = align_up(o_qi + (size_t)routes * intermediate, 256);
     const size_t o_qh32 = align_up(o_asi + sizeof(float) * routes * gi * 4, 256);
     const size_t o_ash32 = align_up(o_qh32 + (rule32 ? (size_t)tokens * hidden_size : 0), 256);
-    const size_t o_es = align_up(o_ash32 + (rule32 ? sizeof(float) * tokens * gh * 4 : 0), 256);
-    const size_t o_es32 = align_up(o_es + sizeof(int32_t) * tokens * gh, 256);
-    const size_t o_esi =
-        align_up(o_es32 + (rule32 ? sizeof(int32_t) * tokens * gh * 4 : 0), 256);
-    const size_t quant_bytes = align_up(o_esi + sizeof(int32_t) * routes * gi * 4, 256);
+    const size_t quant_bytes =
+        align_up(o_ash32 + (rule32 ? sizeof(float) * tokens * gh * 4 : 0), 256);
     void *sm = nullptr, *qb = nullptr, *gu = nullptr, *dn = nullptr;
     int rc;
     if ((rc = b2w4_reserve(ctx, SCR_MOE_A, small_bytes, &sm)) != B2W4_OK ||
@@ -1604,9 +1577,6 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     float* as_inter = reinterpret_cast<float*>(qbb + o_asi);  // [routes][4 * gi]
     int8_t* q_hidden32 = rule32 ? reinterpret_cast<int8_t*>(qbb + o_qh32) : nullptr;
     float* as_hidden32 = rule32 ? reinterpret_cast<float*>(qbb + o_ash32) : nullptr;
-    int32_t* es_hidden = reinterpret_cast<int32_t*>(qbb + o_es);
-    int32_t* es_hidden32 = rule32 ? reinterpret_cast<int32_t*>(qbb + o_es32) : nullptr;
-    int32_t* es_inter = reinterpret_cast<int32_t*>(qbb + o_esi);  // [routes][4 * gi]
     cudaStream_t st = ctx->stream;
 
     const __half* router = static_cast<const __half*>(router_fp16_dev);
@@ -1656,22 +1626,21 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     }
     // which grouped-matmul variant: the few-token one implements the per-128 rule only
     const bool decode = rule32 ? false : tokens <= kFusedSwigluTokens;
-    // (the decode variant takes the rows that the fused routing kernel quantised)
-    if (!decode || !fused) {
+    // (the fused routing kernel has quantised the rows, per 128 values)
+    if (rule32 || !fused) {
         const long long threads = (long long)tokens * gh * 32;
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, moe_quantize_hidden_kernel,
                                            dim3((int)((threads + 255) / 256)), dim3(256), 0, st,
                                            hidden_dev, ldx, tokens, hidden_size, q_hidden,
-                                           as_hidden, es_hidden, q_hidden32, as_hidden32,
-                                           es_hidden32));
+                                           as_hidden, q_hidden32, as_hidden32));
         ctx->launches++;
     }
     // compact positions stay global; the grouped kernels skip experts held elsewhere
     const int32_t* local_offsets = offsets + expert_begin;
     const bool partial = expert_count != num_experts;
     if ((rc = launch_grouped(ctx, gate_up, num_experts, expert_begin, expert_count, routes,
-                             q_hidden, as_hidden, es_hidden, gh, q_hidden32, as_hidden32,
-                             es_hidden32, gh * 4, slots, route_token, static_cast<float*>(gu), decode)) != B2W4_OK)
+                             q_hidden, as_hidden, gh, q_hidden32, as_hidden32, gh * 4, slots,
+                             route_token, static_cast<float*>(gu), decode)) != B2W4_OK)
         return rc;
     // few routes: SwiGLU and its quantiser run inside the down-projection's CTAs
     const bool fuse_swiglu = decode;
@@ -1680,7 +1649,7 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
         B2W4_CUDA(ctx, b2w4_launch_chained(
                            ctx->pdl, moe_swiglu_quant_kernel, dim3((int)((threads + 255) / 256)),
                            dim3(256), 0, st, static_cast<const float*>(gu), routes, intermediate,
-                           q_inter, as_inter, es_inter, gi * 4,
+                           q_inter, as_inter, gi * 4,
                            rule32 ? static_cast<const int32_t*>(offsets) : nullptr, num_experts,
                            partial ? local_offsets : nullptr,
                            partial ? local_offsets + expert_count : nullptr));
@@ -1690,8 +1659,8 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     const bool fused_handover = peers != nullptr && decode;
     // a route's SwiGLU row was quantised by its own expert's rule: one code buffer serves both
     if ((rc = launch_grouped(ctx, down, num_experts, expert_begin, expert_count, routes, q_inter,
-                             as_inter, es_inter, gi * 4, rule32 ? q_inter : nullptr,
-                             rule32 ? as_inter : nullptr, es_inter, gi * 4, slots, nullptr,
+                             as_inter, gi * 4, rule32 ? q_inter : nullptr,
+                             rule32 ? as_inter : nullptr, gi * 4, slots, nullptr,
                              static_cast<float*>(dn), decode,
                              fuse_swiglu ? static_cast<const float*>(gu) : nullptr,
                              fused_handover ? peers : nullptr, stage_rows)) != B2W4_OK)
