@@ -29,6 +29,7 @@ namespace {
 constexpr int kRowsWarps = 10;        // warps per CTA at most
 constexpr int kRowsThreads = kRowsWarps * 32;
 constexpr int kChunk = 4;             // groups per stage
+constexpr int kRelayWarps = 16;       // the same where warps share a chain
 constexpr int kPitch = kChunk * 128 + 16;  // bytes between a stage's rows: conflict-free reads
 
 struct GemmRowsArgs {
@@ -38,6 +39,7 @@ struct GemmRowsArgs {
     const float* as_t;   // activation scales [G][m8], per 32 values [G][m8 / 2][4 blocks][2 rows]
     float* y;
     int ldc, m, m8, n, k, groups, tiles, pairs;
+    int pw;              // KS > 1: warps beside one another per pair, one column block each
     int activation, act_n_begin, act_n_len;
 };
 
@@ -66,14 +68,19 @@ __host__ __device__ constexpr size_t rows_stage_bytes(int m8, int spg, int pairs
 }
 
 // PW warps per pair of weight tiles, CB blocks of eight activation rows per warp, S stages.
-template <int PW, int CB, bool SCL16, bool A32, int S>
-__global__ void __launch_bounds__(kRowsThreads, 2)
+// KS > 1 (few pairs): KS warps share a pair and a column block (PW is not used, a.pw is).  Each
+// takes kChunk / KS groups of a stage, makes their sums and products ws * as, and only then
+// needs the chain values: it has them from the warp that holds the groups before, through shared
+// memory, and hands them on, so that the chain keeps its order.
+template <int PW, int CB, bool SCL16, bool A32, int S, int KS>
+__global__ void __launch_bounds__(KS > 1 ? kRelayWarps * 32 : kRowsThreads, KS > 1 ? 1 : 2)
 gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
     constexpr int SPG = A32 ? 4 : 1;  // scales per group
     constexpr int kScl = SCL16 ? 16 : 32;  // bytes of a tile's scales of a group
     extern __shared__ __align__(128) uint8_t smem[];
     const int G = a.groups, m8 = a.m8;
-    const int warps = blockDim.x / 32, pairs = warps / PW;
+    const int pw = KS > 1 ? a.pw : PW;
+    const int warps = blockDim.x / 32, pairs = warps / (pw * KS);
     const int as_bytes = kChunk * SPG * m8 * 4;
     const int nib_off = as_bytes + m8 * kPitch;
     const int scl_off = nib_off + pairs * 2 * kChunk * 512;
@@ -81,9 +88,10 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tid = lane & 3;
-    const int pair0 = blockIdx.x * pairs, pair = pair0 + warp / PW;
-    const int cb0 = (warp % PW) * CB;  // first column block
-    const int ncb = PW == 1 ? CB : min(CB, m8 / 8 - cb0);  // may be none
+    const int chain = warp / KS, turn = warp % KS;
+    const int pair0 = blockIdx.x * pairs, pair = pair0 + chain / pw;
+    const int cb0 = (chain % pw) * CB;  // first column block
+    const int ncb = PW == 1 || KS > 1 ? CB : min(CB, m8 / 8 - cb0);  // may be none
     const bool busy = pair < a.pairs && ncb > 0;
     const int t0 = 2 * pair;
     const bool two = t0 + 1 < a.tiles;
@@ -154,72 +162,131 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
         const int tl = t0 - 2 * pair0;
         const uint32_t* s_w = reinterpret_cast<const uint32_t*>(s + nib_off) + tl * (kChunk * 128) + lane;
         const uint8_t* s_scl = s + scl_off + tl * (kChunk * kScl) + gid * (kScl / 8);
+        // the words of group i of the stage, split, and the scales of both tiles
+        auto words = [&](int i, uint32_t (&lo)[2][4], uint32_t (&hi)[2][4], uint64_t (&ws2)[2]) {
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const bool have = t == 0 || two;  // a missing tile: zeros
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const uint32_t w = have ? s_w[t * (kChunk * 128) + i * 128 + b * 32] : 0u;
+                    lo[t][b] = (w << 4) & 0xF0F0F0F0u;
+                    hi[t][b] = w & 0xF0F0F0F0u;
+                }
+                const uint8_t* q = s_scl + t * (kChunk * kScl) + i * kScl;
+                const float ws = !have  ? 0.f
+                                 : SCL16 ? __half2float(*reinterpret_cast<const __half*>(q))
+                                         : *reinterpret_cast<const float*>(q);
+                ws2[t] = b2w4_pack2(ws, ws);
+            }
+        };
+        // the sums of a group, per block (A32) or whole, of column block j
+        auto sums = [&](int i, int j, const uint32_t (&lo)[2][4], const uint32_t (&hi)[2][4],
+                        int (&d)[SPG][4]) {
+            const uint4* bp = reinterpret_cast<const uint4*>(rows + j * 8 * kPitch + i * 128);
+            const uint4 be = bp[0], bo = bp[1];
+            const uint32_t bev[4] = {be.x, be.y, be.z, be.w};
+            const uint32_t bov[4] = {bo.x, bo.y, bo.z, bo.w};
+            if (A32) {
+#pragma unroll
+                for (int b = 0; b < SPG; ++b)  // one instruction = one 32-block
+                    rows_mma(d[b], lo[0][b], lo[1][b], hi[0][b], hi[1][b], bev[b], bov[b], start);
+            } else {
+                // two chains of two instructions (latency), joined by one add
+                int e[4];
+                rows_mma(d[0], lo[0][0], lo[1][0], hi[0][0], hi[1][0], bev[0], bov[0], start);
+                rows_mma(e, lo[0][1], lo[1][1], hi[0][1], hi[1][1], bev[1], bov[1],
+                         make_int4(0, 0, 0, 0));
+                rows_mma(d[0], lo[0][2], lo[1][2], hi[0][2], hi[1][2], bev[2], bov[2],
+                         make_int4(d[0][0], d[0][1], d[0][2], d[0][3]));
+                rows_mma(e, lo[0][3], lo[1][3], hi[0][3], hi[1][3], bev[3], bov[3],
+                         make_int4(e[0], e[1], e[2], e[3]));
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+                    d[0][x] += e[x];
+            }
+        };
+        auto scales = [&](int i, int j, uint64_t (&as2)[SPG]) {
+            const uint64_t* at = s_as + (i * (m8 / 2) + j * 4) * SPG;
+            if (A32) {
+                const ulonglong2 a01 = reinterpret_cast<const ulonglong2*>(at)[0];
+                const ulonglong2 a23 = reinterpret_cast<const ulonglong2*>(at)[1];
+                as2[0] = a01.x, as2[SPG / 4] = a01.y, as2[SPG / 2] = a23.x, as2[SPG - 1] = a23.y;
+            } else {
+                as2[0] = at[0];
+            }
+        };
+        // d = 0x49400000 + 16 D: as a float 786432 + D, exactly
+        auto value = [&](int x, int y) {
+            return b2w4_sub2(b2w4_pack2(__int_as_float(x), __int_as_float(y)), magic);
+        };
+        if constexpr (KS > 1) {
+            constexpr int GPW = kChunk / KS;
+            uint64_t v[GPW][SPG][2], f[GPW][SPG][2];
+#pragma unroll
+            for (int i = 0; i < GPW; ++i) {
+                const int at = turn * GPW + i;
+                if (c * kChunk + at < G && busy) {  // warp-uniform
+                    uint32_t lo[2][4], hi[2][4];
+                    uint64_t ws2[2], as2[SPG];
+                    int d[SPG][4];
+                    words(at, lo, hi, ws2);
+                    scales(at, 0, as2);
+                    sums(at, 0, lo, hi, d);
+#pragma unroll
+                    for (int b = 0; b < SPG; ++b) {
+                        v[i][b][0] = value(d[b][0], d[b][1]);
+                        v[i][b][1] = value(d[b][2], d[b][3]);
+                        f[i][b][0] = b2w4_mul2(ws2[0], as2[b]);
+                        f[i][b][1] = b2w4_mul2(ws2[1], as2[b]);
+                    }
+                }
+            }
+            // The chain values: from the warp in front (the first one's come from the last one,
+            // before the barrier of this stage).  Barriers 1..12: (KS - 1) links of each chain.
+            ulonglong2* s_y =
+                reinterpret_cast<ulonglong2*>(smem + S * stage_bytes) + chain * 32 + lane;
+            const int link = 1 + chain * (KS - 1) + turn;
+            if (turn > 0)
+                asm volatile("bar.sync %0, 64;" ::"r"(link - 1) : "memory");
+            if (c > 0 || turn > 0) {
+                const ulonglong2 y2 = *s_y;
+                acc[0][0] = y2.x;
+                acc[0][1] = y2.y;
+            }
+#pragma unroll
+            for (int i = 0; i < GPW; ++i)
+                if (c * kChunk + turn * GPW + i < G && busy) {
+#pragma unroll
+                    for (int b = 0; b < SPG; ++b) {
+                        acc[0][0] = b2w4_fma2(v[i][b][0], f[i][b][0], acc[0][0]);
+                        acc[0][1] = b2w4_fma2(v[i][b][1], f[i][b][1], acc[0][1]);
+                    }
+                }
+            *s_y = make_ulonglong2(acc[0][0], acc[0][1]);
+            if (turn < KS - 1)
+                asm volatile("bar.arrive %0, 64;" ::"r"(link) : "memory");
+            continue;
+        }
 #pragma unroll
         for (int i = 0; i < kChunk; ++i) {
             if (c * kChunk + i < G && busy) {  // warp-uniform
                 uint32_t lo[2][4], hi[2][4];
                 uint64_t ws2[2];
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const bool have = t == 0 || two;  // a missing tile: zeros
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        const uint32_t w = have ? s_w[t * (kChunk * 128) + i * 128 + b * 32] : 0u;
-                        lo[t][b] = (w << 4) & 0xF0F0F0F0u;
-                        hi[t][b] = w & 0xF0F0F0F0u;
-                    }
-                    const uint8_t* q = s_scl + t * (kChunk * kScl) + i * kScl;
-                    const float ws = !have  ? 0.f
-                                     : SCL16 ? __half2float(*reinterpret_cast<const __half*>(q))
-                                             : *reinterpret_cast<const float*>(q);
-                    ws2[t] = b2w4_pack2(ws, ws);
-                }
-                const uint64_t w0 = ws2[0], w1 = ws2[1];
+                words(i, lo, hi, ws2);
 #pragma unroll
                 for (int j = 0; j < CB; ++j) {
                     if (j < ncb) {
-                        const uint4* bp =
-                            reinterpret_cast<const uint4*>(rows + j * 8 * kPitch + i * 128);
-                        const uint4 be = bp[0], bo = bp[1];
-                        const uint32_t bev[4] = {be.x, be.y, be.z, be.w};
-                        const uint32_t bov[4] = {bo.x, bo.y, bo.z, bo.w};
-                        auto fold = [&](const int (&d)[4], uint64_t as2) {
-                            // d = 0x49400000 + 16 D: as a float 786432 + D, exactly
-                            const uint64_t d0 = b2w4_sub2(
-                                b2w4_pack2(__int_as_float(d[0]), __int_as_float(d[1])), magic);
-                            const uint64_t d1 = b2w4_sub2(
-                                b2w4_pack2(__int_as_float(d[2]), __int_as_float(d[3])), magic);
-                            acc[j][0] = b2w4_fma2(d0, b2w4_mul2(w0, as2), acc[j][0]);
-                            acc[j][1] = b2w4_fma2(d1, b2w4_mul2(w1, as2), acc[j][1]);
-                        };
-                        const int at = (i * (m8 / 2) + j * 4) * SPG;
-                        if (A32) {
-                            // one instruction = one 32-block, folded in ascending order
-                            const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(s_as + at);
-                            const ulonglong2 a01 = ap[0], a23 = ap[1];
-                            const uint64_t as2[4] = {a01.x, a01.y, a23.x, a23.y};
+                        uint64_t as2[SPG];
+                        int d[SPG][4];
+                        scales(i, j, as2);
+                        sums(i, j, lo, hi, d);
 #pragma unroll
-                            for (int b = 0; b < 4; ++b) {
-                                int d[4];
-                                rows_mma(d, lo[0][b], lo[1][b], hi[0][b], hi[1][b], bev[b], bov[b],
-                                         start);
-                                fold(d, as2[b]);
-                            }
-                        } else {
-                            // two chains of two instructions (latency), joined by one add
-                            int d[4], e[4];
-                            rows_mma(d, lo[0][0], lo[1][0], hi[0][0], hi[1][0], bev[0], bov[0],
-                                     start);
-                            rows_mma(e, lo[0][1], lo[1][1], hi[0][1], hi[1][1], bev[1], bov[1],
-                                     make_int4(0, 0, 0, 0));
-                            rows_mma(d, lo[0][2], lo[1][2], hi[0][2], hi[1][2], bev[2], bov[2],
-                                     make_int4(d[0], d[1], d[2], d[3]));
-                            rows_mma(e, lo[0][3], lo[1][3], hi[0][3], hi[1][3], bev[3], bov[3],
-                                     make_int4(e[0], e[1], e[2], e[3]));
-#pragma unroll
-                            for (int x = 0; x < 4; ++x)
-                                d[x] += e[x];
-                            fold(d, s_as[at]);
+                        for (int b = 0; b < SPG; ++b) {  // blocks in ascending order
+                            acc[j][0] = b2w4_fma2(value(d[b][0], d[b][1]),
+                                                  b2w4_mul2(ws2[0], as2[b]), acc[j][0]);
+                            acc[j][1] = b2w4_fma2(value(d[b][2], d[b][3]),
+                                                  b2w4_mul2(ws2[1], as2[b]), acc[j][1]);
                         }
                     }
                 }
@@ -228,7 +295,7 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
     }
 
     // y[row][n]: for one row, the eight lanes of a quarter-warp hold eight consecutive n
-    if (busy) {
+    if (busy && turn == KS - 1) {
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int n = (t0 + t) * 8 + gid;
@@ -248,22 +315,36 @@ gemm_w4a8_rows_kernel(const GemmRowsArgs a) {
     }
 }
 
-template <int PW, int CB, bool SCL16, bool A32>
-int rows_launch(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
-    const int ctas = (a.pairs + pairs_per_cta - 1) / pairs_per_cta;
-    const size_t stage = rows_stage_bytes(a.m8, A32 ? 4 : 1, pairs_per_cta, SCL16);
-    // one CTA per SM: a deeper ring
-    const bool deep = ctas <= ctx->sm_count && 6 * stage <= 220 * 1024;
-    auto kern = deep ? gemm_w4a8_rows_kernel<PW, CB, SCL16, A32, 6>
-                     : gemm_w4a8_rows_kernel<PW, CB, SCL16, A32, 3>;
-    const size_t smem = (deep ? 6 : 3) * stage;
-    static b2w4_smem_optin configured[2];  // per instantiation and device
-    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[deep]));
-    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(ctas),
-                                       dim3(pairs_per_cta * PW * 32), smem, ctx->stream,
-                                       a));
+template <int PW, int CB, bool SCL16, bool A32, int S, int KS>
+int rows_launch_as(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
+    auto kern = gemm_w4a8_rows_kernel<PW, CB, SCL16, A32, S, KS>;
+    const int chains = pairs_per_cta * (KS > 1 ? a.pw : PW);
+    const size_t smem = S * rows_stage_bytes(a.m8, A32 ? 4 : 1, pairs_per_cta, SCL16) +
+                        (KS > 1 ? chains * 512 : 0);
+    static b2w4_smem_optin configured;  // per instantiation and device
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured));
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern,
+                                       dim3((a.pairs + pairs_per_cta - 1) / pairs_per_cta),
+                                       dim3(chains * KS * 32), smem, ctx->stream, a));
     ctx->launches++;
     return B2W4_OK;
+}
+// six stages where a CTA has the SM to itself, else three
+bool rows_deep(b2w4_ctx* ctx, const GemmRowsArgs& a, bool scl16, bool a32, int pairs_per_cta) {
+    return (a.pairs + pairs_per_cta - 1) / pairs_per_cta <= ctx->sm_count &&
+           6 * rows_stage_bytes(a.m8, a32 ? 4 : 1, pairs_per_cta, scl16) <= 220 * 1024;
+}
+template <int PW, int CB, bool SCL16, bool A32>
+int rows_launch(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
+    return rows_deep(ctx, a, SCL16, A32, pairs_per_cta)
+               ? rows_launch_as<PW, CB, SCL16, A32, 6, 1>(ctx, a, pairs_per_cta)
+               : rows_launch_as<PW, CB, SCL16, A32, 3, 1>(ctx, a, pairs_per_cta);
+}
+template <bool SCL16, bool A32>
+int rows_relay(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
+    return pairs_per_cta * a.pw * 4 <= kRelayWarps
+               ? rows_launch_as<1, 1, SCL16, A32, 6, 4>(ctx, a, pairs_per_cta)
+               : rows_launch_as<1, 1, SCL16, A32, 6, 2>(ctx, a, pairs_per_cta);
 }
 
 }  // namespace
@@ -307,6 +388,22 @@ int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
         pw = a.pairs * 2 <= room ? 2 : 1;
     else if (ncb == 3)
         pw = a.pairs * 3 <= room ? 3 : 1;
+    const bool scl16 = w->scales_fp16 != 0;
+    // Few pairs per SM: a warp's latency sets the time, so two or four warps share a chain.  Per
+    // 32 values the chain itself is four times as long: with three pairs per SM or more it is
+    // shared for one column block only, and with three or four not at all.  us per call before
+    // -> after, per 32 / per 128 values: [2560, 9728]
+    // 8 rows 24.2 -> 20.3 / 23.6 -> 18.6, 16 rows 26.0 -> 21.3 / 24.3 -> 19.1, 32 rows 33.0 ->
+    // 28.4 / 31.9 -> 23.5; [9728, 2560] (five pairs) 8 rows 8.4 -> 7.7 / 8.0 -> 7.0; [6144, 2560]
+    // (three) 8 rows 6.7 -> 7.1, not taken / 6.8 -> 6.3, 16 rows 7.9 -> 8.1, not taken / 7.6 -> 7.2.
+    a.pw = ncb;
+    const int few = (a.pairs + ctx->sm_count - 1) / ctx->sm_count;
+    if (few * ncb * 2 <= kRelayWarps && (few <= 2 || !a32 || (few > 4 && ncb == 1)) &&
+        rows_deep(ctx, a, scl16, a32, few))
+        return scl16 ? (a32 ? rows_relay<true, true>(ctx, a, few)
+                            : rows_relay<true, false>(ctx, a, few))
+                     : (a32 ? rows_relay<false, true>(ctx, a, few)
+                            : rows_relay<false, false>(ctx, a, few));
     // Pairs per CTA: the fullest SM decides, so the least (CTAs on it) x (pairs of each); a CTA's
     // own share of the activations counts as half a pair.
     int best = 1;
@@ -319,7 +416,6 @@ int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
             best = p;
         }
     }
-    const bool scl16 = w->scales_fp16 != 0;
 #define B2W4_ROWS(PW, CB)                                                                \
     (scl16 ? (a32 ? rows_launch<PW, CB, true, true>(ctx, a, best)                        \
                   : rows_launch<PW, CB, true, false>(ctx, a, best))                      \

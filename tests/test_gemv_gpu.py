@@ -486,6 +486,22 @@ def test_long_rows_split_over_a_cluster(ctx, n, k, f32):
 
 
 @pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
+@pytest.mark.parametrize("m,pairs,k", [(16, 1, 768), (12, 2, 640), (13, 3, 384), (16, 4, 1152),
+                                       (17, 1, 128), (24, 2, 896), (32, 1, 256), (25, 2, 2560),
+                                       (4, 8, 640), (9, 5, 512)])
+def test_few_rows_with_few_pairs_per_multiprocessor(ctx, m, pairs, k, rule):
+    """Two or four warps share the chain of a pair of tiles: 1 to 20 groups (whole stages of four
+    and cut ones), the last pair with one tile, up to the largest number of chains per block (and
+    one past it)."""
+    n = 148 * 16 * pairs - 8
+    blocks = pkg.synth.bg128_weight(20261125, n + k + m, n, k)
+    x = pkg.synth.activations(7, m + 5, m, k)
+    x[m // 2, :128] = 0.0
+    y, _ = run_gpu(ctx, blocks, n, k, x, rule=rule, sums=False, pad=4)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=rule).tobytes()
+
+
+@pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
 @pytest.mark.parametrize("m,n,k", [(2, 16392, 256), (3, 4104, 512), (8, 6152, 640), (5, 1608, 384),
                                    (2, 1608, 6272), (7, 1603, 6144)])
 def test_two_to_eight_rows_on_the_streamed_kernel(ctx, m, n, k, rule):
