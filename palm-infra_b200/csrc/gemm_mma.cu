@@ -1,5 +1,8 @@
-// W4G128 x int8 GEMM for 9..256 activation rows per launch (batched decode, prefill) on the
-// warp-level int8 tensor instruction (mma.sync m16n8k32) with register accumulators.
+// W4G128 x int8 GEMM on the
+// warp-level int8 tensor instruction (mma.sync m16n8k32) with register accumulators, up to 256
+// activation rows per launch.  Calls of more than 32 rows come here when K is above the tensor-core
+// kernels' limit or, per 128 values, while every weight CTA is resident with all activations
+// beside it; smaller calls only when asked for.
 //
 // Arithmetic = the reference's NEON W4A8 kernels: the GEMV applied row by row
 // (kernels/matmul_w4.cpp:211-295 with the per-128 quantiser, kernels/matmul_quant.cpp:578-641)

@@ -7,13 +7,12 @@
 //
 // What bounds it: the issue slots and the fp32 pipe of that chain (M*N*K/32 sums); the MMAs
 // keep the tensor pipe under a tenth busy.  So everything around the chain is kept out of it:
-//   epilogue   eight warps, thread = one token x half of the tile's columns.  Eight columns of
-//              two blocks are fetched from tensor memory while the eight before them are folded,
-//              across hand-overs too, so a warp waits for no fetch; a tile of up to 128 columns
+//   epilogue   sixteen warps, thread = one token x a quarter of the tile's columns, four warps per
+//              scheduler so that one folds while another fetches; a tile of up to 128 columns
 //              (row_tiles) spreads what a group costs beside its columns.
 //   unpack     a nibble becomes a signed byte of 16 q with one AND (high nibble) or a shift
 //              and an AND (low nibble): three instructions per eight weights, so the sums
-//              are 16 D, |16 D| < 2^19.
+//              are 16 D, |16 D| < 2^19.  Three warps, every third group each, whole groups.
 //   to float   the hardware conversion, so that the fp32 pipe sees only the scale product and
 //              the multiply-add, both paired (fma.rn.f32x2).  It also moves the sums from the
 //              registers that the fetch filled to register pairs.  The scales are staged as
@@ -21,9 +20,10 @@
 //   MMA        one thread; two accumulator units (a group each, or half a group where tiles are
 //              wide) or more in tensor memory, and one barrier frees an activation and a weight
 //              stage together.
-// Measured against sixteen epilogue warps with a quarter of at most 64 columns each, fetch and
-// chain in turn: 1000 rows, [4100, 9728], three matmuls 882 -> 715 us; eight layers of a
-// 256-token prompt, all operators, 2.47 -> 2.20 ms.
+// Measured, 1000 rows, [4100, 9728], three matmuls: tiles of at most 64 columns 882 us; of up to
+// 128 with eight epilogue warps and all unpack warps on one group 715 us; this form 618 us (eight
+// layers of a 256-token prompt, all operators: 2.46, 2.20 and 1.95 ms).  At 112 columns a group
+// takes 2490 cycles, of which the chain is 1930.
 // Tokens sit on the MMA's M side (128 per CTA), weight rows on its N side.  The next launch
 // is released at the start (programmatic dependent launch): weights and scales are fetched
 // while the quantiser in front still runs.  Every wait is bounded; on a timeout the kernel
