@@ -308,19 +308,28 @@ static int check_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const void* x, int 
 // Two to eight rows: whether the kernel of gemm_rows.cu (a quantiser's launch, then two latencies
 // of a group per group) is faster than the GEMV kernel on the tensor instruction (one launch; its
 // per-group work grows with the rows, four times as fast per 32 values, and with long rows its CTAs
-// are few).  us, old / new: [9728, 2560] per 32 values 2 rows 8.0 / 9.2, 4 13.5 / 9.2, 8 24.8 / 9.7,
-// per 128 4 6.9 / 8.9, 8 9.7 / 9.2; [2560, 9728] per 32 2 23.5 / 23.0, 8 66.5 / 26.6, per 128 2
-// 10.7 / 22.9, 4 25.3 / 24.0, 8 62.7 / 26.3; [2560, 4096] per 32 4 9.2 / 10.8, 8 21.0 / 11.7, per
-// 128 8 9.6 / 11.7; [19456, 2560] per 32 2 15.0 / 12.0, per 128 2 8.7 / 10.8, 4 13.0 / 10.9;
-// [20000, 1024] per 32 2 6.7 / 5.8, per 128 4 5.1 / 5.5, 8 6.6 / 5.7; [500, 512] never.
+// are few).  us, GEMV kernel / the other: per 32 values [9728, 2560] 2 rows 7.1 / 7.8, 3 7.9 / 7.8, 5
+// 18.7 / 7.8; [2560, 9728] 2 20.1 / 17.7; [1600, 6144] 4 11.2 / 11.1, 5 17.9 / 11.7; [4096, 4096] 4
+// 8.8 / 9.2, 5 17.0 / 8.9; [1600, 2048] 6 5.1 / 5.3, 7 5.6 / 5.3; [20000, 1024] 2 6.0 / 5.4;
+// [12000, 640] 8 5.0 / 4.7.  Per 128 [9728, 2560] 4 6.8 / 7.1, 5 7.7 / 7.0; [2560, 9728] 2 10.2 / 16.6,
+// 3 20.3 / 16.4; [1600, 6144] 5 11.0 / 11.2, 6 12.2 / 11.2; [2560, 4096] 6 7.9 / 8.4, 7 8.5 / 8.3;
+// [19456, 2560] 2 8.8 / 10.0, 3 11.6 / 10.1; [20000, 1024] 4 5.1 / 5.1, 5 6.1 / 5.2; [8192, 1024] never.
 static bool few_rows_streamed(const b2w4_weight* w, int m, int act_rule) {
-    if (m < 2 || w->tiles < 200)
+    const int tiles = w->tiles, groups = w->groups;
+    if (m < 2 || tiles < 200)
         return false;
-    if (act_rule == B2W4_ACT_G32)
-        return w->groups >= 48 || w->tiles >= 2048 || m >= (w->tiles >= 512 ? 3 : 5);
-    if (w->groups >= 48)
-        return m >= 4;
-    return w->tiles >= 768 && (m == 8 || (m >= 4 && w->tiles >= 2048 && w->groups >= 16));
+    if (act_rule == B2W4_ACT_G32) {
+        if (groups >= 48)
+            return m >= (tiles >= 320 ? 2 : 5);
+        if (groups < 8)
+            return m >= 7 && tiles >= 512;
+        return m >= (tiles >= 2048 ? 2 : tiles >= 768 ? 3 : tiles >= 320 ? 5 : 7);
+    }
+    if (groups >= 48)
+        return m >= (tiles >= 320 ? 3 : 6);
+    if (groups < 16)
+        return m >= 5 && tiles >= 2048 && groups >= 8;
+    return tiles >= 320 && m >= (tiles >= 2048 ? 3 : tiles >= 1024 ? 5 : 7);
 }
 
 // Up to eight activation rows stream the weight once through the GEMV kernels (one row:

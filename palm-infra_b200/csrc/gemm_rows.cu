@@ -329,15 +329,20 @@ int rows_launch_as(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
     ctx->launches++;
     return B2W4_OK;
 }
-// six stages where a CTA has the SM to itself, else three
-bool rows_deep(b2w4_ctx* ctx, const GemmRowsArgs& a, bool scl16, bool a32, int pairs_per_cta) {
+// whether a CTA has the SM to itself and room for so many stages
+bool rows_deep(b2w4_ctx* ctx, const GemmRowsArgs& a, bool scl16, bool a32, int pairs_per_cta,
+               int stages) {
     return (a.pairs + pairs_per_cta - 1) / pairs_per_cta <= ctx->sm_count &&
-           6 * rows_stage_bytes(a.m8, a32 ? 4 : 1, pairs_per_cta, scl16) <= 220 * 1024;
+           stages * rows_stage_bytes(a.m8, a32 ? 4 : 1, pairs_per_cta, scl16) <= 220 * 1024;
 }
 template <int PW, int CB, bool SCL16, bool A32>
 int rows_launch(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
-    return rows_deep(ctx, a, SCL16, A32, pairs_per_cta)
-               ? rows_launch_as<PW, CB, SCL16, A32, 6, 1>(ctx, a, pairs_per_cta)
+    // six stages, or five where six do not fit (32 rows of [9728, 2560] per 128 values: three
+    // stages 16.7 us, five 11.9), else three for two CTAs
+    if (rows_deep(ctx, a, SCL16, A32, pairs_per_cta, 6))
+        return rows_launch_as<PW, CB, SCL16, A32, 6, 1>(ctx, a, pairs_per_cta);
+    return rows_deep(ctx, a, SCL16, A32, pairs_per_cta, 5)
+               ? rows_launch_as<PW, CB, SCL16, A32, 5, 1>(ctx, a, pairs_per_cta)
                : rows_launch_as<PW, CB, SCL16, A32, 3, 1>(ctx, a, pairs_per_cta);
 }
 template <bool SCL16, bool A32>
@@ -399,7 +404,7 @@ int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
     a.pw = ncb;
     const int few = (a.pairs + ctx->sm_count - 1) / ctx->sm_count;
     if (few * ncb * 2 <= kRelayWarps && (few <= 2 || !a32 || (few > 4 && ncb == 1)) &&
-        rows_deep(ctx, a, scl16, a32, few))
+        rows_deep(ctx, a, scl16, a32, few, 6))
         return scl16 ? (a32 ? rows_relay<true, true>(ctx, a, few)
                             : rows_relay<true, false>(ctx, a, few))
                      : (a32 ? rows_relay<false, true>(ctx, a, few)

@@ -503,7 +503,8 @@ def test_few_rows_with_few_pairs_per_multiprocessor(ctx, m, pairs, k, rule):
 
 @pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
 @pytest.mark.parametrize("m,n,k", [(2, 16392, 256), (3, 4104, 512), (8, 6152, 640), (5, 1608, 384),
-                                   (2, 1608, 6272), (7, 1603, 6144)])
+                                   (2, 1608, 6272), (7, 1603, 6144), (2, 16392, 1024),
+                                   (3, 2568, 6272)])
 def test_two_to_eight_rows_on_the_streamed_kernel(ctx, m, n, k, rule):
     """Row counts and weights on which few rows take the kernel of 9 to 32 rows: a warp per pair,
     up to ten pairs per CTA."""
