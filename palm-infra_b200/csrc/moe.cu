@@ -796,7 +796,7 @@ moe_combine_staged_kernel(unsigned long long* stage, int stage_rows,
 // the dense small-batch kernel's: phase 1 integer group sums (a weight word w of 8 nibbles
 // splits into signed bytes 16 q, and an accumulator that starts at 0x49400000 ends as the bits of
 // the float 786432 + sum: no pass and no barrier for sums of codes; one token, 128 experts of
-// 768: 23.2 -> 22.4 us), phase 2 the fp32 chain per (tile, route, weight row) in ascending
+// 768: 23.2 -> 22.6 us), phase 2 the fp32 chain per (tile, route, weight row) in ascending
 // group order.
 constexpr int kSW = 8;          // warps
 constexpr int kST = kSW * 32;
@@ -877,6 +877,7 @@ moe_grouped_small_kernel(const GroupedSmallArgs a) {
                      &s_bar[0]);
         }
     }
+    __syncthreads();  // no warp polls the barrier word before it is one
     const int npair = (ntile + 1) >> 1;
     const int n_items = npair * G;
     const uint32_t* s_w32 = reinterpret_cast<const uint32_t*>(s_w);
@@ -913,7 +914,7 @@ moe_grouped_small_kernel(const GroupedSmallArgs a) {
             if (!mbar_wait_bounded(&s_bar[0])) {
                 if (lane == 0)
                     b2w4_report_timeout(a.status);
-                return;  // every thread sees the same barrier: the exit is CTA-uniform
+                return;  // this warp's rows stay unwritten; the status word says so
             }
             weights_ready = true;
         }

@@ -381,3 +381,32 @@ def test_grouped_matmul_pass_edges(ctx, t, h, inter, rule):
     want = ol.moe_forward(hidden, router, 2, inter, gu, dn, rule=rule)
     assert not (want[2] == 2).any()
     check_against_oracle(got, want)
+
+
+def test_one_token_behind_kernels_that_fill_shared_memory(ctx):
+    """The one-token expert matmul waits on a barrier word in shared memory that it makes itself:
+    whatever the kernel before left there, all ones or zeros, every call gives the same bits.
+    The shortest rows and the most warps without work reach the wait soonest."""
+    import torch
+    t, h, e, top_k, inter = 1, 128, 64, 8, 128
+    hidden = pkg.synth.activations(7, 5, t, h)
+    router = pkg.synth.router_weight(20261125, 9, e, h, std=0.3)
+    gu = pkg.synth.bg128_weight(20261125, 500, e * 2 * inter, h)
+    dn = pkg.synth.bg128_weight(20261125, 501, e * h, inter)
+    ctx.set_moe_rule(REF)
+    w_gu, w_dn = (ctx.upload_weight(gu, e * 2 * inter, h), ctx.upload_weight(dn, e * h, inter))
+    xd, rd = torch.from_numpy(hidden).cuda(), torch.from_numpy(router.view(np.int16)).cuda()
+    out = torch.zeros((40, h), device="cuda")
+    # rows whose staged codes are 0xFF / 0x7F bytes and zeros: what is left in shared memory
+    fill = ctx.upload_weight(pkg.synth.bg128_weight(3, 2, 2368, 2560), 2368, 2560)
+    xs = [torch.full((8, 2560), v, device="cuda") for v in (-1.0, 0.0, 1.0)]
+    ys = torch.zeros((8, 2368), device="cuda")
+    for i in range(out.shape[0]):
+        ctx.matmul(fill, xs[i % 3], ys, rule=ol.ACT_G128)
+        ctx.moe_forward(xd, rd, top_k, inter, w_gu, w_dn, out[i:i + 1])
+    ctx.sync()
+    for w in (w_gu, w_dn, fill):
+        w.free()
+    want = ol.moe_forward(hidden, router, top_k, inter, gu, dn, rule=REF)[0]
+    assert torch.equal(out, out[:1].expand_as(out))
+    assert rel_l2(out[0].cpu().numpy(), want[0]) < 1e-6
