@@ -696,3 +696,29 @@ def test_matmuls_that_make_their_rows(ctx, m, n, k, rule):
         ctx.sync()
         assert torch.equal(a, b) and torch.equal(got, want)
     w.free()
+
+
+@pytest.mark.parametrize("n,k", [(272, 128), (272, 2560), (4864, 4096), (272, 4224)])
+def test_step_matmul_reads_norm_weights_that_were_just_written(ctx, n, k):
+    """A norm weight made by the operator in front (1 + w, as some packages store it): read when
+    that operator is done, as b2w4_add_rms_norm reads it."""
+    import torch
+    rng = np.random.default_rng(n + k)
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, n + k, n, k), n, k)
+    x, u, g = (_dev(rng.normal(0, s, (1, k)).astype(np.float32)) for s in (2, 1, 0.2))
+    one = torch.ones((1, k), device="cuda")
+    made = [torch.zeros((1, k), device="cuda") for _ in range(12)]
+    res, hid, want_hid = (torch.zeros((1, k), device="cuda") for _ in range(3))
+    y = torch.zeros((len(made), n), device="cuda")
+    want = torch.zeros((1, n), device="cuda")
+    # (the many rows keep the kernels in front from being done early)
+    wide = [torch.zeros((4096, k), device="cuda") for _ in range(2)]
+    for i, weight in enumerate(made):
+        ctx.copy_rows(wide[0], wide[1], 4096, k)
+        ctx.add(g, one, weight)
+        ctx.step_matmul(w, x, u, weight, 1e-6, res, y=y[i:i + 1], hidden_out=hid)
+    ctx.add_rms_norm(x.clone(), u, one + g, 1e-6, want_hid)
+    ctx.matmul(w, want_hid, want, rule=ol.ACT_G128)
+    ctx.sync()
+    assert torch.equal(hid, want_hid) and torch.equal(y, want.expand_as(y))
+    w.free()
