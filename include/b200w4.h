@@ -399,13 +399,16 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      likewise
  *   b2w4_step_matmul   the matmul of a decode step with its neighbours in it (one row,
  *                      per-128 rule): v = residual (+ update, may be NULL), written to
- *                      residual_out (another buffer than either; may be NULL without
- *                      an update); h = rms_norm(v) * norm_weight, written to hidden_out
- *                      unless NULL; y = w h.  swiglu: w's rows are gate | up and y
- *                      [n / 2] = SwiGLU of them (n a multiple of 16).  token_dev
- *                      instead of y: the greedy token.  All rows 16-byte aligned.  The
- *                      same bits as b2w4_add_rms_norm, b2w4_matmul / b2w4_matmul_argmax
- *                      and b2w4_swiglu in turn
+ *                      residual_out (may be NULL without an update); h = rms_norm(v) *
+ *                      norm_weight, written to hidden_out unless NULL; y = w h.
+ *                      swiglu: w's rows are gate | up and y [n / 2] = SwiGLU of them (n a
+ *                      multiple of 16).  token_dev instead of y: the greedy token.  All
+ *                      rows 16-byte aligned.  The same bits as b2w4_add_rms_norm,
+ *                      b2w4_matmul / b2w4_matmul_argmax and b2w4_swiglu in turn.
+ *                      residual_out and hidden_out overlap neither a row that is read nor
+ *                      another output (refused), but hidden_out may be the residual or the
+ *                      update itself; y may lie over a row that is read or over
+ *                      residual_out.  Such calls take one launch more, as k > 4096 does
  *   b2w4_advance       *counter_dev += by, after history_dev[*counter_dev] = *token_dev
  *                      (both optional).  With the position on the device a decode
  *                      step is the same sequence of launches for every token and can

@@ -527,6 +527,11 @@ int b2w4_matmul_argmax(b2w4_ctx* ctx, const b2w4_weight* w, const float* x_dev, 
     return b2w4_launch_top1_token(ctx, top1.cells, token_dev, m);
 }
 
+static bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return a && b && p < q + b_bytes && q < p + a_bytes;
+}
+
 int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_dev,
                      const float* update_dev, const float* norm_weight_dev, float eps,
                      float* residual_out_dev, float* hidden_out_dev, int swiglu, float* y_dev,
@@ -539,16 +544,31 @@ int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_
     const uintptr_t all = (uintptr_t)residual_dev | (uintptr_t)update_dev |
                           (uintptr_t)norm_weight_dev | (uintptr_t)residual_out_dev |
                           (uintptr_t)hidden_out_dev;
-    if ((all & 15) || residual_out_dev == residual_dev ||
-        (update_dev && residual_out_dev == update_dev))
-        return b2w4_fail(ctx, B2W4_E_INVALID,
-                         "step_matmul: rows must be 16-byte aligned, the new residual apart");
+    if (all & 15)
+        return b2w4_fail(ctx, B2W4_E_INVALID, "step_matmul: rows must be 16-byte aligned");
+    // Rows that share memory.  In one launch some blocks still read the row while others store;
+    // with the row made first the rows read are done with before y, and hidden_out may be the
+    // very row it is made from.
+    const size_t kb = sizeof(float) * w->k;
+    const size_t yb = sizeof(float) * (swiglu ? w->n / 2 : w->n);
+    auto reads = [&](const void* p, size_t bytes) {
+        return overlap(p, bytes, residual_dev, kb) || overlap(p, bytes, update_dev, kb) ||
+               overlap(p, bytes, norm_weight_dev, kb);
+    };
+    const bool in_place =
+        hidden_out_dev && (hidden_out_dev == residual_dev || hidden_out_dev == update_dev);
+    if (reads(residual_out_dev, kb) || overlap(hidden_out_dev, kb, residual_out_dev, kb) ||
+        overlap(hidden_out_dev, kb, y_dev, yb) || (!in_place && reads(hidden_out_dev, kb)) ||
+        (in_place && overlap(hidden_out_dev, kb, norm_weight_dev, kb)))
+        return b2w4_fail(ctx, B2W4_E_INVALID, "step_matmul: rows overlap");
+    const bool row_first =
+        in_place || reads(y_dev, yb) || overlap(y_dev, yb, residual_out_dev, kb);
     b2w4_norm_args norm = {residual_dev, update_dev, norm_weight_dev, eps, residual_out_dev,
                            hidden_out_dev};
-    if (!token_dev && w->k <= kStepNormMaxK)
+    if (!token_dev && !row_first && w->k <= kStepNormMaxK)
         return b2w4_launch_gemv(ctx, w, nullptr, w->k, y_dev, w->n, 1, B2W4_ACT_G128, B2W4_NONE, 0,
                                 -1, nullptr, nullptr, nullptr, &norm, swiglu != 0);
-    // the row made first: many CTAs per SM, or more values than a CTA takes up
+    // the row made first: many CTAs per SM, more values than a CTA takes up, shared memory
     int rc = B2W4_OK;
     void* hidden = hidden_out_dev;
     if (!hidden && (rc = b2w4_reserve(ctx, SCR_STAGE_X, sizeof(float) * w->k, &hidden)) != B2W4_OK)

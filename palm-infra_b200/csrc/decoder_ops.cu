@@ -1515,13 +1515,13 @@ int launch_tile(b2w4_ctx* ctx, const AttnArgs& a, int dim, const AttnPlan& plan,
 }  // namespace
 
 int b2w4_launch_step_norm(b2w4_ctx* ctx, const b2w4_norm_args& n, int k, float* hidden) {
+    if (!n.update && n.residual_out)  // first: hidden may be the residual itself
+        B2W4_CUDA(ctx, cudaMemcpyAsync(n.residual_out, n.residual, sizeof(float) * k,
+                                       cudaMemcpyDeviceToDevice, ctx->stream));
     B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, rms_norm_kernel, dim3(1), dim3(kNormThreads), 0,
                                        ctx->stream, n.residual, k, n.update, k, n.residual_out, k,
                                        n.weight, n.eps, hidden, k));
     ctx->launches++;
-    if (!n.update && n.residual_out)
-        B2W4_CUDA(ctx, cudaMemcpyAsync(n.residual_out, n.residual, sizeof(float) * k,
-                                       cudaMemcpyDeviceToDevice, ctx->stream));
     return B2W4_OK;
 }
 

@@ -722,3 +722,61 @@ def test_step_matmul_reads_norm_weights_that_were_just_written(ctx, n, k):
     ctx.sync()
     assert torch.equal(hid, want_hid) and torch.equal(y, want.expand_as(y))
     w.free()
+
+
+@pytest.mark.parametrize("where", ["residual", "update", "both", "weight", "new residual",
+                                   "half", "in place", "in place of update"])
+@pytest.mark.parametrize("k", [2560, 4224])
+def test_step_matmul_outputs_over_rows_that_are_read(ctx, k, where):
+    """y over the rows the call reads (the very row, the end of one and the start of the next, or
+    its second half), over the new residual, and the normalised row in the place of the one it is
+    made from: the operators in turn, whose inputs are read before their outputs are stored."""
+    import torch
+    n = k
+    rng = np.random.default_rng(k)
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, n + k, n, k), n, k)
+    first = rng.normal(0, 1, (5, k)).astype(np.float32)  # residual, update, weight, new, spare
+    rows = _dev(first)
+    x, u, g, res, spare = (rows[i:i + 1] for i in range(5))
+    flat = rows.view(-1)
+    y = {"residual": x, "update": u, "weight": g, "new residual": res,
+         "both": flat[k // 2:k // 2 + n].view(1, n), "half": flat[3 * k // 2:][:n].view(1, n),
+         "in place": spare, "in place of update": spare}[where]
+    hid = {"in place": x, "in place of update": u}.get(where)
+    want_res, want_hid = _dev(first[:1]), torch.zeros((1, k), device="cuda")
+    want = torch.zeros((1, n), device="cuda")
+    ctx.add_rms_norm(want_res, _dev(first[1:2]), _dev(first[2:3]), 1e-6, want_hid)
+    ctx.matmul(w, want_hid, want, rule=ol.ACT_G128)
+    ctx.step_matmul(w, x, u, g, 1e-6, res, y=y, hidden_out=hid)
+    ctx.sync()
+    assert torch.equal(y, want)
+    if where != "new residual":
+        assert torch.equal(res, want_res)
+    if hid is not None:
+        assert torch.equal(hid, want_hid)
+    w.free()
+
+
+@pytest.mark.parametrize("k", [128, 4224])
+def test_step_matmul_refuses_rows_that_overlap(ctx, k):
+    """The new residual over a part of a row that is read, the normalised row over another output
+    or over a part of a row that is read."""
+    import torch
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, 1, 24, k), 24, k)
+    rows = torch.ones(8 * k, device="cuda")
+    row = lambda at: rows[at:at + k].view(1, k)
+    x, u, g, r = (row(i * k) for i in range(4))
+    y = torch.zeros((1, 24), device="cuda")
+    for kw in (dict(residual_out=row(4), y=y), dict(residual_out=row(2 * k - 4), y=y),
+               dict(residual_out=row(2 * k), y=y),
+               dict(residual_out=r, y=y, hidden_out=row(4)),
+               dict(residual_out=r, y=y, hidden_out=row(k + 4)),
+               dict(residual_out=r, y=y, hidden_out=g),
+               dict(residual_out=r, y=y, hidden_out=r),
+               dict(residual_out=r, y=y, hidden_out=row(4 * k - 4)),
+               dict(residual_out=r, y=rows[5 * k:5 * k + 24].view(1, 24), hidden_out=row(5 * k))):
+        with pytest.raises(pkg.capi.B200W4Error, match="overlap"):
+            ctx.step_matmul(w, x, u, g, 1e-6, **kw)
+    ctx.step_matmul(w, x, u, g, 1e-6, r, y=y, hidden_out=row(4 * k))  # side by side: accepted
+    ctx.sync()
+    w.free()
