@@ -202,6 +202,7 @@ struct b2w4_norm_args {
     float eps;
     float *residual_out, *hidden_out;
 };
+constexpr int kNormWarpMaxK = 256;   // b2w4_rms_norm: rows up to here are summed by one warp
 constexpr int kStepNormMaxK = 4096;  // longest row that the GEMV kernel makes itself
 // the same as a launch of its own (decoder_ops.cu); hidden instead of hidden_out
 int b2w4_launch_step_norm(b2w4_ctx* ctx, const b2w4_norm_args& norm, int k, float* hidden);

@@ -381,7 +381,8 @@ int b2w4_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* x_dev, int lda
 static int matmul_rows(b2w4_ctx* ctx, const b2w4_weight* w, const b2w4_rows& from, float* y,
                        int ldc, int m, int act_rule) {
     // (the norm's quantiser keeps a row in shared memory, and adds as the operator's block does)
-    const bool made = from.kind == b2w4_rows::SWIGLU || (w->k <= kRowsNormMaxK && w->k > 256);
+    const bool made =
+        from.kind == b2w4_rows::SWIGLU || (w->k <= kRowsNormMaxK && w->k > kNormWarpMaxK);
     if (made && m > ctx->gemv_max_rows && ctx->gemm_kind == 0) {
         if (m <= 32)
             return b2w4_launch_gemm_rows(ctx, w, nullptr, 0, y, ldc, m, act_rule, B2W4_NONE, 0, -1,
@@ -565,10 +566,11 @@ int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_
         in_place || reads(y_dev, yb) || overlap(y_dev, yb, residual_out_dev, kb);
     b2w4_norm_args norm = {residual_dev, update_dev, norm_weight_dev, eps, residual_out_dev,
                            hidden_out_dev};
-    if (!token_dev && !row_first && w->k <= kStepNormMaxK)
+    // (a row of up to 256 values alone is summed by one warp, as b2w4_rms_norm does)
+    if (!token_dev && !row_first && w->k <= kStepNormMaxK && (update_dev || w->k > kNormWarpMaxK))
         return b2w4_launch_gemv(ctx, w, nullptr, w->k, y_dev, w->n, 1, B2W4_ACT_G128, B2W4_NONE, 0,
                                 -1, nullptr, nullptr, nullptr, &norm, swiglu != 0);
-    // the row made first: many CTAs per SM, more values than a CTA takes up, shared memory
+    // the row made first: many CTAs per SM, more values than a CTA takes up, shared memory, short
     int rc = B2W4_OK;
     void* hidden = hidden_out_dev;
     if (!hidden && (rc = b2w4_reserve(ctx, SCR_STAGE_X, sizeof(float) * w->k, &hidden)) != B2W4_OK)

@@ -1518,6 +1518,8 @@ int b2w4_launch_step_norm(b2w4_ctx* ctx, const b2w4_norm_args& n, int k, float* 
     if (!n.update && n.residual_out)  // first: hidden may be the residual itself
         B2W4_CUDA(ctx, cudaMemcpyAsync(n.residual_out, n.residual, sizeof(float) * k,
                                        cudaMemcpyDeviceToDevice, ctx->stream));
+    if (!n.update)
+        return b2w4_rms_norm(ctx, n.residual, k, 1, k, n.weight, n.eps, hidden, k);
     B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, rms_norm_kernel, dim3(1), dim3(kNormThreads), 0,
                                        ctx->stream, n.residual, k, n.update, k, n.residual_out, k,
                                        n.weight, n.eps, hidden, k));
@@ -1533,7 +1535,7 @@ int b2w4_rms_norm(b2w4_ctx* ctx, const float* x_dev, int ldx, int rows, int dim,
         return B2W4_E_INVALID;
     if (!x_dev || !weight_dev || !out_dev || rows <= 0 || dim <= 0 || ldx < dim || ldo < dim)
         return b2w4_fail(ctx, B2W4_E_INVALID, "rms_norm: bad argument");
-    if (dim <= 256) {
+    if (dim <= kNormWarpMaxK) {
         const size_t threads = (size_t)rows * 32;
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, rms_norm_warp_kernel,
                                            dim3((unsigned)((threads + 255) / 256)), dim3(256), 0,

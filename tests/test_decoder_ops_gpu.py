@@ -780,3 +780,26 @@ def test_step_matmul_refuses_rows_that_overlap(ctx, k):
     ctx.step_matmul(w, x, u, g, 1e-6, r, y=y, hidden_out=row(4 * k))  # side by side: accepted
     ctx.sync()
     w.free()
+
+
+@pytest.mark.parametrize("k", [128, 256, 384])
+def test_step_matmul_of_a_short_row_alone(ctx, k):
+    """No update: the sum of squares in b2w4_rms_norm's order, one warp up to 256 values."""
+    import torch
+    n = 64
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, n + k, n, k), n, k)
+    rng = np.random.default_rng(k)
+    for _ in range(20):
+        x, g = (_dev(rng.normal(0, 1, (1, k)).astype(np.float32)) for _ in range(2))
+        hid, hid_t, res, want_hid = (torch.zeros((1, k), device="cuda") for _ in range(4))
+        y, want = (torch.zeros((1, n), device="cuda") for _ in range(2))
+        tok, want_tok = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+        ctx.step_matmul(w, x, None, g, 1e-6, res, y=y, hidden_out=hid)
+        ctx.step_matmul(w, x, None, g, 1e-6, None, tokens=tok, hidden_out=hid_t)
+        ctx.rms_norm(x, g, 1e-6, want_hid)
+        ctx.matmul(w, want_hid, want, rule=ol.ACT_G128)
+        ctx.matmul_argmax(w, want_hid, want_tok)
+        ctx.sync()
+        assert torch.equal(hid, want_hid) and torch.equal(hid_t, want_hid)
+        assert torch.equal(y, want) and torch.equal(tok, want_tok) and torch.equal(res, x)
+    w.free()
