@@ -175,7 +175,9 @@ class DenseDecoder:
         if not cfg.experts:
             gu, act = self._b("gu", T, 2 * cfg.intermediate), self._b("act", T, cfg.intermediate)
         dn = self._b("dn", T, H)
-        fused = self.fused_step  # norms and SwiGLU made by the matmuls' quantisers
+        # norms and SwiGLU made by the matmuls' quantisers; up to eight rows have none, and the
+        # operators in turn then use the decoder's buffers instead of the context's scratch
+        fused = self.fused_step and T > 8
         c.embed_rows(self.embed, ids_dev, x)
         if not fused:
             c.rms_norm(x, self.layers[0]["ln1"], cfg.eps, h)
@@ -233,6 +235,9 @@ class DenseDecoder:
         # while the first of them writes the new one
         x, x_new = self._b("x", 1, H), self._b("x_new", 1, H)
         h, o, dn = self._b("h", 1, H), self._b("o", 1, H), self._b("dn", 1, H)
+        # rows that the matmul does not make inside: into the decoder's own buffer, because a
+        # captured step outlives the context's scratch
+        made = h if H > capi.STEP_ROW_MAX or H <= capi.STEP_ROW_MIN else None
         qkv = self._b("qkv", 1, cfg.q_dim + 2 * cfg.kv_dim)
         q, attn = self._b("q", 1, cfg.q_dim), self._b("attn", 1, cfg.q_dim)
         act = None if cfg.experts else self._b("act", 1, inter)
@@ -240,7 +245,7 @@ class DenseDecoder:
         update = None
         for L in self.layers:
             c.step_matmul(L["qkv"], x, update, L["ln1"], cfg.eps,
-                          None if update is None else x_new, y=qkv)
+                          None if update is None else x_new, y=qkv, hidden_out=made)
             if update is not None:
                 x, x_new = x_new, x
             c.attention_step(qkv, cfg.heads, cfg.kv_heads, D, L["q_norm"], L["k_norm"], cfg.eps,
@@ -251,7 +256,8 @@ class DenseDecoder:
                 c.add_rms_norm(x, o, L["ln2"], cfg.eps, h)
                 c.moe_forward(h, L["router"], cfg.top_k, inter, L["gate_up"], L["down"], dn)
             else:
-                c.step_matmul(L["gate_up"], x, o, L["ln2"], cfg.eps, x_new, y=act, swiglu=True)
+                c.step_matmul(L["gate_up"], x, o, L["ln2"], cfg.eps, x_new, y=act, swiglu=True,
+                              hidden_out=made)
                 x, x_new = x_new, x
                 c.matmul(L["down"], act, dn, rule=capi.ACT_G128)
             update = dn

@@ -84,3 +84,37 @@ def test_mixture_of_experts_decoder_tokens_identical(layers, hidden, heads, kv_h
     assert got == want, (got, want, margins)
     assert replayed == want, (replayed, want)
     assert min(margins) > 1e-2
+
+
+@pytest.mark.parametrize("hidden", [256, 2560, 4224])
+def test_captured_step_outlives_grown_scratch(hidden):
+    """A step captured behind one prompt and replayed behind another, of two to eight tokens, and
+    after a matmul that needs far more of the context's scratch: rows that the step's matmuls
+    cannot make inside (more than 4096 values) are in the decoder's own buffers."""
+    import torch
+    dec = pkg.decoder
+    cfg = dec.DecoderConfig(2, hidden, 4, 2, 128, 1024, 2048)
+    weights = dec.synthetic_weights(cfg, seed=hidden)
+    rng = np.random.default_rng(hidden)
+    prompts = [rng.integers(0, 2048, n).tolist() for n in (9, 5, 2)]
+    ctx = pkg.capi.Context(0)
+    model = dec.DenseDecoder(ctx, cfg, weights, capacity=40)
+    want = [model.generate(p, 8) for p in prompts]
+    model.free()
+    ctx.close()
+    ctx = pkg.capi.Context(0)
+    model = dec.DenseDecoder(ctx, cfg, weights, capacity=40)
+    w = ctx.upload_weight(pkg.synth.bg128_weight(3, 1, 256, 9728), 256, 9728)
+    got = []
+    for i, p in enumerate(prompts):
+        got.append(model.generate(p, 8, replay=True))  # captured with the first prompt
+        rows = 300 * (i + 1)
+        merged = torch.randn((rows, 2 * 9728), device="cuda")
+        ctx.matmul_swiglu(w, merged, torch.zeros((rows, 256), device="cuda"))
+        x = torch.randn((8, 9728), device="cuda")
+        ctx.matmul_norm(w, x, None, torch.ones(9728, device="cuda"), 1e-6,
+                        torch.zeros((8, 256), device="cuda"))
+    w.free()
+    model.free()
+    ctx.close()
+    assert got == want
