@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 
 #include "b200w4.h"
 
@@ -48,6 +49,15 @@ struct b2w4_ctx {
     // grow-only scratch (quantised activations, MoE work lists, staging)
     void* scratch[8] = {nullptr};
     size_t scratch_cap[8] = {0};
+    // Quantised rows of calls of two to eight rows (gemm_rows.cu): buffers made with the context,
+    // one per stream that has such calls, so that these calls share nothing with calls on other
+    // streams and no address that a graph could hold is ever given back
+    static constexpr int kFewStreams = 8;
+    static constexpr size_t kFewBytes = 128 * 1024;
+    void* few_rows = nullptr;
+    unsigned long long few_stream[kFewStreams] = {};  // stream ids
+    int few_used = 0;
+    std::mutex few_lock;  // one quantiser and its matmul at a time
     int* flag_dev = nullptr;  // device words: arrival counters, greedy-token cells
     // The status word a kernel sets when a bounded wait gives up lives in mapped pinned HOST
     // memory: the host reads it after a stream synchronise with no copy.  status_dev is the
@@ -121,10 +131,12 @@ bool b2w4_gemm_mma_resident(const b2w4_weight* w, int m, int act_rule, int sm_co
 int b2w4_launch_gemm_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                          float* y, int ldc, int m, int act_rule, int activation,
                          int act_n_begin, int act_n_len);
-// 9..32 rows (gemm_rows.cu)
+// 2..32 rows (gemm_rows.cu); own: b2w4_rows_scratch bytes for the quantised rows, else the
+// context's scratch takes them
+size_t b2w4_rows_scratch(const b2w4_weight* w, int m, int act_rule);
 int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
                           int ldc, int m, int act_rule, int activation, int act_n_begin,
-                          int act_n_len, const b2w4_rows* from = nullptr);
+                          int act_n_len, const b2w4_rows* from = nullptr, void* own = nullptr);
 int b2w4_launch_quantize_mma(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,
                              int act_rule, int8_t* q, float* scales_t, int32_t* es_t);
 int b2w4_launch_quantize_rows(b2w4_ctx* ctx, const float* x, int lda, int m, int k, int m_pad,

@@ -106,7 +106,9 @@ int b2w4_ctx_create(int device, b2w4_ctx** out) {
     if (gmr && atoi(gmr) > 0)
         ctx->gemv_max_rows = atoi(gmr);
     if (cudaMalloc(reinterpret_cast<void**>(&ctx->flag_dev), 256) != cudaSuccess ||
-        cudaMemset(ctx->flag_dev, 0, 256) != cudaSuccess) {
+        cudaMemset(ctx->flag_dev, 0, 256) != cudaSuccess ||
+        cudaMalloc(&ctx->few_rows, ctx->kFewStreams * ctx->kFewBytes) != cudaSuccess) {
+        cudaFree(ctx->flag_dev);
         delete ctx;
         return B2W4_E_NOMEM;
     }
@@ -116,6 +118,7 @@ int b2w4_ctx_create(int device, b2w4_ctx** out) {
                                  0) != cudaSuccess) {
         if (ctx->status_host)
             cudaFreeHost(ctx->status_host);
+        cudaFree(ctx->few_rows);
         cudaFree(ctx->flag_dev);
         delete ctx;
         return B2W4_E_NOMEM;
@@ -135,6 +138,7 @@ void b2w4_ctx_destroy(b2w4_ctx* ctx) {
             cudaFree(ctx->scratch[i]);
     if (ctx->flag_dev)
         cudaFree(ctx->flag_dev);
+    cudaFree(ctx->few_rows);
     if (ctx->status_host)
         cudaFreeHost(ctx->status_host);
     delete ctx;
@@ -332,6 +336,34 @@ static bool few_rows_streamed(const b2w4_weight* w, int m, int act_rule) {
     return tiles >= 320 && m >= (tiles >= 2048 ? 3 : tiles >= 1024 ? 5 : 7);
 }
 
+// The buffer for quantised rows of the context's stream, or null: a capture (its graph may be
+// replayed beside any other call, and outlives what it would hold), rows too long, or more streams
+// than buffers.  The GEMV kernels need none.  Streams are told apart by their id, which is never
+// used twice.  (What a capture pays for that, us in a graph, GEMV kernel / streamed: [9728, 2560]
+// per 32 values 4 rows 8.2 / 7.6, 8 rows 21.8 / 7.7, per 128 8 rows 9.0 / 6.9; [2560, 9728] per 128
+// 8 rows 58 / 18.)
+static void* few_rows_buffer(b2w4_ctx* ctx, size_t bytes) {
+    cudaStreamCaptureStatus capture;
+    unsigned long long id;
+    if (bytes > ctx->kFewBytes)
+        return nullptr;
+    cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
+    if (e == cudaSuccess && capture != cudaStreamCaptureStatusNone)
+        return nullptr;
+    if (e != cudaSuccess || cudaStreamGetId(ctx->stream, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    int i = 0;
+    while (i < ctx->few_used && ctx->few_stream[i] != id)
+        ++i;
+    if (i == ctx->kFewStreams)
+        return nullptr;
+    if (i == ctx->few_used)
+        ctx->few_stream[ctx->few_used++] = id;
+    return static_cast<uint8_t*>(ctx->few_rows) + i * ctx->kFewBytes;
+}
+
 // Up to eight activation rows stream the weight once through the GEMV kernels (one row:
 // dp4a; two to eight: the warp-level int8 tensor instruction) or, as up to 32 rows do, through
 // the kernel of gemm_rows.cu; more rows go to the tcgen05 kernels (K <= 10240).  All produce the same bits for
@@ -342,10 +374,16 @@ static int matmul_dispatch(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, 
     const bool rows = m > ctx->gemv_max_rows;
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (lda & 3) == 0;
     const bool tc = rows && w->groups <= 80;
-    if (m <= 32 && ctx->gemm_kind == 0 &&
-        (rows || (ctx->gemv_max_rows == 8 && few_rows_streamed(w, m, act_rule))))
+    if (m <= 32 && ctx->gemm_kind == 0 && rows)
         return b2w4_launch_gemm_rows(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
                                      act_n_len);
+    if (!rows && ctx->gemm_kind == 0 && ctx->gemv_max_rows == 8 &&
+        few_rows_streamed(w, m, act_rule)) {
+        std::lock_guard<std::mutex> lock(ctx->few_lock);
+        if (void* own = few_rows_buffer(ctx, b2w4_rows_scratch(w, m, act_rule)))
+            return b2w4_launch_gemm_rows(ctx, w, x, lda, y, ldc, m, act_rule, activation,
+                                         act_n_begin, act_n_len, nullptr, own);
+    }
     // mma.sync with the weights in shared memory (its quantiser needs aligned rows): when asked
     // for, when the tensor-core kernel cannot take the call, or, under the per-128 rule, for
     // weights whose CTAs are all resident at once

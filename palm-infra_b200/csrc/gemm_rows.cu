@@ -354,15 +354,22 @@ int rows_relay(b2w4_ctx* ctx, const GemmRowsArgs& a, int pairs_per_cta) {
 
 }  // namespace
 
+size_t b2w4_rows_scratch(const b2w4_weight* w, int m, int act_rule) {
+    const int spg = act_rule == B2W4_ACT_G32 ? 4 : 1, m8 = (m + 7) & ~7;
+    return (size_t)m * w->k + sizeof(float) * w->groups * spg * m8;
+}
+
 int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
                           int ldc, int m, int act_rule, int activation, int act_n_begin,
-                          int act_n_len, const b2w4_rows* from) {
+                          int act_n_len, const b2w4_rows* from, void* own) {
     const bool a32 = act_rule == B2W4_ACT_G32;
     const int G = w->groups, spg = a32 ? 4 : 1, m8 = (m + 7) & ~7;
-    void *qa = nullptr, *sc = nullptr;
+    void *qa = own, *sc = nullptr;
     int rc;
-    if ((rc = b2w4_reserve(ctx, SCR_QA, (size_t)m * w->k, &qa)) != B2W4_OK ||
-        (rc = b2w4_reserve(ctx, SCR_AS, sizeof(float) * G * spg * m8, &sc)) != B2W4_OK)
+    if (own)  // k is whole groups of 128: the scales stay aligned
+        sc = static_cast<uint8_t*>(own) + (size_t)m * w->k;
+    else if ((rc = b2w4_reserve(ctx, SCR_QA, (size_t)m * w->k, &qa)) != B2W4_OK ||
+             (rc = b2w4_reserve(ctx, SCR_AS, sizeof(float) * G * spg * m8, &sc)) != B2W4_OK)
         return rc;
     float* as_t = static_cast<float*>(sc);
     if ((rc = b2w4_launch_quantize_rows(ctx, x, lda, m, w->k, m8, act_rule,

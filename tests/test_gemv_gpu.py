@@ -512,3 +512,88 @@ def test_two_to_eight_rows_on_the_streamed_kernel(ctx, m, n, k, rule):
     x = pkg.synth.activations(7, m + 17, m, k)
     y, _ = run_gpu(ctx, blocks, n, k, x, rule=rule, sums=False, pad=4 if n % 16 else 0)
     assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=rule).tobytes()
+
+
+# (rows, weight, rule) that the streamed kernel of gemm_rows.cu takes below nine rows
+STREAMED = [(2, 9728, 6272, ol.ACT_G32), (4, 9728, 2560, ol.ACT_G32), (8, 9728, 2560, ol.ACT_G128)]
+
+
+def _launches_of(ctx, call):
+    before = ctx.launches
+    call()
+    return ctx.launches - before
+
+
+@pytest.mark.parametrize("m,n,k,rule", STREAMED)
+def test_few_rows_captured_hold_no_scratch(m, n, k, rule):
+    """Two to eight rows as a context's very first matmul, inside a capture; then calls that need
+    far more of the context's scratch; then the graph again, on other rows.  What a graph holds
+    must be neither grown nor freed: the captured call is one launch that quantises inside."""
+    import torch
+    blocks = pkg.synth.bg128_weight(20261125, n + k + m, n, k)
+    ctx = pkg.capi.Context(0)
+    w = ctx.upload_weight(blocks, n, k)
+    xs = [pkg.synth.activations(7, i, m, k) for i in (1, 2)]
+    x, y = torch.from_numpy(xs[0]).cuda(), torch.zeros((m, n), device="cuda")
+    torch.cuda.synchronize()
+    side, other, g = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    x2, y2 = x.clone(), torch.zeros_like(y)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(g, stream=side):
+            ctx.set_stream(side.cuda_stream)
+            assert _launches_of(ctx, lambda: ctx.matmul(w, x, y, rule=rule)) == 1
+            # on another stream while the capture is open: not captured, and does not spoil it
+            ctx.set_stream(other.cuda_stream)
+            assert _launches_of(ctx, lambda: ctx.matmul(w, x2, y2, rule=rule)) == 2
+    ctx.sync()
+    want = ol.matmul_w4(blocks, n, k, xs[0], rule=rule)
+    assert y2.cpu().numpy().tobytes() == want.tobytes() and not y.any()
+    ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+    for rows in (9, 40, 700):
+        big = torch.randn((rows, k), device="cuda")
+        for r in (ol.ACT_G32, ol.ACT_G128):
+            ctx.matmul(w, big, torch.zeros((rows, n), device="cuda"), rule=r)
+    ctx.sync()
+    for host in xs:
+        x.copy_(torch.from_numpy(host))
+        g.replay()
+        torch.cuda.synchronize()
+        want = ol.matmul_w4(blocks, n, k, host, rule=rule)
+        assert y.cpu().numpy().tobytes() == want.tobytes()
+    w.free()
+    ctx.close()
+
+
+@pytest.mark.parametrize("m,n,k,rule", STREAMED)
+def test_few_rows_on_several_streams(m, n, k, rule):
+    """One context used on ten streams in turn, nothing ordered between them: every call's rows are
+    its own.  Eight streams have buffers (a quantiser's launch and the matmul's), the others take
+    the kernel that quantises inside."""
+    import torch
+    blocks = pkg.synth.bg128_weight(20261125, n + k + m, n, k)
+    ctx = pkg.capi.Context(0)
+    w = ctx.upload_weight(blocks, n, k)
+    streams = [torch.cuda.Stream() for _ in range(10)]
+    xs = torch.randn((len(streams), m, k), device="cuda") * torch.arange(
+        1, len(streams) + 1, device="cuda").view(-1, 1, 1)
+    want, ys = (torch.zeros((len(streams), m, n), device="cuda") for _ in range(2))
+    assert len({s.cuda_stream for s in streams}) == len(streams)
+    ctx.set_stream(0)
+    for i in range(len(streams)):  # one row after another
+        for r in range(m):
+            ctx.matmul(w, xs[i, r:r + 1], want[i, r:r + 1], rule=rule)
+    ctx.sync()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        ys.zero_()
+        torch.cuda.synchronize()
+        for i, s in enumerate(streams):
+            ctx.set_stream(s.cuda_stream)
+            assert _launches_of(ctx, lambda: ctx.matmul(w, xs[i], ys[i], rule=rule)) == (
+                2 if i < 8 else 1)
+        torch.cuda.synchronize()
+        assert torch.equal(ys, want)
+    ctx.set_stream(0)
+    w.free()
+    ctx.close()
