@@ -391,6 +391,7 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      block makes the query rows it needs, the one with the last key
  *                      writes the new cache rows.  The same bits as the two calls;
  *                      q_work_dev [heads * dim] is used where they are made after all
+ *                      (an out that lies over qkv, too)
  *   b2w4_matmul_norm   b2w4_add_rms_norm (update NULL: b2w4_rms_norm) and b2w4_matmul of
  *                      its result, which is quantised as it is made and not written;
  *                      the residual is updated in place.  The same bits as the two

@@ -80,6 +80,11 @@ enum ScratchSlot {
 int b2w4_fail(b2w4_ctx* ctx, int code, const char* fmt, ...);
 int b2w4_reserve(b2w4_ctx* ctx, int slot, size_t bytes, void** out);
 
+inline bool b2w4_overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return a && b && p < q + b_bytes && q < p + a_bytes;
+}
+
 #define B2W4_CUDA(ctx, call)                                                      \
     do {                                                                          \
         cudaError_t e__ = (call);                                                 \

@@ -566,11 +566,6 @@ int b2w4_matmul_argmax(b2w4_ctx* ctx, const b2w4_weight* w, const float* x_dev, 
     return b2w4_launch_top1_token(ctx, top1.cells, token_dev, m);
 }
 
-static bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
-    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
-    return a && b && p < q + b_bytes && q < p + a_bytes;
-}
-
 int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_dev,
                      const float* update_dev, const float* norm_weight_dev, float eps,
                      float* residual_out_dev, float* hidden_out_dev, int swiglu, float* y_dev,
@@ -591,17 +586,17 @@ int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_
     const size_t kb = sizeof(float) * w->k;
     const size_t yb = sizeof(float) * (swiglu ? w->n / 2 : w->n);
     auto reads = [&](const void* p, size_t bytes) {
-        return overlap(p, bytes, residual_dev, kb) || overlap(p, bytes, update_dev, kb) ||
-               overlap(p, bytes, norm_weight_dev, kb);
+        return b2w4_overlap(p, bytes, residual_dev, kb) || b2w4_overlap(p, bytes, update_dev, kb) ||
+               b2w4_overlap(p, bytes, norm_weight_dev, kb);
     };
     const bool in_place =
         hidden_out_dev && (hidden_out_dev == residual_dev || hidden_out_dev == update_dev);
-    if (reads(residual_out_dev, kb) || overlap(hidden_out_dev, kb, residual_out_dev, kb) ||
-        overlap(hidden_out_dev, kb, y_dev, yb) || (!in_place && reads(hidden_out_dev, kb)) ||
-        (in_place && overlap(hidden_out_dev, kb, norm_weight_dev, kb)))
+    if (reads(residual_out_dev, kb) || b2w4_overlap(hidden_out_dev, kb, residual_out_dev, kb) ||
+        b2w4_overlap(hidden_out_dev, kb, y_dev, yb) || (!in_place && reads(hidden_out_dev, kb)) ||
+        (in_place && b2w4_overlap(hidden_out_dev, kb, norm_weight_dev, kb)))
         return b2w4_fail(ctx, B2W4_E_INVALID, "step_matmul: rows overlap");
     const bool row_first =
-        in_place || reads(y_dev, yb) || overlap(y_dev, yb, residual_out_dev, kb);
+        in_place || reads(y_dev, yb) || b2w4_overlap(y_dev, yb, residual_out_dev, kb);
     b2w4_norm_args norm = {residual_dev, update_dev, norm_weight_dev, eps, residual_out_dev,
                            hidden_out_dev};
     // (a row of up to 256 values alone is summed by one warp, as b2w4_rms_norm does)

@@ -1729,8 +1729,12 @@ int b2w4_attention_step(b2w4_ctx* ctx, const float* qkv_dev, int heads, int kv_h
     const AttnPlan plan = attn_plan(1, heads, kv_heads, dim, past_dev ? capacity - 1 : past,
                                     capacity, aligned, !ctx->attn_tiles, ctx->attn_cluster,
                                     ctx->sm_count);
+    // out over the rows: blocks would store it while others still read theirs
+    const bool apart = !b2w4_overlap(out_dev, sizeof(float) * heads * dim, qkv_dev,
+                                     sizeof(float) * (heads + 2 * kv_heads) * dim);
     // the refusal of long caches is b2w4_attention's, in every form
-    if (plan.form == ATTN_SPLIT && sizeof(float) * (((keys + 3) & ~3) + kAttnStage) <= 200 * 1024) {
+    if (apart && plan.form == ATTN_SPLIT &&
+        sizeof(float) * (((keys + 3) & ~3) + kAttnStage) <= 200 * 1024) {
         const PrepArgs prep = {qkv_dev, q_weight_dev, k_weight_dev, cos_dev, sin_dev,
                                eps,     k_cache_dev,  v_cache_dev};
         const AttnArgs a = {nullptr, k_cache_dev, v_cache_dev, out_dev,  1,     heads,

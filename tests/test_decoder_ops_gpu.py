@@ -803,3 +803,31 @@ def test_step_matmul_of_a_short_row_alone(ctx, k):
         assert torch.equal(hid, want_hid) and torch.equal(hid_t, want_hid)
         assert torch.equal(y, want) and torch.equal(tok, want_tok) and torch.equal(res, x)
     w.free()
+
+
+@pytest.mark.parametrize("past,heads,kv_heads,dim", [(40, 4, 2, 128), (1000, 32, 8, 128),
+                                                     (300, 6, 6, 64)])
+@pytest.mark.parametrize("at", [0, 64])
+def test_attention_step_over_its_own_rows(ctx, past, heads, kv_heads, dim, at):
+    """The result in the place of the query rows, or over the later ones and the keys, as the two
+    calls allow: they have read every row before the first value is stored."""
+    import torch
+    rng = np.random.default_rng(past + dim + at)
+    cap = past + 70
+    first = rng.normal(0, 1, (1, (heads + 2 * kv_heads) * dim)).astype(np.float32)
+    qw, kw = (_dev(rng.normal(1, 0.1, dim).astype(np.float32)) for _ in range(2))
+    cos, sin = (_dev(t) for t in pkg.decoder.rope_tables(range(cap), dim, 1e6))
+    first_kv = [rng.normal(0, 1, (kv_heads, cap, dim)).astype(np.float32) for _ in range(2)]
+    want_kv, cache = [_dev(c) for c in first_kv], [_dev(c) for c in first_kv]
+    q, want = (torch.zeros((1, heads * dim), device="cuda") for _ in range(2))
+    ctx.qkv_prepare(_dev(first), 1, heads, kv_heads, dim, qw, kw, 1e-6, cos, sin, past, q,
+                    *want_kv, cap)
+    ctx.attention(q, None, None, *want_kv, want, 1, heads, kv_heads, dim, past, cap, dim ** -0.5)
+    qkv = _dev(first)
+    out = qkv.view(-1)[at:at + heads * dim].view(1, -1)
+    ctx.attention_step(qkv, heads, kv_heads, dim, qw, kw, 1e-6, cos, sin, past,
+                       torch.zeros_like(q), *cache, out, cap, dim ** -0.5)
+    ctx.sync()
+    for a, b in zip(cache, want_kv):
+        assert torch.equal(a, b)
+    assert torch.equal(out, want)
