@@ -364,6 +364,18 @@ static void* few_rows_buffer(b2w4_ctx* ctx, size_t bytes) {
     return static_cast<uint8_t*>(ctx->few_rows) + i * ctx->kFewBytes;
 }
 
+// How long a row may be: for more than eight (gemv_max_rows) the tcgen05 kernels' limit or, where
+// rows are aligned, that of the mma.sync kernel, if either is beyond the GEMV kernels'; else theirs.
+// The streamed kernel has no limit, but takes calls of the others on some weights only: it takes
+// what they take, so that a row's length is accepted or not whatever the number of weight rows.
+static bool matmul_accepts(const b2w4_ctx* ctx, const b2w4_weight* w, int m, int act_rule,
+                           bool aligned) {
+    if (m > ctx->gemv_max_rows &&
+        (w->groups <= 80 || (aligned && b2w4_gemm_mma_fits(w, m, act_rule))))
+        return true;
+    return b2w4_gemv_fits(w, m, act_rule);
+}
+
 // Up to eight activation rows stream the weight once through the GEMV kernels (one row:
 // dp4a; two to eight: the warp-level int8 tensor instruction) or, as up to 32 rows do, through
 // the kernel of gemm_rows.cu; more rows go to the tcgen05 kernels (K <= 10240).  All produce the same bits for
@@ -374,6 +386,8 @@ static int matmul_dispatch(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, 
     const bool rows = m > ctx->gemv_max_rows;
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (lda & 3) == 0;
     const bool tc = rows && w->groups <= 80;
+    if (!matmul_accepts(ctx, w, m, act_rule, vec))
+        return b2w4_fail(ctx, B2W4_E_INVALID, "matmul: K=%d is too long for %d rows", w->k, m);
     if (m <= 32 && ctx->gemm_kind == 0 && rows)
         return b2w4_launch_gemm_rows(ctx, w, x, lda, y, ldc, m, act_rule, activation, act_n_begin,
                                      act_n_len);
@@ -418,6 +432,8 @@ int b2w4_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* x_dev, int lda
 // inside (few rows, weights resident in shared memory) get them made in scratch.
 static int matmul_rows(b2w4_ctx* ctx, const b2w4_weight* w, const b2w4_rows& from, float* y,
                        int ldc, int m, int act_rule) {
+    if (!matmul_accepts(ctx, w, m, act_rule, true))  // before the residual is written
+        return b2w4_fail(ctx, B2W4_E_INVALID, "matmul: K=%d is too long for %d rows", w->k, m);
     // (the norm's quantiser keeps a row in shared memory, and adds as the operator's block does)
     const bool made =
         from.kind == b2w4_rows::SWIGLU || (w->k <= kRowsNormMaxK && w->k > kNormWarpMaxK);

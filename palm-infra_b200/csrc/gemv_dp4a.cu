@@ -836,6 +836,14 @@ int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, size_t sme
 
 }  // namespace
 
+// Whether the kernels of up to eight rows take a row this long: one tile per CTA at least.
+bool b2w4_gemv_fits(const b2w4_weight* w, int m, int act_rule) {
+    if (m > 1)
+        return b2w4_gemv_mma_fits(w, m, act_rule);
+    return gemv_smem_bytes(1, w->k, w->groups, 1, w->scales_fp16 != 0,
+                           act_rule == B2W4_ACT_G32) <= 220 * 1024;
+}
+
 // Rows are processed four at a time; each pass streams the weight once.
 int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                      float* y, int ldc, int m, int act_rule, int activation,
@@ -913,7 +921,7 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
         a.d_stride = gemv_d_stride(mt, w->groups, a32);
         // long rows, split over clusters
         if (!a32 && !sums && !tp && !top1 && !norm && !swiglu && ctx->gemv_tpc_override == 0 &&
-            w->groups >= 48 && tpc <= 4) {
+            w->groups >= 48 && tpc <= 4 && b2w4_gemv_fits(w, 1, act_rule)) {
             const int per = (w->groups + kSplit - 1) / kSplit;
             // clusters in one wave of at most 1.75 CTAs per SM, two CTAs' memory per SM
             const int clusters = wave_ctas / kSplit;

@@ -384,6 +384,15 @@ int mma_launch_mt(b2w4_ctx* ctx, const MmaArgs& a, bool scl16, bool a32, size_t 
 
 }  // namespace
 
+// The longest rows: one tile per CTA (and a word more per scale than the kernel needs).
+bool b2w4_gemv_mma_fits(const b2w4_weight* w, int m, int act_rule) {
+    const bool a32 = act_rule == B2W4_ACT_G32;
+    const int mt = m <= 2 ? 2 : (m <= 4 ? 4 : 8);
+    return mma_smem_bytes(mt, w->k, w->groups, 1, w->scales_fp16 != 0, a32) +
+               sizeof(float) * mt * w->groups * (a32 ? 4 : 1) <=
+           220 * 1024;
+}
+
 // Rows are processed eight at a time (the columns of one tensor instruction); each pass
 // streams the weight once.
 int b2w4_launch_gemv_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
@@ -445,8 +454,7 @@ int b2w4_launch_gemv_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, in
                 a.g_magic = 0;
         a.d_stride = mma_d_stride(mt, w->groups, a32);
         const size_t smem = mma_smem_bytes(mt, w->k, w->groups, a.tile_cap, scl16, a32);
-        // (the limit on K: a word more per scale than the kernel needs)
-        if (smem + sizeof(float) * mt * w->groups * (a32 ? 4 : 1) > 220 * 1024)
+        if (!b2w4_gemv_mma_fits(w, mc, act_rule))
             return b2w4_fail(ctx, B2W4_E_INVALID, "gemv: K=%d needs %zu B shared memory",
                              w->k, smem);
         int rc = mt == 2 ? mma_launch_mt<2>(ctx, a, scl16, a32, smem, ctas)

@@ -597,3 +597,33 @@ def test_few_rows_on_several_streams(m, n, k, rule):
     ctx.set_stream(0)
     w.free()
     ctx.close()
+
+
+@pytest.mark.parametrize("m,rule,longest", [(1, ol.ACT_G128, 39552), (1, ol.ACT_G32, 30464),
+                                            (2, ol.ACT_G128, 33280), (4, ol.ACT_G32, 17152),
+                                            (8, ol.ACT_G128, 15360), (8, ol.ACT_G32, 10112),
+                                            (12, ol.ACT_G128, 26368), (32, ol.ACT_G32, 25216)])
+def test_longest_rows(ctx, m, rule, longest):
+    """The longest row of a call does not depend on the number of weight rows, which decides
+    between kernels with and without a limit: the last length that is taken (a row of the result
+    against the oracle) and the first that is refused, before anything is written."""
+    import torch
+    for n in (8, 2568):
+        for k in (longest, longest + 128):
+            w = ctx.upload_weight(pkg.synth.bg128_weight(3, n + k, n, k), n, k)
+            x = pkg.synth.activations(7, m, m, k)
+            xd, y = torch.from_numpy(x).cuda(), torch.full((m, n), -1.0, device="cuda")
+            res, one = torch.ones((m, k), device="cuda"), torch.ones(k, device="cuda")
+            if k == longest:
+                ctx.matmul(w, xd, y, rule=rule)
+                ctx.sync()
+                rows = pkg.synth.bg128_weight(3, n + k, n, k)[:k // 128 * 544]  # the first tile
+                want = ol.matmul_w4(rows, 8, k, x, rule=rule)
+                assert y[:, :8].cpu().numpy().tobytes() == want.tobytes()
+            else:
+                for call in (lambda: ctx.matmul(w, xd, y, rule=rule),
+                             lambda: ctx.matmul_norm(w, res, xd, one, 1e-6, y, rule=rule)):
+                    with pytest.raises(pkg.capi.B200W4Error, match="K="):
+                        call()
+                assert bool((y == -1).all()) and bool((res == 1).all())
+            w.free()
