@@ -403,7 +403,9 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      residual_out (may be NULL without an update); h = rms_norm(v) *
  *                      norm_weight, written to hidden_out unless NULL; y = w h.
  *                      swiglu: w's rows are gate | up and y [n / 2] = SwiGLU of them (n a
- *                      multiple of 16).  token_dev instead of y: the greedy token.  All
+ *                      multiple of 16; rows of up to 20480 values in any case, somewhat more
+ *                      with fp16 scales, where the plain matmul takes up to 39552).
+ *                      token_dev instead of y: the greedy token.  All
  *                      rows 16-byte aligned.  The same bits as b2w4_add_rms_norm,
  *                      b2w4_matmul / b2w4_matmul_argmax and b2w4_swiglu in turn.
  *                      residual_out and hidden_out overlap neither a row that is read nor

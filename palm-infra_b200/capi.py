@@ -14,6 +14,7 @@ ACT_G128, ACT_G32 = 128, 32
 # b2w4_step_matmul makes a row of up to STEP_ROW_MAX values inside (alone, without an update: of
 # more than STEP_ROW_MIN); other rows go through hidden_out or, without it, the context's scratch
 STEP_ROW_MIN, STEP_ROW_MAX = 256, 4096
+STEP_SWIGLU_MAX = 20480  # longest row that it takes with SwiGLU behind, whatever the scales' type
 NONE, SILU, GELU, RELU, RELU_SQUARED = 0, 1, 2, 3, 4
 
 # every symbol include/b200w4.h declares

@@ -231,7 +231,7 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
                      int act_n_begin, int act_n_len, int32_t* sums,
                      const b2w4_tp_args* tp = nullptr, const b2w4_top1_args* top1 = nullptr,
                      const b2w4_norm_args* norm = nullptr, bool swiglu = false);
-bool b2w4_gemv_fits(const b2w4_weight* w, int m, int act_rule);
+bool b2w4_gemv_fits(const b2w4_weight* w, int m, int act_rule, bool swiglu = false);
 bool b2w4_gemv_mma_fits(const b2w4_weight* w, int m, int act_rule);
 int b2w4_launch_tp_gather(b2w4_ctx* ctx, unsigned long long* stage_local, float* y, int m,
                           int ldc);

@@ -613,6 +613,8 @@ int b2w4_step_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const float* residual_
         return b2w4_fail(ctx, B2W4_E_INVALID, "step_matmul: rows overlap");
     const bool row_first =
         in_place || reads(y_dev, yb) || b2w4_overlap(y_dev, yb, residual_out_dev, kb);
+    if (!b2w4_gemv_fits(w, 1, B2W4_ACT_G128, swiglu != 0))  // before anything is written
+        return b2w4_fail(ctx, B2W4_E_INVALID, "step_matmul: K=%d is too long", w->k);
     b2w4_norm_args norm = {residual_dev, update_dev, norm_weight_dev, eps, residual_out_dev,
                            hidden_out_dev};
     // (a row of up to 256 values alone is summed by one warp, as b2w4_rms_norm does)

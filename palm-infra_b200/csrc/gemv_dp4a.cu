@@ -836,11 +836,12 @@ int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, size_t sme
 
 }  // namespace
 
-// Whether the kernels of up to eight rows take a row this long: one tile per CTA at least.
-bool b2w4_gemv_fits(const b2w4_weight* w, int m, int act_rule) {
+// Whether the kernels of up to eight rows take a row this long: one tile per CTA at least, or
+// (one row with SwiGLU) a gate and an up tile.
+bool b2w4_gemv_fits(const b2w4_weight* w, int m, int act_rule, bool swiglu) {
     if (m > 1)
         return b2w4_gemv_mma_fits(w, m, act_rule);
-    return gemv_smem_bytes(1, w->k, w->groups, 1, w->scales_fp16 != 0,
+    return gemv_smem_bytes(1, w->k, w->groups, swiglu ? 2 : 1, w->scales_fp16 != 0,
                            act_rule == B2W4_ACT_G32) <= 220 * 1024;
 }
 

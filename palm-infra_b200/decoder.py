@@ -256,8 +256,12 @@ class DenseDecoder:
                 c.add_rms_norm(x, o, L["ln2"], cfg.eps, h)
                 c.moe_forward(h, L["router"], cfg.top_k, inter, L["gate_up"], L["down"], dn)
             else:
-                c.step_matmul(L["gate_up"], x, o, L["ln2"], cfg.eps, x_new, y=act, swiglu=True,
+                wide = H > capi.STEP_SWIGLU_MAX
+                c.step_matmul(L["gate_up"], x, o, L["ln2"], cfg.eps, x_new,
+                              y=self._b("gu", 1, 2 * inter) if wide else act, swiglu=not wide,
                               hidden_out=made)
+                if wide:
+                    c.swiglu(self._b("gu", 1, 2 * inter), act)
                 x, x_new = x_new, x
                 c.matmul(L["down"], act, dn, rule=capi.ACT_G128)
             update = dn

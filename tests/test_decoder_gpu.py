@@ -118,3 +118,19 @@ def test_captured_step_outlives_grown_scratch(hidden):
     model.free()
     ctx.close()
     assert got == want
+
+
+def test_step_of_a_decoder_with_very_long_rows():
+    """22528 hidden values: a gate and an up tile together are more than a block's memory, one tile
+    is not.  The steps run, eager and captured, with the tokens of the operators in turn."""
+    dec = pkg.decoder
+    cfg = dec.DecoderConfig(1, 22528, 4, 2, 64, 128, 256)
+    weights = dec.synthetic_weights(cfg, seed=3)
+    ctx = pkg.capi.Context(0)
+    tokens = []
+    for fused in (False, None):
+        model = dec.DenseDecoder(ctx, cfg, weights, capacity=16, fused_qkv=fused)
+        tokens += [model.generate([7], 6), model.generate([7], 6, replay=True)]
+        model.free()
+    ctx.close()
+    assert tokens[1:] == tokens[:-1]

@@ -831,3 +831,31 @@ def test_attention_step_over_its_own_rows(ctx, past, heads, kv_heads, dim, at):
     for a, b in zip(cache, want_kv):
         assert torch.equal(a, b)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+def test_step_matmul_swiglu_longest_rows(ctx, f32):
+    """The longest row that the header names, and one that is refused before anything is written."""
+    import torch
+    for k in (20480, 22016):
+        n = 32
+        blocks = np.array(pkg.synth.bg128_weight(3, n + k, n, k), copy=True)
+        if f32:  # scales that fp16 cannot hold
+            blocks.reshape(-1, 544)[:, :32].view(np.float32)[:] *= np.float32(1.0001)
+        w = ctx.upload_weight(blocks, n, k)
+        x, u, g = (torch.randn((1, k), device="cuda") for _ in range(3))
+        res, hid, y = torch.zeros((1, k), device="cuda"), torch.zeros((1, k), device="cuda"), \
+            torch.zeros((1, n // 2), device="cuda")
+        if k == 20480:
+            merged, want = torch.zeros((1, n), device="cuda"), torch.zeros_like(y)
+            ctx.step_matmul(w, x, u, g, 1e-6, res, y=y, swiglu=True, hidden_out=hid)
+            ctx.matmul(w, hid, merged, rule=ol.ACT_G128)
+            ctx.swiglu(merged, want)
+            ctx.sync()
+            assert torch.equal(y, want) and bool(y.any())
+        else:
+            with pytest.raises(pkg.capi.B200W4Error, match="too long"):
+                ctx.step_matmul(w, x, u, g, 1e-6, res, y=y, swiglu=True, hidden_out=hid)
+            ctx.sync()
+            assert not res.any() and not hid.any() and not y.any()
+        w.free()

@@ -21,6 +21,7 @@ class FusedOracleContext(OracleContext):
         inside = tokens is None and w.k <= 4096 and (update is not None or w.k > 256)
         assert inside or hidden_out is not None, f"a row of {w.k} values in the context's scratch"
         assert (tokens is None) != (y is None)
+        assert not swiglu or w.k <= 20480, "more than a gate and an up tile of a block's memory"
         hidden = torch.empty((1, w.k)) if hidden_out is None else hidden_out
         if update is None:
             self.rms_norm(residual, norm_weight, eps, hidden)
@@ -64,7 +65,7 @@ class FusedOracleContext(OracleContext):
 
 
 @pytest.mark.parametrize("experts", [0, 4])
-@pytest.mark.parametrize("hidden", [256, 384, 4224])
+@pytest.mark.parametrize("hidden", [256, 384, 4224, 22528])
 @pytest.mark.parametrize("prompt_len", [5, 9])
 def test_fused_driver_gives_the_tokens_and_holds_no_scratch(hidden, prompt_len, experts):
     cfg = dec.DecoderConfig(2, hidden, 4, 2, 64, 128, 256, experts=experts,
