@@ -488,11 +488,11 @@ def test_long_rows_split_over_a_cluster(ctx, n, k, f32):
 @pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
 @pytest.mark.parametrize("m,pairs,k", [(16, 1, 768), (12, 2, 640), (13, 3, 384), (16, 4, 1152),
                                        (17, 1, 128), (24, 2, 896), (32, 1, 256), (25, 2, 2560),
-                                       (4, 8, 640), (9, 5, 512)])
+                                       (8, 7, 1024), (9, 5, 512)])
 def test_few_rows_with_few_pairs_per_multiprocessor(ctx, m, pairs, k, rule):
     """Two or four warps share the chain of a pair of tiles: 1 to 20 groups (whole stages of four
-    and cut ones), the last pair with one tile, up to the largest number of chains per block (and
-    one past it)."""
+    and cut ones), the last pair with one tile, up to the largest number of chains per block (eight:
+    16 rows of four pairs under the per-128 rule, 25 of two; seven of eight rows) and one past it."""
     n = 148 * 16 * pairs - 8
     blocks = pkg.synth.bg128_weight(20261125, n + k + m, n, k)
     x = pkg.synth.activations(7, m + 5, m, k)
@@ -501,17 +501,53 @@ def test_few_rows_with_few_pairs_per_multiprocessor(ctx, m, pairs, k, rule):
     assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=rule).tobytes()
 
 
-@pytest.mark.parametrize("rule", [ol.ACT_G32, ol.ACT_G128])
-@pytest.mark.parametrize("m,n,k", [(2, 16392, 256), (3, 4104, 512), (8, 6152, 640), (5, 1608, 384),
-                                   (2, 1608, 6272), (7, 1603, 6144), (2, 16392, 1024),
-                                   (3, 2568, 6272)])
-def test_two_to_eight_rows_on_the_streamed_kernel(ctx, m, n, k, rule):
-    """Row counts and weights on which few rows take the kernel of 9 to 32 rows: a warp per pair,
-    up to ten pairs per CTA."""
+BOTH, G32, G128 = (ol.ACT_G32, ol.ACT_G128), (ol.ACT_G32,), (ol.ACT_G128,)
+PER_SM = 148 * 16  # weight rows that give every multiprocessor one pair of tiles
+
+
+def _fp32_scales(blocks):
+    """The same blocks with scales that fp16 cannot hold."""
+    blocks = np.array(blocks, copy=True)
+    s = blocks.reshape(-1, 544)[:, :32].copy().view(np.float32)
+    blocks.reshape(-1, 544)[:, :32] = (s * np.float32(1.0000001) + np.float32(1e-9) *
+                                       (s != 0)).astype(np.float32).view(np.uint8)
+    return blocks
+
+
+# streamed: the rules under which the call goes to the kernel of 9 to 32 rows (a quantiser's launch
+# and the matmul's); else it is one launch of the kernel that quantises inside
+@pytest.mark.parametrize("rule", BOTH)
+@pytest.mark.parametrize("m,n,k,streamed,f32", [
+    (2, 16392, 256, (), False), (3, 4104, 512, (), False), (8, 6152, 640, G32, False),
+    (5, 1608, 384, (), False), (2, 1608, 6272, (), False), (2, 16392, 1024, G32, False),
+    (4, PER_SM * 8 - 8, 640, (), False),
+    (7, 1603, 6144, BOTH, False),             # one pair per multiprocessor, four warps a chain
+    (3, 2568, 6272, BOTH, False), (7, 4104, 512, G32, False),       # two pairs
+    (8, 6152, 2048, BOTH, False),             # three; per 32 a warp per pair, six stages
+    (7, PER_SM * 5 - 8, 2176, BOTH, True), (8, PER_SM * 7 - 8, 1024, BOTH, False),  # two warps
+    (2, PER_SM * 8 - 8, 1024, G32, False), (8, PER_SM * 8 - 8, 2048, BOTH, False),  # five stages
+    (5, PER_SM * 12 - 8, 1024, BOTH, False),  # two blocks per multiprocessor, three stages
+    (8, PER_SM * 12 - 3, 1152, BOTH, True)])
+def test_two_to_eight_rows_on_the_streamed_kernel(ctx, m, n, k, streamed, f32, rule):
+    """Row counts and weights on both sides of the line between the two kernels, and each form of
+    the streamed one with a single column block: chains shared by four and by two warps, a warp per
+    pair with six, five and three stages, fp16 and fp32 scales; the oracle's bits."""
+    import torch
     blocks = pkg.synth.bg128_weight(20261125, n + k + m + 5, n, k)
+    if f32:
+        blocks = _fp32_scales(blocks)
     x = pkg.synth.activations(7, m + 17, m, k)
-    y, _ = run_gpu(ctx, blocks, n, k, x, rule=rule, sums=False, pad=4 if n % 16 else 0)
-    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=rule).tobytes()
+    pad = 4 if n % 16 else 0
+    w = ctx.upload_weight(blocks, n, k)
+    xd = torch.zeros((m, k + pad), device="cuda")
+    xd[:, :k] = torch.from_numpy(x)
+    yd = torch.full((m, n + pad), -7.0, device="cuda")
+    assert _launches_of(ctx, lambda: ctx.matmul(w, xd, yd, rule=rule)) == (
+        2 if rule in streamed else 1)
+    ctx.sync()
+    w.free()
+    assert bool((yd[:, n:] == -7.0).all())
+    assert yd[:, :n].cpu().numpy().tobytes() == ol.matmul_w4(blocks, n, k, x, rule=rule).tobytes()
 
 
 # (rows, weight, rule) that the streamed kernel of gemm_rows.cu takes below nine rows
