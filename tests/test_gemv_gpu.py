@@ -603,14 +603,14 @@ def test_few_rows_captured_hold_no_scratch(m, n, k, rule):
 
 @pytest.mark.parametrize("m,n,k,rule", STREAMED)
 def test_few_rows_on_several_streams(m, n, k, rule):
-    """One context used on ten streams in turn, nothing ordered between them: every call's rows are
-    its own.  Eight streams have buffers (a quantiser's launch and the matmul's), the others take
+    """One context used on 18 streams in turn, nothing ordered between them: every call's rows are
+    its own.  Sixteen streams have buffers (a quantiser's launch and the matmul's), the others take
     the kernel that quantises inside."""
     import torch
     blocks = pkg.synth.bg128_weight(20261125, n + k + m, n, k)
     ctx = pkg.capi.Context(0)
     w = ctx.upload_weight(blocks, n, k)
-    streams = [torch.cuda.Stream() for _ in range(10)]
+    streams = [torch.cuda.Stream() for _ in range(18)]
     xs = torch.randn((len(streams), m, k), device="cuda") * torch.arange(
         1, len(streams) + 1, device="cuda").view(-1, 1, 1)
     want, ys = (torch.zeros((len(streams), m, n), device="cuda") for _ in range(2))
@@ -627,7 +627,7 @@ def test_few_rows_on_several_streams(m, n, k, rule):
         for i, s in enumerate(streams):
             ctx.set_stream(s.cuda_stream)
             assert _launches_of(ctx, lambda: ctx.matmul(w, xs[i], ys[i], rule=rule)) == (
-                2 if i < 8 else 1)
+                2 if i < 16 else 1)
         torch.cuda.synchronize()
         assert torch.equal(ys, want)
     ctx.set_stream(0)
