@@ -397,7 +397,8 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      the residual is updated in place.  The same bits as the two
  *                      calls
  *   b2w4_matmul_swiglu b2w4_swiglu of merged rows [2k] and b2w4_matmul of its result,
- *                      likewise
+ *                      likewise.  Up to eight rows, both have them made in the context's
+ *                      scratch by the separate launches
  *   b2w4_step_matmul   the matmul of a decode step with its neighbours in it (one row,
  *                      per-128 rule): v = residual (+ update, may be NULL), written to
  *                      residual_out (may be NULL without an update); h = rms_norm(v) *
@@ -411,7 +412,10 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      residual_out and hidden_out overlap neither a row that is read nor
  *                      another output (refused), but hidden_out may be the residual or the
  *                      update itself; y may lie over a row that is read or over
- *                      residual_out.  Such calls take one launch more, as k > 4096 does
+ *                      residual_out.  Such calls take one launch more, as k > 4096, the
+ *                      greedy token and k <= 256 without an update do: h goes to
+ *                      hidden_out or, if that is NULL, to the context's scratch (which a
+ *                      captured call should not hold: a larger call frees it)
  *   b2w4_advance       *counter_dev += by, after history_dev[*counter_dev] = *token_dev
  *                      (both optional).  With the position on the device a decode
  *                      step is the same sequence of launches for every token and can

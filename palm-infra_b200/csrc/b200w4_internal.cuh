@@ -132,7 +132,7 @@ constexpr int kRowsNormMaxK = 12160;
 int b2w4_launch_repack(b2w4_ctx* ctx, const void* dev_blocks, b2w4_weight* w);
 int b2w4_launch_quantize(b2w4_ctx* ctx, const float* x, int lda, int m, int k,
                          int act_rule, int8_t* q, float* scales, int layout);
-// 9..256 rows per launch on mma.sync with register accumulators (gemm_mma.cu)
+// up to 256 rows per launch on mma.sync with register accumulators (gemm_mma.cu)
 bool b2w4_gemm_mma_fits(const b2w4_weight* w, int m, int act_rule);
 bool b2w4_gemm_mma_resident(const b2w4_weight* w, int m, int act_rule, int sm_count);
 int b2w4_launch_gemm_mma(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,

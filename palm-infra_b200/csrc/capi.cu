@@ -318,6 +318,7 @@ static int check_matmul(b2w4_ctx* ctx, const b2w4_weight* w, const void* x, int 
 // [12000, 640] 8 5.0 / 4.7.  Per 128 [9728, 2560] 4 6.8 / 7.1, 5 7.7 / 7.0; [2560, 9728] 2 10.2 / 16.6,
 // 3 20.3 / 16.4; [1600, 6144] 5 11.0 / 11.2, 6 12.2 / 11.2; [2560, 4096] 6 7.9 / 8.4, 7 8.5 / 8.3;
 // [19456, 2560] 2 8.8 / 10.0, 3 11.6 / 10.1; [20000, 1024] 4 5.1 / 5.1, 5 6.1 / 5.2; [8192, 1024] never.
+// The tile counts stand for pairs of tiles per multiprocessor of 148 and were measured there only.
 static bool few_rows_streamed(const b2w4_weight* w, int m, int act_rule) {
     const int tiles = w->tiles, groups = w->groups;
     if (m < 2 || tiles < 200)
@@ -378,8 +379,8 @@ static bool matmul_accepts(const b2w4_ctx* ctx, const b2w4_weight* w, int m, int
 
 // Up to eight activation rows stream the weight once through the GEMV kernels (one row:
 // dp4a; two to eight: the warp-level int8 tensor instruction) or, as up to 32 rows do, through
-// the kernel of gemm_rows.cu; more rows go to the tcgen05 kernels (K <= 10240).  All produce the same bits for
-// the same activation rule.
+// the kernel of gemm_rows.cu; more rows go to the tcgen05 kernels (K <= 10240) or, below, to
+// mma.sync.  All produce the same bits for the same activation rule.
 static int matmul_dispatch(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                            float* y, int ldc, int m, int act_rule, int activation,
                            int act_n_begin, int act_n_len) {

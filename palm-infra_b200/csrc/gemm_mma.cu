@@ -374,8 +374,10 @@ bool b2w4_gemm_mma_fits(const b2w4_weight* w, int m, int act_rule) {
 }
 
 // True when, with one CTA per SM, the CTA's weights and ALL groups of the activations fit in
-// shared memory together: the regime this kernel is the fastest in (measured on config 2:
-// 16 rows 14 us against 19 us on the tcgen05 kernel; from 64 rows on the tcgen05 kernel wins).
+// shared memory together: the regime this kernel is the fastest in.  It is asked for more than 32
+// rows under the per-128 rule; us in a graph, this kernel / tcgen05: [9728, 2560] 33 and 40 rows
+// 14.8 / 19.8 (more do not fit); [2560, 2560] 33 rows 12.2 / 14.1, 64 13.7 / 14.1, 128 14.5 / 14.3;
+// [4096, 1024] 33 rows 7.6 / 8.6, 64 8.3 / 8.6, but 96 11.0 / 8.8 and 128 10.9 / 8.8.
 bool b2w4_gemm_mma_resident(const b2w4_weight* w, int m, int act_rule, int sm_count) {
     if (m > kMaxRows)
         return false;

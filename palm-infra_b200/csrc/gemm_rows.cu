@@ -1,5 +1,5 @@
-// W4G128 x int8 matmul for a few activation rows (9..32: batched decode, short prompts) on the
-// warp-level int8 tensor instruction (mma.sync m16n8k32).
+// W4G128 x int8 matmul for a few activation rows (9..32, and 2..8 by few_rows_streamed in capi.cu:
+// batched decode, short prompts) on the warp-level int8 tensor instruction (mma.sync m16n8k32).
 //
 // Arithmetic = the reference's, row by row, under either rule (kernels/matmul_w4.cpp:211-295 with
 // one activation scale per 128 values, :785-901 with one per 32): per group or 32-k block
@@ -9,8 +9,8 @@
 //
 // Work split.  A warp owns a pair of 8-row weight tiles (the sixteen rows of the instruction) and
 // all blocks of eight activation rows (its columns), or, where there are few pairs, several warps
-// share a pair; a CTA holds up to ten warps, so that one or two CTAs per SM take the whole weight
-// in one round.  Weights, codes and scales stream through a ring of shared-memory stages of four
+// share a pair; a CTA holds up to ten warps (sixteen where pairs are shared), so that one or two
+// CTAs per SM take a weight of up to twenty pairs per SM in one round.  Weights, codes and scales stream through a ring of shared-memory stages of four
 // groups, one barrier per stage; the weights of the first stages are on their way before the
 // kernel waits for the quantiser in front (programmatic dependent launch).  (Fetched into
 // registers four groups ahead instead, the weights came no sooner: a warp's outstanding loads
@@ -22,6 +22,10 @@
 // |16 D| <= 128 * 127 * 128 < 2^22: D costs one subtraction, for two columns at once.  (Unsigned
 // bytes q + 8 need a start that depends on the sum of the codes, four more words per instruction
 // to make, copy and read: 16 rows, [9728, 2560], per 32 values, 11.1 -> 9.6 us.)
+//
+// What bounds it: the latency of few warps.  16 rows of [9728, 2560] per 32 values, ten warps per
+// SM: issue slots 45 % busy, DRAM 13 %, a warp waits 5.4 cycles per instruction (1.5 for the result
+// before it, 0.6 for the fp32 pipe, 0.5 at the stage's barrier).
 #include "b200w4_internal.cuh"
 
 namespace {
@@ -408,6 +412,12 @@ int b2w4_launch_gemm_rows(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, i
     // 8 rows 24.2 -> 20.3 / 23.6 -> 18.6, 16 rows 26.0 -> 21.3 / 24.3 -> 19.1, 32 rows 33.0 ->
     // 28.4 / 31.9 -> 23.5; [9728, 2560] (five pairs) 8 rows 8.4 -> 7.7 / 8.0 -> 7.0; [6144, 2560]
     // (three) 8 rows 6.7 -> 7.1, not taken / 6.8 -> 6.3, 16 rows 7.9 -> 8.1, not taken / 7.6 -> 7.2.
+    // Other row lengths, pairs per SM x column blocks (those of more than sixteen warps are not
+    // shared): K = 4096 per 32 1 x 1 12.4 -> 9.3, 1 x 4 17.3 -> 11.0, 2 x 2 12.2 -> 10.6, 5 x 1
+    // 12.5 -> 11.8; per 128 1 x 4 17.1 -> 10.0, 3 x 2 11.0 -> 10.3, 4 x 2 11.3 -> 11.1; K = 1024 from
+    // 0.7 less to 0.4 more.  The line is not the best everywhere: per 32 2 x 4 is slower than
+    // unshared up to K = 4096 (1024 5.2 -> 6.6, 2560 9.4 -> 10.9, 4096 14.4 -> 15.2; 9728 33.1 ->
+    // 29.8), and 7 x 1 is (2560 8.9 -> 11.5, 4096 13.1 -> 15.6).
     a.pw = ncb;
     const int few = (a.pairs + ctx->sm_count - 1) / ctx->sm_count;
     if (few * ncb * 2 <= kRelayWarps && (few <= 2 || !a32 || (few > 4 && ncb == 1)) &&

@@ -920,7 +920,13 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
                     a.ipt_magic = 0;
         }
         a.d_stride = gemv_d_stride(mt, w->groups, a32);
-        // long rows, split over clusters
+        // Long rows, split over clusters, from 48 groups on and where the kernel above has at most
+        // four tiles per CTA.  us in a graph, that kernel / split, by weight rows: K = 9728 1000
+        // 5.9 / 4.2, 2560 7.8 / 6.0, 4096 8.5 / 7.6; K = 6144 4.3 / 3.7, 5.6 / 4.7, 5.8 / 5.8, 6144
+        // rows 7.2 / 7.2, 9728 (more tiles) 12.2 / 13.3; K = 5120 4.1 / 3.4, 5.0 / 4.2, 5.1 / 5.2,
+        // 6144 rows 6.2 / 6.4; K = 4096 3.2 / 3.2, 3.9 / 3.8, 4.1 / 4.6, 4.9 / 5.6; K = 2560 2.9 /
+        // 3.1, 3.3 / 3.5, 3.3 / 3.9, 9728 rows 4.7 / 9.4.  (40 groups on up to 2560 rows would
+        // gain too.)
         if (!a32 && !sums && !tp && !top1 && !norm && !swiglu && ctx->gemv_tpc_override == 0 &&
             w->groups >= 48 && tpc <= 4 && b2w4_gemv_fits(w, 1, act_rule)) {
             const int per = (w->groups + kSplit - 1) / kSplit;

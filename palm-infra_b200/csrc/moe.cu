@@ -482,9 +482,6 @@ moe_route_fused_kernel(const float* __restrict__ hidden, int ldx, int tokens, in
         *arrivals = 0;  // ready for the next launch
 }
 
-// ---- 6. SwiGLU + quantiser: one warp per (route, 128-wide group of I) ------------------
-// inter = (g * 1/(1+exp(-g))) * u with gate = columns [0,I), up = [I,2I)
-// (kernels/moe.cpp:160-183), then the per-128 quantiser; codes in tensor-operand order.
 // Hidden rows for the grouped matmul, one warp per (token, 128-group): codes in tensor-operand
 // order and scales per 128 values, and (q32 != null) per 32 values as well.
 __global__ void moe_quantize_hidden_kernel(const float* __restrict__ hidden, int ldx, int tokens,
@@ -524,6 +521,9 @@ __global__ void moe_quantize_hidden_kernel(const float* __restrict__ hidden, int
     store(amax, false, q + at, scales + (size_t)row * G + g);
 }
 
+// ---- 6. SwiGLU + quantiser: one warp per (route, 128-wide group of I) ------------------
+// inter = (g * 1/(1+exp(-g))) * u with gate = columns [0,I), up = [I,2I)
+// (kernels/moe.cpp:160-183), then the per-128 quantiser; codes in tensor-operand order.
 // one warp: 128 values of one route, written to `group_dst` (the 128 code bytes of the group)
 // and `scale_dst`
 // a32: one scale per 32 values (scale_dst[0..3], the lane's block is lane / 8) instead of one
@@ -1020,9 +1020,8 @@ size_t grouped_small_smem(int k, int groups, int tpc, bool scl16) {
 // each).  A unit is one pass against a pair per warp of a CTA; the units of all experts lie in
 // one line (expert, pass, pairs) of which every CTA takes an equal, contiguous share, two CTAs
 // of eight warps per SM, so that one computes while the other changes to another pass, or one
-// CTA of sixteen warps where a pass's rows leave no room for two.  A pass's int8 rows, scales
-// and accumulator biases are staged in shared memory once and serve all units of the share that
-// belong to it.
+// CTA of sixteen warps where a pass's rows leave no room for two.  A pass's int8 rows and scales
+// are staged in shared memory once and serve all units of the share that belong to it.
 //
 // The integer sums come from the warp-level int8 tensor instruction (mma.sync m16n8k32): the
 // pair's weight rows are its rows, eight routes its columns.  A warp runs the whole K loop of its
@@ -1042,9 +1041,11 @@ size_t grouped_small_smem(int k, int groups, int tpc, bool scl16) {
 // pipe was 68 % busy; 256 tokens, 128 experts of 768: 231 -> 191 us).  D is folded into fp32 chain values
 // y = fma(float(D), fp32(ws*as), y)  that stay in the warp's registers until the last group, two
 // columns per instruction.  The math is the dense kernels', route by route.
-// What bounds it: issue slots (about 110 instructions per group and pair with sixteen routes,
-// most of them the chain and the split of the words), close to the time the weights take from
-// HBM at sixteen routes per expert.
+// What bounds it: nothing alone.  256 tokens over 128 experts of 768, gate_up / down: 0.10 / 0.06
+// ms, about three times what the weights take from HBM (36 / 27 % of its rate), issue slots 62 /
+// 61 % busy, the shared-memory pipe 57 / 54 %; a warp waits 5.8 cycles per instruction with 3.6
+// warps per scheduler (1.5 for the result before it, 1.1 for its turn, 0.8 for the fp32 pipe, 0.6
+// for shared memory).  Experts with more than sixteen routes stream and split their weights again.
 constexpr int kGR = 16;         // routes per pass: two column blocks
 constexpr int kRowPad = 16;     // bytes added to a staged activation row: conflict-free reads
 
@@ -1056,7 +1057,7 @@ struct GroupedArgs {
     // The reference's rule for an expert that holds SEVERAL rows (kernels/moe.cpp:1055-1058
     // -> kernels/matmul_w4.cpp:1125-1154): one activation scale per 32 values.  qa32 / as32 are
     // those rows quantised that way (as32[r][4*g + block]); null = per-128 for every expert.
-    //  An expert with a single row keeps the per-128 rule (:1058-1075).
+    // An expert with a single row keeps the per-128 rule (:1058-1075).
     const int8_t* qa32;
     const float* as32;
     int as_stride, as32_stride;
