@@ -256,6 +256,10 @@ int b2w4_launch_quantize_umma(b2w4_ctx* ctx, const float* x, int lda, int m, int
 int b2w4_launch_gemm_tc(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda,
                         float* y, int ldc, int m, int activation, int act_n_begin,
                         int act_n_len, const b2w4_rows* from = nullptr);
+int b2w4_launch_attention_tc(b2w4_ctx* ctx, const float* q, const float* k_cache,
+                             const float* v_cache, float* out, int tokens, int heads,
+                             int kv_heads, int dim, int past, const int* past_dev, int capacity,
+                             float scale);
 int b2w4_launch_gemm_tc32(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int lda, float* y,
                           int ldc, int m, int activation, int act_n_begin, int act_n_len,
                           const b2w4_rows* from = nullptr);

@@ -859,3 +859,100 @@ def test_step_matmul_swiglu_longest_rows(ctx, f32):
             ctx.sync()
             assert not res.any() and not hid.any() and not y.any()
         w.free()
+
+
+def _attention_fp64_cuda(q, kc, vc, past, scale):
+    """_attention_fp64 on device tensors."""
+    import torch
+    tokens, heads, dim = q.shape
+    kv_heads, keys = kc.shape[0], past + tokens
+    out = torch.empty((tokens, heads, dim), dtype=torch.float64, device="cuda")
+    hidden = torch.arange(keys, device="cuda")[None] > \
+        past + torch.arange(tokens, device="cuda")[:, None]
+    for h in range(heads):
+        g = h // (heads // kv_heads)
+        s = (q[:, h].double() @ kc[g, :keys].double().T) * scale
+        p = torch.softmax(s.masked_fill_(hidden, float("-inf")), 1)
+        v = torch.where((p > 0).any(0)[:, None], vc[g, :keys].double(), 0.0)
+        out[:, h] = p @ v
+    return out
+
+
+LONG_RUNS = [  # tokens, past, heads, kv_heads, dim: the tensor-core kernel
+    (256, 128, 24, 8, 128),   # the shortest, three heads per kv head: 126 of 128 rows in use
+    (1473, 3, 32, 8, 128),    # ragged last tile and last block of keys
+    (261, 700, 40, 1, 128),   # 40 heads per kv head: 120 rows
+    (400, 64, 64, 1, 64), (1500, 1, 16, 16, 64), (640, 0, 40, 8, 64)]
+
+
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", LONG_RUNS)
+def test_long_runs_on_tensor_cores(ctx, tokens, past, heads, kv_heads, dim):
+    """Runs whose products go to the tensor cores in three bf16 pieces, against 64 bits, and no
+    further from them than the one-row arithmetic in fp32 (a tenth more for the luck of one
+    draw); the position on the device leaves the same bits; value rows past the position are NaN.
+    Tolerance as for the split kernel."""
+    import torch
+    capacity, scale = max(384, past + tokens + 9), dim ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(tokens + dim)
+    q = torch.randn((tokens, heads, dim), device="cuda", generator=g)
+    kc, vc = (torch.randn((kv_heads, capacity, dim), device="cuda", generator=g)
+              for _ in range(2))
+    vc[:, past + tokens:] = float("nan")
+    ctx_row = _row_context()
+    outs = []
+    for c, past_dev in ((ctx, None), (ctx_row, None),
+                        (ctx, torch.full((1,), past, dtype=torch.int32, device="cuda"))):
+        out = torch.zeros_like(q)
+        c.attention(q, None, None, kc, vc, out, tokens, heads, kv_heads, dim,
+                    past if past_dev is None else 0, capacity, scale, past_dev)
+        c.sync()
+        outs.append(out)
+    ctx_row.close()
+    want = _attention_fp64_cuda(q, kc, vc, past, scale)
+    err, row_err = (float((o.double() - want).norm() / want.norm()) for o in outs[:2])
+    assert err < 1e-5 and err < 1.1 * row_err
+    assert torch.equal(outs[0], outs[2])
+    assert not torch.equal(outs[0], outs[1])  # not the tile kernel, which has the row's bits
+
+
+@pytest.mark.parametrize("tokens,heads,kv_heads,dim", [(256, 24, 8, 128), (640, 40, 8, 64)])
+def test_long_runs_with_extreme_values(ctx, tokens, heads, kv_heads, dim):
+    """Keys of probability zero whose value rows are not finite, values near the largest number,
+    values so small that bf16 pieces would lose bits, a value row of NaN that is seen: as in
+    test_attention_ignores_value_rows_of_zero_probability, tolerances from there (640 terms:
+    4e-5).  Such tiles are done in fp32, the others are not touched by it."""
+    import torch
+    rng = np.random.default_rng(dim)
+    keys = tokens + 300
+    q1, k, v = _staged(rng, heads, kv_heads, dim, keys, [0.0, 80.0, 160.0])
+    qd = _dev(np.repeat(q1, tokens, axis=0))
+    k[:] = 0.0
+    k[:100, :, 0] = -160.0  # probability zero against the rest
+    kc, vc = (_dev(np.ascontiguousarray(x.transpose(1, 0, 2))) for x in (k, v))
+
+    def run():
+        out = torch.zeros((tokens, heads, dim), device="cuda")
+        ctx.attention(qd, None, None, kc, vc, out, tokens, heads, kv_heads, dim, 300, keys, 1.0)
+        ctx.sync()
+        return out
+
+    clean = vc.clone()
+    clean[:, :100] = 0.0
+    want = _attention_fp64_cuda(qd, kc, clean, 300, 1.0)
+    for bad in (float("nan"), float("inf"), float("-inf")):
+        vc[:, 3] = bad
+        vc[:, 50, dim // 2] = bad
+        got = run()
+        assert torch.isfinite(got).all()
+        assert float((got.double() - want).norm() / want.norm()) < 4e-5
+    vc[:, :100] = 0.0
+    for size, tol in ((3e38, 1e-5), (1e-34, 4e-5)):
+        vc[:, 100:] = torch.rand_like(vc[:, 100:]) * 0.5 + 0.5
+        want = _attention_fp64_cuda(qd, kc, vc, 300, 1.0)
+        vc *= size
+        got = run().double() / size
+        assert float((got - want).norm() / want.norm()) < tol
+    vc.normal_()
+    vc[:, 300 + tokens // 2] = float("nan")  # seen by the second half
+    got = run()
+    assert torch.isnan(got[tokens // 2:]).all() and torch.isfinite(got[:tokens // 2]).all()
