@@ -10,20 +10,27 @@
 //   epilogue   sixteen warps, thread = one token x a quarter of the tile's columns, four warps per
 //              scheduler so that one folds while another fetches; a tile of up to 128 columns
 //              (row_tiles) spreads what a group costs beside its columns.
-//   unpack     a nibble becomes a signed byte of 16 q with one AND (high nibble) or a shift
-//              and an AND (low nibble): three instructions per eight weights, so the sums
-//              are 16 D, |16 D| < 2^19.  Three warps, every third group each, whole groups.
+//   operands   four warps, every fourth group each, whole groups, its MMAs included.  A nibble
+//              becomes a signed byte of 16 q with one AND (high nibble) or a shift and an AND (low
+//              nibble): three instructions per eight weights, so the sums are 16 D, |16 D| < 2^19.
 //   to float   the hardware conversion, so that the fp32 pipe sees only the scale product and
 //              the multiply-add, both paired (fma.rn.f32x2).  It also moves the sums from the
 //              registers that the fetch filled to register pairs.  The scales are staged as
 //              w / 16: a power of two, exact while w * as / 16 is a normal number.
-//   MMA        one thread; two accumulator units (a group each, or half a group where tiles are
-//              wide) or more in tensor memory, and one barrier frees an activation and a weight
-//              stage together.
+//   sums       units of half a group, two or four of them in tensor memory; one barrier frees an
+//              activation and a weight stage together.
 // Measured, 1000 rows, [4100, 9728], three matmuls: tiles of at most 64 columns 882 us; of up to
-// 128 with eight epilogue warps and all unpack warps on one group 715 us; this form 618 us (eight
-// layers of a 256-token prompt, all operators: 2.46, 2.20 and 1.95 ms).  At 112 columns a group
-// takes 2490 cycles, of which the chain is 1930.
+// 128 with eight epilogue warps and all unpack warps on one group 715 us; this form 613 us.  At 112
+// columns a group takes 2180 cycles (clock64, 1.80 GHz): the chain alone, no waits and no other
+// warps, 1830 (conversions 448 of a scheduler's issue slots and 896 cycles of its pipe, paired
+// products and multiply-adds 224 each and 1140 cycles of the fp32 pipe, fetches 360 on top of
+// them); the operand warps beside it 180, the MMAs nothing, waits 170.
+// MMAs issued by the warp that unpacks the group, against one warp for the MMAs and three that
+// unpack: 40 rows of [2560, 9728] 42.2 -> 37.2 us, 256 rows 53.5 -> 50.0, of [2560, 4096] 26.1 ->
+// 24.7, of [19456, 2560] 74.0 -> 72.7, 64 rows of [9728, 2560] 24.1 -> 22.2.
+// Tried on the form before: waits that poll in a loop of four instructions, or with test_wait,
+// 206 -> 221 us a matmul and 42 -> 62 at 40 rows (pollers take issue slots); hand-over through named
+// barriers 235; units of one block 217; the next chunk's fetch under a chunk's sums: no gain.
 // Tokens sit on the MMA's M side (128 per CTA), weight rows on its N side.  The next launch
 // is released at the start (programmatic dependent launch): weights and scales are fetched
 // while the quantiser in front still runs.  Every wait is bounded; on a timeout the kernel
@@ -34,13 +41,12 @@
 
 namespace {
 
-// Roles: one warp that issues MMAs, three that bring operands in, a group in turn, then sixteen
-// epilogue warps (four column quarters x four TMEM lane quarters; a warp's lane quarter is its
-// index mod 4).  640 threads start with 96 registers each; the epilogue's four warpgroups take
+// Roles: four warps that bring a group's operands in and issue its MMAs, a group in turn, then
+// sixteen epilogue warps (four column quarters x four TMEM lane quarters; a warp's lane quarter is
+// its index mod 4).  640 threads start with 96 registers each; the epilogue's four warpgroups take
 // what the first one gives up.
-constexpr int kMmaWarp = 0;
-constexpr int kUnpackWarp0 = 1, kUnpackWarps = 3;
-constexpr int kEpiWarp0 = 4, kEpiWarps = 16;
+constexpr int kFeedWarps = 4;
+constexpr int kEpiWarp0 = kFeedWarps, kEpiWarps = 16;
 constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;
 constexpr int kRegsStart = 96, kRegsEpi = 104, kRegsOther = 64;
 static_assert(kRegsOther + 4 * kRegsEpi <= 5 * kRegsStart, "registers of the block");
@@ -49,7 +55,7 @@ constexpr int kMaxG = 80;  // K <= 10240
 template <int RP>
 struct Smem {
     // activation and unpacked-weight stages (one group each), groups of nibbles in flight
-    static constexpr int kStages = RP <= 64 ? 6 : 4, kRawSlots = RP <= 64 ? 12 : 6;
+    static constexpr int kStages = RP <= 64 ? 6 : 4, kRawSlots = RP <= 64 ? 12 : 4;
     static constexpr int kActStage = 128 * 128;  // 128 tokens x 128 B, swizzled
     static constexpr int kBStage = RP * 128;     // int8 weights, swizzled
     static constexpr int kRawSlot = (RP / 8) * 512;  // nibbles of a group: [tile][512]
@@ -108,13 +114,12 @@ template <int RP, bool SCL16>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a8_tc32_kernel(const GemmArgs a) {
     constexpr int CH = RP / 4;  // columns per epilogue thread
-    // A unit is what the MMA warp hands to the epilogue: the accumulators of a group, four
-    // blocks of RP columns each, or of half a group where four blocks leave no second buffer.
-    constexpr int kUnitBlocks = RP <= 64 ? 4 : 2;
-    constexpr int kAccCols = kUnitBlocks * RP;
+    // A unit is what the MMAs hand to the epilogue: the accumulators of half a group, two blocks
+    // of RP columns each.  Two units or four, so one or two groups, fit the tensor memory.
+    constexpr int kAccCols = 2 * RP;
     constexpr int kStages = Smem<RP>::kStages, kRawSlots = Smem<RP>::kRawSlots;
-    constexpr int kAcc = 512 / kAccCols;
-    static_assert(kAcc >= 2, "no accumulator to run ahead into");
+    constexpr int kAcc = RP <= 64 ? 4 : 2, kAccGroups = kAcc / 2;
+    static_assert(kAcc * kAccCols <= 512, "tensor memory");
     extern __shared__ uint8_t smem_raw[];
     // swizzle atoms need a 1024-byte aligned base
     uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
@@ -129,28 +134,28 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kBarOff);
     uint64_t* act_full = bars;                  // [kStages] activations of a group landed
-    uint64_t* b_full = act_full + kStages;      // [kStages] unpack done
-    uint64_t* ab_free = b_full + kStages;       // [kStages] MMAs that read both retired
+    uint64_t* ab_free = act_full + kStages;     // [kStages] MMAs that read both operands retired
     uint64_t* acc_full = ab_free + kStages;     // [kAcc] unit complete
-    uint64_t* acc_free = acc_full + kAcc;       // [kAcc] epilogue has fetched it
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + kAcc);
+    // [kFeedWarps][2] epilogue has fetched a half of the group; by group mod kFeedWarps, so that
+    // the warp which waits for it sees every phase
+    uint64_t* acc_free = acc_full + kAcc;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2 * kFeedWarps);
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     b2w4_pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(&act_full[s], 1);
-            mbar_init(&b_full[s], 1);
             mbar_init(&ab_free[s], 1);
         }
-        for (int b = 0; b < kAcc; ++b) {
+        for (int b = 0; b < kAcc; ++b)
             mbar_init(&acc_full[b], 1);
+        for (int b = 0; b < 2 * kFeedWarps; ++b)
             mbar_init(&acc_free[b], 4 * ((m_here + 31) / 32));  // the warps that have tokens
-        }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kMmaWarp) {  // one warp owns the TMEM allocation: 512 columns
+    if (warp == 0) {  // one warp owns the TMEM allocation: 512 columns
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(tmem_slot)), "r"(512)
                      : "memory");
@@ -169,58 +174,17 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         return mbar_try_wait(bar, parity) || (!*s_abort && mbar_wait(bar, parity));
     };
 
-    if (warp < kEpiWarp0)
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-    else
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsEpi));
-
-    if (warp == kMmaWarp) {
-        // =============================== MMA issue ===================================
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_i8(RP);
-            const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kActOff));
-            const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kBOff));
-            int u = 0, use = 0;  // unit buffer and how often it has been filled
-            bool ok = true;
-            for (int g = 0; g < G && ok; ++g) {
-                const int s = g % kStages, round = g / kStages;
-                ok = wait(&act_full[s], round & 1) && wait(&b_full[s], round & 1);
-                // descriptor addresses count 16-byte units
-                const uint64_t a_desc = a_desc0 + (uint64_t)(s * (S::kActStage >> 4));
-                const uint64_t b_desc = b_desc0 + (uint64_t)(s * (S::kBStage >> 4));
-#pragma unroll
-                for (int j0 = 0; j0 < 4; j0 += kUnitBlocks) {
-                    ok = ok && (use == 0 || wait(&acc_free[u], (use - 1) & 1));
-                    if (!ok)
-                        break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                    for (int j = 0; j < kUnitBlocks; ++j)  // a K = 32 step = a 32-k block
-                        umma_i8(tmem_base + (uint32_t)(u * kAccCols + j * RP),
-                                a_desc + (uint64_t)((j0 + j) * 2),
-                                b_desc + (uint64_t)((j0 + j) * 2), idesc, 0u);
-                    umma_commit(&acc_full[u]);  // the unit's sums are complete
-                    if (++u == kAcc) {
-                        u = 0;
-                        ++use;
-                    }
-                }
-                if (!ok)
-                    break;
-                umma_commit(&ab_free[s]);  // both stages may be refilled
-            }
-            if (!ok)
-                fail();
-        }
-    } else if (warp < kEpiWarp0) {
-        // ============================ operands of a group ============================
-        // Warp w takes every third group: when the stage is free it starts the bulk copy of the
+    if (warp < kEpiWarp0) {
+        // ============================ operands and MMAs ==============================
+        // Warp w takes every fourth group: when the stage is free it starts the bulk copy of the
         // group's activations and unpacks its nibbles, which it has copied itself, some groups
         // ahead and before the quantiser in front has finished: no barrier between that copy and
-        // its use.  (All unpack warps on one group at a time, a group took their whole latency;
-        // nibbles by one bulk copy per row tile, issuing those took a warp 1700 of a group's
-        // 2500 cycles.)
-        const int w0 = warp - kUnpackWarp0;
+        // its use.  Then a lane issues the group's MMAs.  (One warp that issued the MMAs of all
+        // groups spent 900 cycles a group on waits that were over and on commits, which set the
+        // pace of narrow tiles.  All warps on one group's nibbles at a time, a group took their
+        // whole latency; nibbles by one bulk copy per row tile, issuing those took a warp 1700 of
+        // a group's 2500 cycles.)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
         const uint8_t* nib = a.nib + (size_t)tile0 * G * 512 + lane * 16;
         auto fetch = [&](int g) {
             if (g < G) {
@@ -234,10 +198,10 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        constexpr int kOwn = kRawSlots / kUnpackWarps;  // groups a warp has in flight
-        static_assert(kRawSlots % kUnpackWarps == 0, "slots");
-        for (int i = 0; i < kOwn - 1; ++i)
-            fetch(w0 + i * kUnpackWarps);
+        constexpr int kOwn = kRawSlots / kFeedWarps;  // groups a warp has in flight
+        static_assert(kRawSlots % kFeedWarps == 0, "slots");
+        for (int i = 0; i < kOwn; ++i)
+            fetch(warp + i * kFeedWarps);
         // only the 8-token atoms that hold real tokens are copied; the MMA reads whatever the
         // rest of the 128-token block holds and the epilogue ignores those rows
         const uint32_t act_bytes = (uint32_t)((m_here + 7) / 8) * 1024;
@@ -247,12 +211,15 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         const int sub = lane >> 3, row = lane & 7;
         const uint32_t even = row * 128 + (((2 * sub) ^ row) << 4);
         const uint32_t odd = row * 128 + (((2 * sub + 1) ^ row) << 4);
-        for (int g = w0; g < G; g += kUnpackWarps) {
+        const uint32_t idesc = umma_idesc_i8(RP);
+        const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kActOff));
+        const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(smem + S::kBOff));
+        bool ok = true;
+        for (int g = warp; g < G; g += kFeedWarps) {
             const int s = g % kStages, round = g / kStages;
-            fetch(g + (kOwn - 1) * kUnpackWarps);  // into the slot of the group before
             // MMAs left this stage
             if (round > 0 && !__all_sync(0xffffffffu, wait(&ab_free[s], (round - 1) & 1))) {
-                fail();
+                ok = false;
                 break;
             }
             if (lane == 0) {
@@ -277,18 +244,47 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
                 *reinterpret_cast<uint4*>(bst + t * 1024 + odd) =
                     make_uint4(w.x & kHigh, w.y & kHigh, w.z & kHigh, w.w & kHigh);
             }
+            fetch(g + kOwn * kFeedWarps);  // a lane reads and refills the same words of the slot
             // make the generic-proxy writes visible to the tensor core's async proxy
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0)
-                mbar_arrive(&b_full[s]);
+            if (lane == 0) {
+                ok = wait(&act_full[s], round & 1);
+                // descriptor addresses count 16-byte units
+                const uint64_t a_desc = a_desc0 + (uint64_t)(s * (S::kActStage >> 4));
+                const uint64_t b_desc = b_desc0 + (uint64_t)(s * (S::kBStage >> 4));
+                const int before = g - kAccGroups;  // the group whose sums lay in these units
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int u = g % kAccGroups * 2 + h;
+                    ok = ok && (before < 0 || wait(&acc_free[before % kFeedWarps * 2 + h],
+                                                   before / kFeedWarps & 1));
+                    if (!ok)
+                        break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)  // a K = 32 step = a 32-k block
+                        umma_i8(tmem_base + (uint32_t)(u * kAccCols + j * RP),
+                                a_desc + (uint64_t)((h * 2 + j) * 2),
+                                b_desc + (uint64_t)((h * 2 + j) * 2), idesc, 0u);
+                    umma_commit(&acc_full[u]);  // the unit's sums are complete
+                }
+                if (ok)
+                    umma_commit(&ab_free[s]);  // both operands' stages may be refilled
+            }
+            if (!__all_sync(0xffffffffu, ok))
+                break;
         }
+        if (!ok)
+            fail();
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else {
         // =============================== epilogue ====================================
-        const int ew = warp - kEpiWarp0;       // 0..15
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsEpi));
+        // the same in all lanes, and the compiler knows: fetch addresses in uniform registers
+        const int ew = __shfl_sync(0xffffffffu, warp, 0) - kEpiWarp0;  // 0..15
         const int ch = ew >> 2;                // column quarter
-        const int lq = warp & 3;               // TMEM lane quarter this warp may read
+        const int lq = ew & 3;                 // TMEM lane quarter this warp may read
         const int tok = tok0 + lq * 32 + lane;
         // a warp whose 32 tokens all lie past the last row has no chain to run
         const bool active = lq * 32 < m_here;
@@ -344,64 +340,74 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
         const uint32_t lane_addr = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(ch * CH);
         bool live = true;
         if (active) {
-            int u = 0, use = 0;  // unit buffer and how often it has been filled before
-            auto unit_wait = [&]() {
-                const bool ready = mbar_try_wait(&acc_full[u], use & 1);
+            auto unit_wait = [&](uint64_t* full, int parity) {
+                const bool ready = mbar_try_wait(full, parity);
                 if (!__all_sync(0xffffffffu, ready))
-                    live &= __all_sync(0xffffffffu, ready || wait(&acc_full[u], use & 1)) != 0;
+                    live &= __all_sync(0xffffffffu, ready || wait(full, parity)) != 0;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             };
-            auto unit_done = [&]() {  // every fetch of the unit is in registers
+            auto unit_done = [&](uint64_t* free) {  // every fetch of the unit is in registers
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0)
-                    mbar_arrive(&acc_free[u]);
-                if (++u == kAcc) {
-                    u = 0;
-                    ++use;
-                }
+                    mbar_arrive(free);
             };
             // A chunk is eight columns (the last one of a thread may be four) of two blocks.
             constexpr int kHalf = (CH + 7) / 8, kChunks = 2 * kHalf;  // per block pair, per group
             static_assert(CH % 4 == 0, "columns");
-            for (int g = 0; g < G; ++g) {
-                const float asv[4] = {a0.x, a0.y, a0.z, a0.w};
-                a0 = a1;
-                a1 = load_as(g + 2);
+            auto group = [&](int g, float4& scales) {
+                const float asv[4] = {scales.x, scales.y, scales.z, scales.w};
+                scales = load_as(g + 2);
                 const float* ws = wsf + g * RP;
+                const int u = g % kAccGroups * 2, parity = g / kAccGroups & 1;
+                uint64_t* free = acc_free + g % kFeedWarps * 2;
                 auto step = [&](auto chunk) {
                     constexpr int i = decltype(chunk)::value;
                     constexpr int j = i / kHalf * 2, c = i % kHalf * 8, W = c + 8 <= CH ? 8 : 4;
-                    constexpr int ju = j % kUnitBlocks;
-                    if constexpr (ju == 0 && c == 0)
-                        unit_wait();
+                    constexpr int h = j / 2;  // half of the group
+                    if constexpr (c == 0)
+                        unit_wait(&acc_full[u + h], parity);
                     uint32_t r[2][8];
-                    const uint32_t t = lane_addr + (uint32_t)(u * kAccCols + ju * RP + c);
+                    const uint32_t t = lane_addr + (uint32_t)((u + h) * kAccCols + c);
                     tmem_issue<W>(t, t + RP, r);
                     tmem_wait<W>(r);
-                    if constexpr (i + 1 == kChunks || (kUnitBlocks == 2 && i + 1 == kHalf))
-                        unit_done();
+                    if constexpr (i + 1 == kChunks || i + 1 == kHalf)
+                        unit_done(free + h);
                     // two blocks, in ascending order
                     const uint64_t s0 = b2w4_pack2(asv[j], asv[j]);
                     const uint64_t s1 = b2w4_pack2(asv[j + 1], asv[j + 1]);
 #pragma unroll
-                    for (int h = 0; h < W; h += 4) {
-                        const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(ws + c + h);
+                    for (int e4 = 0; e4 < W; e4 += 4) {
+                        const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(ws + c + e4);
                         auto sums = [&](int b, int e) {
                             return b2w4_pack2(__int2float_rn((int)r[b][e]),
                                               __int2float_rn((int)r[b][e + 1]));
                         };
-                        uint64_t& lo = acc2[(c + h) / 2];
-                        uint64_t& hi = acc2[(c + h) / 2 + 1];
-                        lo = b2w4_fma2(sums(0, h), b2w4_mul2(w2.x, s0), lo);
-                        hi = b2w4_fma2(sums(0, h + 2), b2w4_mul2(w2.y, s0), hi);
-                        lo = b2w4_fma2(sums(1, h), b2w4_mul2(w2.x, s1), lo);
-                        hi = b2w4_fma2(sums(1, h + 2), b2w4_mul2(w2.y, s1), hi);
+                        uint64_t& lo = acc2[(c + e4) / 2];
+                        uint64_t& hi = acc2[(c + e4) / 2 + 1];
+                        lo = b2w4_fma2(sums(0, e4), b2w4_mul2(w2.x, s0), lo);
+                        hi = b2w4_fma2(sums(0, e4 + 2), b2w4_mul2(w2.y, s0), hi);
+                        lo = b2w4_fma2(sums(1, e4), b2w4_mul2(w2.x, s1), lo);
+                        hi = b2w4_fma2(sums(1, e4 + 2), b2w4_mul2(w2.y, s1), hi);
                     }
                 };
                 [&]<int... I>(std::integer_sequence<int, I...>) {
                     (step(std::integral_constant<int, I>()), ...);
                 }(std::make_integer_sequence<int, kChunks>());
+            };
+            // Two groups a turn need no moves of the scales; the code is twice as long, which wide
+            // tiles pay for (measured: 112 columns 205 us a turn of two, 208 of one; 96 columns
+            // 27.4 / 26.7, 128 columns 395 / 389, 48 columns 50.0 / 51.4, 32 columns 37.2 / 38.6).
+            constexpr bool kPairs = RP <= 64 || RP == 112;
+            for (int g = 0; g < G; g += kPairs ? 2 : 1) {
+                group(g, a0);
+                if constexpr (!kPairs) {
+                    const float4 t = a0;  // of the group after the next
+                    a0 = a1;
+                    a1 = t;
+                } else if (g + 1 < G) {
+                    group(g + 1, a1);
+                }
             }
         }
         if (!live)
@@ -454,7 +460,7 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == kMmaWarp) {
+    if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                      ::"r"(tmem_base), "r"(512)
