@@ -138,13 +138,22 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
     return d;
 }
 
+// Where a group's codes lie: its four 32-blocks (16 even-k codes, then 16 odd-k codes) in an order
+// that turns with the group, block s at place s ^ (g % 4).  The four groups that a warp reads with
+// one load are 128 bytes apart and would share their banks (a load took four passes, and the
+// shared-memory pipe was busy for 49 % of an lm_head).  us per launch, graph replay: [151936, 2560]
+// 41.0 -> 39.7, [19456, 2560] 7.46 -> 7.14, [6144, 2560] 3.60 -> 3.39, [9728, 2560] 4.35 -> 4.23,
+// [2560, 4096] 3.84 -> 3.74; a decode step of eight layers behind 300 keys 330.5 -> 324.2.
+__device__ __forceinline__ int code_place(int s, int g) { return s ^ (g & 3); }
+
 // Integer sum of one weight row and group: wt = the row's four 16-byte chunks (one every eight
 // uint4), qa = the group's even / odd de-interleaved codes, es = -8 * sum of the even-k codes.
-__device__ __forceinline__ int group_sum(const uint4* wt, const uint4* qa, int es) {
+__device__ __forceinline__ int group_sum(const uint4* wt, const uint4* qa, int es, int g) {
     int pt = es, qt = 0;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-        const uint4 w = wt[s * 8], ae = qa[s * 2], ao = qa[s * 2 + 1];
+        const int at = code_place(s, g) * 2;
+        const uint4 w = wt[s * 8], ae = qa[at], ao = qa[at + 1];
         int p = dp4a_us((w.x ^ 0x08080808u) & 0x0F0F0F0Fu, ae.x, 0);
         int q = __dp4a((int)(w.x & 0xF0F0F0F0u), (int)ao.x, 0);
         p = dp4a_us((w.y ^ 0x08080808u) & 0x0F0F0F0Fu, ae.y, p);
@@ -354,7 +363,7 @@ gemv_w4a8_kernel(const GemvArgs a) {
             }
             // 32-block h/4 is stored as 16 even-k codes then 16 odd-k codes
             uint8_t* blk = reinterpret_cast<uint8_t*>(s_qa) + (size_t)mi * K + (size_t)g * 128 +
-                           (h >> 2) * 32;
+                           code_place(h >> 2, g) * 32;
             const int j = (h & 3) * 4;
             *reinterpret_cast<char4*>(blk + j) = make_char4(
                 (signed char)c[0], (signed char)c[2], (signed char)c[4], (signed char)c[6]);
@@ -407,7 +416,8 @@ gemv_w4a8_kernel(const GemvArgs a) {
                     int pt = 0, qt = 0;
 #pragma unroll
                     for (int s = 0; s < 4; ++s) {
-                        const uint4 ae = qa[s * 2], ao = qa[s * 2 + 1];
+                        const int place = code_place(s, gl) * 2;  // g % 4 == gl
+                        const uint4 ae = qa[place], ao = qa[place + 1];
                         // two independent chains per sub-block hide dp4a latency
                         int p = dp4a_us(wl[s * 4 + 0], ae.x, 0);
                         int q = __dp4a((int)wh[s * 4 + 0], (int)ao.x, 0);
@@ -591,7 +601,8 @@ gemv_w4a8_split_kernel(const GemvArgs a) {
                 s_as[g] = scale;
                 s_es[g] = -8 * esum;
             }
-            uint8_t* blk = reinterpret_cast<uint8_t*>(s_qa) + (size_t)g * 128 + (h >> 2) * 32;
+            uint8_t* blk =
+                reinterpret_cast<uint8_t*>(s_qa) + (size_t)g * 128 + code_place(h >> 2, g) * 32;
             const int j = (h & 3) * 4;
             *reinterpret_cast<char4*>(blk + j) = make_char4(
                 (signed char)c[0], (signed char)c[2], (signed char)c[4], (signed char)c[6]);
@@ -615,7 +626,7 @@ gemv_w4a8_split_kernel(const GemvArgs a) {
         if (g < n_g) {
             const int at = tl * per + g;
             const int d = group_sum(reinterpret_cast<const uint4*>(s_w) + at * 32 + row,
-                                    s_qa + g * 8, s_es[g]);
+                                    s_qa + g * 8, s_es[g], gl);
             const float ws = SCL16 ? __half2float(reinterpret_cast<const __half*>(s_scl)[at * 8 + row])
                                    : reinterpret_cast<const float*>(s_scl)[at * 8 + row];
             const int slot = (tl / kSplit) * a.d_stride + (g0 + g) * 8 + row, owner = tl % kSplit;
