@@ -16,6 +16,8 @@
 // thread in a fixed order.
 #include <type_traits>
 
+#include <cooperative_groups.h>
+
 #include "b200w4_internal.cuh"
 
 namespace {
@@ -183,14 +185,11 @@ __global__ void moe_router_logits_scalar_kernel(const float* __restrict__ hidden
 constexpr int kMaxTopK = 16;
 constexpr int kSelectMaxExperts = 1024;  // 32 lanes x 32 logits in registers
 
-// routes of token t, by one warp; also returns lane j's expert (lanes >= top_k: undefined).
-// NS = logits per lane (32 * NS >= experts).
+// The first `rounds` routes of a token, by one warp: lane j gets the j-th expert and its logit
+// (lanes from `rounds` on: expert 0, -inf).  NS = logits per lane (32 * NS >= experts).
 template <int NS>
-__device__ __forceinline__ int select_routes_warp(const float* logits, int t,
-                                                  int num_experts, int top_k,
-                                                  int32_t* __restrict__ idx,
-                                                  float* __restrict__ weights, int lane) {
-    const float* row = logits + (size_t)t * num_experts;
+__device__ __forceinline__ int pick_routes_warp(const float* row, int num_experts, int rounds,
+                                                int lane, float& logit) {
     // the lane's logits (experts lane, lane+32, ...) stay in registers for all k rounds
     float mine[NS];
 #pragma unroll
@@ -208,7 +207,7 @@ __device__ __forceinline__ int select_routes_warp(const float* logits, int t,
         const uint32_t u = __float_as_uint(v);
         key[s] = !(v > -INFINITY) ? 0u : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
     }
-    for (int j = 0; j < top_k; ++j) {
+    for (int j = 0; j < rounds; ++j) {
         uint32_t bk = 0u;
         int bs = 0;
 #pragma unroll
@@ -232,6 +231,31 @@ __device__ __forceinline__ int select_routes_warp(const float* logits, int t,
             my_e = (int)we;
         }
     }
+    logit = my_v;
+    return my_e;
+}
+
+// dispatch on the number of experts
+__device__ __forceinline__ int pick_routes_any(const float* row, int num_experts, int rounds,
+                                               int lane, float& logit) {
+    if (num_experts <= 128)
+        return pick_routes_warp<4>(row, num_experts, rounds, lane, logit);
+    if (num_experts <= 256)
+        return pick_routes_warp<8>(row, num_experts, rounds, lane, logit);
+    if (num_experts <= 512)
+        return pick_routes_warp<16>(row, num_experts, rounds, lane, logit);
+    return pick_routes_warp<kSelectMaxExperts / 32>(row, num_experts, rounds, lane, logit);
+}
+
+// Routes of token t, by one warp; also returns lane j's expert (lanes >= top_k: undefined).
+template <int NS>
+__device__ __forceinline__ int select_routes_warp(const float* logits, int t,
+                                                  int num_experts, int top_k,
+                                                  int32_t* __restrict__ idx,
+                                                  float* __restrict__ weights, int lane) {
+    float my_v;
+    const int my_e = pick_routes_warp<NS>(logits + (size_t)t * num_experts, num_experts, top_k,
+                                          lane, my_v);
     const float maximum = __shfl_sync(0xffffffffu, my_v, 0);
     // exp in fp64 and one rounding: agrees with a correctly rounded expf
     const float ex = lane < top_k ? (float)exp((double)__fsub_rn(my_v, maximum)) : 0.f;
@@ -353,11 +377,13 @@ moe_compact_kernel(const int32_t* __restrict__ idx, int tokens, int top_k, int n
 // One launch instead of four: every warp of the grid quantises its share of the hidden rows
 // and computes its share of the router logits; the block that arrives last at a counter (no
 // block waits for another) selects the routes, one warp per token, and compacts them.  Same
-// device functions, same bits as the separate kernels.
+// device functions, same bits as the separate kernels.  !SELECT: it ends with the logits, see
+// GroupedSmallArgs.
 constexpr int kFusedSwigluTokens = 4;
 constexpr int kFusedTokens = 8;
 constexpr int kFusedRoutes = 128;
 constexpr int kFusedThreads = 128;
+template <bool SELECT>
 __global__ void __launch_bounds__(kFusedThreads)
 moe_route_fused_kernel(const float* __restrict__ hidden, int ldx, int tokens, int hidden_size,
                        const __half* __restrict__ router, int num_experts, int top_k,
@@ -404,6 +430,8 @@ moe_route_fused_kernel(const float* __restrict__ hidden, int ldx, int tokens, in
                 router_logits_warp<1, kRouterTok>(hidden, ldx, tokens, hidden_size, router,
                                                   num_experts, logits, t0, e, lane);
     }
+    if constexpr (!SELECT)
+        return;
     // arrival: the last block to get here sees every block's logits
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -801,6 +829,8 @@ moe_combine_staged_kernel(unsigned long long* stage, int stage_rows,
 constexpr int kSW = 8;          // warps
 constexpr int kST = kSW * 32;
 constexpr int kSR = 8;          // routes per pass
+constexpr int kSmallTiles = 16; // tiles per CTA at most
+constexpr int kCombineCluster = 8;
 
 struct GroupedSmallArgs {
     const uint8_t* nib;
@@ -810,6 +840,18 @@ struct GroupedSmallArgs {
     const float* gate_up;     // if set (few routes): the activations are silu(gate)*up of these
                               // fp32 [routes][2K] rows, quantised here instead of read from qa
     const int4* slots;        // y-th expert with routes: (expert, first route, end), else empty
+    // One token, route y is its y-th.  First matmul (kFromLogits): every block picks its own route
+    // from the logits (y + 1 rounds), and the first one writes them all.  (The block that selects
+    // and compacts in the router kernel waits for the others' logits through a fence and a
+    // counter, and this kernel for that block.)  Second matmul (kFromRoutes): idx is read.
+    const float* logits;
+    int num_experts, top_k;
+    int32_t* idx;
+    float* weights;
+    // One token, second matmul: the routes' blocks of one tile range are a cluster (along x), which
+    // combines their rows through distributed shared memory into this row (null: `out` and a
+    // combine launch)
+    float* combined;
     int expert_begin;         // first expert whose weights this aggregate holds
     int expert_count;         // experts held
     const int32_t* row_map;   // route -> activation row, or null for identity
@@ -833,19 +875,34 @@ __device__ __forceinline__ void moe_mma_16x8x32(int (&d)[4], uint32_t a0, uint32
           "r"(c.w));
 }
 
-template <bool SCL16>
+// Where a block's route comes from: the slot records, the logits, the list of the token's routes.
+constexpr int kFromSlots = 0, kFromLogits = 1, kFromRoutes = 2;
+template <bool SCL16, int FROM>
 __global__ void __launch_bounds__(kST, 2)
 moe_grouped_small_kernel(const GroupedSmallArgs a) {
     b2w4_pdl_chain_entry();
     extern __shared__ __align__(128) uint8_t smem[];
     // blockIdx.y walks the experts that have routes, not all experts: a decode token
     // touches top_k of them
-    const int4 slot = a.slots[blockIdx.y];
+    const bool combined = FROM == kFromRoutes && a.combined;
+    const int y = combined ? blockIdx.x : blockIdx.y, x = combined ? blockIdx.y : blockIdx.x;
+    int4 slot = make_int4(0, y, y + 1, 0);
+    if (FROM == kFromSlots) {
+        slot = a.slots[y];
+    } else if (FROM == kFromLogits) {
+        // by every warp: no barrier before the weights are asked for
+        float logit;
+        const int picked =
+            pick_routes_any(a.logits, a.num_experts, y + 1, threadIdx.x & 31, logit);
+        slot.x = __shfl_sync(0xffffffffu, picked, y);
+    } else {
+        slot.x = a.idx[y];
+    }
     const int e_all = slot.x, r0 = slot.y, r1 = slot.z;
     const int e = e_all - a.expert_begin;  // index inside the aggregate held here
     if (e < 0 || e >= a.expert_count)
         return;
-    const int tl0 = blockIdx.x * a.tpc;
+    const int tl0 = x * a.tpc;
     const int ntile = min(a.tpc, a.tiles_e - tl0);
     if (r0 >= r1 || ntile <= 0)
         return;
@@ -878,6 +935,9 @@ moe_grouped_small_kernel(const GroupedSmallArgs a) {
         }
     }
     __syncthreads();  // no warp polls the barrier word before it is one
+    if (FROM == kFromLogits && x == 0 && y == 0 && warp == kSW - 1)
+        select_routes_any(a.logits, 0, a.num_experts, a.top_k, a.idx, a.weights, lane);
+    __shared__ float s_row[FROM == kFromRoutes ? kSmallTiles * 8 : 1];  // this route's rows
     const int npair = (ntile + 1) >> 1;
     const int n_items = npair * G;
     const uint32_t* s_w32 = reinterpret_cast<const uint32_t*>(s_w);
@@ -900,13 +960,13 @@ moe_grouped_small_kernel(const GroupedSmallArgs a) {
         } else {
             for (int i = threadIdx.x; i < mc * (K / 16); i += kST) {
                 const int mi = i / (K / 16), c = i - mi * (K / 16);
-                const int src_row = a.row_map ? a.row_map[base + mi] : base + mi;
+                const int src_row = FROM == kFromLogits ? 0 : a.row_map ? a.row_map[base + mi] : base + mi;
                 s_qa[mi * (K / 16) + c] =
                     reinterpret_cast<const uint4*>(a.qa + (size_t)src_row * K)[c];
             }
             for (int i = threadIdx.x; i < mc * G; i += kST) {
                 const int mi = i / G, g = i - mi * G;
-                const int src_row = a.row_map ? a.row_map[base + mi] : base + mi;
+                const int src_row = FROM == kFromLogits ? 0 : a.row_map ? a.row_map[base + mi] : base + mi;
                 s_as[mi * G + g] = a.as[(size_t)src_row * G + g];
             }
         }
@@ -981,7 +1041,9 @@ moe_grouped_small_kernel(const GroupedSmallArgs a) {
                 acc = __fmaf_rn(dsrc[g * kSR * 8], __fmul_rn(ws, as[g]), acc);
             }
             const int n = (tl0 + tl) * 8 + rr;
-            if (n < a.n_e) {
+            if (combined) {
+                s_row[tl * 8 + rr] = acc;
+            } else if (n < a.n_e) {
                 if (a.peers.world == 0) {
                     a.out[(size_t)(base + mi) * a.n_e + n] = acc;
                 } else {
@@ -1004,6 +1066,33 @@ moe_grouped_small_kernel(const GroupedSmallArgs a) {
             }
         }
         __syncthreads();
+    }
+    if (combined) {
+        // moe_combine_kernel's sum over the routes in ascending expert id, each block its share of
+        // the tile range's rows
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        const int routes = gridDim.x;
+        __shared__ int s_from[kCombineCluster];
+        __shared__ float s_weight[kCombineCluster];
+        if ((int)threadIdx.x < routes) {
+            const int j = threadIdx.x, key = a.idx[j];
+            int rank = 0;
+            for (int o = 0; o < routes; ++o) {
+                const int other = a.idx[o];
+                rank += other < key || (other == key && o < j);
+            }
+            s_from[rank] = j;
+            s_weight[rank] = a.weights[j];
+        }
+        cluster.sync();  // every route's rows, and the order
+        const int rows = min(ntile * 8, a.n_e - tl0 * 8);
+        for (int i = y * kST + threadIdx.x; i < rows; i += routes * kST) {
+            float acc = 0.f;
+            for (int j = 0; j < routes; ++j)
+                acc = __fmaf_rn(s_weight[j], cluster.map_shared_rank(s_row, s_from[j])[i], acc);
+            a.combined[tl0 * 8 + i] = acc;
+        }
+        cluster.sync();  // nobody leaves while its rows may still be read
     }
 }
 
@@ -1359,6 +1448,23 @@ int launch_grouped_as(b2w4_ctx* ctx, const GroupedArgs& a, bool scl16, size_t sm
     return B2W4_OK;
 }
 
+// Tiles per CTA of the few-token kernel.
+int small_tiles(const b2w4_weight* w) {
+    int tpc = kSmallTiles;
+    while (tpc > 2 &&
+           grouped_small_smem(w->k, w->groups, tpc, w->scales_fp16 != 0) > 113 * 1024)
+        tpc -= 2;  // even: tiles are taken in pairs
+    return tpc;
+}
+
+// The routes of a single token; logits null: read from idx.
+struct TokenRoutes {
+    const float* logits;
+    int32_t* idx;
+    float* weights;
+    float* combined;  // GroupedSmallArgs
+};
+
 // `decode` (few tokens): the shared-memory variant, optionally with SwiGLU + quantiser fused
 // into its prologue (fused_gate_up = the gate_up matmul's fp32 output).
 // qa32 / as32: the same rows quantised per 32 values, for experts that hold several routes
@@ -1368,7 +1474,7 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
                    int as_stride, const int8_t* qa32, const float* as32, int as32_stride,
                    const int4* slots, const int32_t* row_map, float* out, bool decode,
                    const float* fused_gate_up = nullptr, const b2w4_tp_args* peers = nullptr,
-                   int stage_rows = 0) {
+                   int stage_rows = 0, const TokenRoutes* token = nullptr) {
     const int n_e = w->n / expert_count;
     const bool scl16 = w->scales_fp16 != 0;
     const int slots_y = routes < num_experts_all ? routes : num_experts_all;  // grid.y
@@ -1379,6 +1485,14 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
         a.qa = qa;
         a.as = as;
         a.slots = slots;
+        if (token) {
+            a.logits = token->logits;
+            a.num_experts = num_experts_all;
+            a.top_k = routes;
+            a.idx = token->idx;
+            a.weights = token->weights;
+            a.combined = token->combined;
+        }
         a.gate_up = fused_gate_up;
         a.expert_begin = expert_begin;
         a.expert_count = expert_count;
@@ -1393,20 +1507,29 @@ int launch_grouped(b2w4_ctx* ctx, const b2w4_weight* w, int num_experts_all, int
         a.groups = w->groups;
         a.n_e = n_e;
         a.tiles_e = n_e / 8;
-        int tpc = 16;
-        while (tpc > 2 && grouped_small_smem(w->k, w->groups, tpc, scl16) > 113 * 1024)
-            tpc -= 2;  // even: tiles are taken in pairs
+        const int tpc = small_tiles(w);
         a.tpc = tpc;
         a.d_stride = grouped_small_d_stride(w->groups);
         const size_t smem = grouped_small_smem(w->k, w->groups, tpc, scl16);
         if (w->k > (scl16 ? 10752 : 10624))  // the limit of the operator
             return b2w4_fail(ctx, B2W4_E_INVALID, "moe: K=%d needs %zu B shared memory", w->k,
                              smem);
-        auto kern = scl16 ? moe_grouped_small_kernel<true> : moe_grouped_small_kernel<false>;
-        static b2w4_smem_optin configured[2];  // per instantiation and device
-        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[scl16]));
-        dim3 grid((a.tiles_e + tpc - 1) / tpc, slots_y);
-        B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kST), smem, ctx->stream, a));
+        const int from = !token ? kFromSlots : token->logits ? kFromLogits : kFromRoutes;
+        auto kern = from == kFromSlots ? (scl16 ? moe_grouped_small_kernel<true, kFromSlots>
+                                                : moe_grouped_small_kernel<false, kFromSlots>)
+                    : from == kFromLogits ? (scl16 ? moe_grouped_small_kernel<true, kFromLogits>
+                                                   : moe_grouped_small_kernel<false, kFromLogits>)
+                                          : (scl16 ? moe_grouped_small_kernel<true, kFromRoutes>
+                                                   : moe_grouped_small_kernel<false, kFromRoutes>);
+        static b2w4_smem_optin configured[6];  // per instantiation and device
+        B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured[from * 2 + scl16]));
+        const int ranges = (a.tiles_e + tpc - 1) / tpc;
+        if (a.combined)
+            B2W4_CUDA(ctx, b2w4_launch_chained_cluster(ctx->pdl, kern, dim3(slots_y, ranges),
+                                                       dim3(kST), slots_y, smem, ctx->stream, a));
+        else
+            B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(ranges, slots_y), dim3(kST),
+                                               smem, ctx->stream, a));
         ctx->launches++;
         return B2W4_OK;
     }
@@ -1553,11 +1676,25 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
         (reinterpret_cast<uintptr_t>(hidden_dev) | reinterpret_cast<uintptr_t>(router)) % 16 == 0 &&
         ldx % 4 == 0;
     const bool fused = aligned && tokens <= kFusedTokens && routes <= kFusedRoutes;
+    // compact positions stay global; the grouped kernels skip experts held elsewhere
+    const int32_t* local_offsets = offsets + expert_begin;
+    const bool partial = expert_count != num_experts;
+    // One token with all experts here: routes need no compaction, each block of the first expert
+    // matmul picks its own, and the second one combines its rows.  Measured: 8 of 128 experts of
+    // 768, rows of 2048, 22.6 -> 17.8 us (19.9 with a combine launch); 8 of 64 of 1024, 3072, 29.0
+    // -> 24.8; 8 of 128 of 1536, 4096, 48.3 -> 46.9; 4 of 64 of 384, 1024, 19.2 -> 16.5.  Tried: the
+    // second matmul's weights brought to L2 by the first (no gain).
+    const bool single = fused && tokens == 1 && !partial && !peers && !route_out;
+    const bool in_cluster = single && top_k <= kCombineCluster;
+    const TokenRoutes first = {logits, idx, wts, nullptr};
+    const TokenRoutes second = {nullptr, idx, wts, in_cluster ? out_dev : nullptr};
     if (fused) {
         // enough blocks to spread the router rows over the SMs, one warp per expert
         const int blocks = (num_experts + kFusedThreads / 32 - 1) / (kFusedThreads / 32);
         B2W4_CUDA(ctx, b2w4_launch_chained(
-                           ctx->pdl, moe_route_fused_kernel, dim3(blocks), dim3(kFusedThreads),
+                           ctx->pdl, single ? moe_route_fused_kernel<false>
+                                            : moe_route_fused_kernel<true>,
+                           dim3(blocks), dim3(kFusedThreads),
                            sizeof(int) * (num_experts + 1), st, hidden_dev, ldx, tokens,
                            hidden_size, router, num_experts, top_k, logits, idx, wts, offsets,
                            route_token, pos, slots, q_hidden, as_hidden, ctx->flag_dev + 4));
@@ -1604,12 +1741,10 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
                                            as_hidden, q_hidden32, as_hidden32));
         ctx->launches++;
     }
-    // compact positions stay global; the grouped kernels skip experts held elsewhere
-    const int32_t* local_offsets = offsets + expert_begin;
-    const bool partial = expert_count != num_experts;
     if ((rc = launch_grouped(ctx, gate_up, num_experts, expert_begin, expert_count, routes,
                              q_hidden, as_hidden, gh, q_hidden32, as_hidden32, gh * 4, slots,
-                             route_token, static_cast<float*>(gu), decode)) != B2W4_OK)
+                             single ? nullptr : route_token, static_cast<float*>(gu), decode,
+                             nullptr, nullptr, 0, single ? &first : nullptr)) != B2W4_OK)
         return rc;
     // few routes: SwiGLU and its quantiser run inside the down-projection's CTAs
     const bool fuse_swiglu = decode;
@@ -1632,7 +1767,8 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
                              rule32 ? as_inter : nullptr, gi * 4, slots, nullptr,
                              static_cast<float*>(dn), decode,
                              fuse_swiglu ? static_cast<const float*>(gu) : nullptr,
-                             fused_handover ? peers : nullptr, stage_rows)) != B2W4_OK)
+                             fused_handover ? peers : nullptr, stage_rows,
+                             single ? &second : nullptr)) != B2W4_OK)
         return rc;
     if (route_out) {
         dim3 grid((hidden_size / 4 + 255) / 256, routes);
@@ -1659,12 +1795,13 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
                            reinterpret_cast<unsigned*>(ctx->flag_dev + 6), ctx->status_dev,
                            ctx->peer_wait_cycles));
         ctx->launches++;
-    } else if (out_dev) {
+    } else if (out_dev && !in_cluster) {
         dim3 grid((hidden_size / 4 + kCombineThreads - 1) / kCombineThreads, tokens);
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, moe_combine_kernel, grid,
                                            dim3(kCombineThreads), 0, st,
-                                           static_cast<const float*>(dn), idx, wts, pos, tokens,
-                                           top_k, hidden_size, out_dev, ldo));
+                                           static_cast<const float*>(dn), idx, wts,
+                                           single ? nullptr : pos, tokens, top_k, hidden_size,
+                                           out_dev, ldo));
         ctx->launches++;
     }
     B2W4_CUDA(ctx, cudaGetLastError());

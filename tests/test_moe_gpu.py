@@ -383,6 +383,31 @@ def test_grouped_matmul_pass_edges(ctx, t, h, inter, rule):
     check_against_oracle(got, want)
 
 
+@pytest.mark.parametrize("h,e,top_k,inter", [
+    (128, 8, 1, 128), (128, 40, 3, 128), (1152, 130, 5, 384), (384, 16, 7, 256), (2048, 300, 8, 768),
+    (256, 600, 9, 128), (256, 16, 16, 128),  # more routes than a cluster: a combine launch
+    (128, 4, 4, 6144)])                      # several waves of blocks
+@pytest.mark.parametrize("router_kind", ["usual", "ties", "nan"])
+def test_one_token(ctx, h, e, top_k, inter, router_kind):
+    """One token: every block of the first expert matmul picks its route, the second one combines
+    in a cluster of the routes (of every size), rows and tiles that fill no block; equal logits
+    (ties to the lower expert) and logits that are NaN (they never qualify)."""
+    hidden = pkg.synth.activations(7, 31 + h + e, 1, h)
+    router = pkg.synth.router_weight(20261125, 41 + e, e, h, std=0.3)
+    if router_kind == "ties":
+        router[:] = router[e // 2]
+    elif router_kind == "nan":
+        router[::2] = np.float16(np.nan)
+    gu = pkg.synth.bg128_weight(20261125, 51 + e, e * 2 * inter, h)
+    dn = pkg.synth.bg128_weight(20261125, 61 + e, e * h, inter)
+    got = run_moe(ctx, hidden, router, top_k, inter, gu, dn)
+    want = ol.moe_forward(hidden, router, top_k, inter, gu, dn, rule=REF)
+    if router_kind == "nan":  # the placeholder slots repeat an expert; logits are NaN on both sides
+        assert (np.isnan(got[1]) == np.isnan(want[1])).all()
+        got, want = ((o, np.nan_to_num(l), i, w) for o, l, i, w in (got, want))
+    check_against_oracle(got, want)
+
+
 def test_one_token_behind_kernels_that_fill_shared_memory(ctx):
     """The one-token expert matmul waits on a barrier word in shared memory that it makes itself:
     whatever the kernel before left there, all ones or zeros, every call gives the same bits.
