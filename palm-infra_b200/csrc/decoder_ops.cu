@@ -525,6 +525,15 @@ struct PrepArgs {
     float eps;
     float *k_cache, *v_cache;
 };
+// RING: the block is alone on its multiprocessor, so key and value rows go through a ring of slots
+// per warp in its shared memory (cp.async): first the warp's keys, then its values, a slot as soon
+// as it has been read, from before the query rows are made to the last value row.  No warp waits for
+// another, and every key and value stays with the warp and lanes that have it without the ring: the
+// same bits.  What it mends: with loads into registers (8 KB of keys or 4 KB of values in flight per
+// warp) each pass over the block's keys waits for its memory round trip, and nothing is on its way
+// while the query rows are made.  (By bulk copies, 2 KB of keys or 512 bytes of values each, a step
+// of eight layers behind 6000 keys took 581 us instead of 455.)
+constexpr int kRingSlots = 5, kSlotBytes = 2048;
 constexpr int kMaxRanges = 16;
 // blocks per multiprocessor that the registers allow
 constexpr int split_blocks(int dim, int hr) { return dim * hr <= 128 ? 4 : dim * hr <= 256 ? 3 : 2; }
@@ -541,8 +550,8 @@ struct SplitSmem {  // floats of dynamic shared memory before the scores
     static constexpr int kScores = (kOdd + 2 + 3) & ~3;         // [keys][HR]
 };
 // k_cache, v_cache: no __restrict__, with PREP the block reads a row that it wrote
-template <int DIM, int HR, int CTAS, bool PREP>
-__global__ void __launch_bounds__(kAttnThreads, split_blocks(DIM, HR))
+template <int DIM, int HR, int CTAS, bool PREP, bool RING>
+__global__ void __launch_bounds__(kAttnThreads, RING ? 2 : split_blocks(DIM, HR))
 attention_split_kernel(const float* __restrict__ q, const float* k_cache, const float* v_cache,
                        float* __restrict__ out, int tokens, int heads, int kv_heads, int past0,
                        const int* __restrict__ past_dev, int capacity, float scale, int one_range,
@@ -575,11 +584,52 @@ attention_split_kernel(const float* __restrict__ q, const float* k_cache, const 
     const float* kc = k_cache + ((size_t)kvh * capacity + j0) * DIM;
     const float* vc = v_cache + ((size_t)kvh * capacity + j0) * DIM;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // value rows: a warp per key (two for 64 features)
+    constexpr int kLanes = DIM / 4 < 32 ? DIM / 4 : 32;  // lanes per value row
+    constexpr int kV4 = DIM / 4 / kLanes;                // float4 per lane
+    constexpr int kKeys = 32 / kLanes;                   // keys per warp and step
+    // RING: a slot holds kSlotKeys keys in a row, or four value steps, of 512 bytes each
+    constexpr int kSlotKeys = kSlotBytes / (DIM * 4), kSlotSteps = kSlotBytes / 512;
+    uint8_t* ring = nullptr;
+    int key_slots = 0, slots = 0, issued = 0;
+    // Copies of slot `i` of the warp's sequence, one group even where there is nothing.
+    auto issue = [&](int i) {
+        uint8_t* dst = ring + i % kRingSlots * kSlotBytes + lane * 16;
+        if (i < slots) {
+            const bool keys = i < key_slots;
+            const int key0 = (i * kAttnWarps + warp) * kSlotKeys;
+            const int step0 = (i - key_slots) * kSlotSteps;
+#pragma unroll
+            for (int u = 0; u < kSlotSteps; ++u) {  // 512 bytes a step
+                const int key = (keys ? key0 + u * kKeys : ((step0 + u) * kAttnWarps + warp) * kKeys) +
+                                lane / kLanes;
+                if (key < n)
+                    cp_async16(reinterpret_cast<float*>(dst + u * 512),
+                               (keys ? kc : vc) + (size_t)key * DIM + lane % kLanes * 4, true);
+            }
+        }
+        cp_async_commit();
+    };
+    const bool owner = n > 0 && j0 + n == visible;  // of the new key, the last one
+    if constexpr (RING) {
+        ring = reinterpret_cast<uint8_t*>(
+                   (reinterpret_cast<uintptr_t>(s_sc + n * HR) + 127) & ~uintptr_t(127)) +
+               warp * kRingSlots * kSlotBytes;
+        // slots that begin before key n, of every eighth
+        auto share = [&](int unit) { return ((n + unit - 1) / unit - warp + kAttnWarps - 1) / kAttnWarps; };
+        key_slots = share(kSlotKeys);
+        slots = key_slots + (share(kKeys) + kSlotSteps - 1) / kSlotSteps;
+        // what does not wait for the new key's row: the keys before its slot
+        const bool last = owner && PREP && (n - 1) / kSlotKeys % kAttnWarps == warp;
+        issued = min(kRingSlots, !owner || !PREP ? slots : last ? key_slots - 1 : key_slots);
+        for (int i = 0; i < issued; ++i)
+            issue(i);
+    }
     if (PREP) {  // query rows to the head of s_acc, which is free until P*V
         const float* cosv = prep.cosv + (size_t)past * (DIM / 2);
         const float* sinv = prep.sinv + (size_t)past * (DIM / 2);
         const size_t row = ((size_t)kvh * capacity + past) * DIM;
-        const bool owner = n > 0 && j0 + n == visible;  // of the new key, the last one
         if (warp < nh) {
             prepare_row<DIM>(prep.qkv + row0 + warp * DIM, prep.q_weight, prep.eps, cosv, sinv,
                              lane, s_acc + warp * DIM);
@@ -594,6 +644,19 @@ attention_split_kernel(const float* __restrict__ q, const float* k_cache, const 
         }
         __syncthreads();
     }
+    if constexpr (RING)
+        for (int i = issued; i < kRingSlots; ++i)
+            issue(i);
+    // Slot i of the warp's sequence, when it is there; after it has been read.
+    auto take = [&](int i) {
+        cp_async_wait<kRingSlots - 1>();
+        __syncwarp();
+        return ring + i % kRingSlots * kSlotBytes;
+    };
+    auto release = [&](int i) {
+        __syncwarp();
+        issue(i + kRingSlots);
+    };
 
     // ---- scores ----
     {
@@ -615,16 +678,21 @@ attention_split_kernel(const float* __restrict__ q, const float* k_cache, const 
         auto score = [&](auto in_flight) {
             constexpr int KI = decltype(in_flight)::value;
             constexpr int kItems = KI * HR;
-            for (int j = warp * 4 * KI; j < n; j += kAttnWarps * 4 * KI) {
+            for (int j = warp * 4 * KI, slot = 0; j < n; j += kAttnWarps * 4 * KI, ++slot) {
                 float4 kr[KI][kF4];
+                // past the end: dropped below
+                const float* rows =
+                    RING ? reinterpret_cast<const float*>(take(slot)) : kc + (size_t)j * DIM;
 #pragma unroll
                 for (int it = 0; it < KI; ++it)
 #pragma unroll
                     for (int i = 0; i < kF4; ++i) {
-                        const int key = min(j + it * 4 + sub, n - 1);  // past the end: dropped below
-                        kr[it][i] = *reinterpret_cast<const float4*>(kc + (size_t)key * DIM + 32 * i +
+                        const int key = RING ? it * 4 + sub : min(it * 4 + sub, n - 1 - j);
+                        kr[it][i] = *reinterpret_cast<const float4*>(rows + key * DIM + 32 * i +
                                                                      4 * part);
                     }
+                if constexpr (RING)
+                    release(slot);
                 float v[kItems];  // item it * HR + h
 #pragma unroll
                 for (int it = 0; it < KI; ++it)
@@ -667,19 +735,17 @@ attention_split_kernel(const float* __restrict__ q, const float* k_cache, const 
                 }
             }
         };
-        if (n <= 4 * kAttnWarps)
+        if constexpr (RING)
+            score(std::integral_constant<int, kSlotKeys / 4>());
+        else if (n <= 4 * kAttnWarps)
             score(std::integral_constant<int, 1>());
         else
             score(std::integral_constant<int, (DIM > 128 ? 2 : 4)>());
     }
     __syncthreads();
 
-    // value rows: a warp per key (two for 64 features), U steps of keys in flight; the first
-    // ones are on their way during the softmax
-    constexpr int kLanes = DIM / 4 < 32 ? DIM / 4 : 32;  // lanes per value row
-    constexpr int kV4 = DIM / 4 / kLanes;                // float4 per lane
-    constexpr int kKeys = 32 / kLanes;                   // keys per warp and step
-    constexpr int U = 8 / kV4;                           // steps in flight
+    // U steps of value rows in flight; the first ones are on their way during the softmax
+    constexpr int U = RING ? kSlotSteps : 8 / kV4;
     const int v_part = lane % kLanes, v_sub = lane / kLanes, v_first = warp * kKeys + v_sub;
     float4 vr[U][kV4];
     auto fetch_values = [&](int j) {
@@ -692,7 +758,7 @@ attention_split_kernel(const float* __restrict__ q, const float* k_cache, const 
                                                             4 * (v_part + kLanes * i));
             }
     };
-    if (v_first < n)
+    if (!RING && v_first < n)
         fetch_values(v_first);
 
     // ---- softmax over the block's keys; a thread's items all belong to head tid % HR ----
@@ -743,9 +809,17 @@ attention_split_kernel(const float* __restrict__ q, const float* k_cache, const 
 #pragma unroll
             for (int i = 0; i < 2 * kV4; ++i)
                 acc[h][i] = 0;
-        for (int j = v_first; j < n; j += kAttnWarps * kKeys * U) {
-            if (j != v_first)
+        for (int j = v_first, slot = key_slots; RING ? slot < slots : j < n;
+             j += kAttnWarps * kKeys * U, ++slot) {
+            if constexpr (RING) {
+                const uint8_t* rows = take(slot);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    vr[u][0] = *reinterpret_cast<const float4*>(rows + u * 512 + lane * 16);
+                release(slot);
+            } else if (j != v_first) {
                 fetch_values(j);
+            }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int key = j + u * kAttnWarps * kKeys;
@@ -1080,15 +1154,17 @@ bool attn_tensor(int tokens, int heads, int dim, int capacity, int sm_count) {
            (long)tokens * heads >= (dim == 128 ? 40l : 160l) * sm_count;
 }
 
-// Whether the device can hold a cluster of the kernel (a slice of it may not have sixteen, or
+// Clusters of the kernel that the device holds at once (a slice of it may not have sixteen, or
 // eight, multiprocessors side by side).
 constexpr size_t kMaxBlockSmem = 220 * 1024;
+// more dynamic shared memory than this, and a multiprocessor holds one block
+constexpr size_t kHalfSmem = 114 * 1024;
 template <typename Kernel>
-bool cluster_fits(Kernel kern, int ctas) {
+int clusters_held(Kernel kern, int ctas, size_t smem) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(kAttnThreads);
-    cfg.dynamicSmemBytes = 32 * 1024;
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = ctas;
@@ -1097,34 +1173,46 @@ bool cluster_fits(Kernel kern, int ctas) {
     cfg.numAttrs = 1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
-        return true;
+        return n;
     (void)cudaGetLastError();
-    return false;
+    return 0;
 }
 
-template <int DIM, int HR, int CTAS, bool PREP>
+template <int DIM, int HR, int CTAS, bool PREP, bool RING>
 int launch_split_as(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
                     bool* placed) {
-    static b2w4_smem_optin cfg, wide, fits;  // fits: 1 yes, 2 no, per device
-    auto kern = attention_split_kernel<DIM, HR, CTAS, PREP>;
+    static b2w4_smem_optin cfg, wide;
+    static b2w4_smem_optin held, held_alone;  // clusters_held + 1, per device
+    auto kern = attention_split_kernel<DIM, HR, CTAS, PREP, RING>;
     const PrepArgs prep = PREP ? *a.prep : PrepArgs();
     const int range = max((keys + CTAS - 1) / CTAS, min(keys, plan.one_range));
-    const size_t smem = sizeof(float) * (SplitSmem<DIM, HR>::kScores + (size_t)range * HR);
+    size_t smem = sizeof(float) * (SplitSmem<DIM, HR>::kScores + (size_t)range * HR);
+    if (RING)
+        smem += 128 + kAttnWarps * kRingSlots * kSlotBytes;
     const dim3 grid(CTAS, a.kv_heads * ((a.heads / a.kv_heads + HR - 1) / HR), a.tokens);
-    if (smem > kMaxBlockSmem)
+    if (smem > (RING ? kHalfSmem : kMaxBlockSmem))
         return B2W4_OK;  // not placed
-    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, cfg));
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, RING ? kHalfSmem + 1 : smem, cfg));
+    if constexpr (CTAS > 1)
+        B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, kern, wide));
+    auto clusters = [&](b2w4_smem_optin& cache, size_t bytes) {
+        size_t& n = cache.bytes[ctx->device];
+        if (!n)
+            n = 1 + clusters_held(kern, CTAS, bytes);
+        return (long)n - 1;
+    };
+    // A ring's blocks go to a multiprocessor each where all their clusters fit that way (sixteen
+    // blocks of eight clusters do not: two waves, 33 us instead of 22).  A step of eight layers
+    // behind 300 keys 317 -> 310 us.
+    if (RING && (CTAS == 1 || clusters(held_alone, kHalfSmem + 1) >= (long)grid.y * grid.z))
+        smem = kHalfSmem + 1;
     if constexpr (CTAS == 1) {
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), smem,
                                            ctx->stream, a.q, a.k_cache, a.v_cache, a.out,
                                            a.tokens, a.heads, a.kv_heads, a.past, a.past_dev,
                                            a.capacity, a.scale, plan.one_range, prep));
     } else {
-        B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, kern, wide));
-        size_t& fit = fits.bytes[ctx->device];
-        if (!fit)
-            fit = cluster_fits(kern, CTAS) ? 1 : 2;
-        if (fit == 2)
+        if (!clusters(held, 32 * 1024))
             return B2W4_OK;
         B2W4_CUDA(ctx, b2w4_launch_chained_cluster(
                            ctx->pdl, kern, grid, dim3(kAttnThreads), CTAS, smem, ctx->stream,
@@ -1138,8 +1226,19 @@ int launch_split_as(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& 
 template <int DIM, int HR, int CTAS>
 int launch_split_ctas(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
                       bool* placed) {
-    return a.prep ? launch_split_as<DIM, HR, CTAS, true>(ctx, a, keys, plan, placed)
-                  : launch_split_as<DIM, HR, CTAS, false>(ctx, a, keys, plan, placed);
+    if (!a.prep)
+        return launch_split_as<DIM, HR, CTAS, false, false>(ctx, a, keys, plan, placed);
+    // a decode step's blocks that have a multiprocessor each; scores that leave no room for the
+    // ring take the launch without it
+    if constexpr (DIM <= 128) {
+        const int sets = (a.heads / a.kv_heads + HR - 1) / HR;
+        if ((long)CTAS * a.kv_heads * sets <= ctx->sm_count) {
+            const int rc = launch_split_as<DIM, HR, CTAS, true, true>(ctx, a, keys, plan, placed);
+            if (rc != B2W4_OK || *placed)
+                return rc;
+        }
+    }
+    return launch_split_as<DIM, HR, CTAS, true, false>(ctx, a, keys, plan, placed);
 }
 // The planned cluster, or the next smaller one that the device can place.
 template <int DIM, int HR>
@@ -1172,8 +1271,6 @@ int launch_split(b2w4_ctx* ctx, const AttnArgs& a, int dim, int keys, const Attn
     }
 }
 
-// more dynamic shared memory than this, and a multiprocessor holds one block
-constexpr size_t kHalfSmem = 114 * 1024;
 template <int DIM, int ROWS, bool ALIGNED>
 int launch_tile_as(b2w4_ctx* ctx, const AttnArgs& a, bool alone) {
     static b2w4_smem_optin cfg;

@@ -956,3 +956,41 @@ def test_long_runs_with_extreme_values(ctx, tokens, heads, kv_heads, dim):
     vc[:, 300 + tokens // 2] = float("nan")  # seen by the second half
     got = run()
     assert torch.isnan(got[tokens // 2:]).all() and torch.isfinite(got[:tokens // 2]).all()
+
+
+@pytest.mark.parametrize("past,heads,kv_heads,dim,cap", [
+    (0, 8, 2, 128, 96), (3, 8, 2, 128, 96), (94, 4, 1, 64, 96),      # one block per kv head
+    (127, 32, 8, 128, 800), (159, 32, 8, 128, 800), (703, 6, 6, 128, 800),
+    (6015, 32, 8, 128, 6100), (5500, 16, 8, 64, 6100),               # the ring turns over
+    (4095, 4, 1, 128, 4096), (2999, 2, 2, 64, 3001)])
+def test_attention_step_through_the_ring(ctx, past, heads, kv_heads, dim, cap):
+    """A decode step whose blocks have a multiprocessor each brings the cache in through a ring:
+    the bits of the separate operators at the edges of a slot's keys, with fewer keys than warps,
+    with more slots than the ring has, and with the new key in the first and in the last slot.
+    Rows past the position are NaN, and so is a key of probability zero's value row."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(past + dim)
+    qkv = torch.randn((1, (heads + 2 * kv_heads) * dim), device="cuda", generator=g)
+    qw, kw = (torch.rand(dim, device="cuda", generator=g) + 0.5 for _ in range(2))
+    cos, sin = (_dev(t) for t in pkg.decoder.rope_tables(range(cap), dim, 1e6))
+    cache = [torch.randn((kv_heads, cap, dim), device="cuda", generator=g) for _ in range(2)]
+    if past > 9:  # a score of -inf: the key never counts, nor does its value row
+        cache[0][:, 5] = float("-inf") * torch.sign(qkv[0, :1]).abs()
+        cache[0][:, 5, 1:] = 0.0
+        cache[1][:, 5] = 0.0
+    for c in cache:
+        c[:, past + 1:] = float("nan")
+    pos = torch.tensor([past], dtype=torch.int32, device="cuda")
+    for position, host in ((None, past), (pos, 0)):
+        want_kv, got_kv = ([c.clone() for c in cache] for _ in range(2))
+        q, want, got = (torch.zeros((1, heads * dim), device="cuda") for _ in range(3))
+        ctx.qkv_prepare(qkv, 1, heads, kv_heads, dim, qw, kw, 1e-6, cos, sin, host, q, *want_kv,
+                        cap, position)
+        ctx.attention(q, None, None, *want_kv, want, 1, heads, kv_heads, dim, host, cap,
+                      dim ** -0.5, position)
+        ctx.attention_step(qkv, heads, kv_heads, dim, qw, kw, 1e-6, cos, sin, host,
+                           torch.zeros_like(q), *got_kv, got, cap, dim ** -0.5, position)
+        ctx.sync()
+        for a, b in zip(got_kv, want_kv):
+            assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
