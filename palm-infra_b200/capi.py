@@ -150,8 +150,9 @@ def lib():
 
 
 def _dptr(t):
-    """Device pointer of a torch CUDA tensor (or None)."""
-    return None if t is None else C.c_void_p(t.data_ptr())
+    """Device pointer of a torch CUDA tensor (or None), as a number: every argument and field that
+    takes one is declared a pointer."""
+    return None if t is None else t.data_ptr()
 
 
 def rope_tables(positions, first_position, rope_dim, theta):
@@ -340,8 +341,10 @@ class Context:
         m = x.shape[0] if m is None else m
         lda = x.stride(0) if lda is None else lda
         ldc = y.stride(0) if ldc is None else ldc
-        self._check(lib().b2w4_matmul(self.handle, w.handle, _dptr(x), lda, _dptr(y), ldc,
-                                      m, rule, act, act_begin, act_len))
+        rc = lib().b2w4_matmul(self.handle, w.handle, _dptr(x), lda, _dptr(y), ldc, m, rule, act,
+                               act_begin, act_len)
+        if rc != 0:
+            self._check(rc)
 
     def matmul_static_scratch(self, w, x, y, m=None, act=NONE, act_begin=0, act_len=-1):
         """The tensor-core matmul with its scratch in the library's fixed device array
