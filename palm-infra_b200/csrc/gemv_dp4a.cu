@@ -117,13 +117,13 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 __device__ __forceinline__ unsigned long long wait_clock() {
     return (unsigned long long)clock64();
 }
-// Waits for phase 0 of an mbarrier; false when the iteration or the time limit runs out.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar) {
-    if (mbar_try_wait(bar, 0))
+// Waits for a phase of an mbarrier; false when the iteration or the time limit runs out.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity = 0) {
+    if (mbar_try_wait(bar, parity))
         return true;
     const unsigned long long t0 = wait_clock();
     for (unsigned spins = 0; spins < kSpinLimit; ++spins) {
-        if (mbar_try_wait(bar, 0))
+        if (mbar_try_wait(bar, parity))
             return true;
         if ((spins & 63) == 63 && wait_clock() - t0 > kWaitLimitCycles)
             return false;
@@ -508,6 +508,63 @@ gemv_w4a8_kernel(const GemvArgs a) {
     }
 }
 
+// The quantiser of gemv_w4a8_kernel for groups [0, n_g) of a row, per 128 values: a half-warp per
+// group, by a CTA of sixteen warps.
+__device__ __forceinline__ void quantize_groups(const float* x, int n_g, uint4* s_qa, float* s_as,
+                                                int* s_es) {
+    constexpr int kWarps = 16;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int half = lane >> 4, h = lane & 15;
+    const bool vec_x = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+#pragma unroll 1
+    for (int base = warp * 2; base < n_g; base += kWarps * 2) {
+        const int g = base + half;
+        const bool live = g < n_g;
+        const float* src = x + (size_t)(live ? g : 0) * 128 + h * 8;
+        float v[8];
+        if (live && vec_x) {
+            const float4 lo = *reinterpret_cast<const float4*>(src);
+            const float4 hi = *reinterpret_cast<const float4*>(src + 4);
+            v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+            v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = live ? src[i] : 0.f;
+        }
+        float amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1)
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+        float scale, inv;
+        b2w4_quant_params(amax, scale, inv);
+        int c[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            c[i] = b2w4_quant_code(v[i], inv);
+        int esum = c[0] + c[2] + c[4] + c[6];
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1)
+            esum += __shfl_xor_sync(0xffffffffu, esum, off);
+        if (!live)
+            continue;
+        if (h == 0) {
+            s_as[g] = scale;
+            s_es[g] = -8 * esum;
+        }
+        uint8_t* blk =
+            reinterpret_cast<uint8_t*>(s_qa) + (size_t)g * 128 + code_place(h >> 2, g) * 32;
+        const int j = (h & 3) * 4;
+        *reinterpret_cast<char4*>(blk + j) = make_char4(
+            (signed char)c[0], (signed char)c[2], (signed char)c[4], (signed char)c[6]);
+        *reinterpret_cast<char4*>(blk + 16 + j) = make_char4(
+            (signed char)c[1], (signed char)c[3], (signed char)c[5], (signed char)c[7]);
+    }
+}
+
 // ---- long rows: the groups split over a cluster ----------------------------------------------
 // A cluster of kSplit CTAs takes `tpc` tiles; CTA r quantises and multiplies groups [r * per,
 // (r + 1) * per) of all of them and stores each (integer sum, scale product) into the shared
@@ -558,58 +615,7 @@ gemv_w4a8_split_kernel(const GemvArgs a) {
         }
     }
     b2w4_pdl_wait();  // activations come from the previous kernel
-    // quantiser, as above: a half-warp per group
-    {
-        const int half = lane >> 4, h = lane & 15;
-        const bool vec_x = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0;
-#pragma unroll 1
-        for (int base = warp * 2; base < n_g; base += kWarps * 2) {
-            const int g = base + half;
-            const bool live = g < n_g;
-            const float* src = a.x + (size_t)(g0 + (live ? g : 0)) * 128 + h * 8;
-            float v[8];
-            if (live && vec_x) {
-                const float4 lo = *reinterpret_cast<const float4*>(src);
-                const float4 hi = *reinterpret_cast<const float4*>(src + 4);
-                v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
-                v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    v[i] = live ? src[i] : 0.f;
-            }
-            float amax = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                amax = fmaxf(amax, fabsf(v[i]));
-#pragma unroll
-            for (int off = 8; off > 0; off >>= 1)
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-            float scale, inv;
-            b2w4_quant_params(amax, scale, inv);
-            int c[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                c[i] = b2w4_quant_code(v[i], inv);
-            int esum = c[0] + c[2] + c[4] + c[6];
-#pragma unroll
-            for (int off = 8; off > 0; off >>= 1)
-                esum += __shfl_xor_sync(0xffffffffu, esum, off);
-            if (!live)
-                continue;
-            if (h == 0) {
-                s_as[g] = scale;
-                s_es[g] = -8 * esum;
-            }
-            uint8_t* blk =
-                reinterpret_cast<uint8_t*>(s_qa) + (size_t)g * 128 + code_place(h >> 2, g) * 32;
-            const int j = (h & 3) * 4;
-            *reinterpret_cast<char4*>(blk + j) = make_char4(
-                (signed char)c[0], (signed char)c[2], (signed char)c[4], (signed char)c[6]);
-            *reinterpret_cast<char4*>(blk + 16 + j) = make_char4(
-                (signed char)c[1], (signed char)c[3], (signed char)c[5], (signed char)c[7]);
-        }
-    }
+    quantize_groups(a.x + (size_t)g0 * 128, n_g, s_qa, s_as, s_es);
     // every CTA of the cluster runs before its shared memory is written from another one
     cluster.sync();
 
@@ -654,6 +660,114 @@ gemv_w4a8_split_kernel(const GemvArgs a) {
             acc = gemv_activation(acc, a.activation);
         a.y[n] = acc;
     }
+}
+
+// ---- weights of many rows (an lm_head): persistent CTAs ---------------------------------------
+// Two CTAs per SM take an equal run of tiles each, in chunks of `tpc` tiles through a ring of
+// kStreamBufs buffers: the weights of the next chunks are on their way while one is computed, and
+// the row is quantised once per CTA, where CTAs of gemv_w4a8_kernel that follow one another on an SM
+// each quantise it and wait for their first weights.  Sums and chains as there: its bits.  A chunk's
+// chains are a warp's per four tiles (others every time) under the next chunk's integer sums.
+constexpr int kStreamBufs = 3, kStreamMaxTpc = 16;
+template <bool SCL16, bool TOP1>
+__global__ void __launch_bounds__(512, 2) gemv_w4a8_stream_kernel(const GemvArgs a) {
+    constexpr int kWarps = 16, kScl = SCL16 ? 16 : 32;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int G = a.groups, tile_bytes = G * 512, scl_bytes = G * kScl;
+    uint8_t* s_w = smem;                                                          // [bufs][tpc][G][512]
+    uint8_t* s_scl = s_w + (size_t)kStreamBufs * a.tpc * tile_bytes;              // [bufs][tpc][G][8]
+    uint4* s_qa = reinterpret_cast<uint4*>(s_scl + (size_t)kStreamBufs * a.tpc * scl_bytes);
+    float* s_as = reinterpret_cast<float*>(s_qa + G * 8);                         // [G]
+    int* s_es = reinterpret_cast<int*>(s_as + G);                                 // [G]
+    float* s_d = reinterpret_cast<float*>(s_es + G);                              // [2][tpc][d_stride]
+    float* s_sc = s_d + 2 * a.tpc * a.d_stride;                                   // the same
+    __shared__ uint64_t s_bar[kStreamBufs];
+    __shared__ unsigned long long s_top1[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gl = lane >> 3, row = lane & 7;
+    const int begin = (int)((long long)a.tiles * blockIdx.x / gridDim.x);
+    const int end = (int)((long long)a.tiles * (blockIdx.x + 1) / gridDim.x);
+    const int chunks = (end - begin + a.tpc - 1) / a.tpc;
+    auto issue = [&](int c) {  // one thread
+        const int tile = begin + c * a.tpc, n = min(a.tpc, end - tile), b = c % kStreamBufs;
+        mbar_expect_tx(&s_bar[b], (uint32_t)(n * (tile_bytes + scl_bytes)));
+        bulk_g2s(s_w + (size_t)b * a.tpc * tile_bytes,
+                 reinterpret_cast<const uint8_t*>(a.nib) + (size_t)tile * tile_bytes,
+                 (uint32_t)(n * tile_bytes), &s_bar[b]);
+        bulk_g2s(s_scl + (size_t)b * a.tpc * scl_bytes,
+                 reinterpret_cast<const uint8_t*>(a.scl) + (size_t)tile * scl_bytes,
+                 (uint32_t)(n * scl_bytes), &s_bar[b]);
+    };
+
+    b2w4_pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < kStreamBufs; ++b)
+            mbar_init(&s_bar[b], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int c = 0; c < min(kStreamBufs, chunks); ++c)
+            issue(c);
+    }
+    if (TOP1 && threadIdx.x < 8)
+        s_top1[threadIdx.x] = 0ull;
+    b2w4_pdl_wait();  // activations come from the previous kernel
+    quantize_groups(a.x, G, s_qa, s_as, s_es);
+    __syncthreads();
+
+    const int ipt = (G + 3) >> 2;
+    unsigned long long best = 0ull;
+    bool timed_out = false;
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+        const int tile0 = begin + c * a.tpc, ntile = min(a.tpc, end - tile0), b = c % kStreamBufs;
+        const uint8_t* w = s_w + (size_t)b * a.tpc * tile_bytes;
+        const uint8_t* scl = s_scl + (size_t)b * a.tpc * scl_bytes;
+        float* d_out = s_d + (c & 1) * a.tpc * a.d_stride;
+        float* sc_out = s_sc + (c & 1) * a.tpc * a.d_stride;
+        if (!timed_out && !mbar_wait_bounded(&s_bar[b], c / kStreamBufs & 1)) {
+            timed_out = true;
+            b2w4_report_timeout(a.status);
+        }
+#pragma unroll 1
+        for (int it = warp; it < ntile * ipt; it += kWarps) {
+            const int tl = a.ipt_magic ? (it * a.ipt_magic) >> 16 : it / ipt;
+            const int g = (it - tl * ipt) * 4 + gl;
+            if (g < G) {
+                const int at = tl * G + g;
+                const int d = group_sum(reinterpret_cast<const uint4*>(w) + at * 32 + row,
+                                        s_qa + g * 8, s_es[g], gl);
+                const float ws = SCL16 ? __half2float(reinterpret_cast<const __half*>(scl)[at * 8 + row])
+                                       : reinterpret_cast<const float*>(scl)[at * 8 + row];
+                const int slot = tl * a.d_stride + g * 8 + row;
+                d_out[slot] = (float)d;
+                sc_out[slot] = __fmul_rn(ws, s_as[g]);
+            }
+        }
+        __syncthreads();  // sums in place, the buffer is free, and so are the sums of chunk c - 1
+        if (threadIdx.x == 0 && c + kStreamBufs < chunks && !timed_out)
+            issue(c + kStreamBufs);
+        const int mine = ((warp - c) & (kWarps - 1)) * 4 + gl;  // the lane's tile
+        if (mine < ntile) {
+            const float* dsrc = d_out + mine * a.d_stride + row;
+            const float* csrc = sc_out + mine * a.d_stride + row;
+            const int n = (tile0 + mine) * 8 + row;
+            float acc = 0.f;
+#pragma unroll 10
+            for (int j = 0; j < G; ++j)
+                acc = __fmaf_rn(dsrc[j * 8], csrc[j * 8], acc);
+            if (n < a.n) {
+                if (b2w4_act_applies(n, a.activation, a.act_n_begin, a.act_n_len, a.n))
+                    acc = gemv_activation(acc, a.activation);
+                if (TOP1) {
+                    const unsigned long long word = b2w4_top1_word(acc, n);
+                    best = word > best ? word : best;
+                }
+                if (!TOP1 || a.y)
+                    a.y[n] = acc;
+            }
+        }
+    }
+    if (TOP1)
+        b2w4_top1_finish(a.top1, best, 0, 1, s_top1);
 }
 
 // Second half of the tensor-parallel exchange: waits (bounded) until every entry of the
@@ -822,6 +936,39 @@ int launch_split(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, size_t smem) {
     return B2W4_OK;
 }
 
+size_t gemv_stream_bytes(int groups, int tpc, int d_stride, bool scl16) {
+    return (size_t)kStreamBufs * tpc * groups * (512 + (scl16 ? 16 : 32)) +
+           (size_t)groups * (128 + 8) + 4 * sizeof(float) * (size_t)tpc * d_stride;
+}
+// Tiles of a chunk: as many as fit half an SM, the count whose items fill the sixteen warps' rounds
+// best; 0: none fits.
+int gemv_stream_tpc(const b2w4_weight* w, int d_stride) {
+    const int ipt = (w->groups + 3) / 4;
+    int best = 0;
+    double best_fill = 0.;
+    for (int t = 1; t <= kStreamMaxTpc; ++t) {
+        const int items = t * ipt;
+        const double fill = (double)items / ((items + 15) / 16 * 16);
+        if (gemv_stream_bytes(w->groups, t, d_stride, w->scales_fp16 != 0) <= 112 * 1024 &&
+            fill >= best_fill) {
+            best = t;
+            best_fill = fill;
+        }
+    }
+    return best;
+}
+template <bool SCL16, bool TOP1>
+int launch_stream(b2w4_ctx* ctx, const GemvArgs& a) {
+    auto kern = gemv_w4a8_stream_kernel<SCL16, TOP1>;
+    static b2w4_smem_optin configured;  // per instantiation and device
+    const size_t smem = gemv_stream_bytes(a.groups, a.tpc, a.d_stride, SCL16);
+    B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured));
+    B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, dim3(2 * ctx->sm_count), dim3(512), smem,
+                                       ctx->stream, a));
+    ctx->launches++;
+    return B2W4_OK;
+}
+
 template <int MT>
 int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, size_t smem) {
     const int mode = a.sums ? kModeSums : (a.top1.cells ? kModeTop1 : kModePlain);
@@ -922,14 +1069,15 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
             const int pairs = w->tiles / 2, ctas = (w->tiles + tpc - 1) / tpc;
             tpc = min(max(2, budget / per_tile / 2 * 2), 2 * ((pairs + ctas - 1) / ctas));
         }
-        a.tpc = tpc;
-        {
+        auto take = [&](int tiles) {
+            a.tpc = tiles;
             const int ipt = (w->groups + 3) / 4;
             a.ipt_magic = 65536 / ipt + 1;
-            for (int it = 0; it < tpc * ipt; ++it)  // exact for every item of a CTA?
+            for (int it = 0; it < tiles * ipt; ++it)  // exact for every item of a CTA?
                 if (((it * a.ipt_magic) >> 16) != it / ipt)
                     a.ipt_magic = 0;
-        }
+        };
+        take(tpc);
         a.d_stride = gemv_d_stride(mt, w->groups, a32);
         // Long rows, split over clusters, from 48 groups on and where the kernel above has at most
         // four tiles per CTA.  us in a graph, that kernel / split, by weight rows: K = 9728 1000
@@ -948,6 +1096,21 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
             if (bytes <= 113 * 1024)
                 return launch_split(ctx, a, scl16, bytes);
             a.tpc = tpc;
+        }
+        // Many rows: persistent CTAs from three and a half CTAs of the kernel above per SM on.  us in
+        // a graph, that kernel / persistent, plain and with the greedy token: K = 2560 25000 rows
+        // (2.4 per SM, not taken) 9.3 / 9.7, 40000 (3.8) 13.1 / 12.3 and 14.6 / 13.8, 100000 27.2 /
+        // 23.8 and 30.6 / 26.2, 151936 39.5 / 35.8 and 42.8 / 38.5; K = 4096 19456 rows (3.3, not
+        // taken) 11.3 / 11.8, 40000 20.2 / 18.1; K = 512 60000 rows (3.2, not taken) 6.5 / 7.7,
+        // 151936 14.3 / 10.7; K = 1024 151936 rows 20.0 / 16.1.
+        if (!a32 && !sums && !tp && !norm && !swiglu && ctx->gemv_tpc_override == 0 &&
+            2 * ((w->tiles + tpc - 1) / tpc) >= 7 * ctx->sm_count &&
+            gemv_stream_tpc(w, a.d_stride) > 0) {
+            take(gemv_stream_tpc(w, a.d_stride));
+            return top1 ? (scl16 ? launch_stream<true, true>(ctx, a)
+                                 : launch_stream<false, true>(ctx, a))
+                        : (scl16 ? launch_stream<true, false>(ctx, a)
+                                 : launch_stream<false, false>(ctx, a));
         }
         size_t smem = gemv_smem_bytes(mt, w->k, w->groups, tpc, scl16, a32);
         if (norm)  // the row's copy, 16-byte aligned behind the barriers

@@ -663,3 +663,41 @@ def test_longest_rows(ctx, m, rule, longest):
                         call()
                 assert bool((y == -1).all()) and bool((res == 1).all())
             w.free()
+
+
+@pytest.mark.parametrize("n,k,f32", [(70001, 128, False), (99993, 384, True), (66305, 1152, False),
+                                     (40961, 2560, False), (30011, 4224, True)])
+def test_many_rows_on_persistent_blocks(ctx, n, k, f32):
+    """One row against weights of many rows, whose blocks take chunks of tiles through a ring: one
+    group and counts that four does not divide, chunks of 3 to 16 tiles, ragged last chunks and
+    tiles, fp32 scales, a row that is not 16-byte aligned, a fused activation, the greedy token with
+    and without the logits; the oracle's bits."""
+    import torch
+    blocks = pkg.synth.bg128_weight(20261125, n + k, n, k)
+    if f32:  # scales that fp16 cannot hold
+        blocks = np.array(blocks, copy=True)
+        s = blocks.reshape(-1, 544)[:, :32].copy().view(np.float32)
+        blocks.reshape(-1, 544)[:, :32] = (s * np.float32(1.0000001) + np.float32(1e-9) *
+                                           (s != 0)).astype(np.float32).view(np.uint8)
+    x = pkg.synth.activations(91, n, 1, k)
+    ref = ol.matmul_w4(blocks, n, k, x)
+    w = ctx.upload_weight(blocks, n, k)
+    at = torch.zeros(k + 4, device="cuda")
+    for off in (0, 1):
+        xd = at[off:off + k].view(1, k)
+        xd.copy_(torch.from_numpy(x))
+        y, logits = (torch.zeros((1, n), device="cuda") for _ in range(2))
+        tok = torch.full((2,), -1, dtype=torch.int32, device="cuda")
+        ctx.matmul(w, xd, y)
+        ctx.matmul_argmax(w, xd, tok[:1], logits)
+        ctx.matmul_argmax(w, xd, tok[1:])
+        ctx.sync()
+        assert y.cpu().numpy().tobytes() == ref.tobytes()
+        assert logits.cpu().numpy().tobytes() == ref.tobytes()
+        assert tok.tolist() == [ol.argmax_token(ref[0])] * 2
+    act, begin, length = 3, n // 2, 1000
+    ctx.matmul(w, torch.from_numpy(x).cuda(), y, act=act, act_begin=begin, act_len=length)
+    ctx.sync()
+    want = ol.apply_activation(ref.copy(), act, begin, length)
+    assert y.cpu().numpy().tobytes() == want.tobytes()
+    w.free()
