@@ -54,7 +54,7 @@ namespace {
 // one activation row: 16 warps of <= 64 registers; more rows keep more integer sums in
 // registers: 8 warps of <= 128 registers.  Either way two CTAs share an SM.
 __host__ __device__ constexpr int gemv_warps(int mt) { return mt == 1 ? 16 : 8; }
-constexpr int kMaxTpc = 16;
+constexpr int kMaxTpc = 16, kWideTpc = 24;  // tiles per CTA; of thirty-two warps
 constexpr unsigned kSpinLimit = 1u << 22;  // bounded waits: give up, flag, return
 constexpr unsigned long long kWaitLimitCycles = 4000000000ull;  // SM cycles: about 2 s
 constexpr int kTpGatherThreads = 256;
@@ -173,10 +173,11 @@ __device__ __noinline__ float gemv_activation(float v, int act) {
     return b2w4_activation(v, act);
 }
 
-template <int MT, bool SCL16, bool A32, int MODE, bool NORM = false>
-__global__ void __launch_bounds__(gemv_warps(MT) * 32, 2)
+// WARPS: of a CTA; sixteen, two CTAs per SM, or the double and one.
+template <int MT, bool SCL16, bool A32, int MODE, bool NORM = false, int WARPS = gemv_warps(MT)>
+__global__ void __launch_bounds__(WARPS * 32, WARPS > 16 ? 1 : 2)
 gemv_w4a8_kernel(const GemvArgs a) {
-    constexpr int kWarps = gemv_warps(MT);
+    constexpr int kWarps = WARPS;
     constexpr int kThreads = kWarps * 32;
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int SPG = A32 ? 4 : 1;  // integer sums per group
@@ -193,8 +194,12 @@ gemv_w4a8_kernel(const GemvArgs a) {
     int* s_es = reinterpret_cast<int*>(s_as + MT * G * SPG);  // -8 * sum of the even-k codes
     float* s_d = reinterpret_cast<float*>(s_es + MT * G * SPG);  // [tpc][G][SPG][MT][8] + pad
     float* s_sc = s_d + (size_t)a.tpc * a.d_stride;        // same shape
+    // NORM: a copy of the row, where the sums come later
+    float* s_row = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_d) + 15) & ~uintptr_t(15));
+    const uintptr_t sums_end = reinterpret_cast<uintptr_t>(s_sc + (size_t)a.tpc * a.d_stride);
+    const uintptr_t row_end = NORM ? reinterpret_cast<uintptr_t>(s_row + K) : 0;
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(
-        (reinterpret_cast<uintptr_t>(s_sc + (size_t)a.tpc * a.d_stride) + 7) & ~uintptr_t(7));
+        ((row_end > sums_end ? row_end : sums_end) + 7) & ~uintptr_t(7));
 
     constexpr bool SUMS = MODE == kModeSums;
     __shared__ unsigned long long s_top1[8];
@@ -271,8 +276,6 @@ gemv_w4a8_kernel(const GemvArgs a) {
         float kept[8], kept_w[8], rms = 0.f;
         if (NORM) {
             __shared__ float s_ss[8];
-            float* s_row = reinterpret_cast<float*>(
-                (reinterpret_cast<uintptr_t>(s_bar + a.tpc + 1) + 15) & ~uintptr_t(15));
             const int g = warp * 2 + half, at = g * 128 + h * 8;
             if (g < G) {
                 load8(a.norm.residual + at, kept);
@@ -450,7 +453,7 @@ gemv_w4a8_kernel(const GemvArgs a) {
         b2w4_report_timeout(a.status);
     __syncthreads();
 
-    __shared__ float s_gu[SWIGLU ? kMaxTpc * 8 : 1];  // gate rows, then up rows
+    __shared__ float s_gu[SWIGLU ? kWideTpc * 8 : 1];  // gate rows, then up rows
     // ---- phase 2: fp32 chain, one thread per (tile, activation row, weight row) ---------
 #pragma unroll 1
     for (int t = threadIdx.x; t < ntile * MT * 8; t += kThreads) {
@@ -891,24 +894,26 @@ int gemv_d_stride(int mt, int groups, bool a32) {
     return groups * (a32 ? 4 : 1) * mt * 8 + 8;
 }
 
-size_t gemv_smem_bytes(int mt, int k, int groups, int tpc, bool scl16, bool a32) {
+size_t gemv_smem_bytes(int mt, int k, int groups, int tpc, bool scl16, bool a32,
+                       bool norm = false) {
     const int spg = a32 ? 4 : 1;
+    const size_t sums = 2 * sizeof(float) * (size_t)tpc * gemv_d_stride(mt, groups, a32);
+    const size_t row = norm ? sizeof(float) * k + 16 : 0;  // its place is the sums'
     return (size_t)tpc * groups * 512 + (size_t)tpc * groups * 8 * (scl16 ? 2 : 4) +
-           (size_t)mt * k + 2 * sizeof(float) * mt * groups * spg +
-           2 * sizeof(float) * (size_t)tpc * gemv_d_stride(mt, groups, a32) + 8 +
+           (size_t)mt * k + 2 * sizeof(float) * mt * groups * spg + (row > sums ? row : sums) + 8 +
            sizeof(uint64_t) * (tpc + 1);
 }
 
-template <int MT, bool SCL16, bool A32, int MODE, bool NORM = false>
+template <int MT, bool SCL16, bool A32, int MODE, bool NORM = false, int WARPS = gemv_warps(MT)>
 int launch_one(b2w4_ctx* ctx, const GemvArgs& a, size_t smem) {
-    auto kern = gemv_w4a8_kernel<MT, SCL16, A32, MODE, NORM>;
+    auto kern = gemv_w4a8_kernel<MT, SCL16, A32, MODE, NORM, WARPS>;
     static b2w4_smem_optin configured;  // per instantiation and device
     B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, smem, configured));
     cudaLaunchConfig_t cfg = {};
     const int per_cta = MODE == kModeSwiglu ? a.tpc / 2 : a.tpc;
     const int tiles = MODE == kModeSwiglu ? a.tiles / 2 : a.tiles;
     cfg.gridDim = dim3((tiles + per_cta - 1) / per_cta);
-    cfg.blockDim = dim3(gemv_warps(MT) * 32);
+    cfg.blockDim = dim3(WARPS * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
@@ -970,9 +975,15 @@ int launch_stream(b2w4_ctx* ctx, const GemvArgs& a) {
 }
 
 template <int MT>
-int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, size_t smem) {
+int launch_mt(b2w4_ctx* ctx, const GemvArgs& a, bool scl16, bool a32, bool wide, size_t smem) {
     const int mode = a.sums ? kModeSums : (a.top1.cells ? kModeTop1 : kModePlain);
     if (a.swiglu || a.norm.weight) {  // a decode step: one row, per-128 rule
+        if (wide && a.norm.weight)
+            return scl16 ? launch_one<MT, true, false, kModeSwiglu, true, 32>(ctx, a, smem)
+                         : launch_one<MT, false, false, kModeSwiglu, true, 32>(ctx, a, smem);
+        if (wide)
+            return scl16 ? launch_one<MT, true, false, kModeSwiglu, false, 32>(ctx, a, smem)
+                         : launch_one<MT, false, false, kModeSwiglu, false, 32>(ctx, a, smem);
         if (a.swiglu && a.norm.weight)
             return scl16 ? launch_one<MT, true, false, kModeSwiglu, true>(ctx, a, smem)
                          : launch_one<MT, false, false, kModeSwiglu, true>(ctx, a, smem);
@@ -1049,6 +1060,7 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
         if (norm)
             a.norm = *norm;
         a.swiglu = swiglu;
+        bool wide = false;
         // Tiles per CTA: a CTA's shared memory stays under half an SM's so that two CTAs share
         // an SM, and the launch is one wave of at most 1.75 CTAs per SM.  Measured on the
         // decode shapes of a 4B dense model (148 SMs): N=9728 K=2560 (1216 tiles) 244 CTAs
@@ -1057,9 +1069,12 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
         // CTAs 8.65.
         const int per_tile = w->groups * (512 + (scl16 ? 16 : 32)) +
                              8 * gemv_d_stride(mt, w->groups, a32);
-        const int budget = 113 * 1024 - mt * w->k - 8 * mt * w->groups * spg - 1024 -
-                           (norm ? 4 * w->k + 16 : 0);
-        int tpc = max(1, min(budget / per_tile, kMaxTpc));
+        const int budget = 113 * 1024 - mt * w->k - 8 * mt * w->groups * spg - 1024;
+        int most = max(1, min(budget / per_tile, kMaxTpc));
+        while (norm && most > 1 &&
+               gemv_smem_bytes(mt, w->k, w->groups, most, scl16, a32, true) > 112 * 1024)
+            --most;  // few tiles: the row needs more room than their sums
+        int tpc = most;
         const int wave_ctas = ctx->sm_count * 7 / 4;
         const int one_wave = (w->tiles + wave_ctas - 1) / wave_ctas;
         tpc = min(tpc, max(1, one_wave));
@@ -1067,7 +1082,16 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
             tpc = min(tpc, ctx->gemv_tpc_override);
         if (swiglu) {  // gate and up tiles in pairs
             const int pairs = w->tiles / 2, ctas = (w->tiles + tpc - 1) / tpc;
-            tpc = min(max(2, budget / per_tile / 2 * 2), 2 * ((pairs + ctas - 1) / ctas));
+            tpc = min(max(2, most / 2 * 2), 2 * ((pairs + ctas - 1) / ctas));
+            // Pairs that two CTAs per SM leave to a second wave: one CTA of twice the warps per SM
+            // ([19456, 2560] with the norm 10.2 -> 8.9 us; 18944 rows, the last of one wave, 8.6).
+            const int all = 2 * ((pairs + ctx->sm_count - 1) / ctx->sm_count);
+            wide = a.top1.cells == nullptr && !a32 &&
+                   (pairs + tpc / 2 - 1) / (tpc / 2) > 2 * ctx->sm_count && all <= kWideTpc &&
+                   gemv_smem_bytes(mt, w->k, w->groups, all, scl16, a32, norm != nullptr) <=
+                       220 * 1024;
+            if (wide)
+                tpc = all;
         }
         auto take = [&](int tiles) {
             a.tpc = tiles;
@@ -1112,13 +1136,12 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
                         : (scl16 ? launch_stream<true, false>(ctx, a)
                                  : launch_stream<false, false>(ctx, a));
         }
-        size_t smem = gemv_smem_bytes(mt, w->k, w->groups, tpc, scl16, a32);
-        if (norm)  // the row's copy, 16-byte aligned behind the barriers
-            smem += sizeof(float) * w->k + 16;
+        const size_t smem =
+            gemv_smem_bytes(mt, w->k, w->groups, tpc, scl16, a32, norm != nullptr);
         if (smem > 220 * 1024)
             return b2w4_fail(ctx, B2W4_E_INVALID, "gemv: K=%d needs %zu B shared memory",
                              w->k, smem);
-        int rc = launch_mt<1>(ctx, a, scl16, a32, smem);  // mt == 1: see the top
+        int rc = launch_mt<1>(ctx, a, scl16, a32, wide, smem);  // mt == 1: see the top
         if (rc != B2W4_OK)
             return rc;
     }

@@ -994,3 +994,32 @@ def test_attention_step_through_the_ring(ctx, past, heads, kv_heads, dim, cap):
         for a, b in zip(got_kv, want_kv):
             assert torch.equal(a.view(torch.int32), b.view(torch.int32))
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("n,k,f32", [(18960, 2560, True), (9600, 4224, False), (37920, 1280, False),
+                                     (19456, 384, False)])
+def test_step_matmul_with_twice_the_warps(ctx, n, k, f32):
+    """SwiGLU over more pairs of tiles than two blocks per multiprocessor hold: one block of twice
+    the warps, with the norm inside and (rows beyond 4096 values) in front, fp32 scales, a last
+    block with fewer pairs; and short rows, whose copy is larger than the sums it lies over."""
+    import torch
+    rng = np.random.default_rng(n + k)
+    blocks = pkg.synth.bg128_weight(3, n + k, n, k)
+    if f32:
+        blocks = np.array(blocks, copy=True)
+        s = blocks.reshape(-1, 544)[:, :32].copy().view(np.float32)
+        blocks.reshape(-1, 544)[:, :32] = (s * np.float32(1.0000001)).view(np.uint8)
+    w = ctx.upload_weight(blocks, n, k)
+    x, u, g = (_dev(rng.normal(m, s, (1, k)).astype(np.float32))
+               for m, s in ((0, 2), (0, 1), (1, 0.2)))
+    res, hid = (torch.zeros((1, k), device="cuda") for _ in range(2))
+    want = torch.zeros((1, n), device="cuda")
+    act, want_act = (torch.zeros((1, n // 2), device="cuda") for _ in range(2))
+    ctx.step_matmul(w, x, u, g, 1e-6, res, y=act, swiglu=True)
+    want_res = x.clone()
+    ctx.add_rms_norm(want_res, u, g, 1e-6, hid)
+    ctx.matmul(w, hid, want, rule=ol.ACT_G128)
+    ctx.swiglu(want, want_act)
+    ctx.sync()
+    assert torch.equal(res, want_res) and torch.equal(act, want_act)
+    w.free()
