@@ -105,7 +105,8 @@ template <typename Kernel>
 inline cudaError_t b2w4_opt_in_smem(b2w4_ctx* ctx, Kernel kern, size_t smem,
                                     b2w4_smem_optin& cache) {
     size_t& have = cache.bytes[ctx->device];
-    if (smem <= 48 * 1024 || smem <= have)
+    // 48 KiB need no leave, counted with the kernel's static part: below 8 KiB everywhere
+    if (smem <= 40 * 1024 || smem <= have)
         return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);

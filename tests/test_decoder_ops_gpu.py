@@ -5,6 +5,10 @@ against the CPU oracle, which is pinned bit for bit against the reference's own 
 over a row (norms, attention scores, softmax) use tree reductions where the reference's loops
 are sequential, and are held to the rounding error of a reassociated fp32 sum: 2e-6 relative
 for the norms, 1e-5 relative L2 for attention."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -1023,3 +1027,28 @@ def test_step_matmul_with_twice_the_warps(ctx, n, k, f32):
     ctx.sync()
     assert torch.equal(res, want_res) and torch.equal(act, want_act)
     w.free()
+
+
+def test_shared_memory_just_below_the_default_limit():
+    """A first call whose dynamic part is below 48 KiB and whose whole is not (SwiGLU of two tiles of
+    [4096, 4736]: 49 000 bytes and 768): in a process of its own, where no larger call came before."""
+    code = """
+import sys; sys.path.insert(0, %r)
+import torch
+from __graft_entry__ import load_package
+pkg = load_package()
+ctx = pkg.capi.Context(0)
+n, k = 4096, 4736
+w = ctx.upload_weight(pkg.synth.bg128_weight(3, 1, n, k), n, k)
+x = torch.randn((1, k), device="cuda")
+out = [torch.zeros((1, s), device="cuda") for s in (k, n // 2, k, n, n // 2)]
+one = torch.ones(k, device="cuda")
+ctx.step_matmul(w, x, None, one, 1e-6, out[0], y=out[1], swiglu=True)
+ctx.rms_norm(x, one, 1e-6, out[2])
+ctx.matmul(w, out[2], out[3], rule=128)
+ctx.swiglu(out[3], out[4])
+ctx.sync()
+assert torch.equal(out[1], out[4])
+""" % os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
