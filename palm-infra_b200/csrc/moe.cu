@@ -1176,17 +1176,12 @@ struct PairWords {
 template <bool SCL16>
 constexpr int kPairSlot = 1024 + (SCL16 ? 32 : 64);
 
-// A constant that stays in its register: an instruction of the tensor pipe takes the accumulator's
-// start value in four, and the compiler makes a constant it can see anew for each one (256 tokens of
-// the 128-expert layer, the call: 193.6 -> 192.6 us).  By whole warps.
-__device__ __forceinline__ int held(int v) { return __shfl_sync(0xffffffffu, v, 0); }
-
 // Folds one group of sixteen weight rows into the chain values of `ncb` blocks of eight routes.
 // acc[j][0]: row gid, routes 2*tid and 2*tid+1 of block j; acc[j][1]: row gid+8.
 template <bool A32>
 __device__ __forceinline__ void pair_group(const PairWords& pw, const uint8_t* rows,
                                            int row_bytes, const float* s_as, int g, int ncb,
-                                           int tid, int4 start, uint64_t (&acc)[2][2]) {
+                                           int tid, uint64_t (&acc)[2][2]) {
     uint32_t lo[2][4], hi[2][4];
 #pragma unroll
     for (int t = 0; t < 2; ++t)
@@ -1196,6 +1191,7 @@ __device__ __forceinline__ void pair_group(const PairWords& pw, const uint8_t* r
             hi[t][b] = pw.w[t][b] & 0xF0F0F0F0u;
         }
     const uint64_t magic = b2w4_pack2(786432.f, 786432.f);
+    const int4 start = make_int4(0x49400000, 0x49400000, 0x49400000, 0x49400000);
     const uint64_t w0 = b2w4_pack2(pw.ws[0], pw.ws[0]), w1 = b2w4_pack2(pw.ws[1], pw.ws[1]);
     auto fold = [&](const int (&c)[4], uint64_t as2, uint64_t (&y)[2]) {
         // c = 0x49400000 + 16 D: as a float 786432 + D, exactly
@@ -1311,8 +1307,6 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
     const long long u_end = total * (blockIdx.x + 1) / gridDim.x;
     const size_t tile_bytes = (size_t)G * 512, scl_tile_bytes = (size_t)G * (SCL16 ? 16 : 32);
 
-    // of every accumulator
-    const int4 start = make_int4(held(0x49400000), held(0x49400000), held(0x49400000), held(0x49400000));
     while (u < u_end) {
         const int pass_all = (int)(u / rounds);
         const int round0 = (int)(u - (long long)pass_all * rounds);
@@ -1406,7 +1400,7 @@ moe_grouped_gemv_kernel(const GroupedArgs a) {
                                   : reinterpret_cast<const float*>(src + 1024)[t * 8 + gid];
                     }
                     pair_group<decltype(rule)::value>(now, rows, row_bytes, s_as, g, ncb, tid,
-                                                      start, acc);
+                                                      acc);
                 }
             };
             if (a32)
