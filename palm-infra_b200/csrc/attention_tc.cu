@@ -5,8 +5,8 @@
 // the smallest).  A product takes six of the nine piece products, the small ones first,
 //   l h' + h l' + m m' + m h' + h m' + h h'
 // what is left out is below 2^-24 of |x x'|; sums are fp32 in tensor memory.  Scores,
-// probabilities, maxima and sums stay fp32, and the output's sum over key blocks is kept in
-// registers with one rounding per block.
+// probabilities (exp in 64 bits, rounded once), maxima and sums stay fp32, and the output's sum
+// over key blocks is kept in registers with one rounding per block.
 //
 // A block takes 128 (token, head) rows of one kv head against blocks of 64 keys, and is alone on
 // its multiprocessor: the pieces of two blocks of keys and values fill shared memory.  The MMA's A
@@ -14,20 +14,21 @@
 // which the softmax adds: an MMA of 128 rows takes 47 cycles for 64 columns and 66 for 128
 // (measured), so Q's m meets the keys' h and m side by side, as 128 columns.  Roles:
 //   rows       eight warps, two threads to a row: 32 of the 64 scores each (running maximum, exp in
-//              32 bits, pieces of the probabilities back to tensor memory) and DIM / 2 of the
+//              64 bits, pieces of the probabilities back to tensor memory) and DIM / 2 of the
 //              output's sums, o = o * alpha + P V of the block
 //   MMA        a thread for the scores, a block ahead, and one for P V
 //   split      seven warps for the keys, seven for the values: from global memory to pieces in the
 //              MMA's layout (values transposed)
 // A score's h h' products go to one sum for one half of the features and to the other for the
 // other: a sum in tensor memory truncates, by less the smaller it is.
-// What bounds it: a step of 64 keys takes about 6000 cycles at DIM = 128.  Its MMAs alone take 2050
+// What bounds it: a step of 64 keys takes about 7500 cycles at DIM = 128.  Its MMAs alone take 2050
 // (scores) and 1600 (P V), its softmax and splits about 4000 of each scheduler (conversions and
-// logic at half rate, paired fp32 instructions two to three cycles each); shared memory serves
-// MMAs, splits and loads for about 3000.  Measured against the tile form: attn_tensor
-// (decoder_ops.cu).  Tried, 1500 tokens of 32 / 8 heads of 128 (167 us): all products with m and h
-// of the keys side by side 156 (error 2.3e-7 instead of 1.8e-7), each alone 188; three warps each
-// to split 197, five 170.
+// logic at half rate, paired fp32 instructions two to three cycles each) and its exp about 2000 of
+// the 64-bit and conversion pipes; shared memory serves MMAs, splits and loads for about 3000.
+// Measured against the tile form: attn_tensor (decoder_ops.cu).  Tried with an exp in 32 bits, 1500
+// tokens of 32 / 8 heads of 128 (167 us; 208 with this one): all products with m and h of the keys
+// side by side 156 (error 2.3e-7 instead of 1.8e-7), each alone 188; three warps each to split 197,
+// five 170.
 // A row that comes out not finite, or so small that a piece of a value may have been lost, sends
 // the tile to the fp32 form (attention_tile.cuh), which has the rule for values of probability
 // zero; nothing is written before that is known.
@@ -141,45 +142,27 @@ __device__ __forceinline__ uint32_t take_piece(uint64_t& v) {
     return p;
 }
 
-// exp of two numbers x <= 0 (NaN stays).  After Cody and Waite, Software Manual for the
-// Elementary Functions (1980): x = n ln 2 + r with ln 2 in two parts, |r| <= 0.35, then the
-// Taylor series to r^7 (the rest is below 2^-27) and two exact powers of two, so that only the
-// last product rounds where the result is below the smallest normal number.  NEAR: x >= -86, one
-// power of two is enough.
-template <bool NEAR>
-__device__ __forceinline__ uint64_t exp2x(uint64_t x) {
-    auto both = [](float c) { return b2w4_pack2(c, c); };
-    if constexpr (!NEAR) {
-        float a, b;
-        b2w4_unpack2(x, a, b);
-        a = a < -110.f ? -110.f : a;  // below the half of the smallest number: zero
-        b = b < -110.f ? -110.f : b;
-        x = b2w4_pack2(a, b);
-    }
-    constexpr float kMagic = 12582912.f;  // 1.5 * 2^23: the sum's low bits are the integer
-    const uint64_t t = b2w4_fma2(x, both(1.44269504f), both(kMagic));
-    const uint64_t n = add2(t, both(-kMagic));
-    uint64_t r = b2w4_fma2(n, both(-0.693359375f), x);
-    r = b2w4_fma2(n, both(2.12194440e-4f), r);
-    uint64_t q = b2w4_fma2(r, both(1.f / 5040.f), both(1.f / 720.f));
-    q = b2w4_fma2(q, r, both(1.f / 120.f));
-    q = b2w4_fma2(q, r, both(1.f / 24.f));
-    q = b2w4_fma2(q, r, both(1.f / 6.f));
-    q = b2w4_fma2(q, r, both(0.5f));
-    const uint64_t u = b2w4_fma2(b2w4_mul2(r, r), q, r);
-    uint64_t e = add2(u, both(1.f));
-    float t0, t1;
-    b2w4_unpack2(t, t0, t1);
-    int n0 = __float_as_int(t0) - __float_as_int(kMagic);
-    int n1 = __float_as_int(t1) - __float_as_int(kMagic);
-    auto power = [](int i) { return __int_as_float((int)((uint32_t)i << 23) + 0x3f800000); };
-    if constexpr (!NEAR) {
-        const int c0 = max(n0, -100), c1 = max(n1, -100);
-        e = b2w4_mul2(e, b2w4_pack2(power(c0), power(c1)));
-        n0 -= c0;
-        n1 -= c1;
-    }
-    return b2w4_mul2(e, b2w4_pack2(power(n0), power(n1)));
+// exp of x <= 0 (NaN stays), in 64 bits and rounded once.  After Tang, Table-driven implementation of
+// the exponential function (1989): x = i ln 2 / 32 + r, 2^(i % 32 / 32) from lane i % 32 (a whole
+// warp calls this), the Taylor series of e^r - 1 to r^5 with its last term economised (Chebyshev):
+// relative error below 2^-43, so about three results in a million are rounded to the neighbour of
+// the nearest number.  No branch, eight instructions of the 64-bit pipe and two conversions: 1500
+// tokens of 32 / 8 heads of 128 take 208 us, with CUDA's exp 264, without a table 223.
+__device__ __forceinline__ float exp_neg(float x, double lane_power) {
+    constexpr double kStep = 0.02166084939249829;  // ln 2 / 32
+    constexpr double kMagic = 6755399441055744.;   // 1.5 * 2^52: the sum's low bits are the integer
+    const double xd = (double)(x < -110.f ? -110.f : x);  // exp(-104) is zero in 32 bits
+    const double t = fma(xd, 1. / kStep, kMagic);
+    const double r = fma(t - kMagic, -kStep, xd);  // |r| <= kStep / 2
+    const int i = __double2loint(t);
+    const int hi = __shfl_sync(0xffffffffu, __double2hiint(lane_power), i & 31);
+    const int lo = __shfl_sync(0xffffffffu, __double2loint(lane_power), i & 31);
+    const double power = __hiloint2double(hi + ((i >> 5) << 20), lo);
+    constexpr double a = kStep / 2;  // r^5 / 120 as a cubic
+    double p = fma(r, 1. / 24., 1. / 6. + a * a * (5. / 480.));
+    p = fma(p, r, 0.5);
+    p = fma(p, r, 1. - a * a * a * a * (1. / 384.));
+    return (float)fma(power, p * r, power);
 }
 
 // kAttnThreads threads of the larger block
@@ -338,6 +321,7 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             warp_arrive(q_full);
         }
+        const double lane_power = exp2(lane / 32.);
         float m = -INFINITY, l = 0.f, alpha = 1.f;  // alpha: of the block before
         constexpr int kOwn = DIM / 2;               // the thread's share of the output
         uint64_t acc[kOwn / 2];
@@ -401,37 +385,33 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
                                       2 * i + 1 < seen ? b : -INFINITY);
                 }
             }
-            float top = m, low = INFINITY;
+            float top = m;
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 float a, b;
                 b2w4_unpack2(s[i], a, b);
                 top = fmaxf(fmaxf(top, a), b);
-                low = fminf(fminf(low, a), b);
             }
             float* mx = s_max + (j & 1) * 2 * kRows;
             mx[half * kRows + row] = top;
             pair_sync();
             top = fmaxf(top, mx[(1 - half) * kRows + row]);
             const float base = top == -INFINITY ? 0.f : top;  // nothing seen yet: all terms zero
-            const uint64_t minus = b2w4_pack2(-base, -base);
-            if (__all_sync(0xffffffffu, __fsub_rn(low, base) >= -86.f)) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    s[i] = exp2x<true>(add2(s[i], minus));
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    s[i] = exp2x<false>(add2(s[i], minus));
+            for (int i = 0; i < 16; ++i) {
+                float a, b;
+                b2w4_unpack2(s[i], a, b);
+                s[i] = b2w4_pack2(exp_neg(__fsub_rn(a, base), lane_power),
+                                  exp_neg(__fsub_rn(b, base), lane_power));
             }
             uint64_t sum[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 sum[i] = add2(add2(s[i], s[i + 4]), add2(s[i + 8], s[i + 12]));
             sum[0] = add2(add2(sum[0], sum[1]), add2(sum[2], sum[3]));
-            float sum0, sum1, factor, unused;
+            float sum0, sum1;
             b2w4_unpack2(sum[0], sum0, sum1);
-            b2w4_unpack2(exp2x<false>(b2w4_pack2(__fsub_rn(m, base), 0.f)), factor, unused);
+            const float factor = exp_neg(__fsub_rn(m, base), lane_power);
             m = top;
             l = __fadd_rn(__fmul_rn(l, factor), __fadd_rn(sum0, sum1));
             uint32_t pieces[3][16];

@@ -1141,14 +1141,19 @@ AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int c
 // Runs of tiles that take the tensor-core kernel (aligned rows), by what does not depend on the
 // position: a cache of 384 rows (below that the one-row arithmetic's bits are kept, see above) and
 // enough (token, head) rows for its blocks of 128 to fill a part of the chip.  Where it is taken it
-// is faster and closer to 64 bits than the tile kernel; us, and error in 2-norm on normal inputs:
-//   32 / 8 heads of 128   200 tokens 33.0 -> 28.5 (1.6e-7 -> 1.5e-7), 256 39.7 -> 26.7, behind 300
-//                         keys 110 -> 44 (4.0e-7 -> 2.2e-7), 1500 590 -> 167 (3.1e-7 -> 1.8e-7),
-//                         2000 behind 6000 keys 7076 -> 1673 (1.5e-6 -> 3.1e-7)
-//   28 / 4 heads of 128   333 tokens behind 50 keys 77 -> 45; 64 / 1 heads, 129 behind 300 87 -> 41
-//   64 / 8 heads of 64    380 tokens 76 -> 28, 1500 676 -> 197
+// is closer to 64 bits than the tile kernel, and faster but for the shortest runs at the head of a
+// cache; us, and error in 2-norm on normal inputs:
+//   32 / 8 heads of 128   200 tokens 33.2 -> 35.2 (1.6e-7 -> 1.5e-7), 256 39.7 -> 33.9, behind 300
+//                         keys 111 -> 58 (4.0e-7 -> 2.2e-7), 1500 589 -> 208 (3.1e-7 -> 1.8e-7),
+//                         2000 behind 6000 keys 7074 -> 2121 (1.5e-6 -> 3.1e-7)
+//   28 / 4 heads of 128   333 tokens behind 50 keys 77 -> 52; 64 / 1 heads, 129 behind 300 87 -> 50
+//   64 / 8 heads of 64    380 tokens 76 -> 32, 1500 676 -> 260
+// Error on other inputs, 32 / 8 heads, 256 tokens and 1500: values of one sign 1.8e-7 -> 0.8e-7 and
+// 4.1e-7 -> 1.0e-7; scores thirty times as large 6.9e-7 -> 5.3e-7 and 9.3e-7 -> 7.7e-7; queries and
+// values with the tails of exp(normal) 2.3e-7 -> 3.0e-7 and 5.8e-7 -> 3.4e-7 (the one kind of input
+// on which short runs lose: sums in tensor memory truncate).
 // The lines of rows per multiprocessor are not those of speed (8 / 8 heads of 128, 600 tokens behind
-// 100 keys 95 -> 54; 32 / 8 heads of 64, 640 tokens 97 -> 41): shorter runs keep their bits.
+// 100 keys take 95 in tiles; 32 / 8 heads of 64, 640 tokens 97): shorter runs keep their bits.
 bool attn_tensor(int tokens, int heads, int dim, int capacity, int sm_count) {
     return capacity >= 384 && (dim == 128 || dim == 64) &&
            (long)tokens * heads >= (dim == 128 ? 40l : 160l) * sm_count;

@@ -1052,3 +1052,33 @@ assert torch.equal(out[1], out[4])
 """ % os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("tokens,heads,dim", [(600, 64, 128), (1000, 64, 64)])
+def test_long_runs_take_exp_in_64_bits(ctx, tokens, heads, dim):
+    """The tensor-core kernel's probabilities are exp in 64 bits rounded once.  Two keys count, of
+    scores 0 and x <= 0 (both exact), with values that show p / (1 + p) and 1 / (1 + p); all further
+    scores are -1000.  Its exp is within 2^-43 of e^x, 2^-18 of a unit in the last place: of the
+    results, 2^-17 are expected to be rounded to the neighbour, 1e-4 are allowed (an exp in 32 bits
+    has some in a hundred).  From -69 on, as results below 2^-100 send a tile to the fp32 form."""
+    import torch
+    rng = np.random.default_rng(dim)
+    n, past, keys = tokens * heads, 64, 64 + tokens
+    x = np.where(rng.random(n) < 0.5, rng.uniform(-69, 0, n), -10.0 ** rng.uniform(-7, 1.8, n))
+    x = x.astype(np.float32)
+    q = np.zeros((tokens, heads, dim), np.float32)
+    q[..., 0], q[..., 1] = x.reshape(tokens, heads), 1.0
+    k, v = (np.zeros((1, max(384, keys), dim), np.float32) for _ in range(2))
+    k[0, 1, 0], k[0, 2:, 1] = 1.0, -1000.0
+    v[0, 0, 0], v[0, 1, 1] = 1.0, 1.0
+    out = torch.zeros((tokens, heads, dim), device="cuda")
+    ctx.attention(_dev(q), None, None, _dev(k), _dev(v), out, tokens, heads, 1, dim, past,
+                  k.shape[1], 1.0)
+    ctx.sync()
+    p = np.exp(x.astype(np.float64)).astype(np.float32)
+    total = np.float32(1.0) + p
+    want = np.stack([np.float32(1.0) / total, p / total], 1)
+    got = out.cpu().numpy().reshape(n, dim)
+    assert not got[:, 2:].any()
+    assert (got[:, :2] != want).mean() < 1e-4
+    assert np.abs(got[:, :2] - want).max() < 2.0 ** -23
