@@ -1,8 +1,8 @@
 // Causal attention of a long run of tokens over the cache on tcgen05.mma kind::f16: the products
 // of attention_tile.cuh with every fp32 operand as the sum of three bf16 numbers.
 //
-// x = h + m + l, each the bf16 nearest to what is left: 24 bits, so the sum is x (to 2^-133 for
-// the smallest).  A product takes six of the nine piece products, the small ones first,
+// x = h + m + l, each the bf16 nearest to what is left: 24 bits, so the sum is x unless x has bits
+// below 2^-133, the smallest bf16, or rounds to infinity.  A product takes six of the nine piece products, the small ones first,
 //   l h' + h l' + m m' + m h' + h m' + h h'
 // what is left out is below 2^-24 of |x x'|; sums are fp32 in tensor memory.  Scores,
 // probabilities (exp in 64 bits, rounded once), maxima and sums stay fp32, and the output's sum
@@ -26,12 +26,15 @@
 // logic at half rate, paired fp32 instructions two to three cycles each) and its exp about 2000 of
 // the 64-bit and conversion pipes; shared memory serves MMAs, splits and loads for about 3000.
 // Measured against the tile form: attn_tensor (decoder_ops.cu).  Tried with an exp in 32 bits, 1500
-// tokens of 32 / 8 heads of 128 (167 us; 208 with this one): all products with m and h of the keys
-// side by side 156 (error 2.3e-7 instead of 1.8e-7), each alone 188; three warps each to split 197,
-// five 170.
-// A row that comes out not finite, or so small that a piece of a value may have been lost, sends
-// the tile to the fp32 form (attention_tile.cuh), which has the rule for values of probability
-// zero; nothing is written before that is known.
+// tokens of 32 / 8 heads of 128 (167 us; 208 with this one, 214 with the checks below): all products
+// with m and h of the keys side by side 156 (error 2.3e-7 instead of 1.8e-7), each alone 188; three
+// warps each to split 197, five 170.
+// Some tiles go to the fp32 form (attention_tile.cuh), which has the rule for values of probability
+// zero; nothing is written before that is known:
+//   a result that is not finite, or not zero and below 2^-100 (a product of pieces may have been lost)
+//   a query, key or value that its pieces do not sum to (what is left after the third is not zero)
+//   a probability that its pieces do not sum to (below 2^-110, at most 2^-134 is lost), where a
+//   value is 2^32 or more, or a result zero or below 2^-60: up to 2^17 keys lose less than 2^-85
 // Every wait is bounded; on a timeout the kernel flags the status word and drains.
 #include "attention_tile.cuh"
 #include "tcgen05_ops.cuh"
@@ -43,6 +46,7 @@ constexpr int kRows = 128;   // (token, head) rows of a block
 constexpr int kRowWarps = 8, kScoreWarp = 8, kOutWarp = 9, kSplitWarp0 = 10;
 constexpr int kSplitWarps = 7;  // for the keys, and as many for the values
 constexpr int kTcThreads = (kSplitWarp0 + 2 * kSplitWarps) * 32;
+constexpr float kLarge = 0x1p32f, kSmall = 0x1p-100f, kSmallLost = 0x1p-60f;  // see above
 constexpr int kRegsStart = 80, kRegsRows = 128, kRegsOther = 56;
 static_assert(kRowWarps * 32 == kAttnThreads);
 static_assert(2 * kRegsRows + 4 * kRegsOther <= 6 * kRegsStart, "registers of the block");
@@ -209,7 +213,8 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
     uint64_t* v_free = bars + 14;       // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    volatile int* s_odd = s_abort + 1;
+    volatile int* s_odd = s_abort + 1;   // to the fp32 form
+    volatile int* s_lost = s_abort + 2;  // bits of a probability
     float* s_max = reinterpret_cast<float*>(smem + S::kMax);
 
     b2w4_pdl_launch_dependents();
@@ -228,7 +233,7 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
             mbar_init(&v_free[b], 1);
         }
         *s_abort = 0;
-        *s_odd = 0;
+        *s_odd = *s_lost = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kScoreWarp) {
@@ -292,6 +297,7 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
         auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(3 + quarter) : "memory"); };
         {
             const float4* src = reinterpret_cast<const float4*>(q + (vis ? row_offset(row) : 0));
+            uint64_t left = 0ull;
 #pragma unroll 1
             for (int c = half * (DIM / 2); c < (half + 1) * (DIM / 2); c += 32) {
                 uint64_t v[16];
@@ -311,11 +317,16 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
                         tmem_st16(lane_addr + T::kQ + p * (DIM / 2) + c / 2, r);
                 }
 #pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    left |= v[i];
+#pragma unroll
                 for (int i = 0; i < 4; ++i)
                     *reinterpret_cast<uint4*>(smem + S::kQ + c / 64 * S::kQPart +
                                               place(row, c % 64 / 8 + i)) =
                         make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
             }
+            if (left)
+                *s_odd = 1;
             tmem_st_wait();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -420,6 +431,12 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
                     pieces[p][i] = take_piece(s[i]);
+            uint64_t left = 0ull;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                left |= s[i];
+            if (left)
+                *s_lost = 1;
             // the product before has read the probabilities
             if (j)
                 await(o_full, (j - 1) & 1);
@@ -440,20 +457,28 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
         mx[half * kRows + row] = l;
         pair_sync();
         const float total = __fadd_rn(mx[row], mx[kRows + row]);
+        // every warp's words are there since the last block's probabilities were
+        const bool lost = *s_lost;
+        const float small = lost ? kSmallLost : kSmall;
         bool odd = false;
+        if (lost)
+            for (int i = threadIdx.x; i < vis_max * (DIM / 4); i += kAttnThreads) {
+                const float4 f = reinterpret_cast<const float4*>(vc)[i];
+                odd |= fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))) >= kLarge;
+            }
 #pragma unroll
         for (int i = 0; i < kOwn / 2; ++i) {
             float a, b;
             b2w4_unpack2(acc[i], a, b);
             a = __fdiv_rn(a, total);
             b = __fdiv_rn(b, total);
-            auto plain = [](float v) {  // zero, or 2^-100 <= |v| < inf
-                return v == 0.f || (fabsf(v) >= 0x1p-100f && fabsf(v) < INFINITY);
+            auto plain = [&](float v) {
+                return (v == 0.f && !lost) || (fabsf(v) >= small && fabsf(v) < INFINITY);
             };
-            odd |= !plain(a) || !plain(b);
+            odd |= vis && (!plain(a) || !plain(b));
             acc[i] = b2w4_pack2(a, b);
         }
-        if (odd && vis)
+        if (odd)
             *s_odd = 1;
         PartSync::sync();
         if (vis && !*s_odd && !*s_abort) {
@@ -598,6 +623,7 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
                     break;
                 }
                 uint8_t* dst = ring + (j & 1) * S::kBuf;
+                uint64_t left = 0ull;
 #pragma unroll
                 for (int u = 0; u < kOwn; ++u) {
                     const int task = w0 + kSplitWarps * u;
@@ -618,7 +644,10 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
                         o.w = take_piece(x[3]);
                         *reinterpret_cast<uint4*>(to + p * piece) = o;
                     }
+                    left |= x[0] | x[1] | x[2] | x[3];
                 }
+                if (left)
+                    *s_odd = 1;
                 // make the generic-proxy writes visible to the tensor core's async proxy
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 warp_arrive(&full[j & 1]);

@@ -1143,11 +1143,11 @@ AttnPlan attn_plan(int tokens, int heads, int kv_heads, int dim, int past, int c
 // enough (token, head) rows for its blocks of 128 to fill a part of the chip.  Where it is taken it
 // is closer to 64 bits than the tile kernel, and faster but for the shortest runs at the head of a
 // cache; us, and error in 2-norm on normal inputs:
-//   32 / 8 heads of 128   200 tokens 33.2 -> 35.2 (1.6e-7 -> 1.5e-7), 256 39.7 -> 33.9, behind 300
-//                         keys 111 -> 58 (4.0e-7 -> 2.2e-7), 1500 589 -> 208 (3.1e-7 -> 1.8e-7),
-//                         2000 behind 6000 keys 7074 -> 2121 (1.5e-6 -> 3.1e-7)
-//   28 / 4 heads of 128   333 tokens behind 50 keys 77 -> 52; 64 / 1 heads, 129 behind 300 87 -> 50
-//   64 / 8 heads of 64    380 tokens 76 -> 32, 1500 676 -> 260
+//   32 / 8 heads of 128   200 tokens 33.2 -> 35.3 (1.6e-7 -> 1.5e-7), 256 39.7 -> 34.7, behind 300
+//                         keys 111 -> 59 (4.0e-7 -> 2.2e-7), 1500 589 -> 214 (3.1e-7 -> 1.8e-7),
+//                         2000 behind 6000 keys 7074 -> 2172 (1.5e-6 -> 3.1e-7)
+//   28 / 4 heads of 128   333 tokens behind 50 keys 77 -> 52; 64 / 1 heads, 129 behind 300 87 -> 51
+//   64 / 8 heads of 64    380 tokens 76 -> 34, 1500 676 -> 277
 // Error on other inputs, 32 / 8 heads, 256 tokens and 1500: values of one sign 1.8e-7 -> 0.8e-7 and
 // 4.1e-7 -> 1.0e-7; scores thirty times as large 6.9e-7 -> 5.3e-7 and 9.3e-7 -> 7.7e-7; queries and
 // values with the tails of exp(normal) 2.3e-7 -> 3.0e-7 and 5.8e-7 -> 3.4e-7 (the one kind of input

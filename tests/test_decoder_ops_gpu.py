@@ -1082,3 +1082,57 @@ def test_long_runs_take_exp_in_64_bits(ctx, tokens, heads, dim):
     assert not got[:, 2:].any()
     assert (got[:, :2] != want).mean() < 1e-4
     assert np.abs(got[:, :2] - want).max() < 2.0 ** -23
+
+
+@pytest.mark.parametrize("tokens,heads,kv_heads,dim", [(256, 24, 8, 128), (640, 40, 8, 64)])
+def test_long_runs_whose_pieces_lose_bits(ctx, tokens, heads, kv_heads, dim):
+    """Queries, keys, values and probabilities with bits below 2^-133, which three bf16 pieces drop:
+    as precise as in fp32.  Keys or queries near 2^-124 against rows near 2^124 (tolerance of the
+    forms); values near 2^-138 averaged (they and the result are multiples of 2^-149); one key with
+    probability p and value v, where a key of value zero has all the rest: a product of three
+    roundings, 2^-22, and half of 2^-149 where it is not a normal number."""
+    import torch
+    past, g = 300, torch.Generator(device="cuda").manual_seed(dim)
+    keys = past + tokens
+
+    def rand(*shape):
+        return torch.randn(shape, device="cuda", generator=g)
+
+    def run(q, kc, vc):
+        out = torch.full((tokens, heads, dim), 7.0, device="cuda")
+        ctx.attention(q, None, None, kc, vc, out, tokens, heads, kv_heads, dim, past, keys, 1.0)
+        ctx.sync()
+        return out.double(), _attention_fp64_cuda(q, kc, vc, past, 1.0)
+
+    q, kc, vc = rand(tokens, heads, dim), rand(kv_heads, keys, dim), rand(kv_heads, keys, dim)
+    q *= dim ** -0.5
+    for up, down in ((q, kc), (kc, q)):
+        a, b = up * 2.0 ** 124, down * 2.0 ** -124
+        got, want = run(*((a, b) if up is q else (b, a)), vc)
+        assert float((got - want).norm() / want.norm()) < 1e-5
+    got, want = run(torch.zeros_like(q), kc, (torch.rand_like(vc) + 0.5) * 2.0 ** -138)
+    assert float((got - want).abs().max()) <= 2.0 ** -149 and bool(got.all())
+
+    q[:], kc[:], vc[:] = 0.0, 0.0, 0.0
+    q[..., 0] = kc[:, 1, 0] = 1.0
+    kc[:, 2:, 0] = -1000.0
+    for x, v in ((-85.0, 1e38), (-80.0, 3e33), (-86.0, 2.0 ** 30), (-84.5, 2.0 ** 30),
+                 (-74.2, 2.0 ** -21), (-60.0, 2.0 ** -50), (-74.2, 2.0 ** -39), (-103.0, 1e30)):
+        kc[:, 1, 0] = x
+        vc[:, 1, ::2] = v
+        got, want = run(q, kc, vc)
+        # exp(-103) in 32 bits is 1.3e-45 or 2^-149
+        p = float(np.float32(np.exp(np.float64(x))))
+        want *= p / np.exp(x)
+        assert float((got - want).abs().max()) <= 2.0 ** -22 * float(want.max()) + 2.0 ** -149
+        assert not got[..., 1::2].any()
+    # probabilities that lose bits and count for nothing: in pieces, with zeros and without
+    kc[:, 1, 0] = -80.0
+    vc.copy_(rand(*vc.shape))
+    got, want = run(q, kc, vc)
+    assert float((got - want).norm() / want.norm()) < 1e-5
+    vc[:, 0, ::2] = 0.0
+    got, want = run(q, kc, vc)
+    assert float((got - want).norm() / want.norm()) < 1e-5
+    tiny = float((got - want)[..., ::2].norm() / want[..., ::2].norm())
+    assert tiny < 1e-5
