@@ -478,17 +478,18 @@ attention_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cac
             odd |= vis && (!plain(a) || !plain(b));
             acc[i] = b2w4_pack2(a, b);
         }
-        if (odd)
-            *s_odd = 1;
-        PartSync::sync();
-        if (vis && !*s_odd && !*s_abort) {
+        // One answer for all rows, as the fp32 form has barriers that each of them must meet: the MMA
+        // threads still wait for their last commits and may report a failure at any time.
+        const bool failed = PartSync::any(*s_abort);
+        const bool again = PartSync::any(odd || *s_odd);
+        if (vis && !again && !failed) {
             ulonglong2* dst = reinterpret_cast<ulonglong2*>(out + row_offset(row) + half * kOwn);
 #pragma unroll
             for (int i = 0; i < kOwn / 4; ++i)
                 dst[i] = make_ulonglong2(acc[2 * i], acc[2 * i + 1]);
         }
         // the last product has retired, so nothing reads or writes the buffers any more
-        if (*s_odd && !*s_abort) {
+        if (again && !failed) {
             const int tq_part = 64 / rep, end = min(tokens, t0 + tq);
             for (int t = t0; t < end; t += tq_part) {
                 attention_tile<DIM, 64, true, PartSync>(
