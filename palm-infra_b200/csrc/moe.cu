@@ -974,7 +974,10 @@ moe_grouped_small_kernel(const GroupedSmallArgs a) {
             if (!mbar_wait_bounded(&s_bar[0])) {
                 if (lane == 0)
                     b2w4_report_timeout(a.status);
-                return;  // this warp's rows stay unwritten; the status word says so
+                // The status word says that the rows are void.  In a cluster the warp goes on with
+                // what is there, to both of its barriers: the other blocks read this one's rows.
+                if (!combined)
+                    return;
             }
             weights_ready = true;
         }
