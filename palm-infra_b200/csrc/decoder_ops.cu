@@ -525,11 +525,12 @@ struct PrepArgs {
     float eps;
     float *k_cache, *v_cache;
 };
-// RING: the block is alone on its multiprocessor, so key and value rows go through a ring of slots
-// per warp in its shared memory (cp.async): first the warp's keys, then its values, a slot as soon
-// as it has been read, from before the query rows are made to the last value row.  No warp waits for
-// another, and every key and value stays with the warp and lanes that have it without the ring: the
-// same bits.  What it mends: with loads into registers (8 KB of keys or 4 KB of values in flight per
+// RING: there are no more blocks than multiprocessors, one or two to each, so key and value rows go
+// through a ring of slots per warp in their shared memory (cp.async): first the warp's keys, then its
+// values, a slot as soon as it has been read, from before the query rows are made to the last value
+// row.  No warp waits for another.  The same bits as without: a key's dot product has one order in
+// whichever warp it is made (a warp has four keys in a row at 128 features, eight at 64; without the
+// ring up to sixteen), and every value stays with its warp and lanes.  What it mends: with loads into registers (8 KB of keys or 4 KB of values in flight per
 // warp) each pass over the block's keys waits for its memory round trip, and nothing is on its way
 // while the query rows are made.  (By bulk copies, 2 KB of keys or 512 bytes of values each, a step
 // of eight layers behind 6000 keys took 581 us instead of 455.)
@@ -1187,7 +1188,7 @@ template <int DIM, int HR, int CTAS, bool PREP, bool RING>
 int launch_split_as(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& plan,
                     bool* placed) {
     static b2w4_smem_optin cfg, wide;
-    static b2w4_smem_optin held, held_alone;  // clusters_held + 1, per device
+    static b2w4_smem_optin held;  // clusters_held + 1, per device
     auto kern = attention_split_kernel<DIM, HR, CTAS, PREP, RING>;
     const PrepArgs prep = PREP ? *a.prep : PrepArgs();
     const int range = max((keys + CTAS - 1) / CTAS, min(keys, plan.one_range));
@@ -1200,16 +1201,20 @@ int launch_split_as(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& 
     B2W4_CUDA(ctx, b2w4_opt_in_smem(ctx, kern, RING ? kHalfSmem + 1 : smem, cfg));
     if constexpr (CTAS > 1)
         B2W4_CUDA(ctx, b2w4_opt_in_cluster(ctx, kern, wide));
-    auto clusters = [&](b2w4_smem_optin& cache, size_t bytes) {
-        size_t& n = cache.bytes[ctx->device];
+    // a ring: asked with the most that its launch may take
+    long clusters = 0;
+    if (CTAS > 1) {
+        size_t& n = held.bytes[ctx->device];
         if (!n)
-            n = 1 + clusters_held(kern, CTAS, bytes);
-        return (long)n - 1;
-    };
+            n = 1 + clusters_held(kern, CTAS, RING ? kHalfSmem + 1 : 32 * 1024);
+        clusters = (long)n - 1;
+        if (!clusters)
+            return B2W4_OK;  // without a ring, or a smaller cluster
+    }
     // A ring's blocks go to a multiprocessor each where all their clusters fit that way (sixteen
     // blocks of eight clusters do not: two waves, 33 us instead of 22).  A step of eight layers
     // behind 300 keys 317 -> 310 us.
-    if (RING && (CTAS == 1 || clusters(held_alone, kHalfSmem + 1) >= (long)grid.y * grid.z))
+    if (RING && (CTAS == 1 || clusters >= (long)grid.y * grid.z))
         smem = kHalfSmem + 1;
     if constexpr (CTAS == 1) {
         B2W4_CUDA(ctx, b2w4_launch_chained(ctx->pdl, kern, grid, dim3(kAttnThreads), smem,
@@ -1217,8 +1222,6 @@ int launch_split_as(b2w4_ctx* ctx, const AttnArgs& a, int keys, const AttnPlan& 
                                            a.tokens, a.heads, a.kv_heads, a.past, a.past_dev,
                                            a.capacity, a.scale, plan.one_range, prep));
     } else {
-        if (!clusters(held, 32 * 1024))
-            return B2W4_OK;
         B2W4_CUDA(ctx, b2w4_launch_chained_cluster(
                            ctx->pdl, kern, grid, dim3(kAttnThreads), CTAS, smem, ctx->stream,
                            a.q, a.k_cache, a.v_cache, a.out, a.tokens, a.heads, a.kv_heads,
