@@ -395,10 +395,12 @@ gemm_w4a8_tc32_kernel(const GemmArgs a) {
                     (step(std::integral_constant<int, I>()), ...);
                 }(std::make_integer_sequence<int, kChunks>());
             };
-            // Two groups a turn need no moves of the scales; the code is twice as long, which wide
-            // tiles pay for (measured: 112 columns 205 us a turn of two, 208 of one; 96 columns
-            // 27.4 / 26.7, 128 columns 395 / 389, 48 columns 50.0 / 51.4, 32 columns 37.2 / 38.6).
-            constexpr bool kPairs = RP <= 64 || RP == 112;
+            // Two groups a turn need no moves of the scales, but the code is twice as long: taken where
+            // a group's is short.  Time of two a turn to one, K = 1024 / 2560 / 9728, one to five sizes
+            // each, fp16 and fp32 scales alike: 32 columns 0.99 / 0.98 / 0.97, 48 1.00 / 0.99 / 0.98, 64
+            // 0.98 / 0.97 / 0.96, 80 0.98 / 0.96 / 0.95, 96 1.02 / 1.01 / 1.00, 112 1.02 / 1.01 / 1.01,
+            // 128 1.01 / 1.01 / 1.01.
+            constexpr bool kPairs = RP <= 80;
             for (int g = 0; g < G; g += kPairs ? 2 : 1) {
                 group(g, a0);
                 if constexpr (!kPairs) {

@@ -701,3 +701,15 @@ def test_many_rows_on_persistent_blocks(ctx, n, k, f32):
     want = ol.apply_activation(ref.copy(), act, begin, length)
     assert y.cpu().numpy().tobytes() == want.tobytes()
     w.free()
+
+
+@pytest.mark.parametrize("m,n,k", [(900, 1068, 896), (500, 1900, 1152), (900, 1224, 384),
+                                   (1000, 1380, 1024), (500, 2500, 1408)])
+def test_per32_tensor_core_tiles_of_64_and_80_columns(ctx_tc, m, n, k):
+    """The two tile widths between those of test_per32_tensor_core_tiles_bit_exact that take two
+    groups a turn, with odd and even numbers of groups, fewer and more than pipeline stages."""
+    blocks = pkg.synth.bg128_weight(20261125, n + k + m + 2, n, k)
+    x = pkg.synth.activations(7, m + 11, m, k)
+    x[m // 2] = np.sign(x[m // 2])  # every code +-127: the largest sums
+    y, _ = run_gpu(ctx_tc, blocks, n, k, x, rule=ol.ACT_G32, sums=False, pad=4 if n % 16 else 0)
+    assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).tobytes()
