@@ -947,21 +947,40 @@ size_t gemv_stream_bytes(int groups, int tpc, int d_stride, bool scl16) {
 }
 // Tiles of a chunk: as many as fit half an SM, the count whose items fill the sixteen warps' rounds
 // best; 0: none fits.
-int gemv_stream_tpc(const b2w4_weight* w, int d_stride) {
-    const int ipt = (w->groups + 3) / 4;
+int gemv_stream_tpc(int groups, bool scl16) {
+    const int ipt = (groups + 3) / 4, d_stride = gemv_d_stride(1, groups, false);
     int best = 0;
     double best_fill = 0.;
     for (int t = 1; t <= kStreamMaxTpc; ++t) {
         const int items = t * ipt;
         const double fill = (double)items / ((items + 15) / 16 * 16);
-        if (gemv_stream_bytes(w->groups, t, d_stride, w->scales_fp16 != 0) <= 112 * 1024 &&
-            fill >= best_fill) {
+        if (gemv_stream_bytes(groups, t, d_stride, scl16) <= 112 * 1024 && fill >= best_fill) {
             best = t;
             best_fill = fill;
         }
     }
     return best;
 }
+// The chunk with which a launch of `ctas` CTAs of gemv_w4a8_kernel goes to the persistent kernel, or
+// 0: it does not.  Lines in CTAs per SM.  Time of the persistent kernel to that one, plain / greedy
+// token, in a graph over weights larger than L2:
+//   three tiles and more   from 3.5.  At the line K = 256 0.82 / 0.72, 512 0.88 / 0.78, 768 0.99 / 0.97,
+//                          1024 1.02 / 1.00, 1280 0.92 / 0.94, 1792 0.92 / 0.93, 2560 0.96 / 0.94; at
+//                          eight 0.77 / 0.73 (512), 0.80 / 0.79 (1024), 0.87 / 0.85 (2560)
+//   two tiles              from 4.5.  At 3.5, 4.5 and 8: K = 2816 1.00 / 1.04, 0.96 / 0.94, 0.96 / 0.96;
+//                          3584 1.01 / 1.05, 0.98 / 0.94, 0.95 / 0.94; 4096 1.02 / 1.02, 0.96 / 0.93,
+//                          0.89 / 0.89
+//   one tile               from 4.5, and 40 groups: the sixteen warps take 64 groups a round, and a
+//                          round of fewer leaves more of them idle than the ring gives.  K = 4352
+//                          (34) 1.08 / 1.10, 1.03 / 1.08, 1.10 / 1.13; 4864 (38) 1.15 / 1.17, 1.06 /
+//                          1.04, 1.06 / 1.05; 5120 1.02 / 1.11, 0.95 / 0.98, 0.96 / 0.99; 5632 1.02 /
+//                          1.07, 0.91 / 0.95, 0.92 / 0.97; 7680 1.02 / 1.05, 0.93 / 0.94, 0.87 / 0.87
+// fp32 scales: within 0.02 of these, by the chunk they have (K = 4096 one tile, 1.06 / 1.02 at 4.5).
+int gemv_stream_chunk(int groups, bool scl16, int ctas, int sm_count) {
+    const int t = gemv_stream_tpc(groups, scl16);
+    return 2l * ctas < (t >= 3 ? 7l : 9l) * sm_count || (t == 1 && groups < 40) ? 0 : t;
+}
+
 template <bool SCL16, bool TOP1>
 int launch_stream(b2w4_ctx* ctx, const GemvArgs& a) {
     auto kern = gemv_w4a8_stream_kernel<SCL16, TOP1>;
@@ -1012,6 +1031,11 @@ bool b2w4_gemv_fits(const b2w4_weight* w, int m, int act_rule, bool swiglu) {
         return b2w4_gemv_mma_fits(w, m, act_rule);
     return gemv_smem_bytes(1, w->k, w->groups, swiglu ? 2 : 1, w->scales_fp16 != 0,
                            act_rule == B2W4_ACT_G32) <= 220 * 1024;
+}
+
+// What gemv_stream_chunk says, for checks without a device.
+extern "C" int b2w4_gemv_stream_plan(int groups, int scales_fp16, int ctas, int sm_count) {
+    return gemv_stream_chunk(groups, scales_fp16 != 0, ctas, sm_count);
 }
 
 // Rows are processed four at a time; each pass streams the weight once.
@@ -1121,20 +1145,17 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
                 return launch_split(ctx, a, scl16, bytes);
             a.tpc = tpc;
         }
-        // Many rows: persistent CTAs from three and a half CTAs of the kernel above per SM on.  us in
-        // a graph, that kernel / persistent, plain and with the greedy token: K = 2560 25000 rows
-        // (2.4 per SM, not taken) 9.3 / 9.7, 40000 (3.8) 13.1 / 12.3 and 14.6 / 13.8, 100000 27.2 /
-        // 23.8 and 30.6 / 26.2, 151936 39.5 / 35.8 and 42.8 / 38.5; K = 4096 19456 rows (3.3, not
-        // taken) 11.3 / 11.8, 40000 20.2 / 18.1; K = 512 60000 rows (3.2, not taken) 6.5 / 7.7,
-        // 151936 14.3 / 10.7; K = 1024 151936 rows 20.0 / 16.1.
-        if (!a32 && !sums && !tp && !norm && !swiglu && ctx->gemv_tpc_override == 0 &&
-            2 * ((w->tiles + tpc - 1) / tpc) >= 7 * ctx->sm_count &&
-            gemv_stream_tpc(w, a.d_stride) > 0) {
-            take(gemv_stream_tpc(w, a.d_stride));
-            return top1 ? (scl16 ? launch_stream<true, true>(ctx, a)
-                                 : launch_stream<false, true>(ctx, a))
-                        : (scl16 ? launch_stream<true, false>(ctx, a)
-                                 : launch_stream<false, false>(ctx, a));
+        // Many rows: persistent CTAs.
+        if (!a32 && !sums && !tp && !norm && !swiglu && ctx->gemv_tpc_override == 0) {
+            const int chunk = gemv_stream_chunk(w->groups, scl16, (w->tiles + tpc - 1) / tpc,
+                                                ctx->sm_count);
+            if (chunk > 0) {
+                take(chunk);
+                return top1 ? (scl16 ? launch_stream<true, true>(ctx, a)
+                                     : launch_stream<false, true>(ctx, a))
+                            : (scl16 ? launch_stream<true, false>(ctx, a)
+                                     : launch_stream<false, false>(ctx, a));
+            }
         }
         const size_t smem =
             gemv_smem_bytes(mt, w->k, w->groups, tpc, scl16, a32, norm != nullptr);

@@ -703,6 +703,40 @@ def test_many_rows_on_persistent_blocks(ctx, n, k, f32):
     w.free()
 
 
+@pytest.mark.parametrize("n,k,f32,tiles", [(21801, 4096, False, 2), (23001, 3584, True, 2),
+                                           (16501, 5120, True, 1), (11101, 7680, False, 1)])
+def test_persistent_blocks_of_few_tiles(ctx, n, k, f32, tiles):
+    """Chunks of two tiles and of one, just above their line, plain and with the greedy token: the
+    oracle's bits."""
+    import ctypes as C
+    import torch
+    blocks = pkg.synth.bg128_weight(20261125, n + k, n, k)
+    if f32:  # scales that fp16 cannot hold
+        blocks = np.array(blocks, copy=True)
+        s = blocks.reshape(-1, 544)[:, :32].copy().view(np.float32)
+        blocks.reshape(-1, 544)[:, :32] = (s * np.float32(1.0000001) + np.float32(1e-9) *
+                                           (s != 0)).astype(np.float32).view(np.uint8)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148:  # four (up to 4096 values a row), three or two tiles in a block of the other kernel
+        per = 4 if k <= 4096 else 3 if k <= 6144 else 2
+        plan = C.CDLL(pkg.capi.LIB_PATH).b2w4_gemv_stream_plan
+        assert plan(k // 128, not f32, -(-(-(-n // 8)) // per), sms) == tiles
+    x = pkg.synth.activations(91, n, 1, k)
+    ref = ol.matmul_w4(blocks, n, k, x)
+    w = ctx.upload_weight(blocks, n, k)
+    xd = torch.from_numpy(x).cuda()
+    y, logits = (torch.zeros((1, n), device="cuda") for _ in range(2))
+    tok = torch.full((2,), -1, dtype=torch.int32, device="cuda")
+    ctx.matmul(w, xd, y)
+    ctx.matmul_argmax(w, xd, tok[:1], logits)
+    ctx.matmul_argmax(w, xd, tok[1:])
+    ctx.sync()
+    assert y.cpu().numpy().tobytes() == ref.tobytes()
+    assert logits.cpu().numpy().tobytes() == ref.tobytes()
+    assert tok.tolist() == [ol.argmax_token(ref[0])] * 2
+    w.free()
+
+
 @pytest.mark.parametrize("m,n,k", [(900, 1068, 896), (500, 1900, 1152), (900, 1224, 384),
                                    (1000, 1380, 1024), (500, 2500, 1408)])
 def test_per32_tensor_core_tiles_of_64_and_80_columns(ctx_tc, m, n, k):
