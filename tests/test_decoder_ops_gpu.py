@@ -962,28 +962,10 @@ def test_long_runs_with_extreme_values(ctx, tokens, heads, kv_heads, dim):
     assert torch.isnan(got[tokens // 2:]).all() and torch.isfinite(got[:tokens // 2]).all()
 
 
-@pytest.mark.parametrize("past,heads,kv_heads,dim,cap", [
-    (0, 8, 2, 128, 96), (3, 8, 2, 128, 96), (94, 4, 1, 64, 96),      # one block per kv head
-    (127, 32, 8, 128, 800), (159, 32, 8, 128, 800), (703, 6, 6, 128, 800),
-    (6015, 32, 8, 128, 6100), (5500, 16, 8, 64, 6100),               # the ring turns over
-    (4095, 4, 1, 128, 4096), (2999, 2, 2, 64, 3001)])
-def test_attention_step_through_the_ring(ctx, past, heads, kv_heads, dim, cap):
-    """A decode step whose blocks have a multiprocessor each brings the cache in through a ring:
-    the bits of the separate operators at the edges of a slot's keys, with fewer keys than warps,
-    with more slots than the ring has, and with the new key in the first and in the last slot.
-    Rows past the position are NaN, and so is a key of probability zero's value row."""
+def _step_both_ways(ctx, qkv, heads, kv_heads, dim, qw, kw, cos, sin, past, cap, cache):
+    """A decode step with its operators apart and in one launch, the position given by the host and
+    on the device: the same bits in the caches and in the result, which is returned."""
     import torch
-    g = torch.Generator(device="cuda").manual_seed(past + dim)
-    qkv = torch.randn((1, (heads + 2 * kv_heads) * dim), device="cuda", generator=g)
-    qw, kw = (torch.rand(dim, device="cuda", generator=g) + 0.5 for _ in range(2))
-    cos, sin = (_dev(t) for t in pkg.decoder.rope_tables(range(cap), dim, 1e6))
-    cache = [torch.randn((kv_heads, cap, dim), device="cuda", generator=g) for _ in range(2)]
-    if past > 9:  # a score of -inf: the key never counts, nor does its value row
-        cache[0][:, 5] = float("-inf") * torch.sign(qkv[0, :1]).abs()
-        cache[0][:, 5, 1:] = 0.0
-        cache[1][:, 5] = 0.0
-    for c in cache:
-        c[:, past + 1:] = float("nan")
     pos = torch.tensor([past], dtype=torch.int32, device="cuda")
     for position, host in ((None, past), (pos, 0)):
         want_kv, got_kv = ([c.clone() for c in cache] for _ in range(2))
@@ -998,6 +980,67 @@ def test_attention_step_through_the_ring(ctx, past, heads, kv_heads, dim, cap):
         for a, b in zip(got_kv, want_kv):
             assert torch.equal(a.view(torch.int32), b.view(torch.int32))
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    return want
+
+
+RING_STEPS = [  # past, heads, kv_heads, dim, cap
+    (0, 8, 2, 128, 96), (3, 8, 2, 128, 96), (94, 4, 1, 64, 96),      # one block per kv head
+    (127, 32, 8, 128, 800), (159, 32, 8, 128, 800), (703, 6, 6, 128, 800),
+    (6015, 32, 8, 128, 6100), (5500, 16, 8, 64, 6100),               # the ring turns over
+    (4095, 4, 1, 128, 4096), (2999, 2, 2, 64, 3001)]
+
+
+@pytest.mark.parametrize("past,heads,kv_heads,dim,cap", RING_STEPS)
+def test_attention_step_through_the_ring(ctx, past, heads, kv_heads, dim, cap):
+    """A decode step whose blocks have a multiprocessor each brings the cache in through a ring:
+    the bits of the separate operators at the edges of a slot's keys, with fewer keys than warps,
+    with more slots than the ring has, and with the new key in the first and in the last slot.
+    Rows past the position are NaN; all scores and results are finite, so what is compared is made
+    of the rows that the ring brought."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(past + dim)
+    qkv = torch.randn((1, (heads + 2 * kv_heads) * dim), device="cuda", generator=g)
+    qw, kw = (torch.rand(dim, device="cuda", generator=g) + 0.5 for _ in range(2))
+    cos, sin = (_dev(t) for t in pkg.decoder.rope_tables(range(cap), dim, 1e6))
+    cache = [torch.randn((kv_heads, cap, dim), device="cuda", generator=g) for _ in range(2)]
+    for c in cache:
+        c[:, past + 1:] = float("nan")
+    want = _step_both_ways(ctx, qkv, heads, kv_heads, dim, qw, kw, cos, sin, past, cap, cache)
+    assert bool(torch.isfinite(want).all())
+
+
+@pytest.mark.parametrize("past,heads,kv_heads,dim,cap", RING_STEPS[2:])
+def test_ring_ignores_value_rows_of_zero_probability(ctx, past, heads, kv_heads, dim, cap):
+    """Keys at both ends of the cache that point away from every query head of their kv head, which
+    are alike: probability zero for all of them, so their value rows of NaN count for nothing and
+    the result stays the one that the ring's rows give, against 64 bits too."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(past + dim + 1)
+    rep = heads // kv_heads
+    qkv = torch.randn((1, (heads + 2 * kv_heads) * dim), device="cuda", generator=g)
+    rows = qkv.view(heads + 2 * kv_heads, dim)
+    alike = rows[:kv_heads].repeat_interleave(rep, 0).clone()
+    rows[:heads] = alike + 0.1 * rows[:heads]
+    qw, kw = (torch.rand(dim, device="cuda", generator=g) + 0.5 for _ in range(2))
+    cos, sin = (_dev(t) for t in pkg.decoder.rope_tables(range(cap), dim, 1e6))
+    cache = [torch.randn((kv_heads, cap, dim), device="cuda", generator=g) for _ in range(2)]
+    q = torch.zeros((1, heads * dim), device="cuda")
+    kv = [c.clone() for c in cache]
+    ctx.qkv_prepare(qkv, 1, heads, kv_heads, dim, qw, kw, 1e-6, cos, sin, past, q, *kv, cap)
+    ctx.sync()
+    away = -100.0 * q.view(kv_heads, rep, dim).mean(1)
+    for key in (5, past - 1):
+        cache[0][:, key], cache[1][:, key] = away, float("nan")
+    for c in cache:
+        c[:, past + 1:] = float("nan")
+    want = _step_both_ways(ctx, qkv, heads, kv_heads, dim, qw, kw, cos, sin, past, cap, cache)
+    assert bool(torch.isfinite(want).all())
+    for c, new in zip(cache, kv):
+        c[:, past] = new[:, past]
+    cache[1][:, [5, past - 1]] = 0.0
+    ref = _attention_fp64_cuda(q.view(1, heads, dim), *cache, past, dim ** -0.5)
+    got = want.view(1, heads, dim).double()
+    assert float((got - ref).norm() / ref.norm()) < 1e-5
 
 
 @pytest.mark.parametrize("n,k,f32", [(18960, 2560, True), (9600, 4224, False), (37920, 1280, False),
@@ -1136,3 +1179,38 @@ def test_long_runs_whose_pieces_lose_bits(ctx, tokens, heads, kv_heads, dim):
     assert float((got - want).norm() / want.norm()) < 1e-5
     tiny = float((got - want)[..., ::2].norm() / want[..., ::2].norm())
     assert tiny < 1e-5
+
+
+@pytest.mark.parametrize("tokens,past,heads,kv_heads,dim", [(256, 128, 24, 8, 128), (640, 0, 40, 8, 64),
+                                                            (2000, 6000, 4, 1, 128)])
+@pytest.mark.parametrize("kind", ["values of one sign", "flat", "sharp", "large scores"])
+def test_long_runs_on_other_inputs(ctx, tokens, past, heads, kv_heads, dim, kind):
+    """The tensor-core kernel is nearer to 64 bits than the one-row arithmetic in fp32 where its
+    truncated sums are all of one sign, where every key counts or only a few do, and where all scores
+    are large."""
+    import torch
+    keys, scale = past + tokens, dim ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(tokens + dim + 1)
+    q = torch.randn((tokens, heads, dim), device="cuda", generator=g)
+    kc, vc = (torch.randn((kv_heads, max(384, keys), dim), device="cuda", generator=g)
+              for _ in range(2))
+    if kind == "values of one sign":
+        vc = torch.rand_like(vc) * 0.5 + 0.5
+    elif kind == "flat":
+        q, vc = q * 0.01, vc.abs()
+    elif kind == "sharp":
+        q = q * 30.0
+    else:
+        q, kc = (q * 0.2).clamp(-0.9, 0.9) + 8.0, (kc * 0.2).clamp(-0.9, 0.9) + 1.0
+    ctx_row = _row_context()
+    outs = []
+    for c in (ctx, ctx_row):
+        out = torch.zeros_like(q)
+        c.attention(q, None, None, kc, vc, out, tokens, heads, kv_heads, dim, past, kc.shape[1],
+                    scale)
+        c.sync()
+        outs.append(out)
+    ctx_row.close()
+    want = _attention_fp64_cuda(q, kc, vc, past, scale)
+    err, row_err = (float((o.double() - want).norm() / want.norm()) for o in outs)
+    assert err < row_err < 1e-5
