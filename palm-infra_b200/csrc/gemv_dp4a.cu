@@ -1110,7 +1110,7 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
             // Pairs that two CTAs per SM leave to a second wave: one CTA of twice the warps per SM
             // ([19456, 2560] with the norm 10.2 -> 8.9 us; 18944 rows, the last of one wave, 8.6).
             const int all = 2 * ((pairs + ctx->sm_count - 1) / ctx->sm_count);
-            wide = a.top1.cells == nullptr && !a32 &&
+            wide = a.top1.cells == nullptr && !a32 && ctx->gemv_tpc_override == 0 &&
                    (pairs + tpc / 2 - 1) / (tpc / 2) > 2 * ctx->sm_count && all <= kWideTpc &&
                    gemv_smem_bytes(mt, w->k, w->groups, all, scl16, a32, norm != nullptr) <=
                        220 * 1024;

@@ -1214,3 +1214,43 @@ def test_long_runs_on_other_inputs(ctx, tokens, past, heads, kv_heads, dim, kind
     want = _attention_fp64_cuda(q, kc, vc, past, scale)
     err, row_err = (float((o.double() - want).norm() / want.norm()) for o in outs)
     assert err < row_err < 1e-5
+
+
+def test_step_matmul_keeps_the_cap_on_tiles():
+    """B2W4_GEMV_TPC caps the tiles of a block, also where a SwiGLU would else take blocks of twice
+    the warps: one pair of tiles each, the default's bits."""
+    import torch
+    driver = pytest.importorskip("cuda.bindings.driver")
+    n, k, stream = 9728, 2560, torch.cuda.Stream()
+    blocks = pkg.synth.bg128_weight(3, n + k, n, k)
+    x, one = torch.randn((1, k), device="cuda"), torch.ones(k, device="cuda")
+    results, grids = [], []
+    for cap in (None, "2"):
+        if cap:
+            os.environ["B2W4_GEMV_TPC"] = cap
+        try:
+            c = pkg.capi.Context(0)
+        finally:
+            os.environ.pop("B2W4_GEMV_TPC", None)
+        w = c.upload_weight(blocks, n, k)
+        res, y = torch.zeros((1, k), device="cuda"), torch.zeros((1, n // 2), device="cuda")
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph, stream=stream):
+            c.set_stream(torch.cuda.current_stream().cuda_stream)
+            c.step_matmul(w, x, None, one, 1e-6, res, y=y, swiglu=True)
+        raw = driver.CUgraph(init_value=graph.raw_cuda_graph())
+        count = driver.cuGraphGetNodes(raw)[-1]
+        assert count == 1
+        node = driver.cuGraphGetNodes(raw, count)[1][0]
+        grids.append(driver.cuGraphKernelNodeGetParams(node)[1].gridDimX)
+        graph.instantiate()
+        graph.replay()
+        torch.cuda.synchronize()
+        results.append(y)
+        del graph
+        c.set_stream(torch.cuda.current_stream().cuda_stream)
+        w.free()
+        c.close()
+    assert grids[1] == n // 16 and grids[0] < grids[1]
+    assert torch.equal(*results)
