@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(512, 2) gemv_w4a8_stream_kernel(const GemvArgs
 
     const int ipt = (G + 3) >> 2;
     unsigned long long best = 0ull;
-    bool timed_out = false;
+    int waits = chunks;  // chunks that the thread waits for: all, or those before a timeout
 #pragma unroll 1
     for (int c = 0; c < chunks; ++c) {
         const int tile0 = begin + c * a.tpc, ntile = min(a.tpc, end - tile0), b = c % kStreamBufs;
@@ -726,8 +726,8 @@ __global__ void __launch_bounds__(512, 2) gemv_w4a8_stream_kernel(const GemvArgs
         const uint8_t* scl = s_scl + (size_t)b * a.tpc * scl_bytes;
         float* d_out = s_d + (c & 1) * a.tpc * a.d_stride;
         float* sc_out = s_sc + (c & 1) * a.tpc * a.d_stride;
-        if (!timed_out && !mbar_wait_bounded(&s_bar[b], c / kStreamBufs & 1)) {
-            timed_out = true;
+        if (c < waits && !mbar_wait_bounded(&s_bar[b], c / kStreamBufs & 1)) {
+            waits = c;
             b2w4_report_timeout(a.status);
         }
 #pragma unroll 1
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(512, 2) gemv_w4a8_stream_kernel(const GemvArgs
             }
         }
         __syncthreads();  // sums in place, the buffer is free, and so are the sums of chunk c - 1
-        if (threadIdx.x == 0 && c + kStreamBufs < chunks && !timed_out)
+        if (threadIdx.x == 0 && c + kStreamBufs < chunks && c < waits)
             issue(c + kStreamBufs);
         const int mine = ((warp - c) & (kWarps - 1)) * 4 + gl;  // the lane's tile
         if (mine < ntile) {
@@ -769,6 +769,10 @@ __global__ void __launch_bounds__(512, 2) gemv_w4a8_stream_kernel(const GemvArgs
             }
         }
     }
+    // after a timeout: not gone before the copies on their way have been waited for once more
+    if (threadIdx.x == 0)
+        for (int c = waits; c < min(chunks, waits + kStreamBufs); ++c)
+            mbar_wait_bounded(&s_bar[c % kStreamBufs], c / kStreamBufs & 1);
     if (TOP1)
         b2w4_top1_finish(a.top1, best, 0, 1, s_top1);
 }
