@@ -370,7 +370,11 @@ size_t b2w4_chain_weight_bytes(const b2w4_chain* chain);
  *                      heads of 64, 128 or 256 features on 16-byte aligned rows take
  *                      the keys in one block or over a cluster of blocks (up to seven
  *                      tokens, and runs that would leave most of the chip idle), or
- *                      in tiles with a running softmax; any other size or alignment
+ *                      in tiles with a running softmax, long runs of heads of 64 or
+ *                      128 on a cache of 384 rows or more with the products on the
+ *                      tensor cores (every 32-bit operand as three bf16 numbers, which
+ *                      sum to it; sums in 32 bits, truncated; what that cannot hold is
+ *                      done in 32 bits); any other size or alignment
  *                      one block per (token, head), runs of the three head sizes
  *                      tiles too.  The forms sum in different orders, so a token's
  *                      row agrees between them to fp32 rounding, not bit for bit;

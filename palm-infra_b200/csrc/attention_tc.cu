@@ -21,10 +21,11 @@
 //              MMA's layout (values transposed)
 // A score's h h' products go to one sum for one half of the features and to the other for the
 // other: a sum in tensor memory truncates, by less the smaller it is.
-// What bounds it: a step of 64 keys takes about 7500 cycles at DIM = 128.  Its MMAs alone take 2050
+// What bounds it: a step of 64 keys takes about 7700 cycles at DIM = 128.  Its MMAs alone take 2050
 // (scores) and 1600 (P V), its softmax and splits about 4000 of each scheduler (conversions and
-// logic at half rate, paired fp32 instructions two to three cycles each) and its exp about 2000 of
-// the 64-bit and conversion pipes; shared memory serves MMAs, splits and loads for about 3000.
+// logic at half rate, paired fp32 instructions two to three cycles each); the exp lengthens the rows'
+// chain by 1500 (530 instructions of a scheduler's 64-bit pipe, which is busy for 1100); shared
+// memory serves MMAs, splits and loads for about 3000.
 // Measured against the tile form: attn_tensor (decoder_ops.cu).  Tried with an exp in 32 bits, 1500
 // tokens of 32 / 8 heads of 128 (167 us; 208 with this one, 214 with the checks below): all products
 // with m and h of the keys side by side 156 (error 2.3e-7 instead of 1.8e-7), each alone 188; three

@@ -26,8 +26,8 @@
 // products and multiply-adds 224 each and 1140 cycles of the fp32 pipe, fetches 360 on top of
 // them); the operand warps beside it 180, the MMAs nothing, waits 170.
 // MMAs issued by the warp that unpacks the group, against one warp for the MMAs and three that
-// unpack: 40 rows of [2560, 9728] 42.2 -> 37.2 us, 256 rows 53.5 -> 50.0, of [2560, 4096] 26.1 ->
-// 24.7, of [19456, 2560] 74.0 -> 72.7, 64 rows of [9728, 2560] 24.1 -> 22.2.
+// unpack: 40 rows of [2560, 9728] 41.7 -> 36.4 us, 256 rows 53.3 -> 49.7, of [2560, 4096] 25.7 ->
+// 24.1, of [19456, 2560] 73.9 -> 73.3, 64 rows of [9728, 2560] 23.6 -> 21.6.
 // Tried on the form before: waits that poll in a loop of four instructions, or with test_wait,
 // 206 -> 221 us a matmul and 42 -> 62 at 40 rows (pollers take issue slots); hand-over through named
 // barriers 235; units of one block 217; the next chunk's fetch under a chunk's sums: no gain.

@@ -1684,9 +1684,11 @@ static int moe_run(b2w4_ctx* ctx, const float* hidden_dev, int ldx, int tokens, 
     const bool partial = expert_count != num_experts;
     // One token with all experts here: routes need no compaction, each block of the first expert
     // matmul picks its own, and the second one combines its rows.  Measured: 8 of 128 experts of
-    // 768, rows of 2048, 22.6 -> 17.8 us (19.9 with a combine launch); 8 of 64 of 1024, 3072, 29.0
-    // -> 24.8; 8 of 128 of 1536, 4096, 48.3 -> 46.9; 4 of 64 of 384, 1024, 19.2 -> 16.5.  Tried: the
-    // second matmul's weights brought to L2 by the first (no gain).
+    // 768, rows of 2048, 22.6 -> 17.8 us for one token again and again (19.9 with a combine launch), a
+    // call on its own 27.6 -> 21.5, with experts that no call before had 28.7 -> 23.6, with nothing in
+    // L2 29.7 -> 25.7.  In a graph, tokens of other experts in turn, weights not in L2: 22.5 -> 17.3; 8
+    // of 64 of 1024, 3072, 30.6 -> 25.4; 8 of 128 of 1536, 4096, 49.1 -> 48.9; 4 of 64 of 384, 1024,
+    // 18.5 -> 15.5.  Tried: the second matmul's weights brought to L2 by the first (no gain).
     const bool single = fused && tokens == 1 && !partial && !peers && !route_out;
     const bool in_cluster = single && top_k <= kCombineCluster;
     const TokenRoutes first = {logits, idx, wts, nullptr};
