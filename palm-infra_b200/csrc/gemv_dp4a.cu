@@ -1132,12 +1132,13 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
         take(tpc);
         a.d_stride = gemv_d_stride(mt, w->groups, a32);
         // Long rows, split over clusters, from 48 groups on and where the kernel above has at most
-        // four tiles per CTA.  us in a graph, that kernel / split, by weight rows: K = 9728 1000
-        // 5.9 / 4.2, 2560 7.8 / 6.0, 4096 8.5 / 7.6; K = 6144 4.3 / 3.7, 5.6 / 4.7, 5.8 / 5.8, 6144
-        // rows 7.2 / 7.2, 9728 (more tiles) 12.2 / 13.3; K = 5120 4.1 / 3.4, 5.0 / 4.2, 5.1 / 5.2,
-        // 6144 rows 6.2 / 6.4; K = 4096 3.2 / 3.2, 3.9 / 3.8, 4.1 / 4.6, 4.9 / 5.6; K = 2560 2.9 /
-        // 3.1, 3.3 / 3.5, 3.3 / 3.9, 9728 rows 4.7 / 9.4.  (40 groups on up to 2560 rows would
-        // gain too.)
+        // four tiles per CTA and all clusters run at once.  us in a graph, that kernel / split, by
+        // weight rows: K = 9728 1000 5.9 / 4.2, 2560 7.8 / 6.0, 4096 8.5 / 7.6; K = 6144 4.3 / 3.7,
+        // 5.6 / 4.7, 5.8 / 5.8, 6144 rows 7.2 / 7.2, 8704 9.9 / 8.3, and with a second wave 9728 10.5 /
+        // 13.7, 12288 12.2 / 14.2, 20000 17.9 / 22.7; K = 5120 4.1 / 3.4, 5.0 / 4.2, 5.1 / 5.2, 6144
+        // rows 6.2 / 6.4; K = 4096 3.2 / 3.2, 3.9 / 3.8, 4.1 / 4.6, 4.9 / 5.6; K = 2560 2.9 / 3.1, 3.3 /
+        // 3.5, 3.3 / 3.9, 9728 rows 4.7 / 9.4.  (40 groups on up to 2560 rows would gain too; 49 to 56
+        // on 4096 to 6144 lose: 6656 5.7 / 5.9, 6.5 / 6.9, 7.0 / 7.6.)
         if (!a32 && !sums && !tp && !top1 && !norm && !swiglu && ctx->gemv_tpc_override == 0 &&
             w->groups >= 48 && tpc <= 4 && b2w4_gemv_fits(w, 1, act_rule)) {
             const int per = (w->groups + kSplit - 1) / kSplit;
@@ -1145,7 +1146,8 @@ int b2w4_launch_gemv(b2w4_ctx* ctx, const b2w4_weight* w, const float* x, int ld
             const int clusters = wave_ctas / kSplit;
             a.tpc = min(kSplitMaxTiles, (w->tiles + clusters - 1) / clusters);
             const size_t bytes = gemv_split_bytes(per, a.tpc, a.d_stride, scl16);
-            if (bytes <= 113 * 1024)
+            if (bytes <= 113 * 1024 &&
+                (w->tiles + a.tpc - 1) / a.tpc * kSplit <= 2 * ctx->sm_count)
                 return launch_split(ctx, a, scl16, bytes);
             a.tpc = tpc;
         }

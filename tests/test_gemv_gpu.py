@@ -747,3 +747,40 @@ def test_per32_tensor_core_tiles_of_64_and_80_columns(ctx_tc, m, n, k):
     x[m // 2] = np.sign(x[m // 2])  # every code +-127: the largest sums
     y, _ = run_gpu(ctx_tc, blocks, n, k, x, rule=ol.ACT_G32, sums=False, pad=4 if n % 16 else 0)
     assert y.tobytes() == ol.matmul_w4(blocks, n, k, x, rule=ol.ACT_G32).tobytes()
+
+
+@pytest.mark.parametrize("n,k,split", [(8704, 6144, True), (9472, 6144, True), (9480, 6144, False),
+                                       (20000, 6144, False), (2560, 9728, True)])
+def test_split_rows_in_one_wave_of_clusters(ctx, n, k, split):
+    """Long rows are split over clusters of four where all of them run at once (two blocks per
+    multiprocessor); the oracle's bits on either side of the line."""
+    import torch
+    driver = pytest.importorskip("cuda.bindings.driver")
+    blocks = pkg.synth.bg128_weight(20261125, n + k, n, k)
+    x = pkg.synth.activations(91, n, 1, k)
+    w = ctx.upload_weight(blocks, n, k)
+    xd, y = torch.from_numpy(x).cuda(), torch.zeros((1, n), device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    try:
+        with torch.cuda.graph(graph):
+            ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+            ctx.matmul(w, xd, y)
+    finally:
+        ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+    raw = driver.CUgraph(init_value=graph.raw_cuda_graph())
+    count = driver.cuGraphGetNodes(raw)[-1]
+    assert count == 1
+    node = driver.cuGraphGetNodes(raw, count)[1][0]
+    grid = driver.cuGraphKernelNodeGetParams(node)[1].gridDimX
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148:
+        per = 3 if k == 6144 else 2  # tiles in a block of the kernel that does not split
+        other = 2 * sms if n == 20000 else -(-(n // 8) // per)  # persistent blocks
+        assert grid % 4 == 0 and grid <= 2 * sms if split else grid == other
+    graph.instantiate()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert y.cpu().numpy().tobytes() == ol.matmul_w4(blocks, n, k, x).tobytes()
+    del graph
+    w.free()
